@@ -33,11 +33,10 @@ TraceState g_ts;
 constexpr size_t MAX_ENTRIES = 50000;
 constexpr size_t MAX_PROGRAMS = 16;
 
+// One multiply per value: an entry has about twenty of them and a ResNet-50 inference 330 entries.
 inline void mix(uint64_t &h, uint64_t v) {
-  for (int i = 0; i < 8; ++i) {
-    h = (h ^ (v & 0xFF)) * 1099511628211ull;
-    v >>= 8;
-  }
+  h = (h ^ v) * 0x9e3779b97f4a7c15ull;
+  h ^= h >> 32;
 }
 
 bool overlaps(uintptr_t a, int64_t abytes, uintptr_t b, int64_t bbytes) {
