@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "conv_tc_dev.cuh"
+#include "conv_tc_split.cuh"
 #include "kernels.h"
 #include "runtime.h"
 
@@ -462,6 +463,9 @@ struct Plan {
   bool pn;   // pixel-N variant
   bool pair; // CTA-pair form: the grid is launched as clusters of two
   bool duo;  // two independent CTAs per SM (one epilogue warp per TMEM quadrant)
+  bool sk;   // split-reduction kernel (conv_tc_split.cu): `s` instead of `p`
+  bool f16, split;
+  SkParams s;
   size_t smem;
   bool ok;
 };
@@ -475,8 +479,6 @@ static TcFastDiv make_fastdiv(int d) {
   f.shift = (uint32_t)(s - 1);
   return f;
 }
-
-static int floordiv(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
 #ifdef OCCAMY_TC_TIMERS
 // analysis builds only: the device words the kernels' role timers add to
@@ -494,6 +496,201 @@ extern "C" void occamy_tc_timers(long long *out, int clear) {
   if (clear) cudaMemset(tc_timer_words(), 0, 20 * sizeof(long long));
 }
 #endif
+
+static int floordiv(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
+
+// Tensor maps of the A operand and the list of filter taps that read through them.
+static bool make_operand_maps(const TcConvArgs &a, bool flat, int Qg, int bk, const uint32_t *boxA,
+                              CUtensorMap *tmA, TcTap *taps, int *num_taps, bool counted) {
+  const int parts = a.split ? 3 : 1, combos = a.split ? 6 : 1;
+  static const int a_part[6] = {0, 0, 0, 1, 1, 2};
+  const int64_t plane = (int64_t)a.N * a.H * a.W * a.Cf;   // elements of one activation part
+  bool ok = true;
+  *num_taps = 0;
+  if (flat) {
+    const uint64_t dims[4] = {(uint64_t)a.Cf, (uint64_t)Qg, 1, 1};
+    const uint64_t st[3] = {(uint64_t)a.Cf * 2, (uint64_t)Qg * a.Cf * 2, (uint64_t)Qg * a.Cf * 2};
+    for (int part = 0; part < parts; ++part)
+      ok &= make_map(&tmA[part], a.x + part * plane, 4, dims, st, boxA, bk * 2, counted);
+    for (int j = 0; j < combos; ++j) taps[(*num_taps)++] = TcTap{a.split ? a_part[j] : 0, 0, 0};
+    return ok;
+  }
+  // one tensor map per (row phase, column phase) of the stride
+  const int sh = a.stride_h, sw = a.stride_w;
+  int map_of[2][2] = {{-1, -1}, {-1, -1}};
+  int nmaps = 0;
+  for (int r = 0; r < a.R; ++r)
+    for (int s2 = 0; s2 < a.S; ++s2) {
+      const int eh = r - a.pad_h, ew = s2 - a.pad_w;
+      const int ah = floordiv(eh, sh), bh = eh - ah * sh;
+      const int aw = floordiv(ew, sw), bw = ew - aw * sw;
+      if (map_of[bh][bw] < 0) {
+        const int Hm = (a.H - bh + sh - 1) / sh, Wm = (a.W - bw + sw - 1) / sw;
+        // elements from one pixel to the next and from one row to the next (the folded
+        // form's pixels are overlapping windows of a padded row)
+        const int64_t px = a.w_step ? a.w_step : a.Cf;
+        const int64_t rowe = a.row_elems ? a.row_elems : (int64_t)a.W * a.Cf;
+        const bf16 *ptr = a.x + bh * rowe + bw * px;
+        const uint64_t dims[4] = {(uint64_t)a.Cf, (uint64_t)(Wm > 0 ? Wm : 1),
+                                  (uint64_t)(Hm > 0 ? Hm : 1), (uint64_t)a.N};
+        const uint64_t st[3] = {(uint64_t)(sw * px * 2), (uint64_t)(sh * rowe * 2),
+                                (uint64_t)(a.H * rowe * 2)};
+        // the maps of one stride phase, one per operand part, sit next to one another
+        for (int part = 0; part < parts; ++part)
+          ok &= make_map(&tmA[nmaps * parts + part], ptr + part * plane, 4, dims, st, boxA, bk * 2, counted);
+        map_of[bh][bw] = nmaps++;
+      }
+      for (int j = 0; j < combos; ++j)
+        taps[(*num_taps)++] = TcTap{map_of[bh][bw] * parts + (a.split ? a_part[j] : 0), aw, ah};
+    }
+  return ok;
+}
+
+// ---- split-reduction kernel (conv_tc_split.cu) -------------------------------------
+struct SkChoice {
+  int bn, splits, stages;
+  double cost;   // modelled microseconds; < 0: not possible
+};
+
+// Tile width and number of CTAs that share a tile's reduction: the lowest modelled time, all CTAs
+// resident at once (a second wave costs as much as the first: 256->256 3x3 at 14x14, batch 32, 100
+// CTAs of 128 channels 12.3 us, 200 of 64 channels 18.1 us).  The model is a fit, within 10 %, to a
+// sweep of the twelve layer shapes of ResNet-50 at batch 1 to 64, times per layer in a chain of
+// dependent launches:
+//   fixed     launch to launch, first load to last store: 3.25 / 3.65 / 4.6 us at 32 / 64 / 128 channels
+//   k-steps   the tensor pipe (four MMAs of 48.5 cycles up to 64 channels, of 64 at 128) plus what the
+//             L2 adds with many CTAs reading
+//   cluster   0.3 us and, per CTA of the cluster, the exchange of the partial sums
+static SkChoice sk_choose(const TcConvArgs &a, long sp_tiles, int rows, int ksteps, int bk, int a_bytes, int nsm) {
+  SkChoice best{0, 1, 0, -1.0};
+  for (int bn = 128; bn >= 32; bn /= 2) {
+    if (bn > 32 && bn / 2 >= a.K) continue;   // half as wide would do
+#ifdef OCCAMY_TUNING
+    if (const char *f = getenv("OCCAMY_SK_BN")) if (atoi(f) != bn) continue;
+#endif
+    const long tiles = sp_tiles * ((a.K + bn - 1) / bn);
+    const int stage_bytes = a_bytes + bn * bk * 2;
+    // A few-channel stem sums in filter-row order, one accumulator, like the kernel that takes the max
+    // pool along: a model gives the same bits whether that fusion happens or not.
+    const int issuers = a.w_step ? 1 : sk_issuers(bn, a.split != 0);
+    for (int s = 1; s <= (a.w_step ? 1 : SK_MAX_SPLITS) && s <= ksteps; ++s) {
+      // (clusters of more than two leave some SMs of every GPC without a partner)
+      long most = s <= 2 ? nsm : nsm - nsm / 9;
+#ifdef OCCAMY_TUNING
+      if (const char *f = getenv("OCCAMY_SK_S")) if ((atoi(f) < ksteps ? atoi(f) : ksteps) != s) continue;
+      if (getenv("OCCAMY_SK_S")) most = 2 * nsm;
+#endif
+      const long ctas = tiles * s;
+      if (ctas > most) break;
+      const int rows_owner = (rows + s - 1) / s;
+      const int share = (ksteps + s - 1) / s;
+      // Half of the SM's shared memory leaves room for the next layer's prologue; a ring of eight
+      // stages (or all of a CTA's k-steps) is worth more than that: 256->256 3x3 at 14x14, batch 8,
+      // 10.0 us with four stages, 7.4 us with eight.
+      int stages = 0;
+      const size_t fixed = sk_smem_bytes(bn, 0, a_bytes, bk, s, rows_owner) + 16 * SK_MAX_STAGES;
+      for (size_t limit : {TC_SMEM_DUO - 1024, (size_t)TC_SMEM_LIMIT}) {
+        stages = fixed < limit ? (int)((limit - fixed) / stage_bytes) : 0;
+        if (stages > SK_MAX_STAGES) stages = SK_MAX_STAGES;
+        if (stages >= share) stages = share;
+        else stages = stages / issuers * issuers;
+        if (stages >= 8 || stages == share) break;
+      }
+      if (stages < 1) continue;
+      double step = bn == 32 ? 0.095 + 0.00006 * ctas : bn == 64 ? 0.12 + 0.00025 * ctas : 0.155 + 0.0005 * ctas;
+      step *= bk == 64 ? 1.0 : 0.75;
+      if (issuers < 2) step += 0.12;
+      const double exchange = s > 1 ? 0.3 + s * (0.05 + 0.4 * rows / 128.0) : 0.0;
+      const double cost = (bn == 32 ? 3.25 : bn == 64 ? 3.65 : 4.6) + share * step + exchange;
+      if (best.cost < 0 || cost < best.cost) best = SkChoice{bn, s, stages, cost};
+    }
+  }
+  return best;
+}
+
+static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, double rival, Plan *pl) {
+#ifdef OCCAMY_TUNING
+  const char *force = getenv("OCCAMY_SK");
+  if (force && !strcmp(force, "0")) return false;
+#endif
+  const bool flat = a.R == 1 && a.S == 1 && a.stride_h == 1 && a.stride_w == 1 && a.pad_h == 0 &&
+                    a.pad_w == 0 && a.w_step == 0;
+  const int bk = pick_bk(a.Cf);
+  int Qg = a.Q, Pg = a.P, Ng = a.N;
+  if (flat) {
+    Qg = a.N * a.P * a.Q;
+    Pg = Ng = 1;
+  }
+  SkParams &p = pl->s;
+  choose_box(Qg, Pg, Ng, 128, &p.tw, &p.th, &p.tn);
+  p.tiles_w = (Qg + p.tw - 1) / p.tw;
+  p.tiles_h = (Pg + p.th - 1) / p.th;
+  const long sp_tiles = (long)p.tiles_w * p.tiles_h * ((Ng + p.tn - 1) / p.tn);
+  p.rows = p.tw * p.th * p.tn;
+  p.bk = bk;
+  p.cblocks = (a.Cf + bk - 1) / bk;
+  p.ksteps = a.R * a.S * (a.split ? 6 : 1) * p.cblocks;
+  p.a_bytes = ((p.rows + 7) / 8 * 8 * bk * 2 + 1023) / 1024 * 1024;
+  const SkChoice c = sk_choose(a, sp_tiles, p.rows, p.ksteps, bk, p.a_bytes, nsm);
+  if (c.cost < 0) return false;
+#ifdef OCCAMY_TUNING
+  if (!(force && !strcmp(force, "2")))
+#endif
+  if (rival >= 0 && c.cost >= rival) return false;
+  const int bn = c.bn;
+  p.stages = c.stages;
+  p.splits = c.splits;
+  const int share = (p.ksteps + c.splits - 1) / c.splits;
+  p.issuers = a.w_step ? 1 : sk_issuers(c.bn, a.split != 0) < share ? sk_issuers(c.bn, a.split != 0) : share;
+  p.rows_owner = (p.rows + c.splits - 1) / c.splits;
+  p.tiles_k = (a.K + bn - 1) / bn;
+  p.div_k = make_fastdiv(p.tiles_k);
+  p.div_w = make_fastdiv(p.tiles_w);
+  p.div_h = make_fastdiv(p.tiles_h);
+  p.div_cb = make_fastdiv(p.cblocks);
+  p.K = a.K;
+  p.gq = Qg; p.gp = Pg; p.gn = Ng;
+  p.bias = a.bias;
+  p.residual = a.residual;
+  p.y = a.y;
+  p.out_f32 = a.out_f32;
+  p.ldo = a.ldo;
+  p.out_hw = a.out_f32 && a.out_nchw ? a.P * a.Q : 0;
+  p.out_vec4 = a.out_f32 && !p.out_hw && a.ldo % 4 == 0 && (uintptr_t)a.out_f32 % 16 == 0;
+  p.lo = a.act == ACT_RELU ? 0.0f : (a.act == ACT_CLIP ? a.lo : -INFINITY);
+  p.hi = a.act == ACT_CLIP ? a.hi : INFINITY;
+  p.consts_ready = a.consts_ready;
+  p.err = err_word;
+  const uint32_t boxA[4] = {(uint32_t)bk, (uint32_t)p.tw, (uint32_t)p.th, (uint32_t)p.tn};
+  TcTap taps[TC_MAX_TAPS];
+  int num_taps = 0;
+  bool ok = make_operand_maps(a, flat, Qg, bk, boxA, p.tmA, taps, &num_taps, counted);
+  for (int t = 0; t < num_taps; ++t) {
+    if (abs(taps[t].dw) > 127 || abs(taps[t].dh) > 127) return false;
+    p.taps[t] = SkTap{(int8_t)taps[t].map, (int8_t)taps[t].dw, (int8_t)taps[t].dh, 0};
+  }
+  const uint64_t dims[3] = {(uint64_t)a.Cf, (uint64_t)a.K, (uint64_t)num_taps};
+  const uint64_t st[2] = {(uint64_t)a.Cf * 2, (uint64_t)a.K * a.Cf * 2};
+  const uint32_t box[3] = {(uint32_t)bk, (uint32_t)bn, 1};
+  ok &= make_map(&p.tmB, a.w, 3, dims, st, box, bk * 2, counted);
+  if (!ok) return false;
+  pl->sk = true;
+  pl->f16 = a.f16 != 0;
+  pl->split = a.split != 0;
+  pl->bn = bn;
+  pl->p.total_tiles = (int)sp_tiles * p.tiles_k;
+  pl->smem = sk_smem_bytes(bn, p.stages, p.a_bytes, bk, p.splits, p.rows_owner);
+  // the MMA reads 128 rows from the start of every activation stage
+  const size_t reach = (size_t)(p.stages - 1) * p.a_bytes + 128 * bk * 2;
+  if (pl->smem < reach) pl->smem = reach;
+  pl->ok = true;
+#ifdef OCCAMY_TUNING
+  if (getenv("OCCAMY_TC_PLAN_LOG"))
+    fprintf(stderr, "[skplan] K %d Cf %d RS %d px %dx%dx%d rows %d bn %d splits %d ksteps %d stages %d tiles %d smem %zu cost %.2f rival %.2f\n",
+            a.K, a.Cf, a.R * a.S, Qg, Pg, Ng, p.rows, bn, p.splits, p.ksteps, p.stages, pl->p.total_tiles, pl->smem, c.cost, rival);
+#endif
+  return true;
+}
 
 static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool counted,
                        bool allow_halo = true) {
@@ -513,9 +710,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   p.ldo = a.ldo;
   p.out_hw = a.out_f32 && a.out_nchw ? a.P * a.Q : 0;
   // fp32 operands as three bf16 parts: six (activation part, filter part) products per tap
-  const int parts = a.split ? 3 : 1, combos = a.split ? 6 : 1;
-  static const int a_part[6] = {0, 0, 0, 1, 1, 2};
-  const int64_t plane = (int64_t)a.N * a.H * a.W * a.Cf;   // elements of one activation part
+  const int combos = a.split ? 6 : 1;
   p.err = err_word;
 #ifdef OCCAMY_TC_TIMERS
   p.timers = tc_timer_words();
@@ -595,6 +790,16 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   p.div_w = make_fastdiv(p.tiles_w);
   p.div_h = make_fastdiv(p.tiles_h);
 
+  {
+    // The split-reduction kernel where its modelled time is lower.  Of the persistent kernels, fitted to
+    // the same sweep: 3.1 us and 0.27 us per k-step of a CTA's tiles (0.49 us in the pixel-N form,
+    // whose tiles are twice as tall; a whole tile of the halo form takes 0.9 us).
+    const int per_wave = pair ? nsm / 2 : nsm;
+    const double waves = (double)((p.total_tiles + per_wave - 1) / per_wave);
+    const int ks = p.cblocks * a.R * a.S * combos;
+    const double tile_us = halo ? 0.9 : pn ? 0.49 * ks : (bn == 256 ? 0.4 : 0.0) + 0.27 * ks * (bk == 64 ? 1.0 : 0.75);
+    if (sk_plan(a, err_word, nsm, counted, 3.1 + waves * tile_us, &pl)) return pl;
+  }
   const uint32_t boxA[4] = {(uint32_t)bk, (uint32_t)p.tw, (uint32_t)p.th, (uint32_t)p.tn};
   bool ok = true;
   if (halo) {
@@ -603,44 +808,8 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
     const uint32_t box[4] = {64u, (uint32_t)p.tw, (uint32_t)(p.th + 2), 1u};
     ok &= make_map(&p.tmA[0], a.x, 4, dims, st, box, 128, counted);
     p.num_taps = 9;
-  } else if (flat) {
-    const uint64_t dims[4] = {(uint64_t)a.Cf, (uint64_t)Qg, 1, 1};
-    const uint64_t st[3] = {(uint64_t)a.Cf * 2, (uint64_t)Qg * a.Cf * 2, (uint64_t)Qg * a.Cf * 2};
-    for (int part = 0; part < parts; ++part)
-      ok &= make_map(&p.tmA[part], a.x + part * plane, 4, dims, st, boxA, bk * 2, counted);
-    p.num_taps = combos;
-    for (int j = 0; j < combos; ++j) p.taps[j] = TcTap{a.split ? a_part[j] : 0, 0, 0};
   } else {
-    // one tensor map per (row phase, column phase) of the stride
-    const int sh = a.stride_h, sw = a.stride_w;
-    int map_of[2][2] = {{-1, -1}, {-1, -1}};
-    int nmaps = 0;
-    p.num_taps = 0;
-    for (int r = 0; r < a.R; ++r)
-      for (int s2 = 0; s2 < a.S; ++s2) {
-        const int eh = r - a.pad_h, ew = s2 - a.pad_w;
-        const int ah = floordiv(eh, sh), bh = eh - ah * sh;
-        const int aw = floordiv(ew, sw), bw = ew - aw * sw;
-        if (map_of[bh][bw] < 0) {
-          const int Hm = (a.H - bh + sh - 1) / sh, Wm = (a.W - bw + sw - 1) / sw;
-          // elements from one pixel to the next and from one row to the next (the folded
-          // form's pixels are overlapping windows of a padded row)
-          const int64_t px = a.w_step ? a.w_step : a.Cf;
-          const int64_t rowe = a.row_elems ? a.row_elems : (int64_t)a.W * a.Cf;
-          const bf16 *ptr = a.x + bh * rowe + bw * px;
-          const uint64_t dims[4] = {(uint64_t)a.Cf, (uint64_t)(Wm > 0 ? Wm : 1),
-                                    (uint64_t)(Hm > 0 ? Hm : 1), (uint64_t)a.N};
-          const uint64_t st[3] = {(uint64_t)(sw * px * 2), (uint64_t)(sh * rowe * 2),
-                                  (uint64_t)(a.H * rowe * 2)};
-          // the maps of one stride phase, one per operand part, sit next to one another
-          for (int part = 0; part < parts; ++part)
-            ok &= make_map(&p.tmA[nmaps * parts + part], ptr + part * plane, 4, dims, st, boxA,
-                           bk * 2, counted);
-          map_of[bh][bw] = nmaps++;
-        }
-        for (int j = 0; j < combos; ++j)
-          p.taps[p.num_taps++] = TcTap{map_of[bh][bw] * parts + (a.split ? a_part[j] : 0), aw, ah};
-      }
+    ok &= make_operand_maps(a, flat, Qg, bk, boxA, p.tmA, p.taps, &p.num_taps, counted);
   }
   {
     const uint64_t dims[3] = {(uint64_t)a.Cf, (uint64_t)a.K, (uint64_t)(a.R * a.S * combos)};
@@ -782,6 +951,11 @@ static void launch_plan_pn(const Plan &pl, int num_sms, cudaStream_t s) {
 }
 
 static void launch_any(const Plan &pl, int num_sms, cudaStream_t s) {
+  if (pl.sk) {
+    if (!sk_launch(pl.s, pl.bn, pl.f16, pl.split, pl.p.total_tiles, pl.smem, s))
+      set_error(997, "tensor-core conv: no split-reduction kernel for this tile");
+    return;
+  }
   if (pl.pn) {
     launch_plan_pn(pl, num_sms, s);
     return;
@@ -816,6 +990,9 @@ void launch_tc_conv(const TcConvArgs &a, cudaStream_t s) {
   ArgsKey key;
   memset(&key, 0, sizeof(key));
   key.a = a;
+#ifdef OCCAMY_TUNING   // sweeps change the environment between launches
+  if (getenv("OCCAMY_TC_NOCACHE")) plans.clear();
+#endif
   auto it = plans.find(key);
   if (it == plans.end()) {
     if (plans.size() > 4096) plans.clear();

@@ -1,0 +1,464 @@
+// Implicit-GEMM convolution / GEMM for problems with few output tiles: small batches, late layers,
+// classifier heads.
+//
+// The persistent kernel (conv_tc_dev.cuh) gives a tile to one CTA, which walks its whole reduction;
+// with 13 tiles of 72 k-steps (a 3x3 layer on 512 channels, batch 8) most SMs are idle and a layer
+// takes the 18 us of that serial chain.  Here a cluster of up to eight CTAs shares a tile: each
+// multiplies its share of the k-steps into its own TMEM, the partial sums meet over distributed
+// shared memory, and every CTA finishes (bias, residual, clamp, store) its share of the tile's rows.
+// One tile per cluster, nothing persistent: what counts is the latency from the end of the previous
+// layer to the start of the next, so
+//   * the first stages' weight tiles are requested before the wait for the previous kernel;
+//   * the loading thread never waits for a stage when a CTA's share fits the ring;
+//   * the residual and the bias are fetched while the products are being accumulated;
+//   * results go from registers to global memory as 16-byte pieces.  (Through shared memory and one
+//     TMA store the tile's end took 0.5 to 0.9 us longer: 256->64 at 56x56, batch 1, 3.3 -> 4.2 us.)
+// Measured times are at the dispatch rule (conv_tc.cu, sk_choose).
+//
+// Up to four warps issue the MMAs (one lane each, k-steps in turn, an accumulator of their own each)
+// and as many load (one lane each, k-steps in turn), then all eight warps drain the accumulators (two
+// per TMEM lane quadrant, half of the columns each).  Several threads per role, because one thread's
+// round of barrier poll, issue and commit takes 450 to 600 cycles whatever it moves, and the four MMAs
+// of a k-step 200 to 260.  A ring that is reused has a multiple of that many stages: a stage then always
+// belongs to the same two threads, and no barrier can be two phases behind the one that waits on it.
+#include "conv_tc_split.cuh"
+
+#include "kernels.h"
+#include "runtime.h"
+
+namespace occ {
+
+namespace {
+
+__device__ __forceinline__ void cluster_arrive_release() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait_acquire() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c),
+               "r"(d)
+               : "memory");
+}
+
+// Eight channels, sum + bias in v -> residual, clamp, 16-bit values.
+template <bool F16>
+__device__ __forceinline__ uint4 sk_pack16(const SkParams &p, float *v, const uint4 &res) {
+  if (p.residual) {
+    const uint32_t w[4] = {res.x, res.y, res.z, res.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float a, b;
+      f2_unpack(pair16_to_f2<F16>(w[j]), a, b);
+      v[2 * j] += a;
+      v[2 * j + 1] += b;
+    }
+  }
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    o[j] = f2_to_bf16x2<F16>(f2_pack(tc_act(v[2 * j], p.lo, p.hi), tc_act(v[2 * j + 1], p.lo, p.hi)));
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+__device__ __forceinline__ void sk_finish32(const SkParams &p, float *v, int64_t lin, int c) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = tc_act(v[j], p.lo, p.hi);
+  if (p.out_hw) {
+    const int64_t img = lin / p.out_hw;
+    float *o = p.out_f32 + (img * p.K + c) * p.out_hw + (lin - img * p.out_hw);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (c + j < p.K) o[(int64_t)j * p.out_hw] = v[j];
+    return;
+  }
+  float *o = p.out_f32 + lin * p.ldo + c;
+  if (p.out_vec4 && c + 8 <= p.K) {
+    reinterpret_cast<float4 *>(o)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4 *>(o)[1] = make_float4(v[4], v[5], v[6], v[7]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (c + j < p.K) o[j] = v[j];
+  }
+}
+
+}  // namespace
+
+//   BN     output channels of a tile (N of the MMA)
+//   F16    operands and 16-bit output are fp16, else bf16
+//   SPLIT  fp32 operands carried as bf16 parts: tap 0 of every six goes to the main accumulator, the
+//          five correction products to a second one
+//   CL     a tile has more than one CTA
+//   F32    fp32 output
+// One flavour per instantiation: these kernels run for a few microseconds, and every stretch of code
+// that is not in the instruction cache yet costs a tenth of that.
+template <int BN, bool F16, bool SPLIT, bool CL, bool F32>
+__global__ void __launch_bounds__(SK_THREADS, BN == 128 ? 1 : 2)
+    tc_split_kernel(const __grid_constant__ SkParams p) {
+  constexpr uint32_t IDESC = (1u << 4) | (F16 ? 0u : ((1u << 7) | (1u << 10))) |
+                             ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+  constexpr int NI = sk_issuers(BN, SPLIT);
+  constexpr int NACC = NI * (SPLIT ? 2 : 1);                       // accumulators: issuer x (main, correction)
+  static_assert(NACC * BN <= 256, "two CTAs share the 512 TMEM columns of an SM");
+  constexpr int HALF = BN / 2;          // columns of one epilogue thread
+  constexpr int G8 = BN / 8;            // eight-channel groups of a tile row
+
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  if ((smem_u32(smem_raw) & 1023u) != 0u) {
+    if (threadIdx.x == 0) atomicExch(p.err, 1007);
+    return;
+  }
+  const int stages = p.stages, bk = p.bk, splits = CL ? p.splits : 1;
+  const uint32_t a_bytes = (uint32_t)p.a_bytes, b_bytes = (uint32_t)BN * bk * 2u;
+  const uint32_t sA = smem_u32(smem_raw), sB = sA + stages * a_bytes, sX = sB + stages * b_bytes;
+  const uint32_t x_bytes = CL ? (uint32_t)(splits * p.rows_owner) * BN * 4u : 0u;   // partial sums
+  uint8_t *misc = smem_raw + (sX + x_bytes - sA);
+  float *bias_s = reinterpret_cast<float *>(misc);                       // BN floats
+  int *lin_s = reinterpret_cast<int *>(misc + BN * 4);                   // 128 pixel numbers, -1: none
+  uint64_t *bars = reinterpret_cast<uint64_t *>(misc + BN * 4 + 512);
+  const uint32_t bar0 = smem_u32(bars);
+  auto full_bar = [&](int s) { return bar0 + 8u * s; };
+  auto empty_bar = [&](int s) { return bar0 + 8u * (stages + s); };
+  const uint32_t done_bar = bar0 + 16u * stages;
+  volatile uint32_t *tmem_holder = reinterpret_cast<volatile uint32_t *>(bars + 2 * stages + 1);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 2 * stages + 2);
+  // which accumulators hold anything, one word per issuer: bit 0 main, bit 1 correction
+  volatile int *used = reinterpret_cast<volatile int *>(bars + 2 * stages + 3);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // Fewer accumulators when there are fewer k-steps: CTAs of the next layer that share this SM need
+  // TMEM columns as well.  A power of two.
+  const int ni = p.issuers;
+  const uint32_t cols = (uint32_t)(ni == 3 ? 4 : ni) * (SPLIT ? 2u : 1u) * BN;
+  const int rank = CL ? (int)cluster_ctarank() : 0;
+  const int tile = (int)blockIdx.x / splits;
+  // channel tiles fastest, then columns, rows and images of the pixel grid
+  TcTile tl;
+  {
+    const uint32_t sp = tc_fdiv((uint32_t)tile, p.div_k);
+    const uint32_t s2 = tc_fdiv(sp, p.div_w), nn = tc_fdiv(s2, p.div_h);
+    tl.k0 = (int)((uint32_t)tile - sp * (uint32_t)p.tiles_k) * BN;
+    tl.q0 = (int)(sp - s2 * (uint32_t)p.tiles_w) * p.tw;
+    tl.p0 = (int)(s2 - nn * (uint32_t)p.tiles_h) * p.th;
+    tl.n0 = (int)nn * p.tn;
+  }
+  const int ks0 = (int)((int64_t)p.ksteps * rank / splits), ks1 = (int)((int64_t)p.ksteps * (rank + 1) / splits);
+  const int mine = ks1 - ks0;           // k-steps of this CTA
+  int err_code = 0;
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_map(&p.tmB);
+    tma_prefetch_map(&p.tmA[p.taps[0].map]);
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    mbar_init(done_bar, (uint32_t)ni);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 3) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32((const void *)tmem_holder)),
+                 "r"(cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (warp >= 4) {   // pixel number of every row of the tile
+    const int row = (int)threadIdx.x - 128;
+    const int r2 = row / p.tw, q = tl.q0 + row - r2 * p.tw;
+    const int r3 = r2 / p.th, pp = tl.p0 + r2 - r3 * p.th, n = tl.n0 + r3;
+    const bool ok = row < p.rows && q < p.gq && pp < p.gp && n < p.gn;
+    lin_s[row] = ok ? (n * p.gp + pp) * p.gq + q : -1;
+  }
+  tc_fence_before();
+  __syncthreads();
+  if constexpr (CL) cluster_arrive_release();   // waited for before the first remote store
+  tc_fence_after();
+  const uint32_t tmem = *tmem_holder;
+  const uint32_t tx_bytes = (uint32_t)p.rows * bk * 2u + b_bytes;
+  const int ahead = min(stages, mine);        // k-steps that need no stage to become free
+
+  // (tap, channel block) of a k-step of this CTA
+  auto load_b = [&](int i, int s) {
+    const uint32_t t = tc_fdiv((uint32_t)(ks0 + i), p.div_cb);
+    tma_load_3d(sB + s * b_bytes, &p.tmB, full_bar(s), (ks0 + i - (int)t * p.cblocks) * bk, tl.k0, (int)t);
+  };
+  auto load_a = [&](int i, int s) {
+    const uint32_t t = tc_fdiv((uint32_t)(ks0 + i), p.div_cb);
+    const SkTap tap = p.taps[t];
+    tma_load_4d(sA + s * a_bytes, &p.tmA[tap.map], full_bar(s), (ks0 + i - (int)t * p.cblocks) * bk,
+                tl.q0 + tap.dw, tl.p0 + tap.dh, tl.n0);
+  };
+  // The k-steps of the first ring turn are requested by one lane each: a single thread's chain of
+  // index arithmetic, arming arrival and request per k-step is time on the layer's critical path.
+  const int first = warp >= 4 ? warp - 4 + 4 * lane : SK_MAX_STAGES;
+  if (first < ahead && p.consts_ready) {
+    mbar_expect_tx(full_bar(first), tx_bytes);
+    load_b(first, first);
+  }
+  pdl_launch_dependents();
+  pdl_wait();   // from here on memory that other kernels write is read and written
+
+  // residual pieces this thread will add: fetched now, used after the products
+  uint4 res[BN / 16];
+  const int row0 = rank * p.rows_owner;
+  const int nrows = CL ? min(p.rows_owner, p.rows - row0) : 0;   // rows this CTA finishes
+  const int items = nrows * G8;
+  const int quad = warp & 3, part = warp >> 2, row = quad * 32 + lane;
+
+  if (first < ahead) {
+    if (!p.consts_ready) mbar_expect_tx(full_bar(first), tx_bytes);
+    load_a(first, first);
+    if (!p.consts_ready) load_b(first, first);
+  }
+  if (warp >= 4 && warp < 4 + ni && lane == 0) {
+    // later turns (stages is a multiple of ni then): k-step i goes to stage i % stages, loader i % ni
+    int s = warp - 4;
+    uint32_t phase = 0;
+    for (int i = stages + s; i < mine; i += ni) {
+      if (!mbar_wait_hot(empty_bar(s), phase, abort_flag)) {
+        err_code = 1;
+        break;
+      }
+      mbar_expect_tx(full_bar(s), tx_bytes);
+      load_b(i, s);
+      load_a(i, s);
+      s += ni;
+      if (s >= stages) {
+        s -= stages;
+        phase ^= 1u;
+      }
+    }
+  } else if (warp < ni && lane == 0) {
+    const uint64_t a0 = make_smem_desc(sA, bk), b0 = make_smem_desc(sB, bk);
+    const uint32_t a_hi = (uint32_t)(a0 >> 32), b_hi = (uint32_t)(b0 >> 32);
+    const uint32_t a_step = a_bytes >> 4, b_step = b_bytes >> 4;
+    const uint32_t d0 = tmem + (uint32_t)(warp * (SPLIT ? 2 * BN : BN));
+    uint32_t seen = 0;
+    auto run = [&](auto nk_c) {
+      constexpr int NK = decltype(nk_c)::value;
+      uint32_t phase = 0;
+      int s = warp;
+      for (int i = warp; i < mine; i += ni) {
+        uint32_t d = d0, bit = 1u;
+        if constexpr (SPLIT) {
+          const uint32_t tap = tc_fdiv((uint32_t)(ks0 + i), p.div_cb);
+          if (tap % 6u != 0u) {
+            d = d0 + (uint32_t)BN;
+            bit = 2u;
+          }
+        }
+        const uint32_t a_lo = (uint32_t)a0 + (uint32_t)s * a_step, b_lo = (uint32_t)b0 + (uint32_t)s * b_step;
+        const uint32_t more = seen & bit;
+        if (!mbar_wait_hot(full_bar(s), phase, abort_flag)) {
+          err_code = 3;
+          return;
+        }
+        tc_fence_after();
+#pragma unroll
+        for (int kk = 0; kk < NK; ++kk)
+          mma_lohi(d, a_lo + 2u * kk, a_hi, b_lo + 2u * kk, b_hi, IDESC, kk ? 1u : more);
+        seen |= bit;
+        if (i + stages < mine) tc_commit(empty_bar(s));   // nobody waits for the last ones
+        s += ni;
+        if (s >= stages) {   // (a ring as long as the share is never reused)
+          s -= stages;
+          phase ^= 1u;
+        }
+      }
+      tc_commit(done_bar);
+    };
+    if (bk == 64) run(std::integral_constant<int, 4>{});
+    else if (bk == 32) run(std::integral_constant<int, 2>{});
+    else run(std::integral_constant<int, 1>{});
+    used[warp] = (int)seen;
+  }
+  __syncwarp();
+  if (threadIdx.x < BN)
+    bias_s[threadIdx.x] = (p.bias && tl.k0 + (int)threadIdx.x < p.K) ? p.bias[tl.k0 + threadIdx.x] : 0.0f;
+  if (!F32 && p.residual) {
+    if constexpr (CL) {
+#pragma unroll
+      for (int u = 0; u < BN / 16; ++u) {
+        const int it = (int)threadIdx.x + u * SK_THREADS;
+        const int r = it / G8, c = tl.k0 + (it % G8) * 8;
+        const int lin = it < items ? lin_s[row0 + r] : -1;
+        if (lin >= 0 && c < p.K)
+          res[u] = *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(p.residual) +
+                                                    (int64_t)lin * p.K + c);
+      }
+    } else {
+      const int lin = lin_s[row];
+#pragma unroll
+      for (int u = 0; u < BN / 16; ++u) {
+        const int c = tl.k0 + part * HALF + u * 8;
+        if (lin >= 0 && c < p.K)
+          res[u] = *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(p.residual) +
+                                                    (int64_t)lin * p.K + c);
+      }
+    }
+  }
+  __syncwarp();
+  if (!err_code && !mbar_wait(done_bar, 0, abort_flag)) err_code = 4;
+  tc_fence_after();
+  __syncthreads();   // bias_s
+
+  auto finish = [&](float *v, const uint4 &rs, int lin, int c) {
+    if constexpr (F32) sk_finish32(p, v, lin, c);
+    else
+      *reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(p.y) + (int64_t)lin * p.K + c) =
+          sk_pack16<F16>(p, v, rs);
+  };
+  int used_all[NI];
+#pragma unroll
+  for (int w = 0; w < NI; ++w) used_all[w] = w < ni ? used[w] : 0;
+  // columns of this thread's row, 32 at a time (16 for a 32-channel tile): the sum of the accumulators
+  constexpr int CH = HALF < 32 ? HALF : 32;
+  const uint32_t t_row = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(part * HALF);
+  auto load_sum = [&](int h, uint32_t *r) {
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < NACC; ++k) {
+      if (!((used_all[SPLIT ? k / 2 : k] >> (SPLIT ? k & 1 : 0)) & 1)) continue;   // the same for all threads
+      uint32_t t[CH];
+      tc_ld<CH>(t_row + (uint32_t)(k * BN + h * CH), t);
+      tc_ld_wait();
+#pragma unroll
+      for (int j = 0; j < CH; ++j)
+        r[j] = any ? __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(t[j])) : t[j];
+      any = true;
+    }
+  };
+  if constexpr (CL) {
+    cluster_wait_acquire();   // every CTA of the cluster has started
+    const int owner = row / p.rows_owner;
+    const uint32_t dst = row < p.rows ? cluster_map(sX, (uint32_t)owner) +
+                                            (uint32_t)(rank * p.rows_owner + row - owner * p.rows_owner) * (BN * 4u)
+                                      : 0u;
+#pragma unroll
+    for (int h = 0; h < HALF / CH; ++h) {
+      uint32_t r[CH];
+      load_sum(h, r);
+      if (row < p.rows && !err_code) {
+#pragma unroll
+        for (int j = 0; j < CH / 4; ++j) {
+          // 16-byte pieces of a row are permuted by its number: eight lanes, eight bank groups
+          const uint32_t piece = (uint32_t)((part * HALF + h * CH) / 4 + j) ^ (uint32_t)(row & 7);
+          st_cluster_v4(dst + piece * 16u, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+        }
+      }
+      __syncwarp();
+    }
+    __syncwarp();
+    tc_fence_before();
+    cluster_arrive_release();
+    cluster_wait_acquire();
+    const uint8_t *xs = smem_raw + (sX - sA);
+    auto item = [&](int it, int r, int g, const uint4 &rs) {
+      const int lin = lin_s[row0 + r], c = tl.k0 + g * 8;
+      if (lin < 0 || c >= p.K) return;
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = bias_s[g * 8 + j];
+      const uint32_t sw = (uint32_t)((row0 + r) & 7);
+      for (int k = 0; k < splits; ++k) {
+        const uint8_t *b = xs + (size_t)(k * p.rows_owner + r) * (BN * 4);
+        const float4 a = *reinterpret_cast<const float4 *>(b + (((uint32_t)(2 * g)) ^ sw) * 16u);
+        const float4 e = *reinterpret_cast<const float4 *>(b + (((uint32_t)(2 * g + 1)) ^ sw) * 16u);
+        v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+        v[4] += e.x; v[5] += e.y; v[6] += e.z; v[7] += e.w;
+      }
+      finish(v, rs, lin, c);
+    };
+    if (!err_code) {
+      if (F32 && p.out_hw) {   // consecutive threads on consecutive pixels of one channel
+        for (int it = threadIdx.x; it < items; it += SK_THREADS) item(it, it % nrows, it / nrows, res[0]);
+      } else {
+#pragma unroll
+        for (int u = 0; u < BN / 16; ++u) {
+          const int it = (int)threadIdx.x + u * SK_THREADS;
+          if (it < items) item(it, it / G8, it % G8, res[u]);
+        }
+      }
+    }
+  } else {
+    const int lin = lin_s[row];
+#pragma unroll
+    for (int h = 0; h < HALF / CH; ++h) {
+      uint32_t r[CH];
+      load_sum(h, r);
+      if (lin >= 0 && !err_code) {
+#pragma unroll
+        for (int u = 0; u < CH / 8; ++u) {
+          const int cl = part * HALF + h * CH + u * 8;
+          if (tl.k0 + cl >= p.K) break;
+          float v[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[u * 8 + j]) + bias_s[cl + j];
+          finish(v, res[h * (CH / 8) + u], lin, tl.k0 + cl);
+        }
+      }
+    }
+    tc_fence_before();
+  }
+
+  if (err_code) {
+    atomicExch(p.err, 1000 + err_code);
+    *abort_flag = 1;
+    for (int i = 0; i < 50; ++i) __nanosleep(20000);   // copies in flight land before memory goes
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 3)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(cols)
+                 : "memory");
+}
+
+size_t sk_smem_bytes(int bn, int stages, int a_bytes, int bk, int splits, int rows_owner) {
+  const size_t x = splits > 1 ? (size_t)splits * rows_owner * bn * 4 : 0;
+  return (size_t)stages * (a_bytes + bn * bk * 2) + x +
+         bn * 4 + 512 + 8 * (2 * stages + 6);
+}
+
+template <int BN, bool F16, bool SPLIT, bool CL, bool F32>
+static void sk_launch_one(const SkParams &p, int tiles, size_t smem, cudaStream_t s) {
+  auto kernel = tc_split_kernel<BN, F16, SPLIT, CL, F32>;
+  static unsigned char attr_done[TC_MAX_DEVICES] = {};
+  if (tc_first_use_on_device(attr_done)) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_LIMIT);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  }
+  tc_launch_pdl(kernel, tiles * p.splits, SK_THREADS, smem, s, p, p.splits);
+}
+
+template <int BN>
+static void sk_launch_bn(const SkParams &p, bool f16, bool split, int tiles, size_t smem, cudaStream_t s) {
+  const bool cl = p.splits > 1, f32 = p.out_f32 != nullptr;
+  if (split) {
+    if (cl) sk_launch_one<BN, false, true, true, true>(p, tiles, smem, s);
+    else sk_launch_one<BN, false, true, false, true>(p, tiles, smem, s);
+  } else if (f16) {
+    if (cl && f32) sk_launch_one<BN, true, false, true, true>(p, tiles, smem, s);
+    else if (cl) sk_launch_one<BN, true, false, true, false>(p, tiles, smem, s);
+    else if (f32) sk_launch_one<BN, true, false, false, true>(p, tiles, smem, s);
+    else sk_launch_one<BN, true, false, false, false>(p, tiles, smem, s);
+  } else {
+    if (cl && f32) sk_launch_one<BN, false, false, true, true>(p, tiles, smem, s);
+    else if (cl) sk_launch_one<BN, false, false, true, false>(p, tiles, smem, s);
+    else if (f32) sk_launch_one<BN, false, false, false, true>(p, tiles, smem, s);
+    else sk_launch_one<BN, false, false, false, false>(p, tiles, smem, s);
+  }
+}
+
+bool sk_launch(const SkParams &p, int bn, bool f16, bool split, int tiles, size_t smem, cudaStream_t s) {
+  if (bn == 32) sk_launch_bn<32>(p, f16, split, tiles, smem, s);
+  else if (bn == 64) sk_launch_bn<64>(p, f16, split, tiles, smem, s);
+  else if (bn == 128) sk_launch_bn<128>(p, f16, split, tiles, smem, s);
+  else return false;
+  return true;
+}
+
+}  // namespace occ

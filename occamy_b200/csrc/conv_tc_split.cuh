@@ -1,0 +1,51 @@
+// Parameter block of the split-reduction convolution kernel (conv_tc_split.cu) and its launcher.
+#pragma once
+#include "conv_tc_dev.cuh"
+
+namespace occ {
+
+constexpr int SK_THREADS = 256;
+constexpr int SK_MAX_SPLITS = 8;       // portable cluster size
+constexpr int SK_MAX_STAGES = 16;
+
+struct SkTap {
+  int8_t map, dw, dh, pad;
+};
+
+struct alignas(64) SkParams {
+  CUtensorMap tmA[TC_MAX_AMAPS];
+  CUtensorMap tmB;
+  SkTap taps[TC_MAX_TAPS];
+  int cblocks, bk, stages, ksteps;     // ksteps = taps * cblocks
+  int issuers;                         // threads that issue MMAs: sk_issuers(), but no more than k-steps
+  int splits;                          // CTAs (one cluster) that share a tile's reduction
+  TcFastDiv div_k, div_w, div_h, div_cb;
+  int tiles_k, tiles_w, tiles_h;
+  int tw, th, tn;
+  int rows;                            // pixels of a tile's box (<= 128)
+  int rows_owner;                      // rows each CTA of the cluster sums up and stores
+  int a_bytes;                         // bytes of a stage's activation tile (multiple of 1024)
+  int K, gq, gp, gn;
+  const float *bias;
+  const void *residual;                // 16-bit NHWC like the output, or null
+  void *y;                             // 16-bit NHWC output (when out_f32 is null)
+  float *out_f32;
+  int ldo, out_hw;                     // as in TcParams
+  int out_vec4;                        // row-major fp32 output whose rows are 16-byte aligned
+  float lo, hi;
+  int consts_ready;
+  int *err;
+};
+
+// Threads that issue MMAs (and that load) in a kernel: as many accumulators as fit the 256 TMEM
+// columns a CTA may use, four at most.  A ring with fewer stages than the CTA has k-steps must have a
+// multiple of this many.
+__host__ __device__ constexpr int sk_issuers(int bn, bool split) {
+  return 256 / (bn * (split ? 2 : 1)) < 4 ? 256 / (bn * (split ? 2 : 1)) : 4;
+}
+// Shared memory a launch needs.
+size_t sk_smem_bytes(int bn, int stages, int a_bytes, int bk, int splits, int rows_owner);
+// `split` selects the kernels whose operands are bf16 parts of fp32 values (see TC_MODE_SPLIT).
+bool sk_launch(const SkParams &p, int bn, bool f16, bool split, int tiles, size_t smem, cudaStream_t s);
+
+}  // namespace occ

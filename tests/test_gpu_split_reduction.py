@@ -1,0 +1,64 @@
+"""The split-reduction convolution / GEMM kernel (few output tiles, a cluster of CTAs per tile) at the
+edges of its tiles and of its splits, against the CPU oracle."""
+import numpy as np
+import pytest
+
+from helpers import max_rel_err, run_graph_oracle
+from occamy_b200 import graphs, replay
+from occamy_b200 import runtime as rt
+
+pytestmark = pytest.mark.gpu
+
+TOL = {rt.MATH_FP32: 1e-4, rt.MATH_BF16: 2e-2, rt.MATH_F16: 2e-2}
+
+# (N, C, H, W, K, R, stride): reductions of 1 to 72 k-steps in 1 to 8 shares, equal or not; tiles of 1
+# to 128 pixels, several images per tile, channel counts that leave a partial last tile
+SHAPES = [
+    (1, 16, 1, 1, 8, 1, 1),
+    (1, 64, 7, 7, 40, 1, 1),
+    (1, 512, 7, 7, 512, 3, 1),
+    (3, 512, 7, 7, 200, 3, 1),
+    (2, 448, 5, 9, 72, 3, 2),
+    (1, 2048, 7, 7, 136, 1, 1),
+    (2, 272, 13, 11, 96, 3, 1),
+    (4, 96, 12, 12, 264, 3, 1),
+    (1, 1024, 14, 14, 256, 1, 2),
+]
+
+
+@pytest.mark.parametrize("mode", sorted(TOL))
+@pytest.mark.parametrize("shape", SHAPES)
+def test_conv_with_residual(binding, shape, mode):
+    """conv + bias + shortcut + ReLU, as separate calls and (third pass) as one kernel."""
+    N, C, H, W, K, R, st = shape
+    g = graphs.Graph((N, C, H, W), seed=sum(shape))
+    ws, bs = g.he_conv(K, C, 1, 1)
+    short = g.conv(0, ws, bs, strides=(st, st))
+    w, b = g.he_conv(K, C, R, R)
+    y = g.conv(0, w, b, pads=(R // 2, R // 2), strides=(st, st))
+    g.mark_output(g.relu(g.add(y, short)))
+    x = graphs.make_input(g, 1)
+    (want,) = run_graph_oracle(g, x)
+    rt.set_math_mode(mode)
+    p = g.to_program()
+    p.lower(fuse=replay.FUSE_REFERENCE)
+    for _ in range(3):
+        (got,) = p.run(binding, x)
+        assert max_rel_err(got, want) <= TOL[mode]
+    assert rt.last_error() == 0
+
+
+@pytest.mark.parametrize("mode", sorted(TOL))
+@pytest.mark.parametrize("M,K,N", [(1, 2048, 1000), (5, 4096, 4096), (33, 1280, 10), (128, 512, 1000), (130, 4096, 36)])
+def test_gemm(binding, M, K, N, mode):
+    g = graphs.Graph((M, K), seed=M + N)
+    g.mark_output(g.linear(0, K, N))
+    x = graphs.make_input(g, 2)
+    (want,) = run_graph_oracle(g, x)
+    rt.set_math_mode(mode)
+    p = g.to_program()
+    p.lower(fuse=replay.FUSE_REFERENCE)
+    for _ in range(2):
+        (got,) = p.run(binding, x)
+        assert max_rel_err(got, want) <= TOL[mode]
+    assert rt.last_error() == 0
