@@ -1,8 +1,10 @@
 // The C-ABI entry points on the CNN hot path (declared in include/occamy_dnn_api.h) and
 // the dispatch between the fp32 NCHW kernels and the bf16 NHWC / tensor-core kernels.
 #include <cstring>
+#include <initializer_list>
 #include <vector>
 
+#include "graph_replay.h"
 #include "kernels.h"
 #include "runtime.h"
 #include "trace.h"
@@ -69,13 +71,15 @@ enum PackLayout { PACK_KRSC = 1, PACK_DW = 2, PACK_FOLD = 3, PACK_RAW = 4, PACK_
 // launch_split3_nchw); off with OCCAMY_FP32_TC=0 or occamy_set_fp32_tensor_cores(0), which
 // leaves the CUDA-core kernels.
 int g_fp32_tc = -1;
-bool fp32_tc_enabled() {
+}  // namespace
+bool occ::fp32_on_tensor_cores() {
   if (g_fp32_tc < 0) {
     const char *e = getenv("OCCAMY_FP32_TC");
     g_fp32_tc = (e && !strcmp(e, "0")) ? 0 : 1;
   }
   return g_fp32_tc == 1;
 }
+namespace {
 
 // Device pointer of the packed form of the filter at `w`; resident across calls when the
 // filter was uploaded from host memory (a compiled model's constant), otherwise packed
@@ -106,7 +110,9 @@ void *packed_weights(const float *w, int layout, size_t packed_bytes, int K, int
   ensure_f32(w);
   void *dst = nullptr;
   if (cacheable) {
+    graph_stop_capture();   // packed once, not in every inference
     PackedWeight &pw = r.wcache[key];
+    if (pw.dev) graph_forget_all();   // graphs refer to the old contents
     if (pw.dev && pw.bytes != packed_bytes) {
       OCC_CUDA(cudaStreamSynchronize(r.stream));
       OCC_CUDA(cudaFree(pw.dev));
@@ -132,7 +138,8 @@ void *packed_weights(const float *w, int layout, size_t packed_bytes, int K, int
   return dst;
 }
 
-// Small fp32 constants (biases): the resident copy when there is one, else the tensor itself.
+// fp32 constants used as they are (biases mostly): the resident copy when there is one, else the
+// tensor itself.
 const float *resident_f32(const float *p, size_t bytes) {
   uintptr_t base;
   TensorRec *rec = reg_find(p, &base);
@@ -386,9 +393,11 @@ void before_write_hook(const void *p, size_t bytes) { pending_guard_range(p, byt
 
 Role step(Entry &e, bool passive) {
   rt().before_write = before_write_hook;
+  if (graph_covers(e)) return R_SKIP;
   bool deviated = false;
   const Role role = trace_step(e, &deviated);
   if (deviated) {
+    graph_stop_capture();
     flush_pending();
     // Tensors that fusion skipped earlier in this inference stay unwritten.  The recorded
     // program had no reader for them; should this (different) program read one, that read
@@ -405,6 +414,23 @@ Role step(Entry &e, bool passive) {
   }
   return role;
 }
+
+// A call's arguments in its trace entry (run_again makes the call from them).
+void put(Entry &e, std::initializer_list<const void *> ptrs) {
+  int i = 0;
+  for (const void *p : ptrs) e.args.p[i++] = const_cast<void *>(p);
+}
+// appends n values behind the ones already there
+void put(Entry &e, int &at, const int64_t *d, int64_t n) {
+  for (int64_t i = 0; i < n && at < 24; ++i) e.args.v[at++] = d[i];
+}
+void put(Entry &e, int &at, int64_t v) { put(e, at, &v, 1); }
+
+// Opens every traced entry point: when the call has been carried out, a recorded stretch of calls
+// may begin or end behind it.
+struct CallScope {
+  ~CallScope() { graph_after_call(); }
+};
 
 void elide(void *p) {
   uintptr_t base;
@@ -470,7 +496,12 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
   g.Q = shape_ok ? (g.W + 2 * g.pad_w - g.S) / g.stride_w + 1 : 0;
   const bool depthwise = g.groups > 1 && g.groups == g.C && g.K == g.C;
 
+  CallScope scope;
   Entry e = trace_entry(sym);
+  int at = 0;
+  put(e, {x, w, bias, y});
+  put(e, at, dX, 4); put(e, at, dW, 4); put(e, at, pads, 2); put(e, at, strides, 2);
+  put(e, at, groups); put(e, at, act_mode);
   te_ptr(e, x); te_ptr(e, w); te_ptr(e, bias); te_ptr(e, y);
   te_dims(e, dX, 4); te_dims(e, dW, 4); te_dims(e, pads, 2); te_dims(e, strides, 2);
   te_i(e, groups); te_i(e, act_mode);
@@ -488,6 +519,7 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
   e.poolable = e.fusable && r.mode == MATH_BF16 && !depthwise && g.C <= 4 && g.K == 64 && g.stride_w == 2 && g.Q <= 128 &&
                g.S <= 16 && g.R <= 11;
   const Role role = step(e, false);
+  if (role == R_SKIP) return y;
 
   if (!shape_ok) {
     set_error(997, "convolution: inconsistent shape");
@@ -519,12 +551,12 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
       return y;
     }
   }
-  if (r.mode == MATH_FP32 && fp32_tc_enabled() && conv_f32_on_tensor_cores(x, w, bias, g, y)) return y;
+  if (r.mode == MATH_FP32 && fp32_on_tensor_cores() && conv_f32_on_tensor_cores(x, w, bias, g, y)) return y;
   ensure_f32(x);
-  ensure_f32(w);
-  if (bias) ensure_f32(bias);
-  if (depthwise) launch_depthwise_f32(x, w, bias, y, g, r.stream);
-  else launch_conv_f32(x, w, bias, y, g, r.stream);
+  const float *wd = resident_f32(w, (size_t)numel4(dW) * 4);
+  const float *bd = bias ? resident_f32(bias, (size_t)g.K * 4) : nullptr;
+  if (depthwise) launch_depthwise_f32(x, wd, bd, y, g, r.stream);
+  else launch_conv_f32(x, wd, bd, y, g, r.stream);
   mark_f32(y);
   return y;
 }
@@ -554,6 +586,7 @@ cudaError_t wrapDNNMalloc(void **devPtr, size_t size) {
   rt();
   cudaError_t err = cudaMalloc(devPtr, size ? size : 1);
   if (err != cudaSuccess) die("Malloc", err, size);
+  CallScope scope;
   Entry e = trace_entry(S_MALLOC);
   te_i(e, (int64_t)size);
   e.out = (uintptr_t)*devPtr;
@@ -605,22 +638,30 @@ cudaError_t wrapDNNMemPoolInit(void **devPtr, size_t size) {
   g_pools.push_back(PoolRec{*devPtr, size});
   if ((int64_t)size > r.counters[CNT_POOL_HWM]) r.counters[CNT_POOL_HWM] = (int64_t)size;
   trace_set_pool(*devPtr, size);
+  CallScope scope;
   Entry e = trace_entry(S_POOLINIT);
   te_i(e, (int64_t)size);
   step(e, false);
   return cudaSuccess;
 }
 
+static void hand_out(void *p, size_t bytes) {
+  CallScope scope;
+  Entry e = trace_entry(S_MEMOFFSET);
+  te_ptr(e, p);
+  te_i(e, (int64_t)bytes);
+  e.out = (uintptr_t)p;
+  e.out_bytes = (int64_t)bytes;
+  put(e, {p});
+  e.args.v[0] = (int64_t)bytes;
+  if (step(e, true) == R_SKIP) return;
+  pending_guard_range(p, bytes, false);
+  reg_new(p, bytes, FMT_ZERO);
+}
+
 cudaError_t wrapDNNMemOffset(void **devPtr, void *basePtr, size_t offset, size_t mallocSize) {
   *devPtr = (char *)basePtr + offset;
-  Entry e = trace_entry(S_MEMOFFSET);
-  te_ptr(e, *devPtr);
-  te_i(e, (int64_t)mallocSize);
-  e.out = (uintptr_t)*devPtr;
-  e.out_bytes = (int64_t)mallocSize;
-  step(e, true);
-  pending_guard_range(*devPtr, mallocSize, false);
-  reg_new(*devPtr, mallocSize, FMT_ZERO);
+  hand_out(*devPtr, mallocSize);
   return cudaSuccess;
 }
 
@@ -629,18 +670,28 @@ cudaError_t wrapDNNMemcpy(void *dst, const void *src, size_t count_, int kind,
   Runtime &r = rt();
   if (count_ == 0) return cudaSuccess;
   cudaError_t err = cudaSuccess;
+  CallScope scope;
   if (kind == 1 || kind == 3) {
     Entry e = trace_entry(kind == 1 ? S_H2D : S_D2D);
-    te_ptr(e, dst);
+    if (kind == 1) te_ptr(e, dst);
+    else te_ptr_or_elsewhere(e, dst);
     te_i(e, (int64_t)count_);
+    put(e, {dst});
+    e.args.v[0] = (int64_t)count_;
+    uint64_t hash = 0;
+    if (kind == 1) {
+      hash = host_hash(src, count_);
+      e.args.v[1] = (int64_t)hash;
+      e.host = src;
+    }
     if (kind == 3) {
-      te_ptr(e, src);
+      te_ptr_or_elsewhere(e, src);
       e.in[0] = (uintptr_t)src;
       e.in_bytes[0] = (int64_t)count_;
     }
     e.out = (uintptr_t)dst;
     e.out_bytes = (int64_t)count_;
-    step(e, kind == 1);
+    if (step(e, kind == 1) == R_SKIP) return cudaSuccess;
     if (kind == 3) {
       pending_guard_range(dst, count_, true);
       ensure_f32(src);
@@ -652,7 +703,7 @@ cudaError_t wrapDNNMemcpy(void *dst, const void *src, size_t count_, int kind,
     if (kind == 1 && whole) {
       rec->host_src = src;
       rec->host_bytes = count_;
-      rec->host_hash = host_hash(src, count_);
+      rec->host_hash = hash;
       // A constant whose packed form is already resident need not cross PCIe again; the
       // copy is made later only if something other than a convolution / GEMM reads it.
       if (r.cache_weights) {
@@ -665,7 +716,11 @@ cudaError_t wrapDNNMemcpy(void *dst, const void *src, size_t count_, int kind,
         }
       }
     }
-    if (kind == 1) pending_guard_range(dst, count_, true);
+    if (kind == 1) {
+      graph_before_upload();
+      trace_mark_uploaded();
+      pending_guard_range(dst, count_, true);
+    }
     const bool in_pool = g_cur_pool && (uintptr_t)dst >= (uintptr_t)g_cur_pool &&
                          (uintptr_t)dst + count_ <= (uintptr_t)g_cur_pool + g_cur_pool_bytes;
     if (kind == 1 && whole && in_pool && count_ >= (1u << 20) && pool_cache_blocks() >= 2) {
@@ -757,6 +812,7 @@ cudaError_t wrapDNNDealloc(void *devPtr) {
       g_pools.erase(g_pools.begin() + i);
       break;
     }
+  CallScope scope;
   if (was_pool) {
     Entry e = trace_entry(S_POOLFREE);
     step(e, false);   // runs whatever is still held back
@@ -807,11 +863,13 @@ cudaError_t wrapDNNDealloc(void *devPtr) {
 int cudnnCreate(cudnnContext **handle) {
   rt();
   *handle = reinterpret_cast<cudnnContext *>(malloc(16));
+  graph_inference_begin();
   flush_pending();
   trace_begin();
   return *handle ? 0 : 2;
 }
 int cudnnDestroy(cudnnContext *handle) {
+  graph_inference_end();
   flush_pending();
   trace_end();
   free(handle);
@@ -846,12 +904,17 @@ float *DNNActiveFunc(cudnnContext *, float *x, int64_t dimX[4], int32_t mode, fl
   Runtime &r = rt();
   const int64_t n = numel4(dimX);
   const int act = mode == 0 ? ACT_SIGMOID : (mode == 1 ? ACT_RELU : (mode == 2 ? ACT_TANH : ACT_IDENTITY));
+  CallScope scope;
   Entry e = trace_entry(S_ACTIVE);
+  int at = 0;
+  put(e, {x, y});
+  put(e, at, dimX, 4); put(e, at, mode);
   te_ptr(e, x); te_ptr(e, y); te_dims(e, dimX, 4); te_i(e, mode);
   e.in[0] = (uintptr_t)x; e.in_bytes[0] = n * 4; e.out = (uintptr_t)y; e.out_bytes = n * 4;
   for (int i = 0; i < 4; ++i) e.dims[i] = dimX[i];
   e.kind = mode == 1 ? CK_RELU : CK_NONE;
   const Role role = step(e, false);
+  if (role == R_SKIP) return y;
   if (role == R_ABSORB && g_pending.active) {
     const ConvGeom &g = g_pending.g;
     if (mode == 1 && x == g_pending.out && !g_pending.act_set && dimX[0] == g.N &&
@@ -879,12 +942,18 @@ float *DNNActiveFunc(cudnnContext *, float *x, int64_t dimX[4], int32_t mode, fl
 float *CUDAClipFunc(float *x, float *y, int64_t *dimOut, float lo, float hi, int64_t rank) {
   Runtime &r = rt();
   const int64_t n = prod(dimOut, rank);
+  CallScope scope;
   Entry e = trace_entry(S_CLIP);
+  int at = 0;
+  put(e, {x, y});
+  put(e, at, rank); put(e, at, dimOut, rank);
+  e.args.f[0] = lo; e.args.f[1] = hi;
   te_ptr(e, x); te_ptr(e, y); te_dims(e, dimOut, (int)rank); te_f(e, lo); te_f(e, hi);
   e.in[0] = (uintptr_t)x; e.in_bytes[0] = n * 4; e.out = (uintptr_t)y; e.out_bytes = n * 4;
   for (int i = 0; i < 4 && i < rank; ++i) e.dims[i] = dimOut[i];
   e.kind = rank == 4 ? CK_CLIP : CK_NONE;
   const Role role = step(e, false);
+  if (role == R_SKIP) return y;
   if (role == R_ABSORB && g_pending.active) {
     const ConvGeom &g = g_pending.g;
     if (rank == 4 && x == g_pending.out && !g_pending.act_set && dimOut[0] == g.N &&
@@ -927,7 +996,13 @@ float *DNNTensorOpFunc(cudnnContext *, int64_t opMode, float *A, int64_t *dimA, 
   const bool bias_shape = rank_ok && rankA == 4 && dB[0] == 1 && dB[1] == dimA[1] && dB[2] == 1 &&
                           dB[3] == 1 && !same;
 
+  CallScope scope;
   Entry e = trace_entry(S_TENSOR_OP);
+  int at = 0;
+  put(e, {A, B, out});
+  put(e, at, opMode); put(e, at, rankA); put(e, at, rankB);
+  if (rank_ok) { put(e, at, dimA, rankA); put(e, at, dimB, rankB); }
+  e.args.f[0] = bias;
   te_ptr(e, A); te_ptr(e, B); te_ptr(e, out);
   te_i(e, opMode); te_f(e, bias);
   if (rank_ok) { te_dims(e, dimA, rankA); te_dims(e, dB, rankA); }
@@ -938,6 +1013,7 @@ float *DNNTensorOpFunc(cudnnContext *, int64_t opMode, float *A, int64_t *dimA, 
   for (int i = 0; i < 4 && i < rankA; ++i) e.dims[i] = dimA[i];
   if (opMode == 0 && bias == 1.0f) e.kind = bias_shape ? CK_BIAS_ADD : (same ? CK_SAME_ADD : CK_NONE);
   const Role role = step(e, false);
+  if (role == R_SKIP) return out;
 
   if (!rank_ok) {
     set_error(996, "tensor op: unsupported rank");
@@ -990,12 +1066,13 @@ float *DNNTensorOpFunc(cudnnContext *, int64_t opMode, float *A, int64_t *dimA, 
     }
   }
   ensure_f32(A);
-  if (opMode != 4) ensure_f32(B);
+  // a constant (the C operand of a Gemm, say) is read from its resident copy
+  const float *Bd = opMode != 4 ? resident_f32(B, (size_t)prod(dB, rankA) * 4) : B;
   if (opMode != 0 && opMode != 1 && opMode != 4) {
     set_error(996, "tensor op: unsupported mode");
     return out;
   }
-  launch_tensor_op_f32((int)opMode, A, B, out, rankA, dimA, dB, bias, r.stream);
+  launch_tensor_op_f32((int)opMode, A, Bd, out, rankA, dimA, dB, bias, r.stream);
   mark_f32(out);
   return out;
 }
@@ -1007,7 +1084,11 @@ static float *pool_common(int sym, float *x, int64_t *dI, float *y, int64_t *dO,
   const int N = (int)dI[0], C = (int)dI[1], H = (int)dI[2], W = (int)dI[3];
   const int P = (int)dO[2], Q = (int)dO[3];
   const int ph = (int)padding[0], pw = (int)padding[2];
+  CallScope scope;
   Entry e = trace_entry(sym);
+  int at = 0;
+  put(e, {x, y});
+  put(e, at, dI, 4); put(e, at, dO, 4); put(e, at, kernel, 2); put(e, at, padding, 4); put(e, at, stride, 2);
   te_ptr(e, x); te_ptr(e, y); te_dims(e, dI, 4); te_dims(e, dO, 4); te_dims(e, kernel, 2);
   te_dims(e, padding, 4); te_dims(e, stride, 2);
   e.in[0] = (uintptr_t)x; e.in_bytes[0] = numel4(dI) * 4; e.out = (uintptr_t)y;
@@ -1016,6 +1097,7 @@ static float *pool_common(int sym, float *x, int64_t *dI, float *y, int64_t *dO,
       pw == 1 && padding[1] == 1 && padding[3] == 1)
     e.kind = CK_POOL_3S2;
   const Role role = step(e, false);
+  if (role == R_SKIP) return y;
   if (role == R_ABSORB && g_pending.active) {
     // the held-back stem convolution and this pool run as one kernel
     ConvJob &j = g_pending;
@@ -1075,13 +1157,18 @@ float *DNNAveragePoolFunc(cudnnContext *, float *x, int64_t dimIn[4], float *y, 
 float *DNNReduceFunc(cudnnContext *, int32_t rank, float *x, int64_t *dimIn, float *y,
                      int64_t *dimOut, int32_t mode) {
   Runtime &r = rt();
+  CallScope scope;
   Entry e = trace_entry(S_REDUCE);
+  int at = 0;
+  put(e, {x, y});
+  put(e, at, rank); put(e, at, mode);
+  if (rank <= 8 && rank > 0) { put(e, at, dimIn, rank); put(e, at, dimOut, rank); }
   te_ptr(e, x); te_ptr(e, y); te_i(e, mode);
   if (rank <= 8 && rank > 0) { te_dims(e, dimIn, rank); te_dims(e, dimOut, rank); }
   e.in[0] = (uintptr_t)x; e.out = (uintptr_t)y;
   e.out_bytes = rank <= 8 && rank > 0 ? prod(dimOut, rank) * 4 : 0;
   e.in_bytes[0] = rank <= 8 && rank > 0 ? prod(dimIn, rank) * 4 : 0;
-  step(e, false);
+  if (step(e, false) == R_SKIP) return y;
   if (mode != 5 || rank > 8) {
     set_error(995, "reduce: only mode 5 (mean) is implemented");
     return y;
@@ -1108,14 +1195,19 @@ float *CUBLASMatmul2dFunc(int64_t /*rank*/, float *A, int64_t dimA[2], float *B,
   const int M = (int)(transA ? dimA[1] : dimA[0]);
   const int K = (int)(transA ? dimA[0] : dimA[1]);
   const int N = (int)(transB ? dimB[0] : dimB[1]);
+  CallScope scope;
   Entry e = trace_entry(S_MATMUL);
+  int at = 0;
+  put(e, {A, B, out});
+  put(e, at, dimA, 2); put(e, at, dimB, 2); put(e, at, transA); put(e, at, transB);
+  e.args.f[0] = alpha; e.args.f[1] = beta;
   te_ptr(e, A); te_ptr(e, B); te_ptr(e, out); te_dims(e, dimA, 2); te_dims(e, dimB, 2);
   te_f(e, alpha); te_f(e, beta); te_i(e, transA); te_i(e, transB);
   e.in[0] = (uintptr_t)A; e.in[1] = (uintptr_t)B; e.in[2] = beta != 0.0f ? (uintptr_t)out : 0;
   e.out = (uintptr_t)out; e.out_bytes = (int64_t)M * N * 4;
   e.in_bytes[0] = dimA[0] * dimA[1] * 4; e.in_bytes[1] = dimB[0] * dimB[1] * 4;
   e.in_bytes[2] = e.out_bytes;
-  step(e, false);
+  if (step(e, false) == R_SKIP) return out;
   if (r.log) fprintf(stderr, "[occamy] matmul2d M%d N%d K%d tA%d tB%d\n", M, N, K, (int)transA, (int)transB);
   const bool out_zero = is_zero(out);
   if (r.mode != MATH_FP32 && !transA && transB && alpha == 1.0f && (beta == 0.0f || out_zero) &&
@@ -1144,7 +1236,7 @@ float *CUBLASMatmul2dFunc(int64_t /*rank*/, float *A, int64_t dimA[2], float *B,
       }
     }
   }
-  if (r.mode == MATH_FP32 && fp32_tc_enabled() && !transA && transB && alpha == 1.0f &&
+  if (r.mode == MATH_FP32 && fp32_on_tensor_cores() && !transA && transB && alpha == 1.0f &&
       (beta == 0.0f || out_zero) && M > 0 && (double)M * N * K >= 1e6) {
     // the same split-operand scheme as the convolutions, as a 1x1 convolution over M "pixels"
     const int Kp = (K + 15) / 16 * 16;
@@ -1173,9 +1265,9 @@ float *CUBLASMatmul2dFunc(int64_t /*rank*/, float *A, int64_t dimA[2], float *B,
     }
   }
   ensure_f32(A);
-  ensure_f32(B);
+  const float *Bd = resident_f32(B, (size_t)(dimB[0] * dimB[1]) * 4);
   if (beta != 0.0f) ensure_f32(out);
-  launch_gemm_f32(A, B, out, M, N, K, (int)dimA[1], (int)dimB[1], alpha, out_zero ? 0.0f : beta,
+  launch_gemm_f32(A, Bd, out, M, N, K, (int)dimA[1], (int)dimB[1], alpha, out_zero ? 0.0f : beta,
                   transA != 0, transB != 0, r.stream);
   mark_f32(out);
   return out;
@@ -1188,11 +1280,15 @@ float *CUDASoftmaxFunc(float *x, int64_t *dimIn, float *y, int64_t * /*dimOut*/,
   int64_t outer = 1, inner = 1;
   for (int64_t i = 0; i < axis; ++i) outer *= dimIn[i];
   for (int64_t i = axis + 1; i < rank; ++i) inner *= dimIn[i];
+  CallScope scope;
   Entry e = trace_entry(S_SOFTMAX);
+  int at = 0;
+  put(e, {x, y});
+  put(e, at, axis); put(e, at, rank); put(e, at, dimIn, rank);
   te_ptr(e, x); te_ptr(e, y); te_dims(e, dimIn, (int)rank); te_i(e, axis);
   e.in[0] = (uintptr_t)x; e.out = (uintptr_t)y; e.out_bytes = prod(dimIn, rank) * 4;
   e.in_bytes[0] = e.out_bytes;
-  step(e, false);
+  if (step(e, false) == R_SKIP) return y;
   ensure_f32(x);
   launch_softmax_f32(x, y, outer, dimIn[axis], inner, r.stream);
   mark_f32(y);
@@ -1202,10 +1298,14 @@ float *CUDASoftmaxFunc(float *x, int64_t *dimIn, float *y, int64_t * /*dimOut*/,
 static float *copy_common(int sym, float *x, int64_t *dimIn, int64_t rank, float *y) {
   Runtime &r = rt();
   const int64_t n = prod(dimIn, rank);
+  CallScope scope;
   Entry e = trace_entry(sym);
+  int at = 0;
+  put(e, {x, y});
+  put(e, at, rank); put(e, at, dimIn, rank);
   te_ptr(e, x); te_ptr(e, y); te_dims(e, dimIn, (int)rank);
   e.in[0] = (uintptr_t)x; e.in_bytes[0] = n * 4; e.out = (uintptr_t)y; e.out_bytes = n * 4;
-  step(e, false);
+  if (step(e, false) == R_SKIP) return y;
   ensure_f32(x);
   OCC_CUDA(cudaMemcpyAsync(y, x, (size_t)n * 4, cudaMemcpyDeviceToDevice, r.stream));
   mark_f32(y);
@@ -1224,12 +1324,59 @@ float *CUDAReshapeFunc(float *x, int64_t *dimIn, int64_t rank, float *y) {
 // Called by the entry points outside this file: they take part in no chain and their
 // reads are not tracked, so they end the speculation for this inference.
 void occamy_internal_opaque_call(void) {
+  graph_settle();
   Entry e = trace_entry(S_OPAQUE);
   step(e, false);
 }
 
+}  // extern "C"
+
+// ---------------------------------------------------------------- made again
+void occ::flush_held_back() { flush_pending(); }
+bool occ::anything_held_back() { return g_pending.active; }
+
+// The call of entry `e`, its pool pointers `shift` bytes further on; `host` is the source of a constant.
+void occ::run_again(const Entry &e, intptr_t shift, uintptr_t pool_base, size_t pool_bytes, const void *host) {
+  void *p[4];
+  for (int k = 0; k < 4; ++k) {
+    const uintptr_t a = (uintptr_t)e.args.p[k];
+    p[k] = (void *)(a >= pool_base && a < pool_base + pool_bytes ? a + shift : a);
+  }
+  float *const f[4] = {(float *)p[0], (float *)p[1], (float *)p[2], (float *)p[3]};
+  int64_t v[24];
+  memcpy(v, e.args.v, sizeof(v));
+  switch (e.sym) {
+    case S_MEMOFFSET: hand_out(p[0], (size_t)v[0]); break;
+    case S_H2D: wrapDNNMemcpy(p[0], host, (size_t)v[0], 1, nullptr); break;
+    case S_CONV:
+      DNNConvFunc(nullptr, f[0], v, f[1], v + 4, nullptr, 0, 0, v[12], v + 8, v + 10, f[3]);
+      break;
+    case S_CONV_BIAS_ACT:
+      DNNConvBiasActivFunc(nullptr, f[0], v, f[1], v + 4, f[2], v, nullptr, 0, 0, v + 8, v + 10, v[13], f[3]);
+      break;
+    case S_ACTIVE: DNNActiveFunc(nullptr, f[0], v, (int32_t)v[4], f[1]); break;
+    case S_CLIP: CUDAClipFunc(f[0], f[1], v + 1, e.args.f[0], e.args.f[1], v[0]); break;
+    case S_TENSOR_OP:
+      DNNTensorOpFunc(nullptr, v[0], f[0], v + 3, (int32_t)v[1], f[1], v + 3 + v[1], (int32_t)v[2], f[2], v + 3,
+                      (int32_t)v[1], e.args.f[0]);
+      break;
+    case S_MAXPOOL: DNNMaxPoolFunc(nullptr, f[0], v, f[1], v + 4, v + 8, v + 10, v + 14); break;
+    case S_AVGPOOL: DNNAveragePoolFunc(nullptr, f[0], v, f[1], v + 4, v + 8, v + 10, v + 14); break;
+    case S_REDUCE: DNNReduceFunc(nullptr, (int32_t)v[0], f[0], v + 2, f[1], v + 2 + v[0], (int32_t)v[1]); break;
+    case S_MATMUL:
+      CUBLASMatmul2dFunc(2, f[0], v, f[1], v + 2, f[2], v, f[2], v, e.args.f[0], e.args.f[1], v[4], v[5]);
+      break;
+    case S_SOFTMAX: CUDASoftmaxFunc(f[0], v + 2, f[1], v + 2, v[0], v[1]); break;
+    case S_FLATTEN: CUDAFlattenFunc(f[0], v + 1, f[1], v + 1, 1, v[0]); break;
+    case S_RESHAPE: CUDAReshapeFunc(f[0], v + 1, v[0], f[1]); break;
+    default: break;   // a window holds no other calls
+  }
+}
+
+extern "C" {
 // ---------------------------------------------------------------- controls
 void occamy_set_math_mode(int mode) {
+  graph_settle();
   flush_pending();   // what is held back was prepared for the mode it arrived in
   rt().mode = mode == 0 ? MATH_FP32 : (mode == 2 ? MATH_F16 : MATH_BF16);
 }
@@ -1248,6 +1395,7 @@ int occamy_last_error(int clear) {
 
 int occamy_synchronize(void) {
   Runtime &r = rt();
+  graph_settle();
   flush_pending();
   cudaError_t e = cudaStreamSynchronize(r.stream);
   if (e != cudaSuccess) set_error((int)e, "synchronize");
@@ -1263,9 +1411,14 @@ int occamy_synchronize(void) {
   return (int)e;
 }
 
-cudaStream_t occamy_stream(void) { return rt().stream; }
+cudaStream_t occamy_stream(void) {
+  rt();
+  graph_settle();   // the caller may order work of its own behind the calls made so far
+  return rt().stream;
+}
 
 void occamy_selftest_bounded_wait(void) {
+  graph_settle();
   flush_pending();
   launch_selftest_bounded_wait(rt().stream);
 }
@@ -1280,12 +1433,14 @@ void occamy_clear_weight_cache(void);
 
 void occamy_profile_begin(void) {
   Runtime &r = rt();
+  graph_settle();
   r.prof_count = 0;
   r.profiling = true;
 }
 
 int occamy_profile_end(float *ms, int cap) {
   Runtime &r = rt();
+  graph_settle();
   flush_pending();
   r.profiling = false;
   OCC_CUDA(cudaStreamSynchronize(r.stream));
@@ -1300,19 +1455,26 @@ int occamy_profile_end(float *ms, int cap) {
 }
 
 void occamy_set_cross_call_fusion(int on) {
+  graph_settle();
   flush_pending();
   trace_set_enabled(on != 0);
 }
 
-void occamy_set_fp32_tensor_cores(int on) { g_fp32_tc = on ? 1 : 0; }
+void occamy_set_fp32_tensor_cores(int on) {
+  graph_settle();
+  g_fp32_tc = on ? 1 : 0;
+}
 
 void occamy_set_weight_cache(int on) {
+  graph_settle();
   if (!on) occamy_clear_weight_cache();
   rt().cache_weights = on != 0;
 }
 
 void occamy_clear_weight_cache(void) {
   Runtime &r = rt();
+  graph_settle();
+  graph_forget_all();
   flush_pending();
   OCC_CUDA(cudaStreamSynchronize(r.stream));
   for (auto &kv : r.wcache)

@@ -3,6 +3,7 @@
 
 #include <cstring>
 
+#include "graph_replay.h"
 #include "kernels.h"
 
 namespace occ {
@@ -152,6 +153,7 @@ void ensure_f32(const void *p) {
     OCC_CUDA(cudaMemsetAsync((void *)base, 0, rec->bytes, r.stream));
     r.main_copies++;
   } else if (rec->fmt == FMT_PENDING) {
+    graph_stop_capture();
     OCC_CUDA(cudaMemcpyAsync((void *)base, rec->host_src, rec->host_bytes, cudaMemcpyHostToDevice,
                              r.stream));
     r.main_copies++;
@@ -171,6 +173,7 @@ void *scratch_get(int slot, size_t bytes) {
   Runtime &r = rt();
   if (r.scratch_bytes[slot] >= bytes) return r.scratch[slot];
   // Growing: work already enqueued may still use the old block.
+  graph_forget_all();
   if (r.scratch[slot]) {
     OCC_CUDA(cudaStreamSynchronize(r.stream));
     OCC_CUDA(cudaFree(r.scratch[slot]));

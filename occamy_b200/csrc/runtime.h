@@ -99,6 +99,9 @@ struct Runtime {
   std::vector<cudaEvent_t> prof_events;
 };
 
+// fp32 mode: dense convolutions and GEMMs go to the tensor cores (occamy_set_fp32_tensor_cores)
+bool fp32_on_tensor_cores();
+
 Runtime &rt();  // lazily initialised on the current device
 
 void set_error(int code, const char *where);

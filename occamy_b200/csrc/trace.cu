@@ -1,6 +1,7 @@
 // Recording, matching and analysis of per-inference call traces (see trace.h).
 #include "trace.h"
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 
@@ -10,25 +11,25 @@ namespace occ {
 
 namespace {
 
-struct TraceProgram {
-  std::vector<uint64_t> sigs;
-  std::vector<uint8_t> roles;
-};
-
 struct TraceState {
   int enabled = -1;
   bool in_inference = false;
   bool matched_so_far = false;   // at least one recorded program still matches
-  std::vector<Entry> rec;
+  std::vector<Entry> rec;        // calls of this inference behind the adopted prefix
+  TraceProgram *prefix = nullptr;   // program whose first prefix_len calls this inference made in one go
+  size_t prefix_len = 0;
   std::vector<TraceProgram> programs;
   std::vector<int> cands;
   uintptr_t pool_base = 0;
   size_t pool_bytes = 0;
+  uintptr_t last_pool_base = 0;   // the pool of this inference, also after it was given back
+  size_t last_pool_bytes = 0;
   int elided = 0;
   int64_t fused_chains = 0;
 };
 
-TraceState g_ts;
+// never destroyed: recorded programs own CUDA graphs, and the driver may be gone by then
+TraceState &g_ts = *new TraceState;
 
 constexpr size_t MAX_ENTRIES = 50000;
 constexpr size_t MAX_PROGRAMS = 16;
@@ -132,6 +133,24 @@ void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles) {
   }
 }
 
+// Writes the adopted prefix out as calls of this inference, their pointers moved to its pool.
+void trace_rewind_entries() {
+  TraceState &ts = g_ts;
+  if (!ts.prefix_len) return;
+  std::vector<Entry> all(ts.prefix->entries.begin(), ts.prefix->entries.begin() + ts.prefix_len);
+  const uintptr_t from = ts.prefix->pool_base, bytes = ts.prefix->pool_bytes, to = ts.last_pool_base;
+  auto move = [&](uintptr_t a) { return a >= from && a < from + bytes ? a - from + to : a; };
+  for (Entry &e : all) {
+    for (int k = 0; k < 3; ++k) e.in[k] = move(e.in[k]);
+    e.out = move(e.out);
+    for (int k = 0; k < 4; ++k) e.args.p[k] = (void *)move((uintptr_t)e.args.p[k]);
+  }
+  all.insert(all.end(), ts.rec.begin(), ts.rec.end());
+  ts.rec.swap(all);
+  ts.prefix = nullptr;
+  ts.prefix_len = 0;
+}
+
 }  // namespace
 
 bool trace_enabled() {
@@ -148,6 +167,8 @@ void trace_set_enabled(bool on) {
     g_ts.programs.clear();
     g_ts.cands.clear();
     g_ts.rec.clear();
+    g_ts.prefix = nullptr;
+    g_ts.prefix_len = 0;
     g_ts.in_inference = false;
   }
 }
@@ -165,6 +186,12 @@ void te_ptr(Entry &e, const void *p) {
     a = (a - g_ts.pool_base) | (1ull << 63);
   mix(e.sig, (uint64_t)a);
 }
+void te_ptr_or_elsewhere(Entry &e, const void *p) {
+  uintptr_t a = (uintptr_t)p;
+  if (!g_ts.pool_base) mix(e.sig, (uint64_t)a);
+  else if (a >= g_ts.pool_base && a < g_ts.pool_base + g_ts.pool_bytes) te_ptr(e, p);
+  else mix(e.sig, 1);
+}
 void te_i(Entry &e, int64_t v) { mix(e.sig, (uint64_t)v); }
 void te_f(Entry &e, float v) {
   uint32_t u;
@@ -179,13 +206,13 @@ Role trace_step(Entry &e, bool *deviated) {
   *deviated = false;
   TraceState &ts = g_ts;
   if (!trace_enabled() || !ts.in_inference) return R_EAGER;
-  if (ts.rec.size() >= MAX_ENTRIES) {  // not a compiled model's call pattern: stop tracing
+  if (trace_index() >= MAX_ENTRIES) {  // not a compiled model's call pattern: stop tracing
     ts.in_inference = false;
     *deviated = ts.matched_so_far;
     ts.matched_so_far = false;
     return R_EAGER;
   }
-  const size_t index = ts.rec.size();
+  const size_t index = trace_index();
   Role role = R_EAGER;
   if (!ts.cands.empty()) {
     size_t keep = 0;
@@ -216,6 +243,8 @@ void trace_begin() {
   ts.in_inference = true;
   ts.matched_so_far = false;
   ts.rec.clear();
+  ts.prefix = nullptr;
+  ts.prefix_len = 0;
   ts.elided = 0;
   ts.cands.clear();
   for (size_t i = 0; i < ts.programs.size(); ++i) ts.cands.push_back((int)i);
@@ -225,24 +254,68 @@ void trace_end() {
   TraceState &ts = g_ts;
   if (!trace_enabled() || !ts.in_inference) return;
   ts.in_inference = false;
+  const size_t n = trace_index();
   bool known = false;
   for (int c : ts.cands)
-    if (ts.programs[c].sigs.size() == ts.rec.size()) known = true;
-  if (!known && !ts.rec.empty()) {
+    if (ts.programs[c].sigs.size() == n) known = true;
+  if (!known && n) {
+    trace_rewind_entries();
     TraceProgram p;
-    p.sigs.reserve(ts.rec.size());
+    p.sigs.reserve(n);
     for (const Entry &e : ts.rec) p.sigs.push_back(e.sig);
     analyse(ts.rec, p.roles);
+    p.entries.swap(ts.rec);
+    p.pool_base = ts.last_pool_base;
+    p.pool_bytes = ts.last_pool_bytes;
     if (ts.programs.size() >= MAX_PROGRAMS) ts.programs.erase(ts.programs.begin());
     ts.programs.push_back(std::move(p));
   }
   ts.rec.clear();
+  ts.prefix = nullptr;
+  ts.prefix_len = 0;
   ts.cands.clear();
+}
+
+// ---- prefixes made in one go (graph_replay.cu) ------------------------------------
+bool trace_active() { return trace_enabled() && g_ts.in_inference; }
+size_t trace_index() { return g_ts.prefix_len + g_ts.rec.size(); }
+TraceProgram *trace_candidate() {
+  return g_ts.cands.size() == 1 ? &g_ts.programs[g_ts.cands[0]] : nullptr;
+}
+void trace_mark_uploaded() {
+  if (trace_active() && !g_ts.rec.empty()) g_ts.rec.back().uploaded = true;
+}
+bool trace_has_own_entries() { return g_ts.prefix_len == 0; }
+const std::vector<Entry> &trace_entries() { return g_ts.rec; }
+uintptr_t trace_pool_base() { return g_ts.pool_base; }
+size_t trace_pool_bytes() { return g_ts.pool_bytes; }
+
+void trace_adopt_prefix(TraceProgram *p, size_t n) {
+  g_ts.rec.clear();
+  g_ts.prefix = p;
+  g_ts.prefix_len = n;
+}
+
+void trace_rewind(TraceProgram *p, size_t n) {
+  TraceState &ts = g_ts;
+  trace_adopt_prefix(p, n);
+  trace_rewind_entries();
+  ts.cands.clear();
+  for (size_t i = 0; i < ts.programs.size(); ++i) {
+    const TraceProgram &q = ts.programs[i];
+    if (q.sigs.size() >= n && std::equal(q.sigs.begin(), q.sigs.begin() + n, p->sigs.begin()))
+      ts.cands.push_back((int)i);
+  }
+  ts.matched_so_far = true;
 }
 
 void trace_set_pool(void *base, size_t bytes) {
   g_ts.pool_base = (uintptr_t)base;
   g_ts.pool_bytes = bytes;
+  if (base) {
+    g_ts.last_pool_base = (uintptr_t)base;
+    g_ts.last_pool_bytes = bytes;
+  }
 }
 
 void trace_note_elided() {

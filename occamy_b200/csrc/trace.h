@@ -14,6 +14,7 @@
 #pragma once
 #include <cstddef>
 #include <cstdint>
+#include <memory>
 #include <vector>
 
 namespace occ {
@@ -24,12 +25,20 @@ enum Sym {
   S_MATMUL, S_SOFTMAX, S_FLATTEN, S_RESHAPE, S_OPAQUE
 };
 
-enum Role { R_EAGER = 0, R_DEFER = 1, R_ABSORB = 2 };
+// R_SKIP: the call is part of a recorded stretch that runs as one CUDA graph (graph_replay.h)
+enum Role { R_EAGER = 0, R_DEFER = 1, R_ABSORB = 2, R_SKIP = 3 };
 
 // kind of a tensor-op / activation entry, as far as chains care
 enum ChainKind {
   CK_NONE = 0, CK_BIAS_ADD = 1, CK_SAME_ADD = 2, CK_RELU = 3, CK_CLIP = 4,
   CK_POOL_3S2 = 5   // max pool 3x3, stride 2, pad 1
+};
+
+// The call's own arguments, enough to make it again (graph_replay.cu, run_again).
+struct CallArgs {
+  void *p[4] = {nullptr, nullptr, nullptr, nullptr};
+  int64_t v[24] = {};
+  float f[2] = {0.f, 0.f};
 };
 
 struct Entry {
@@ -44,6 +53,9 @@ struct Entry {
   bool fusable = false;    // convolution that the bf16 path takes (may head a chain)
   bool depthwise = false;
   bool poolable = false;   // convolution whose kernel can take a following CK_POOL_3S2 along
+  bool uploaded = false;   // S_H2D: bytes crossed to the device (not a constant that is already there)
+  const void *host = nullptr;   // S_H2D: source
+  CallArgs args;
 };
 
 // Signature building.  Device pointers are taken relative to the active pool when they
@@ -54,6 +66,21 @@ void te_i(Entry &e, int64_t v);
 void te_f(Entry &e, float v);
 void te_dims(Entry &e, const int64_t *d, int n);
 
+// A pointer that names the same tensor only when it lies in the active pool; any other device
+// address counts as "elsewhere" while a pool is active (the caller's batch, its result buffer).
+void te_ptr_or_elsewhere(Entry &e, const void *p);
+
+// A recorded inference: the calls between cudnnCreate and cudnnDestroy and the role of each.
+struct GraphPlan;
+struct TraceProgram {
+  std::vector<uint64_t> sigs;
+  std::vector<uint8_t> roles;
+  std::vector<Entry> entries;
+  uintptr_t pool_base = 0;     // pool the entries' pointers refer to
+  size_t pool_bytes = 0;
+  std::shared_ptr<GraphPlan> graph;
+};
+
 // Records the call and returns the role the matching recorded program gives it.
 // *deviated is set when this call is the first of the inference that matches no recorded
 // program although earlier calls did.
@@ -61,6 +88,19 @@ Role trace_step(Entry &e, bool *deviated);
 
 void trace_begin();                 // cudnnCreate
 void trace_end();                   // cudnnDestroy: analyse and store if the sequence is new
+// ---- for graph_replay.cu ----
+bool trace_active();                // between the two, and tracing
+size_t trace_index();               // calls of this inference so far
+TraceProgram *trace_candidate();    // the one recorded program that matches so far, or null
+void trace_mark_uploaded();         // the call recorded last moved bytes to the device
+bool trace_has_own_entries();       // this inference was recorded call by call
+const std::vector<Entry> &trace_entries();
+// The calls up to `n` are those of `p`, made without trace_step().
+void trace_adopt_prefix(TraceProgram *p, size_t n);
+// The same, as if they had been made one by one: what follows is recorded and matched anew.
+void trace_rewind(TraceProgram *p, size_t n);
+uintptr_t trace_pool_base();
+size_t trace_pool_bytes();
 void trace_set_pool(void *base, size_t bytes);
 void trace_note_elided();           // a tensor of this inference was skipped by a fusion
 bool trace_has_elided();

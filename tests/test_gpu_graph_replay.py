@@ -1,0 +1,183 @@
+"""Recorded inferences that run as CUDA graphs: same bits as call by call, and every way out of one
+(another constant, another continuation, a wait or the end in the middle)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import max_rel_err, run_graph_oracle
+from occamy_b200 import graphs, replay
+from occamy_b200 import runtime as rt
+
+pytestmark = pytest.mark.gpu
+
+PASSES = 9   # recorded, fused, quiet, captured once per pool block, then replayed
+
+
+def _model(name, math, fuse, batch=2):
+    rt.set_math_mode(math)
+    kw = {"softmax": True} if name == "resnet50" else {}
+    g = getattr(graphs, name)(batch=batch, seed=3, image=64, **kw)
+    p = g.to_program()
+    p.lower(fuse=fuse)
+    return g, p
+
+
+@pytest.mark.parametrize("io", ["host", "device"])
+@pytest.mark.parametrize("name,math,fuse", [
+    ("resnet50", rt.MATH_BF16, 1), ("resnet50", rt.MATH_BF16, 0), ("resnet50", rt.MATH_FP32, 1),
+    ("mobilenet_v2", rt.MATH_F16, 1), ("vgg16", rt.MATH_BF16, 1)])
+def test_same_bits_and_launches(binding, name, math, fuse, io):
+    g, p = _model(name, math, fuse)
+    xs = [graphs.make_input(g, s) for s in (1, 2)]
+    dev = [torch.from_numpy(x).cuda() for x in xs]
+    outs, launches = [], []
+    for i in range(PASSES):
+        n0 = rt.counters()["launches"]
+        if io == "host":
+            (y,) = p.run(binding, xs[i % 2])
+        else:
+            yd = torch.empty(g.shapes[g.outputs[0]], device="cuda")
+            torch.cuda.synchronize()
+            p.run_raw(binding, dev[i % 2].data_ptr(), 3, [yd.data_ptr()], 3)
+            rt.synchronize()
+            y = yd.cpu().numpy()
+        outs.append(y)
+        launches.append(rt.counters()["launches"] - n0)
+    assert rt.last_error() == 0
+    for i in range(3, PASSES):   # pass 2 ran call by call with the chains of pass 1
+        assert np.array_equal(outs[i], outs[i - 2])
+    assert len(set(launches[3:])) == 1
+    (want,) = run_graph_oracle(g, xs[0])
+    assert max_rel_err(outs[-1 if PASSES % 2 else -2], want) <= (1e-4 if math == rt.MATH_FP32 else 3e-2)
+
+
+def test_changed_constant_is_seen(binding):
+    g, p = _model("vgg16", rt.MATH_BF16, 1)
+    x = graphs.make_input(g, 1)
+    conv = [n for n in g.nodes if n.op == "conv"][5]
+    w = next(a for a in p._keep if a.shape == g.consts[conv.ins[1]].shape and np.array_equal(a, g.consts[conv.ins[1]]))
+    for _ in range(PASSES):
+        (before,) = p.run(binding, x)
+    old = w.copy()
+    for scale in (1.5, 0.5, 1.0):   # there and back again
+        w[...] = old * scale
+        g.consts[conv.ins[1]] = w
+        (want,) = run_graph_oracle(g, x)
+        for _ in range(PASSES):
+            (y,) = p.run(binding, x)
+            assert max_rel_err(y, want) <= 3e-2
+    assert np.array_equal(y, before)
+    assert rt.last_error() == 0
+
+
+def test_two_sets_of_weights(binding):
+    """One architecture, two models served in turn: same calls, other constants."""
+    rt.set_math_mode(rt.MATH_BF16)
+    models = []
+    for seed in (1, 2):
+        g = graphs.resnet50(batch=1, seed=seed, image=64, softmax=False)
+        p = g.to_program()
+        p.lower(fuse=1)
+        x = graphs.make_input(g, seed)
+        models.append((p, x, run_graph_oracle(g, x)[0]))
+    for i in range(4 * PASSES):
+        p, x, want = models[(i * i // 3) % 2]
+        (y,) = p.run(binding, x)
+        assert max_rel_err(y, want) <= 2e-2
+    assert rt.last_error() == 0
+
+
+def test_other_continuation(binding):
+    """Two models with the same first layers: the recorded one is left in the middle of its window."""
+    rt.set_math_mode(rt.MATH_F16)   # 18 layers: bf16 storage alone is off by 5e-2
+    models = []
+    for tail in ("relu", "clip", "add"):
+        g = graphs.Graph((2, 16, 20, 20), seed=5)
+        y = 0
+        for _ in range(18):
+            w, b = g.he_conv(16, 16, 3, 3)
+            y = g.relu(g.conv(y, w, b, pads=(1, 1)))
+        y = g.relu(y) if tail == "relu" else g.clip(y, 0.0, 0.7) if tail == "clip" else g.add(y, y)
+        g.mark_output(y)
+        p = g.to_program()
+        p.lower(fuse=1)
+        x = graphs.make_input(g, 4)
+        models.append((p, x, run_graph_oracle(g, x)[0]))
+    for which in [0] * PASSES + [1, 0, 1, 0, 0] + [1] * PASSES + [2, 0, 1, 2, 2, 1, 0]:
+        p, x, want = models[which]
+        (y,) = p.run(binding, x)
+        assert max_rel_err(y, want) <= 2e-2
+    assert rt.last_error() == 0
+
+
+class _HandModel:
+    """x -> conv -> conv -> ... by direct ABI calls, so that a test can stop in the middle."""
+
+    def __init__(self, layers=20, c=16, hw=12):
+        r = np.random.default_rng(0)
+        self.n, self.shape = layers, (1, c, hw, hw)
+        self.w = [(r.standard_normal((c, c, 3, 3)) * 0.08).astype(np.float32) for _ in range(layers)]
+        self.b = [(r.standard_normal(c) * 0.1).astype(np.float32) for _ in range(layers)]
+        self.x = r.standard_normal(self.shape).astype(np.float32)
+
+    def run(self, upto=None, between=None, read_at=None):
+        L = rt.lib()
+        h, pool, out = C.c_void_p(), C.c_void_p(), None
+        L.cudnnCreate(C.byref(h))
+        L.wrapDNNMemPoolInit(C.byref(pool), 1 << 22)
+        at = 0
+
+        def place(nbytes):
+            nonlocal at
+            p = C.c_void_p()
+            L.wrapDNNMemOffset(C.byref(p), pool, at, nbytes)
+            at += (nbytes + 31) // 32 * 32
+            return p.value
+        cur = place(self.x.nbytes)
+        L.wrapDNNMemcpy(cur, self.x.ctypes.data, self.x.nbytes, 1, None)
+        res = []
+        for i in range(self.n if upto is None else upto):
+            w, b = place(self.w[i].nbytes), place(self.b[i].nbytes)
+            L.wrapDNNMemcpy(w, self.w[i].ctypes.data, self.w[i].nbytes, 1, None)
+            L.wrapDNNMemcpy(b, self.b[i].ctypes.data, self.b[i].nbytes, 1, None)
+            y = place(self.x.nbytes)
+            L.DNNConvBiasActivFunc(h, cur, rt.dims(self.shape), w, rt.dims(self.w[i].shape), b,
+                                   rt.dims((1, self.shape[1], 1, 1)), None, 0, 0, rt.dims((1, 1)),
+                                   rt.dims((1, 1)), 1, y)
+            cur = y
+            if between is not None and i == between[0]:
+                between[1]()
+            if read_at == i:
+                mid = np.empty(self.shape, np.float32)
+                L.wrapDNNMemcpy(mid.ctypes.data, cur, mid.nbytes, 2, None)
+                res.append(mid)
+        out = np.empty(self.shape, np.float32)
+        L.wrapDNNMemcpy(out.ctypes.data, cur, out.nbytes, 2, None)
+        L.wrapDNNDealloc(pool)
+        L.cudnnDestroy(h)
+        return [out] + res
+
+
+def test_ways_out_of_the_middle(native_libs):
+    rt.set_math_mode(rt.MATH_BF16)
+    m = _HandModel()
+    (want,) = m.run()
+    for i in (3, 14, 19):
+        full = {}
+        for _ in range(PASSES):
+            (y,) = m.run()
+            assert np.array_equal(y, want)
+        # a wait, a question for the stream, a read of an intermediate, an early end
+        (y,) = m.run(between=(i, lambda: rt.synchronize()))
+        assert np.array_equal(y, want)
+        (y,) = m.run(between=(i, lambda: rt.lib().occamy_stream()))
+        assert np.array_equal(y, want)
+        y, mid = m.run(read_at=i)
+        assert np.array_equal(y, want)
+        (early,) = m.run(upto=i + 1)
+        assert np.array_equal(early, mid)
+        (y,) = m.run()
+        assert np.array_equal(y, want)
+    assert rt.last_error() == 0
