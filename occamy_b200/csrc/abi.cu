@@ -170,11 +170,22 @@ struct ConvJob {
   // device ranges still to be read: [0] input, [1] residual operand, [2] a bias that is read
   // from the caller's tensor (no resident copy exists)
   uintptr_t dep_lo[3] = {0, 0, 0}, dep_hi[3] = {0, 0, 0};
+  // a matrix product: `g` says N x K results (P = Q = 1), `a` how they are computed
+  bool product = false;
+  bool out16 = false;             // ... whose reader is another product: 16-bit result
   // folded (few-channel) form: what the fused convolution + pool kernel needs besides `a`
   const bf16 *w_stem = nullptr;   // filter in that kernel's layout, packed while the filter is live
 };
 
 ConvJob g_pending;  // convolution held back while later calls are folded into it
+const ConvJob *g_launching = nullptr;   // job whose output buffer is being looked for
+
+bool job_reads(const ConvJob &j, const void *home) {
+  return j.a.x == home || j.a.residual == home || j.dw_x == home;
+}
+bool home_held_hook(const void *home) {
+  return (g_pending.active && job_reads(g_pending, home)) || (g_launching && job_reads(*g_launching, home));
+}
 
 // A bias without a resident copy is read from the caller's tensor when the (possibly held-back)
 // kernel finally runs: until then that tensor must neither be freed nor overwritten.
@@ -238,8 +249,8 @@ bool prepare_dense(const float *x, const float *w, const float *bias, const Conv
   } else {
     const bf16 *xb = nullptr;
     if (is_act16(x, g.N, g.C, g.H, g.W)) {
-      xb = (const bf16 *)x;
-      if (Cp == g.C) {
+      xb = act16_ptr(x);
+      if (Cp == g.C && (const void *)xb == x) {
         job.dep_lo[0] = (uintptr_t)x;
         job.dep_hi[0] = (uintptr_t)x + (size_t)g.N * g.C * g.H * g.W * 2;
       }
@@ -283,9 +294,11 @@ bool prepare_depthwise(const float *x, const float *w, const float *bias, const 
   if (g.C % 8 != 0) return false;
   job.dep_lo[0] = job.dep_hi[0] = 0;
   if (is_act16(x, g.N, g.C, g.H, g.W)) {
-    job.dw_x = (const bf16 *)x;
-    job.dep_lo[0] = (uintptr_t)x;
-    job.dep_hi[0] = (uintptr_t)x + (size_t)g.N * g.C * g.H * g.W * 2;
+    job.dw_x = act16_ptr(x);
+    if ((const void *)job.dw_x == x) {
+      job.dep_lo[0] = (uintptr_t)x;
+      job.dep_hi[0] = (uintptr_t)x + (size_t)g.N * g.C * g.H * g.W * 2;
+    }
   } else {
     ensure_f32(x);
     bf16 *xc = (bf16 *)scratch_get(0, (size_t)g.N * g.C * g.H * g.W * 2);
@@ -313,54 +326,58 @@ bool ranges_overlap(uintptr_t alo, uintptr_t ahi, uintptr_t blo, uintptr_t bhi) 
 void launch_job(ConvJob &job) {
   Runtime &r = rt();
   const ConvGeom &g = job.g;
-  // A convolution that was held back may find its output placed over memory it still has
-  // to read (the planner reuses a tensor's bytes as soon as the recorded program no longer
-  // needs them).  The input then moves to scratch first; a residual operand may stay only
-  // if the output covers it exactly (each tile reads its residual before it is stored).
+  // A convolution that was held back may find its output placed over memory it still has to read
+  // (the planner reuses a tensor's bytes as soon as the recorded program no longer needs them).  The
+  // result then goes to a buffer of its own, which the tensor's record points to; a residual operand
+  // that the output covers exactly may stay (each tile reads its residual before it is stored).
+  // (Copying the input out of the way instead cost 1.5 to 40 us per such layer and broke the chain of
+  // overlapping launches: 17 copies in an unfused ResNet-50, 10 in MobileNetV2.)
   const uintptr_t olo = (uintptr_t)job.out;
-  const uintptr_t ohi = olo + (size_t)g.N * g.K * g.P * g.Q * 2;
-  if (ranges_overlap(olo, ohi, job.dep_lo[0], job.dep_hi[0])) {
-    const size_t bytes = job.dep_hi[0] - job.dep_lo[0];
-    void *tmp = scratch_get(4, bytes);
-    OCC_CUDA(cudaMemcpyAsync(tmp, (const void *)job.dep_lo[0], bytes, cudaMemcpyDeviceToDevice,
-                             r.stream));
-    if (job.depthwise) job.dw_x = (const bf16 *)tmp;
-    else job.a.x = (const bf16 *)tmp;
-    count(CNT_LAUNCHES);
+  const size_t obytes = (size_t)g.N * g.K * g.P * g.Q * 2;
+  const uintptr_t ohi = olo + obytes;
+  void *dst = job.out;
+  if (job.product && !job.out16) {   // fp32 result, at its own address
+    for (int k = 0; k < 3; k += 2) {
+      if (!ranges_overlap(olo, ohi + obytes, job.dep_lo[k], job.dep_hi[k])) continue;
+      const size_t bytes = job.dep_hi[k] - job.dep_lo[k];
+      void *tmp = scratch_get(k ? 7 : 4, bytes);
+      OCC_CUDA(cudaMemcpyAsync(tmp, (const void *)job.dep_lo[k], bytes, cudaMemcpyDeviceToDevice, r.stream));
+      if (k) job.a.bias = (const float *)tmp;
+      else job.a.x = (const bf16 *)tmp;
+      count(CNT_LAUNCHES);
+    }
+    job.a.act = g.act; job.a.lo = g.lo; job.a.hi = g.hi;
+    job.a.out_f32 = job.out;
+    job.a.ldo = g.K;
+    job.a.out_nchw = job.a.R * job.a.S > 1;   // [N][K][1][1]: the same rows
+    launch_tc_conv(job.a, r.stream);
+    mark_f32(job.out);
+    return;
   }
-  if (ranges_overlap(olo, ohi, job.dep_lo[1], job.dep_hi[1]) &&
-      !(olo == job.dep_lo[1] && ohi == job.dep_hi[1])) {
-    const size_t bytes = job.dep_hi[1] - job.dep_lo[1];
-    void *tmp = scratch_get(5, bytes);
-    OCC_CUDA(cudaMemcpyAsync(tmp, (const void *)job.dep_lo[1], bytes, cudaMemcpyDeviceToDevice,
-                             r.stream));
-    job.a.residual = (const bf16 *)tmp;
-    count(CNT_LAUNCHES);
-  }
-  if (ranges_overlap(olo, ohi, job.dep_lo[2], job.dep_hi[2])) {
-    const size_t bytes = job.dep_hi[2] - job.dep_lo[2];
-    void *tmp = scratch_get(7, bytes);
-    OCC_CUDA(cudaMemcpyAsync(tmp, (const void *)job.dep_lo[2], bytes, cudaMemcpyDeviceToDevice,
-                             r.stream));
-    if (job.depthwise) job.bias = (const float *)tmp;
-    else job.a.bias = (const float *)tmp;
-    count(CNT_LAUNCHES);
+  const bool in_place = olo == job.dep_lo[1] && ohi == job.dep_hi[1];
+  if (ranges_overlap(olo, ohi, job.dep_lo[0], job.dep_hi[0]) ||
+      (ranges_overlap(olo, ohi, job.dep_lo[1], job.dep_hi[1]) && !in_place) ||
+      ranges_overlap(olo, ohi, job.dep_lo[2], job.dep_hi[2])) {
+    g_launching = &job;
+    dst = home_acquire(obytes);
+    g_launching = nullptr;
+    if (!dst) return;
   }
   if (job.depthwise) {
-    launch_depthwise_bf16(job.dw_x, job.dw_w, job.bias, (bf16 *)job.out, g, mode_f16(), r.stream);
+    launch_depthwise_bf16(job.dw_x, job.dw_w, job.bias, (bf16 *)dst, g, mode_f16(), r.stream);
   } else {
-    job.a.y = (bf16 *)job.out;
+    job.a.y = (bf16 *)dst;
     job.a.act = g.act; job.a.lo = g.lo; job.a.hi = g.hi;
     launch_tc_conv(job.a, r.stream);
   }
-  mark_act16(job.out, g.N, g.K, g.P, g.Q);
+  mark_act16(job.out, g.N, g.K, g.P, g.Q, dst == job.out ? nullptr : dst);
 }
 
 // Executes the held-back convolution as far as it has been built up.
 void flush_pending() {
   if (!g_pending.active) return;
   g_pending.active = false;
-  if (g_pending.absorbed) trace_count_chain();
+  if (g_pending.absorbed && !g_pending.product) trace_count_chain();   // convolution chains
   launch_job(g_pending);
 }
 
@@ -393,11 +410,13 @@ void before_write_hook(const void *p, size_t bytes) { pending_guard_range(p, byt
 
 Role step(Entry &e, bool passive) {
   rt().before_write = before_write_hook;
+  rt().home_held = home_held_hook;
   if (graph_covers(e)) return R_SKIP;
   bool deviated = false;
   const Role role = trace_step(e, &deviated);
   if (deviated) {
     graph_stop_capture();
+    g_pending.out16 = false;   // who reads it is not known any more
     flush_pending();
     // Tensors that fusion skipped earlier in this inference stay unwritten.  The recorded
     // program had no reader for them; should this (different) program read one, that read
@@ -770,23 +789,22 @@ cudaError_t wrapDNNMemcpy(void *dst, const void *src, size_t count_, int kind,
       // convert into scratch instead of in place: the tensor keeps its fast format
       const size_t elems = (size_t)(rec->n * rec->c * rec->h * rec->w);
       float *tmp = (float *)scratch_get(2, elems * 4);
-      launch_nhwc_bf16_to_nchw_f32((const bf16 *)src, tmp, (int)rec->n, (int)rec->c, (int)rec->h,
+      launch_nhwc_bf16_to_nchw_f32(act16_ptr(src), tmp, (int)rec->n, (int)rec->c, (int)rec->h,
                                    (int)rec->w, rec->fmt == FMT_F16_NHWC, r.stream);
       count(CNT_MATERIALIZE);
       from = tmp;
     } else {
       ensure_f32(src);
     }
-    err = cudaMemcpyAsync(dst, from, count_, cudaMemcpyDeviceToHost, r.stream);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(r.stream);
-    // surface a kernel-side watchdog report, if any
-    if (r.dev_err && r.host_err) {
-      cudaMemcpy(r.host_err, r.dev_err, sizeof(int), cudaMemcpyDeviceToHost);
-      if (*r.host_err) {
-        set_error(*r.host_err, "kernel watchdog");
-        cudaMemset(r.dev_err, 0, sizeof(int));
-      }
+    // Small results go through a pinned buffer: one transfer the driver need not stage.
+    if (count_ <= STAGE_BYTES && !r.host_stage) {
+      if (cudaMallocHost(&r.host_stage, STAGE_BYTES) != cudaSuccess) cudaGetLastError();
     }
+    void *to = count_ <= STAGE_BYTES && r.host_stage ? r.host_stage : dst;
+    err = cudaMemcpyAsync(to, from, count_, cudaMemcpyDeviceToHost, r.stream);
+    if (err == cudaSuccess) err = cudaStreamSynchronize(r.stream);
+    if (err == cudaSuccess && to != dst) memcpy(dst, to, count_);
+    poll_watchdog();
   } else {
     Entry e = trace_entry(S_OPAQUE);
     step(e, false);
@@ -928,7 +946,7 @@ float *DNNActiveFunc(cudnnContext *, float *x, int64_t dimX[4], int32_t mode, fl
     flush_pending();
   }
   if (is_act16(x, dimX[0], dimX[1], dimX[2], dimX[3])) {
-    launch_add_act_bf16((const bf16 *)x, nullptr, nullptr, (int)dimX[1], (bf16 *)y, n, act, 0.f,
+    launch_add_act_bf16(act16_ptr(x), nullptr, nullptr, (int)dimX[1], (bf16 *)y, n, act, 0.f,
                         0.f, mode_f16(), r.stream);
     mark_act16(y, dimX[0], dimX[1], dimX[2], dimX[3]);
     return y;
@@ -969,7 +987,7 @@ float *CUDAClipFunc(float *x, float *y, int64_t *dimOut, float lo, float hi, int
     flush_pending();
   }
   if (rank == 4 && is_act16(x, dimOut[0], dimOut[1], dimOut[2], dimOut[3])) {
-    launch_add_act_bf16((const bf16 *)x, nullptr, nullptr, (int)dimOut[1], (bf16 *)y, n, ACT_CLIP,
+    launch_add_act_bf16(act16_ptr(x), nullptr, nullptr, (int)dimOut[1], (bf16 *)y, n, ACT_CLIP,
                         lo, hi, mode_f16(), r.stream);
     mark_act16(y, dimOut[0], dimOut[1], dimOut[2], dimOut[3]);
     return y;
@@ -1012,6 +1030,7 @@ float *DNNTensorOpFunc(cudnnContext *, int64_t opMode, float *A, int64_t *dimA, 
   e.in_bytes[1] = rank_ok ? prod(dB, rankA) * 4 : 0;
   for (int i = 0; i < 4 && i < rankA; ++i) e.dims[i] = dimA[i];
   if (opMode == 0 && bias == 1.0f) e.kind = bias_shape ? CK_BIAS_ADD : (same ? CK_SAME_ADD : CK_NONE);
+  if (opMode == 0 && bias == 1.0f && rank_ok && rankA == 2 && dB[0] == 1 && dB[1] == dimA[1]) e.kind = CK_ROW_BIAS;
   const Role role = step(e, false);
   if (role == R_SKIP) return out;
 
@@ -1021,8 +1040,9 @@ float *DNNTensorOpFunc(cudnnContext *, int64_t opMode, float *A, int64_t *dimA, 
   }
   if (role == R_ABSORB && g_pending.active) {
     const ConvGeom &g = g_pending.g;
-    const bool dims_ok = dimA[0] == g.N && dimA[1] == g.K && dimA[2] == g.P && dimA[3] == g.Q;
-    if (e.kind == CK_BIAS_ADD && dims_ok && A == g_pending.out && !g_pending.bias_set &&
+    const bool dims_ok = dimA[0] == g.N && dimA[1] == g.K &&
+                         (rankA == 2 ? g_pending.product : dimA[2] == g.P && dimA[3] == g.Q);
+    if ((e.kind == CK_BIAS_ADD || e.kind == CK_ROW_BIAS) && dims_ok && A == g_pending.out && !g_pending.bias_set &&
         !g_pending.res_set && !g_pending.act_set) {
       const float *bd = resident_f32(B, (size_t)g.K * 4);
       if (g_pending.depthwise) g_pending.bias = bd;
@@ -1033,14 +1053,16 @@ float *DNNTensorOpFunc(cudnnContext *, int64_t opMode, float *A, int64_t *dimA, 
       pending_retarget(out);
       return out;
     }
-    if (e.kind == CK_SAME_ADD && dims_ok && !g_pending.depthwise && !g_pending.res_set &&
+    if (e.kind == CK_SAME_ADD && dims_ok && !g_pending.depthwise && !g_pending.product && !g_pending.res_set &&
         !g_pending.act_set && ((A == g_pending.out) != (B == g_pending.out))) {
       const float *other = A == g_pending.out ? B : A;
       if (is_act16(other, g.N, g.K, g.P, g.Q)) {
-        g_pending.a.residual = (const bf16 *)other;
+        g_pending.a.residual = act16_ptr(other);
         g_pending.res_set = true;
-        g_pending.dep_lo[1] = (uintptr_t)other;
-        g_pending.dep_hi[1] = (uintptr_t)other + (size_t)g.N * g.K * g.P * g.Q * 2;
+        if ((const void *)g_pending.a.residual == other) {
+          g_pending.dep_lo[1] = (uintptr_t)other;
+          g_pending.dep_hi[1] = (uintptr_t)other + (size_t)g.N * g.K * g.P * g.Q * 2;
+        }
         pending_retarget(out);
         return out;
       }
@@ -1051,7 +1073,7 @@ float *DNNTensorOpFunc(cudnnContext *, int64_t opMode, float *A, int64_t *dimA, 
       is_act16(A, dimA[0], dimA[1], dimA[2], dimA[3])) {
     const int64_t n = numel4(dimA);
     if (same && is_act16(B, dimA[0], dimA[1], dimA[2], dimA[3])) {
-      launch_add_act_bf16((const bf16 *)A, (const bf16 *)B, nullptr, (int)dimA[1], (bf16 *)out, n,
+      launch_add_act_bf16(act16_ptr(A), act16_ptr(B), nullptr, (int)dimA[1], (bf16 *)out, n,
                           ACT_IDENTITY, 0.f, 0.f, mode_f16(), r.stream);
       mark_act16(out, dimA[0], dimA[1], dimA[2], dimA[3]);
       return out;
@@ -1059,7 +1081,7 @@ float *DNNTensorOpFunc(cudnnContext *, int64_t opMode, float *A, int64_t *dimA, 
     if (bias_shape) {
       // a bias vector uploaded from host memory is kept resident like the filters are
       const float *bd = resident_f32(B, (size_t)dimA[1] * 4);
-      launch_add_act_bf16((const bf16 *)A, nullptr, bd, (int)dimA[1], (bf16 *)out, n, ACT_IDENTITY,
+      launch_add_act_bf16(act16_ptr(A), nullptr, bd, (int)dimA[1], (bf16 *)out, n, ACT_IDENTITY,
                           0.f, 0.f, mode_f16(), r.stream);
       mark_act16(out, dimA[0], dimA[1], dimA[2], dimA[3]);
       return out;
@@ -1098,6 +1120,7 @@ static float *pool_common(int sym, float *x, int64_t *dI, float *y, int64_t *dO,
     e.kind = CK_POOL_3S2;
   const Role role = step(e, false);
   if (role == R_SKIP) return y;
+  const bool for_matmul = (trace_last_flags() & RF_FOR_MATMUL) != 0;
   if (role == R_ABSORB && g_pending.active) {
     // the held-back stem convolution and this pool run as one kernel
     ConvJob &j = g_pending;
@@ -1132,9 +1155,11 @@ static float *pool_common(int sym, float *x, int64_t *dI, float *y, int64_t *dO,
     flush_pending();
   }
   if (r.mode != MATH_FP32 && C % 8 == 0 && is_act16(x, N, C, H, W)) {
-    launch_pool_bf16((const bf16 *)x, (bf16 *)y, N, C, H, W, P, Q, (int)kernel[0], (int)kernel[1],
+    // read by a Flatten and the product behind it: where the Flatten need not move it
+    void *home = for_matmul ? home_acquire((size_t)N * C * P * Q * 2) : nullptr;
+    launch_pool_bf16(act16_ptr(x), (bf16 *)(home ? home : y), N, C, H, W, P, Q, (int)kernel[0], (int)kernel[1],
                      ph, pw, (int)stride[0], (int)stride[1], avg, mode_f16(), r.stream);
-    mark_act16(y, N, C, P, Q);
+    mark_act16(y, N, C, P, Q, home);
     return y;
   }
   ensure_f32(x);
@@ -1169,6 +1194,7 @@ float *DNNReduceFunc(cudnnContext *, int32_t rank, float *x, int64_t *dimIn, flo
   e.out_bytes = rank <= 8 && rank > 0 ? prod(dimOut, rank) * 4 : 0;
   e.in_bytes[0] = rank <= 8 && rank > 0 ? prod(dimIn, rank) * 4 : 0;
   if (step(e, false) == R_SKIP) return y;
+  const bool for_matmul = (trace_last_flags() & RF_FOR_MATMUL) != 0;
   if (mode != 5 || rank > 8) {
     set_error(995, "reduce: only mode 5 (mean) is implemented");
     return y;
@@ -1176,9 +1202,11 @@ float *DNNReduceFunc(cudnnContext *, int32_t rank, float *x, int64_t *dimIn, flo
   if (rank == 4 && dimOut[2] == 1 && dimOut[3] == 1 && dimOut[0] == dimIn[0] &&
       dimOut[1] == dimIn[1] && dimIn[1] % 8 == 0 &&
       is_act16(x, dimIn[0], dimIn[1], dimIn[2], dimIn[3])) {
-    launch_gap_bf16((const bf16 *)x, y, (int)dimIn[0], (int)(dimIn[2] * dimIn[3]), (int)dimIn[1],
+    void *home = for_matmul ? home_acquire((size_t)(dimIn[0] * dimIn[1]) * 2) : nullptr;
+    launch_gap_bf16(act16_ptr(x), y, (bf16 *)home, (int)dimIn[0], (int)(dimIn[2] * dimIn[3]), (int)dimIn[1],
                     mode_f16(), r.stream);
-    mark_f32(y);
+    if (home) mark_act16(y, dimIn[0], dimIn[1], 1, 1, home);
+    else mark_f32(y);
     return y;
   }
   ensure_f32(x);
@@ -1207,31 +1235,68 @@ float *CUBLASMatmul2dFunc(int64_t /*rank*/, float *A, int64_t dimA[2], float *B,
   e.out = (uintptr_t)out; e.out_bytes = (int64_t)M * N * 4;
   e.in_bytes[0] = dimA[0] * dimA[1] * 4; e.in_bytes[1] = dimB[0] * dimB[1] * 4;
   e.in_bytes[2] = e.out_bytes;
-  if (step(e, false) == R_SKIP) return out;
-  if (r.log) fprintf(stderr, "[occamy] matmul2d M%d N%d K%d tA%d tB%d\n", M, N, K, (int)transA, (int)transB);
+  e.dims[0] = M; e.dims[1] = N;
   const bool out_zero = is_zero(out);
-  if (r.mode != MATH_FP32 && !transA && transB && alpha == 1.0f && (beta == 0.0f || out_zero) &&
-      K % 16 == 0 && M > 0) {
-    TcConvArgs a;
+  e.fusable = r.mode != MATH_FP32 && !transA && transB && alpha == 1.0f && (beta == 0.0f || out_zero) &&
+              K % 16 == 0 && M > 0;
+  const Role role = step(e, false);
+  if (role == R_SKIP) return out;
+  if (r.log) fprintf(stderr, "[occamy] matmul2d M%d N%d K%d tA%d tB%d\n", M, N, K, (int)transA, (int)transB);
+  if (e.fusable) {
+    ConvJob job;
+    TcConvArgs &a = job.a;
     memset(&a, 0, sizeof(a));
     a.N = 1; a.H = 1; a.W = M; a.Cf = K; a.K = N; a.P = 1; a.Q = M; a.R = 1; a.S = 1;
     a.stride_h = a.stride_w = 1;
     a.act = ACT_IDENTITY;
-    a.out_f32 = out;
-    a.ldo = N;
     a.f16 = mode_f16() ? 1 : 0;
+    int c = K;   // channels of A where it is an image that a Flatten passed on
+    uintptr_t base = 0;
+    const TensorRec *rec = reg_find(A, &base);
+    const bool image = rec && base == (uintptr_t)A && is_act16(A, rec->n, rec->c, rec->h, rec->w) && rec->n == M &&
+                       rec->c * rec->h * rec->w == K && rec->h * rec->w <= 64 && rec->c % 16 == 0;
+    if (image && rec->h * rec->w > 1) {
+      // NHWC rows against [N][c][h][w] filters: a convolution whose filter covers the whole image
+      c = (int)rec->c;
+      a.N = M; a.H = (int)rec->h; a.W = (int)rec->w; a.Cf = c; a.P = a.Q = 1; a.R = a.H; a.S = a.W;
+    }
+    a.out_f32 = out;
+    a.out_nchw = a.R * a.S > 1;
+    a.ldo = N;
     a.x = (const bf16 *)16;
     a.w = (const bf16 *)16;
     if (tc_conv_supported(a)) {
-      ensure_f32(A);
-      bf16 *ab = (bf16 *)scratch_get(0, (size_t)M * K * 2);
-      const bf16 *wb = (const bf16 *)packed_weights(B, PACK_KRSC, (size_t)N * K * 2, N, K, 1, 1, 0, 0);
-      if (ab && wb) {
+      if (image) {
+        a.x = act16_ptr(A);
+        if ((const void *)a.x == A) {
+          job.dep_lo[0] = (uintptr_t)A;
+          job.dep_hi[0] = (uintptr_t)A + (size_t)M * K * 2;
+        }
+      } else {
+        ensure_f32(A);
+        bf16 *ab = (bf16 *)scratch_get(0, (size_t)M * K * 2);
         launch_f32_to_bf16(A, ab, (int64_t)M * K, mode_f16(), r.stream);
         a.x = ab;
-        a.w = wb;
-        launch_tc_conv(a, r.stream);
-        mark_f32(out);
+      }
+      a.w = (const bf16 *)packed_weights(B, PACK_KRSC, (size_t)N * K * 2, N, c, a.R, a.S, 0, c);
+      if (a.x && a.w) {
+        a.consts_ready = g_pack_was_resident ? 1 : 0;
+        a.out_f32 = nullptr;
+        a.out_nchw = 0;
+        ConvGeom &g = job.g;
+        memset(&g, 0, sizeof(g));
+        g.N = M; g.K = N; g.P = g.Q = 1; g.C = c; g.H = a.H; g.W = a.W; g.R = a.R; g.S = a.S;
+        g.groups = g.stride_h = g.stride_w = 1;
+        g.act = ACT_IDENTITY;
+        job.product = true;
+        job.out16 = (trace_last_flags() & RF_FOR_MATMUL) && N % 16 == 0;
+        job.out = out;
+        if (role == R_DEFER) {
+          g_pending = job;
+          g_pending.active = true;
+          return out;
+        }
+        launch_job(job);
         return out;
       }
     }
@@ -1306,6 +1371,13 @@ static float *copy_common(int sym, float *x, int64_t *dimIn, int64_t rank, float
   te_ptr(e, x); te_ptr(e, y); te_dims(e, dimIn, (int)rank);
   e.in[0] = (uintptr_t)x; e.in_bytes[0] = n * 4; e.out = (uintptr_t)y; e.out_bytes = n * 4;
   if (step(e, false) == R_SKIP) return y;
+  // A tensor in a buffer of its own goes by its record: the same values in the same logical order.
+  if (sym == S_FLATTEN && rank == 4 && is_act16(x, dimIn[0], dimIn[1], dimIn[2], dimIn[3]) &&
+      (const void *)act16_ptr(x) != x) {
+    pending_guard_range(y, (size_t)n * 4, true);
+    mark_act16(y, dimIn[0], dimIn[1], dimIn[2], dimIn[3], act16_ptr(x));
+    return y;
+  }
   ensure_f32(x);
   OCC_CUDA(cudaMemcpyAsync(y, x, (size_t)n * 4, cudaMemcpyDeviceToDevice, r.stream));
   mark_f32(y);
@@ -1399,13 +1471,7 @@ int occamy_synchronize(void) {
   flush_pending();
   cudaError_t e = cudaStreamSynchronize(r.stream);
   if (e != cudaSuccess) set_error((int)e, "synchronize");
-  if (r.dev_err && r.host_err) {
-    cudaMemcpy(r.host_err, r.dev_err, sizeof(int), cudaMemcpyDeviceToHost);
-    if (*r.host_err) {
-      set_error(*r.host_err, "kernel watchdog");
-      cudaMemset(r.dev_err, 0, sizeof(int));
-    }
-  }
+  poll_watchdog();
   const int na = noalloc_poll_error(true);
   if (na > 0) set_error(na, "kernel watchdog (occamy_conv_bias_act_noalloc)");
   return (int)e;
@@ -1481,6 +1547,16 @@ void occamy_clear_weight_cache(void) {
     if (kv.second.dev) cudaFree(kv.second.dev);
   r.wcache.clear();
   r.resident.clear();
+  for (size_t i = 0; i < r.homes.size();) {   // buffers no tensor is in
+    bool used = false;
+    for (const auto &kv : r.recs) used = used || kv.second.home == r.homes[i].ptr;
+    if (used) {
+      ++i;
+      continue;
+    }
+    cudaFree(r.homes[i].ptr);
+    r.homes.erase(r.homes.begin() + i);
+  }
 }
 
 }  // extern "C"

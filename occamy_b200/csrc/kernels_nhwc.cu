@@ -407,7 +407,8 @@ void launch_pool_bf16(const bf16 *x, bf16 *y, int N, int C, int H, int W, int P,
 constexpr int GAP_ROWS = 16;
 template <bool F16>
 __global__ void __launch_bounds__(8 * GAP_ROWS) gap_bf16_kernel(const bf16x8 *__restrict__ x,
-                                                               float *__restrict__ y, int HW, int C8) {
+                                                               float *__restrict__ y, uint16_t *__restrict__ y16,
+                                                               int HW, int C8) {
   __shared__ float part[GAP_ROWS][8][8];
   const int lane8 = threadIdx.x & 7, prow = threadIdx.x >> 3;
   const int c8 = blockIdx.x * 8 + lane8;
@@ -431,16 +432,20 @@ __global__ void __launch_bounds__(8 * GAP_ROWS) gap_bf16_kernel(const bf16x8 *__
 #pragma unroll
     for (int r = 0; r < GAP_ROWS; ++r) s += part[r][l][k];
     const int c = (blockIdx.x * 8 + l) * 8 + k;
-    if (blockIdx.x * 8 + l < C8) y[n * C8 * 8 + c] = s * (1.0f / (float)HW);
+    if (blockIdx.x * 8 + l < C8) {
+      const float mean = s * (1.0f / (float)HW);
+      if (y16) y16[n * C8 * 8 + c] = f32_to_elem<F16>(mean);
+      else y[n * C8 * 8 + c] = mean;
+    }
   }
 }
 
-void launch_gap_bf16(const bf16 *x, float *y, int N, int HW, int C, bool f16, cudaStream_t s) {
+void launch_gap_bf16(const bf16 *x, float *y, bf16 *y16, int N, int HW, int C, bool f16, cudaStream_t s) {
   if ((int64_t)N * C == 0) return;
   const int C8 = C / 8;
   const dim3 grid((unsigned)((C8 + 7) / 8), (unsigned)N);
-  if (f16) gap_bf16_kernel<true><<<grid, 8 * GAP_ROWS, 0, s>>>((const bf16x8 *)x, y, HW, C8);
-  else gap_bf16_kernel<false><<<grid, 8 * GAP_ROWS, 0, s>>>((const bf16x8 *)x, y, HW, C8);
+  if (f16) gap_bf16_kernel<true><<<grid, 8 * GAP_ROWS, 0, s>>>((const bf16x8 *)x, y, (uint16_t *)y16, HW, C8);
+  else gap_bf16_kernel<false><<<grid, 8 * GAP_ROWS, 0, s>>>((const bf16x8 *)x, y, (uint16_t *)y16, HW, C8);
   count(CNT_LAUNCHES);
 }
 

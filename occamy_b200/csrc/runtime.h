@@ -35,6 +35,9 @@ struct TensorRec {
   size_t bytes = 0;  // extent of the allocation handed to the caller
   Fmt fmt = FMT_F32;
   int64_t n = 0, c = 0, h = 0, w = 0;  // logical NCHW dims of a 16-bit NHWC tensor
+  // Where a 16-bit tensor's bytes are when not at the tensor's own address (home_acquire()): its
+  // address was still to be read by the kernel that wrote it, or the tensor outlives its address.
+  const void *home = nullptr;
   const void *host_src = nullptr;      // source of the last host->device upload, if any
   size_t host_bytes = 0;
   uint64_t host_hash = 0;
@@ -86,13 +89,21 @@ struct Runtime {
   std::unordered_map<const void *, std::pair<size_t, uint64_t>> resident;
   void *scratch[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   size_t scratch_bytes[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  int *dev_err = nullptr;   // device word the kernels' bounded waits report into
-  int *host_err = nullptr;  // pinned mirror
+  int *dev_err = nullptr;   // word the kernels' bounded waits report into, as the device sees it
+  int *host_err = nullptr;  // the same word (mapped host memory)
+  void *host_stage = nullptr;   // pinned, STAGE_BYTES: small results on their way to pageable memory
   bool log = false;
   bool cache_weights = true;
   // called before the runtime itself writes into a caller-owned range (lazy zero fill,
   // deferred upload, layout conversion), so that a held-back kernel can read it first
   void (*before_write)(const void *p, size_t bytes) = nullptr;
+  // whether a held-back kernel is still to read the buffer at `home`
+  bool (*home_held)(const void *home) = nullptr;
+  struct Home {
+    void *ptr;
+    size_t bytes;
+  };
+  std::vector<Home> homes;
   // optional CUDA-event pair around every tensor-core launch (occamy_profile_begin/end)
   bool profiling = false;
   int prof_count = 0;
@@ -111,6 +122,10 @@ void set_error(int code, const char *where);
     if (e_ != cudaSuccess) ::occ::set_error((int)e_, #call);  \
   } while (0)
 
+constexpr size_t STAGE_BYTES = 256 * 1024;
+// After a wait for the stream: report a kernel whose bounded wait ran out, if any.
+void poll_watchdog();
+
 // ---- registry --------------------------------------------------------------
 // Record that [p, p+bytes) now is a fresh tensor; drops records it overlaps.
 void reg_new(void *p, size_t bytes, Fmt fmt);
@@ -123,9 +138,15 @@ void ensure_f32(const void *p);
 // the element type of the CURRENT mode (a tensor left behind in the other 16-bit type is
 // converted back to fp32 by its next reader, like any other foreign format).
 bool is_act16(const void *p, int64_t n, int64_t c, int64_t h, int64_t w);
-// Mark p as fully overwritten by an fp32 kernel / by a 16-bit NHWC kernel of the current mode.
+// Mark p as fully overwritten by an fp32 kernel / by a 16-bit NHWC kernel of the current mode
+// (`home`: into that buffer instead of p's own bytes).
 void mark_f32(void *p);
-void mark_act16(void *p, int64_t n, int64_t c, int64_t h, int64_t w);
+void mark_act16(void *p, int64_t n, int64_t c, int64_t h, int64_t w, const void *home = nullptr);
+// The bytes of a tensor that is_act16().
+const __nv_bfloat16 *act16_ptr(const void *p);
+// A buffer for a 16-bit tensor that cannot be written at its own address; in use as long as a tensor
+// record (or a kernel that is held back, see home_held) refers to it.  A handful are kept.
+void *home_acquire(size_t bytes);
 // The current mode stores fp16 (else bf16) in its 16-bit tensors.
 bool mode_f16();
 // A tensor that reads as zero and has not been written since it was handed out.

@@ -24,6 +24,7 @@ struct TraceState {
   size_t pool_bytes = 0;
   uintptr_t last_pool_base = 0;   // the pool of this inference, also after it was given back
   size_t last_pool_bytes = 0;
+  uint8_t last_flags = 0;
   int elided = 0;
   int64_t fused_chains = 0;
 };
@@ -68,12 +69,70 @@ bool same_dims(const Entry &a, const Entry &b) {
          a.dims[3] == b.dims[3];
 }
 
+// True when what reads [p, p+bytes) from entry `from` on, until the range is handed out again or
+// freed, are matrix products (as their first operand) and Flattens whose result only such read.
+bool only_matmuls_read(const std::vector<Entry> &rec, uintptr_t p, int64_t bytes, size_t from) {
+  bool any = false;
+  for (size_t t = from; t < rec.size(); ++t) {
+    const Entry &e = rec[t];
+    for (int k = 0; k < 3; ++k) {
+      if (!e.in[k] || !overlaps(e.in[k], e.in_bytes[k] > 0 ? e.in_bytes[k] : 1, p, bytes)) continue;
+      const bool product = e.sym == S_MATMUL && k == 0 && e.in[0] == p && e.fusable;
+      const bool flat = e.sym == S_FLATTEN && e.in[0] == p && only_matmuls_read(rec, e.out, e.out_bytes, t + 1);
+      if (!product && !flat) return false;
+      any = true;
+    }
+    if ((e.sym == S_MEMOFFSET || e.sym == S_MALLOC) && overlaps(e.out, e.out_bytes, p, bytes)) return any;
+    if ((e.sym == S_DEALLOC && e.out == p) || e.sym == S_POOLFREE) return any;
+    if (e.sym == S_OPAQUE) return false;
+    if (e.sym != S_MEMOFFSET && e.sym != S_MALLOC && e.out && overlaps(e.out, e.out_bytes, p, bytes)) return false;
+  }
+  return false;
+}
+
 // Marks the chains of a finished inference: R_DEFER on the convolution, R_ABSORB on the
 // calls folded into it.
 void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles) {
   roles.assign(rec.size(), R_EAGER);
   for (size_t i = 0; i < rec.size(); ++i) {
     const Entry &c = rec[i];
+    if ((c.sym == S_REDUCE || c.sym == S_AVGPOOL || c.sym == S_MAXPOOL) && c.out != c.in[0] &&
+        only_matmuls_read(rec, c.out, c.out_bytes, i + 1))
+      roles[i] |= RF_FOR_MATMUL;
+    if (c.sym == S_MATMUL && c.fusable) {
+      // product -> bias row (in place or not) -> ReLU
+      bool bias_set = false, act_set = false;
+      uintptr_t cur = c.out;
+      size_t last = i;
+      std::vector<size_t> members;
+      for (size_t j = i + 1; j < rec.size() && !act_set; ++j) {
+        const Entry &f = rec[j];
+        if (is_passive(f.sym)) {
+          if ((f.sym == S_MEMOFFSET || f.sym == S_MALLOC) && overlaps(f.out, f.out_bytes, cur, c.out_bytes)) break;
+          if (f.sym == S_DEALLOC && f.out == cur) break;
+          continue;
+        }
+        const bool shape = f.dims[0] == c.dims[0] && f.dims[1] == c.dims[1] && f.out_bytes == c.out_bytes;
+        const bool take = shape && f.in[0] == cur &&
+                          ((f.sym == S_TENSOR_OP && f.kind == CK_ROW_BIAS && !bias_set) ||
+                           (f.sym == S_ACTIVE && f.kind == CK_RELU));
+        if (!take) break;
+        if (f.out != cur && !dies_unread(rec, cur, c.out_bytes, j + 1)) break;
+        if (f.sym == S_TENSOR_OP) bias_set = true;
+        else act_set = true;
+        members.push_back(j);
+        last = j;
+        cur = f.out;
+      }
+      if (!members.empty()) {
+        roles[i] |= R_DEFER;
+        for (size_t m : members) roles[m] |= R_ABSORB;
+      }
+      if (only_matmuls_read(rec, cur, c.out_bytes, last + 1)) {
+        roles[i] |= RF_FOR_MATMUL;   // on the product, for the chain as a whole
+      }
+      continue;
+    }
     if ((c.sym != S_CONV && c.sym != S_CONV_BIAS_ACT) || !c.fusable) continue;
     bool bias_set = c.sym == S_CONV_BIAS_ACT;
     bool act_set = c.sym == S_CONV_BIAS_ACT && c.kind != 5;
@@ -128,8 +187,8 @@ void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles) {
       }
     }
     if (members.empty()) continue;
-    roles[i] = R_DEFER;
-    for (size_t m : members) roles[m] = R_ABSORB;
+    roles[i] |= R_DEFER;
+    for (size_t m : members) roles[m] |= R_ABSORB;
   }
 }
 
@@ -205,6 +264,7 @@ void te_dims(Entry &e, const int64_t *d, int n) {
 Role trace_step(Entry &e, bool *deviated) {
   *deviated = false;
   TraceState &ts = g_ts;
+  ts.last_flags = 0;
   if (!trace_enabled() || !ts.in_inference) return R_EAGER;
   if (trace_index() >= MAX_ENTRIES) {  // not a compiled model's call pattern: stop tracing
     ts.in_inference = false;
@@ -213,6 +273,7 @@ Role trace_step(Entry &e, bool *deviated) {
     return R_EAGER;
   }
   const size_t index = trace_index();
+  ts.last_flags = 0;
   Role role = R_EAGER;
   if (!ts.cands.empty()) {
     size_t keep = 0;
@@ -224,9 +285,14 @@ Role trace_step(Entry &e, bool *deviated) {
     if (keep) {
       // recorded programs that share this prefix must agree on the call's role (two models
       // with the same first layers may continue differently); otherwise it runs as it stands
-      role = (Role)ts.programs[ts.cands[0]].roles[index];
+      const uint8_t r = ts.programs[ts.cands[0]].roles[index];
+      role = (Role)(r & 0x0F);
+      ts.last_flags = r & 0xF0;
       for (size_t k = 1; k < keep; ++k)
-        if ((Role)ts.programs[ts.cands[k]].roles[index] != role) role = R_EAGER;
+        if (ts.programs[ts.cands[k]].roles[index] != r) {
+          role = R_EAGER;
+          ts.last_flags = 0;
+        }
       ts.matched_so_far = true;
     } else {
       *deviated = ts.matched_so_far;
@@ -277,6 +343,7 @@ void trace_end() {
 }
 
 // ---- prefixes made in one go (graph_replay.cu) ------------------------------------
+uint8_t trace_last_flags() { return g_ts.last_flags; }
 bool trace_active() { return trace_enabled() && g_ts.in_inference; }
 size_t trace_index() { return g_ts.prefix_len + g_ts.rec.size(); }
 TraceProgram *trace_candidate() {

@@ -5,6 +5,7 @@
 // calls between cudnnCreate and cudnnDestroy (the compiled function's prologue and
 // epilogue).  When an inference ends it looks for chains
 //     convolution -> [+ bias [1,K,1,1]] -> [+ same-shape tensor] -> [ReLU | Clip]
+//     matrix product -> [+ bias row] -> [ReLU]
 // (and, for a few-channel stem convolution, a 3x3 / stride 2 max pool behind it)
 // whose intermediate results nobody else reads before their memory is handed out again,
 // and marks them.  The next time the same call sequence comes by, the convolution of such
@@ -31,7 +32,8 @@ enum Role { R_EAGER = 0, R_DEFER = 1, R_ABSORB = 2, R_SKIP = 3 };
 // kind of a tensor-op / activation entry, as far as chains care
 enum ChainKind {
   CK_NONE = 0, CK_BIAS_ADD = 1, CK_SAME_ADD = 2, CK_RELU = 3, CK_CLIP = 4,
-  CK_POOL_3S2 = 5   // max pool 3x3, stride 2, pad 1
+  CK_POOL_3S2 = 5,  // max pool 3x3, stride 2, pad 1
+  CK_ROW_BIAS = 6   // rank 2: the same row added to every row
 };
 
 // The call's own arguments, enough to make it again (graph_replay.cu, run_again).
@@ -50,7 +52,7 @@ struct Entry {
   int64_t out_bytes = 0;   // fp32 extent of `out` (range size for the memory calls)
   int64_t dims[4] = {0, 0, 0, 0};
   int kind = CK_NONE;      // ChainKind, or the activation mode of a fused convolution
-  bool fusable = false;    // convolution that the bf16 path takes (may head a chain)
+  bool fusable = false;    // convolution or product that the 16-bit path takes (may head a chain)
   bool depthwise = false;
   bool poolable = false;   // convolution whose kernel can take a following CK_POOL_3S2 along
   bool uploaded = false;   // S_H2D: bytes crossed to the device (not a constant that is already there)
@@ -72,9 +74,12 @@ void te_ptr_or_elsewhere(Entry &e, const void *p);
 
 // A recorded inference: the calls between cudnnCreate and cudnnDestroy and the role of each.
 struct GraphPlan;
+// flag beside a call's role: whatever reads its result is a matrix product (possibly behind a Flatten),
+// so the result may be kept in the 16-bit form that product takes
+constexpr uint8_t RF_FOR_MATMUL = 0x10;
 struct TraceProgram {
   std::vector<uint64_t> sigs;
-  std::vector<uint8_t> roles;
+  std::vector<uint8_t> roles;   // Role | RF_*
   std::vector<Entry> entries;
   uintptr_t pool_base = 0;     // pool the entries' pointers refer to
   size_t pool_bytes = 0;
@@ -86,6 +91,7 @@ struct TraceProgram {
 // program although earlier calls did.
 Role trace_step(Entry &e, bool *deviated);
 
+uint8_t trace_last_flags();         // RF_* of the call trace_step() was last given
 void trace_begin();                 // cudnnCreate
 void trace_end();                   // cudnnDestroy: analyse and store if the sequence is new
 // ---- for graph_replay.cu ----
