@@ -309,7 +309,10 @@ bool prepare_depthwise(const float *x, const float *w, const float *bias, const 
   job.dw_w = (const float *)packed_weights(w, PACK_DW, (size_t)g.R * g.S * g.C * 4, g.K, g.C, g.R,
                                           g.S, 0, 0);
   if (!job.dw_w) return false;
+  bool ready = g_pack_was_resident;
   job.bias = bias ? resident_f32(bias, (size_t)g.C * 4) : nullptr;
+  if (bias) ready = ready && g_pack_was_resident;
+  job.a.consts_ready = ready ? 1 : 0;
   job_track_bias(job, job.bias, bias, g.C);
   job.depthwise = true;
   job.g = g;
@@ -364,7 +367,7 @@ void launch_job(ConvJob &job) {
     if (!dst) return;
   }
   if (job.depthwise) {
-    launch_depthwise_bf16(job.dw_x, job.dw_w, job.bias, (bf16 *)dst, g, mode_f16(), r.stream);
+    launch_depthwise_bf16(job.dw_x, job.dw_w, job.bias, (bf16 *)dst, g, mode_f16(), job.a.consts_ready != 0, r.stream);
   } else {
     job.a.y = (bf16 *)dst;
     job.a.act = g.act; job.a.lo = g.lo; job.a.hi = g.hi;

@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(256) conv_f32_kernel(const float *__restrict__
                                                        const float *__restrict__ w,
                                                        const float *__restrict__ bias,
                                                        float *__restrict__ y, ConvGeom g) {
+  chain_begin();
   __shared__ float sW[CT_K][CT_M + 4];
   __shared__ float sX[CT_K][CT_N + 4];
   const int Cg = g.C / g.groups, Kg = g.K / g.groups;
@@ -127,7 +128,7 @@ void launch_conv_f32(const float *x, const float *w, const float *bias, float *y
   const int64_t Mtot = (int64_t)g.N * g.P * g.Q;
   dim3 grid((unsigned)((Mtot + CT_N - 1) / CT_N), (unsigned)((Kg + CT_M - 1) / CT_M),
             (unsigned)g.groups);
-  conv_f32_kernel<<<grid, 256, 0, s>>>(x, w, bias, y, g);
+  launch_chained(conv_f32_kernel, grid, 256, 0, s, x, w, bias, y, g);
   count(CNT_LAUNCHES);
   count(CNT_SIMT_LAUNCHES);
 }
@@ -137,6 +138,7 @@ void launch_conv_f32(const float *x, const float *w, const float *bias, float *y
 __global__ void depthwise_f32_kernel(const float *__restrict__ x, const float *__restrict__ w,
                                      const float *__restrict__ bias, float *__restrict__ y,
                                      ConvGeom g, int64_t total) {
+  chain_begin();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int q = (int)(i % g.Q);
@@ -162,7 +164,7 @@ __global__ void depthwise_f32_kernel(const float *__restrict__ x, const float *_
 void launch_depthwise_f32(const float *x, const float *w, const float *bias, float *y,
                           const ConvGeom &g, cudaStream_t s) {
   const int64_t total = (int64_t)g.N * g.C * g.P * g.Q;
-  depthwise_f32_kernel<<<grid_for(total, 256), 256, 0, s>>>(x, w, bias, y, g, total);
+  launch_chained(depthwise_f32_kernel, grid_for(total, 256), 256, 0, s, x, w, bias, y, g, total);
   count(CNT_LAUNCHES);
 }
 
@@ -178,6 +180,7 @@ struct Bcast {
 __global__ void tensor_op_f32_kernel(int mode, const float *A,
                                      const float *B, float *out,
                                      Bcast bc, float biasB, int64_t total) {
+  chain_begin();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
     int64_t rem = i, ib = 0;
@@ -198,6 +201,7 @@ __global__ void tensor_op_f32_kernel(int mode, const float *A,
 __global__ void tensor_op_same_f32_kernel(int mode, const float4 *A,
                                           const float4 *B, float4 *out,
                                           float biasB, int64_t n4) {
+  chain_begin();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n4;
        i += (int64_t)gridDim.x * blockDim.x) {
     const float4 a = A[i], b = B[i];
@@ -219,6 +223,7 @@ __global__ void tensor_op_same_f32_kernel(int mode, const float4 *A,
 __global__ void bias_plane_f32_kernel(int mode, const float *A,
                                       const float *B, float *out, int C,
                                       int64_t HW, float biasB) {
+  chain_begin();
   const int64_t plane = blockIdx.x;
   const float b = biasB * B[plane % C];
   const float *a = A + plane * HW;
@@ -239,14 +244,14 @@ void launch_tensor_op_f32(int mode, const float *A, const float *B, float *out, 
   if (total == 0) return;
   const bool aligned = (((uintptr_t)A | (uintptr_t)B | (uintptr_t)out) & 15) == 0;
   if ((same || mode == 4) && aligned && total % 4 == 0) {
-    tensor_op_same_f32_kernel<<<grid_for(total / 4, 256, 2), 256, 0, s>>>(
+    launch_chained(tensor_op_same_f32_kernel, grid_for(total / 4, 256, 2), 256, 0, s, 
         mode, (const float4 *)A, (const float4 *)(mode == 4 ? A : B), (float4 *)out, biasB,
         total / 4);
   } else if (mode != 4 && rank == 4 && dimB[0] == 1 && dimB[2] == 1 && dimB[3] == 1 &&
              dimB[1] == dimA[1] && dimA[2] * dimA[3] < 65535 * 1024) {
     const int64_t HW = dimA[2] * dimA[3];
     dim3 grid((unsigned)(dimA[0] * dimA[1]), (unsigned)((HW + 1023) / 1024));
-    bias_plane_f32_kernel<<<grid, 256, 0, s>>>(mode, A, B, out, (int)dimA[1], HW, biasB);
+    launch_chained(bias_plane_f32_kernel, grid, 256, 0, s, mode, A, B, out, (int)dimA[1], HW, biasB);
   } else {
     Bcast bc;
     bc.rank = rank;
@@ -256,7 +261,7 @@ void launch_tensor_op_f32(int mode, const float *A, const float *B, float *out, 
       bc.strideB[i] = dimB[i] == 1 ? 0 : sb;
       sb *= dimB[i];
     }
-    tensor_op_f32_kernel<<<grid_for(total, 256), 256, 0, s>>>(mode, A, mode == 4 ? A : B, out, bc,
+    launch_chained(tensor_op_f32_kernel, grid_for(total, 256), 256, 0, s, mode, A, mode == 4 ? A : B, out, bc,
                                                                biasB, total);
   }
   count(CNT_LAUNCHES);
@@ -264,6 +269,7 @@ void launch_tensor_op_f32(int mode, const float *A, const float *B, float *out, 
 
 __global__ void act_f32_kernel(const float *x, float *y, int64_t n,
                                int act, float lo, float hi) {
+  chain_begin();
   const int64_t n4 = n / 4;
   const float4 *x4 = (const float4 *)x;
   float4 *y4 = (float4 *)y;
@@ -281,6 +287,7 @@ __global__ void act_f32_kernel(const float *x, float *y, int64_t n,
 
 __global__ void act_f32_scalar_kernel(const float *x, float *y,
                                       int64_t n, int act, float lo, float hi) {
+  chain_begin();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     y[i] = act_apply(x[i], act, lo, hi);
@@ -290,9 +297,9 @@ void launch_act_f32(const float *x, float *y, int64_t n, int act, float lo, floa
                     cudaStream_t s) {
   if (n == 0) return;
   if ((((uintptr_t)x | (uintptr_t)y) & 15) == 0)
-    act_f32_kernel<<<grid_for(n / 4 + 1, 256, 2), 256, 0, s>>>(x, y, n, act, lo, hi);
+    launch_chained(act_f32_kernel, grid_for(n / 4 + 1, 256, 2), 256, 0, s, x, y, n, act, lo, hi);
   else
-    act_f32_scalar_kernel<<<grid_for(n, 256), 256, 0, s>>>(x, y, n, act, lo, hi);
+    launch_chained(act_f32_scalar_kernel, grid_for(n, 256), 256, 0, s, x, y, n, act, lo, hi);
   count(CNT_LAUNCHES);
 }
 
@@ -302,6 +309,7 @@ void launch_act_f32(const float *x, float *y, int64_t n, int act, float lo, floa
 __global__ void pool_f32_kernel(const float *__restrict__ x, float *__restrict__ y, int H, int W,
                                 int P, int Q, int kh, int kw, int pad_h, int pad_w, int sh,
                                 int sw, bool avg, int64_t total) {
+  chain_begin();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int q = (int)(i % Q);
@@ -328,7 +336,7 @@ void launch_pool_f32(const float *x, float *y, int N, int C, int H, int W, int P
                      int kw, int pad_h, int pad_w, int sh, int sw, bool avg, cudaStream_t s) {
   const int64_t total = (int64_t)N * C * P * Q;
   if (total == 0) return;
-  pool_f32_kernel<<<grid_for(total, 256), 256, 0, s>>>(x, y, H, W, P, Q, kh, kw, pad_h, pad_w, sh,
+  launch_chained(pool_f32_kernel, grid_for(total, 256), 256, 0, s, x, y, H, W, P, Q, kh, kw, pad_h, pad_w, sh,
                                                        sw, avg, total);
   count(CNT_LAUNCHES);
 }
@@ -345,6 +353,7 @@ struct ReduceShape {
 
 __global__ void reduce_mean_f32_kernel(const float *__restrict__ x, float *__restrict__ y,
                                        ReduceShape rs, int64_t n_out, int64_t n_red) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -391,7 +400,7 @@ void launch_reduce_mean_f32(const float *x, float *y, int rank, const int64_t *d
     }
   }
   if (n_out == 0) return;
-  reduce_mean_f32_kernel<<<grid_for(n_out * 32, 256), 256, 0, s>>>(x, y, rs, n_out, n_red);
+  launch_chained(reduce_mean_f32_kernel, grid_for(n_out * 32, 256), 256, 0, s, x, y, rs, n_out, n_red);
   count(CNT_LAUNCHES);
 }
 
@@ -404,6 +413,7 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(const float *__restrict__
                                                        int K, int64_t sam, int64_t sak,
                                                        int64_t sbk, int64_t sbn, float alpha,
                                                        float beta) {
+  chain_begin();
   __shared__ float sA[CT_K][CT_M + 4];
   __shared__ float sB[CT_K][CT_N + 4];
   const int t = threadIdx.x, tx = t % 16, ty = t / 16;
@@ -458,7 +468,7 @@ void launch_gemm_f32(const float *A, const float *B, float *out, int M, int N, i
   const int64_t sam = transA ? 1 : lda, sak = transA ? lda : 1;
   const int64_t sbk = transB ? 1 : ldb, sbn = transB ? ldb : 1;
   dim3 grid((N + CT_N - 1) / CT_N, (M + CT_M - 1) / CT_M);
-  gemm_f32_kernel<<<grid, 256, 0, s>>>(A, B, out, M, N, K, sam, sak, sbk, sbn, alpha, beta);
+  launch_chained(gemm_f32_kernel, grid, 256, 0, s, A, B, out, M, N, K, sam, sak, sbk, sbn, alpha, beta);
   count(CNT_LAUNCHES);
   count(CNT_SIMT_LAUNCHES);
 }
@@ -485,6 +495,7 @@ __device__ __forceinline__ float block_reduce(float v, bool is_max, float *sh) {
 
 __global__ void softmax_f32_kernel(const float *x, float *y,
                                    int64_t len, int64_t inner) {
+  chain_begin();
   __shared__ float sh[32];
   const int64_t slice = blockIdx.x;
   const int64_t base = (slice / inner) * len * inner + slice % inner;
@@ -503,7 +514,7 @@ __global__ void softmax_f32_kernel(const float *x, float *y,
 void launch_softmax_f32(const float *x, float *y, int64_t outer, int64_t len, int64_t inner,
                         cudaStream_t s) {
   if (outer * inner == 0) return;
-  softmax_f32_kernel<<<(unsigned)(outer * inner), 128, 0, s>>>(x, y, len, inner);
+  launch_chained(softmax_f32_kernel, (unsigned)(outer * inner), 128, 0, s, x, y, len, inner);
   count(CNT_LAUNCHES);
 }
 

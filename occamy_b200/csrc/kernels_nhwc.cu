@@ -142,6 +142,7 @@ __device__ __forceinline__ bf16x8 pack8(const float *f) {
 template <bool F16>
 __global__ void nchw_to_nhwc_kernel(const float *__restrict__ x, uint16_t *__restrict__ y, int C,
                                     int HW) {
+  chain_begin();
   __shared__ float tile[32][33];
   const int n = blockIdx.z;
   const int c0 = blockIdx.y * 32, p0 = blockIdx.x * 32;
@@ -161,6 +162,7 @@ __global__ void nchw_to_nhwc_kernel(const float *__restrict__ x, uint16_t *__res
 template <bool F16>
 __global__ void nhwc_to_nchw_kernel(const uint16_t *__restrict__ x, float *__restrict__ y, int C,
                                     int HW) {
+  chain_begin();
   __shared__ float tile[32][33];
   const int n = blockIdx.z;
   const int c0 = blockIdx.y * 32, p0 = blockIdx.x * 32;
@@ -182,8 +184,8 @@ void launch_nchw_f32_to_nhwc_bf16(const float *x, bf16 *y, int N, int C, int H, 
   const int HW = H * W;
   if ((int64_t)N * C * HW == 0) return;
   dim3 grid((HW + 31) / 32, (C + 31) / 32, N), block(32, 8);
-  if (f16) nchw_to_nhwc_kernel<true><<<grid, block, 0, s>>>(x, (uint16_t *)y, C, HW);
-  else nchw_to_nhwc_kernel<false><<<grid, block, 0, s>>>(x, (uint16_t *)y, C, HW);
+  if (f16) launch_chained(nchw_to_nhwc_kernel<true>, grid, block, 0, s, x, (uint16_t *)y, C, HW);
+  else launch_chained(nchw_to_nhwc_kernel<false>, grid, block, 0, s, x, (uint16_t *)y, C, HW);
   count(CNT_LAUNCHES);
 }
 
@@ -192,13 +194,14 @@ void launch_nhwc_bf16_to_nchw_f32(const bf16 *x, float *y, int N, int C, int H, 
   const int HW = H * W;
   if ((int64_t)N * C * HW == 0) return;
   dim3 grid((HW + 31) / 32, (C + 31) / 32, N), block(32, 8);
-  if (f16) nhwc_to_nchw_kernel<true><<<grid, block, 0, s>>>((const uint16_t *)x, y, C, HW);
-  else nhwc_to_nchw_kernel<false><<<grid, block, 0, s>>>((const uint16_t *)x, y, C, HW);
+  if (f16) launch_chained(nhwc_to_nchw_kernel<true>, grid, block, 0, s, (const uint16_t *)x, y, C, HW);
+  else launch_chained(nhwc_to_nchw_kernel<false>, grid, block, 0, s, (const uint16_t *)x, y, C, HW);
   count(CNT_LAUNCHES);
 }
 
 template <bool F16>
 __global__ void f32_to_bf16_kernel(const float *__restrict__ x, uint16_t *__restrict__ y, int64_t n) {
+  chain_begin();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     y[i] = f32_to_elem<F16>(x[i]);
@@ -206,8 +209,8 @@ __global__ void f32_to_bf16_kernel(const float *__restrict__ x, uint16_t *__rest
 
 void launch_f32_to_bf16(const float *x, bf16 *y, int64_t n, bool f16, cudaStream_t s) {
   if (n == 0) return;
-  if (f16) f32_to_bf16_kernel<true><<<grid_for(n, 256), 256, 0, s>>>(x, (uint16_t *)y, n);
-  else f32_to_bf16_kernel<false><<<grid_for(n, 256), 256, 0, s>>>(x, (uint16_t *)y, n);
+  if (f16) launch_chained(f32_to_bf16_kernel<true>, grid_for(n, 256), 256, 0, s, x, (uint16_t *)y, n);
+  else launch_chained(f32_to_bf16_kernel<false>, grid_for(n, 256), 256, 0, s, x, (uint16_t *)y, n);
   count(CNT_LAUNCHES);
 }
 
@@ -217,6 +220,7 @@ void launch_f32_to_bf16(const float *x, bf16 *y, int64_t n, bool f16, cudaStream
 template <bool F16>
 __global__ void add_act_bf16_kernel(const bf16x8 *a, const bf16x8 *b, const float *bias_c, int C8,
                                     bf16x8 *out, int64_t n8, int act, float lo, float hi) {
+  chain_begin();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n8;
        i += (int64_t)gridDim.x * blockDim.x) {
     float f[8], g2[8];
@@ -242,10 +246,10 @@ void launch_add_act_bf16(const bf16 *a, const bf16 *b, const float *bias_c, int 
                          int64_t n, int act, float lo, float hi, bool f16, cudaStream_t s) {
   if (n == 0) return;
   if (f16)
-    add_act_bf16_kernel<true><<<grid_for(n / 8, 256), 256, 0, s>>>(
+    launch_chained(add_act_bf16_kernel<true>, grid_for(n / 8, 256), 256, 0, s, 
         (const bf16x8 *)a, (const bf16x8 *)b, bias_c, C / 8, (bf16x8 *)out, n / 8, act, lo, hi);
   else
-    add_act_bf16_kernel<false><<<grid_for(n / 8, 256), 256, 0, s>>>(
+    launch_chained(add_act_bf16_kernel<false>, grid_for(n / 8, 256), 256, 0, s, 
         (const bf16x8 *)a, (const bf16x8 *)b, bias_c, C / 8, (bf16x8 *)out, n / 8, act, lo, hi);
   count(CNT_LAUNCHES);
 }
@@ -260,6 +264,7 @@ __global__ void __launch_bounds__(256) pool_bf16_kernel(const bf16x8 *__restrict
                                                         int W, int P, int Q, int kh, int kw,
                                                         int pad_h, int pad_w, int sh, int sw,
                                                         int64_t total) {
+  chain_begin();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int c8 = (int)(i % C8);
@@ -311,6 +316,7 @@ __global__ void __launch_bounds__(256) pool_win_bf16_kernel(const bf16x8 *__rest
                                                             bf16x8 *__restrict__ y, int C8, int H,
                                                             int W, int Q, int pad_h, int pad_w,
                                                             unsigned per_image, unsigned chunks) {
+  chain_begin();
   const unsigned n = blockIdx.x / chunks;
   const unsigned j = (blockIdx.x - n * chunks) * 256u + threadIdx.x;
   if (j >= per_image) return;
@@ -364,7 +370,7 @@ static void launch_pool_win(const bf16 *x, bf16 *y, int N, int C, int H, int W, 
   const unsigned chunks = (per_image + 255u) / 256u;
   const unsigned grid = chunks * (unsigned)N;
   auto go = [&](auto kern) {
-    kern<<<grid, 256, 0, s>>>((const bf16x8 *)x, (bf16x8 *)y, C / 8, H, W, Q, pad_h, pad_w, per_image,
+    launch_chained(kern, grid, 256, 0, s, (const bf16x8 *)x, (bf16x8 *)y, C / 8, H, W, Q, pad_h, pad_w, per_image,
                               chunks);
   };
   if (avg && f16) go(pool_win_bf16_kernel<K, S, true, true>);
@@ -390,7 +396,7 @@ void launch_pool_bf16(const bf16 *x, bf16 *y, int N, int C, int H, int W, int P,
   }
   const int grid = grid_for(total, 256);
   auto go = [&](auto kern) {
-    kern<<<grid, 256, 0, s>>>((const bf16x8 *)x, (bf16x8 *)y, C / 8, H, W, P, Q, kh, kw, pad_h, pad_w, sh,
+    launch_chained(kern, grid, 256, 0, s, (const bf16x8 *)x, (bf16x8 *)y, C / 8, H, W, P, Q, kh, kw, pad_h, pad_w, sh,
                               sw, total);
   };
   if (avg && f16) go(pool_bf16_kernel<true, true>);
@@ -409,6 +415,7 @@ template <bool F16>
 __global__ void __launch_bounds__(8 * GAP_ROWS) gap_bf16_kernel(const bf16x8 *__restrict__ x,
                                                                float *__restrict__ y, uint16_t *__restrict__ y16,
                                                                int HW, int C8) {
+  chain_begin();
   __shared__ float part[GAP_ROWS][8][8];
   const int lane8 = threadIdx.x & 7, prow = threadIdx.x >> 3;
   const int c8 = blockIdx.x * 8 + lane8;
@@ -444,8 +451,8 @@ void launch_gap_bf16(const bf16 *x, float *y, bf16 *y16, int N, int HW, int C, b
   if ((int64_t)N * C == 0) return;
   const int C8 = C / 8;
   const dim3 grid((unsigned)((C8 + 7) / 8), (unsigned)N);
-  if (f16) gap_bf16_kernel<true><<<grid, 8 * GAP_ROWS, 0, s>>>((const bf16x8 *)x, y, (uint16_t *)y16, HW, C8);
-  else gap_bf16_kernel<false><<<grid, 8 * GAP_ROWS, 0, s>>>((const bf16x8 *)x, y, (uint16_t *)y16, HW, C8);
+  if (f16) launch_chained(gap_bf16_kernel<true>, grid, 8 * GAP_ROWS, 0, s, (const bf16x8 *)x, y, (uint16_t *)y16, HW, C8);
+  else launch_chained(gap_bf16_kernel<false>, grid, 8 * GAP_ROWS, 0, s, (const bf16x8 *)x, y, (uint16_t *)y16, HW, C8);
   count(CNT_LAUNCHES);
 }
 
@@ -459,6 +466,7 @@ template <bool CLAMP, bool F16>
 __global__ void depthwise_bf16_kernel(const bf16x8 *__restrict__ x, const float *__restrict__ w,
                                       const float *__restrict__ bias, bf16x8 *__restrict__ y,
                                       ConvGeom g, int64_t total, float lo, float hi) {
+  chain_begin();
   const int C8 = g.C / 8;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -588,6 +596,7 @@ __global__ void __launch_bounds__(256, CH == 2 ? 4 : 2) depthwise3x3_tile_kernel
     const uint4 *__restrict__ x, const float *__restrict__ w, const float *__restrict__ bias,
     uint32_t *__restrict__ y, ConvGeom g, int G, int cols, int TH, int tiles_q, int tiles_c, int ntiles,
     int run_len, int run_total, float act_lo, float act_hi, int act_flags, uint32_t act_hi2) {
+  chain_begin();
   constexpr int NP = CH / 2;      // channel pairs (32-bit words of bf16) per thread
   constexpr int LG = 8 / CH;      // threads per 16-byte channel group
   extern __shared__ uint4 dw_smem[];
@@ -794,7 +803,10 @@ __global__ void __launch_bounds__(128, 4)
     depthwise3x3_strip_h2_kernel(const uint4 *__restrict__ x, const float *__restrict__ w,
                                  const float *__restrict__ bias, uint4 *__restrict__ y, ConvGeom g,
                                  int strips, int strip_rows, int64_t total, int act_flags,
-                                 uint32_t act_hi2, int ahead) {
+                                 uint32_t act_hi2, int ahead, int consts_ready) {
+  // filter and bias that were resident before the launch are fetched while the kernel before still runs
+  chain_next();
+  if (!consts_ready) chain_wait();
   const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;   // the launcher keeps total < 2^31
   if (idx >= (uint32_t)total) return;
   const int C8 = g.C / 8;
@@ -826,6 +838,7 @@ __global__ void __launch_bounds__(128, 4)
     bh[2] = h2_from_floats(b.x, b.y);
     bh[3] = h2_from_floats(b.z, b.w);
   }
+  if (consts_ready) chain_wait();
   // Input columns of the window.  A column outside the image (first and last output column
   // only) is read from the middle column instead and its three taps get weight zero, so the
   // loop has no per-column test.
@@ -937,7 +950,7 @@ __global__ void __launch_bounds__(128, 4)
 }
 
 void launch_depthwise_bf16(const bf16 *x, const float *w_rsc, const float *bias, bf16 *y,
-                           const ConvGeom &g, bool f16, cudaStream_t s) {
+                           const ConvGeom &g, bool f16, bool consts_ready, cudaStream_t s) {
   const int64_t total = (int64_t)g.N * g.P * g.Q * (g.C / 8);
   if (total == 0) return;
   const int C8 = g.C / 8;
@@ -989,11 +1002,11 @@ void launch_depthwise_bf16(const bf16 *x, const float *w_rsc, const float *bias,
       const int act_flags = (act_lo == 0.0f ? 1 : 0) | (act_hi != INFINITY ? 2 : 0);
       const uint32_t act_hi2 = (uint32_t)hbits * 0x10001u;
       if (ST == 1)
-        depthwise3x3_strip_h2_kernel<1><<<grid, 128, 0, s>>>((const uint4 *)x, w_rsc, bias, (uint4 *)y, g,
-                                                            strips, strip_rows, threads, act_flags, act_hi2, ahead);
+        launch_chained(depthwise3x3_strip_h2_kernel<1>, grid, 128, 0, s, (const uint4 *)x, w_rsc, bias, (uint4 *)y, g,
+                                                            strips, strip_rows, threads, act_flags, act_hi2, ahead, (int)consts_ready);
       else
-        depthwise3x3_strip_h2_kernel<2><<<grid, 128, 0, s>>>((const uint4 *)x, w_rsc, bias, (uint4 *)y, g,
-                                                            strips, strip_rows, threads, act_flags, act_hi2, ahead);
+        launch_chained(depthwise3x3_strip_h2_kernel<2>, grid, 128, 0, s, (const uint4 *)x, w_rsc, bias, (uint4 *)y, g,
+                                                            strips, strip_rows, threads, act_flags, act_hi2, ahead, (int)consts_ready);
       count(CNT_LAUNCHES);
       return;
     }
@@ -1075,7 +1088,7 @@ void launch_depthwise_bf16(const bf16 *x, const float *w_rsc, const float *bias,
         cudaFuncSetAttribute(depthwise3x3_tile_kernel<2, false, 4, true>, attr, lim);
       }
       auto go = [&](auto kern) {
-        kern<<<grid, 256, smem, s>>>((const uint4 *)x, w_rsc, bias, (uint32_t *)y, g, G, cols, TH, tiles_q,
+        launch_chained(kern, grid, 256, smem, s, (const uint4 *)x, w_rsc, bias, (uint32_t *)y, g, G, cols, TH, tiles_q,
                                      tiles_c, ntiles, run_len, run_total, act_lo, act_hi, act_flags,
                                      act_hi2);
       };
@@ -1098,16 +1111,16 @@ void launch_depthwise_bf16(const bf16 *x, const float *w_rsc, const float *bias,
     const float lo = g.act == ACT_RELU ? 0.0f : (g.act == ACT_CLIP ? g.lo : -INFINITY);
     const float hi = g.act == ACT_CLIP ? g.hi : INFINITY;
     if (f16)
-      depthwise_bf16_kernel<true, true><<<grid_for(total, 256), 256, 0, s>>>(
+      launch_chained(depthwise_bf16_kernel<true, true>, grid_for(total, 256), 256, 0, s, 
           (const bf16x8 *)x, w_rsc, bias, (bf16x8 *)y, g, total, lo, hi);
     else
-      depthwise_bf16_kernel<true, false><<<grid_for(total, 256), 256, 0, s>>>(
+      launch_chained(depthwise_bf16_kernel<true, false>, grid_for(total, 256), 256, 0, s, 
           (const bf16x8 *)x, w_rsc, bias, (bf16x8 *)y, g, total, lo, hi);
   } else if (f16) {
-    depthwise_bf16_kernel<false, true><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_chained(depthwise_bf16_kernel<false, true>, grid_for(total, 256), 256, 0, s, 
         (const bf16x8 *)x, w_rsc, bias, (bf16x8 *)y, g, total, 0.f, 0.f);
   } else {
-    depthwise_bf16_kernel<false, false><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_chained(depthwise_bf16_kernel<false, false>, grid_for(total, 256), 256, 0, s, 
         (const bf16x8 *)x, w_rsc, bias, (bf16x8 *)y, g, total, 0.f, 0.f);
   }
   count(CNT_LAUNCHES);
@@ -1134,6 +1147,7 @@ __device__ __forceinline__ void split3(float v, uint16_t &hi, uint16_t &mid, uin
 // apart, through a 32 x 32 tile like the plain layout conversion.
 __global__ void split3_nchw_kernel(const float *__restrict__ x, uint16_t *__restrict__ y, int C, int Cp,
                                    int HW, int64_t plane) {
+  chain_begin();
   __shared__ float tile[32][33];
   const int n = blockIdx.z;
   const int c0 = blockIdx.y * 32, p0 = blockIdx.x * 32;
@@ -1161,13 +1175,14 @@ void launch_split3_nchw(const float *x, bf16 *y, int N, int C, int Cp, int H, in
   const int HW = H * W;
   if ((int64_t)N * C * HW == 0) return;
   dim3 grid((HW + 31) / 32, (Cp + 31) / 32, N), block(32, 8);
-  split3_nchw_kernel<<<grid, block, 0, s>>>(x, (uint16_t *)y, C, Cp, HW, (int64_t)N * HW * Cp);
+  launch_chained(split3_nchw_kernel, grid, block, 0, s, x, (uint16_t *)y, C, Cp, HW, (int64_t)N * HW * Cp);
   count(CNT_LAUNCHES);
 }
 
 // x fp32 [M][K] (row length ld) -> three planes [M][Kp] bf16
 __global__ void split3_rows_kernel(const float *__restrict__ x, uint16_t *__restrict__ y, int K, int Kp,
                                    int ld, int64_t total, int64_t plane) {
+  chain_begin();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int k = (int)(i % Kp);
@@ -1183,7 +1198,7 @@ __global__ void split3_rows_kernel(const float *__restrict__ x, uint16_t *__rest
 void launch_split3_rows(const float *x, bf16 *y, int M, int K, int Kp, int ld, cudaStream_t s) {
   const int64_t total = (int64_t)M * Kp;
   if (total == 0) return;
-  split3_rows_kernel<<<grid_for(total, 256), 256, 0, s>>>(x, (uint16_t *)y, K, Kp, ld, total, total);
+  launch_chained(split3_rows_kernel, grid_for(total, 256), 256, 0, s, x, (uint16_t *)y, K, Kp, ld, total, total);
   count(CNT_LAUNCHES);
 }
 
@@ -1244,6 +1259,7 @@ void launch_pack_krsc_bf16(const float *w, bf16 *out, int K, int C, int R, int S
 // that is not a multiple of the MMA's 16 is padded before the tensor-core convolution).
 __global__ void pad_channels_kernel(const bf16x8 *__restrict__ x, bf16x8 *__restrict__ y, int C8,
                                     int Cp8, int64_t total) {
+  chain_begin();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int c = (int)(i % Cp8);
@@ -1258,7 +1274,7 @@ __global__ void pad_channels_kernel(const bf16x8 *__restrict__ x, bf16x8 *__rest
 void launch_pad_channels_bf16(const bf16 *x, bf16 *y, int64_t pixels, int C, int Cp, cudaStream_t s) {
   const int64_t total = pixels * (Cp / 8);
   if (total == 0) return;
-  pad_channels_kernel<<<grid_for(total, 256), 256, 0, s>>>((const bf16x8 *)x, (bf16x8 *)y, C / 8, Cp / 8,
+  launch_chained(pad_channels_kernel, grid_for(total, 256), 256, 0, s, (const bf16x8 *)x, (bf16x8 *)y, C / 8, Cp / 8,
                                                         total);
   count(CNT_LAUNCHES);
 }
@@ -1316,6 +1332,7 @@ void launch_pack_fold_bf16(const float *w, bf16 *out, int K, int C, int R, int S
 template <int CP, bool F16>
 __global__ void __launch_bounds__(256) pad_input_kernel(const float *__restrict__ x, bf16 *__restrict__ out, int C,
                                  int H, int W, int Wp, int pad_w, int64_t rows_total) {
+  chain_begin();
   constexpr int ROWS = 8;                        // image rows per CTA
   const int pieces_row = Wp * CP / 8;
   const int64_t plane = (int64_t)H * W;
@@ -1357,7 +1374,7 @@ void launch_pad_input_bf16(const float *x, bf16 *out, int N, int C, int H, int W
   const int threads = pieces_row >= 256 ? 256 : (pieces_row + 31) / 32 * 32;
   const int64_t rows = (int64_t)N * H;
   const unsigned grid = (unsigned)((rows + 7) / 8);
-  auto go = [&](auto kern) { kern<<<grid, threads, 0, s>>>(x, out, C, H, W, Wp, pad_w, rows); };
+  auto go = [&](auto kern) { launch_chained(kern, grid, threads, 0, s, x, out, C, H, W, Wp, pad_w, rows); };
   if (f16) {
     if (Cp == 4) go(pad_input_kernel<4, true>);
     else if (Cp == 8) go(pad_input_kernel<8, true>);
