@@ -552,15 +552,28 @@ struct SkChoice {
   double cost;   // modelled microseconds; < 0: not possible
 };
 
+// Threads that issue a CTA's k-steps, each into an accumulator of its own: as many as there is work and
+// TMEM for (a k-step takes 0.27 us with one, about 0.14 with two, 0.09 with four).
+static int sk_pick_issuers(const TcConvArgs &a, int bn, int share) {
+  // A few-channel stem sums in filter-row order, one accumulator, like the kernel that takes the max
+  // pool along: a model gives the same bits whether that fusion happens or not.
+  if (a.w_step) return 1;
+  const int most = sk_issuers(bn, a.split != 0);
+  return share < most ? share : most;
+}
+
 // Tile width and number of CTAs that share a tile's reduction: the lowest modelled time, all CTAs
 // resident at once (a second wave costs as much as the first: 256->256 3x3 at 14x14, batch 32, 100
 // CTAs of 128 channels 12.3 us, 200 of 64 channels 18.1 us).  The model is a fit, within 10 %, to a
 // sweep of the twelve layer shapes of ResNet-50 at batch 1 to 64, times per layer in a chain of
 // dependent launches:
-//   fixed     launch to launch, first load to last store: 3.25 / 3.65 / 4.6 us at 32 / 64 / 128 channels
+//   fixed     launch to launch, first load to last store: 2.35 / 3.05 / 3.7 us at 32 / 64 / 128 channels,
+//             and more CTAs to launch
 //   k-steps   the tensor pipe (four MMAs of 48.5 cycles up to 64 channels, of 64 at 128) plus what the
 //             L2 adds with many CTAs reading
-//   cluster   0.3 us and, per CTA of the cluster, the exchange of the partial sums
+//   cluster   launching clusters and exchanging partial sums, by the number of CTAs
+// The fixed part was 0.8 us longer before the epilogue's code was fetched ahead of time, the exchange
+// 0.7 us longer with a cluster barrier behind plain remote stores.
 static SkChoice sk_choose(const TcConvArgs &a, long sp_tiles, int rows, int ksteps, int bk, int a_bytes, int nsm) {
   SkChoice best{0, 1, 0, -1.0};
   for (int bn = 128; bn >= 32; bn /= 2) {
@@ -570,9 +583,6 @@ static SkChoice sk_choose(const TcConvArgs &a, long sp_tiles, int rows, int kste
 #endif
     const long tiles = sp_tiles * ((a.K + bn - 1) / bn);
     const int stage_bytes = a_bytes + bn * bk * 2;
-    // A few-channel stem sums in filter-row order, one accumulator, like the kernel that takes the max
-    // pool along: a model gives the same bits whether that fusion happens or not.
-    const int issuers = a.w_step ? 1 : sk_issuers(bn, a.split != 0);
     for (int s = 1; s <= (a.w_step ? 1 : SK_MAX_SPLITS) && s <= ksteps; ++s) {
       // (clusters of more than two leave some SMs of every GPC without a partner)
       long most = s <= 2 ? nsm : nsm - nsm / 9;
@@ -584,6 +594,7 @@ static SkChoice sk_choose(const TcConvArgs &a, long sp_tiles, int rows, int kste
       if (ctas > most) break;
       const int rows_owner = (rows + s - 1) / s;
       const int share = (ksteps + s - 1) / s;
+      const int issuers = sk_pick_issuers(a, bn, share);
       // Half of the SM's shared memory leaves room for the next layer's prologue; a ring of eight
       // stages (or all of a CTA's k-steps) is worth more than that: 256->256 3x3 at 14x14, batch 8,
       // 10.0 us with four stages, 7.4 us with eight.
@@ -597,11 +608,13 @@ static SkChoice sk_choose(const TcConvArgs &a, long sp_tiles, int rows, int kste
         if (stages >= 8 || stages == share) break;
       }
       if (stages < 1) continue;
-      double step = bn == 32 ? 0.095 + 0.00006 * ctas : bn == 64 ? 0.12 + 0.00025 * ctas : 0.155 + 0.0005 * ctas;
+      const double n = (double)ctas;
+      double step = bn == 32 ? 0.085 + 0.00008 * n : bn == 64 ? 0.105 + 0.00027 * n : 0.16 + 0.0004 * n;
       step *= bk == 64 ? 1.0 : 0.75;
-      if (issuers < 2) step += 0.12;
-      const double exchange = s > 1 ? 0.3 + s * (0.05 + 0.4 * rows / 128.0) : 0.0;
-      const double cost = (bn == 32 ? 3.25 : bn == 64 ? 3.65 : 4.6) + share * step + exchange;
+      if (issuers < 2 && share > 1) step += 0.12;
+      const double fixed_us = bn == 32 ? 2.35 + 0.006 * n : bn == 64 ? 3.05 + 0.008 * n : 3.7 + 0.008 * n;
+      const double exchange = 0.52 + n * (0.0104 + 0.013 * rows / 128.0) + (bn == 128 ? 3.25 : 0.0);
+      const double cost = fixed_us + share * step + (s > 1 ? exchange : 0.0);
       if (best.cost < 0 || cost < best.cost) best = SkChoice{bn, s, stages, cost};
     }
   }
@@ -641,7 +654,7 @@ static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, d
   p.stages = c.stages;
   p.splits = c.splits;
   const int share = (p.ksteps + c.splits - 1) / c.splits;
-  p.issuers = a.w_step ? 1 : sk_issuers(c.bn, a.split != 0) < share ? sk_issuers(c.bn, a.split != 0) : share;
+  p.issuers = sk_pick_issuers(a, c.bn, share);
   p.rows_owner = (p.rows + c.splits - 1) / c.splits;
   p.tiles_k = (a.K + bn - 1) / bn;
   p.div_k = make_fastdiv(p.tiles_k);
@@ -797,7 +810,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
     const int per_wave = pair ? nsm / 2 : nsm;
     const double waves = (double)((p.total_tiles + per_wave - 1) / per_wave);
     const int ks = p.cblocks * a.R * a.S * combos;
-    const double tile_us = halo ? 0.9 : pn ? 0.49 * ks : (bn == 256 ? 0.4 : 0.0) + 0.27 * ks * (bk == 64 ? 1.0 : 0.75);
+    const double tile_us = halo ? 0.9 : pn ? 0.49 * ks : (bn == 256 ? 0.1 : 0.0) + 0.27 * ks * (bk == 64 ? 1.0 : 0.75);
     if (sk_plan(a, err_word, nsm, counted, 3.1 + waves * tile_us, &pl)) return pl;
   }
   const uint32_t boxA[4] = {(uint32_t)bk, (uint32_t)p.tw, (uint32_t)p.th, (uint32_t)p.tn};

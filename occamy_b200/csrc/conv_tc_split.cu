@@ -36,9 +36,25 @@ __device__ __forceinline__ void cluster_arrive_release() {
 __device__ __forceinline__ void cluster_wait_acquire() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c),
-               "r"(d)
+// Stores that happen when `on` is set: predicated instructions, not branches, so that the code in front of
+// them runs (and is fetched) either way -- see the rehearsal below.
+// (to another CTA's shared memory, counted there on the barrier `bar` as the bytes arrive)
+__device__ __forceinline__ void st_async_v4_if(bool on, uint32_t addr, uint32_t bar, uint32_t a, uint32_t b,
+                                               uint32_t c, uint32_t d) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.u32 p, %6, 0;\n"
+      "@p st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];\n}" ::"r"(addr),
+      "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar), "r"((uint32_t)on)
+      : "memory");
+}
+__device__ __forceinline__ void st_global_v4_if(bool on, void *addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %5, 0;\n@p st.global.v4.b32 [%0], {%1, %2, %3, %4};\n}" ::"l"(addr),
+               "r"(a), "r"(b), "r"(c), "r"(d), "r"((uint32_t)on)
+               : "memory");
+}
+__device__ __forceinline__ void st_global_if(bool on, float *addr, float v) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p st.global.f32 [%0], %1;\n}" ::"l"(addr), "f"(v),
+               "r"((uint32_t)on)
                : "memory");
 }
 
@@ -61,25 +77,23 @@ __device__ __forceinline__ uint4 sk_pack16(const SkParams &p, float *v, const ui
     o[j] = f2_to_bf16x2<F16>(f2_pack(tc_act(v[2 * j], p.lo, p.hi), tc_act(v[2 * j + 1], p.lo, p.hi)));
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
-__device__ __forceinline__ void sk_finish32(const SkParams &p, float *v, int64_t lin, int c) {
+__device__ __forceinline__ void sk_finish32(const SkParams &p, bool on, float *v, int64_t lin, int c) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) v[j] = tc_act(v[j], p.lo, p.hi);
-  if (p.out_hw) {
-    const int64_t img = lin / p.out_hw;
-    float *o = p.out_f32 + (img * p.K + c) * p.out_hw + (lin - img * p.out_hw);
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (c + j < p.K) o[(int64_t)j * p.out_hw] = v[j];
-    return;
-  }
+  int64_t step = 1;
   float *o = p.out_f32 + lin * p.ldo + c;
+  if (p.out_hw) {
+    const uint32_t img = (uint32_t)lin / (uint32_t)p.out_hw;
+    step = p.out_hw;
+    o = p.out_f32 + ((int64_t)img * p.K + c) * step + ((uint32_t)lin - img * (uint32_t)p.out_hw);
+  }
   if (p.out_vec4 && c + 8 <= p.K) {
-    reinterpret_cast<float4 *>(o)[0] = make_float4(v[0], v[1], v[2], v[3]);
-    reinterpret_cast<float4 *>(o)[1] = make_float4(v[4], v[5], v[6], v[7]);
+    st_global_v4_if(on, o, __float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+    st_global_v4_if(on, o + 4, __float_as_uint(v[4]), __float_as_uint(v[5]), __float_as_uint(v[6]),
+                    __float_as_uint(v[7]));
   } else {
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (c + j < p.K) o[j] = v[j];
+    for (int j = 0; j < 8; ++j) st_global_if(on && c + j < p.K, o + j * step, v[j]);
   }
 }
 
@@ -94,7 +108,7 @@ __device__ __forceinline__ void sk_finish32(const SkParams &p, float *v, int64_t
 // One flavour per instantiation: these kernels run for a few microseconds, and every stretch of code
 // that is not in the instruction cache yet costs a tenth of that.
 template <int BN, bool F16, bool SPLIT, bool CL, bool F32>
-__global__ void __launch_bounds__(SK_THREADS, BN == 128 ? 1 : 2)
+__global__ void __launch_bounds__(SK_THREADS, 2)
     tc_split_kernel(const __grid_constant__ SkParams p) {
   constexpr uint32_t IDESC = (1u << 4) | (F16 ? 0u : ((1u << 7) | (1u << 10))) |
                              ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
@@ -120,11 +134,11 @@ __global__ void __launch_bounds__(SK_THREADS, BN == 128 ? 1 : 2)
   const uint32_t bar0 = smem_u32(bars);
   auto full_bar = [&](int s) { return bar0 + 8u * s; };
   auto empty_bar = [&](int s) { return bar0 + 8u * (stages + s); };
-  const uint32_t done_bar = bar0 + 16u * stages;
-  volatile uint32_t *tmem_holder = reinterpret_cast<volatile uint32_t *>(bars + 2 * stages + 1);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 2 * stages + 2);
+  const uint32_t done_bar = bar0 + 16u * stages, sums_bar = done_bar + 8u;
+  volatile uint32_t *tmem_holder = reinterpret_cast<volatile uint32_t *>(bars + 2 * stages + 2);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 2 * stages + 3);
   // which accumulators hold anything, one word per issuer: bit 0 main, bit 1 correction
-  volatile int *used = reinterpret_cast<volatile int *>(bars + 2 * stages + 3);
+  volatile int *used = reinterpret_cast<volatile int *>(bars + 2 * stages + 4);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Fewer accumulators when there are fewer k-steps: CTAs of the next layer that share this SM need
@@ -155,8 +169,13 @@ __global__ void __launch_bounds__(SK_THREADS, BN == 128 ? 1 : 2)
       mbar_init(empty_bar(s), 1);
     }
     mbar_init(done_bar, (uint32_t)ni);
+    mbar_init(sums_bar, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if constexpr (CL) {   // partial sums to come: my rows, from every CTA of the cluster
+      const int n = min(p.rows_owner, p.rows - rank * p.rows_owner);
+      mbar_expect_tx(sums_bar, n > 0 ? (uint32_t)(splits * n * BN * 4) : 0u);
+    }
   }
   if (warp == 3) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -213,71 +232,10 @@ __global__ void __launch_bounds__(SK_THREADS, BN == 128 ? 1 : 2)
     load_a(first, first);
     if (!p.consts_ready) load_b(first, first);
   }
-  if (warp >= 4 && warp < 4 + ni && lane == 0) {
-    // later turns (stages is a multiple of ni then): k-step i goes to stage i % stages, loader i % ni
-    int s = warp - 4;
-    uint32_t phase = 0;
-    for (int i = stages + s; i < mine; i += ni) {
-      if (!mbar_wait_hot(empty_bar(s), phase, abort_flag)) {
-        err_code = 1;
-        break;
-      }
-      mbar_expect_tx(full_bar(s), tx_bytes);
-      load_b(i, s);
-      load_a(i, s);
-      s += ni;
-      if (s >= stages) {
-        s -= stages;
-        phase ^= 1u;
-      }
-    }
-  } else if (warp < ni && lane == 0) {
-    const uint64_t a0 = make_smem_desc(sA, bk), b0 = make_smem_desc(sB, bk);
-    const uint32_t a_hi = (uint32_t)(a0 >> 32), b_hi = (uint32_t)(b0 >> 32);
-    const uint32_t a_step = a_bytes >> 4, b_step = b_bytes >> 4;
-    const uint32_t d0 = tmem + (uint32_t)(warp * (SPLIT ? 2 * BN : BN));
-    uint32_t seen = 0;
-    auto run = [&](auto nk_c) {
-      constexpr int NK = decltype(nk_c)::value;
-      uint32_t phase = 0;
-      int s = warp;
-      for (int i = warp; i < mine; i += ni) {
-        uint32_t d = d0, bit = 1u;
-        if constexpr (SPLIT) {
-          const uint32_t tap = tc_fdiv((uint32_t)(ks0 + i), p.div_cb);
-          if (tap % 6u != 0u) {
-            d = d0 + (uint32_t)BN;
-            bit = 2u;
-          }
-        }
-        const uint32_t a_lo = (uint32_t)a0 + (uint32_t)s * a_step, b_lo = (uint32_t)b0 + (uint32_t)s * b_step;
-        const uint32_t more = seen & bit;
-        if (!mbar_wait_hot(full_bar(s), phase, abort_flag)) {
-          err_code = 3;
-          return;
-        }
-        tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < NK; ++kk)
-          mma_lohi(d, a_lo + 2u * kk, a_hi, b_lo + 2u * kk, b_hi, IDESC, kk ? 1u : more);
-        seen |= bit;
-        if (i + stages < mine) tc_commit(empty_bar(s));   // nobody waits for the last ones
-        s += ni;
-        if (s >= stages) {   // (a ring as long as the share is never reused)
-          s -= stages;
-          phase ^= 1u;
-        }
-      }
-      tc_commit(done_bar);
-    };
-    if (bk == 64) run(std::integral_constant<int, 4>{});
-    else if (bk == 32) run(std::integral_constant<int, 2>{});
-    else run(std::integral_constant<int, 1>{});
-    used[warp] = (int)seen;
+  if (warp >= 4) {   // (the other four warps issue MMAs)
+    const int i = (int)threadIdx.x - 128;
+    if (i < BN) bias_s[i] = (p.bias && tl.k0 + i < p.K) ? p.bias[tl.k0 + i] : 0.0f;
   }
-  __syncwarp();
-  if (threadIdx.x < BN)
-    bias_s[threadIdx.x] = (p.bias && tl.k0 + (int)threadIdx.x < p.K) ? p.bias[tl.k0 + threadIdx.x] : 0.0f;
   if (!F32 && p.residual) {
     if constexpr (CL) {
 #pragma unroll
@@ -300,104 +258,187 @@ __global__ void __launch_bounds__(SK_THREADS, BN == 128 ? 1 : 2)
       }
     }
   }
-  __syncwarp();
-  if (!err_code && !mbar_wait(done_bar, 0, abort_flag)) err_code = 4;
-  tc_fence_after();
-  __syncthreads();   // bias_s
 
-  auto finish = [&](float *v, const uint4 &rs, int lin, int c) {
-    if constexpr (F32) sk_finish32(p, v, lin, c);
-    else
-      *reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(p.y) + (int64_t)lin * p.K + c) =
-          sk_pack16<F16>(p, v, rs);
-  };
-  int used_all[NI];
-#pragma unroll
-  for (int w = 0; w < NI; ++w) used_all[w] = w < ni ? used[w] : 0;
-  // columns of this thread's row, 32 at a time (16 for a 32-channel tile): the sum of the accumulators
-  constexpr int CH = HALF < 32 ? HALF : 32;
+  // what this thread does with the sums, worked out while they are being made
+  constexpr int CH = NACC > 1 || HALF < 32 ? 16 : 32;   // columns per step: of all accumulators at once
   const uint32_t t_row = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(part * HALF);
-  auto load_sum = [&](int h, uint32_t *r) {
-    bool any = false;
-#pragma unroll
-    for (int k = 0; k < NACC; ++k) {
-      if (!((used_all[SPLIT ? k / 2 : k] >> (SPLIT ? k & 1 : 0)) & 1)) continue;   // the same for all threads
-      uint32_t t[CH];
-      tc_ld<CH>(t_row + (uint32_t)(k * BN + h * CH), t);
-      tc_ld_wait();
-#pragma unroll
-      for (int j = 0; j < CH; ++j)
-        r[j] = any ? __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(t[j])) : t[j];
-      any = true;
+  const int lin_row = lin_s[row];
+  uint32_t dst = 0, dst_bar = 0;   // CL: where my row's partial sums go, and who counts them there
+  if constexpr (CL) {
+    const int owner = row / p.rows_owner;
+    if (row < p.rows) {
+      dst = cluster_map(sX, (uint32_t)owner) +
+            (uint32_t)(rank * p.rows_owner + row - owner * p.rows_owner) * (BN * 4u);
+      dst_bar = cluster_map(sums_bar, (uint32_t)owner);
+    }
+  }
+  auto finish = [&](bool on, float *v, const uint4 &rs, int lin, int c) {
+    if constexpr (F32) {
+      sk_finish32(p, on, v, lin, c);
+    } else {
+      const uint4 o = sk_pack16<F16>(p, v, rs);
+      st_global_v4_if(on, reinterpret_cast<uint16_t *>(p.y) + (int64_t)lin * p.K + c, o.x, o.y, o.z, o.w);
     }
   };
-  if constexpr (CL) {
-    cluster_wait_acquire();   // every CTA of the cluster has started
-    const int owner = row / p.rows_owner;
-    const uint32_t dst = row < p.rows ? cluster_map(sX, (uint32_t)owner) +
-                                            (uint32_t)(rank * p.rows_owner + row - owner * p.rows_owner) * (BN * 4u)
-                                      : 0u;
+
+  // Warps 4-7 go through the epilogue twice.  The first time is a rehearsal, right after the first
+  // loads have been requested: whatever it computes is not stored.  It brings the code into the
+  // instruction cache while the operands travel; fetched when the sums are ready it took 1000 to 2000
+  // cycles of a layer's 6000 to 10000 (times at the dispatch rule).
+#pragma unroll 1
+  for (int pass = warp >= 4 ? 0 : 1; pass < 2; ++pass) {
+    const bool real = pass != 0;
+    int used_all[NI];
+    if (real) {
+    if (warp >= 4 && warp < 4 + ni && lane == 0) {
+      // later turns (stages is a multiple of ni then): k-step i goes to stage i % stages, loader i % ni
+      int s = warp - 4;
+      uint32_t phase = 0;
+      for (int i = stages + s; i < mine; i += ni) {
+        if (!mbar_wait_hot(empty_bar(s), phase, abort_flag)) {
+          err_code = 1;
+          break;
+        }
+        mbar_expect_tx(full_bar(s), tx_bytes);
+        load_b(i, s);
+        load_a(i, s);
+        s += ni;
+        if (s >= stages) {
+          s -= stages;
+          phase ^= 1u;
+        }
+      }
+    } else if (warp < ni && lane == 0) {
+      const uint64_t a0 = make_smem_desc(sA, bk), b0 = make_smem_desc(sB, bk);
+      const uint32_t a_hi = (uint32_t)(a0 >> 32), b_hi = (uint32_t)(b0 >> 32);
+      const uint32_t a_step = a_bytes >> 4, b_step = b_bytes >> 4;
+      const uint32_t d0 = tmem + (uint32_t)(warp * (SPLIT ? 2 * BN : BN));
+      uint32_t seen = 0;
+      auto run = [&](auto nk_c) {
+        constexpr int NK = decltype(nk_c)::value;
+        uint32_t phase = 0;
+        int s = warp;
+        for (int i = warp; i < mine; i += ni) {
+          uint32_t d = d0, bit = 1u;
+          if constexpr (SPLIT) {
+            const uint32_t tap = tc_fdiv((uint32_t)(ks0 + i), p.div_cb);
+            if (tap % 6u != 0u) {
+              d = d0 + (uint32_t)BN;
+              bit = 2u;
+            }
+          }
+          const uint32_t a_lo = (uint32_t)a0 + (uint32_t)s * a_step, b_lo = (uint32_t)b0 + (uint32_t)s * b_step;
+          const uint32_t more = seen & bit;
+          if (!mbar_wait_hot(full_bar(s), phase, abort_flag)) {
+            err_code = 3;
+            return;
+          }
+          tc_fence_after();
+  #pragma unroll
+          for (int kk = 0; kk < NK; ++kk)
+            mma_lohi(d, a_lo + 2u * kk, a_hi, b_lo + 2u * kk, b_hi, IDESC, kk ? 1u : more);
+          seen |= bit;
+          if (i + stages < mine) tc_commit(empty_bar(s));   // nobody waits for the last ones
+          s += ni;
+          if (s >= stages) {   // (a ring as long as the share is never reused)
+            s -= stages;
+            phase ^= 1u;
+          }
+        }
+        tc_commit(done_bar);
+      };
+      if (bk == 64) run(std::integral_constant<int, 4>{});
+      else if (bk == 32) run(std::integral_constant<int, 2>{});
+      else run(std::integral_constant<int, 1>{});
+      used[warp] = (int)seen;
+    }
+      __syncwarp();
+      if (!err_code && !mbar_wait(done_bar, 0, abort_flag)) err_code = 4;
+      tc_fence_after();
+      __syncthreads();   // bias_s, used
+    }
 #pragma unroll
-    for (int h = 0; h < HALF / CH; ++h) {
-      uint32_t r[CH];
-      load_sum(h, r);
-      if (row < p.rows && !err_code) {
+    for (int w = 0; w < NI; ++w) used_all[w] = w >= ni ? 0 : real ? used[w] : (SPLIT ? 3 : 1);
+    // CH columns of this thread's row from column h * CH on: the sum of the accumulators, which are all
+    // requested before the first is waited for
+    auto load_sum = [&](int h, uint32_t *r) {
+      uint32_t t[NACC][CH];
+#pragma unroll
+      for (int k = 0; k < NACC; ++k) {
+        if ((used_all[SPLIT ? k / 2 : k] >> (SPLIT ? k & 1 : 0)) & 1) {   // the same for all threads
+          tc_ld<CH>(t_row + (uint32_t)(k * BN + h * CH), t[k]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < CH; ++j) t[k][j] = 0u;
+        }
+      }
+      tc_ld_wait();
+#pragma unroll
+      for (int j = 0; j < CH; ++j) {
+        float v = __uint_as_float(t[0][j]);
+#pragma unroll
+        for (int k = 1; k < NACC; ++k) v += __uint_as_float(t[k][j]);
+        r[j] = __float_as_uint(v);
+      }
+    };
+    if constexpr (CL) {
+      if (real) cluster_wait_acquire();   // every CTA of the cluster has started
+      const bool on = real && row < p.rows && !err_code;
+#pragma unroll
+      for (int h = 0; h < HALF / CH; ++h) {
+        uint32_t r[CH];
+        load_sum(h, r);
 #pragma unroll
         for (int j = 0; j < CH / 4; ++j) {
           // 16-byte pieces of a row are permuted by its number: eight lanes, eight bank groups
           const uint32_t piece = (uint32_t)((part * HALF + h * CH) / 4 + j) ^ (uint32_t)(row & 7);
-          st_cluster_v4(dst + piece * 16u, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          st_async_v4_if(on, dst + piece * 16u, dst_bar, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
         }
       }
       __syncwarp();
-    }
-    __syncwarp();
-    tc_fence_before();
-    cluster_arrive_release();
-    cluster_wait_acquire();
-    const uint8_t *xs = smem_raw + (sX - sA);
-    auto item = [&](int it, int r, int g, const uint4 &rs) {
-      const int lin = lin_s[row0 + r], c = tl.k0 + g * 8;
-      if (lin < 0 || c >= p.K) return;
-      float v[8];
+      if (real && !err_code && !mbar_wait(sums_bar, 0, abort_flag)) err_code = 6;
+      const uint8_t *xs = smem_raw + (sX - sA);
+      auto item = [&](bool live, int r, int g, const uint4 &rs) {
+        r = live ? r : 0;
+        g = live ? g : 0;
+        const int lin = lin_s[row0 + r < 128 ? row0 + r : 0], c = tl.k0 + g * 8;
+        float v[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = bias_s[g * 8 + j];
-      const uint32_t sw = (uint32_t)((row0 + r) & 7);
-      for (int k = 0; k < splits; ++k) {
-        const uint8_t *b = xs + (size_t)(k * p.rows_owner + r) * (BN * 4);
-        const float4 a = *reinterpret_cast<const float4 *>(b + (((uint32_t)(2 * g)) ^ sw) * 16u);
-        const float4 e = *reinterpret_cast<const float4 *>(b + (((uint32_t)(2 * g + 1)) ^ sw) * 16u);
-        v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
-        v[4] += e.x; v[5] += e.y; v[6] += e.z; v[7] += e.w;
-      }
-      finish(v, rs, lin, c);
-    };
-    if (!err_code) {
+        for (int j = 0; j < 8; ++j) v[j] = bias_s[g * 8 + j];
+        const uint32_t sw = (uint32_t)((row0 + r) & 7);
+#pragma unroll 4
+        for (int k = 0; k < splits; ++k) {
+          const uint8_t *b = xs + (size_t)(k * p.rows_owner + r) * (BN * 4);
+          const float4 a = *reinterpret_cast<const float4 *>(b + (((uint32_t)(2 * g)) ^ sw) * 16u);
+          const float4 e = *reinterpret_cast<const float4 *>(b + (((uint32_t)(2 * g + 1)) ^ sw) * 16u);
+          v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+          v[4] += e.x; v[5] += e.y; v[6] += e.z; v[7] += e.w;
+        }
+        finish(real && live && lin >= 0 && c < p.K && !err_code, v, rs, lin, c);
+      };
       if (F32 && p.out_hw) {   // consecutive threads on consecutive pixels of one channel
-        for (int it = threadIdx.x; it < items; it += SK_THREADS) item(it, it % nrows, it / nrows, res[0]);
+        const int n = nrows > 0 ? nrows : 1, end = real ? items : (int)threadIdx.x + 1;
+        for (int it = threadIdx.x; it < end; it += SK_THREADS) item(it < items, it % n, it / n, res[0]);
       } else {
 #pragma unroll
         for (int u = 0; u < BN / 16; ++u) {
           const int it = (int)threadIdx.x + u * SK_THREADS;
-          if (it < items) item(it, it / G8, it % G8, res[u]);
+          if (u == 0 || it < items) item(it < items, it / G8, it % G8, res[u]);
         }
       }
-    }
-  } else {
-    const int lin = lin_s[row];
+    } else {
 #pragma unroll
-    for (int h = 0; h < HALF / CH; ++h) {
-      uint32_t r[CH];
-      load_sum(h, r);
-      if (lin >= 0 && !err_code) {
+      for (int h = 0; h < HALF / CH; ++h) {
+        uint32_t r[CH];
+        load_sum(h, r);
 #pragma unroll
         for (int u = 0; u < CH / 8; ++u) {
           const int cl = part * HALF + h * CH + u * 8;
-          if (tl.k0 + cl >= p.K) break;
           float v[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[u * 8 + j]) + bias_s[cl + j];
-          finish(v, res[h * (CH / 8) + u], lin, tl.k0 + cl);
+          finish(real && lin_row >= 0 && tl.k0 + cl < p.K && !err_code, v, res[h * (CH / 8) + u], lin_row,
+                 tl.k0 + cl);
         }
       }
     }
@@ -411,6 +452,14 @@ __global__ void __launch_bounds__(SK_THREADS, BN == 128 ? 1 : 2)
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (CL) {
+    // A CTA that has its partial sums has heard from all the others and may go.  One that gave up stays
+    // until the others have gone (each of their waits is bounded): they may still be sending to it.
+    if (*abort_flag) {
+      cluster_arrive_release();
+      cluster_wait_acquire();
+    }
+  }
   if (warp == 3)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(cols)
@@ -420,7 +469,7 @@ __global__ void __launch_bounds__(SK_THREADS, BN == 128 ? 1 : 2)
 size_t sk_smem_bytes(int bn, int stages, int a_bytes, int bk, int splits, int rows_owner) {
   const size_t x = splits > 1 ? (size_t)splits * rows_owner * bn * 4 : 0;
   return (size_t)stages * (a_bytes + bn * bk * 2) + x +
-         bn * 4 + 512 + 8 * (2 * stages + 6);
+         bn * 4 + 512 + 8 * (2 * stages + 7);
 }
 
 template <int BN, bool F16, bool SPLIT, bool CL, bool F32>
