@@ -197,6 +197,17 @@ void job_track_bias(ConvJob &job, const float *used, const float *callers, int c
   }
 }
 
+// The folded form of a few-channel convolution: channels padded so that one output column's step along
+// the row is a multiple of 16 bytes, width taps padded to whole steps, pixels per padded row.
+void stem_geometry(const ConvGeom &g, int &Cp, int &Sp, int &Wp) {
+  Cp = g.C <= 4 ? (g.stride_w % 2 == 0 ? 4 : 8) : (g.C <= 8 ? 8 : 16);
+  const int unit = 16 / Cp;
+  Sp = (g.S + unit - 1) / unit * unit;
+  Wp = g.pad_w + g.W;
+  if (Wp < (g.Q - 1) * g.stride_w + Sp) Wp = (g.Q - 1) * g.stride_w + Sp;
+  Wp = (Wp + 7) / 8 * 8;
+}
+
 bool prepare_dense(const float *x, const float *w, const float *bias, const ConvGeom &g,
                    ConvJob &job) {
   Runtime &r = rt();
@@ -210,13 +221,7 @@ bool prepare_dense(const float *x, const float *w, const float *bias, const Conv
   const bool folded = g.C < 16;
   int Sp = 0, Cp = 0, Wp = 0;
   if (folded) {
-    // channels padded so that one output column's step along the row is a multiple of 16 bytes
-    Cp = g.C <= 4 ? (g.stride_w % 2 == 0 ? 4 : 8) : (g.C <= 8 ? 8 : 16);
-    const int unit = 16 / Cp;
-    Sp = (g.S + unit - 1) / unit * unit;
-    Wp = g.pad_w + g.W;
-    if (Wp < (g.Q - 1) * g.stride_w + Sp) Wp = (g.Q - 1) * g.stride_w + Sp;
-    Wp = (Wp + 7) / 8 * 8;
+    stem_geometry(g, Cp, Sp, Wp);
     a.H = g.H; a.W = g.Q; a.Cf = Sp * Cp;
     a.R = g.R; a.S = 1;
     a.pad_h = g.pad_h; a.pad_w = 0; a.stride_h = g.stride_h; a.stride_w = 1;
@@ -239,11 +244,19 @@ bool prepare_dense(const float *x, const float *w, const float *bias, const Conv
 
   job.dep_lo[0] = job.dep_hi[0] = 0;
   if (folded) {
-    ensure_f32(x);
-    bf16 *xf = (bf16 *)scratch_get(0, (size_t)g.N * g.H * Wp * Cp * 2);
-    if (!xf) return false;
-    launch_pad_input_bf16(x, xf, g.N, g.C, g.H, g.W, Wp, Cp, g.pad_w, mode_f16(), r.stream);
-    a.x = xf;
+    uintptr_t base = 0;
+    const TensorRec *rec = reg_find(x, &base);
+    if (rec && base == (uintptr_t)x && rec->fmt == FMT_STEM_ROWS && rec->n == g.N && rec->c == g.C && rec->h == g.H &&
+        rec->w == g.W && rec->stem_wp == Wp && rec->stem_cp == Cp && rec->stem_pad == g.pad_w &&
+        rec->stem_f16 == (int)mode_f16()) {
+      a.x = (const bf16 *)rec->home;   // brought in in this form
+    } else {
+      ensure_f32(x);
+      bf16 *xf = (bf16 *)scratch_get(0, (size_t)g.N * g.H * Wp * Cp * 2);
+      if (!xf) return false;
+      launch_pad_input_bf16(x, xf, g.N, g.C, g.H, g.W, Wp, Cp, g.pad_w, mode_f16(), r.stream);
+      a.x = xf;
+    }
     a.w = (const bf16 *)packed_weights(w, PACK_FOLD, (size_t)g.R * g.K * a.Cf * 2, g.K, g.C, g.R,
                                        g.S, Sp, Cp);
   } else {
@@ -421,6 +434,8 @@ Role step(Entry &e, bool passive) {
     graph_stop_capture();
     g_pending.out16 = false;   // who reads it is not known any more
     flush_pending();
+    for (auto &kv : rt().recs)   // nor who reads the inputs: back to their plain form
+      if (kv.second.dev_src) ensure_f32((const void *)kv.first);
     // Tensors that fusion skipped earlier in this inference stay unwritten.  The recorded
     // program had no reader for them; should this (different) program read one, that read
     // reports error 990.  A shared prefix alone - two models with the same first layers - is
@@ -447,6 +462,44 @@ void put(Entry &e, int &at, const int64_t *d, int64_t n) {
   for (int64_t i = 0; i < n && at < 24; ++i) e.args.v[at++] = d[i];
 }
 void put(Entry &e, int &at, int64_t v) { put(e, at, &v, 1); }
+
+// A device-to-device copy into tensor `rec` whose readers are convolutions of the 16-bit path: brings it in
+// in the form they take, straight from the source (the plain copy and the conversion behind it moved
+// the batch twice: 79 us of a batch-256 ResNet-50).  False when the form is not known.
+bool copy_for_conv(const float *src, float *dst, size_t bytes, TensorRec *rec) {
+  Runtime &r = rt();
+  const Entry *rd = (trace_last_flags() & RF_FOR_CONV) ? trace_last_reader() : nullptr;
+  if (!rd || r.mode == MATH_FP32) return false;
+  const int64_t *v = rd->args.v;   // dX[4], dW[4], pads[2], strides[2], groups
+  ConvGeom g;
+  memset(&g, 0, sizeof(g));
+  g.N = (int)v[0]; g.C = (int)v[1]; g.H = (int)v[2]; g.W = (int)v[3];
+  g.R = (int)v[6]; g.S = (int)v[7];
+  g.pad_w = (int)v[9]; g.stride_w = (int)v[11];
+  if ((size_t)numel4(v) * 4 != bytes) return false;
+  void *home;
+  if (g.C >= 16) {
+    home = home_acquire(bytes / 2);
+    if (!home) return false;
+    launch_nchw_f32_to_nhwc_bf16(src, (bf16 *)home, g.N, g.C, g.H, g.W, mode_f16(), r.stream);
+    mark_act16(dst, g.N, g.C, g.H, g.W, home);
+  } else {
+    if (v[12] != 1) return false;
+    g.Q = (g.W + 2 * g.pad_w - g.S) / g.stride_w + 1;
+    int Cp, Sp, Wp;
+    stem_geometry(g, Cp, Sp, Wp);
+    home = home_acquire((size_t)g.N * g.H * Wp * Cp * 2);
+    if (!home) return false;
+    launch_pad_input_bf16(src, (bf16 *)home, g.N, g.C, g.H, g.W, Wp, Cp, g.pad_w, mode_f16(), r.stream);
+    rec->fmt = FMT_STEM_ROWS;
+    rec->n = g.N; rec->c = g.C; rec->h = g.H; rec->w = g.W;
+    rec->home = home;
+    rec->stem_wp = Wp; rec->stem_cp = Cp; rec->stem_pad = g.pad_w; rec->stem_f16 = mode_f16();
+    rec->host_src = nullptr;
+  }
+  rec->dev_src = src;
+  return true;
+}
 
 // Opens every traced entry point: when the call has been carried out, a recorded stretch of calls
 // may begin or end behind it.
@@ -714,13 +767,23 @@ cudaError_t wrapDNNMemcpy(void *dst, const void *src, size_t count_, int kind,
     e.out = (uintptr_t)dst;
     e.out_bytes = (int64_t)count_;
     if (step(e, kind == 1) == R_SKIP) return cudaSuccess;
+    uintptr_t base;
     if (kind == 3) {
       pending_guard_range(dst, count_, true);
+      const TensorRec *from = reg_find(src, &base);
+      if (from && base == (uintptr_t)src && fmt_is_16(from->fmt) && !reg_find(dst) &&
+          (size_t)(from->n * from->c * from->h * from->w) * 4 == count_) {
+        // a 16-bit result on its way out: converted straight into the caller's memory
+        launch_nhwc_bf16_to_nchw_f32(act16_ptr(src), (float *)dst, (int)from->n, (int)from->c, (int)from->h,
+                                     (int)from->w, from->fmt == FMT_F16_NHWC, r.stream);
+        count(CNT_MATERIALIZE);
+        return cudaSuccess;
+      }
       ensure_f32(src);
     }
-    uintptr_t base;
     TensorRec *rec = reg_find(dst, &base);
     const bool whole = rec && base == (uintptr_t)dst && count_ + 32 > rec->bytes;
+    if (kind == 3 && whole && copy_for_conv((const float *)src, (float *)dst, count_, rec)) return cudaSuccess;
     if (rec && !whole) ensure_f32(dst);
     if (kind == 1 && whole) {
       rec->host_src = src;
@@ -776,6 +839,7 @@ cudaError_t wrapDNNMemcpy(void *dst, const void *src, size_t count_, int kind,
     if (kind == 1) count(CNT_H2D_BYTES, (int64_t)count_);
     if (rec && whole) {
       rec->fmt = FMT_F32;
+      rec->home = rec->dev_src = nullptr;
       if (kind == 3) rec->host_src = nullptr;
     }
   } else if (kind == 2) {

@@ -2,6 +2,7 @@
 #include "graph_replay.h"
 
 #include <cstring>
+#include <map>
 
 namespace occ {
 
@@ -42,6 +43,7 @@ struct Variant {
   uintptr_t pool_base = 0;
   int flags = 0;
   uint64_t epoch = 0, used = 0;
+  std::vector<SavedRec> before;   // the pool's records when the window began: the forms its inputs are in
   std::vector<Constant> constants;
   std::vector<Segment> segments;
 };
@@ -113,8 +115,26 @@ void save_registry(std::vector<SavedRec> &out, uintptr_t base, size_t bytes) {
 
 void restore_registry(const std::vector<SavedRec> &in, uintptr_t base, size_t bytes) {
   auto &recs = rt().recs;
+  std::map<uintptr_t, const void *> sources;   // this inference's, not those of the captured one
+  for (auto it = recs.lower_bound(base); it != recs.end() && it->first < base + bytes; ++it)
+    if (it->second.dev_src) sources[it->first] = it->second.dev_src;
   recs.erase(recs.lower_bound(base), recs.lower_bound(base + bytes));
-  for (const SavedRec &s : in) recs.emplace_hint(recs.end(), base + s.offset, s.rec);
+  for (const SavedRec &s : in) {
+    TensorRec rec = s.rec;
+    if (rec.dev_src) rec.dev_src = sources.count(base + s.offset) ? sources[base + s.offset] : nullptr;
+    recs.emplace(base + s.offset, rec);
+  }
+}
+
+bool same_registry(const std::vector<SavedRec> &a, uintptr_t base, size_t bytes) {
+  auto &recs = rt().recs;
+  auto it = recs.lower_bound(base);
+  for (const SavedRec &s : a) {
+    if (it == recs.end() || it->first != base + s.offset || it->second.fmt != s.rec.fmt || it->second.home != s.rec.home)
+      return false;
+    ++it;
+  }
+  return it == recs.end() || it->first >= base + bytes;
 }
 
 // ---- capture --------------------------------------------------------------------
@@ -279,7 +299,9 @@ void start_window() {
   const uintptr_t base = trace_pool_base();
   gr.left.clear();
   for (auto &v : plan.variants)
-    if (v->pool_base == base && v->flags == mode_flags() && v->epoch == gr.epoch) gr.left.push_back(v.get());
+    if (v->pool_base == base && v->flags == mode_flags() && v->epoch == gr.epoch &&
+        same_registry(v->before, base, trace_pool_bytes()))
+      gr.left.push_back(v.get());
   gr.next = plan.begin;
   gr.seg = gr.constant = 0;
   if (!gr.left.empty()) {
@@ -290,6 +312,7 @@ void start_window() {
     gr.building->pool_base = base;
     gr.building->flags = mode_flags();
     gr.building->epoch = gr.epoch;
+    save_registry(gr.building->before, base, trace_pool_bytes());
     if (!begin_segment()) {
       gr.building.reset();
       gr.state = PLAIN;

@@ -162,7 +162,7 @@ void mark_f32(void *p) {
     return;
   }
   rec->fmt = FMT_F32;
-  rec->home = nullptr;
+  rec->home = rec->dev_src = nullptr;
   rec->host_src = nullptr;
 }
 
@@ -181,6 +181,7 @@ void mark_act16(void *p, int64_t n, int64_t c, int64_t h, int64_t w, const void 
   rec->h = h;
   rec->w = w;
   rec->home = home;
+  rec->dev_src = nullptr;
   rec->host_src = nullptr;
 }
 
@@ -206,6 +207,10 @@ void ensure_f32(const void *p) {
                              r.stream));
     r.main_copies++;
     count(CNT_H2D_BYTES, (int64_t)rec->host_bytes);
+  } else if (rec->dev_src) {
+    OCC_CUDA(cudaMemcpyAsync((void *)base, rec->dev_src, (size_t)(rec->n * rec->c * rec->h * rec->w) * 4, cudaMemcpyDeviceToDevice, r.stream));
+    r.main_copies++;
+    rec->home = rec->dev_src = nullptr;
   } else if (fmt_is_16(rec->fmt)) {
     const void *tmp = rec->home;
     if (!tmp) {

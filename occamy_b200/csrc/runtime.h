@@ -27,7 +27,8 @@ enum Fmt {
   FMT_BF16_NHWC = 2,  // produced by a tensor-core-mode kernel: bf16, NHWC, dims below
   FMT_PENDING = 3,    // host->device upload deferred (constant already packed on device)
   FMT_ELIDED = 4,     // never written: a cross-call fusion skipped it (reading it is an error)
-  FMT_F16_NHWC = 5    // like FMT_BF16_NHWC with fp16 elements (MATH_F16)
+  FMT_F16_NHWC = 5,   // like FMT_BF16_NHWC with fp16 elements (MATH_F16)
+  FMT_STEM_ROWS = 6   // padded channels-last rows for a few-channel convolution, in `home`
 };
 inline bool fmt_is_16(Fmt f) { return f == FMT_BF16_NHWC || f == FMT_F16_NHWC; }
 
@@ -38,6 +39,10 @@ struct TensorRec {
   // Where a 16-bit tensor's bytes are when not at the tensor's own address (home_acquire()): its
   // address was still to be read by the kernel that wrote it, or the tensor outlives its address.
   const void *home = nullptr;
+  // Device address the tensor was copied from, when the copy brought it in in another form; the plain
+  // form is fetched from there if something asks for it after all.
+  const void *dev_src = nullptr;
+  int stem_wp = 0, stem_cp = 0, stem_pad = 0, stem_f16 = 0;   // FMT_STEM_ROWS: its geometry and element type
   const void *host_src = nullptr;      // source of the last host->device upload, if any
   size_t host_bytes = 0;
   uint64_t host_hash = 0;

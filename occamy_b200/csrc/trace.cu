@@ -90,12 +90,38 @@ bool only_matmuls_read(const std::vector<Entry> &rec, uintptr_t p, int64_t bytes
   return false;
 }
 
+// The first reader of [p, p+bytes) from entry `from` on when all readers are convolutions of the 16-bit
+// path with this tensor as their input (one only, if it has the few channels of a stem); -1 otherwise.
+int only_convs_read(const std::vector<Entry> &rec, uintptr_t p, int64_t bytes, size_t from) {
+  int first = -1;
+  for (size_t t = from; t < rec.size(); ++t) {
+    const Entry &e = rec[t];
+    for (int k = 0; k < 3; ++k) {
+      if (!e.in[k] || !overlaps(e.in[k], e.in_bytes[k] > 0 ? e.in_bytes[k] : 1, p, bytes)) continue;
+      if (k != 0 || (e.sym != S_CONV && e.sym != S_CONV_BIAS_ACT) || e.in[0] != p || !e.fusable ||
+          e.in_bytes[0] != bytes)
+        return -1;
+      const bool few = e.args.v[1] < 16;
+      if (first >= 0 && (few || rec[first].args.v[1] < 16)) return -1;
+      if (first < 0) first = (int)t;
+    }
+    if ((e.sym == S_MEMOFFSET || e.sym == S_MALLOC) && overlaps(e.out, e.out_bytes, p, bytes)) return first;
+    if ((e.sym == S_DEALLOC && e.out == p) || e.sym == S_POOLFREE) return first;
+    if (e.sym == S_OPAQUE) return -1;
+    if (e.sym != S_MEMOFFSET && e.sym != S_MALLOC && e.out && overlaps(e.out, e.out_bytes, p, bytes)) return -1;
+  }
+  return -1;
+}
+
 // Marks the chains of a finished inference: R_DEFER on the convolution, R_ABSORB on the
 // calls folded into it.
-void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles) {
+void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles, std::vector<int> &reader) {
   roles.assign(rec.size(), R_EAGER);
+  reader.assign(rec.size(), -1);
   for (size_t i = 0; i < rec.size(); ++i) {
     const Entry &c = rec[i];
+    if (c.sym == S_D2D && (reader[i] = only_convs_read(rec, c.out, c.out_bytes, i + 1)) >= 0)
+      roles[i] |= RF_FOR_CONV;
     if ((c.sym == S_REDUCE || c.sym == S_AVGPOOL || c.sym == S_MAXPOOL) && c.out != c.in[0] &&
         only_matmuls_read(rec, c.out, c.out_bytes, i + 1))
       roles[i] |= RF_FOR_MATMUL;
@@ -289,7 +315,9 @@ Role trace_step(Entry &e, bool *deviated) {
       role = (Role)(r & 0x0F);
       ts.last_flags = r & 0xF0;
       for (size_t k = 1; k < keep; ++k)
-        if (ts.programs[ts.cands[k]].roles[index] != r) {
+        if (ts.programs[ts.cands[k]].roles[index] != r ||
+            ((r & RF_FOR_CONV) && ts.programs[ts.cands[k]].sigs[ts.programs[ts.cands[k]].reader[index]] !=
+                                      ts.programs[ts.cands[0]].sigs[ts.programs[ts.cands[0]].reader[index]])) {
           role = R_EAGER;
           ts.last_flags = 0;
         }
@@ -329,7 +357,7 @@ void trace_end() {
     TraceProgram p;
     p.sigs.reserve(n);
     for (const Entry &e : ts.rec) p.sigs.push_back(e.sig);
-    analyse(ts.rec, p.roles);
+    analyse(ts.rec, p.roles, p.reader);
     p.entries.swap(ts.rec);
     p.pool_base = ts.last_pool_base;
     p.pool_bytes = ts.last_pool_bytes;
@@ -344,6 +372,12 @@ void trace_end() {
 
 // ---- prefixes made in one go (graph_replay.cu) ------------------------------------
 uint8_t trace_last_flags() { return g_ts.last_flags; }
+const Entry *trace_last_reader() {
+  TraceProgram *p = g_ts.cands.empty() ? nullptr : &g_ts.programs[g_ts.cands[0]];
+  const size_t n = trace_index();
+  if (!p || !n || n > p->reader.size() || p->reader[n - 1] < 0) return nullptr;
+  return &p->entries[p->reader[n - 1]];
+}
 bool trace_active() { return trace_enabled() && g_ts.in_inference; }
 size_t trace_index() { return g_ts.prefix_len + g_ts.rec.size(); }
 TraceProgram *trace_candidate() {

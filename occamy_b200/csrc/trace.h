@@ -77,9 +77,13 @@ struct GraphPlan;
 // flag beside a call's role: whatever reads its result is a matrix product (possibly behind a Flatten),
 // so the result may be kept in the 16-bit form that product takes
 constexpr uint8_t RF_FOR_MATMUL = 0x10;
+// on a device-to-device copy: what reads the tensor are convolutions on the 16-bit path, so the copy may
+// bring it in in their form (TraceProgram::reader names the first of them)
+constexpr uint8_t RF_FOR_CONV = 0x20;
 struct TraceProgram {
   std::vector<uint64_t> sigs;
   std::vector<uint8_t> roles;   // Role | RF_*
+  std::vector<int> reader;      // RF_FOR_CONV: call that reads the result first
   std::vector<Entry> entries;
   uintptr_t pool_base = 0;     // pool the entries' pointers refer to
   size_t pool_bytes = 0;
@@ -92,6 +96,7 @@ struct TraceProgram {
 Role trace_step(Entry &e, bool *deviated);
 
 uint8_t trace_last_flags();         // RF_* of the call trace_step() was last given
+const Entry *trace_last_reader();   // the recorded call that first reads its result (RF_FOR_CONV)
 void trace_begin();                 // cudnnCreate
 void trace_end();                   // cudnnDestroy: analyse and store if the sequence is new
 // ---- for graph_replay.cu ----

@@ -181,3 +181,58 @@ def test_ways_out_of_the_middle(native_libs):
         (y,) = m.run()
         assert np.array_equal(y, want)
     assert rt.last_error() == 0
+
+
+@pytest.mark.parametrize("c", [3, 16])
+def test_device_input_in_convolution_form(native_libs, c):
+    """A batch copied in on the device arrives in the form its convolution takes; a program with the same
+    beginning that reads it otherwise still sees the plain fp32 values."""
+    rt.set_math_mode(rt.MATH_BF16)
+    L = rt.lib()
+    r = np.random.default_rng(1)
+    w = (r.standard_normal((16, c, 3, 3)) * 0.2).astype(np.float32)
+    b = r.standard_normal(16).astype(np.float32)
+    from oracle import ref
+
+    def infer(x, conv):
+        xd = torch.from_numpy(x).cuda()
+        torch.cuda.synchronize()
+        h, pool = C.c_void_p(), C.c_void_p()
+        L.cudnnCreate(C.byref(h))
+        L.wrapDNNMemPoolInit(C.byref(pool), 1 << 20)
+        offs, at = [], 0
+        for n in (x.nbytes, w.nbytes, b.nbytes, x.shape[0] * 16 * x.shape[2] * x.shape[3] * 4):
+            offs.append(at)
+            at += (n + 31) // 32 * 32
+
+        def place(i, n):
+            p = C.c_void_p()
+            L.wrapDNNMemOffset(C.byref(p), pool, offs[i], n)
+            return p.value
+        px = place(0, x.nbytes)
+        L.wrapDNNMemcpy(px, xd.data_ptr(), x.nbytes, 3, None)
+        oshape = (x.shape[0], 16) + x.shape[2:] if conv else x.shape
+        if conv:
+            pw, pb = place(1, w.nbytes), place(2, b.nbytes)
+            L.wrapDNNMemcpy(pw, w.ctypes.data, w.nbytes, 1, None)
+            L.wrapDNNMemcpy(pb, b.ctypes.data, b.nbytes, 1, None)
+            py = place(3, int(np.prod(oshape)) * 4)
+            L.DNNConvBiasActivFunc(h, px, rt.dims(x.shape), pw, rt.dims(w.shape), pb, rt.dims((1, 16, 1, 1)), None,
+                                   0, 0, rt.dims((1, 1)), rt.dims((1, 1)), 5, py)
+        else:
+            py = place(3, x.nbytes)
+            L.DNNActiveFunc(h, px, rt.dims(x.shape), 1, py)
+        out = np.empty(oshape, np.float32)
+        L.wrapDNNMemcpy(out.ctypes.data, py, out.nbytes, 2, None)
+        L.wrapDNNDealloc(pool)
+        L.cudnnDestroy(h)
+        return out
+
+    for conv in [True] * 6 + [False, True, False] + [False] * 6 + [True, False]:
+        x = r.standard_normal((2, c, 9, 11)).astype(np.float32)
+        y = infer(x, conv)
+        if conv:
+            assert max_rel_err(y, ref.conv2d(x, w, b, (1, 1))) <= 2e-2
+        else:
+            assert np.array_equal(y, np.maximum(x, 0))
+    assert rt.last_error() == 0
