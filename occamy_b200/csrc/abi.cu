@@ -66,9 +66,9 @@ void die(const char *what, cudaError_t e, size_t size) {
   exit(-1);
 }
 
-enum PackLayout { PACK_KRSC = 1, PACK_DW = 2, PACK_FOLD = 3, PACK_RAW = 4, PACK_STEM = 5, PACK_SPLIT = 6 };
+enum PackLayout { PACK_KRSC = 1, PACK_DW = 2, PACK_FOLD = 3, PACK_RAW = 4, PACK_STEM = 5, PACK_PARTS = 6 };
 // fp32 mode: dense convolutions and GEMMs on the tensor cores with split operands (see
-// launch_split3_nchw); off with OCCAMY_FP32_TC=0 or occamy_set_fp32_tensor_cores(0), which
+// kernels_parts.cu); off with OCCAMY_FP32_TC=0 or occamy_set_fp32_tensor_cores(0), which
 // leaves the CUDA-core kernels.
 int g_fp32_tc = -1;
 }  // namespace
@@ -96,7 +96,7 @@ void *packed_weights(const float *w, int layout, size_t packed_bytes, int K, int
   TensorRec *rec = reg_find(w, &base);
   const bool cacheable = r.cache_weights && rec && base == (uintptr_t)w && rec->host_src;
   // fp32 layouts are shared by the two 16-bit modes, 16-bit ones are packed per element type
-  const bool f16 = mode_f16() && layout != PACK_DW && layout != PACK_RAW && layout != PACK_SPLIT;
+  const bool f16 = mode_f16() && layout != PACK_DW && layout != PACK_RAW && layout != PACK_PARTS;
   WeightKey key{nullptr, 0, layout * 4096 + Sp * 64 + Cp + (f16 ? (1 << 20) : 0)};
   if (cacheable) {
     key.src = rec->host_src;
@@ -133,7 +133,7 @@ void *packed_weights(const float *w, int layout, size_t packed_bytes, int K, int
   else if (layout == PACK_RAW)
     OCC_CUDA(cudaMemcpyAsync(dst, w, packed_bytes, cudaMemcpyDeviceToDevice, r.stream));
   else if (layout == PACK_STEM) launch_pack_stem_bf16(w, (bf16 *)dst, C, R, S, Cp, Sp * Cp, r.stream);
-  else if (layout == PACK_SPLIT) launch_pack_krsc_split(w, (bf16 *)dst, K, C, R, S, Cp, r.stream);
+  else if (layout == PACK_PARTS) launch_pack_split3(w, (bf16 *)dst, K, C, R, S, Sp, Cp, r.stream);
   else launch_pack_fold_bf16(w, (bf16 *)dst, K, C, R, S, Sp, Cp, f16, r.stream);
   return dst;
 }
@@ -160,7 +160,7 @@ struct ConvJob {
   bool active = false;
   bool depthwise = false;
   ConvGeom g;
-  TcConvArgs a;               // dense: tensor-core arguments (x, w, bias resolved)
+  TcConvArgs a = {};          // dense: tensor-core arguments (x, w, bias resolved)
   const bf16 *dw_x = nullptr; // depthwise
   const float *dw_w = nullptr;
   const float *bias = nullptr;
@@ -173,6 +173,8 @@ struct ConvJob {
   // a matrix product: `g` says N x K results (P = Q = 1), `a` how they are computed
   bool product = false;
   bool out16 = false;             // ... whose reader is another product: 16-bit result
+  // fp32 mode (a.split): the result goes out in three planes (FMT_PARTS), else as plain fp32
+  bool out_parts = false;
   // folded (few-channel) form: what the fused convolution + pool kernel needs besides `a`
   const bf16 *w_stem = nullptr;   // filter in that kernel's layout, packed while the filter is live
 };
@@ -301,6 +303,65 @@ bool prepare_dense(const float *x, const float *w, const float *bias, const Conv
   return true;
 }
 
+// fp32 mode on the tensor cores: x and the filter are carried as three bf16 parts each and the six part
+// products that matter are accumulated in fp32 (conv_tc_split.cu).  False when the shape is outside what
+// the kernel takes (the CUDA-core kernel runs then).
+bool parts_shape_ok(const ConvGeom &g) {
+  // Tiny problems stay on the CUDA-core kernel: the passes around this one cost more than it saves.
+  return fp32_on_tensor_cores() && g.groups == 1 && g.R * g.S <= 64 && g.stride_h <= 2 && g.stride_w <= 2 &&
+         (g.act == ACT_IDENTITY || g.act == ACT_RELU || g.act == ACT_CLIP) &&
+         (double)g.N * g.P * g.Q * g.K * g.C * g.R * g.S >= 1e6;
+}
+
+bool prepare_parts(const float *x, const float *w, const float *bias, const ConvGeom &g, ConvJob &job) {
+  Runtime &r = rt();
+  if (!parts_shape_ok(g)) return false;
+  TcConvArgs &a = job.a;
+  memset(&a, 0, sizeof(a));
+  a.N = g.N; a.H = g.H; a.K = g.K; a.P = g.P; a.Q = g.Q; a.R = g.R;
+  a.pad_h = g.pad_h; a.stride_h = g.stride_h;
+  a.act = g.act; a.lo = g.lo; a.hi = g.hi;
+  a.split = 1;
+  a.out_nchw = 1;
+  a.ldo = g.K;
+  const bool folded = g.C < 16 && g.R <= 16;
+  int Sp = 0, Cp = (g.C + 15) / 16 * 16, Wp = 0;
+  if (folded) {
+    stem_geometry(g, Cp, Sp, Wp);
+    a.W = g.Q; a.Cf = Sp * Cp; a.S = 1;
+    a.stride_w = 1;
+    a.w_step = g.stride_w * Cp;
+    a.row_elems = Wp * Cp;
+  } else {
+    a.W = g.W; a.Cf = Cp; a.S = g.S;
+    a.pad_w = g.pad_w; a.stride_w = g.stride_w;
+  }
+  a.x = a.w = (const bf16 *)16;
+  a.out_f32 = job.out;
+  if (!tc_conv_supported(a)) return false;
+  if (Cp == g.C && is_parts(x, g.N, g.C, g.H, g.W)) {
+    a.x = act16_ptr(x);
+  } else {
+    ensure_f32(x);
+    bf16 *xs = (bf16 *)scratch_get(0, (size_t)6 * g.N * g.H * (folded ? a.row_elems : g.W * Cp));
+    if (!xs) return false;
+    if (folded) launch_split3_pad(x, xs, g.N, g.C, g.H, g.W, Wp, Cp, g.pad_w, r.stream);
+    else launch_split3_nchw(x, xs, g.N, g.C, Cp, g.H, g.W, r.stream);
+    a.x = xs;
+  }
+  a.w = (const bf16 *)packed_weights(w, PACK_PARTS, (size_t)6 * a.R * a.S * g.K * a.Cf, g.K, g.C, g.R, g.S, Sp, Cp);
+  if (!a.w) return false;
+  bool ready = g_pack_was_resident;
+  a.bias = bias ? resident_f32(bias, (size_t)g.K * 4) : nullptr;
+  if (bias) ready = ready && g_pack_was_resident;
+  a.consts_ready = ready ? 1 : 0;
+  job_track_bias(job, a.bias, bias, g.K);
+  job.g = g;
+  job.bias_set = bias != nullptr;
+  job.act_set = g.act != ACT_IDENTITY;
+  return true;
+}
+
 bool prepare_depthwise(const float *x, const float *w, const float *bias, const ConvGeom &g,
                        ConvJob &job) {
   Runtime &r = rt();
@@ -352,7 +413,19 @@ void launch_job(ConvJob &job) {
   const size_t obytes = (size_t)g.N * g.K * g.P * g.Q * 2;
   const uintptr_t ohi = olo + obytes;
   void *dst = job.out;
-  if (job.product && !job.out16) {   // fp32 result, at its own address
+  job.a.act = g.act; job.a.lo = g.lo; job.a.hi = g.hi;
+  if (job.a.split && job.out_parts) {
+    g_launching = &job;
+    void *planes = home_acquire(obytes * 3);
+    g_launching = nullptr;
+    if (!planes) return;
+    job.a.y = (bf16 *)planes;
+    job.a.out_f32 = nullptr;
+    launch_tc_conv(job.a, r.stream);
+    mark_parts(job.out, g.N, g.K, g.P, g.Q, planes);
+    return;
+  }
+  if (job.a.split || (job.product && !job.out16)) {   // fp32 result, at its own address
     for (int k = 0; k < 3; k += 2) {
       if (!ranges_overlap(olo, ohi + obytes, job.dep_lo[k], job.dep_hi[k])) continue;
       const size_t bytes = job.dep_hi[k] - job.dep_lo[k];
@@ -362,10 +435,9 @@ void launch_job(ConvJob &job) {
       else job.a.x = (const bf16 *)tmp;
       count(CNT_LAUNCHES);
     }
-    job.a.act = g.act; job.a.lo = g.lo; job.a.hi = g.hi;
     job.a.out_f32 = job.out;
     job.a.ldo = g.K;
-    job.a.out_nchw = job.a.R * job.a.S > 1;   // [N][K][1][1]: the same rows
+    job.a.out_nchw = !job.product || job.a.R * job.a.S > 1;   // (a product's [N][K][1][1]: the same rows)
     launch_tc_conv(job.a, r.stream);
     mark_f32(job.out);
     return;
@@ -383,7 +455,6 @@ void launch_job(ConvJob &job) {
     launch_depthwise_bf16(job.dw_x, job.dw_w, job.bias, (bf16 *)dst, g, mode_f16(), job.a.consts_ready != 0, r.stream);
   } else {
     job.a.y = (bf16 *)dst;
-    job.a.act = g.act; job.a.lo = g.lo; job.a.hi = g.hi;
     launch_tc_conv(job.a, r.stream);
   }
   mark_act16(job.out, g.N, g.K, g.P, g.Q, dst == job.out ? nullptr : dst);
@@ -413,7 +484,8 @@ void pending_guard_range(const void *p, size_t bytes, bool writes) {
       }
   // the tensor it is going to write must also still belong to it
   const uintptr_t olo = (uintptr_t)g_pending.out;
-  const uintptr_t ohi = olo + (size_t)g_pending.g.N * g_pending.g.K * g_pending.g.P * g_pending.g.Q * 2;
+  const size_t elem = g_pending.a.split || g_pending.product ? 4 : 2;
+  const uintptr_t ohi = olo + (size_t)g_pending.g.N * g_pending.g.K * g_pending.g.P * g_pending.g.Q * elem;
   if (ranges_overlap(lo, hi, olo, ohi)) {
     if (rt().log) fprintf(stderr, "[occamy] held-back conv runs early: output re-handed out\n");
     flush_pending();
@@ -433,6 +505,7 @@ Role step(Entry &e, bool passive) {
   if (deviated) {
     graph_stop_capture();
     g_pending.out16 = false;   // who reads it is not known any more
+    g_pending.out_parts = g_pending.a.split && g_pending.res_set;
     flush_pending();
     for (auto &kv : rt().recs)   // nor who reads the inputs: back to their plain form
       if (kv.second.dev_src) ensure_f32((const void *)kv.first);
@@ -514,46 +587,6 @@ void elide(void *p) {
   trace_note_elided();
 }
 
-// fp32 mode on the tensor cores: x and the filter are carried as three bf16 parts each and the
-// six part products that matter are accumulated in fp32 (TMEM); the result is written as the
-// ABI's fp32 NCHW tensor by the kernel's epilogue.  False when the shape is outside what the
-// kernel takes (the CUDA-core kernel runs then).
-bool conv_f32_on_tensor_cores(const float *x, const float *w, const float *bias, const ConvGeom &g,
-                              float *y) {
-  Runtime &r = rt();
-  if (g.groups != 1 || g.R * g.S * 6 > 64) return false;
-  if (g.act != ACT_IDENTITY && g.act != ACT_RELU && g.act != ACT_CLIP) return false;
-  const int Cp = (g.C + 15) / 16 * 16;
-  TcConvArgs a;
-  memset(&a, 0, sizeof(a));
-  a.N = g.N; a.H = g.H; a.W = g.W; a.Cf = Cp; a.K = g.K; a.P = g.P; a.Q = g.Q; a.R = g.R; a.S = g.S;
-  a.pad_h = g.pad_h; a.pad_w = g.pad_w; a.stride_h = g.stride_h; a.stride_w = g.stride_w;
-  a.act = g.act; a.lo = g.lo; a.hi = g.hi;
-  a.split = 1;
-  a.out_f32 = y;
-  a.out_nchw = 1;
-  a.ldo = g.K;
-  a.x = (const bf16 *)16;
-  a.w = (const bf16 *)16;
-  if (!tc_conv_supported(a)) return false;
-  // Tiny problems stay on the CUDA-core kernel: three extra passes cost more than they save.
-  if ((double)g.N * g.P * g.Q * g.K * g.C * g.R * g.S < 1e6) return false;
-  ensure_f32(x);
-  bf16 *xs = (bf16 *)scratch_get(0, (size_t)3 * g.N * g.H * g.W * Cp * 2);
-  if (!xs) return false;
-  launch_split3_nchw(x, xs, g.N, g.C, Cp, g.H, g.W, r.stream);
-  const bf16 *ws = (const bf16 *)packed_weights(w, PACK_SPLIT, (size_t)6 * g.R * g.S * g.K * Cp * 2, g.K,
-                                                 g.C, g.R, g.S, 0, Cp);
-  if (!ws) return false;
-  a.x = xs;
-  a.w = ws;
-  a.bias = bias ? resident_f32(bias, (size_t)g.K * 4) : nullptr;
-  a.consts_ready = 0;
-  launch_tc_conv(a, r.stream);
-  mark_f32(y);
-  return true;
-}
-
 float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t *dW, float *bias,
                    int64_t groups, const int64_t *pads, const int64_t *strides, int act, float lo,
                    float hi, int64_t act_mode, float *y) {
@@ -590,6 +623,8 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
   e.fusable = shape_ok && r.mode != MATH_FP32 && g.P > 0 && g.Q > 0 && g.N > 0 &&
               (depthwise ? g.C % 8 == 0
                          : (g.groups == 1 && g.K % 8 == 0 && (g.C < 16 || g.C % 8 == 0)));
+  e.parts = shape_ok && r.mode == MATH_FP32 && g.P > 0 && g.Q > 0 && g.N > 0 && !depthwise && parts_shape_ok(g);
+  e.fusable = e.fusable || e.parts;
   // the fused convolution + max-pool kernel takes 64-channel stems whose column step is 16 bytes
   e.poolable = e.fusable && r.mode == MATH_BF16 && !depthwise && g.C <= 4 && g.K == 64 && g.stride_w == 2 && g.Q <= 128 &&
                g.S <= 16 && g.R <= 11;
@@ -626,7 +661,20 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
       return y;
     }
   }
-  if (r.mode == MATH_FP32 && fp32_on_tensor_cores() && conv_f32_on_tensor_cores(x, w, bias, g, y)) return y;
+  if (e.parts) {
+    ConvJob job;
+    job.out = y;
+    if (prepare_parts(x, w, bias, g, job)) {
+      job.out_parts = (trace_last_flags() & RF_FOR_PARTS) && g.K % 16 == 0;
+      if (role == R_DEFER) {
+        g_pending = job;
+        g_pending.active = true;
+      } else {
+        launch_job(job);
+      }
+      return y;
+    }
+  }
   ensure_f32(x);
   const float *wd = resident_f32(w, (size_t)numel4(dW) * 4);
   const float *bd = bias ? resident_f32(bias, (size_t)g.K * 4) : nullptr;
@@ -644,6 +692,9 @@ void pending_retarget(float *out) {
     elide(g_pending.out);
     g_pending.out = out;
   }
+  // (a residual exists in planes only, and only such results can take one along)
+  g_pending.out_parts = g_pending.a.split && !g_pending.product && g_pending.g.K % 16 == 0 &&
+                        (g_pending.res_set || (trace_last_flags() & RF_FOR_PARTS));
 }
 
 int64_t prod(const int64_t *d, int64_t rank) {
@@ -1123,7 +1174,8 @@ float *DNNTensorOpFunc(cudnnContext *, int64_t opMode, float *A, int64_t *dimA, 
     if (e.kind == CK_SAME_ADD && dims_ok && !g_pending.depthwise && !g_pending.product && !g_pending.res_set &&
         !g_pending.act_set && ((A == g_pending.out) != (B == g_pending.out))) {
       const float *other = A == g_pending.out ? B : A;
-      if (is_act16(other, g.N, g.K, g.P, g.Q)) {
+      const bool parts = g_pending.a.split && g.K % 16 == 0 && is_parts(other, g.N, g.K, g.P, g.Q);
+      if (parts || (!g_pending.a.split && is_act16(other, g.N, g.K, g.P, g.Q))) {
         g_pending.a.residual = act16_ptr(other);
         g_pending.res_set = true;
         if ((const void *)g_pending.a.residual == other) {
@@ -1229,6 +1281,15 @@ static float *pool_common(int sym, float *x, int64_t *dI, float *y, int64_t *dO,
     mark_act16(y, N, C, P, Q, home);
     return y;
   }
+  if (r.mode == MATH_FP32 && is_parts(x, N, C, H, W)) {
+    void *home = home_acquire((size_t)N * C * P * Q * 6);
+    if (home) {
+      launch_pool3(act16_ptr(x), (bf16 *)home, N, C, H, W, P, Q, (int)kernel[0], (int)kernel[1], ph, pw,
+                   (int)stride[0], (int)stride[1], avg, r.stream);
+      mark_parts(y, N, C, P, Q, home);
+      return y;
+    }
+  }
   ensure_f32(x);
   launch_pool_f32(x, y, N, C, H, W, P, Q, (int)kernel[0], (int)kernel[1], ph, pw, (int)stride[0],
                   (int)stride[1], avg, r.stream);
@@ -1276,6 +1337,12 @@ float *DNNReduceFunc(cudnnContext *, int32_t rank, float *x, int64_t *dimIn, flo
     else mark_f32(y);
     return y;
   }
+  if (r.mode == MATH_FP32 && rank == 4 && dimOut[2] == 1 && dimOut[3] == 1 && dimOut[0] == dimIn[0] &&
+      dimOut[1] == dimIn[1] && is_parts(x, dimIn[0], dimIn[1], dimIn[2], dimIn[3])) {
+    launch_gap3(act16_ptr(x), y, (int)dimIn[0], (int)(dimIn[2] * dimIn[3]), (int)dimIn[1], r.stream);
+    mark_f32(y);
+    return y;
+  }
   ensure_f32(x);
   launch_reduce_mean_f32(x, y, rank, dimIn, dimOut, r.stream);
   mark_f32(y);
@@ -1304,8 +1371,9 @@ float *CUBLASMatmul2dFunc(int64_t /*rank*/, float *A, int64_t dimA[2], float *B,
   e.in_bytes[2] = e.out_bytes;
   e.dims[0] = M; e.dims[1] = N;
   const bool out_zero = is_zero(out);
-  e.fusable = r.mode != MATH_FP32 && !transA && transB && alpha == 1.0f && (beta == 0.0f || out_zero) &&
-              K % 16 == 0 && M > 0;
+  const bool parts = r.mode == MATH_FP32;
+  e.fusable = !transA && transB && alpha == 1.0f && (beta == 0.0f || out_zero) && M > 0 &&
+              (parts ? fp32_on_tensor_cores() && (double)M * N * K >= 1e6 : K % 16 == 0);
   const Role role = step(e, false);
   if (role == R_SKIP) return out;
   if (r.log) fprintf(stderr, "[occamy] matmul2d M%d N%d K%d tA%d tB%d\n", M, N, K, (int)transA, (int)transB);
@@ -1313,14 +1381,16 @@ float *CUBLASMatmul2dFunc(int64_t /*rank*/, float *A, int64_t dimA[2], float *B,
     ConvJob job;
     TcConvArgs &a = job.a;
     memset(&a, 0, sizeof(a));
-    a.N = 1; a.H = 1; a.W = M; a.Cf = K; a.K = N; a.P = 1; a.Q = M; a.R = 1; a.S = 1;
+    const int Kp = (K + 15) / 16 * 16;
+    a.split = parts ? 1 : 0;
+    a.N = 1; a.H = 1; a.W = M; a.Cf = Kp; a.K = N; a.P = 1; a.Q = M; a.R = 1; a.S = 1;
     a.stride_h = a.stride_w = 1;
     a.act = ACT_IDENTITY;
     a.f16 = mode_f16() ? 1 : 0;
     int c = K;   // channels of A where it is an image that a Flatten passed on
     uintptr_t base = 0;
     const TensorRec *rec = reg_find(A, &base);
-    const bool image = rec && base == (uintptr_t)A && is_act16(A, rec->n, rec->c, rec->h, rec->w) && rec->n == M &&
+    const bool image = !parts && rec && base == (uintptr_t)A && is_act16(A, rec->n, rec->c, rec->h, rec->w) && rec->n == M &&
                        rec->c * rec->h * rec->w == K && rec->h * rec->w <= 64 && rec->c % 16 == 0;
     if (image && rec->h * rec->w > 1) {
       // NHWC rows against [N][c][h][w] filters: a convolution whose filter covers the whole image
@@ -1339,13 +1409,19 @@ float *CUBLASMatmul2dFunc(int64_t /*rank*/, float *A, int64_t dimA[2], float *B,
           job.dep_lo[0] = (uintptr_t)A;
           job.dep_hi[0] = (uintptr_t)A + (size_t)M * K * 2;
         }
+      } else if (parts) {
+        ensure_f32(A);
+        bf16 *as = (bf16 *)scratch_get(0, (size_t)6 * M * Kp);
+        if (as) launch_split3_rows(A, as, M, K, Kp, (int)dimA[1], r.stream);
+        a.x = as;
       } else {
         ensure_f32(A);
         bf16 *ab = (bf16 *)scratch_get(0, (size_t)M * K * 2);
         launch_f32_to_bf16(A, ab, (int64_t)M * K, mode_f16(), r.stream);
         a.x = ab;
       }
-      a.w = (const bf16 *)packed_weights(B, PACK_KRSC, (size_t)N * K * 2, N, c, a.R, a.S, 0, c);
+      a.w = (const bf16 *)(parts ? packed_weights(B, PACK_PARTS, (size_t)6 * N * Kp, N, K, 1, 1, 0, Kp)
+                                 : packed_weights(B, PACK_KRSC, (size_t)N * K * 2, N, c, a.R, a.S, 0, c));
       if (a.x && a.w) {
         a.consts_ready = g_pack_was_resident ? 1 : 0;
         a.out_f32 = nullptr;
@@ -1356,7 +1432,7 @@ float *CUBLASMatmul2dFunc(int64_t /*rank*/, float *A, int64_t dimA[2], float *B,
         g.groups = g.stride_h = g.stride_w = 1;
         g.act = ACT_IDENTITY;
         job.product = true;
-        job.out16 = (trace_last_flags() & RF_FOR_MATMUL) && N % 16 == 0;
+        job.out16 = !parts && (trace_last_flags() & RF_FOR_MATMUL) && N % 16 == 0;
         job.out = out;
         if (role == R_DEFER) {
           g_pending = job;
@@ -1364,34 +1440,6 @@ float *CUBLASMatmul2dFunc(int64_t /*rank*/, float *A, int64_t dimA[2], float *B,
           return out;
         }
         launch_job(job);
-        return out;
-      }
-    }
-  }
-  if (r.mode == MATH_FP32 && fp32_on_tensor_cores() && !transA && transB && alpha == 1.0f &&
-      (beta == 0.0f || out_zero) && M > 0 && (double)M * N * K >= 1e6) {
-    // the same split-operand scheme as the convolutions, as a 1x1 convolution over M "pixels"
-    const int Kp = (K + 15) / 16 * 16;
-    TcConvArgs a;
-    memset(&a, 0, sizeof(a));
-    a.N = 1; a.H = 1; a.W = M; a.Cf = Kp; a.K = N; a.P = 1; a.Q = M; a.R = 1; a.S = 1;
-    a.stride_h = a.stride_w = 1;
-    a.act = ACT_IDENTITY;
-    a.split = 1;
-    a.out_f32 = out;
-    a.ldo = N;
-    a.x = (const bf16 *)16;
-    a.w = (const bf16 *)16;
-    if (tc_conv_supported(a)) {
-      ensure_f32(A);
-      bf16 *as = (bf16 *)scratch_get(0, (size_t)3 * M * Kp * 2);
-      const bf16 *ws = (const bf16 *)packed_weights(B, PACK_SPLIT, (size_t)6 * N * Kp * 2, N, K, 1, 1, 0, Kp);
-      if (as && ws) {
-        launch_split3_rows(A, as, M, K, Kp, (int)dimA[1], r.stream);
-        a.x = as;
-        a.w = ws;
-        launch_tc_conv(a, r.stream);
-        mark_f32(out);
         return out;
       }
     }

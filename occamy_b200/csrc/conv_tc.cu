@@ -395,7 +395,7 @@ static int pick_bk(int Cf) {
 // Output-channel tile.  Wide tiles re-read the activations less and keep the tensor pipe
 // busier per instruction, but when a layer has few pixels they leave SMs idle; pick the
 // width with the lowest modelled time: waves x (k-steps x cost per k-step + epilogue slabs).
-static int pick_bn(int K, long sp_tiles, int ksteps, int num_sms, int widest_allowed = 256) {
+static int pick_bn(int K, long sp_tiles, int ksteps, int num_sms) {
 #ifdef OCCAMY_TUNING   // sweep builds only: force the tile width from the environment
   if (const char *f = getenv("OCCAMY_TC_BN")) {
     const int v = atoi(f);
@@ -405,7 +405,7 @@ static int pick_bn(int K, long sp_tiles, int ksteps, int num_sms, int widest_all
   const int cand[4] = {256, 128, 64, 32};
   const double kcost[4] = {900.0, 780.0, 715.0, 700.0};  // cycles per 64-deep k-step
   int widest = 32;
-  while (widest < K && widest < widest_allowed) widest *= 2;
+  while (widest < K && widest < 256) widest *= 2;
   int best = widest;
   double best_cost = -1.0;
   for (int i = 0; i < 4; ++i) {
@@ -428,9 +428,9 @@ bool tc_conv_supported(const TcConvArgs &a) {
   if (a.act != ACT_IDENTITY && a.act != ACT_RELU && a.act != ACT_CLIP) return false;
   if (a.stride_h < 1 || a.stride_w < 1 || a.stride_h > 2 || a.stride_w > 2) return false;
   if (a.w_step && ((a.w_step * 2) % 16 || (a.row_elems * 2) % 16 || a.S != 1)) return false;
-  if (a.R * a.S * (a.split ? 6 : 1) > TC_MAX_TAPS) return false;
+  if (a.R * a.S > TC_MAX_TAPS) return false;
   if (!a.out_f32 && a.K % 8 != 0) return false;
-  if (a.split && (!a.out_f32 || a.w_step || a.f16)) return false;
+  if (a.split && (a.f16 || a.pad_h > 64 || a.pad_w > 64)) return false;
   if (a.out_f32 && a.residual) return false;
   // the row-major fp32 output is indexed by the flattened pixel number (plain GEMM view only)
   if (a.out_f32 && !a.out_nchw && !(a.R == 1 && a.S == 1 && a.stride_h == 1 && a.stride_w == 1 &&
@@ -439,7 +439,7 @@ bool tc_conv_supported(const TcConvArgs &a) {
   if ((uintptr_t)a.x % 16 || (uintptr_t)a.w % 16) return false;
   if (a.y && (uintptr_t)a.y % 16) return false;
   if ((int64_t)a.N * a.P * a.Q >= (1ll << 31)) return false;
-  if (a.K > 4096) return false;   // the bias vector has to fit in shared memory
+  if (a.K > 4096 && !a.split) return false;   // the bias vector has to fit in shared memory
   return true;
 }
 
@@ -502,9 +502,8 @@ static int floordiv(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b);
 // Tensor maps of the A operand and the list of filter taps that read through them.
 static bool make_operand_maps(const TcConvArgs &a, bool flat, int Qg, int bk, const uint32_t *boxA,
                               CUtensorMap *tmA, TcTap *taps, int *num_taps, bool counted) {
-  const int parts = a.split ? 3 : 1, combos = a.split ? 6 : 1;
-  static const int a_part[6] = {0, 0, 0, 1, 1, 2};
-  const int64_t plane = (int64_t)a.N * a.H * a.W * a.Cf;   // elements of one activation part
+  const int parts = sk_parts(a.split != 0);   // fp32 operands: three planes, as many maps next to one another
+  const int64_t plane = (int64_t)a.N * a.H * (a.row_elems ? a.row_elems : a.W * a.Cf);
   bool ok = true;
   *num_taps = 0;
   if (flat) {
@@ -512,7 +511,7 @@ static bool make_operand_maps(const TcConvArgs &a, bool flat, int Qg, int bk, co
     const uint64_t st[3] = {(uint64_t)a.Cf * 2, (uint64_t)Qg * a.Cf * 2, (uint64_t)Qg * a.Cf * 2};
     for (int part = 0; part < parts; ++part)
       ok &= make_map(&tmA[part], a.x + part * plane, 4, dims, st, boxA, bk * 2, counted);
-    for (int j = 0; j < combos; ++j) taps[(*num_taps)++] = TcTap{a.split ? a_part[j] : 0, 0, 0};
+    taps[(*num_taps)++] = TcTap{0, 0, 0};
     return ok;
   }
   // one tensor map per (row phase, column phase) of the stride
@@ -535,13 +534,11 @@ static bool make_operand_maps(const TcConvArgs &a, bool flat, int Qg, int bk, co
                                   (uint64_t)(Hm > 0 ? Hm : 1), (uint64_t)a.N};
         const uint64_t st[3] = {(uint64_t)(sw * px * 2), (uint64_t)(sh * rowe * 2),
                                 (uint64_t)(a.H * rowe * 2)};
-        // the maps of one stride phase, one per operand part, sit next to one another
         for (int part = 0; part < parts; ++part)
           ok &= make_map(&tmA[nmaps * parts + part], ptr + part * plane, 4, dims, st, boxA, bk * 2, counted);
         map_of[bh][bw] = nmaps++;
       }
-      for (int j = 0; j < combos; ++j)
-        taps[(*num_taps)++] = TcTap{map_of[bh][bw] * parts + (a.split ? a_part[j] : 0), aw, ah};
+      taps[(*num_taps)++] = TcTap{map_of[bh][bw] * parts, aw, ah};
     }
   return ok;
 }
@@ -572,6 +569,10 @@ static int sk_pick_issuers(const TcConvArgs &a, int bn, int share) {
 //   k-steps   the tensor pipe (four MMAs of 48.5 cycles up to 64 channels, of 64 at 128) plus what the
 //             L2 adds with many CTAs reading
 //   cluster   launching clusters and exchanging partial sums, by the number of CTAs
+// Split operands: any number of waves, for this is their only kernel.  The products of a 32-deep k-step
+// are 12 MMAs' worth, 768 cycles at 128 channels; shared memory, which delivers the operands and takes in
+// the next ones, is what bounds it at 900 to 1100.  ResNet-50, batch 16, fp32: 2.59 -> 1.47 ms against
+// six k-steps of one part product each on the persistent kernel, with results in fp32 between the layers.
 // The fixed part was 0.8 us longer before the epilogue's code was fetched ahead of time, the exchange
 // 0.7 us longer with a cluster barrier behind plain remote stores.
 static SkChoice sk_choose(const TcConvArgs &a, long sp_tiles, int rows, int ksteps, int bk, int a_bytes, int nsm) {
@@ -582,7 +583,7 @@ static SkChoice sk_choose(const TcConvArgs &a, long sp_tiles, int rows, int kste
     if (const char *f = getenv("OCCAMY_SK_BN")) if (atoi(f) != bn) continue;
 #endif
     const long tiles = sp_tiles * ((a.K + bn - 1) / bn);
-    const int stage_bytes = a_bytes + bn * bk * 2;
+    const int stage_bytes = sk_parts(a.split != 0) * (a_bytes + bn * bk * 2);
     for (int s = 1; s <= (a.w_step ? 1 : SK_MAX_SPLITS) && s <= ksteps; ++s) {
       // (clusters of more than two leave some SMs of every GPC without a partner)
       long most = s <= 2 ? nsm : nsm - nsm / 9;
@@ -591,7 +592,7 @@ static SkChoice sk_choose(const TcConvArgs &a, long sp_tiles, int rows, int kste
       if (getenv("OCCAMY_SK_S")) most = 2 * nsm;
 #endif
       const long ctas = tiles * s;
-      if (ctas > most) break;
+      if (ctas > most && !(a.split && s == 1)) break;
       const int rows_owner = (rows + s - 1) / s;
       const int share = (ksteps + s - 1) / s;
       const int issuers = sk_pick_issuers(a, bn, share);
@@ -599,22 +600,26 @@ static SkChoice sk_choose(const TcConvArgs &a, long sp_tiles, int rows, int kste
       // stages (or all of a CTA's k-steps) is worth more than that: 256->256 3x3 at 14x14, batch 8,
       // 10.0 us with four stages, 7.4 us with eight.
       int stages = 0;
-      const size_t fixed = sk_smem_bytes(bn, 0, a_bytes, bk, s, rows_owner) + 16 * SK_MAX_STAGES;
+      const size_t fixed = sk_smem_bytes(bn, 0, a_bytes, bk, s, rows_owner, a.split != 0) + 16 * SK_MAX_STAGES;
       for (size_t limit : {TC_SMEM_DUO - 1024, (size_t)TC_SMEM_LIMIT}) {
         stages = fixed < limit ? (int)((limit - fixed) / stage_bytes) : 0;
         if (stages > SK_MAX_STAGES) stages = SK_MAX_STAGES;
         if (stages >= share) stages = share;
         else stages = stages / issuers * issuers;
         if (stages >= 8 || stages == share) break;
+        if (ctas > nsm && stages >= 2) break;   // two to an SM, one's end behind the other's products
       }
       if (stages < 1) continue;
-      const double n = (double)ctas;
+      const double n = (double)(ctas < nsm ? ctas : nsm);
       double step = bn == 32 ? 0.085 + 0.00008 * n : bn == 64 ? 0.105 + 0.00027 * n : 0.16 + 0.0004 * n;
       step *= bk == 64 ? 1.0 : 0.75;
       if (issuers < 2 && share > 1) step += 0.12;
+      if (a.split) step = (bn == 128 ? 0.43 : 0.32) * (bk == 32 ? 1.0 : 0.5);   // the tensor pipe
       const double fixed_us = bn == 32 ? 2.35 + 0.006 * n : bn == 64 ? 3.05 + 0.008 * n : 3.7 + 0.008 * n;
       const double exchange = 0.52 + n * (0.0104 + 0.013 * rows / 128.0) + (bn == 128 ? 3.25 : 0.0);
-      const double cost = fixed_us + share * step + (s > 1 ? exchange : 0.0);
+      const double waves = (double)((ctas + nsm - 1) / nsm);   // more than one: split operands only
+      const double cost = a.split ? fixed_us + waves * (share * step + 0.6) + (s > 1 ? exchange : 0.0)
+                                  : fixed_us + share * step + (s > 1 ? exchange : 0.0);
       if (best.cost < 0 || cost < best.cost) best = SkChoice{bn, s, stages, cost};
     }
   }
@@ -628,7 +633,8 @@ static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, d
 #endif
   const bool flat = a.R == 1 && a.S == 1 && a.stride_h == 1 && a.stride_w == 1 && a.pad_h == 0 &&
                     a.pad_w == 0 && a.w_step == 0;
-  const int bk = pick_bk(a.Cf);
+  // (split operands: six tiles per stage, so half as deep; twice as deep is 5 to 9 % slower, one CTA to an SM)
+  const int bk = a.split ? (a.Cf > 16 ? 32 : 16) : pick_bk(a.Cf);
   int Qg = a.Q, Pg = a.P, Ng = a.N;
   if (flat) {
     Qg = a.N * a.P * a.Q;
@@ -642,7 +648,7 @@ static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, d
   p.rows = p.tw * p.th * p.tn;
   p.bk = bk;
   p.cblocks = (a.Cf + bk - 1) / bk;
-  p.ksteps = a.R * a.S * (a.split ? 6 : 1) * p.cblocks;
+  p.ksteps = a.R * a.S * p.cblocks;
   p.a_bytes = ((p.rows + 7) / 8 * 8 * bk * 2 + 1023) / 1024 * 1024;
   const SkChoice c = sk_choose(a, sp_tiles, p.rows, p.ksteps, bk, p.a_bytes, nsm);
   if (c.cost < 0) return false;
@@ -666,6 +672,7 @@ static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, d
   p.bias = a.bias;
   p.residual = a.residual;
   p.y = a.y;
+  p.plane = (int64_t)a.N * a.P * a.Q * a.K;
   p.out_f32 = a.out_f32;
   p.ldo = a.ldo;
   p.out_hw = a.out_f32 && a.out_nchw ? a.P * a.Q : 0;
@@ -682,7 +689,7 @@ static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, d
     if (abs(taps[t].dw) > 127 || abs(taps[t].dh) > 127) return false;
     p.taps[t] = SkTap{(int8_t)taps[t].map, (int8_t)taps[t].dw, (int8_t)taps[t].dh, 0};
   }
-  const uint64_t dims[3] = {(uint64_t)a.Cf, (uint64_t)a.K, (uint64_t)num_taps};
+  const uint64_t dims[3] = {(uint64_t)a.Cf, (uint64_t)a.K, (uint64_t)num_taps * sk_parts(a.split != 0)};
   const uint64_t st[2] = {(uint64_t)a.Cf * 2, (uint64_t)a.K * a.Cf * 2};
   const uint32_t box[3] = {(uint32_t)bk, (uint32_t)bn, 1};
   ok &= make_map(&p.tmB, a.w, 3, dims, st, box, bk * 2, counted);
@@ -692,9 +699,9 @@ static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, d
   pl->split = a.split != 0;
   pl->bn = bn;
   pl->p.total_tiles = (int)sp_tiles * p.tiles_k;
-  pl->smem = sk_smem_bytes(bn, p.stages, p.a_bytes, bk, p.splits, p.rows_owner);
-  // the MMA reads 128 rows from the start of every activation stage
-  const size_t reach = (size_t)(p.stages - 1) * p.a_bytes + 128 * bk * 2;
+  pl->smem = sk_smem_bytes(bn, p.stages, p.a_bytes, bk, p.splits, p.rows_owner, a.split != 0);
+  // the MMA reads 128 rows from the start of every activation tile
+  const size_t reach = (size_t)(p.stages * sk_parts(a.split != 0) - 1) * p.a_bytes + 128 * bk * 2;
   if (pl->smem < reach) pl->smem = reach;
   pl->ok = true;
 #ifdef OCCAMY_TUNING
@@ -710,6 +717,10 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   Plan pl;
   memset(&pl, 0, sizeof(pl));
   TcParams &p = pl.p;
+  if (a.split) {
+    sk_plan(a, err_word, num_sms > 0 ? num_sms : 148, counted, -1.0, &pl);
+    return pl;
+  }
   const int bk = pick_bk(a.Cf);
   p.bk = bk;
   p.cblocks = (a.Cf + bk - 1) / bk;
@@ -722,8 +733,6 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   p.out_f32 = a.out_f32;
   p.ldo = a.ldo;
   p.out_hw = a.out_f32 && a.out_nchw ? a.P * a.Q : 0;
-  // fp32 operands as three bf16 parts: six (activation part, filter part) products per tap
-  const int combos = a.split ? 6 : 1;
   p.err = err_word;
 #ifdef OCCAMY_TC_TIMERS
   p.timers = tc_timer_words();
@@ -752,7 +761,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   // than the plain one, which hurts the HBM-bound 1x1 layers
   // 3x3 / stride 1 / pad 1 with 64 -> 64 channels and rows of at most 126 pixels: the input
   // block of a tile is loaded once and the taps are windows of it (TC_MODE_HALO)
-  const bool halo = allow_halo && halo_allowed && !a.f16 && !a.split && !a.out_f32 && a.R == 3 && a.S == 3 &&
+  const bool halo = allow_halo && halo_allowed && !a.f16 && !a.out_f32 && a.R == 3 && a.S == 3 &&
                     a.stride_h == 1 && a.stride_w == 1 && a.pad_h == 1 && a.pad_w == 1 &&
                     a.Cf == 64 && a.K == 64 && a.W + 2 <= 128 && a.w_step == 0 && a.Q == a.W &&
                     a.P == a.H;
@@ -777,7 +786,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   const int bn = pn ? 128
                     : halo ? 64
                     : pick_bn(a.K, (long)p.tiles_w * p.tiles_h * p.tiles_n,
-                              (a.R * a.S * combos * a.Cf + 63) / 64, nsm, a.split ? 128 : 256);
+                              (a.R * a.S * a.Cf + 63) / 64, nsm);
   pl.bn = bn;
   p.tiles_k = (a.K + bn - 1) / bn;
   p.sp_tiles = p.tiles_w * p.tiles_h * p.tiles_n;
@@ -809,7 +818,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
     // whose tiles are twice as tall; a whole tile of the halo form takes 0.9 us).
     const int per_wave = pair ? nsm / 2 : nsm;
     const double waves = (double)((p.total_tiles + per_wave - 1) / per_wave);
-    const int ks = p.cblocks * a.R * a.S * combos;
+    const int ks = p.cblocks * a.R * a.S;
     const double tile_us = halo ? 0.9 : pn ? 0.49 * ks : (bn == 256 ? 0.1 : 0.0) + 0.27 * ks * (bk == 64 ? 1.0 : 0.75);
     if (sk_plan(a, err_word, nsm, counted, 3.1 + waves * tile_us, &pl)) return pl;
   }
@@ -825,14 +834,14 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
     ok &= make_operand_maps(a, flat, Qg, bk, boxA, p.tmA, p.taps, &p.num_taps, counted);
   }
   {
-    const uint64_t dims[3] = {(uint64_t)a.Cf, (uint64_t)a.K, (uint64_t)(a.R * a.S * combos)};
+    const uint64_t dims[3] = {(uint64_t)a.Cf, (uint64_t)a.K, (uint64_t)(a.R * a.S)};
     const uint64_t st[2] = {(uint64_t)a.Cf * 2, (uint64_t)a.K * a.Cf * 2};
     const uint32_t box[3] = {(uint32_t)bk, (uint32_t)(pair ? bn / 2 : bn), 1};
     ok &= make_map(&p.tmB, a.w, 3, dims, st, box, bk * 2, counted);
   }
   // For 256-wide tiles with a long reduction, 32-channel slabs free enough shared memory
   // for a fourth ring stage, which those layers need more than a cheap epilogue.
-  const int ksteps64 = (a.R * a.S * combos * a.Cf + 63) / 64;
+  const int ksteps64 = (a.R * a.S * a.Cf + 63) / 64;
   int dc = pn ? 64 : (bn < 64 ? bn : (bn == 256 && bk == 64 && ksteps64 >= 16 ? 32 : 64));
   if (a.out_f32 && bn >= 64) dc = 64;   // the fp32-output flavour is compiled for 64-channel slabs
 #ifdef OCCAMY_TUNING
@@ -845,7 +854,6 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
                          (halo ? TC_MODE_HALO : 0));
   if (a.f16) pl.mode |= TC_MODE_F16;
   if (pair) pl.mode |= TC_MODE_PAIR;
-  if (a.split) pl.mode |= TC_MODE_SPLIT;
   if (!a.out_f32) {
     const uint64_t dims[4] = {(uint64_t)a.K, (uint64_t)Qg, (uint64_t)Pg, (uint64_t)Ng};
     const uint64_t st[3] = {(uint64_t)a.K * 2, (uint64_t)Qg * a.K * 2, (uint64_t)Pg * Qg * a.K * 2};
@@ -862,7 +870,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   const size_t b_tile_bytes = (size_t)(pair ? bn / 2 : bn) * bk * 2;
   // (With two CTAs per SM the single loading thread of a CTA is what the others wait for, and
   // weights of up to 16 KB pay as well: 144->24 at 56x56 has nine k-steps of 1 KB each.)
-  const bool duo_wanted = !pn && !halo && !pair && !a.split && !a.out_f32 && dc == 32 && bn == 32 && nsm >= 2;
+  const bool duo_wanted = !pn && !halo && !pair && !a.out_f32 && dc == 32 && bn == 32 && nsm >= 2;
   bool bres = !pn && !halo && !pair && p.tiles_k == 1 &&
               ksteps_tile * b_tile_bytes <= (size_t)(duo_wanted ? 16 : 4) * 1024;
 #ifdef OCCAMY_TUNING
@@ -888,7 +896,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   bool duo = duo_wanted;
 #ifdef OCCAMY_TUNING
   if (const char *f = getenv("OCCAMY_TC_DUO"))
-    duo = atoi(f) != 0 && !pn && !halo && !pair && !a.split && !a.out_f32 && dc == 32 && bn == 32;
+    duo = atoi(f) != 0 && !pn && !halo && !pair && !a.out_f32 && dc == 32 && bn == 32;
 #endif
   int dbuf = 0, pend = 0, stages = 0;
   for (;; duo = false) {

@@ -116,12 +116,6 @@ constexpr int TC_MODE_F16 = 16;
 // flop of the single-CTA form, which is what bounds the long-reduction layers.  No multicast
 // load is involved: every TMA load has one destination.
 constexpr int TC_MODE_PAIR = 32;
-// fp32 operands carried as bf16 parts (six taps per filter tap, see the planner): the hi * hi
-// products go into one accumulator and the five correction products into a second one, which
-// the epilogue adds.  The tensor core truncates when it adds into an fp32 accumulator, a bias
-// toward zero that grows with the number of additions at full magnitude; kept apart, the small
-// terms cost the main sum no additions (and their own truncation is 2^-8 smaller).
-constexpr int TC_MODE_SPLIT = 64;
 
 // ------------------------------------------------------------------ PTX wrappers
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -512,10 +506,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
   constexpr bool HALO = (MODE & TC_MODE_HALO) != 0;
   constexpr bool F16 = (MODE & TC_MODE_F16) != 0;
   constexpr bool PAIR = (MODE & TC_MODE_PAIR) != 0;
-  constexpr bool SPLIT = (MODE & TC_MODE_SPLIT) != 0;
   static_assert(!(PAIR && (HALO || F32)), "the CTA-pair form exists for the plain epilogues only");
-  static_assert(!SPLIT || (F32 && !HALO && BN <= 128), "split operands: fp32 output, four accumulators");
-  constexpr int ACC_COLS = SPLIT ? 2 * BN : BN;   // TMEM columns of one tile's accumulator(s)
   constexpr int EPI_THREADS = 128 * EW;
   constexpr int STORE_WARP = 2 + 4 * EW;
   constexpr int CW = DC / EW;                  // channels one epilogue thread handles per slab
@@ -524,7 +515,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
   // fp32 accumulator; A and B formats: 1 = bf16, 0 = fp16; N / 8 and M / 16
   constexpr uint32_t IDESC = (1u << 4) | (F16 ? 0u : ((1u << 7) | (1u << 10))) |
                              ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((PAIR ? 256 : 128) >> 4) << 24);
-  constexpr uint32_t TMEM_COLS = 2 * ACC_COLS < 32 ? 32 : 2 * ACC_COLS;
+  constexpr uint32_t TMEM_COLS = 2 * BN < 32 ? 32 : 2 * BN;
   constexpr int BROWS = PAIR ? BN / 2 : BN;    // rows of the B tile this CTA loads
 
   // The swizzled operand tiles need 1024-byte alignment.  The kernel has no static shared
@@ -816,11 +807,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
               return;
             }
             tc_fence_after();
-            const uint32_t d_tmem = tmem_base + (uint32_t)(acc * ACC_COLS);
-            // split operands: tap 0 of every group of six is hi * hi and goes to the main
-            // accumulator, the other five (corrections) to the second one
-            uint32_t seen_main = 0, seen_corr = 0;
-            int cb_in_tap = 0, combo = 0;
+            const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
             for (int ks = 0; ks < ksteps; ++ks) {
               if (!TCT_WAIT(1, mbar_wait_hot(full_bar(stage), phase, abort_flag))) {
                 err_code = 3;
@@ -828,20 +815,6 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
               }
               tc_fence_after();
               const uint32_t bl = bres ? b_lo0 + (uint32_t)ks * b_step : b_lo;
-              if constexpr (SPLIT) {
-                const bool corr = combo != 0;
-                const uint32_t d = corr ? d_tmem + (uint32_t)BN : d_tmem;
-                const uint32_t first = corr ? seen_corr : seen_main;
-#pragma unroll
-                for (int kk = 0; kk < NK; ++kk)
-                  mma_lohi(d, a_lo + 2u * kk, a_hi, bl + 2u * kk, b_hi, IDESC, kk ? 1u : first);
-                if (corr) seen_corr = 1u;
-                else seen_main = 1u;
-                if (++cb_in_tap == p.cblocks) {
-                  cb_in_tap = 0;
-                  if (++combo == 6) combo = 0;
-                }
-              } else {
 #pragma unroll
                 for (int kk = 0; kk < NK; ++kk) {
                   const uint32_t accumulate = kk ? 1u : (uint32_t)(ks != 0);
@@ -850,7 +823,6 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
                   else
                     mma_lohi(d_tmem, a_lo + 2u * kk, a_hi, bl + 2u * kk, b_hi, IDESC, accumulate);
                 }
-              }
               if constexpr (PAIR) tc_commit_pair(empty_bar(stage));   // frees the stage in both CTAs
               else tc_commit(empty_bar(stage));
               a_lo += a_step;
@@ -1062,7 +1034,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
       }
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) +
-                             (uint32_t)(acc * ACC_COLS + part * CW);
+                             (uint32_t)(acc * BN + part * CW);
       // every TMEM read of this tile has landed: the MMA warp may overwrite the buffer
       auto release_acc = [&]() {
         tc_fence_before();
@@ -1160,20 +1132,6 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
       // worked on and the loop body (two slabs) stays small.
       uint32_t ra[CW], rb[CW];
       bool ok = true;
-      if constexpr (SPLIT) {
-        // main and correction accumulators of a slab are read together and added here
-#pragma unroll 1
-        for (int sl = 0; sl < nslab && ok; ++sl) {
-          tc_ld<CW>(t_row + (uint32_t)(sl * DC), ra);
-          tc_ld<CW>(t_row + (uint32_t)(BN + sl * DC), rb);
-          tc_ld_wait();
-          if (sl + 1 == nslab) release_acc();
-#pragma unroll
-          for (int j = 0; j < CW; ++j)
-            ra[j] = __float_as_uint(__uint_as_float(ra[j]) + __uint_as_float(rb[j]));
-          ok = slab(ra, sl);
-        }
-      } else {
       tc_ld<CW>(t_row, ra);
 #pragma unroll 1
       for (int sl = 0; sl < nslab && ok; sl += 2) {
@@ -1187,7 +1145,6 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
           else release_acc();
           ok = slab(rb, sl + 1);
         }
-      }
       }
       if (!ok) {
         err_code = 5;
@@ -1324,12 +1281,6 @@ inline bool tc_launch_mode(const TcParams &p, int mode, int grid, size_t smem, c
         tc_launch_one<BN, DC, P2 | H2 | TC_MODE_RES | TC_MODE_CLAMP>(p, grid, smem, s);
         return true;
       default: break;
-    }
-  }
-  if constexpr (WITH_F32 && BN <= 128) {
-    if (mode == (TC_MODE_SPLIT | TC_MODE_F32 | TC_MODE_CLAMP)) {
-      tc_launch_one<BN, DC, TC_MODE_SPLIT | TC_MODE_F32 | TC_MODE_CLAMP>(p, grid, smem, s);
-      return true;
     }
   }
   constexpr int H = TC_MODE_F16;

@@ -47,6 +47,12 @@ __device__ __forceinline__ void st_async_v4_if(bool on, uint32_t addr, uint32_t 
       "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar), "r"((uint32_t)on)
       : "memory");
 }
+__device__ __forceinline__ void st_shared_v4_if(bool on, uint32_t addr, uint32_t a, uint32_t b, uint32_t c,
+                                                uint32_t d) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %5, 0;\n@p st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n}" ::"r"(addr),
+               "r"(a), "r"(b), "r"(c), "r"(d), "r"((uint32_t)on)
+               : "memory");
+}
 __device__ __forceinline__ void st_global_v4_if(bool on, void *addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %5, 0;\n@p st.global.v4.b32 [%0], {%1, %2, %3, %4};\n}" ::"l"(addr),
                "r"(a), "r"(b), "r"(c), "r"(d), "r"((uint32_t)on)
@@ -97,23 +103,61 @@ __device__ __forceinline__ void sk_finish32(const SkParams &p, bool on, float *v
   }
 }
 
+// The same for three-part output: the residual's parts add up to its fp32 value exactly, the result is
+// cut into parts again.
+__device__ __forceinline__ void sk_finish_parts(const SkParams &p, bool on, float *v, const uint4 *r, int64_t lin,
+                                                int c) {
+  const int64_t at = lin * p.K + c;
+  if (p.residual) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float a[3], b[3];
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        f2_unpack(pair16_to_f2<false>(e == 0 ? r[j].x : e == 1 ? r[j].y : e == 2 ? r[j].z : r[j].w), a[j], b[j]);
+      v[2 * e] += (a[0] + a[1]) + a[2];
+      v[2 * e + 1] += (b[0] + b[1]) + b[2];
+    }
+  }
+  uint32_t o[3][4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float a = tc_act(v[2 * e], p.lo, p.hi), b = tc_act(v[2 * e + 1], p.lo, p.hi);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      o[j][e] = f2_to_bf16x2<false>(f2_pack(a, b));
+      const float ta = __uint_as_float(o[j][e] << 16), tb = __uint_as_float(o[j][e] & 0xffff0000u);
+      a = fabsf(ta) < INFINITY ? a - ta : 0.0f;   // exact: what the part left over
+      b = fabsf(tb) < INFINITY ? b - tb : 0.0f;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+    st_global_v4_if(on, reinterpret_cast<uint16_t *>(p.y) + j * p.plane + at, o[j][0], o[j][1], o[j][2], o[j][3]);
+}
+
 }  // namespace
 
 //   BN     output channels of a tile (N of the MMA)
 //   F16    operands and 16-bit output are fp16, else bf16
-//   SPLIT  fp32 operands carried as bf16 parts: tap 0 of every six goes to the main accumulator, the
-//          five correction products to a second one
+//   SPLIT  fp32 operands carried as three bf16 parts hi + mid + lo (24 mantissa bits).  A product is the
+//          sum of six part products (the three left out are below 2^-24 of it), each exact in fp32:
+//          hi*hi goes to the main accumulator, hi*mid, hi*lo, mid*hi, mid*mid, lo*hi to others (one more
+//          at 128 channels, else two, so that an activation part meets its filter parts in one MMA).
+//          The tensor core truncates when it adds into an fp32 accumulator, a bias toward zero that
+//          grows with the number of additions at full magnitude; kept apart, the small terms cost the
+//          main sum none.  A stage holds the three parts of either operand once for all six products.
 //   CL     a tile has more than one CTA
-//   F32    fp32 output
+//   F32    fp32 output (else 16-bit values; with SPLIT the three parts of fp32 ones)
 // One flavour per instantiation: these kernels run for a few microseconds, and every stretch of code
 // that is not in the instruction cache yet costs a tenth of that.
 template <int BN, bool F16, bool SPLIT, bool CL, bool F32>
 __global__ void __launch_bounds__(SK_THREADS, 2)
     tc_split_kernel(const __grid_constant__ SkParams p) {
-  constexpr uint32_t IDESC = (1u << 4) | (F16 ? 0u : ((1u << 7) | (1u << 10))) |
-                             ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+  constexpr uint32_t IDESC0 = (1u << 4) | (F16 ? 0u : ((1u << 7) | (1u << 10))) | ((uint32_t)(128 >> 4) << 24);
+  constexpr uint32_t NSHIFT = 17 - 3;   // of N in the instruction descriptor
   constexpr int NI = sk_issuers(BN, SPLIT);
-  constexpr int NACC = NI * (SPLIT ? 2 : 1);                       // accumulators: issuer x (main, correction)
+  constexpr int NACC = SPLIT ? (BN == 128 ? 2 : 3) : NI;           // accumulators
   static_assert(NACC * BN <= 256, "two CTAs share the 512 TMEM columns of an SM");
   constexpr int HALF = BN / 2;          // columns of one epilogue thread
   constexpr int G8 = BN / 8;            // eight-channel groups of a tile row
@@ -124,10 +168,17 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
     return;
   }
   const int stages = p.stages, bk = p.bk, splits = CL ? p.splits : 1;
-  const uint32_t a_bytes = (uint32_t)p.a_bytes, b_bytes = (uint32_t)BN * bk * 2u;
-  const uint32_t sA = smem_u32(smem_raw), sB = sA + stages * a_bytes, sX = sB + stages * b_bytes;
-  const uint32_t x_bytes = CL ? (uint32_t)(splits * p.rows_owner) * BN * 4u : 0u;   // partial sums
-  uint8_t *misc = smem_raw + (sX + x_bytes - sA);
+  constexpr int PARTS = sk_parts(SPLIT);
+  // Sums that pass through shared memory, so that neighbouring threads finish neighbouring channels: those
+  // of a cluster, and results in three planes, whose 16-byte pieces written row by row cost twice the
+  // products' time (256->1024 at 14x14, batch 16, with residual: 36.8 us, this way 22.6).
+  constexpr bool ITEMS = CL || (SPLIT && !F32);
+  const uint32_t a_tile = (uint32_t)p.a_bytes, b_tile = (uint32_t)BN * bk * 2u;
+  const uint32_t a_bytes = PARTS * a_tile, b_bytes = PARTS * b_tile;   // of a stage
+  const uint32_t sA = smem_u32(smem_raw), sB = sA + stages * a_bytes;
+  // partial sums: behind the ring, or (of one CTA) where the ring was
+  const uint32_t sX = CL ? sB + stages * b_bytes : sA, x_bytes = ITEMS ? (uint32_t)(splits * p.rows_owner) * BN * 4u : 0u;
+  uint8_t *misc = smem_raw + max(sX + x_bytes - sA, stages * (a_bytes + b_bytes));
   float *bias_s = reinterpret_cast<float *>(misc);                       // BN floats
   int *lin_s = reinterpret_cast<int *>(misc + BN * 4);                   // 128 pixel numbers, -1: none
   uint64_t *bars = reinterpret_cast<uint64_t *>(misc + BN * 4 + 512);
@@ -137,14 +188,14 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   const uint32_t done_bar = bar0 + 16u * stages, sums_bar = done_bar + 8u;
   volatile uint32_t *tmem_holder = reinterpret_cast<volatile uint32_t *>(bars + 2 * stages + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 2 * stages + 3);
-  // which accumulators hold anything, one word per issuer: bit 0 main, bit 1 correction
+  // which accumulators hold anything, one word per issuer
   volatile int *used = reinterpret_cast<volatile int *>(bars + 2 * stages + 4);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Fewer accumulators when there are fewer k-steps: CTAs of the next layer that share this SM need
   // TMEM columns as well.  A power of two.
   const int ni = p.issuers;
-  const uint32_t cols = (uint32_t)(ni == 3 ? 4 : ni) * (SPLIT ? 2u : 1u) * BN;
+  const uint32_t cols = SPLIT ? (BN == 128 ? 256u : 4u * BN) : (uint32_t)(ni == 3 ? 4 : ni) * BN;
   const int rank = CL ? (int)cluster_ctarank() : 0;
   const int tile = (int)blockIdx.x / splits;
   // channel tiles fastest, then columns, rows and images of the pixel grid
@@ -196,19 +247,24 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   if constexpr (CL) cluster_arrive_release();   // waited for before the first remote store
   tc_fence_after();
   const uint32_t tmem = *tmem_holder;
-  const uint32_t tx_bytes = (uint32_t)p.rows * bk * 2u + b_bytes;
+  const uint32_t tx_bytes = PARTS * (uint32_t)p.rows * bk * 2u + b_bytes;
   const int ahead = min(stages, mine);        // k-steps that need no stage to become free
 
   // (tap, channel block) of a k-step of this CTA
   auto load_b = [&](int i, int s) {
     const uint32_t t = tc_fdiv((uint32_t)(ks0 + i), p.div_cb);
-    tma_load_3d(sB + s * b_bytes, &p.tmB, full_bar(s), (ks0 + i - (int)t * p.cblocks) * bk, tl.k0, (int)t);
+#pragma unroll
+    for (int j = 0; j < PARTS; ++j)
+      tma_load_3d(sB + s * b_bytes + j * b_tile, &p.tmB, full_bar(s), (ks0 + i - (int)t * p.cblocks) * bk, tl.k0,
+                  (int)t * PARTS + j);
   };
   auto load_a = [&](int i, int s) {
     const uint32_t t = tc_fdiv((uint32_t)(ks0 + i), p.div_cb);
     const SkTap tap = p.taps[t];
-    tma_load_4d(sA + s * a_bytes, &p.tmA[tap.map], full_bar(s), (ks0 + i - (int)t * p.cblocks) * bk,
-                tl.q0 + tap.dw, tl.p0 + tap.dh, tl.n0);
+#pragma unroll
+    for (int j = 0; j < PARTS; ++j)
+      tma_load_4d(sA + s * a_bytes + j * a_tile, &p.tmA[tap.map + j], full_bar(s),
+                  (ks0 + i - (int)t * p.cblocks) * bk, tl.q0 + tap.dw, tl.p0 + tap.dh, tl.n0);
   };
   // The k-steps of the first ring turn are requested by one lane each: a single thread's chain of
   // index arithmetic, arming arrival and request per k-step is time on the layer's critical path.
@@ -223,7 +279,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   // residual pieces this thread will add: fetched now, used after the products
   uint4 res[BN / 16];
   const int row0 = rank * p.rows_owner;
-  const int nrows = CL ? min(p.rows_owner, p.rows - row0) : 0;   // rows this CTA finishes
+  const int nrows = ITEMS ? min(p.rows_owner, p.rows - row0) : 0;   // rows this CTA finishes
   const int items = nrows * G8;
   const int quad = warp & 3, part = warp >> 2, row = quad * 32 + lane;
 
@@ -236,7 +292,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
     const int i = (int)threadIdx.x - 128;
     if (i < BN) bias_s[i] = (p.bias && tl.k0 + i < p.K) ? p.bias[tl.k0 + i] : 0.0f;
   }
-  if (!F32 && p.residual) {
+  if (!F32 && !SPLIT && p.residual) {
     if constexpr (CL) {
 #pragma unroll
       for (int u = 0; u < BN / 16; ++u) {
@@ -275,7 +331,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   auto finish = [&](bool on, float *v, const uint4 &rs, int lin, int c) {
     if constexpr (F32) {
       sk_finish32(p, on, v, lin, c);
-    } else {
+    } else if constexpr (!SPLIT) {
       const uint4 o = sk_pack16<F16>(p, v, rs);
       st_global_v4_if(on, reinterpret_cast<uint16_t *>(p.y) + (int64_t)lin * p.K + c, o.x, o.y, o.z, o.w);
     }
@@ -312,32 +368,43 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
       const uint64_t a0 = make_smem_desc(sA, bk), b0 = make_smem_desc(sB, bk);
       const uint32_t a_hi = (uint32_t)(a0 >> 32), b_hi = (uint32_t)(b0 >> 32);
       const uint32_t a_step = a_bytes >> 4, b_step = b_bytes >> 4;
-      const uint32_t d0 = tmem + (uint32_t)(warp * (SPLIT ? 2 * BN : BN));
+      const uint32_t d0 = tmem + (uint32_t)(warp * BN);
       uint32_t seen = 0;
       auto run = [&](auto nk_c) {
         constexpr int NK = decltype(nk_c)::value;
         uint32_t phase = 0;
         int s = warp;
         for (int i = warp; i < mine; i += ni) {
-          uint32_t d = d0, bit = 1u;
-          if constexpr (SPLIT) {
-            const uint32_t tap = tc_fdiv((uint32_t)(ks0 + i), p.div_cb);
-            if (tap % 6u != 0u) {
-              d = d0 + (uint32_t)BN;
-              bit = 2u;
-            }
-          }
           const uint32_t a_lo = (uint32_t)a0 + (uint32_t)s * a_step, b_lo = (uint32_t)b0 + (uint32_t)s * b_step;
-          const uint32_t more = seen & bit;
+          const uint32_t more = seen;
           if (!mbar_wait_hot(full_bar(s), phase, abort_flag)) {
             err_code = 3;
             return;
           }
           tc_fence_after();
-  #pragma unroll
-          for (int kk = 0; kk < NK; ++kk)
-            mma_lohi(d, a_lo + 2u * kk, a_hi, b_lo + 2u * kk, b_hi, IDESC, kk ? 1u : more);
-          seen |= bit;
+          // activation part PA times N / BN filter parts from PB on, which lie one after the other, into
+          // as many accumulators from D on
+          auto products = [&](int pa, int pb, int d, uint32_t n, bool opens) {
+#pragma unroll
+            for (int kk = 0; kk < NK; ++kk)
+              mma_lohi(d0 + (uint32_t)(d * BN), a_lo + (uint32_t)pa * (a_tile >> 4) + 2u * kk, a_hi,
+                       b_lo + (uint32_t)pb * (b_tile >> 4) + 2u * kk, b_hi, IDESC0 | (n << NSHIFT),
+                       opens && kk == 0 ? more : 1u);
+          };
+          if constexpr (!SPLIT) {
+            products(0, 0, 0, BN, true);
+          } else if constexpr (BN == 128) {
+            products(0, 0, 0, 2 * BN, true);
+            products(0, 2, 1, BN, false);
+            products(1, 0, 1, BN, false);
+            products(1, 1, 1, BN, false);
+            products(2, 0, 1, BN, false);
+          } else {
+            products(0, 0, 0, 3 * BN, true);
+            products(1, 0, 1, 2 * BN, false);
+            products(2, 0, 2, BN, false);
+          }
+          seen = 1u;
           if (i + stages < mine) tc_commit(empty_bar(s));   // nobody waits for the last ones
           s += ni;
           if (s >= stages) {   // (a ring as long as the share is never reused)
@@ -358,14 +425,14 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
       __syncthreads();   // bias_s, used
     }
 #pragma unroll
-    for (int w = 0; w < NI; ++w) used_all[w] = w >= ni ? 0 : real ? used[w] : (SPLIT ? 3 : 1);
+    for (int w = 0; w < NI; ++w) used_all[w] = w >= ni ? 0 : real ? used[w] : 1;
     // CH columns of this thread's row from column h * CH on: the sum of the accumulators, which are all
     // requested before the first is waited for
     auto load_sum = [&](int h, uint32_t *r) {
       uint32_t t[NACC][CH];
 #pragma unroll
       for (int k = 0; k < NACC; ++k) {
-        if ((used_all[SPLIT ? k / 2 : k] >> (SPLIT ? k & 1 : 0)) & 1) {   // the same for all threads
+        if (used_all[SPLIT ? 0 : k]) {   // the same for all threads
           tc_ld<CH>(t_row + (uint32_t)(k * BN + h * CH), t[k]);
         } else {
 #pragma unroll
@@ -381,8 +448,10 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
         r[j] = __float_as_uint(v);
       }
     };
-    if constexpr (CL) {
-      if (real) cluster_wait_acquire();   // every CTA of the cluster has started
+    if constexpr (ITEMS) {
+      if constexpr (CL) {
+        if (real) cluster_wait_acquire();   // every CTA of the cluster has started
+      }
       const bool on = real && row < p.rows && !err_code;
 #pragma unroll
       for (int h = 0; h < HALF / CH; ++h) {
@@ -392,13 +461,21 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
         for (int j = 0; j < CH / 4; ++j) {
           // 16-byte pieces of a row are permuted by its number: eight lanes, eight bank groups
           const uint32_t piece = (uint32_t)((part * HALF + h * CH) / 4 + j) ^ (uint32_t)(row & 7);
-          st_async_v4_if(on, dst + piece * 16u, dst_bar, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          if constexpr (CL)
+            st_async_v4_if(on, dst + piece * 16u, dst_bar, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          else
+            st_shared_v4_if(on, sX + (uint32_t)row * (BN * 4u) + piece * 16u, r[4 * j], r[4 * j + 1], r[4 * j + 2],
+                            r[4 * j + 3]);
         }
       }
       __syncwarp();
-      if (real && !err_code && !mbar_wait(sums_bar, 0, abort_flag)) err_code = 6;
+      if constexpr (CL) {
+        if (real && !err_code && !mbar_wait(sums_bar, 0, abort_flag)) err_code = 6;
+      } else {
+        if (real) __syncthreads();
+      }
       const uint8_t *xs = smem_raw + (sX - sA);
-      auto item = [&](bool live, int r, int g, const uint4 &rs) {
+      auto item = [&](bool live, int r, int g, const uint4 *rs) {
         r = live ? r : 0;
         g = live ? g : 0;
         const int lin = lin_s[row0 + r < 128 ? row0 + r : 0], c = tl.k0 + g * 8;
@@ -414,16 +491,39 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
           v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
           v[4] += e.x; v[5] += e.y; v[6] += e.z; v[7] += e.w;
         }
-        finish(real && live && lin >= 0 && c < p.K && !err_code, v, rs, lin, c);
+        const bool store = real && live && lin >= 0 && c < p.K && !err_code;
+        if constexpr (SPLIT && !F32) sk_finish_parts(p, store, v, rs, lin, c);
+        else finish(store, v, *rs, lin, c);
       };
       if (F32 && p.out_hw) {   // consecutive threads on consecutive pixels of one channel
         const int n = nrows > 0 ? nrows : 1, end = real ? items : (int)threadIdx.x + 1;
-        for (int it = threadIdx.x; it < end; it += SK_THREADS) item(it < items, it % n, it / n, res[0]);
+        for (int it = threadIdx.x; it < end; it += SK_THREADS) item(it < items, it % n, it / n, res);
+      } else if constexpr (SPLIT && !F32) {
+        constexpr int B = 2;   // residuals of so many items are requested at a time
+#pragma unroll 1
+        for (int u = 0; u < (real ? BN / 16 : B); u += B) {
+          uint4 rs[B][3];
+#pragma unroll
+          for (int b = 0; b < B; ++b) {
+            const int it = (int)threadIdx.x + (u + b) * SK_THREADS, r = it / G8, c = tl.k0 + (it % G8) * 8;
+            const int lin = real && it < items ? lin_s[row0 + r] : -1;
+            if (p.residual && lin >= 0 && c < p.K)
+#pragma unroll
+              for (int j = 0; j < 3; ++j)
+                rs[b][j] = *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(p.residual) +
+                                                            j * p.plane + (int64_t)lin * p.K + c);
+          }
+#pragma unroll
+          for (int b = 0; b < B; ++b) {
+            const int it = (int)threadIdx.x + (u + b) * SK_THREADS;
+            item(it < items, it / G8, it % G8, rs[b]);
+          }
+        }
       } else {
 #pragma unroll
         for (int u = 0; u < BN / 16; ++u) {
           const int it = (int)threadIdx.x + u * SK_THREADS;
-          if (u == 0 || it < items) item(it < items, it / G8, it % G8, res[u]);
+          if (u == 0 || it < items) item(it < items, it / G8, it % G8, res + u);
         }
       }
     } else {
@@ -466,10 +566,10 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
                  : "memory");
 }
 
-size_t sk_smem_bytes(int bn, int stages, int a_bytes, int bk, int splits, int rows_owner) {
-  const size_t x = splits > 1 ? (size_t)splits * rows_owner * bn * 4 : 0;
-  return (size_t)stages * (a_bytes + bn * bk * 2) + x +
-         bn * 4 + 512 + 8 * (2 * stages + 7);
+size_t sk_smem_bytes(int bn, int stages, int a_bytes, int bk, int splits, int rows_owner, bool split) {
+  const size_t ring = (size_t)stages * sk_parts(split) * (a_bytes + bn * bk * 2);
+  const size_t x = (size_t)splits * rows_owner * bn * 4;
+  return (splits > 1 ? ring + x : split && x > ring ? x : ring) + bn * 4 + 512 + 8 * (2 * stages + 7);
 }
 
 template <int BN, bool F16, bool SPLIT, bool CL, bool F32>
@@ -487,8 +587,10 @@ template <int BN>
 static void sk_launch_bn(const SkParams &p, bool f16, bool split, int tiles, size_t smem, cudaStream_t s) {
   const bool cl = p.splits > 1, f32 = p.out_f32 != nullptr;
   if (split) {
-    if (cl) sk_launch_one<BN, false, true, true, true>(p, tiles, smem, s);
-    else sk_launch_one<BN, false, true, false, true>(p, tiles, smem, s);
+    if (cl && f32) sk_launch_one<BN, false, true, true, true>(p, tiles, smem, s);
+    else if (cl) sk_launch_one<BN, false, true, true, false>(p, tiles, smem, s);
+    else if (f32) sk_launch_one<BN, false, true, false, true>(p, tiles, smem, s);
+    else sk_launch_one<BN, false, true, false, false>(p, tiles, smem, s);
   } else if (f16) {
     if (cl && f32) sk_launch_one<BN, true, false, true, true>(p, tiles, smem, s);
     else if (cl) sk_launch_one<BN, true, false, true, false>(p, tiles, smem, s);

@@ -24,11 +24,13 @@ struct alignas(64) SkParams {
   int tw, th, tn;
   int rows;                            // pixels of a tile's box (<= 128)
   int rows_owner;                      // rows each CTA of the cluster sums up and stores
-  int a_bytes;                         // bytes of a stage's activation tile (multiple of 1024)
+  int a_bytes;                         // bytes of an activation tile in a stage (multiple of 1024)
   int K, gq, gp, gn;
   const float *bias;
-  const void *residual;                // 16-bit NHWC like the output, or null
-  void *y;                             // 16-bit NHWC output (when out_f32 is null)
+  const void *residual;                // in the form of y, or null
+  void *y;                             // 16-bit NHWC output (when out_f32 is null); with split operands
+                                       // three planes (hi, mid, lo) of `plane` elements each
+  int64_t plane;
   float *out_f32;
   int ldo, out_hw;                     // as in TcParams
   int out_vec4;                        // row-major fp32 output whose rows are 16-byte aligned
@@ -38,14 +40,16 @@ struct alignas(64) SkParams {
 };
 
 // Threads that issue MMAs (and that load) in a kernel: as many accumulators as fit the 256 TMEM
-// columns a CTA may use, four at most.  A ring with fewer stages than the CTA has k-steps must have a
-// multiple of this many.
+// columns a CTA may use, four at most; one for split operands, whose k-step has 12 or 24 MMAs.  A ring
+// with fewer stages than the CTA has k-steps must have a multiple of this many.
 __host__ __device__ constexpr int sk_issuers(int bn, bool split) {
-  return 256 / (bn * (split ? 2 : 1)) < 4 ? 256 / (bn * (split ? 2 : 1)) : 4;
+  return split ? 1 : 256 / bn < 4 ? 256 / bn : 4;
 }
+// Operand tiles of either side in a stage: fp32 values travel as three bf16 parts (hi, mid, lo).
+__host__ __device__ constexpr int sk_parts(bool split) { return split ? 3 : 1; }
 // Shared memory a launch needs.
-size_t sk_smem_bytes(int bn, int stages, int a_bytes, int bk, int splits, int rows_owner);
-// `split` selects the kernels whose operands are bf16 parts of fp32 values (see TC_MODE_SPLIT).
+size_t sk_smem_bytes(int bn, int stages, int a_bytes, int bk, int splits, int rows_owner, bool split);
+// `split` selects the kernels whose operands are bf16 parts of fp32 values.
 bool sk_launch(const SkParams &p, int bn, bool f16, bool split, int tiles, size_t smem, cudaStream_t s);
 
 }  // namespace occ

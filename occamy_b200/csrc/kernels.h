@@ -106,15 +106,21 @@ void launch_pack_fold_bf16(const float *w, bf16 *out, int K, int C, int R, int S
 void launch_pad_input_bf16(const float *x, bf16 *out, int N, int C, int H, int W, int Wp, int Cp,
                            int pad_w, bool f16, cudaStream_t s);
 
-// ---- fp32 carried as three bf16 parts (fp32 mode on the tensor cores) ----------
-// x fp32 NCHW -> three consecutive NHWC planes [N][H][W][Cp] (hi, mid, lo), zero channels up to Cp
+// ---- fp32 carried as three bf16 parts (fp32 mode on the tensor cores, kernels_parts.cu) ----------
+// x fp32 NCHW -> three consecutive NHWC planes [N][H][W][Cp] (hi, mid, lo), zero channels up to Cp ...
 void launch_split3_nchw(const float *x, bf16 *y, int N, int C, int Cp, int H, int W, cudaStream_t s);
+// ... and back (C channels)
+void launch_join3_nchw(const bf16 *x, float *y, int N, int C, int H, int W, cudaStream_t s);
 // x fp32 [M][K], rows `ld` floats apart -> three consecutive planes [M][Kp]
 void launch_split3_rows(const float *x, bf16 *y, int M, int K, int Kp, int ld, cudaStream_t s);
-// fp32 KCRS -> bf16 [R*S*6][K][Cp]: six filter parts per tap, in the order the kernel pairs
-// them with the activation parts
-void launch_pack_krsc_split(const float *w, bf16 *out, int K, int C, int R, int S, int Cp,
-                            cudaStream_t s);
+// launch_pad_input_bf16 in three planes
+void launch_split3_pad(const float *x, bf16 *y, int N, int C, int H, int W, int Wp, int Cp, int pad_w,
+                       cudaStream_t s);
+void launch_pool3(const bf16 *x, bf16 *y, int N, int C, int H, int W, int P, int Q, int kh, int kw, int pad_h,
+                  int pad_w, int sh, int sw, bool avg, cudaStream_t s);
+void launch_gap3(const bf16 *x, float *y, int N, int HW, int C, cudaStream_t s);
+// fp32 KCRS -> bf16 [R*S][3][K][Cp], or folded (Sp > 0) [R][3][K][Sp*Cp]
+void launch_pack_split3(const float *w, bf16 *out, int K, int C, int R, int S, int Sp, int Cp, cudaStream_t s);
 
 // ---- tcgen05 implicit-GEMM convolution / GEMM --------------------------------
 struct TcConvArgs {
@@ -126,8 +132,8 @@ struct TcConvArgs {
   float *out_f32;        // fp32 output (else null): row-major [N*P*Q][ldo] (GEMM head) ...
   int ldo;
   int out_nchw;          // ... or, when set, the NCHW tensor [N][K][P][Q] itself
-  int split;             // fp32 operands as bf16 parts: x points at three planes (hi, mid, lo) of
-                         // N*H*W*Cf elements each, w holds six parts per tap (launch_pack_krsc_split)
+  int split;             // fp32 operands as bf16 parts: x (and residual and y, where given) points at
+                         // three planes, hi, mid, lo, one after the other; w holds three parts per tap
   int N, H, W, Cf;       // A tensor dims (W already = Q for the folded form)
   int K, P, Q;
   int R, S;              // taps looped over (S = 1 for the folded form)

@@ -104,12 +104,19 @@ TensorRec *reg_find(const void *p, uintptr_t *base) {
 
 bool mode_f16() { return rt().mode == MATH_F16; }
 
-bool is_act16(const void *p, int64_t n, int64_t c, int64_t h, int64_t w) {
+static bool is_in_format(const void *p, Fmt want, int64_t n, int64_t c, int64_t h, int64_t w) {
   uintptr_t base;
   TensorRec *rec = reg_find(p, &base);
-  const Fmt want = mode_f16() ? FMT_F16_NHWC : FMT_BF16_NHWC;
   return rec && base == (uintptr_t)p && rec->fmt == want && rec->n == n && rec->c == c &&
          rec->h == h && rec->w == w;
+}
+
+bool is_act16(const void *p, int64_t n, int64_t c, int64_t h, int64_t w) {
+  return is_in_format(p, mode_f16() ? FMT_F16_NHWC : FMT_BF16_NHWC, n, c, h, w);
+}
+
+bool is_parts(const void *p, int64_t n, int64_t c, int64_t h, int64_t w) {
+  return is_in_format(p, FMT_PARTS, n, c, h, w);
 }
 
 const __nv_bfloat16 *act16_ptr(const void *p) {
@@ -166,10 +173,9 @@ void mark_f32(void *p) {
   rec->host_src = nullptr;
 }
 
-void mark_act16(void *p, int64_t n, int64_t c, int64_t h, int64_t w, const void *home) {
+static void mark_format(void *p, Fmt fmt, int64_t n, int64_t c, int64_t h, int64_t w, const void *home) {
   uintptr_t base;
   TensorRec *rec = reg_find(p, &base);
-  const Fmt fmt = mode_f16() ? FMT_F16_NHWC : FMT_BF16_NHWC;
   if (!rec || base != (uintptr_t)p) {
     // Unknown or interior pointer: record it as its own tensor of the fp32 extent.
     reg_new(p, (size_t)(n * c * h * w) * 4, fmt);
@@ -183,6 +189,14 @@ void mark_act16(void *p, int64_t n, int64_t c, int64_t h, int64_t w, const void 
   rec->home = home;
   rec->dev_src = nullptr;
   rec->host_src = nullptr;
+}
+
+void mark_act16(void *p, int64_t n, int64_t c, int64_t h, int64_t w, const void *home) {
+  mark_format(p, mode_f16() ? FMT_F16_NHWC : FMT_BF16_NHWC, n, c, h, w, home);
+}
+
+void mark_parts(void *p, int64_t n, int64_t c, int64_t h, int64_t w, const void *home) {
+  mark_format(p, FMT_PARTS, n, c, h, w, home);
 }
 
 void ensure_f32(const void *p) {
@@ -222,6 +236,11 @@ void ensure_f32(const void *p) {
     rec->home = nullptr;
     launch_nhwc_bf16_to_nchw_f32((const bf16 *)tmp, (float *)base, (int)rec->n, (int)rec->c,
                                  (int)rec->h, (int)rec->w, rec->fmt == FMT_F16_NHWC, r.stream);
+    count(CNT_MATERIALIZE);
+  } else if (rec->fmt == FMT_PARTS) {
+    launch_join3_nchw((const bf16 *)rec->home, (float *)base, (int)rec->n, (int)rec->c, (int)rec->h, (int)rec->w,
+                      r.stream);
+    rec->home = nullptr;
     count(CNT_MATERIALIZE);
   }
   rec->fmt = FMT_F32;

@@ -28,7 +28,8 @@ enum Fmt {
   FMT_PENDING = 3,    // host->device upload deferred (constant already packed on device)
   FMT_ELIDED = 4,     // never written: a cross-call fusion skipped it (reading it is an error)
   FMT_F16_NHWC = 5,   // like FMT_BF16_NHWC with fp16 elements (MATH_F16)
-  FMT_STEM_ROWS = 6   // padded channels-last rows for a few-channel convolution, in `home`
+  FMT_STEM_ROWS = 6,  // padded channels-last rows for a few-channel convolution, in `home`
+  FMT_PARTS = 7       // fp32 as three bf16 parts: three NHWC planes in `home` (fp32 mode, kernels_parts.cu)
 };
 inline bool fmt_is_16(Fmt f) { return f == FMT_BF16_NHWC || f == FMT_F16_NHWC; }
 
@@ -147,7 +148,10 @@ bool is_act16(const void *p, int64_t n, int64_t c, int64_t h, int64_t w);
 // (`home`: into that buffer instead of p's own bytes).
 void mark_f32(void *p);
 void mark_act16(void *p, int64_t n, int64_t c, int64_t h, int64_t w, const void *home = nullptr);
-// The bytes of a tensor that is_act16().
+// The same for fp32 values in three planes (FMT_PARTS); they always have a buffer of their own.
+bool is_parts(const void *p, int64_t n, int64_t c, int64_t h, int64_t w);
+void mark_parts(void *p, int64_t n, int64_t c, int64_t h, int64_t w, const void *home);
+// The bytes of a tensor that is_act16() or is_parts().
 const __nv_bfloat16 *act16_ptr(const void *p);
 // A buffer for a 16-bit tensor that cannot be written at its own address; in use as long as a tensor
 // record (or a kernel that is held back, see home_held) refers to it.  A handful are kept.

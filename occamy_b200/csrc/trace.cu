@@ -113,6 +113,32 @@ int only_convs_read(const std::vector<Entry> &rec, uintptr_t p, int64_t bytes, s
   return -1;
 }
 
+// True when everything that reads [p, p+bytes) from entry `from` on, until the range is handed out again
+// or freed, takes fp32 values in three planes: dense convolutions of fp32 mode, sums folded into one,
+// pools and means.
+bool only_parts_read(const std::vector<Entry> &rec, const std::vector<uint8_t> &roles, uintptr_t p, int64_t bytes,
+                     size_t from) {
+  bool any = false;
+  for (size_t t = from; t < rec.size(); ++t) {
+    const Entry &e = rec[t];
+    for (int k = 0; k < 3; ++k) {
+      if (!e.in[k] || !overlaps(e.in[k], e.in_bytes[k] > 0 ? e.in_bytes[k] : 1, p, bytes)) continue;
+      if (e.in[k] != p || e.in_bytes[k] != bytes) return false;
+      const bool conv = (e.sym == S_CONV || e.sym == S_CONV_BIAS_ACT) && k == 0 && e.parts;
+      const bool sum = e.sym == S_TENSOR_OP && e.kind == CK_SAME_ADD && (roles[t] & 0xF) == R_ABSORB;
+      const bool pool = e.sym == S_MAXPOOL || e.sym == S_AVGPOOL || e.sym == S_REDUCE;
+      if (!conv && !sum && !pool) return false;
+      any = true;
+    }
+    if ((e.sym == S_MEMOFFSET || e.sym == S_MALLOC) && overlaps(e.out, e.out_bytes, p, bytes)) return any;
+    if ((e.sym == S_DEALLOC && e.out == p) || e.sym == S_POOLFREE) return any;
+    if (e.sym == S_OPAQUE) return false;
+    if (any && e.out == p && e.out_bytes == bytes) return true;
+    if (e.sym != S_MEMOFFSET && e.sym != S_MALLOC && e.out && overlaps(e.out, e.out_bytes, p, bytes)) return false;
+  }
+  return false;
+}
+
 // Marks the chains of a finished inference: R_DEFER on the convolution, R_ABSORB on the
 // calls folded into it.
 void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles, std::vector<int> &reader) {
@@ -216,6 +242,10 @@ void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles, std::ve
     roles[i] |= R_DEFER;
     for (size_t m : members) roles[m] |= R_ABSORB;
   }
+  for (size_t i = 0; i < rec.size(); ++i)   // (after the roles are known)
+    if ((rec[i].parts || (roles[i] & 0xF) == R_ABSORB) &&
+        only_parts_read(rec, roles, rec[i].out, rec[i].out_bytes, i + 1))
+      roles[i] |= RF_FOR_PARTS;
 }
 
 // Writes the adopted prefix out as calls of this inference, their pointers moved to its pool.

@@ -52,7 +52,8 @@ struct Entry {
   int64_t out_bytes = 0;   // fp32 extent of `out` (range size for the memory calls)
   int64_t dims[4] = {0, 0, 0, 0};
   int kind = CK_NONE;      // ChainKind, or the activation mode of a fused convolution
-  bool fusable = false;    // convolution or product that the 16-bit path takes (may head a chain)
+  bool fusable = false;    // convolution or product that the tensor cores take (may head a chain)
+  bool parts = false;      // ... in fp32 mode: operands as bf16 parts of fp32 values
   bool depthwise = false;
   bool poolable = false;   // convolution whose kernel can take a following CK_POOL_3S2 along
   bool uploaded = false;   // S_H2D: bytes crossed to the device (not a constant that is already there)
@@ -80,6 +81,9 @@ constexpr uint8_t RF_FOR_MATMUL = 0x10;
 // on a device-to-device copy: what reads the tensor are convolutions on the 16-bit path, so the copy may
 // bring it in in their form (TraceProgram::reader names the first of them)
 constexpr uint8_t RF_FOR_CONV = 0x20;
+// on a convolution in fp32 mode or a call folded into one: all that reads the result takes it in three
+// planes of parts (FMT_PARTS)
+constexpr uint8_t RF_FOR_PARTS = 0x40;
 struct TraceProgram {
   std::vector<uint64_t> sigs;
   std::vector<uint8_t> roles;   // Role | RF_*
