@@ -66,7 +66,7 @@ void die(const char *what, cudaError_t e, size_t size) {
   exit(-1);
 }
 
-enum PackLayout { PACK_KRSC = 1, PACK_DW = 2, PACK_FOLD = 3, PACK_RAW = 4, PACK_STEM = 5, PACK_PARTS = 6 };
+enum PackLayout { PACK_KRSC = 1, PACK_DW = 2, PACK_FOLD = 3, PACK_RAW = 4, PACK_STEM = 5, PACK_PARTS = 6, PACK_BIAS3 = 7, PACK_IR_HALF = 8 };
 // fp32 mode: dense convolutions and GEMMs on the tensor cores with split operands (see
 // kernels_parts.cu); off with OCCAMY_FP32_TC=0 or occamy_set_fp32_tensor_cores(0), which
 // leaves the CUDA-core kernels.
@@ -107,10 +107,21 @@ void *packed_weights(const float *w, int layout, size_t packed_bytes, int K, int
       return it->second.dev;
     }
   }
-  ensure_f32(w);
   void *dst = nullptr;
   if (cacheable) {
     graph_stop_capture();   // packed once, not in every inference
+    if (rec->fmt == FMT_PENDING) {
+      // Not on the device: it goes through a buffer of the runtime's.  (Its own place may still hold what a
+      // held-back kernel has to read.)
+      void *tmp = scratch_get(8, rec->host_bytes);
+      if (!tmp) return nullptr;
+      OCC_CUDA(cudaMemcpyAsync(tmp, rec->host_src, rec->host_bytes, cudaMemcpyHostToDevice, r.stream));
+      r.main_copies++;
+      count(CNT_H2D_BYTES, (int64_t)rec->host_bytes);
+      w = (const float *)tmp;
+    } else {
+      ensure_f32(w);
+    }
     PackedWeight &pw = r.wcache[key];
     if (pw.dev) graph_forget_all();   // graphs refer to the old contents
     if (pw.dev && pw.bytes != packed_bytes) {
@@ -125,6 +136,7 @@ void *packed_weights(const float *w, int layout, size_t packed_bytes, int K, int
     dst = pw.dev;
     r.resident[rec->host_src] = std::make_pair(rec->host_bytes, rec->host_hash);
   } else {
+    ensure_f32(w);
     dst = scratch_get(layout == PACK_STEM ? 5 : 1, packed_bytes);
   }
   if (!dst) return nullptr;
@@ -133,9 +145,20 @@ void *packed_weights(const float *w, int layout, size_t packed_bytes, int K, int
   else if (layout == PACK_RAW)
     OCC_CUDA(cudaMemcpyAsync(dst, w, packed_bytes, cudaMemcpyDeviceToDevice, r.stream));
   else if (layout == PACK_STEM) launch_pack_stem_bf16(w, (bf16 *)dst, C, R, S, Cp, Sp * Cp, r.stream);
+  else if (layout == PACK_BIAS3) launch_pack_bias3(w, (bf16 *)dst, K, f16, r.stream);
+  else if (layout == PACK_IR_HALF) launch_pack_ir_half(w, dst, K, R * S, r.stream);
   else if (layout == PACK_PARTS) launch_pack_split3(w, (bf16 *)dst, K, C, R, S, Sp, Cp, r.stream);
   else launch_pack_fold_bf16(w, (bf16 *)dst, K, C, R, S, Sp, Cp, f16, r.stream);
   return dst;
+}
+
+// A constant in the form the inverted-residual kernel takes it (the first convolution's bias as parts; the
+// depthwise filter or bias as fp16); null unless it stays on the device.
+const void *packed_for_block(const float *c, int layout, size_t bytes, int E, int R) {
+  uintptr_t base;
+  const TensorRec *rec = reg_find(c, &base);
+  if (!rt().cache_weights || !rec || base != (uintptr_t)c || !rec->host_src) return nullptr;
+  return packed_weights(c, layout, bytes, E, 0, R, R, 0, 0);
 }
 
 // fp32 constants used as they are (biases mostly): the resident copy when there is one, else the
@@ -175,18 +198,28 @@ struct ConvJob {
   bool out16 = false;             // ... whose reader is another product: 16-bit result
   // fp32 mode (a.split): the result goes out in three planes (FMT_PARTS), else as plain fp32
   bool out_parts = false;
+  // one of the convolutions of an inverted residual: its result only goes to the next one / its input
+  // only comes from the one before (and is not there yet)
+  bool linked = false, joined = false;
+  // (the constants of one once more, packed_for_block(): a first bias, a depthwise filter and bias)
+  const void *block_w = nullptr, *block_b = nullptr;
   // folded (few-channel) form: what the fused convolution + pool kernel needs besides `a`
   const bf16 *w_stem = nullptr;   // filter in that kernel's layout, packed while the filter is live
 };
 
 ConvJob g_pending;  // convolution held back while later calls are folded into it
+ConvJob g_front[2]; // ... and the ones before it that it has joined, not launched yet either
+int g_fronts = 0;
 const ConvJob *g_launching = nullptr;   // job whose output buffer is being looked for
 
 bool job_reads(const ConvJob &j, const void *home) {
   return j.a.x == home || j.a.residual == home || j.dw_x == home;
 }
 bool home_held_hook(const void *home) {
-  return (g_pending.active && job_reads(g_pending, home)) || (g_launching && job_reads(*g_launching, home));
+  for (int i = 0; i < g_fronts; ++i)
+    if (job_reads(g_front[i], home)) return true;
+  return ((g_pending.active || g_fronts) && job_reads(g_pending, home)) ||
+         (g_launching && job_reads(*g_launching, home));
 }
 
 // A bias without a resident copy is read from the caller's tensor when the (possibly held-back)
@@ -210,6 +243,8 @@ void stem_geometry(const ConvGeom &g, int &Cp, int &Sp, int &Wp) {
   Wp = (Wp + 7) / 8 * 8;
 }
 
+// `job.linked` (the first convolution of an inverted residual): x is taken as it is, without the padding of
+// its channels; `job.joined`: x is not there yet.
 bool prepare_dense(const float *x, const float *w, const float *bias, const ConvGeom &g,
                    ConvJob &job) {
   Runtime &r = rt();
@@ -263,9 +298,12 @@ bool prepare_dense(const float *x, const float *w, const float *bias, const Conv
                                        g.S, Sp, Cp);
   } else {
     const bf16 *xb = nullptr;
-    if (is_act16(x, g.N, g.C, g.H, g.W)) {
+    const bool as_is = job.linked || job.joined;
+    if (job.joined) {
+      // (resolved when it is launched)
+    } else if (is_act16(x, g.N, g.C, g.H, g.W)) {
       xb = act16_ptr(x);
-      if (Cp == g.C && (const void *)xb == x) {
+      if ((Cp == g.C || as_is) && (const void *)xb == x) {
         job.dep_lo[0] = (uintptr_t)x;
         job.dep_hi[0] = (uintptr_t)x + (size_t)g.N * g.C * g.H * g.W * 2;
       }
@@ -276,7 +314,7 @@ bool prepare_dense(const float *x, const float *w, const float *bias, const Conv
       launch_nchw_f32_to_nhwc_bf16(x, xc, g.N, g.C, g.H, g.W, mode_f16(), r.stream);
       xb = xc;
     }
-    if (Cp != g.C) {   // the kernel reads the padded copy, made now: no dependence on x later
+    if (Cp != g.C && !as_is) {   // the kernel reads the padded copy, made now: no dependence on x later
       bf16 *xp = (bf16 *)scratch_get(6, (size_t)g.N * Cp * g.H * g.W * 2);
       if (!xp) return false;
       launch_pad_channels_bf16(xb, xp, (int64_t)g.N * g.H * g.W, g.C, Cp, r.stream);
@@ -291,6 +329,10 @@ bool prepare_dense(const float *x, const float *w, const float *bias, const Conv
   a.bias = bias ? resident_f32(bias, (size_t)g.K * 4) : nullptr;
   if (bias) ready = ready && g_pack_was_resident;
   job_track_bias(job, a.bias, bias, g.K);
+  if (bias && job.linked && !job.joined) {
+    job.block_b = packed_for_block(bias, PACK_BIAS3, (size_t)g.K * 32, g.K, 0);
+    ready = ready && g_pack_was_resident;
+  }
   // filter and bias were on the device before this call: the kernel may fetch them while the
   // kernel before it is still running
   a.consts_ready = ready ? 1 : 0;
@@ -367,7 +409,9 @@ bool prepare_depthwise(const float *x, const float *w, const float *bias, const 
   Runtime &r = rt();
   if (g.C % 8 != 0) return false;
   job.dep_lo[0] = job.dep_hi[0] = 0;
-  if (is_act16(x, g.N, g.C, g.H, g.W)) {
+  if (job.joined) {
+    job.dw_x = nullptr;
+  } else if (is_act16(x, g.N, g.C, g.H, g.W)) {
     job.dw_x = act16_ptr(x);
     if ((const void *)job.dw_x == x) {
       job.dep_lo[0] = (uintptr_t)x;
@@ -386,6 +430,14 @@ bool prepare_depthwise(const float *x, const float *w, const float *bias, const 
   bool ready = g_pack_was_resident;
   job.bias = bias ? resident_f32(bias, (size_t)g.C * 4) : nullptr;
   if (bias) ready = ready && g_pack_was_resident;
+  if (job.linked && mode_f16()) {
+    job.block_w = packed_for_block(w, PACK_IR_HALF, (size_t)g.C * 18, g.C, 3);
+    ready = ready && g_pack_was_resident;
+    if (bias) {
+      job.block_b = packed_for_block(bias, PACK_IR_HALF, (size_t)g.C * 2, g.C, 1);
+      ready = ready && g_pack_was_resident;
+    }
+  }
   job.a.consts_ready = ready ? 1 : 0;
   job_track_bias(job, job.bias, bias, g.C);
   job.depthwise = true;
@@ -400,7 +452,8 @@ bool ranges_overlap(uintptr_t alo, uintptr_t ahi, uintptr_t blo, uintptr_t bhi) 
   return ahi > alo && bhi > blo && alo < bhi && blo < ahi;
 }
 
-void launch_job(ConvJob &job) {
+// `apart`: the result goes to a buffer of its own, which is returned.
+const bf16 *launch_job(ConvJob &job, bool apart = false) {
   Runtime &r = rt();
   const ConvGeom &g = job.g;
   // A convolution that was held back may find its output placed over memory it still has to read
@@ -418,12 +471,12 @@ void launch_job(ConvJob &job) {
     g_launching = &job;
     void *planes = home_acquire(obytes * 3);
     g_launching = nullptr;
-    if (!planes) return;
+    if (!planes) return nullptr;
     job.a.y = (bf16 *)planes;
     job.a.out_f32 = nullptr;
     launch_tc_conv(job.a, r.stream);
     mark_parts(job.out, g.N, g.K, g.P, g.Q, planes);
-    return;
+    return nullptr;
   }
   if (job.a.split || (job.product && !job.out16)) {   // fp32 result, at its own address
     for (int k = 0; k < 3; k += 2) {
@@ -440,16 +493,16 @@ void launch_job(ConvJob &job) {
     job.a.out_nchw = !job.product || job.a.R * job.a.S > 1;   // (a product's [N][K][1][1]: the same rows)
     launch_tc_conv(job.a, r.stream);
     mark_f32(job.out);
-    return;
+    return nullptr;
   }
   const bool in_place = olo == job.dep_lo[1] && ohi == job.dep_hi[1];
-  if (ranges_overlap(olo, ohi, job.dep_lo[0], job.dep_hi[0]) ||
+  if (apart || ranges_overlap(olo, ohi, job.dep_lo[0], job.dep_hi[0]) ||
       (ranges_overlap(olo, ohi, job.dep_lo[1], job.dep_hi[1]) && !in_place) ||
       ranges_overlap(olo, ohi, job.dep_lo[2], job.dep_hi[2])) {
     g_launching = &job;
     dst = home_acquire(obytes);
     g_launching = nullptr;
-    if (!dst) return;
+    if (!dst) return nullptr;
   }
   if (job.depthwise) {
     launch_depthwise_bf16(job.dw_x, job.dw_w, job.bias, (bf16 *)dst, g, mode_f16(), job.a.consts_ready != 0, r.stream);
@@ -457,15 +510,84 @@ void launch_job(ConvJob &job) {
     job.a.y = (bf16 *)dst;
     launch_tc_conv(job.a, r.stream);
   }
-  mark_act16(job.out, g.N, g.K, g.P, g.Q, dst == job.out ? nullptr : dst);
+  if (!apart) {
+    mark_act16(job.out, g.N, g.K, g.P, g.Q, dst == job.out ? nullptr : dst);
+  } else {   // its tensor may be gone by now: whoever joined this convolution was its only reader
+    uintptr_t base;
+    const TensorRec *rec = reg_find(job.out, &base);
+    if (rec && base == olo && rec->fmt == FMT_ELIDED) mark_act16(job.out, g.N, g.K, g.P, g.Q, dst);
+  }
+  return (const bf16 *)dst;
+}
+
+// The three convolutions of an inverted residual in one kernel; false when they have to run one by one.
+bool launch_block(ConvJob &a, ConvJob &b, ConvJob &c) {
+  Runtime &r = rt();
+  if (a.depthwise || !b.depthwise || c.depthwise || c.linked || !a.block_b) return false;
+  IrArgs ir;
+  memset(&ir, 0, sizeof(ir));
+  const ConvJob *job[3] = {&a, &b, &c};
+  for (int i = 0; i < 3; ++i) {
+    const ConvGeom &g = job[i]->g;
+    ir.lo[i] = g.act == ACT_RELU ? 0.0f : g.act == ACT_CLIP ? g.lo : -INFINITY;
+    ir.hi[i] = g.act == ACT_CLIP ? g.hi : INFINITY;
+    if (g.act != ACT_IDENTITY && g.act != ACT_RELU && g.act != ACT_CLIP) return false;
+  }
+  const ConvGeom &g = c.g;
+  ir.x = a.a.x; ir.w1 = a.a.w; ir.b1 = (const bf16 *)a.block_b;
+  ir.w2 = b.dw_w; ir.b2 = b.bias;
+  if (mode_f16()) {
+    ir.w2 = b.block_w; ir.b2 = b.block_b;
+    if (!ir.w2 || (b.bias && !ir.b2)) return false;
+  }
+  ir.w3 = c.a.w; ir.b3 = c.a.bias;
+  ir.residual = c.a.residual;
+  ir.N = g.N; ir.H = a.g.H; ir.W = a.g.W; ir.C = a.g.C; ir.E = a.g.K; ir.K = g.K; ir.P = g.P; ir.Q = g.Q;
+  ir.stride = b.g.stride_h;
+  ir.f16 = mode_f16();
+  ir.consts_ready = a.a.consts_ready && b.a.consts_ready && c.a.consts_ready;
+  if (!ir_supported(ir.N, ir.C, ir.E, ir.K, ir.H, ir.W, ir.P, ir.Q, ir.stride, ir.f16)) return false;
+  // the output must not land on anything the block reads: tiles read beyond their own pixels
+  const uintptr_t olo = (uintptr_t)c.out;
+  const size_t obytes = (size_t)g.N * g.K * g.P * g.Q * 2;
+  bool clash = false;
+  for (const ConvJob *j : job)
+    for (int k = 0; k < 3; ++k) clash = clash || ranges_overlap(olo, olo + obytes, j->dep_lo[k], j->dep_hi[k]);
+  void *dst = clash ? home_acquire(obytes) : c.out;
+  if (!dst) return false;
+  ir.y = (bf16 *)dst;
+  if (!launch_ir(ir, r.stream)) return false;
+  mark_act16(c.out, g.N, g.K, g.P, g.Q, clash ? dst : nullptr);
+  return true;
 }
 
 // Executes the held-back convolution as far as it has been built up.
 void flush_pending() {
   if (!g_pending.active) return;
   g_pending.active = false;
+  for (int i = 0; i < g_fronts; ++i)
+    if (g_front[i].absorbed) trace_count_chain();
   if (g_pending.absorbed && !g_pending.product) trace_count_chain();   // convolution chains
-  launch_job(g_pending);
+  if (g_fronts != 2 || !launch_block(g_front[0], g_front[1], g_pending)) {
+    const bf16 *x = nullptr;
+    auto resolve = [&](ConvJob &job) {
+      const ConvGeom &g = job.g;
+      if (job.joined) (job.depthwise ? job.dw_x : job.a.x) = x;
+      if ((job.linked || job.joined) && !job.depthwise && job.a.Cf != g.C) {
+        bf16 *xp = (bf16 *)scratch_get(6, (size_t)g.N * job.a.Cf * g.H * g.W * 2);
+        launch_pad_channels_bf16(job.a.x, xp, (int64_t)g.N * g.H * g.W, g.C, job.a.Cf, rt().stream);
+        job.a.x = xp;
+        job.dep_lo[0] = job.dep_hi[0] = 0;
+      }
+    };
+    for (int i = 0; i < g_fronts; ++i) {
+      resolve(g_front[i]);
+      x = launch_job(g_front[i], true);
+    }
+    resolve(g_pending);
+    launch_job(g_pending);
+  }
+  g_fronts = 0;
 }
 
 // [p, p+bytes) is about to be overwritten or freed (`writes`), or merely handed out again:
@@ -476,12 +598,15 @@ void pending_guard_range(const void *p, size_t bytes, bool writes) {
   if (!g_pending.active) return;
   const uintptr_t lo = (uintptr_t)p, hi = lo + bytes;
   if (writes)
-    for (int k = 0; k < 3; ++k)
-      if (ranges_overlap(lo, hi, g_pending.dep_lo[k], g_pending.dep_hi[k])) {
-        if (rt().log) fprintf(stderr, "[occamy] held-back conv runs early: input %d overwritten\n", k);
-        flush_pending();
-        return;
-      }
+    for (int j = 0; j <= g_fronts; ++j) {
+      const ConvJob &job = j < g_fronts ? g_front[j] : g_pending;
+      for (int k = 0; k < 3; ++k)
+        if (ranges_overlap(lo, hi, job.dep_lo[k], job.dep_hi[k])) {
+          if (rt().log) fprintf(stderr, "[occamy] held-back conv runs early: input %d overwritten\n", k);
+          flush_pending();
+          return;
+        }
+    }
   // the tensor it is going to write must also still belong to it
   const uintptr_t olo = (uintptr_t)g_pending.out;
   const size_t elem = g_pending.a.split || g_pending.product ? 4 : 2;
@@ -516,7 +641,7 @@ Role step(Entry &e, bool passive) {
     if (trace_has_elided() && rt().log)
       fprintf(stderr, "[occamy] call sequence left the recorded one after tensors were skipped\n");
   }
-  if (!passive && role != R_ABSORB) {
+  if (!passive && role != R_ABSORB && !((trace_last_flags() & RF_JOIN) && g_pending.active && g_pending.linked)) {
     if (g_pending.active && rt().log)
       fprintf(stderr, "[occamy] held-back conv closed by call sym %d (absorbed %d)\n", e.sym,
               g_pending.absorbed);
@@ -630,6 +755,13 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
                g.S <= 16 && g.R <= 11;
   const Role role = step(e, false);
   if (role == R_SKIP) return y;
+  bool join = false;
+  if (g_pending.active) {   // left by step() because this call was recorded as joining it
+    const ConvGeom &f = g_pending.g;
+    join = role == R_DEFER && e.fusable && !e.parts && g_fronts < 2 && g_pending.out == x && f.N == g.N && f.K == g.C &&
+           f.P == g.H && f.Q == g.W && (depthwise ? g_fronts == 0 : g_fronts == 1 && g.C % 16 == 0);
+    if (!join) flush_pending();
+  }
 
   if (!shape_ok) {
     set_error(997, "convolution: inconsistent shape");
@@ -642,8 +774,23 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
             (int)role);
   if (r.mode != MATH_FP32) {
     ConvJob job;
-    const bool ok = depthwise ? prepare_depthwise(x, w, bias, g, job)
-                              : (g.groups == 1 && prepare_dense(x, w, bias, g, job));
+    const uint8_t flags = trace_last_flags();
+    // (the first of three takes its input as it is)
+    job.linked = role == R_DEFER && (flags & RF_LINK) && (join || (!(flags & RF_JOIN) && is_act16(x, g.N, g.C, g.H, g.W)));
+    job.joined = join;
+    bool ok = depthwise ? prepare_depthwise(x, w, bias, g, job)
+                        : (g.groups == 1 && prepare_dense(x, w, bias, g, job));
+    if (join && ok && g_pending.active) {
+      // nothing else reads what the one in front would have written
+      g_front[g_fronts++] = g_pending;
+      elide(g_pending.out);
+    } else if (join) {
+      // cannot be carried on with, or a constant's upload was about to overwrite something the ones in
+      // front still had to read, and they have run
+      flush_pending();
+      job = ConvJob();
+      ok = depthwise ? prepare_depthwise(x, w, bias, g, job) : prepare_dense(x, w, bias, g, job);
+    }
     if (ok) {
       job.out = y;
       if (role == R_DEFER) {   // later calls of the recorded sequence fold into this one
@@ -1058,7 +1205,7 @@ float *DNNActiveFunc(cudnnContext *, float *x, int64_t dimX[4], int32_t mode, fl
       pending_retarget(y);
       g_pending.g.act = ACT_RELU;
       g_pending.act_set = true;
-      flush_pending();   // an activation closes the chain
+      if (!g_pending.linked) flush_pending();   // an activation closes the chain
       return y;
     }
     flush_pending();
@@ -1099,7 +1246,7 @@ float *CUDAClipFunc(float *x, float *y, int64_t *dimOut, float lo, float hi, int
       g_pending.g.lo = lo;
       g_pending.g.hi = hi;
       g_pending.act_set = true;
-      flush_pending();
+      if (!g_pending.linked) flush_pending();
       return y;
     }
     flush_pending();
@@ -1163,15 +1310,25 @@ float *DNNTensorOpFunc(cudnnContext *, int64_t opMode, float *A, int64_t *dimA, 
     if ((e.kind == CK_BIAS_ADD || e.kind == CK_ROW_BIAS) && dims_ok && A == g_pending.out && !g_pending.bias_set &&
         !g_pending.res_set && !g_pending.act_set) {
       const float *bd = resident_f32(B, (size_t)g.K * 4);
-      if (g_pending.depthwise) g_pending.bias = bd;
-      else g_pending.a.bias = bd;
-      job_track_bias(g_pending, bd, B, g.K);
-      if (!g_pack_was_resident) g_pending.a.consts_ready = 0;
-      g_pending.bias_set = true;
-      pending_retarget(out);
-      return out;
+      bool ready = g_pack_was_resident;
+      const void *block_b = nullptr;
+      if (g_pending.linked && (!g_pending.depthwise || mode_f16())) {
+        block_b = g_pending.depthwise ? packed_for_block(B, PACK_IR_HALF, (size_t)g.K * 2, g.K, 1)
+                                      : packed_for_block(B, PACK_BIAS3, (size_t)g.K * 32, g.K, 0);
+        ready = ready && g_pack_was_resident;
+      }
+      if (g_pending.active) {   // (an upload of B may have had to run it early)
+        if (g_pending.depthwise) g_pending.bias = bd;
+        else g_pending.a.bias = bd;
+        g_pending.block_b = block_b;
+        job_track_bias(g_pending, bd, B, g.K);
+        if (!ready) g_pending.a.consts_ready = 0;
+        g_pending.bias_set = true;
+        pending_retarget(out);
+        return out;
+      }
     }
-    if (e.kind == CK_SAME_ADD && dims_ok && !g_pending.depthwise && !g_pending.product && !g_pending.res_set &&
+    if (g_pending.active && e.kind == CK_SAME_ADD && dims_ok && !g_pending.depthwise && !g_pending.product && !g_pending.res_set &&
         !g_pending.act_set && ((A == g_pending.out) != (B == g_pending.out))) {
       const float *other = A == g_pending.out ? B : A;
       const bool parts = g_pending.a.split && g.K % 16 == 0 && is_parts(other, g.N, g.K, g.P, g.Q);

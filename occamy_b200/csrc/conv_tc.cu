@@ -329,8 +329,8 @@ static CUtensorMapSwizzle swizzle_for(int row_bytes) {
 // bf16 tensor map of rank `rank` (<= 4): dims/box innermost first, strides in bytes for
 // dims 1..rank-1.  `counted` is false only while a plan is built for the allocation-free
 // entry point, which must not touch the lazily initialised runtime state.
-static bool make_map(CUtensorMap *m, const void *ptr, int rank, const uint64_t *dims,
-                     const uint64_t *strides, const uint32_t *box, int row_bytes, bool counted) {
+bool make_map(CUtensorMap *m, const void *ptr, int rank, const uint64_t *dims,
+              const uint64_t *strides, const uint32_t *box, int row_bytes, bool counted) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
   cuuint64_t gd[4], gs[3];
@@ -470,7 +470,7 @@ struct Plan {
   bool ok;
 };
 
-static TcFastDiv make_fastdiv(int d) {
+TcFastDiv make_fastdiv(int d) {
   TcFastDiv f{0u, 0u};
   if (d <= 1) return f;
   int s = 0;

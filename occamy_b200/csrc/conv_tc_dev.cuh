@@ -1219,6 +1219,11 @@ inline void tc_launch_pdl(Kernel kernel, int grid, int threads, size_t smem, cud
 // launcher keeps one flag array and asks this helper whether the attribute still has to be set
 // on the device the launch goes to.
 constexpr int TC_MAX_DEVICES = 64;
+// ---- host helpers (conv_tc.cu)
+// Tiled tensor map over 16-bit elements; rows of `row_bytes` in shared memory, swizzled to match.
+bool make_map(CUtensorMap *m, const void *ptr, int rank, const uint64_t *dims, const uint64_t *strides,
+              const uint32_t *box, int row_bytes, bool counted);
+TcFastDiv make_fastdiv(int d);
 inline bool tc_first_use_on_device(unsigned char (&done)[TC_MAX_DEVICES]) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= TC_MAX_DEVICES) return true;

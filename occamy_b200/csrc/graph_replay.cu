@@ -193,6 +193,7 @@ void close_segment(GraphPlan &plan) {
   s.end = trace_index();
   const bool last = s.end == plan.end;
   if (last) flush_held_back();
+  if (gr.state != CAPTURING) return;   // what was held back needed a new buffer: the capture is broken off
   for (int i = 0; i < 8; ++i) s.counters[i] = r.counters[i] - gr.base_counters[i];
   s.counters[CNT_H2D_SKIPPED] = s.counters[CNT_POOL_HWM] = 0;   // counted as the calls are checked
   s.copies = r.main_copies - gr.base_copies;

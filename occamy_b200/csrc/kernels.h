@@ -168,6 +168,26 @@ void launch_pack_stem_bf16(const float *w, bf16 *out, int C, int R, int S, int C
                            cudaStream_t s);
 bool launch_stem_pool(const StemPoolArgs &a, int *err_word, int num_sms, cudaStream_t s);
 
+// ---- inverted residual: 1x1 -> 3x3 depthwise (pad 1) -> 1x1 [+ shortcut] (inverted_residual.cu) -----
+struct IrArgs {
+  const bf16 *x;                // 16-bit NHWC [N][H][W][C]
+  const bf16 *w1, *w3;          // [E][C padded to 16], [K][E]
+  const void *w2, *b2;          // [9][E] and [E] (or null): fp16 (launch_pack_ir_half), in the bf16 mode fp32
+  const bf16 *b1;               // launch_pack_bias3 form
+  const float *b3;              // or null
+  const bf16 *residual;         // like y, or null
+  bf16 *y;                      // [N][P][Q][K]
+  int N, H, W, C, E, K, P, Q, stride;
+  float lo[3], hi[3];           // clamp behind each stage
+  int f16, consts_ready;
+};
+// bias [E] -> 16-bit [E][16]: three parts that add up to it, zeros
+void launch_pack_bias3(const float *b, bf16 *out, int E, bool f16, cudaStream_t s);
+// fp32 [E][T] -> fp16 [T][E]
+void launch_pack_ir_half(const float *w, void *out, int E, int T, cudaStream_t s);
+bool ir_supported(int N, int C, int E, int K, int H, int W, int P, int Q, int stride, bool f16);
+bool launch_ir(const IrArgs &a, cudaStream_t s);
+
 // Enqueues a one-thread kernel whose bounded mbarrier wait must run out (see conv_tc.cu).
 void launch_selftest_bounded_wait(cudaStream_t s);
 

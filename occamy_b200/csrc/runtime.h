@@ -93,8 +93,8 @@ struct Runtime {
   std::unordered_map<WeightKey, PackedWeight, WeightKeyHash> wcache;
   // host sources whose packed form is resident: source -> (bytes, fingerprint)
   std::unordered_map<const void *, std::pair<size_t, uint64_t>> resident;
-  void *scratch[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-  size_t scratch_bytes[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  void *scratch[9] = {};
+  size_t scratch_bytes[9] = {};
   int *dev_err = nullptr;   // word the kernels' bounded waits report into, as the device sees it
   int *host_err = nullptr;  // the same word (mapped host memory)
   void *host_stage = nullptr;   // pinned, STAGE_BYTES: small results on their way to pageable memory

@@ -5,6 +5,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "kernels.h"
 #include "runtime.h"
 
 namespace occ {
@@ -125,7 +126,7 @@ bool only_parts_read(const std::vector<Entry> &rec, const std::vector<uint8_t> &
       if (!e.in[k] || !overlaps(e.in[k], e.in_bytes[k] > 0 ? e.in_bytes[k] : 1, p, bytes)) continue;
       if (e.in[k] != p || e.in_bytes[k] != bytes) return false;
       const bool conv = (e.sym == S_CONV || e.sym == S_CONV_BIAS_ACT) && k == 0 && e.parts;
-      const bool sum = e.sym == S_TENSOR_OP && e.kind == CK_SAME_ADD && (roles[t] & 0xF) == R_ABSORB;
+      const bool sum = e.sym == S_TENSOR_OP && e.kind == CK_SAME_ADD && (roles[t] & ROLE_BITS) == R_ABSORB;
       const bool pool = e.sym == S_MAXPOOL || e.sym == S_AVGPOOL || e.sym == S_REDUCE;
       if (!conv && !sum && !pool) return false;
       any = true;
@@ -144,6 +145,10 @@ bool only_parts_read(const std::vector<Entry> &rec, const std::vector<uint8_t> &
 void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles, std::vector<int> &reader) {
   roles.assign(rec.size(), R_EAGER);
   reader.assign(rec.size(), -1);
+  // of every convolution: the last call folded into it, and the tensor that one writes
+  std::vector<size_t> chain_last(rec.size(), 0);
+  std::vector<uintptr_t> chain_out(rec.size(), 0);
+  std::vector<bool> chain_res(rec.size(), false);
   for (size_t i = 0; i < rec.size(); ++i) {
     const Entry &c = rec[i];
     if (c.sym == S_D2D && (reader[i] = only_convs_read(rec, c.out, c.out_bytes, i + 1)) >= 0)
@@ -238,12 +243,55 @@ void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles, std::ve
         break;
       }
     }
+    chain_last[i] = members.empty() ? i : members.back();
+    chain_out[i] = cur;
+    chain_res[i] = res_set;
     if (members.empty()) continue;
     roles[i] |= R_DEFER;
     for (size_t m : members) roles[m] |= R_ABSORB;
   }
+  // Inverted residuals: a 1x1 convolution whose result only a 3x3 depthwise one reads, whose result only
+  // another 1x1 one reads.
+  auto next_alone = [&](size_t i) -> size_t {   // the convolution that alone reads the chain of `i`, or 0
+    const uintptr_t cur = chain_out[i];
+    const int64_t bytes = rec[i].out_bytes;
+    for (size_t j = chain_last[i] + 1; j < rec.size(); ++j) {
+      const Entry &f = rec[j];
+      if (is_passive(f.sym)) {
+        if ((f.sym == S_MEMOFFSET || f.sym == S_MALLOC) && overlaps(f.out, f.out_bytes, cur, bytes)) return 0;
+        if (f.sym == S_DEALLOC && f.out == cur) return 0;
+        continue;
+      }
+      const bool conv = (f.sym == S_CONV || f.sym == S_CONV_BIAS_ACT) && f.fusable && !f.parts && f.in[0] == cur &&
+                        f.in_bytes[0] == bytes && f.in[1] != cur;
+      return conv && dies_unread(rec, cur, bytes, j + 1) ? j : 0;
+    }
+    return 0;
+  };
+  auto one_by_one = [](const Entry &e) {
+    const int64_t *v = e.args.v;   // dX[4], dW[4], pads[2], strides[2], groups
+    return !e.depthwise && v[6] == 1 && v[7] == 1 && v[8] == 0 && v[9] == 0 && v[10] == 1 && v[11] == 1 && v[12] == 1;
+  };
+  for (size_t i = 0; i < rec.size(); ++i) {
+    const Entry &a = rec[i];
+    if ((a.sym != S_CONV && a.sym != S_CONV_BIAS_ACT) || !a.fusable || a.parts || !one_by_one(a) || chain_res[i])
+      continue;
+    const size_t j = next_alone(i);
+    if (!j) continue;
+    const int64_t *w = rec[j].args.v;
+    if (!rec[j].depthwise || w[6] != 3 || w[7] != 3 || w[8] != 1 || w[9] != 1 || w[10] != w[11] || chain_res[j]) continue;
+    const size_t k = next_alone(j);
+    if (!k || !one_by_one(rec[k])) continue;
+    const int64_t *v = a.args.v;
+    if (!ir_supported((int)v[0], (int)v[1], (int)v[4], (int)rec[k].args.v[4], (int)v[2], (int)v[3],
+                      (int)rec[k].dims[2], (int)rec[k].dims[3], (int)w[10], mode_f16()))
+      continue;
+    roles[i] = (uint8_t)(R_DEFER | RF_LINK);
+    roles[j] = (uint8_t)(R_DEFER | RF_LINK | RF_JOIN);
+    roles[k] = (uint8_t)(R_DEFER | RF_JOIN);
+  }
   for (size_t i = 0; i < rec.size(); ++i)   // (after the roles are known)
-    if ((rec[i].parts || (roles[i] & 0xF) == R_ABSORB) &&
+    if ((rec[i].parts || (roles[i] & ROLE_BITS) == R_ABSORB) &&
         only_parts_read(rec, roles, rec[i].out, rec[i].out_bytes, i + 1))
       roles[i] |= RF_FOR_PARTS;
 }
@@ -342,8 +390,8 @@ Role trace_step(Entry &e, bool *deviated) {
       // recorded programs that share this prefix must agree on the call's role (two models
       // with the same first layers may continue differently); otherwise it runs as it stands
       const uint8_t r = ts.programs[ts.cands[0]].roles[index];
-      role = (Role)(r & 0x0F);
-      ts.last_flags = r & 0xF0;
+      role = (Role)(r & ROLE_BITS);
+      ts.last_flags = r & (uint8_t)~ROLE_BITS;
       for (size_t k = 1; k < keep; ++k)
         if (ts.programs[ts.cands[k]].roles[index] != r ||
             ((r & RF_FOR_CONV) && ts.programs[ts.cands[k]].sigs[ts.programs[ts.cands[k]].reader[index]] !=

@@ -6,6 +6,7 @@
 // epilogue).  When an inference ends it looks for chains
 //     convolution -> [+ bias [1,K,1,1]] -> [+ same-shape tensor] -> [ReLU | Clip]
 //     matrix product -> [+ bias row] -> [ReLU]
+//     1x1 convolution chain -> 3x3 depthwise chain -> 1x1 convolution chain
 // (and, for a few-channel stem convolution, a 3x3 / stride 2 max pool behind it)
 // whose intermediate results nobody else reads before their memory is handed out again,
 // and marks them.  The next time the same call sequence comes by, the convolution of such
@@ -84,6 +85,11 @@ constexpr uint8_t RF_FOR_CONV = 0x20;
 // on a convolution in fp32 mode or a call folded into one: all that reads the result takes it in three
 // planes of parts (FMT_PARTS)
 constexpr uint8_t RF_FOR_PARTS = 0x40;
+// on convolutions that run together with the next one (RF_LINK) or the one before (RF_JOIN): the three of
+// an inverted residual, which become one kernel
+constexpr uint8_t RF_LINK = 0x04;
+constexpr uint8_t RF_JOIN = 0x08;
+constexpr uint8_t ROLE_BITS = 0x03;
 struct TraceProgram {
   std::vector<uint64_t> sigs;
   std::vector<uint8_t> roles;   // Role | RF_*

@@ -1,0 +1,54 @@
+"""The inverted-residual kernel (1x1 -> 3x3 depthwise -> 1x1 as one launch) at the edges of its tiles, chunks
+and clusters, against the CPU oracle."""
+import pytest
+
+from helpers import max_rel_err, run_graph_oracle
+from occamy_b200 import graphs, replay
+from occamy_b200 import runtime as rt
+
+pytestmark = pytest.mark.gpu
+
+# (N, C, H, W, E, K, stride): channels that are no multiple of a chunk or of the MMA's 16; one tile and many;
+# ragged tiles; reductions in one to three input tiles; chunks shared by 1 to 8 CTAs
+SHAPES = [
+    (1, 16, 13, 9, 96, 24, 2),
+    (2, 24, 20, 28, 144, 24, 1),
+    (1, 24, 15, 17, 144, 32, 2),
+    (3, 32, 28, 28, 192, 32, 1),
+    (1, 64, 14, 14, 384, 96, 1),
+    (3, 96, 14, 11, 576, 160, 2),
+    (1, 160, 7, 7, 960, 160, 1),
+    (40, 160, 7, 7, 960, 160, 1),
+    (2, 40, 5, 3, 48, 8, 1),
+    (30, 16, 60, 60, 96, 24, 2),
+]
+
+
+@pytest.mark.parametrize("mode", [rt.MATH_BF16, rt.MATH_F16])
+@pytest.mark.parametrize("fuse", [replay.FUSE_REFERENCE, replay.FUSE_NONE])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_block(binding, shape, fuse, mode):
+    N, C, H, W, E, K, st = shape
+    g = graphs.Graph((N, C, H, W), seed=sum(shape))
+    x = g.clip(g.conv(0, *g.he_conv(C, C, 1, 1)), 0.0, 6.0)
+    y = g.clip(g.conv(x, *g.he_conv(E, C, 1, 1)), 0.0, 6.0)
+    y = g.clip(g.conv(y, *g.he_conv(E, 1, 3, 3), groups=E, pads=(1, 1), strides=(st, st)), 0.0, 6.0)
+    y = g.conv(y, *g.he_conv(K, E, 1, 1))
+    if st == 1 and K == C:
+        y = g.add(x, y)
+    g.mark_output(y)
+    v = graphs.make_input(g, 1)
+    (want,) = run_graph_oracle(g, v)
+    rt.set_math_mode(mode)
+    rt.lib().occamy_set_cross_call_fusion(0)   # forgets what was recorded
+    rt.lib().occamy_set_cross_call_fusion(1)
+    p = g.to_program()
+    p.lower(fuse=fuse)
+    launches = []
+    for _ in range(4):
+        before = rt.counters()["launches"]
+        (got,) = p.run(binding, v)
+        launches.append(rt.counters()["launches"] - before)
+        assert max_rel_err(got, want) <= 2e-2
+    assert launches[2] < launches[0]
+    assert rt.last_error() == 0
