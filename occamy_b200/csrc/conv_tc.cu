@@ -759,27 +759,39 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
 #endif
   // worth it only where the tensor pipe is the limit: the transposing epilogue is slower
   // than the plain one, which hurts the HBM-bound 1x1 layers
-  // 3x3 / stride 1 / pad 1 with 64 -> 64 channels and rows of at most 126 pixels: the input
-  // block of a tile is loaded once and the taps are windows of it (TC_MODE_HALO)
+  // 3x3 / stride 1 / pad 1 with 64 -> 64 channels: the input block of a tile is loaded once and the taps are
+  // windows of it (TC_MODE_HALO)
   const bool halo = allow_halo && halo_allowed && !a.f16 && !a.out_f32 && a.R == 3 && a.S == 3 &&
                     a.stride_h == 1 && a.stride_w == 1 && a.pad_h == 1 && a.pad_w == 1 &&
-                    a.Cf == 64 && a.K == 64 && a.W + 2 <= 128 && a.w_step == 0 && a.Q == a.W &&
+                    a.Cf == 64 && a.K == 64 && a.w_step == 0 && a.Q == a.W &&
                     a.P == a.H;
   const bool pn = !halo && pn_allowed && !a.f16 && !a.out_f32 && a.K <= 128 && a.R * a.S > 1 &&
                   a.R * a.S * a.Cf >= 9 * 64;
   pl.pn = pn;
   if (halo) {
-    p.tw = a.W + 2;                      // two junk columns that the store clips
-    p.th = 128 / p.tw < a.P ? 128 / p.tw : a.P;
+    // Column strips `tw` wide: the fewest tiles, then the smallest input block (its rows carry a column on
+    // either side, and there is a row above and below).
+    long best_tiles = -1, best_block = 0;
+    for (int n = 1; n <= (a.W + 7) / 8; ++n) {
+      const int w = (a.W + n - 1) / n, wp = w + 2, h = 128 / wp < a.P ? 128 / wp : a.P;
+      if (h < 1) continue;
+      const long tiles = (long)((a.W + w - 1) / w) * ((a.P + h - 1) / h), block = (long)(h + 2) * wp;
+      if (best_tiles < 0 || tiles < best_tiles || (tiles == best_tiles && block < best_block)) {
+        best_tiles = tiles;
+        best_block = block;
+        p.tw = w;
+        p.th = h;
+      }
+    }
     p.tn = 1;
     p.halo = 1;
-    p.halo_wp = p.tw;
-    p.halo_a_bytes = ((p.th + 2) * p.tw * 128 + 1023) / 1024 * 1024;
+    p.halo_wp = p.tw + 2;
+    p.halo_a_bytes = ((p.th + 2) * p.halo_wp * 128 + 1023) / 1024 * 1024;
   } else {
     choose_box(Qg, Pg, Ng, pn ? 256 : 128, &p.tw, &p.th, &p.tn);
   }
   p.n_mma = (p.tw * p.th * p.tn + 15) / 16 * 16;
-  p.tiles_w = halo ? 1 : (Qg + p.tw - 1) / p.tw;
+  p.tiles_w = (Qg + p.tw - 1) / p.tw;
   p.tiles_h = (Pg + p.th - 1) / p.th;
   p.tiles_n = (Ng + p.tn - 1) / p.tn;
   const int nsm = num_sms > 0 ? num_sms : 148;
@@ -827,7 +839,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   if (halo) {
     const uint64_t dims[4] = {(uint64_t)a.Cf, (uint64_t)a.W, (uint64_t)a.H, (uint64_t)a.N};
     const uint64_t st[3] = {(uint64_t)a.Cf * 2, (uint64_t)a.W * a.Cf * 2, (uint64_t)a.H * a.W * a.Cf * 2};
-    const uint32_t box[4] = {64u, (uint32_t)p.tw, (uint32_t)(p.th + 2), 1u};
+    const uint32_t box[4] = {64u, (uint32_t)p.halo_wp, (uint32_t)(p.th + 2), 1u};
     ok &= make_map(&p.tmA[0], a.x, 4, dims, st, box, 128, counted);
     p.num_taps = 9;
   } else {

@@ -100,11 +100,11 @@ constexpr int TC_MODE_RES = 1;     // adds a residual tensor
 constexpr int TC_MODE_CLAMP = 2;   // general clamp to [lo, hi]; otherwise ReLU
 constexpr int TC_MODE_F32 = 4;     // fp32 row-major output straight to global memory (GEMM head)
 // 3x3 / stride 1 / pad 1 with 64 input channels and resident weights: the producer loads a
-// tile's input block (its rows plus one row above and below, whole image width plus one zero
-// column on either side) ONCE and the nine taps are windows of that block, shifted by whole
-// pixels - a swizzled operand may start at any multiple of 128 bytes inside a 1024-aligned
-// buffer.  The tile is th full rows of width W + 2; its two extra columns are junk that the
-// TMA store clips.
+// tile's input block (its rows plus one row above and below, its columns plus one on either side)
+// ONCE and the nine taps are windows of that block, shifted by whole pixels - a swizzled operand may
+// start at any multiple of 128 bytes inside a 1024-aligned buffer.  The accumulator's rows are th rows
+// of the block's width; two of its columns are junk that the epilogue leaves out of the slab.
+// 64->64 at 224x224, batch 64: 509 us in the pixel-N form, whose k-steps load every pixel nine times,
 constexpr int TC_MODE_HALO = 8;
 // Operands and output are fp16 instead of bf16 (same MMA kind, same rate, other format bits
 // in the instruction descriptor and other conversion instructions in the epilogue).
@@ -674,8 +674,8 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
             break;
           }
           mbar_expect_tx(full_bar(stage), blk_bytes);
-          // column -1 and row p0 - 1 onwards; what lies outside the image arrives as zeros
-          tma_load_4d(sA + stage * a_bytes, &p.tmA[0], full_bar(stage), 0, -1, tl.p0 - 1, tl.n0);
+          // column q0 - 1 and row p0 - 1 onwards; what lies outside the image arrives as zeros
+          tma_load_4d(sA + stage * a_bytes, &p.tmA[0], full_bar(stage), 0, tl.q0 - 1, tl.p0 - 1, tl.n0);
           if (++stage == stages) {
             stage = 0;
             phase ^= 1u;
@@ -996,10 +996,18 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
     const int part = (warp - 2) >> 2;        // which part of a slab's channels
     const int row = quad * 32 + lane;        // accumulator row == pixel index in the tile
     const int et = threadIdx.x - 64;         // 0..EPI_THREADS-1
+    // halo form: accumulator rows run through the input block's columns, a slab holds the tile's only
+    int srow = row;
+    bool keep = true;
+    if constexpr (HALO) {
+      const int h = row / p.halo_wp, w = row - h * p.halo_wp;
+      keep = w < p.tw && h < p.th;
+      srow = keep ? h * p.tw + w : 0;
+    }
     // swizzled offsets of this thread's 16-byte pieces inside a slab buffer
     uint32_t soff[CW / 8];
 #pragma unroll
-    for (int c4 = 0; c4 < CW / 8; ++c4) soff[c4] = slab_off(row, part * (CW / 8) + c4, DC * 2);
+    for (int c4 = 0; c4 < CW / 8; ++c4) soff[c4] = slab_off(srow, part * (CW / 8) + c4, DC * 2);
     // The whole bias vector goes to shared memory once: a global load per tile would put
     // the memory latency on every tile's critical path.
     for (int i = et; i < p.bias_floats; i += EPI_THREADS)
@@ -1115,8 +1123,9 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
           }
 #pragma unroll
           for (int c4 = 0; c4 < CW / 8; ++c4)
-            *reinterpret_cast<uint4 *>(dptr + soff[c4]) =
-                make_uint4(pk[c4 * 4], pk[c4 * 4 + 1], pk[c4 * 4 + 2], pk[c4 * 4 + 3]);
+            if (keep)
+              *reinterpret_cast<uint4 *>(dptr + soff[c4]) =
+                  make_uint4(pk[c4 * 4], pk[c4 * 4 + 1], pk[c4 * 4 + 2], pk[c4 * 4 + 3]);
           // this warp's part of the slab is written: tell the store thread
           fence_async_smem();
           __syncwarp();
