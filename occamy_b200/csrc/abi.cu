@@ -625,6 +625,7 @@ Role step(Entry &e, bool passive) {
   rt().before_write = before_write_hook;
   rt().home_held = home_held_hook;
   if (graph_covers(e)) return R_SKIP;
+  graph_uncovered();
   bool deviated = false;
   const Role role = trace_step(e, &deviated);
   if (deviated) {
@@ -1003,6 +1004,15 @@ cudaError_t wrapDNNMemcpy(void *dst, const void *src, size_t count_, int kind,
       graph_before_upload();
       trace_mark_uploaded();
       pending_guard_range(dst, count_, true);
+    }
+    if (kind == 1 && whole && count_ >= (4u << 20)) {
+      if (!g_copy_stream) OCC_CUDA(cudaStreamCreateWithFlags(&g_copy_stream, cudaStreamNonBlocking));
+      if (graph_upload_in_pieces(dst, src, count_, g_copy_stream)) {
+        count(CNT_H2D_BYTES, (int64_t)count_);
+        rec->fmt = FMT_F32;
+        rec->home = rec->dev_src = nullptr;
+        return cudaSuccess;
+      }
     }
     const bool in_pool = g_cur_pool && (uintptr_t)dst >= (uintptr_t)g_cur_pool &&
                          (uintptr_t)dst + count_ <= (uintptr_t)g_cur_pool + g_cur_pool_bytes;
@@ -1679,13 +1689,10 @@ void occamy_internal_opaque_call(void) {
 void occ::flush_held_back() { flush_pending(); }
 bool occ::anything_held_back() { return g_pending.active; }
 
-// The call of entry `e`, its pool pointers `shift` bytes further on; `host` is the source of a constant.
-void occ::run_again(const Entry &e, intptr_t shift, uintptr_t pool_base, size_t pool_bytes, const void *host) {
+// The call of entry `e`, its pointers where `place` says; `host` is the source of a constant.
+void occ::run_again(const Entry &e, const std::function<void *(void *)> &place, const void *host) {
   void *p[4];
-  for (int k = 0; k < 4; ++k) {
-    const uintptr_t a = (uintptr_t)e.args.p[k];
-    p[k] = (void *)(a >= pool_base && a < pool_base + pool_bytes ? a + shift : a);
-  }
+  for (int k = 0; k < 4; ++k) p[k] = place(e.args.p[k]);
   float *const f[4] = {(float *)p[0], (float *)p[1], (float *)p[2], (float *)p[3]};
   int64_t v[24];
   memcpy(v, e.args.v, sizeof(v));
@@ -1819,6 +1826,7 @@ void occamy_clear_weight_cache(void) {
     if (kv.second.dev) cudaFree(kv.second.dev);
   r.wcache.clear();
   r.resident.clear();
+  graph_free_memory();
   for (size_t i = 0; i < r.homes.size();) {   // buffers no tensor is in
     bool used = false;
     for (const auto &kv : r.recs) used = used || kv.second.home == r.homes[i].ptr;

@@ -25,8 +25,15 @@ struct SavedRec {
   TensorRec rec;
 };
 
+// A window cut up by images: its calls are made for a piece of the batch after the other, each piece as one
+// graph, on tensors in memory of the runtime's.  What it is for is a batch that comes from the host: the
+// pieces are computed while the later ones are still on their way (batch 256 of a ResNet-50 takes 2.9 ms to
+// arrive and 3.1 to compute).
+constexpr int MAX_PIECES = 3;
+
 struct Segment {
   cudaGraphExec_t exec = nullptr;   // null: the calls enqueue nothing
+  cudaGraphExec_t pieces[MAX_PIECES] = {};   // instead of exec, in a window cut up by images
   size_t end = 0;                   // one past its last call
   std::vector<SavedRec> after;      // registry records of the pool when it has been enqueued
   int64_t counters[8] = {};         // what its calls count
@@ -46,6 +53,7 @@ struct Variant {
   std::vector<SavedRec> before;   // the pool's records when the window began: the forms its inputs are in
   std::vector<Constant> constants;
   std::vector<Segment> segments;
+  bool pieces = false;            // one segment, cut up by images
 };
 
 }  // namespace
@@ -54,6 +62,7 @@ struct GraphPlan {
   size_t begin = 0, end = 0;   // the window: calls [begin, end)
   bool ready = false;          // an inference ran with nothing to upload or allocate inside it
   int failures = 0;
+  int piece_failures = 0;
   std::vector<std::unique_ptr<Variant>> variants;
   ~GraphPlan();
 };
@@ -80,6 +89,11 @@ struct Replay {
   int64_t base_counters[8] = {};
   int64_t base_copies = 0, base_chains = 0;
   std::vector<cudaGraphExec_t> trash;   // launched once, destroyed when the stream is idle
+  // an upload that is being made in pieces, and the event behind each
+  int pieces_coming = 0;
+  cudaEvent_t piece_here[MAX_PIECES] = {};
+  void *piece_memory = nullptr;         // where the tensors of a window cut up by images are
+  size_t piece_bytes = 0;
 };
 Replay &gr = *new Replay;   // never destroyed, like the programs it refers to
 
@@ -271,9 +285,269 @@ void take_back() {
   trace_rewind(p, from);
   gr.again = true;
   for (size_t i = from; i < upto; ++i)
-    run_again(p->entries[i], (intptr_t)(base - p->pool_base), p->pool_base, p->pool_bytes,
+    run_again(p->entries[i],
+              [&](void *q) {
+                const uintptr_t a = (uintptr_t)q;
+                return (void *)(a >= p->pool_base && a < p->pool_base + p->pool_bytes ? a - p->pool_base + base : a);
+              },
               gr.hosts[i - p->graph->begin]);
   gr.again = false;
+}
+
+void wait_for_upload() {
+  if (!gr.pieces_coming) return;
+  OCC_CUDA(cudaStreamWaitEvent(rt().stream, gr.piece_here[gr.pieces_coming - 1], 0));
+  gr.pieces_coming = 0;
+}
+
+// ---- windows cut up by images -------------------------------------------------------
+// Images of each piece: the first is what is waited for, so it is the smallest (256 images: 64, 96, 96
+// took 4.5 ms where three of 85 took 4.7).  None for batches below 128, whose pieces lose more in
+// efficiency than the upload takes.
+int piece_images(int64_t n, int64_t *images) {
+  if (n < 128) return 0;
+  images[0] = n / 4 / 8 * 8;
+  images[1] = (n - images[0]) / 2 / 8 * 8;
+  images[2] = n - images[0] - images[1];
+  return MAX_PIECES;
+}
+
+struct Cut {
+  std::vector<Entry> calls;    // of the whole inference, those of the window for one piece
+  std::vector<uint8_t> roles;
+  uintptr_t x = 0, out = 0;
+  int64_t x_bytes = 0, out_bytes = 0, batch = 0;
+  size_t x_until = 0, out_from = 0;   // calls between which these addresses mean the input and the result
+};
+
+// The call that uploads the batch: the one right before the window.
+bool find_input(const TraceProgram &p, Cut &c) {
+  const size_t begin = p.graph->begin;
+  if (begin == 0 || p.entries[begin - 1].sym != S_H2D) return false;
+  const Entry &up = p.entries[begin - 1];
+  c.x = up.out;
+  c.x_bytes = up.out_bytes;
+  for (size_t i = begin; i < p.graph->end; ++i) {
+    const Entry &e = p.entries[i];
+    if (e.sym != S_CONV && e.sym != S_CONV_BIAS_ACT) continue;
+    c.batch = e.args.v[0];
+    return e.in[0] == c.x && e.in_bytes[0] == c.x_bytes;
+  }
+  return false;
+}
+
+// Rewrites the window's calls for `images` of the batch; false when a call is not one image after the other.
+bool cut_up(const TraceProgram &p, int64_t images, Cut &c) {
+  const int64_t N = c.batch;
+  const size_t begin = p.graph->begin, end = p.graph->end;
+  std::map<uintptr_t, int64_t> batch, constants;   // tensors by address, with their bytes
+  batch[c.x] = c.x_bytes;
+  c.x_until = end;
+  c.calls = p.entries;
+  auto drop = [](std::map<uintptr_t, int64_t> &m, uintptr_t a, int64_t bytes) {
+    for (auto it = m.begin(); it != m.end();)
+      if (it->first < a + (uintptr_t)bytes && a < it->first + (uintptr_t)it->second) it = m.erase(it);
+      else ++it;
+  };
+  std::map<uintptr_t, size_t> handed_out;   // last call that did
+  for (size_t i = 0; i < end; ++i) {
+    Entry &e = c.calls[i];
+    int64_t *v = e.args.v;
+    if (e.sym == S_MEMOFFSET) {
+      drop(batch, e.out, e.out_bytes);
+      drop(constants, e.out, e.out_bytes);
+      handed_out[e.out] = i;
+      if (i >= begin && c.x_until == end && !batch.count(c.x)) c.x_until = i;
+      if (i < begin && e.out == c.x) batch[c.x] = c.x_bytes;
+      continue;
+    }
+    if (e.sym == S_H2D) {
+      if (i >= begin) {   // (one that is there before the batch is not the pieces' own)
+        if (!handed_out.count(e.out) || handed_out[e.out] < begin) return false;
+        constants[e.out] = e.out_bytes;
+      }
+      continue;
+    }
+    if (i < begin) continue;
+    auto scaled = [&](int64_t &d) {
+      if (d != N) return false;
+      d = images;
+      return true;
+    };
+    if (!batch.count(e.in[0])) return false;
+    bool ok = true, second_scaled = false;
+    switch (e.sym) {
+      case S_CONV:
+      case S_CONV_BIAS_ACT:
+        ok = scaled(v[0]) && constants.count(e.in[1]) && (!e.in[2] || constants.count(e.in[2]));
+        break;
+      case S_ACTIVE: ok = scaled(v[0]); break;
+      case S_CLIP: ok = scaled(v[1]); break;
+      case S_TENSOR_OP:
+        ok = scaled(v[3]);
+        if (e.in[1] && batch.count(e.in[1])) ok = ok && v[1] == v[2] && scaled(v[3 + v[1]]) && (second_scaled = true);
+        else ok = ok && (!e.in[1] || (constants.count(e.in[1]) && (v[2] < v[1] || v[3 + v[1]] == 1)));
+        break;
+      case S_MAXPOOL:
+      case S_AVGPOOL: ok = scaled(v[0]) && scaled(v[4]); break;
+      case S_REDUCE: ok = scaled(v[2]) && scaled(v[2 + v[0]]); break;
+      case S_MATMUL: ok = v[4] == 0 && scaled(v[0]) && constants.count(e.in[1]); break;
+      case S_SOFTMAX: ok = scaled(v[2]) && v[0] > 0; break;
+      case S_FLATTEN:
+      case S_RESHAPE: ok = scaled(v[1]); break;
+      default: ok = false;
+    }
+    if (!ok || e.out_bytes % N || e.in_bytes[0] % N) return false;
+    batch[e.out] = e.out_bytes;
+    if (e.dims[0] == N) e.dims[0] = images;
+    e.out_bytes = e.out_bytes / N * images;
+    e.in_bytes[0] = e.in_bytes[0] / N * images;
+    if (second_scaled) e.in_bytes[1] = e.in_bytes[1] / N * images;
+    if (e.sym == S_MATMUL && e.in[2]) e.in_bytes[2] = e.out_bytes;
+  }
+  // one tensor is read behind the window: rows of fp32
+  for (size_t i = end; i < c.calls.size(); ++i) {
+    const Entry &e = c.calls[i];
+    for (int k = 0; k < 3; ++k) {
+      if (!e.in[k] || e.in[k] < p.pool_base || e.in[k] >= p.pool_base + p.pool_bytes) continue;
+      if ((c.out && e.in[k] != c.out) || !batch.count(e.in[k]) || e.in_bytes[k] != batch[e.in[k]]) return false;
+      c.out = e.in[k];
+      c.out_bytes = e.in_bytes[k];
+    }
+  }
+  if (!c.out || !handed_out.count(c.out) || handed_out[c.out] < begin) return false;
+  c.out_from = handed_out[c.out];
+  for (size_t i = end; i-- > begin;)
+    if (c.calls[i].out == c.out && computes(c.calls[i].sym)) {
+      const int sym = c.calls[i].sym;
+      if (sym != S_MATMUL && sym != S_SOFTMAX && !(sym == S_TENSOR_OP && c.calls[i].kind == CK_ROW_BIAS)) return false;
+      break;
+    }
+  trace_roles(c.calls, c.roles);
+  return true;
+}
+
+// Makes the window's calls for one piece: images [at, at + images) of the batch.
+void make_piece(const TraceProgram &p, const Cut &c, int64_t at, int64_t images, const std::vector<const void *> &hosts) {
+  const uintptr_t real = trace_pool_base(), mine = (uintptr_t)gr.piece_memory;
+  const uintptr_t x = c.x - p.pool_base + real + (uintptr_t)(c.x_bytes / c.batch * at);
+  const uintptr_t out = mine + p.pool_bytes + (uintptr_t)(c.out_bytes / c.batch * at);
+  gr.again = true;
+  for (size_t i = p.graph->begin; i < p.graph->end; ++i) {
+    if (i == c.out_from) {
+      reg_new((void *)out, (size_t)(c.out_bytes / c.batch * images), FMT_ZERO);
+      continue;
+    }
+    trace_force(c.roles[i]);
+    run_again(c.calls[i],
+              [&](void *q) -> void * {
+                const uintptr_t a = (uintptr_t)q;
+                if (a < p.pool_base || a >= p.pool_base + p.pool_bytes) return q;
+                if (a == c.x && i < c.x_until) return (void *)x;
+                if (a == c.out && i > c.out_from) return (void *)out;
+                return (void *)(a - p.pool_base + mine);
+              },
+              hosts[i - p.graph->begin]);
+  }
+  trace_force_end();
+  flush_held_back();
+  gr.again = false;
+}
+
+// An inference has just run its window as the graphs of `v`: make the variant that is cut up by images.
+void build_pieces(TraceProgram &p, const Variant &v) {
+  GraphPlan &plan = *p.graph;
+  Cut c;
+  int64_t images[MAX_PIECES];
+  if (plan.piece_failures >= MAX_FAILURES) return;
+  for (const auto &o : plan.variants)
+    if (o->pieces && o->pool_base == v.pool_base && o->flags == v.flags && o->epoch == gr.epoch) return;
+  if (!find_input(p, c) || c.x_bytes < (16 << 20) || !piece_images(c.batch, images) || !cut_up(p, images[2], c)) {
+    plan.piece_failures = MAX_FAILURES;
+    return;
+  }
+  Runtime &r = rt();
+  plan.piece_failures++;   // taken back below
+  const size_t bytes = p.pool_bytes + (size_t)c.out_bytes;
+  if (gr.piece_bytes < bytes) {
+    graph_free_memory();
+    if (cudaMalloc(&gr.piece_memory, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      gr.piece_memory = nullptr;
+      plan.piece_failures = MAX_FAILURES;
+      return;
+    }
+    gr.piece_bytes = bytes;
+  }
+  const uintptr_t mine = (uintptr_t)gr.piece_memory;
+  const std::vector<const void *> hosts = gr.hosts;
+  int64_t counters[8];
+  memcpy(counters, r.counters, sizeof(counters));
+  const int64_t copies = r.main_copies;
+  auto fresh = [&]() { reg_drop_range((void *)mine, gr.piece_bytes); };
+  // the batch's own record covers its place, as it will when the window begins
+  restore_registry(v.before, v.pool_base, trace_pool_bytes());
+  // once as they are, the largest piece: buffers are allocated, constants packed
+  fresh();
+  make_piece(p, c, c.batch - images[2], images[2], hosts);
+  std::unique_ptr<Variant> n(new Variant);
+  n->pool_base = v.pool_base;
+  n->flags = v.flags;
+  n->before = v.before;
+  n->constants = v.constants;
+  n->pieces = true;
+  n->segments.resize(1);
+  Segment &s = n->segments[0];
+  s.end = plan.end;
+  bool ok = true;
+  const uint64_t epoch = gr.epoch;
+  int64_t at = 0;
+  for (int k = 0; k < MAX_PIECES && ok; at += images[k++]) {
+    Cut piece = c;
+    piece.out = 0;
+    ok = cut_up(p, images[k], piece) && cudaStreamSynchronize(r.stream) == cudaSuccess &&
+         cudaStreamBeginCapture(r.stream, cudaStreamCaptureModeRelaxed) == cudaSuccess;
+    if (!ok) break;
+    fresh();
+    memcpy(gr.base_counters, r.counters, sizeof(gr.base_counters));
+    const int64_t copies0 = r.main_copies, chains0 = trace_fused_chains();
+    make_piece(p, piece, at, images[k], hosts);
+    if (k + 1 == MAX_PIECES)
+      OCC_CUDA(cudaMemcpyAsync((void *)(c.out - p.pool_base + v.pool_base), (void *)(mine + p.pool_bytes),
+                               (size_t)c.out_bytes, cudaMemcpyDeviceToDevice, r.stream));
+    cudaGraph_t g = nullptr;
+    ok = cudaStreamEndCapture(r.stream, &g) == cudaSuccess && g &&
+         cudaGraphInstantiate(&s.pieces[k], g, 0) == cudaSuccess;
+    if (g) cudaGraphDestroy(g);
+    for (int i = 0; i < 8; ++i) s.counters[i] += r.counters[i] - gr.base_counters[i];
+    s.copies += r.main_copies - copies0;
+    s.chains += trace_fused_chains() - chains0;
+  }
+  s.counters[CNT_H2D_SKIPPED] = s.counters[CNT_POOL_HWM] = 0;
+  cudaGetLastError();
+  reg_drop_range((void *)mine, gr.piece_bytes);
+  restore_registry(v.segments.back().after, v.pool_base, trace_pool_bytes());
+  memcpy(r.counters, counters, sizeof(counters));
+  r.main_copies = copies;
+  if (!ok || epoch != gr.epoch) {
+    for (cudaGraphExec_t e : s.pieces)
+      if (e) gr.trash.push_back(e);
+    return;
+  }
+  // of the pool's tensors the result alone is there afterwards
+  for (const SavedRec &o : v.segments.back().after) {
+    SavedRec rec = o;
+    if (v.pool_base + o.offset != c.out - p.pool_base + v.pool_base && o.rec.fmt != FMT_PENDING && o.rec.fmt != FMT_ZERO) {
+      rec.rec.fmt = FMT_ELIDED;
+      rec.rec.home = rec.rec.dev_src = nullptr;
+    }
+    s.after.push_back(rec);
+  }
+  n->epoch = gr.epoch;
+  n->used = ++gr.tick;
+  GR_LOG("window cut up: %lld images\n", (long long)c.batch);
+  add_variant(plan, std::move(n));
+  plan.piece_failures = 0;
 }
 
 void launch_segment() {
@@ -281,7 +555,16 @@ void launch_segment() {
   Variant &v = *gr.left[0];
   const Segment &s = v.segments[gr.seg];
   gr.left.resize(1);   // the others may differ from here on
-  if (s.exec) OCC_CUDA(cudaGraphLaunch(s.exec, r.stream));
+  if (v.pieces) {
+    for (int i = 0; i < MAX_PIECES; ++i) {
+      if (i < gr.pieces_coming) OCC_CUDA(cudaStreamWaitEvent(r.stream, gr.piece_here[i], 0));
+      OCC_CUDA(cudaGraphLaunch(s.pieces[i], r.stream));
+    }
+    gr.pieces_coming = 0;
+  } else {
+    wait_for_upload();
+    if (s.exec) OCC_CUDA(cudaGraphLaunch(s.exec, r.stream));
+  }
   for (int i = 0; i < 8; ++i) r.counters[i] += s.counters[i];
   r.main_copies += s.copies;
   for (int64_t i = 0; i < s.chains; ++i) trace_count_chain();
@@ -291,6 +574,7 @@ void launch_segment() {
     v.used = ++gr.tick;
     gr.state = PLAIN;
     gr.left.clear();
+    if (!v.pieces) build_pieces(*gr.prog, v);
   }
 }
 
@@ -298,11 +582,18 @@ void start_window() {
   gr.prog = trace_candidate();
   GraphPlan &plan = *gr.prog->graph;
   const uintptr_t base = trace_pool_base();
-  gr.left.clear();
-  for (auto &v : plan.variants)
-    if (v->pool_base == base && v->flags == mode_flags() && v->epoch == gr.epoch &&
-        same_registry(v->before, base, trace_pool_bytes()))
-      gr.left.push_back(v.get());
+  auto select = [&](bool pieces) {
+    gr.left.clear();
+    for (auto &v : plan.variants)
+      if (v->pool_base == base && v->flags == mode_flags() && v->epoch == gr.epoch && v->pieces == pieces &&
+          same_registry(v->before, base, trace_pool_bytes()))
+        gr.left.push_back(v.get());
+  };
+  select(gr.pieces_coming > 0);
+  if (gr.pieces_coming && gr.left.empty()) {
+    wait_for_upload();
+    select(false);
+  }
   gr.next = plan.begin;
   gr.seg = gr.constant = 0;
   if (!gr.left.empty()) {
@@ -327,8 +618,51 @@ void start_window() {
 
 GraphPlan::~GraphPlan() {
   for (auto &v : variants)
-    for (Segment &s : v->segments)
+    for (Segment &s : v->segments) {
       if (s.exec) gr.trash.push_back(s.exec);
+      for (cudaGraphExec_t e : s.pieces)
+        if (e) gr.trash.push_back(e);
+    }
+}
+
+bool graph_upload_in_pieces(void *dst, const void *src, size_t bytes, cudaStream_t copy_stream) {
+  if (gr.state != IDLE || !allowed()) return false;
+  TraceProgram *p = trace_candidate();
+  if (!p || !p->graph || trace_index() != p->graph->begin) return false;
+  const uintptr_t base = trace_pool_base();
+  bool there = false;
+  for (auto &v : p->graph->variants)
+    there = there || (v->pieces && v->pool_base == base && v->flags == mode_flags() && v->epoch == gr.epoch);
+  Cut c;
+  int64_t images[MAX_PIECES];
+  if (!there || !find_input(*p, c) || (size_t)c.x_bytes != bytes || c.x - p->pool_base + base != (uintptr_t)dst ||
+      !piece_images(c.batch, images))
+    return false;
+  // behind what is enqueued already: it may still read or write the memory
+  for (cudaEvent_t &e : gr.piece_here)
+    if (!e) OCC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  OCC_CUDA(cudaEventRecord(gr.piece_here[0], rt().stream));
+  OCC_CUDA(cudaStreamWaitEvent(copy_stream, gr.piece_here[0], 0));
+  size_t at = 0;
+  for (int k = 0; k < MAX_PIECES; ++k) {
+    const size_t n = bytes / (size_t)c.batch * (size_t)images[k];
+    OCC_CUDA(cudaMemcpyAsync((char *)dst + at, (const char *)src + at, n, cudaMemcpyHostToDevice, copy_stream));
+    OCC_CUDA(cudaEventRecord(gr.piece_here[k], copy_stream));
+    at += n;
+  }
+  gr.pieces_coming = MAX_PIECES;
+  return true;
+}
+
+void graph_uncovered() { wait_for_upload(); }
+
+void graph_free_memory() {
+  if (!gr.piece_memory) return;
+  graph_forget_all();
+  OCC_CUDA(cudaStreamSynchronize(rt().stream));
+  OCC_CUDA(cudaFree(gr.piece_memory));
+  gr.piece_memory = nullptr;
+  gr.piece_bytes = 0;
 }
 
 bool graph_covers(const Entry &e) {
@@ -417,6 +751,7 @@ void graph_forget_all() {
 
 void graph_inference_begin() {
   graph_settle();
+  wait_for_upload();
   empty_trash(gr.trash.size() > 64);
   gr.state = IDLE;
   gr.prog = nullptr;

@@ -12,6 +12,8 @@
 // inference back: the calls that no launched graph covers are made again one by one, then the
 // differing one as it stands.
 #pragma once
+#include <functional>
+
 #include "runtime.h"
 #include "trace.h"
 
@@ -29,14 +31,22 @@ void graph_settle();
 void graph_stop_capture();
 // The same for an upload, which the trace notes as well: a window does not reach across it.
 void graph_before_upload();
+// An upload of `bytes` to `dst`, recorded just now, is about to start.  When the inference's window exists
+// cut up by images, the upload is made in as many pieces on `copy_stream`, and true is returned: the window
+// takes the pieces as they arrive, and any other call waits for the last.
+bool graph_upload_in_pieces(void *dst, const void *src, size_t bytes, cudaStream_t copy_stream);
 // Device memory that graphs may refer to is about to be freed or its contents replaced.
 void graph_forget_all();
+// A call is about to be carried out that no graph covers.
+void graph_uncovered();
+// Frees what windows cut up by images work in.
+void graph_free_memory();
 // cudnnCreate / cudnnDestroy.
 void graph_inference_begin();
 void graph_inference_end();
 
 // abi.cu: makes a recorded call again.
-void run_again(const Entry &e, intptr_t pool_shift, uintptr_t pool_base, size_t pool_bytes, const void *host);
+void run_again(const Entry &e, const std::function<void *(void *)> &place, const void *host);
 // abi.cu: enqueues a held-back convolution; whether there is one.
 void flush_held_back();
 bool anything_held_back();

@@ -26,6 +26,7 @@ struct TraceState {
   uintptr_t last_pool_base = 0;   // the pool of this inference, also after it was given back
   size_t last_pool_bytes = 0;
   uint8_t last_flags = 0;
+  int forced = -1;               // role of the next call, see trace_force()
   int elided = 0;
   int64_t fused_chains = 0;
 };
@@ -365,10 +366,21 @@ void te_dims(Entry &e, const int64_t *d, int n) {
   for (int i = 0; i < n; ++i) mix(e.sig, (uint64_t)d[i]);
 }
 
+void trace_roles(const std::vector<Entry> &calls, std::vector<uint8_t> &roles) {
+  std::vector<int> reader;
+  analyse(calls, roles, reader);
+}
+void trace_force(uint8_t role) { g_ts.forced = role; }
+void trace_force_end() { g_ts.forced = -1; }
+
 Role trace_step(Entry &e, bool *deviated) {
   *deviated = false;
   TraceState &ts = g_ts;
   ts.last_flags = 0;
+  if (ts.forced >= 0) {
+    ts.last_flags = (uint8_t)(ts.forced & ~ROLE_BITS);
+    return (Role)(ts.forced & ROLE_BITS);
+  }
   if (!trace_enabled() || !ts.in_inference) return R_EAGER;
   if (trace_index() >= MAX_ENTRIES) {  // not a compiled model's call pattern: stop tracing
     ts.in_inference = false;

@@ -120,6 +120,11 @@ const std::vector<Entry> &trace_entries();
 void trace_adopt_prefix(TraceProgram *p, size_t n);
 // The same, as if they had been made one by one: what follows is recorded and matched anew.
 void trace_rewind(TraceProgram *p, size_t n);
+// The roles `analyse` gives the calls of an inference; and the role of the next call, whatever was recorded
+// (calls made outside an inference's own sequence).
+void trace_roles(const std::vector<Entry> &calls, std::vector<uint8_t> &roles);
+void trace_force(uint8_t role);
+void trace_force_end();
 uintptr_t trace_pool_base();
 size_t trace_pool_bytes();
 void trace_set_pool(void *base, size_t bytes);
