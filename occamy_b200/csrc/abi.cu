@@ -1404,6 +1404,9 @@ static float *pool_common(int sym, float *x, int64_t *dI, float *y, int64_t *dO,
   if (!avg && kernel[0] == 3 && kernel[1] == 3 && stride[0] == 2 && stride[1] == 2 && ph == 1 &&
       pw == 1 && padding[1] == 1 && padding[3] == 1)
     e.kind = CK_POOL_3S2;
+  if (!avg && kernel[0] == 2 && kernel[1] == 2 && stride[0] == 2 && stride[1] == 2 && !padding[0] && !padding[1] &&
+      !padding[2] && !padding[3] && P == H / 2 && Q == W / 2)
+    e.kind = CK_POOL_2S2;
   const Role role = step(e, false);
   if (role == R_SKIP) return y;
   const bool for_matmul = (trace_last_flags() & RF_FOR_MATMUL) != 0;
@@ -1438,6 +1441,24 @@ static float *pool_common(int sym, float *x, int64_t *dI, float *y, int64_t *dO,
       }
     }
     if (done) return y;
+    if (e.kind == CK_POOL_2S2 && !for_matmul && !j.depthwise && !j.product && !j.linked && !j.joined && !j.res_set && !j.a.split &&
+        j.a.Cf == g.C && x == j.out && N == g.N && C == g.K && H == g.P && W == g.Q) {
+      TcConvArgs a = j.a;
+      a.act = g.act; a.lo = g.lo; a.hi = g.hi;
+      a.y = (bf16 *)16;
+      a.bias = nullptr;
+      a.consts_ready = 0;
+      if (tc_conv_takes_pool(a)) {
+        elide(j.out);
+        j.out = y;
+        j.g.P = P;
+        j.g.Q = Q;
+        j.a.pool2 = 1;
+        j.absorbed++;
+        flush_pending();
+        return y;
+      }
+    }
     flush_pending();
   }
   if (r.mode != MATH_FP32 && C % 8 == 0 && is_act16(x, N, C, H, W)) {
@@ -1684,6 +1705,23 @@ void occamy_internal_opaque_call(void) {
 }
 
 }  // extern "C"
+
+// Whether the convolution of entry `e` takes a 2x2 max pool behind it along.
+bool occ::entry_takes_pool(const Entry &e) {
+  const int64_t *v = e.args.v;   // dX[4], dW[4], pads[2], strides[2], groups
+  if (!e.fusable || e.parts || e.depthwise || v[1] % 16 || v[12] != 1) return false;
+  TcConvArgs a;
+  memset(&a, 0, sizeof(a));
+  a.N = (int)v[0]; a.H = (int)v[2]; a.W = (int)v[3]; a.Cf = (int)v[1];
+  a.K = (int)v[4]; a.R = (int)v[6]; a.S = (int)v[7];
+  a.P = (int)e.dims[2]; a.Q = (int)e.dims[3];
+  a.pad_h = (int)v[8]; a.pad_w = (int)v[9]; a.stride_h = (int)v[10]; a.stride_w = (int)v[11];
+  a.act = ACT_RELU;
+  a.f16 = mode_f16() ? 1 : 0;
+  a.x = a.w = (const bf16 *)16;
+  a.y = (bf16 *)16;
+  return tc_conv_takes_pool(a);
+}
 
 // ---------------------------------------------------------------- made again
 void occ::flush_held_back() { flush_pending(); }

@@ -626,6 +626,23 @@ static SkChoice sk_choose(const TcConvArgs &a, long sp_tiles, int rows, int kste
   return best;
 }
 
+// Pixel box of a layer whose 2x2 max pool is taken along: columns a power of two up to 16, rows even.
+static void pool_box(int Q, int P, int N, int *tw, int *th, int *tn) {
+  long best = -1;
+  for (int w = 16; w >= 2; w /= 2)
+    for (int h = 2; h <= P + 1 && w * h <= 128; h += 2) {
+      int n = 128 / (w * h);
+      if (n > N) n = N;
+      const long tiles = (long)((Q + w - 1) / w) * ((P + h - 1) / h) * ((N + n - 1) / n);
+      if (best < 0 || tiles < best) {
+        best = tiles;
+        *tw = w;
+        *th = h;
+        *tn = n;
+      }
+    }
+}
+
 static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, double rival, Plan *pl) {
 #ifdef OCCAMY_TUNING
   const char *force = getenv("OCCAMY_SK");
@@ -768,7 +785,16 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   const bool pn = !halo && pn_allowed && !a.f16 && !a.out_f32 && a.K <= 128 && a.R * a.S > 1 &&
                   a.R * a.S * a.Cf >= 9 * 64;
   pl.pn = pn;
-  if (halo) {
+  if (halo && a.pool2) {
+    p.tw = 14;   // 16 lanes to an input row
+    p.th = 8;
+    p.tn = 1;
+    p.halo = 1;
+    p.halo_wp = 16;
+    p.halo_a_bytes = 10 * 16 * 128;
+  } else if (a.pool2) {
+    pool_box(Qg, Pg, Ng, &p.tw, &p.th, &p.tn);
+  } else if (halo) {
     // Column strips `tw` wide: the fewest tiles, then the smallest input block (its rows carry a column on
     // either side, and there is a row above and below).
     long best_tiles = -1, best_block = 0;
@@ -832,7 +858,8 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
     const double waves = (double)((p.total_tiles + per_wave - 1) / per_wave);
     const int ks = p.cblocks * a.R * a.S;
     const double tile_us = halo ? 0.9 : pn ? 0.49 * ks : (bn == 256 ? 0.1 : 0.0) + 0.27 * ks * (bk == 64 ? 1.0 : 0.75);
-    if (sk_plan(a, err_word, nsm, counted, 3.1 + waves * tile_us, &pl)) return pl;
+    if (!a.pool2 && sk_plan(a, err_word, nsm, counted, 3.1 + waves * tile_us, &pl)) return pl;
+    if (a.pool2 && !halo && !pair) return pl;   // (not ok: tc_conv_takes_pool() said so)
   }
   const uint32_t boxA[4] = {(uint32_t)bk, (uint32_t)p.tw, (uint32_t)p.th, (uint32_t)p.tn};
   bool ok = true;
@@ -866,10 +893,13 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
                          (halo ? TC_MODE_HALO : 0));
   if (a.f16) pl.mode |= TC_MODE_F16;
   if (pair) pl.mode |= TC_MODE_PAIR;
+  if (a.pool2) pl.mode |= TC_MODE_POOL;
   if (!a.out_f32) {
-    const uint64_t dims[4] = {(uint64_t)a.K, (uint64_t)Qg, (uint64_t)Pg, (uint64_t)Ng};
-    const uint64_t st[3] = {(uint64_t)a.K * 2, (uint64_t)Qg * a.K * 2, (uint64_t)Pg * Qg * a.K * 2};
-    const uint32_t box[4] = {(uint32_t)dc, (uint32_t)p.tw, (uint32_t)p.th, (uint32_t)p.tn};
+    const int half = a.pool2 ? 2 : 1;
+    const uint64_t Qo = (uint64_t)(Qg / half), Po = (uint64_t)(Pg / half);
+    const uint64_t dims[4] = {(uint64_t)a.K, Qo, Po, (uint64_t)Ng};
+    const uint64_t st[3] = {(uint64_t)a.K * 2, Qo * a.K * 2, Po * Qo * a.K * 2};
+    const uint32_t box[4] = {(uint32_t)dc, (uint32_t)(p.tw / half), (uint32_t)(p.th / half), (uint32_t)p.tn};
     ok &= make_map(&p.tmD, a.y, 4, dims, st, box, dc * 2, counted);
     if (a.residual) ok &= make_map(&p.tmR, a.residual, 4, dims, st, box, dc * 2, counted);
   }
@@ -972,6 +1002,20 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   if (halo && !ok) return build_plan(a, err_word, num_sms, counted, false);   // e.g. the block map was refused
   pl.ok = ok;
   return pl;
+}
+
+// Whether a 2x2 / stride 2 max pool behind this convolution is better taken along.
+bool tc_conv_takes_pool(TcConvArgs a) {
+  if (a.P < 2 || a.Q < 2 || a.split || a.out_f32 || a.residual || a.w_step || a.K % 8 || !tc_conv_supported(a)) return false;
+  const bool halo = !a.f16 && a.R == 3 && a.S == 3 && a.stride_h == 1 && a.stride_w == 1 && a.pad_h == 1 &&
+                    a.pad_w == 1 && a.Cf == 64 && a.K == 64;
+  const bool flat = a.R == 1 && a.S == 1;
+  if (flat || (!halo && (a.K % 256 || a.R * a.S * a.Cf < 16 * 64))) return false;
+  const Plan alone = build_plan(a, nullptr, rt().num_sms, false);
+  if (!alone.ok || alone.sk || !(alone.p.halo || alone.pair)) return false;
+  a.pool2 = 1;
+  const Plan pooled = build_plan(a, nullptr, rt().num_sms, false);
+  return pooled.ok && (pooled.p.halo || pooled.pair) && pooled.p.total_tiles <= alone.p.total_tiles * 1.15 + 1;
 }
 
 static void launch_plan_pn(const Plan &pl, int num_sms, cudaStream_t s) {

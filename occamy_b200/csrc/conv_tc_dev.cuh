@@ -116,6 +116,11 @@ constexpr int TC_MODE_F16 = 16;
 // flop of the single-CTA form, which is what bounds the long-reduction layers.  No multicast
 // load is involved: every TMA load has one destination.
 constexpr int TC_MODE_PAIR = 32;
+// A 2x2 / stride 2 max pool behind the layer: the tile's rows are columns x rows of the image with a
+// power-of-two pitch of at most 16, so that the four pixels of a window are lanes of one warp; their
+// 16-bit results meet by shuffles and a quarter of the slab is stored.  (A pass of its own over the
+// 224x224 layer of a VGG-16 took 85 us at batch 64, and its input 60 to write.)
+constexpr int TC_MODE_POOL = 64;
 
 // ------------------------------------------------------------------ PTX wrappers
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -347,6 +352,13 @@ __device__ __forceinline__ uint64_t pair16_to_f2(uint32_t w) {
     return f2_pack(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
   }
 }
+template <bool F16>
+__device__ __forceinline__ uint32_t tc_max2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  if constexpr (F16) asm("max.NaN.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  else asm("max.NaN.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
 __device__ __forceinline__ void tc_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
@@ -506,6 +518,8 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
   constexpr bool HALO = (MODE & TC_MODE_HALO) != 0;
   constexpr bool F16 = (MODE & TC_MODE_F16) != 0;
   constexpr bool PAIR = (MODE & TC_MODE_PAIR) != 0;
+  constexpr bool POOL = (MODE & TC_MODE_POOL) != 0;
+  static_assert(!POOL || (!(MODE & (TC_MODE_RES | TC_MODE_F32)) && (HALO || PAIR)), "pooled forms");
   static_assert(!(PAIR && (HALO || F32)), "the CTA-pair form exists for the plain epilogues only");
   constexpr int EPI_THREADS = 128 * EW;
   constexpr int STORE_WARP = 2 + 4 * EW;
@@ -930,7 +944,8 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
               break;
             }
             if (!ghost)   // the duplicate tile of an odd last pair is computed, not stored
-              tma_store_4d(&p.tmD, sD + b * SLAB_BYTES, tl.k0 + sl * DC, tl.q0, tl.p0, tl.n0);
+              tma_store_4d(&p.tmD, sD + b * SLAB_BYTES, tl.k0 + sl * DC, POOL ? tl.q0 >> 1 : tl.q0,
+                           POOL ? tl.p0 >> 1 : tl.p0, tl.n0);
             tma_store_commit();
             // Up to store_pend of my earlier stores may still be reading their buffers; the
             // one before those is done, and its buffer goes to the slab dbuf further on.
@@ -1003,6 +1018,12 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
       const int h = row / p.halo_wp, w = row - h * p.halo_wp;
       keep = w < p.tw && h < p.th;
       srow = keep ? h * p.tw + w : 0;
+    }
+    const int pool_down = HALO ? p.halo_wp : p.tw;   // lanes from a pixel to the one below
+    if constexpr (POOL) {
+      const int r2 = row / pool_down, w = row - r2 * pool_down, n = r2 / p.th, h = r2 - n * p.th;
+      keep = w < p.tw && n < p.tn && !(w & 1) && !(h & 1);
+      srow = keep ? (n * (p.th / 2) + h / 2) * (p.tw / 2) + w / 2 : 0;
     }
     // swizzled offsets of this thread's 16-byte pieces inside a slab buffer
     uint32_t soff[CW / 8];
@@ -1119,6 +1140,13 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
               pk[j] = f2_to_bf16x2<F16>(f2_pack(tc_act(a, act_lo, act_hi), tc_act(b, act_lo, act_hi)));
             } else {
               pk[j] = f2_to_bf16x2_relu<F16>(v2[j]);   // ReLU rides on the conversion
+            }
+          }
+          if constexpr (POOL) {
+#pragma unroll
+            for (int j = 0; j < CW / 2; ++j) {
+              pk[j] = tc_max2<F16>(pk[j], __shfl_xor_sync(0xffffffffu, pk[j], 1));
+              pk[j] = tc_max2<F16>(pk[j], __shfl_xor_sync(0xffffffffu, pk[j], pool_down));
             }
           }
 #pragma unroll
@@ -1294,6 +1322,14 @@ inline bool tc_launch_mode(const TcParams &p, int mode, int grid, size_t smem, c
       case P2 | H2 | TC_MODE_RES | TC_MODE_CLAMP:
         tc_launch_one<BN, DC, P2 | H2 | TC_MODE_RES | TC_MODE_CLAMP>(p, grid, smem, s);
         return true;
+      case P2 | TC_MODE_POOL: tc_launch_one<BN, DC, P2 | TC_MODE_POOL>(p, grid, smem, s); return true;
+      case P2 | TC_MODE_POOL | TC_MODE_CLAMP:
+        tc_launch_one<BN, DC, P2 | TC_MODE_POOL | TC_MODE_CLAMP>(p, grid, smem, s);
+        return true;
+      case P2 | H2 | TC_MODE_POOL: tc_launch_one<BN, DC, P2 | H2 | TC_MODE_POOL>(p, grid, smem, s); return true;
+      case P2 | H2 | TC_MODE_POOL | TC_MODE_CLAMP:
+        tc_launch_one<BN, DC, P2 | H2 | TC_MODE_POOL | TC_MODE_CLAMP>(p, grid, smem, s);
+        return true;
       default: break;
     }
   }
@@ -1331,6 +1367,10 @@ inline bool tc_launch_mode(const TcParams &p, int mode, int grid, size_t smem, c
   if constexpr (WITH_HALO) {
     switch (mode) {
       case TC_MODE_HALO: tc_launch_one<BN, DC, TC_MODE_HALO>(p, grid, smem, s); return true;
+      case TC_MODE_HALO | TC_MODE_POOL: tc_launch_one<BN, DC, TC_MODE_HALO | TC_MODE_POOL>(p, grid, smem, s); return true;
+      case TC_MODE_HALO | TC_MODE_POOL | TC_MODE_CLAMP:
+        tc_launch_one<BN, DC, TC_MODE_HALO | TC_MODE_POOL | TC_MODE_CLAMP>(p, grid, smem, s);
+        return true;
       case TC_MODE_HALO | TC_MODE_RES:
         tc_launch_one<BN, DC, TC_MODE_HALO | TC_MODE_RES>(p, grid, smem, s);
         return true;

@@ -147,6 +147,7 @@ struct TcConvArgs {
   // Filter (and bias) were resident on the device before this call was made, i.e. no work
   // enqueued earlier in the stream produces them.
   int consts_ready;
+  int pool2;             // y is the 2x2 / stride 2 max pool of the result (tc_conv_takes_pool())
 };
 // ---- few-channel convolution fused with the 3x3 / stride 2 / pad 1 max pool after it -----
 struct StemPoolArgs {
@@ -193,6 +194,7 @@ void launch_selftest_bounded_wait(cudaStream_t s);
 
 // Returns false when the shape is outside what the kernel supports (caller falls back).
 bool tc_conv_supported(const TcConvArgs &a);
+bool tc_conv_takes_pool(TcConvArgs a);
 void launch_tc_conv(const TcConvArgs &a, cudaStream_t s);
 // Same kernel, no runtime state, no caches, no allocation; false when the plan fails.
 bool launch_tc_conv_stateless(const TcConvArgs &a, int *err_word, int num_sms, cudaStream_t s);

@@ -226,9 +226,9 @@ void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles, std::ve
       members.push_back(j);
       cur = f.out;
     }
-    // a stem convolution takes the max pool behind it along, when the pool is the only
-    // reader of the full-resolution tensor
-    if (c.poolable && !res_set) {
+    // a stem convolution takes the max pool behind it along, some others a 2x2 one, when the pool is the
+    // only reader of the full-resolution tensor
+    if (!res_set && !c.depthwise && !c.parts) {
       const size_t from = members.empty() ? i + 1 : members.back() + 1;
       for (size_t j = from; j < rec.size(); ++j) {
         const Entry &f = rec[j];
@@ -238,8 +238,8 @@ void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles, std::ve
           if (f.sym == S_DEALLOC && f.out == cur) break;
           continue;
         }
-        if (f.sym == S_MAXPOOL && f.kind == CK_POOL_3S2 && f.in[0] == cur && f.out != cur &&
-            dies_unread(rec, cur, cur_bytes, j + 1))
+        if (f.sym == S_MAXPOOL && f.in[0] == cur && f.out != cur && dies_unread(rec, cur, cur_bytes, j + 1) &&
+            ((c.poolable && f.kind == CK_POOL_3S2) || (f.kind == CK_POOL_2S2 && entry_takes_pool(c))))
           members.push_back(j);
         break;
       }

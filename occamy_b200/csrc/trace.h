@@ -34,7 +34,8 @@ enum Role { R_EAGER = 0, R_DEFER = 1, R_ABSORB = 2, R_SKIP = 3 };
 enum ChainKind {
   CK_NONE = 0, CK_BIAS_ADD = 1, CK_SAME_ADD = 2, CK_RELU = 3, CK_CLIP = 4,
   CK_POOL_3S2 = 5,  // max pool 3x3, stride 2, pad 1
-  CK_ROW_BIAS = 6   // rank 2: the same row added to every row
+  CK_ROW_BIAS = 6,  // rank 2: the same row added to every row
+  CK_POOL_2S2 = 7   // max pool 2x2, stride 2, no padding
 };
 
 // The call's own arguments, enough to make it again (graph_replay.cu, run_again).
@@ -122,6 +123,8 @@ void trace_adopt_prefix(TraceProgram *p, size_t n);
 void trace_rewind(TraceProgram *p, size_t n);
 // The roles `analyse` gives the calls of an inference; and the role of the next call, whatever was recorded
 // (calls made outside an inference's own sequence).
+// (abi.cu) whether the convolution's kernel can take a following CK_POOL_2S2 along
+bool entry_takes_pool(const Entry &e);
 void trace_roles(const std::vector<Entry> &calls, std::vector<uint8_t> &roles);
 void trace_force(uint8_t role);
 void trace_force_end();
