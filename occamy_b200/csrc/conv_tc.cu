@@ -882,6 +882,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   // for a fourth ring stage, which those layers need more than a cheap epilogue.
   const int ksteps64 = (a.R * a.S * a.Cf + 63) / 64;
   int dc = pn ? 64 : (bn < 64 ? bn : (bn == 256 && bk == 64 && ksteps64 >= 16 ? 32 : 64));
+  if (bn == 64 && a.w_step && a.R <= 3 && !pn && !halo && !a.out_f32 && nsm >= 2) dc = 32;   // few-channel stems: two CTAs per SM, below
   if (a.out_f32 && bn >= 64) dc = 64;   // the fp32-output flavour is compiled for 64-channel slabs
 #ifdef OCCAMY_TUNING
   if (const char *f = getenv("OCCAMY_TC_DC"))   // slab width of the 256-wide tiles
@@ -912,7 +913,8 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   const size_t b_tile_bytes = (size_t)(pair ? bn / 2 : bn) * bk * 2;
   // (With two CTAs per SM the single loading thread of a CTA is what the others wait for, and
   // weights of up to 16 KB pay as well: 144->24 at 56x56 has nine k-steps of 1 KB each.)
-  const bool duo_wanted = !pn && !halo && !pair && !a.out_f32 && dc == 32 && bn == 32 && nsm >= 2;
+  const bool duo_wanted = !pn && !halo && !pair && !a.out_f32 && nsm >= 2 &&
+                          dc == 32 && bn <= 64;
   bool bres = !pn && !halo && !pair && p.tiles_k == 1 &&
               ksteps_tile * b_tile_bytes <= (size_t)(duo_wanted ? 16 : 4) * 1024;
 #ifdef OCCAMY_TUNING
@@ -933,12 +935,14 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   // traffic, but each of the single-threaded roles (loads, MMA issue, slab stores) spends about
   // a thousand cycles of dependent instructions and barrier round trips on it; two resident
   // CTAs overlap those (measured 1.2x to 1.6x on the layers with up to 32 output channels; no
-  // gain for 64-channel tiles).  They share the SM's shared memory, registers (one epilogue warp per TMEM
+  // gain for 64-channel tiles, but for the few-channel stems with three filter rows: 3->64 3x3 at 224x224
+  // 181 -> 148 us at batch 64, 23.9 -> 15.8 at 5, stride 2 batch 64 61 -> 34; 5x5 42 -> 45, 7x7 100 -> 94).
+  // They share the SM's shared memory, registers (one epilogue warp per TMEM
   // quadrant, 256 threads) and TMEM (at most 256 columns each).
   bool duo = duo_wanted;
 #ifdef OCCAMY_TUNING
   if (const char *f = getenv("OCCAMY_TC_DUO"))
-    duo = atoi(f) != 0 && !pn && !halo && !pair && !a.out_f32 && dc == 32 && bn == 32;
+    duo = atoi(f) != 0 && !pn && !halo && !pair && !a.out_f32 && duo_wanted;
 #endif
   int dbuf = 0, pend = 0, stages = 0;
   for (;; duo = false) {
@@ -1044,9 +1048,8 @@ static void launch_any(const Plan &pl, int num_sms, cudaStream_t s) {
   bool ok;
   if (pl.duo) {
     grid = pl.p.total_tiles < 2 * num_sms ? pl.p.total_tiles : 2 * num_sms;
-    ok = pl.bn == 32   ? tc_launch_32_32_duo(pl.p, pl.mode, grid, pl.smem, s)
-         : pl.bn == 64 ? tc_launch_64_64_duo(pl.p, pl.mode, grid, pl.smem, s)
-                       : tc_launch_128_64_duo(pl.p, pl.mode, grid, pl.smem, s);
+    ok = pl.bn == 32 ? tc_launch_32_32_duo(pl.p, pl.mode, grid, pl.smem, s)
+                     : tc_launch_64_32_duo(pl.p, pl.mode, grid, pl.smem, s);
     if (!ok) set_error(997, "tensor-core conv: no two-per-SM kernel for this epilogue");
     return;
   }

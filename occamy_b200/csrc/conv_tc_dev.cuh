@@ -415,6 +415,7 @@ __device__ __forceinline__ void tc_ld8(uint32_t taddr, uint32_t *r) {
 }
 template <int W>
 __device__ __forceinline__ void tc_ld(uint32_t taddr, uint32_t *r) {
+  static_assert(W == 32 || W == 16 || W == 8, "columns of one load");
   if constexpr (W == 32) tc_ld32(taddr, r);
   else if constexpr (W == 16) tc_ld16(taddr, r);
   else tc_ld8(taddr, r);
@@ -1224,8 +1225,7 @@ bool tc_launch_128_64(const TcParams &p, int mode, int grid, size_t smem, cudaSt
 bool tc_launch_64_64(const TcParams &p, int mode, int grid, size_t smem, cudaStream_t s);
 bool tc_launch_32_32(const TcParams &p, int mode, int grid, size_t smem, cudaStream_t s);
 bool tc_launch_32_32_duo(const TcParams &p, int mode, int grid, size_t smem, cudaStream_t s);
-bool tc_launch_64_64_duo(const TcParams &p, int mode, int grid, size_t smem, cudaStream_t s);
-bool tc_launch_128_64_duo(const TcParams &p, int mode, int grid, size_t smem, cudaStream_t s);
+bool tc_launch_64_32_duo(const TcParams &p, int mode, int grid, size_t smem, cudaStream_t s);
 
 // Launch with programmatic stream serialisation (see pdl_wait); `cluster` > 1 launches the
 // grid as thread-block clusters of that many CTAs.
