@@ -243,21 +243,17 @@ void stem_geometry(const ConvGeom &g, int &Cp, int &Sp, int &Wp) {
   Wp = (Wp + 7) / 8 * 8;
 }
 
-// `job.linked` (the first convolution of an inverted residual): x is taken as it is, without the padding of
-// its channels; `job.joined`: x is not there yet.
-bool prepare_dense(const float *x, const float *w, const float *bias, const ConvGeom &g,
-                   ConvJob &job) {
-  Runtime &r = rt();
+// A dense convolution of the 16-bit path as the kernels are told of it, but for where its operands are;
+// false when they do not take it.  Cp, Sp, Wp: how the input is stored (stem_geometry(), when it is folded).
+bool dense_args(const ConvGeom &g, TcConvArgs &a, int &Cp, int &Sp, int &Wp) {
+  memset(&a, 0, sizeof(a));
   if (g.groups != 1 || g.K % 8 != 0) return false;
   if (g.act != ACT_IDENTITY && g.act != ACT_RELU && g.act != ACT_CLIP) return false;
-  TcConvArgs &a = job.a;
-  memset(&a, 0, sizeof(a));
   a.N = g.N; a.K = g.K; a.P = g.P; a.Q = g.Q;
   a.act = g.act; a.lo = g.lo; a.hi = g.hi;
   a.f16 = mode_f16() ? 1 : 0;
-  const bool folded = g.C < 16;
-  int Sp = 0, Cp = 0, Wp = 0;
-  if (folded) {
+  Sp = Cp = Wp = 0;
+  if (g.C < 16) {
     stem_geometry(g, Cp, Sp, Wp);
     a.H = g.H; a.W = g.Q; a.Cf = Sp * Cp;
     a.R = g.R; a.S = 1;
@@ -277,7 +273,18 @@ bool prepare_dense(const float *x, const float *w, const float *bias, const Conv
   a.x = (const bf16 *)16;  // placeholders so the support check sees aligned pointers
   a.w = (const bf16 *)16;
   a.y = (bf16 *)16;
-  if (!tc_conv_supported(a)) return false;
+  return tc_conv_supported(a);
+}
+
+// `job.linked` (the first convolution of an inverted residual): x is taken as it is, without the padding of
+// its channels; `job.joined`: x is not there yet.
+bool prepare_dense(const float *x, const float *w, const float *bias, const ConvGeom &g,
+                   ConvJob &job) {
+  Runtime &r = rt();
+  TcConvArgs &a = job.a;
+  int Sp, Cp, Wp;
+  if (!dense_args(g, a, Cp, Sp, Wp)) return false;
+  const bool folded = g.C < 16;
 
   job.dep_lo[0] = job.dep_hi[0] = 0;
   if (folded) {
@@ -713,11 +720,9 @@ void elide(void *p) {
   trace_note_elided();
 }
 
-float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t *dW, float *bias,
-                   int64_t groups, const int64_t *pads, const int64_t *strides, int act, float lo,
-                   float hi, int64_t act_mode, float *y) {
-  Runtime &r = rt();
-  ConvGeom g;
+// Geometry of a convolution call; false when its shapes do not fit together.
+bool conv_geometry(const int64_t *dX, const int64_t *dW, int64_t groups, const int64_t *pads, const int64_t *strides,
+                   int act, float lo, float hi, ConvGeom &g) {
   g.N = (int)dX[0]; g.C = (int)dX[1]; g.H = (int)dX[2]; g.W = (int)dX[3];
   g.K = (int)dW[0]; g.R = (int)dW[2]; g.S = (int)dW[3];
   g.groups = (int)(groups < 1 ? 1 : groups);
@@ -728,6 +733,23 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
                           dW[1] * g.groups != g.C);
   g.P = shape_ok ? (g.H + 2 * g.pad_h - g.R) / g.stride_h + 1 : 0;
   g.Q = shape_ok ? (g.W + 2 * g.pad_w - g.S) / g.stride_w + 1 : 0;
+  return shape_ok;
+}
+
+// Activation of the fused convolution call's mode; mode 3 is ReLU6.
+int act_of_mode(int64_t mode, float &lo, float &hi) {
+  lo = 0.f;
+  hi = mode == 3 ? 6.f : 0.f;
+  return mode == 1 ? ACT_RELU : mode == 3 ? ACT_CLIP : mode == 0 ? ACT_SIGMOID : mode == 2 ? ACT_TANH : ACT_IDENTITY;
+}
+
+float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t *dW, float *bias,
+                   int64_t groups, const int64_t *pads, const int64_t *strides, int64_t act_mode, float *y) {
+  Runtime &r = rt();
+  ConvGeom g;
+  float lo, hi;
+  const int act = act_of_mode(act_mode, lo, hi);
+  const bool shape_ok = conv_geometry(dX, dW, groups, pads, strides, act, lo, hi, g);
   const bool depthwise = g.groups > 1 && g.groups == g.C && g.K == g.C;
 
   CallScope scope;
@@ -1173,8 +1195,7 @@ int cudnnDestroy(cudnnContext *handle) {
 float *DNNConvFunc(cudnnContext *, float *x, int64_t dimX[4], float *w, int64_t dimW[4],
                    float * /*workspace*/, int64_t /*workspaceSize*/, int64_t /*algo*/,
                    int64_t groups, int64_t pads[2], int64_t strides[2], float *y) {
-  return conv_common(S_CONV, x, dimX, w, dimW, nullptr, groups, pads, strides, ACT_IDENTITY, 0.f,
-                     0.f, 5, y);
+  return conv_common(S_CONV, x, dimX, w, dimW, nullptr, groups, pads, strides, 5, y);
 }
 
 float *DNNConvBiasActivFunc(cudnnContext *, float *x, int64_t dimX[4], float *w, int64_t dimW[4],
@@ -1182,14 +1203,7 @@ float *DNNConvBiasActivFunc(cudnnContext *, float *x, int64_t dimX[4], float *w,
                             int64_t /*workspaceSize*/, int64_t /*algo*/, int64_t pads[2],
                             int64_t strides[2], int64_t activMode, float *y) {
   (void)dimB;
-  int act = ACT_IDENTITY;
-  float lo = 0.f, hi = 0.f;
-  if (activMode == 1) act = ACT_RELU;
-  else if (activMode == 3) { act = ACT_CLIP; lo = 0.f; hi = 6.f; }
-  else if (activMode == 0) act = ACT_SIGMOID;
-  else if (activMode == 2) act = ACT_TANH;
-  return conv_common(S_CONV_BIAS_ACT, x, dimX, w, dimW, bias, 1, pads, strides, act, lo, hi,
-                     activMode, y);
+  return conv_common(S_CONV_BIAS_ACT, x, dimX, w, dimW, bias, 1, pads, strides, activMode, y);
 }
 
 // ---------------------------------------------------------------- element-wise
@@ -1705,6 +1719,20 @@ void occamy_internal_opaque_call(void) {
 }
 
 }  // extern "C"
+
+// Whether the convolution of entry `e` reads its input in the 16-bit path's form, whatever the mode it was
+// recorded in: wider than that, Entry::fusable goes by channel counts alone.
+bool occ::entry_reads_16(const Entry &e) {
+  const int64_t *v = e.args.v;   // dX[4], dW[4], pads[2], strides[2], groups, activation mode
+  ConvGeom g;
+  float lo, hi;
+  const int act = act_of_mode(v[13], lo, hi);
+  if (!conv_geometry(v, v + 4, v[12], v + 8, v + 10, act, lo, hi, g) || g.P <= 0 || g.Q <= 0 || g.N <= 0) return false;
+  if (g.groups > 1) return g.groups == g.C && g.K == g.C && g.C % 8 == 0;   // as prepare_depthwise()
+  TcConvArgs a;
+  int Cp, Sp, Wp;
+  return dense_args(g, a, Cp, Sp, Wp);
+}
 
 // Whether the convolution of entry `e` takes a 2x2 max pool behind it along.
 bool occ::entry_takes_pool(const Entry &e) {

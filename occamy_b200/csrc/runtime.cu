@@ -222,6 +222,7 @@ void ensure_f32(const void *p) {
     r.main_copies++;
     count(CNT_H2D_BYTES, (int64_t)rec->host_bytes);
   } else if (rec->dev_src) {
+    graph_stop_capture();   // the caller's memory, elsewhere in the next inference
     OCC_CUDA(cudaMemcpyAsync((void *)base, rec->dev_src, (size_t)(rec->n * rec->c * rec->h * rec->w) * 4, cudaMemcpyDeviceToDevice, r.stream));
     r.main_copies++;
     rec->home = rec->dev_src = nullptr;

@@ -100,8 +100,8 @@ int only_convs_read(const std::vector<Entry> &rec, uintptr_t p, int64_t bytes, s
     const Entry &e = rec[t];
     for (int k = 0; k < 3; ++k) {
       if (!e.in[k] || !overlaps(e.in[k], e.in_bytes[k] > 0 ? e.in_bytes[k] : 1, p, bytes)) continue;
-      if (k != 0 || (e.sym != S_CONV && e.sym != S_CONV_BIAS_ACT) || e.in[0] != p || !e.fusable ||
-          e.in_bytes[0] != bytes)
+      if (k != 0 || (e.sym != S_CONV && e.sym != S_CONV_BIAS_ACT) || e.in[0] != p || e.in_bytes[0] != bytes ||
+          !entry_reads_16(e))
         return -1;
       const bool few = e.args.v[1] < 16;
       if (first >= 0 && (few || rec[first].args.v[1] < 16)) return -1;

@@ -123,8 +123,10 @@ void trace_adopt_prefix(TraceProgram *p, size_t n);
 void trace_rewind(TraceProgram *p, size_t n);
 // The roles `analyse` gives the calls of an inference; and the role of the next call, whatever was recorded
 // (calls made outside an inference's own sequence).
-// (abi.cu) whether the convolution's kernel can take a following CK_POOL_2S2 along
+// (abi.cu) whether the convolution's kernel can take a following CK_POOL_2S2 along; whether it reads its input
+// as a 16-bit tensor
 bool entry_takes_pool(const Entry &e);
+bool entry_reads_16(const Entry &e);
 void trace_roles(const std::vector<Entry> &calls, std::vector<uint8_t> &roles);
 void trace_force(uint8_t role);
 void trace_force_end();

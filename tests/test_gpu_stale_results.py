@@ -1,0 +1,39 @@
+"""Replayed inferences must compute from this inference's inputs and constants, whichever way those came in:
+hand-made call sequences with a fresh input for every pass, against the CPU oracle."""
+import numpy as np
+import pytest
+import torch
+
+from calls import Inference, rand
+from helpers import max_rel_err
+from occamy_b200 import runtime as rt
+from oracle import ref
+
+pytestmark = pytest.mark.gpu
+
+PASSES = 10   # recorded, fused, quiet, captured once per pool block, then replayed
+
+
+def device(a):
+    t = torch.from_numpy(a).cuda()
+    torch.cuda.synchronize()
+    return t
+
+
+# convolutions that the 16-bit path refuses: by their activation, their stride, their channels
+@pytest.mark.parametrize("c,k,r,stride,act", [(16, 16, 3, 1, 0), (16, 16, 3, 1, 2), (3, 16, 11, 4, 1), (16, 16, 3, 3, 5),
+                                              (20, 16, 3, 1, 1), (3, 12, 3, 1, 1)])
+def test_device_input_of_a_refused_convolution(native_libs, c, k, r, stride, act):
+    rt.set_math_mode(rt.MATH_BF16)
+    w, b = rand(1, k, c, r, r, scale=0.2), rand(2, k)
+    kept = []   # no address comes twice
+    for i in range(PASSES):
+        x = rand(100 + i, 2, c, 23, 21)
+        kept.append(device(x))
+        with Inference() as f:
+            y, o = f.conv(f.copy(kept[-1].data_ptr(), x.nbytes), x.shape, f.put(w), w.shape, f.put(b), (1, 1),
+                          (stride, stride), act=act)
+            got = f.get(y, o)
+        want = ref.conv2d(x, w, b, (1, 1), (stride, stride), act=act)
+        assert max_rel_err(got, want) <= 2e-2, i
+    assert rt.last_error() == 0
