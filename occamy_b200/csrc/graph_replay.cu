@@ -140,12 +140,22 @@ void restore_registry(const std::vector<SavedRec> &in, uintptr_t base, size_t by
   }
 }
 
+// The same tensors in the same form.  Constants uploaded before the window are among them: the graphs refer to
+// what was packed from that very source (of others it does not matter where their contents came from).
+bool same_record(const TensorRec &a, const TensorRec &b) {
+  if (a.bytes != b.bytes || a.fmt != b.fmt || a.home != b.home) return false;
+  if (a.fmt == FMT_PENDING) return a.host_src == b.host_src && a.host_bytes == b.host_bytes && a.host_hash == b.host_hash;
+  if (a.fmt == FMT_F32 || a.fmt == FMT_ZERO || a.fmt == FMT_ELIDED) return true;
+  return a.n == b.n && a.c == b.c && a.h == b.h && a.w == b.w &&
+         (a.fmt != FMT_STEM_ROWS || (a.stem_wp == b.stem_wp && a.stem_cp == b.stem_cp && a.stem_pad == b.stem_pad &&
+                                     a.stem_f16 == b.stem_f16));
+}
+
 bool same_registry(const std::vector<SavedRec> &a, uintptr_t base, size_t bytes) {
   auto &recs = rt().recs;
   auto it = recs.lower_bound(base);
   for (const SavedRec &s : a) {
-    if (it == recs.end() || it->first != base + s.offset || it->second.fmt != s.rec.fmt || it->second.home != s.rec.home)
-      return false;
+    if (it == recs.end() || it->first != base + s.offset || !same_record(it->second, s.rec)) return false;
     ++it;
   }
   return it == recs.end() || it->first >= base + bytes;

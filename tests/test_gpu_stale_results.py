@@ -37,3 +37,21 @@ def test_device_input_of_a_refused_convolution(native_libs, c, k, r, stride, act
         want = ref.conv2d(x, w, b, (1, 1), (stride, stride), act=act)
         assert max_rel_err(got, want) <= 2e-2, i
     assert rt.last_error() == 0
+
+
+def test_constants_in_front_of_the_batch(native_libs):
+    """Two sets of weights at addresses of their own, uploaded before the batch: each inference uses its own."""
+    rt.set_math_mode(rt.MATH_BF16)
+    sets = [[(rand(10 * s + i, 16, 16, 3, 3, scale=0.1), rand(50 + 10 * s + i, 16)) for i in range(3)] for s in (0, 1)]
+    for i in range(4 * PASSES):
+        layers = sets[(i * i // 3) % 2]
+        x = want = rand(i, 2, 16, 12, 12)
+        with Inference() as f:
+            ws = [(f.put(w), f.put(b)) for w, b in layers]
+            y = f.put(x)
+            for (w, b), (pw, pb) in zip(layers, ws):
+                y, o = f.conv(y, x.shape, pw, w.shape, pb, (1, 1), act=1)
+                want = ref.conv2d(want, w, b, (1, 1), act=1)
+            got = f.get(y, o)
+        assert max_rel_err(got, want) <= 2e-2, i
+    assert rt.last_error() == 0
