@@ -152,12 +152,18 @@ void *packed_weights(const float *w, int layout, size_t packed_bytes, int K, int
   return dst;
 }
 
+// Whether the packed form of `p` stays on the device.  One that does not is packed into scratch, where the next
+// one replaces it: its convolution has to be launched before another is prepared.
+bool stays_packed(const float *p) {
+  uintptr_t base;
+  const TensorRec *rec = reg_find(p, &base);
+  return rt().cache_weights && rec && base == (uintptr_t)p && rec->host_src;
+}
+
 // A constant in the form the inverted-residual kernel takes it (the first convolution's bias as parts; the
 // depthwise filter or bias as fp16); null unless it stays on the device.
 const void *packed_for_block(const float *c, int layout, size_t bytes, int E, int R) {
-  uintptr_t base;
-  const TensorRec *rec = reg_find(c, &base);
-  if (!rt().cache_weights || !rec || base != (uintptr_t)c || !rec->host_src) return nullptr;
+  if (!stays_packed(c)) return nullptr;
   return packed_weights(c, layout, bytes, E, 0, R, R, 0, 0);
 }
 
@@ -781,7 +787,7 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
   bool join = false;
   if (g_pending.active) {   // left by step() because this call was recorded as joining it
     const ConvGeom &f = g_pending.g;
-    join = role == R_DEFER && e.fusable && !e.parts && g_fronts < 2 && g_pending.out == x && f.N == g.N && f.K == g.C &&
+    join = role == R_DEFER && e.fusable && !e.parts && stays_packed(w) && g_fronts < 2 && g_pending.out == x && f.N == g.N && f.K == g.C &&
            f.P == g.H && f.Q == g.W && (depthwise ? g_fronts == 0 : g_fronts == 1 && g.C % 16 == 0);
     if (!join) flush_pending();
   }
@@ -799,7 +805,7 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
     ConvJob job;
     const uint8_t flags = trace_last_flags();
     // (the first of three takes its input as it is)
-    job.linked = role == R_DEFER && (flags & RF_LINK) && (join || (!(flags & RF_JOIN) && is_act16(x, g.N, g.C, g.H, g.W)));
+    job.linked = role == R_DEFER && (flags & RF_LINK) && stays_packed(w) && (join || (!(flags & RF_JOIN) && is_act16(x, g.N, g.C, g.H, g.W)));
     job.joined = join;
     bool ok = depthwise ? prepare_depthwise(x, w, bias, g, job)
                         : (g.groups == 1 && prepare_dense(x, w, bias, g, job));

@@ -2,9 +2,11 @@
 and clusters, against the CPU oracle."""
 import pytest
 
+from calls import Inference, rand
 from helpers import max_rel_err, run_graph_oracle
 from occamy_b200 import graphs, replay
 from occamy_b200 import runtime as rt
+from oracle import ref
 
 pytestmark = pytest.mark.gpu
 
@@ -51,4 +53,34 @@ def test_block(binding, shape, fuse, mode):
         launches.append(rt.counters()["launches"] - before)
         assert max_rel_err(got, want) <= 2e-2
     assert launches[2] < launches[0]
+    assert rt.last_error() == 0
+
+
+@pytest.mark.parametrize("mode", [rt.MATH_BF16, rt.MATH_F16])
+@pytest.mark.parametrize("filters", ["no cache", "from the device", "from the host"])
+def test_block_with_filters_that_do_not_stay(native_libs, filters, mode):
+    """Filters without a resident packed copy: each of the three convolutions still gets its own."""
+    rt.set_math_mode(mode)
+    shape, E, K = (1, 16, 14, 14), 96, 24
+    ws = [rand(1, 16, 16, 1, 1, scale=0.3), rand(2, E, 16, 1, 1, scale=0.3), rand(3, E, 1, 3, 3, scale=0.3),
+          rand(4, K, E, 1, 1, scale=0.1)]
+    dev = [rt.DeviceBuffer.from_numpy(w) for w in ws]
+    groups = (1, 1, E, 1)
+    rt.lib().occamy_set_weight_cache(0 if filters == "no cache" else 1)
+    try:
+        for i in range(6):
+            x = rand(10 + i, *shape)
+            with Inference() as f:
+                y, o, want = f.put(x), shape, x
+                for w, d, n in zip(ws, dev, groups):
+                    pw = f.copy(d.ptr, w.nbytes) if filters == "from the device" else f.put(w)
+                    pads = (w.shape[2] // 2,) * 2
+                    y, o = f.conv(y, o, pw, w.shape, pads=pads, groups=n)
+                    want = ref.conv2d(want, w, None, pads, groups=n)
+                    if w is not ws[-1]:
+                        y, want = f.clip(y, o, 0.0, 6.0), ref.clip(want, 0.0, 6.0)
+                got = f.get(y, o)
+            assert max_rel_err(got, want) <= 2e-2, i
+    finally:
+        rt.lib().occamy_set_weight_cache(1)
     assert rt.last_error() == 0
