@@ -446,9 +446,17 @@ __global__ void __launch_bounds__(IR_THREADS, 2) ir_kernel(const __grid_constant
         if (p.b2) V::filter(wd + 9u * WD_ROW, bt);
         else bt[0] = bt[1] = 0;
         const int units = p.tw * p.segs;
+        // The last chunk may reach past the E channels (E is a multiple of 16: a thread's four are all in or all
+        // out).  No filter was loaded for those, and their results meet the zeros that fill up the second
+        // filter: they have to be zero, not whatever the sums make of it.
+        const bool beyond = chunk_e0(c) + 4 * dq >= p.E;
 #pragma unroll 1
         for (int u = warp * COLS + dsub; u < units; u += 8 * COLS) {   // (tw is a multiple of eight: no warp is split)
           Unit w = u < 8 * COLS ? first_unit : unit(u);
+          if (beyond) {
+            for (; w.rows > 0; --w.rows, w.dst += dst_down) ir_sts64(w.dst, 0u, 0u);
+            continue;
+          }
           typename V::T win[3][3][2];   // [input row % 3][column][channel pair]
           auto load = [&](int slot) {
 #pragma unroll

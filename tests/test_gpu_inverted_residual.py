@@ -1,5 +1,6 @@
 """The inverted-residual kernel (1x1 -> 3x3 depthwise -> 1x1 as one launch) at the edges of its tiles, chunks
 and clusters, against the CPU oracle."""
+import numpy as np
 import pytest
 
 from calls import Inference, rand
@@ -83,4 +84,33 @@ def test_block_with_filters_that_do_not_stay(native_libs, filters, mode):
             assert max_rel_err(got, want) <= 2e-2, i
     finally:
         rt.lib().occamy_set_weight_cache(1)
+    assert rt.last_error() == 0
+
+
+@pytest.mark.parametrize("mode", [rt.MATH_BF16, rt.MATH_F16])
+@pytest.mark.parametrize("act", ["none", "relu", "clip"])
+@pytest.mark.parametrize("N,C,H,E,K", [(1, 16, 14, 48, 24), (1, 24, 14, 144, 24), (40, 16, 28, 48, 16), (1, 64, 14, 96, 64),
+                                       (1, 16, 14, 80, 24)])
+def test_last_chunk(binding, N, C, H, E, K, act, mode):
+    """Channels of the last chunk that do not exist count as zero, whatever an earlier kernel left in shared memory:
+    NaN here.  (A clamp of the depthwise results would hide it.)"""
+    g = graphs.Graph((N, C, H, H), seed=E + C)
+
+    def end(v):
+        return v if act == "none" else g.relu(v) if act == "relu" else g.clip(v, 0.0, 6.0)
+
+    x = g.conv(0, *g.he_conv(C, C, 1, 1))
+    y = end(g.conv(x, *g.he_conv(E, C, 1, 1)))
+    y = end(g.conv(y, *g.he_conv(E, 1, 3, 3), groups=E, pads=(1, 1)))
+    g.mark_output(g.conv(y, *g.he_conv(K, E, 1, 1)))
+    rt.set_math_mode(mode)
+    p = g.to_program()
+    p.lower(fuse=replay.FUSE_REFERENCE)
+    v = graphs.make_input(g, 1)
+    bad = np.full_like(v, np.nan)
+    (want,) = run_graph_oracle(g, v)
+    for i in range(6):
+        p.run(binding, bad)   # leaves NaN in every shared memory
+        (got,) = p.run(binding, v)
+        assert max_rel_err(got, want) <= 2e-2, i
     assert rt.last_error() == 0
