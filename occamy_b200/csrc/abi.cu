@@ -542,8 +542,9 @@ bool launch_block(ConvJob &a, ConvJob &b, ConvJob &c) {
   const ConvJob *job[3] = {&a, &b, &c};
   for (int i = 0; i < 3; ++i) {
     const ConvGeom &g = job[i]->g;
-    ir.lo[i] = g.act == ACT_RELU ? 0.0f : g.act == ACT_CLIP ? g.lo : -INFINITY;
-    ir.hi[i] = g.act == ACT_CLIP ? g.hi : INFINITY;
+    ir.floor[i] = g.act == ACT_RELU ? 0.0f : -INFINITY;
+    ir.lo[i] = g.act == ACT_CLIP ? g.lo : NAN;
+    ir.hi[i] = g.act == ACT_CLIP ? g.hi : NAN;
     if (g.act != ACT_IDENTITY && g.act != ACT_RELU && g.act != ACT_CLIP) return false;
   }
   const ConvGeom &g = c.g;

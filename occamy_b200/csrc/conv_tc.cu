@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_conv_pn_kernel(const __grid_
       else run_tiles(std::integral_constant<int, 1>{});
     }
   } else {
-    const float act_lo = p.lo, act_hi = p.hi;
+    const float act_floor = p.floor, act_lo = p.lo, act_hi = p.hi;
     const int quad = warp & 3;                 // TMEM lane quadrant = 32 output channels
     const int half = (warp - 2) >> 2;          // which 128 of the 256 pixel columns
     const int c_local = quad * 32 + lane;      // this thread's channel within the 128-tile
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_conv_pn_kernel(const __grid_
                 dslab + slab_off(pix, cin >> 3, 128) + (cin & 7) * 2);
             float v = __uint_as_float(r[j]) + bias;
             if (p.has_res) v += __bfloat162float(*cell);
-            *cell = __float2bfloat16_rn(tc_act(v, act_lo, act_hi));
+            *cell = __float2bfloat16_rn(tc_act(v, act_floor, act_lo, act_hi));
           }
         }
       }
@@ -694,8 +694,9 @@ static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, d
   p.ldo = a.ldo;
   p.out_hw = a.out_f32 && a.out_nchw ? a.P * a.Q : 0;
   p.out_vec4 = a.out_f32 && !p.out_hw && a.ldo % 4 == 0 && (uintptr_t)a.out_f32 % 16 == 0;
-  p.lo = a.act == ACT_RELU ? 0.0f : (a.act == ACT_CLIP ? a.lo : -INFINITY);
-  p.hi = a.act == ACT_CLIP ? a.hi : INFINITY;
+  p.floor = a.act == ACT_RELU ? 0.0f : -INFINITY;
+  p.lo = a.act == ACT_CLIP ? a.lo : NAN;
+  p.hi = a.act == ACT_CLIP ? a.hi : NAN;
   p.consts_ready = a.consts_ready;
   p.err = err_word;
   const uint32_t boxA[4] = {(uint32_t)bk, (uint32_t)p.tw, (uint32_t)p.th, (uint32_t)p.tn};
@@ -745,8 +746,9 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   p.bias = a.bias;
   p.has_res = a.residual ? 1 : 0;
   p.act = a.act;
-  p.lo = a.act == ACT_RELU ? 0.0f : (a.act == ACT_CLIP ? a.lo : -INFINITY);
-  p.hi = a.act == ACT_CLIP ? a.hi : INFINITY;
+  p.floor = a.act == ACT_RELU ? 0.0f : -INFINITY;
+  p.lo = a.act == ACT_CLIP ? a.lo : NAN;
+  p.hi = a.act == ACT_CLIP ? a.hi : NAN;
   p.out_f32 = a.out_f32;
   p.ldo = a.ldo;
   p.out_hw = a.out_f32 && a.out_nchw ? a.P * a.Q : 0;

@@ -46,7 +46,7 @@ struct alignas(64) TcParams {
   const float *bias;
   int has_res, act;
   int gq, gp, gn;        // extents of the output grid the tiles are cut from
-  float lo, hi;
+  float floor, lo, hi;                 // tc_act()
   float *out_f32;
   int ldo;
   int out_hw;            // fp32 output: 0 = row-major [pixel][ldo]; else P * Q of an NCHW tensor
@@ -441,8 +441,12 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, int bk) {
 
 // The fused activations (identity, ReLU, clipped ReLU) are all a clamp to [lo, hi]; keeping
 // the epilogue to that one form keeps its unrolled body small.
-__device__ __forceinline__ float tc_act(float v, float lo, float hi) {
-  return fminf(fmaxf(v, lo), hi);
+// A bound that is NaN is none; where there is one a NaN becomes the lower one, as the ABI's clip has it.
+__device__ __forceinline__ float tc_clip(float v, float lo, float hi) { return fminf(fmaxf(v, lo), hi); }
+// Any activation the tensor-core kernels take: `floor` 0 for ReLU, which keeps NaN, else -inf.
+__device__ __forceinline__ float tc_act(float v, float floor, float lo, float hi) {
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(v) : "f"(floor));
+  return tc_clip(v, lo, hi);
 }
 
 // Byte offset of 16-byte chunk `chunk` of row `row` inside a staged slab whose rows are
@@ -1035,7 +1039,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
     for (int i = et; i < p.bias_floats; i += EPI_THREADS)
       bias_s[i] = (p.bias && i < p.K) ? p.bias[i] : 0.0f;
     epi_bar_n<EPI_THREADS>();
-    const float act_lo = p.lo, act_hi = p.hi;
+    const float act_floor = p.floor, act_lo = p.lo, act_hi = p.hi;
     int acc = 0;
     uint32_t acc_phase = 0;
     uint32_t buf = 0, buf_phase = 0;         // slab buffer the next slab goes through
@@ -1099,9 +1103,9 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
               for (int j = 0; j < CW / 2; ++j) {
                 float a, b;
                 f2_unpack(v2[j], a, b);
-                if (c0 + 2 * j < p.K) o[(int64_t)(2 * j) * p.out_hw] = tc_act(a, act_lo, act_hi);
+                if (c0 + 2 * j < p.K) o[(int64_t)(2 * j) * p.out_hw] = tc_act(a, act_floor, act_lo, act_hi);
                 if (c0 + 2 * j + 1 < p.K)
-                  o[(int64_t)(2 * j + 1) * p.out_hw] = tc_act(b, act_lo, act_hi);
+                  o[(int64_t)(2 * j + 1) * p.out_hw] = tc_act(b, act_floor, act_lo, act_hi);
               }
             }
             return true;
@@ -1113,8 +1117,8 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
             for (int j = 0; j < CW / 2; ++j) {
               float a, b;
               f2_unpack(v2[j], a, b);
-              if (c0 + 2 * j < p.K) o[2 * j] = tc_act(a, act_lo, act_hi);
-              if (c0 + 2 * j + 1 < p.K) o[2 * j + 1] = tc_act(b, act_lo, act_hi);
+              if (c0 + 2 * j < p.K) o[2 * j] = tc_act(a, act_floor, act_lo, act_hi);
+              if (c0 + 2 * j + 1 < p.K) o[2 * j + 1] = tc_act(b, act_floor, act_lo, act_hi);
             }
           }
           return true;
@@ -1138,7 +1142,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
             if constexpr (CLAMP) {
               float a, b;
               f2_unpack(v2[j], a, b);
-              pk[j] = f2_to_bf16x2<F16>(f2_pack(tc_act(a, act_lo, act_hi), tc_act(b, act_lo, act_hi)));
+              pk[j] = f2_to_bf16x2<F16>(f2_pack(tc_clip(a, act_lo, act_hi), tc_clip(b, act_lo, act_hi)));
             } else {
               pk[j] = f2_to_bf16x2_relu<F16>(v2[j]);   // ReLU rides on the conversion
             }

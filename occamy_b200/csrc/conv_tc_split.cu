@@ -80,12 +80,12 @@ __device__ __forceinline__ uint4 sk_pack16(const SkParams &p, float *v, const ui
   uint32_t o[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j)
-    o[j] = f2_to_bf16x2<F16>(f2_pack(tc_act(v[2 * j], p.lo, p.hi), tc_act(v[2 * j + 1], p.lo, p.hi)));
+    o[j] = f2_to_bf16x2<F16>(f2_pack(tc_act(v[2 * j], p.floor, p.lo, p.hi), tc_act(v[2 * j + 1], p.floor, p.lo, p.hi)));
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 __device__ __forceinline__ void sk_finish32(const SkParams &p, bool on, float *v, int64_t lin, int c) {
 #pragma unroll
-  for (int j = 0; j < 8; ++j) v[j] = tc_act(v[j], p.lo, p.hi);
+  for (int j = 0; j < 8; ++j) v[j] = tc_act(v[j], p.floor, p.lo, p.hi);
   int64_t step = 1;
   float *o = p.out_f32 + lin * p.ldo + c;
   if (p.out_hw) {
@@ -122,7 +122,7 @@ __device__ __forceinline__ void sk_finish_parts(const SkParams &p, bool on, floa
   uint32_t o[3][4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    float a = tc_act(v[2 * e], p.lo, p.hi), b = tc_act(v[2 * e + 1], p.lo, p.hi);
+    float a = tc_act(v[2 * e], p.floor, p.lo, p.hi), b = tc_act(v[2 * e + 1], p.floor, p.lo, p.hi);
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       o[j][e] = f2_to_bf16x2<false>(f2_pack(a, b));

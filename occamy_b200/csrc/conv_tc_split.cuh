@@ -34,7 +34,7 @@ struct alignas(64) SkParams {
   float *out_f32;
   int ldo, out_hw;                     // as in TcParams
   int out_vec4;                        // row-major fp32 output whose rows are 16-byte aligned
-  float lo, hi;
+  float floor, lo, hi;                 // tc_act()
   int consts_ready;
   int *err;
 };

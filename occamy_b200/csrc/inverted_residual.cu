@@ -49,9 +49,10 @@ struct alignas(64) IrParams {
   int rows_owner;                      // output pixels each CTA of a cluster finishes
   TcFastDiv div_iw, div_tw, div_w, div_h, div_g8;
   uint32_t x_bytes, ex_bytes;          // one input tile; the chunk's expanded pixels
-  float lo3, hi3;
-  uint32_t lo1, hi1, lo2, hi2;         // clamps after the first two stages, as 16-bit pairs
-  int zero_inside;                     // lo1 <= 0 <= hi1
+  float floor3, lo3, hi3;              // tc_act()
+  uint32_t lo1, hi1, lo2, hi2;         // bounds after the first two stages, as 16-bit pairs
+  int clip1;                           // the first ones are a clip's (else hi1 is none)
+  int zero_inside;                     // zero is within the first one
   int consts_ready;
   int *err;
 };
@@ -87,9 +88,9 @@ __device__ __forceinline__ uint2 ir_lds64(uint32_t addr) {
   return v;
 }
 // Pairs of 16-bit values.  Rounding is monotonic, so clamping rounded values to rounded bounds is
-// rounding the clamped value.
+// rounding the clamped value.  A clip makes a bound of NaN, as the ABI's does ...
 template <bool F16>
-__device__ __forceinline__ uint32_t ir_clamp(uint32_t v, uint32_t lo, uint32_t hi) {
+__device__ __forceinline__ uint32_t ir_clip(uint32_t v, uint32_t lo, uint32_t hi) {
   if constexpr (F16) {
     asm("max.f16x2 %0, %0, %1;" : "+r"(v) : "r"(lo));
     asm("min.f16x2 %0, %0, %1;" : "+r"(v) : "r"(hi));
@@ -97,6 +98,21 @@ __device__ __forceinline__ uint32_t ir_clamp(uint32_t v, uint32_t lo, uint32_t h
     asm("max.bf16x2 %0, %0, %1;" : "+r"(v) : "r"(lo));
     asm("min.bf16x2 %0, %0, %1;" : "+r"(v) : "r"(hi));
   }
+  return v;
+}
+// ... ReLU (lo 0) and no activation (lo -inf) keep it,
+template <bool F16>
+__device__ __forceinline__ uint32_t ir_floor(uint32_t v, uint32_t lo) {
+  if constexpr (F16) asm("max.NaN.f16x2 %0, %0, %1;" : "+r"(v) : "r"(lo));
+  else asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(v) : "r"(lo));
+  return v;
+}
+// and so does any bound on the depthwise sums, where fp16 sums that overflow can make one.
+template <bool F16>
+__device__ __forceinline__ uint32_t ir_clamp(uint32_t v, uint32_t lo, uint32_t hi) {
+  v = ir_floor<F16>(v, lo);
+  if constexpr (F16) asm("min.NaN.f16x2 %0, %0, %1;" : "+r"(v) : "r"(hi));
+  else asm("min.NaN.bf16x2 %0, %0, %1;" : "+r"(v) : "r"(hi));
   return v;
 }
 template <bool F16>
@@ -422,7 +438,14 @@ __global__ void __launch_bounds__(IR_THREADS, 2) ir_kernel(const __grid_constant
           uint32_t v[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            v[j] = ir_clamp<F16>(ir_cvt<F16>(__uint_as_float(r[k * 8 + 2 * j]), __uint_as_float(r[k * 8 + 2 * j + 1])), lo, hi);
+            v[j] = ir_cvt<F16>(__uint_as_float(r[k * 8 + 2 * j]), __uint_as_float(r[k * 8 + 2 * j + 1]));
+          if (p.clip1) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = ir_clip<F16>(v[j], lo, hi);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = ir_floor<F16>(v[j], lo);
+          }
           if (px < pin) ir_sts128(row + (((uint32_t)(part * (EC / 16) + k) ^ key) << 4), v);
         }
       }
@@ -552,7 +575,7 @@ __global__ void __launch_bounds__(IR_THREADS, 2) ir_kernel(const __grid_constant
               const float2 bias = *reinterpret_cast<const float2 *>(b3_s + k * 16 + h * 8 + 2 * j);
               a += __uint_as_float(r[h * 8 + 2 * j]) + bias.x;
               b += __uint_as_float(r[h * 8 + 2 * j + 1]) + bias.y;
-              out[j] = f2_to_bf16x2<F16>(f2_pack(tc_act(a, p.lo3, p.hi3), tc_act(b, p.lo3, p.hi3)));
+              out[j] = f2_to_bf16x2<F16>(f2_pack(tc_act(a, p.floor3, p.lo3, p.hi3), tc_act(b, p.floor3, p.lo3, p.hi3)));
             }
             if (on && k * 16 + h * 8 < p.K && !err_code)
               *reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(p.y) + at + k * 16 + h * 8) =
@@ -642,7 +665,7 @@ __global__ void __launch_bounds__(IR_THREADS, 2) ir_kernel(const __grid_constant
         for (int j = 0; j < 4; ++j) {
           float a = 0.f, b = 0.f;
           if (p.residual) f2_unpack(pair16_to_f2<F16>(w[j]), a, b);
-          out[j] = f2_to_bf16x2<F16>(f2_pack(tc_act(v[2 * j] + a, p.lo3, p.hi3), tc_act(v[2 * j + 1] + b, p.lo3, p.hi3)));
+          out[j] = f2_to_bf16x2<F16>(f2_pack(tc_act(v[2 * j] + a, p.floor3, p.lo3, p.hi3), tc_act(v[2 * j + 1] + b, p.floor3, p.lo3, p.hi3)));
         }
         *reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(p.y) + at) = make_uint4(out[0], out[1], out[2], out[3]);
       };
@@ -859,10 +882,13 @@ IrPlan ir_build(const IrArgs &a) {
   p.div_g8 = make_fastdiv(a.K / 8);
   p.tiles = p.tiles_w * p.tiles_h * a.N;
   pl.c.smem = ir_smem(c.ec, p.kcs, p.bk, p.iw * p.ih, c.tw * c.th, p.Kp, c.splits, a.f16 != 0, &p.x_bytes, &p.ex_bytes);
-  p.lo1 = pair_bits(a.lo[0], a.f16); p.hi1 = pair_bits(a.hi[0], a.f16);
-  p.lo2 = pair_bits(a.lo[1], a.f16); p.hi2 = pair_bits(a.hi[1], a.f16);
-  p.zero_inside = a.lo[0] <= 0.0f && a.hi[0] >= 0.0f;
-  p.lo3 = a.lo[2]; p.hi3 = a.hi[2];
+  p.clip1 = a.lo[0] == a.lo[0];
+  p.lo1 = pair_bits(p.clip1 ? a.lo[0] : a.floor[0], a.f16);
+  p.hi1 = pair_bits(p.clip1 ? a.hi[0] : INFINITY, a.f16);
+  p.lo2 = pair_bits(a.lo[1] == a.lo[1] ? a.lo[1] : a.floor[1], a.f16);
+  p.hi2 = pair_bits(a.hi[1] == a.hi[1] ? a.hi[1] : INFINITY, a.f16);
+  p.zero_inside = !(a.lo[0] > 0.0f || a.hi[0] < 0.0f);
+  p.floor3 = a.floor[2]; p.lo3 = a.lo[2]; p.hi3 = a.hi[2];
   p.consts_ready = a.consts_ready;
   p.err = r.dev_err;
   bool ok = true;

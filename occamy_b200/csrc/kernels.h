@@ -179,7 +179,7 @@ struct IrArgs {
   const bf16 *residual;         // like y, or null
   bf16 *y;                      // [N][P][Q][K]
   int N, H, W, C, E, K, P, Q, stride;
-  float lo[3], hi[3];           // clamp behind each stage
+  float floor[3], lo[3], hi[3]; // activation behind each stage: ReLU's 0 (else -inf), a clip's bounds (else NaN)
   int f16, consts_ready;
 };
 // bias [E] -> 16-bit [E][16]: three parts that add up to it, zeros

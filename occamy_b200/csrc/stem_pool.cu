@@ -340,8 +340,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stem_pool_kernel(const StemPara
             float x0, x1, x2, x3;
             f2_unpack(v0, x0, x1);
             f2_unpack(v1, x2, x3);
-            pk[2 * j] = f2_to_bf16x2(f2_pack(tc_act(x0, lo, hi), tc_act(x1, lo, hi)));
-            pk[2 * j + 1] = f2_to_bf16x2(f2_pack(tc_act(x2, lo, hi), tc_act(x3, lo, hi)));
+            pk[2 * j] = f2_to_bf16x2(f2_pack(tc_clip(x0, lo, hi), tc_clip(x1, lo, hi)));
+            pk[2 * j + 1] = f2_to_bf16x2(f2_pack(tc_clip(x2, lo, hi), tc_clip(x3, lo, hi)));
           }
         }
         if (!mbar_wait_sleepy(cr_empty(cs), cph ^ 1u, abort_flag)) {

@@ -114,3 +114,27 @@ def test_last_chunk(binding, N, C, H, E, K, act, mode):
         (got,) = p.run(binding, v)
         assert max_rel_err(got, want) <= 2e-2, i
     assert rt.last_error() == 0
+
+
+@pytest.mark.parametrize("act", ["relu", "none"])
+def test_overflow_of_the_depthwise_sums(binding, act):
+    """fp16 sums that overflow in both directions are NaN, not a bound.  (A clip, by the ABI, makes a bound of NaN.)"""
+    N, C, E, H = 1, 16, 96, 14
+    g = graphs.Graph((N, C, H, H), seed=1)
+    wx, bx = g.he_conv(C, C, 1, 1)
+    x = g.conv(0, wx, bx)
+    w1, b1 = np.zeros((E, C, 1, 1), np.float32), np.full(E, 6e4, np.float32)
+    dw = np.zeros((E, 1, 3, 3), np.float32)
+    dw[:, 0, 0], dw[:, 0, 2] = 6e4, -6e4     # +inf from the row above, -inf from the row below
+    y = g.relu(g.conv(x, w1, b1))
+    y = g.conv(y, dw, np.zeros(E, np.float32), groups=E, pads=(1, 1))
+    y = g.relu(y) if act == "relu" else y
+    g.mark_output(g.conv(y, *g.he_conv(24, E, 1, 1)))
+    rt.set_math_mode(rt.MATH_F16)
+    p = g.to_program()
+    p.lower(fuse=replay.FUSE_REFERENCE)
+    v = graphs.make_input(g, 1)
+    for i in range(4):   # the first runs convolution by convolution
+        (got,) = p.run(binding, v)
+        assert np.isnan(got[:, :, 1:-1]).all(), i
+    assert rt.last_error() == 0

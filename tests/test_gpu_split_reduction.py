@@ -3,9 +3,11 @@ edges of its tiles and of its splits, against the CPU oracle."""
 import numpy as np
 import pytest
 
+from calls import Inference, rand
 from helpers import max_rel_err, run_graph_oracle
 from occamy_b200 import graphs, replay
 from occamy_b200 import runtime as rt
+from oracle import ref
 
 pytestmark = pytest.mark.gpu
 
@@ -61,4 +63,35 @@ def test_gemm(binding, M, K, N, mode):
     for _ in range(2):
         (got,) = p.run(binding, x)
         assert max_rel_err(got, want) <= TOL[mode]
+    assert rt.last_error() == 0
+
+
+@pytest.mark.parametrize("mode", [rt.MATH_FP32, rt.MATH_BF16, rt.MATH_F16])
+@pytest.mark.parametrize("act", [1, 5])
+def test_nan_stays(native_libs, mode, act):
+    """ReLU and no activation keep NaN, in the kernels for few tiles as well."""
+    rt.set_math_mode(mode)
+    w, b = rand(1, 64, 64, 3, 3, scale=0.1), rand(2, 64)
+    fc = rand(3, 48, 64, scale=0.1)
+    x = rand(4, 2, 64, 14, 14)
+    x[0, 3, 5, 6] = np.nan
+    m = rand(5, 4, 64)
+    m[1, 7] = np.nan
+    want, want2 = ref.conv2d(x, w, b, (1, 1), act=act), ref.matmul2d(m, fc, transB=1)
+    if act == 1:
+        want2 = np.where(np.isnan(want2), want2, np.maximum(want2, 0))
+    for i in range(4):
+        with Inference() as f:
+            y, o = f.conv(f.put(x), x.shape, f.put(w), w.shape, f.put(b), (1, 1), act=act)
+            got = f.get(y, o)
+            y, o = f.matmul(f.put(m), m.shape, f.put(fc), fc.shape)
+            if act == 1:
+                y2 = f.place(int(np.prod(o)) * 4)
+                rt.lib().DNNActiveFunc(f.h, y, rt.dims(o + (1, 1)), 1, y2)
+                y = y2
+            got2 = f.get(y, o)
+        for g, t in ((got, want), (got2, want2)):
+            assert np.array_equal(np.isnan(g), np.isnan(t)), i
+            ok = ~np.isnan(t)
+            assert max_rel_err(g[ok], t[ok]) <= 2e-2
     assert rt.last_error() == 0
