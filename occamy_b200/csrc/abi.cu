@@ -550,9 +550,9 @@ bool launch_block(ConvJob &a, ConvJob &b, ConvJob &c) {
   const ConvGeom &g = c.g;
   ir.x = a.a.x; ir.w1 = a.a.w; ir.b1 = (const bf16 *)a.block_b;
   ir.w2 = b.dw_w; ir.b2 = b.bias;
-  if (mode_f16()) {
+  if (mode_f16()) {   // the kernel sums in fp16, which is for those depthwise convolutions that do so by themselves
     ir.w2 = b.block_w; ir.b2 = b.block_b;
-    if (!ir.w2 || (b.bias && !ir.b2)) return false;
+    if (!depthwise_sums_in_half(b.g) || !ir.w2 || (b.bias && !ir.b2)) return false;
   }
   ir.w3 = c.a.w; ir.b3 = c.a.bias;
   ir.residual = c.a.residual;

@@ -493,13 +493,10 @@ __global__ void __launch_bounds__(IR_THREADS, 2) ir_kernel(const __grid_constant
           auto output = [&](int a, int b, int d) {   // window slots of the three filter rows
             typename V::T s[2] = {bt[0], bt[1]};
 #pragma unroll
-            for (int j = 0; j < 3; ++j)
+            for (int j = 0; j < 9; ++j)   // row by row, like the kernel for this stage alone
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                s[h] = V::fma(win[a][j][h], wt[j][h], s[h]);
-                s[h] = V::fma(win[b][j][h], wt[3 + j][h], s[h]);
-                s[h] = V::fma(win[d][j][h], wt[6 + j][h], s[h]);
-              }
+              for (int h = 0; h < 2; ++h)
+                s[h] = V::fma(win[j < 3 ? a : j < 6 ? b : d][j % 3][h], wt[j][h], s[h]);
             ir_sts64(w.dst, ir_clamp<F16>(V::out(s[0]), p.lo2, p.hi2), ir_clamp<F16>(V::out(s[1]), p.lo2, p.hi2));
             w.dst += dst_down;
           };

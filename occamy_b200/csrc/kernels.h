@@ -86,6 +86,8 @@ void launch_pool_bf16(const bf16 *x, bf16 *y, int N, int C, int H, int W, int P,
                       cudaStream_t s);
 // Global average pool: x [N, HW, C] 16-bit -> y [N, C] fp32, or y16 [N, C] 16-bit when that is given.
 void launch_gap_bf16(const bf16 *x, float *y, bf16 *y16, int N, int HW, int C, bool f16, cudaStream_t s);
+// Whether the fp16 mode's kernel for this depthwise convolution sums in fp16 (else in fp32).
+bool depthwise_sums_in_half(const ConvGeom &g);
 // Depthwise RxS convolution on 16-bit NHWC, weights fp32 packed [R*S][C], fused bias + act.
 void launch_depthwise_bf16(const bf16 *x, const float *w_rsc, const float *bias, bf16 *y,
                            const ConvGeom &g, bool f16, bool consts_ready, cudaStream_t s);

@@ -949,6 +949,17 @@ __global__ void __launch_bounds__(128, 4)
   }
 }
 
+// The packed fp16 kernel takes bounds that fp16 holds exactly (lower bound 0 or none), relies on a valid middle
+// column and on 32-bit thread numbers.
+bool depthwise_sums_in_half(const ConvGeom &g) {
+  const float lo = g.act == ACT_RELU ? 0.0f : (g.act == ACT_CLIP ? g.lo : -INFINITY);
+  const float hi = g.act == ACT_CLIP ? g.hi : INFINITY;
+  return g.R == 3 && g.S == 3 && g.stride_h == g.stride_w && (g.stride_h == 1 || g.stride_h == 2) &&
+         (g.act == ACT_IDENTITY || g.act == ACT_RELU || g.act == ACT_CLIP) && (lo == 0.0f || lo == -INFINITY) &&
+         (hi == INFINITY || host_elem_value(host_elem_bits(hi, true), true) == hi) && g.pad_w >= 0 && g.pad_w <= 1 &&
+         (int64_t)g.N * g.P * g.Q * (g.C / 8) * 16 < (int64_t)1 << 31;
+}
+
 void launch_depthwise_bf16(const bf16 *x, const float *w_rsc, const float *bias, bf16 *y,
                            const ConvGeom &g, bool f16, bool consts_ready, cudaStream_t s) {
   const int64_t total = (int64_t)g.N * g.P * g.Q * (g.C / 8);
@@ -969,13 +980,9 @@ void launch_depthwise_bf16(const bf16 *x, const float *w_rsc, const float *bias,
     // Channels per thread: 4.  (2 halves the registers and doubles the resident CTAs, but the
     // kernel is bound by its instruction count, which grows: measured 1.4x slower.)
     // fp16 mode with bounds fp16 holds: 8, computed on packed fp16 pairs (see the kernel).
-    bool h2 = f16 && packed;
+    bool strip = f16 && depthwise_sums_in_half(g);
 #ifdef OCCAMY_TUNING
-    if (const char *f = getenv("OCCAMY_DW_H2")) h2 = h2 && atoi(f) != 0;
-#endif
-    // the kernel relies on a valid middle column and on 32-bit thread numbers
-    bool strip = h2 && g.pad_w >= 0 && g.pad_w <= 1 && total * 16 < (int64_t)1 << 31;
-#ifdef OCCAMY_TUNING
+    if (const char *f = getenv("OCCAMY_DW_H2")) strip = strip && atoi(f) != 0;
     if (const char *f = getenv("OCCAMY_DW_STRIP")) strip = strip && atoi(f) != 0;
 #endif
     if (strip) {

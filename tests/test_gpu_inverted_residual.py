@@ -138,3 +138,25 @@ def test_overflow_of_the_depthwise_sums(binding, act):
         (got,) = p.run(binding, v)
         assert np.isnan(got[:, :, 1:-1]).all(), i
     assert rt.last_error() == 0
+
+
+@pytest.mark.parametrize("hi,sums_in_half", [(6.1, False), (6.0, True)])
+def test_precision_of_the_depthwise_sums(binding, hi, sums_in_half):
+    """2048 + 1 - 2048: 1 in fp32, 0 in fp16.  In the fp16 mode the depthwise kernel whose clamp has a bound that fp16
+    does not hold (6.1) sums in fp32, and a block with one must not do otherwise.  (The first pass clamps apart.)"""
+    N, C, E, K, H = 1, 16, 96, 24, 14
+    g = graphs.Graph((N, C, H, H), seed=1)
+    dw = np.zeros((E, 1, 3, 3), np.float32)
+    dw[:, 0, 0, 0], dw[:, 0, 1, 1], dw[:, 0, 2, 2] = 2048.0, 1.0, -2048.0
+    x = g.conv(0, *g.he_conv(C, C, 1, 1))
+    y = g.clip(g.conv(x, np.zeros((E, C, 1, 1), np.float32), np.ones(E, np.float32)), 0.0, 6.0)
+    y = g.clip(g.conv(y, dw, np.zeros(E, np.float32), groups=E, pads=(1, 1)), 0.0, hi)
+    g.mark_output(g.conv(y, np.full((K, E, 1, 1), 0.125, np.float32), np.zeros(K, np.float32)))
+    rt.set_math_mode(rt.MATH_F16)
+    p = g.to_program()
+    p.lower(fuse=replay.FUSE_REFERENCE)
+    v = graphs.make_input(g, 1)
+    for i in range(4):
+        (got,) = p.run(binding, v)
+        assert i == 0 or (got[:, :, 1:-1, 1:-1] == (0.0 if sums_in_half else E / 8)).all(), i
+    assert rt.last_error() == 0
