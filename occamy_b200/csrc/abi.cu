@@ -181,6 +181,15 @@ const float *resident_f32(const float *p, size_t bytes) {
   return p;
 }
 
+// The second operand of an element-wise call or of a product, the filter of a convolution on the CUDA cores.
+// It may be an input of the model as well as a constant, and of a large one the fingerprint is a sample: those are
+// read from the tensor itself, uploaded in full every time.
+const float *operand_f32(const float *p, size_t bytes) {
+  if (bytes <= HASH_WHOLE) return resident_f32(p, bytes);
+  ensure_f32(p);
+  return p;
+}
+
 // ---- a convolution resolved down to launch arguments ------------------------------
 // `prepare_*` does everything that depends on the inputs' current state (layout
 // conversion into scratch, packed-weight lookup, bias lookup); what is left is a launch
@@ -853,8 +862,8 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
     }
   }
   ensure_f32(x);
-  const float *wd = resident_f32(w, (size_t)numel4(dW) * 4);
-  const float *bd = bias ? resident_f32(bias, (size_t)g.K * 4) : nullptr;
+  const float *wd = operand_f32(w, (size_t)numel4(dW) * 4);
+  const float *bd = bias ? operand_f32(bias, (size_t)g.K * 4) : nullptr;
   if (depthwise) launch_depthwise_f32(x, wd, bd, y, g, r.stream);
   else launch_conv_f32(x, wd, bd, y, g, r.stream);
   mark_f32(y);
@@ -1395,8 +1404,8 @@ float *DNNTensorOpFunc(cudnnContext *, int64_t opMode, float *A, int64_t *dimA, 
     }
   }
   ensure_f32(A);
-  // a constant (the C operand of a Gemm, say) is read from its resident copy
-  const float *Bd = opMode != 4 ? resident_f32(B, (size_t)prod(dB, rankA) * 4) : B;
+  // a small constant (the C operand of a Gemm, say) is read from its resident copy
+  const float *Bd = opMode != 4 ? operand_f32(B, (size_t)prod(dB, rankA) * 4) : B;
   if (opMode != 0 && opMode != 1 && opMode != 4) {
     set_error(996, "tensor op: unsupported mode");
     return out;
@@ -1654,7 +1663,7 @@ float *CUBLASMatmul2dFunc(int64_t /*rank*/, float *A, int64_t dimA[2], float *B,
     }
   }
   ensure_f32(A);
-  const float *Bd = resident_f32(B, (size_t)(dimB[0] * dimB[1]) * 4);
+  const float *Bd = operand_f32(B, (size_t)(dimB[0] * dimB[1]) * 4);
   if (beta != 0.0f) ensure_f32(out);
   launch_gemm_f32(A, Bd, out, M, N, K, (int)dimA[1], (int)dimB[1], alpha, out_zero ? 0.0f : beta,
                   transA != 0, transB != 0, r.stream);

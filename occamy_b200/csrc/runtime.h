@@ -165,6 +165,8 @@ void *scratch_get(int slot, size_t bytes);
 // Error word of the allocation-free entry point on the current device (0 when it was never
 // used there); see no_alloc.cu.
 int noalloc_poll_error(bool clear);
+// Fingerprint of a host buffer; of one up to HASH_WHOLE bytes every byte counts, of a larger one a sample.
+constexpr size_t HASH_WHOLE = 16 * 1024;
 uint64_t host_hash(const void *src, size_t bytes);
 
 inline void count(Counter c, int64_t v = 1) { rt().counters[c] += v; }

@@ -55,3 +55,20 @@ def test_constants_in_front_of_the_batch(native_libs):
             got = f.get(y, o)
         assert max_rel_err(got, want) <= 2e-2, i
     assert rt.last_error() == 0
+
+
+def test_large_operand_changed_in_one_place(native_libs):
+    """An operand of an element-wise call or a product may be an input: every byte of it counts."""
+    rt.set_math_mode(rt.MATH_BF16)
+    x, z, m = rand(1, 1, 64, 64, 64), rand(2, 1, 64, 64, 64), rand(3, 256, 512)
+    a = rand(4, 8, 256)
+    for i in range(PASSES):
+        z.reshape(-1)[70001 + 4099 * i] += 3.0
+        m.reshape(-1)[30001 + 4099 * i] += 3.0
+        with Inference() as f:
+            s = f.get(f.op(0, f.put(x), x.shape, f.put(z), z.shape), x.shape)
+            y, o = f.matmul(f.put(a), a.shape, f.put(m), m.shape, trans_b=0)
+            y = f.get(y, o)
+        assert np.array_equal(s, x + z), i
+        assert max_rel_err(y, ref.matmul2d(a, m)) <= 2e-2, i
+    assert rt.last_error() == 0
