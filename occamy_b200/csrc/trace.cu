@@ -352,8 +352,8 @@ void te_ptr(Entry &e, const void *p) {
 }
 void te_ptr_or_elsewhere(Entry &e, const void *p) {
   uintptr_t a = (uintptr_t)p;
-  if (!g_ts.pool_base) mix(e.sig, (uint64_t)a);
-  else if (a >= g_ts.pool_base && a < g_ts.pool_base + g_ts.pool_bytes) te_ptr(e, p);
+  const bool inside = a >= g_ts.pool_base && a < g_ts.pool_base + g_ts.pool_bytes;
+  if (!g_ts.pool_base || inside || reg_find(p)) te_ptr(e, p);
   else mix(e.sig, 1);
 }
 void te_i(Entry &e, int64_t v) { mix(e.sig, (uint64_t)v); }

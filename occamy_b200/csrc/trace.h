@@ -71,8 +71,8 @@ void te_i(Entry &e, int64_t v);
 void te_f(Entry &e, float v);
 void te_dims(Entry &e, const int64_t *d, int n);
 
-// A pointer that names the same tensor only when it lies in the active pool; any other device
-// address counts as "elsewhere" while a pool is active (the caller's batch, its result buffer).
+// The same for a copy's other end: while a pool is active, any device address that is no tensor of the runtime's
+// counts as "elsewhere" (the caller's batch, its result buffer).
 void te_ptr_or_elsewhere(Entry &e, const void *p);
 
 // A recorded inference: the calls between cudnnCreate and cudnnDestroy and the role of each.

@@ -72,3 +72,23 @@ def test_large_operand_changed_in_one_place(native_libs):
         assert np.array_equal(s, x + z), i
         assert max_rel_err(y, ref.matmul2d(a, m)) <= 2e-2, i
     assert rt.last_error() == 0
+
+
+def test_copies_from_tensors_outside_the_pool(native_libs):
+    """The same calls but for which of two tensors of the runtime's, outside the pool, is copied in."""
+    rt.set_math_mode(rt.MATH_BF16)
+    x, w, b = rand(1, 1, 16, 12, 12), rand(2, 16, 16, 3, 3, scale=0.1), rand(3, 16)
+    t, u = rt.DeviceBuffer(x.nbytes), rt.DeviceBuffer.from_numpy(rand(4, *x.shape))
+    mid = ref.conv2d(x, w, b, (1, 1))
+    for i, which in enumerate([u] * 4 + [t, u, t, t, u, t]):
+        with Inference() as f:
+            px, pw, pb = f.put(x), f.put(w), f.put(b)
+            f.conv(px, x.shape, pw, w.shape, pb, (1, 1), act=5, y=t.ptr)
+            r = f.relu(t.ptr, x.shape)
+            got = f.get(f.copy(which.ptr, x.nbytes), x.shape), f.get(r, x.shape)
+        if i == 4:   # leaves the recorded sequence behind a tensor that was skipped: reported, and recorded anew
+            assert rt.last_error() == 990
+            continue
+        assert max_rel_err(got[0], mid if which is t else rand(4, *x.shape)) <= 2e-2
+        assert max_rel_err(got[1], np.maximum(mid, 0)) <= 2e-2
+        assert rt.last_error() == 0
