@@ -656,8 +656,7 @@ Role step(Entry &e, bool passive) {
     g_pending.out16 = false;   // who reads it is not known any more
     g_pending.out_parts = g_pending.a.split && g_pending.res_set;
     flush_pending();
-    for (auto &kv : rt().recs)   // nor who reads the inputs: back to their plain form
-      if (kv.second.dev_src) ensure_f32((const void *)kv.first);
+    settle_sources();   // nor who reads the inputs: back to their plain form
     // Tensors that fusion skipped earlier in this inference stay unwritten.  The recorded
     // program had no reader for them; should this (different) program read one, that read
     // reports error 990.  A shared prefix alone - two models with the same first layers - is
@@ -687,11 +686,12 @@ void put(Entry &e, int &at, int64_t v) { put(e, at, &v, 1); }
 
 // A device-to-device copy into tensor `rec` whose readers are convolutions of the 16-bit path: brings it in
 // in the form they take, straight from the source (the plain copy and the conversion behind it moved
-// the batch twice: 79 us of a batch-256 ResNet-50).  False when the form is not known.
+// the batch twice: 79 us of a batch-256 ResNet-50).  False when the form is not known, or when the source is a
+// tensor of the runtime's, whose memory later calls may write.
 bool copy_for_conv(const float *src, float *dst, size_t bytes, TensorRec *rec) {
   Runtime &r = rt();
   const Entry *rd = (trace_last_flags() & RF_FOR_CONV) ? trace_last_reader() : nullptr;
-  if (!rd || r.mode == MATH_FP32) return false;
+  if (!rd || r.mode == MATH_FP32 || reg_find(src)) return false;
   const int64_t *v = rd->args.v;   // dX[4], dW[4], pads[2], strides[2], groups
   ConvGeom g;
   memset(&g, 0, sizeof(g));
@@ -1095,6 +1095,7 @@ cudaError_t wrapDNNMemcpy(void *dst, const void *src, size_t count_, int kind,
     e.in[0] = (uintptr_t)src;
     e.in_bytes[0] = (int64_t)count_;
     step(e, false);
+    settle_sources();   // (the call waits for the stream)
     uintptr_t base;
     TensorRec *rec = reg_find(src, &base);
     const void *from = src;
@@ -1121,6 +1122,7 @@ cudaError_t wrapDNNMemcpy(void *dst, const void *src, size_t count_, int kind,
   } else {
     Entry e = trace_entry(S_OPAQUE);
     step(e, false);
+    settle_sources();
     err = cudaMemcpyAsync(dst, src, count_, (cudaMemcpyKind)kind, r.stream);
     if (err == cudaSuccess) err = cudaStreamSynchronize(r.stream);
   }
@@ -1178,6 +1180,7 @@ cudaError_t wrapDNNDealloc(void *devPtr) {
     step(e, true);
     pending_guard_range(devPtr, bytes ? bytes : 1, true);
   }
+  settle_sources();
   OCC_CUDA(cudaStreamSynchronize(r.stream));
   if (bytes) reg_drop_range(devPtr, bytes);
   cudaError_t err = cudaFree(devPtr);
@@ -1732,6 +1735,7 @@ void occamy_internal_opaque_call(void) {
   graph_settle();
   Entry e = trace_entry(S_OPAQUE);
   step(e, false);
+  settle_sources();
 }
 
 }  // extern "C"
@@ -1830,6 +1834,7 @@ int occamy_synchronize(void) {
   Runtime &r = rt();
   graph_settle();
   flush_pending();
+  settle_sources();
   cudaError_t e = cudaStreamSynchronize(r.stream);
   if (e != cudaSuccess) set_error((int)e, "synchronize");
   poll_watchdog();
@@ -1841,6 +1846,7 @@ int occamy_synchronize(void) {
 cudaStream_t occamy_stream(void) {
   rt();
   graph_settle();   // the caller may order work of its own behind the calls made so far
+  settle_sources();
   return rt().stream;
 }
 

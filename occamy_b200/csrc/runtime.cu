@@ -247,6 +247,13 @@ void ensure_f32(const void *p) {
   rec->fmt = FMT_F32;
 }
 
+void settle_sources() {
+  std::vector<uintptr_t> all;
+  for (const auto &kv : rt().recs)
+    if (kv.second.dev_src) all.push_back(kv.first);
+  for (uintptr_t p : all) ensure_f32((const void *)p);
+}
+
 void *scratch_get(int slot, size_t bytes) {
   Runtime &r = rt();
   if (r.scratch_bytes[slot] >= bytes) return r.scratch[slot];

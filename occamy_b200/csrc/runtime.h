@@ -40,8 +40,9 @@ struct TensorRec {
   // Where a 16-bit tensor's bytes are when not at the tensor's own address (home_acquire()): its
   // address was still to be read by the kernel that wrote it, or the tensor outlives its address.
   const void *home = nullptr;
-  // Device address the tensor was copied from, when the copy brought it in in another form; the plain
-  // form is fetched from there if something asks for it after all.
+  // Caller's device memory the tensor was copied from, when the copy brought it in in another form; the plain
+  // form is fetched from there if something asks for it after all, and before the caller can know that the
+  // copy has been made and use that memory for something else (settle_sources()).
   const void *dev_src = nullptr;
   int stem_wp = 0, stem_cp = 0, stem_pad = 0, stem_f16 = 0;   // FMT_STEM_ROWS: its geometry and element type
   const void *host_src = nullptr;      // source of the last host->device upload, if any
@@ -140,6 +141,8 @@ void reg_drop_range(void *p, size_t bytes);
 TensorRec *reg_find(const void *p, uintptr_t *base = nullptr);
 // Make the bytes behind p plain fp32 NCHW (memset, upload or layout conversion as needed).
 void ensure_f32(const void *p);
+// The same for every tensor that would have to be fetched from where it was copied from (TensorRec::dev_src).
+void settle_sources();
 // True when p is the base of a 16-bit NHWC tensor with exactly these logical dims, stored in
 // the element type of the CURRENT mode (a tensor left behind in the other 16-bit type is
 // converted back to fp32 by its next reader, like any other foreign format).

@@ -92,3 +92,37 @@ def test_copies_from_tensors_outside_the_pool(native_libs):
         assert max_rel_err(got[0], mid if which is t else rand(4, *x.shape)) <= 2e-2
         assert max_rel_err(got[1], np.maximum(mid, 0)) <= 2e-2
         assert rt.last_error() == 0
+
+
+@pytest.mark.parametrize("outside", [True, False])
+def test_source_of_a_copy_is_overwritten(native_libs, outside):
+    """What was copied in stays what it was, whatever happens to where it came from."""
+    rt.set_math_mode(rt.MATH_BF16)
+    w, b, z = rand(1, 16, 16, 3, 3, scale=0.1), rand(2, 16), rand(3, 1, 16, 12, 12)
+
+    def run(x, conv):
+        with Inference() as f:
+            src, at = device(x), f.at
+            s = f.place(x.nbytes)
+            t = f.place(x.nbytes)
+            rt.lib().wrapDNNMemcpy(s, src.data_ptr(), x.nbytes, 3, None)
+            rt.lib().wrapDNNMemcpy(t, src.data_ptr() if outside else s, x.nbytes, 3, None)
+            if outside:
+                rt.synchronize()
+                src.zero_()
+                torch.cuda.synchronize()
+            else:
+                f.put(z, at=at)
+            if conv:
+                y, o = f.conv(t, x.shape, f.put(w), w.shape, f.put(b), (1, 1), act=5)
+            else:
+                y, o = f.relu(t, x.shape), x.shape
+            return f.get(y, o)
+    for i, conv in enumerate([True] * 7 + [False, True, False] + [True] * 4 + [False]):
+        x = rand(20 + i, 1, 16, 12, 12)
+        got = run(x, conv)
+        if conv:
+            assert max_rel_err(got, ref.conv2d(x, w, b, (1, 1))) <= 2e-2
+        else:
+            assert np.array_equal(got, np.maximum(x, 0))
+    assert rt.last_error() == 0
