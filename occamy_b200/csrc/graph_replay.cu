@@ -588,10 +588,21 @@ void launch_segment() {
   }
 }
 
+// Graphs write into buffers of the runtime's that were free when they were captured.  The values of this
+// inference's tensors that are in such buffers are compared (same_registry); those of tensors outside the pool
+// move to their tensors' own memory.
+void clear_homes(uintptr_t base, size_t bytes) {
+  std::vector<uintptr_t> all;
+  for (const auto &kv : rt().recs)
+    if (kv.second.home && (kv.first < base || kv.first >= base + bytes)) all.push_back(kv.first);
+  for (uintptr_t p : all) ensure_f32((const void *)p);
+}
+
 void start_window() {
   gr.prog = trace_candidate();
   GraphPlan &plan = *gr.prog->graph;
   const uintptr_t base = trace_pool_base();
+  clear_homes(base, trace_pool_bytes());
   auto select = [&](bool pieces) {
     gr.left.clear();
     for (auto &v : plan.variants)

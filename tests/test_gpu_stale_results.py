@@ -6,6 +6,7 @@ import torch
 
 from calls import Inference, rand
 from helpers import max_rel_err
+from occamy_b200 import graphs
 from occamy_b200 import runtime as rt
 from oracle import ref
 
@@ -125,4 +126,29 @@ def test_source_of_a_copy_is_overwritten(native_libs, outside):
             assert max_rel_err(got, ref.conv2d(x, w, b, (1, 1))) <= 2e-2
         else:
             assert np.array_equal(got, np.maximum(x, 0))
+    assert rt.last_error() == 0
+
+
+def test_tensor_outside_the_pool_in_a_buffer_of_the_runtime(binding):
+    """An in-place convolution by direct calls leaves its result in a buffer of the runtime's; a model that was
+    captured while that buffer was free is replayed before the result is read."""
+    rt.set_math_mode(rt.MATH_BF16)
+    g = graphs.resnet50(batch=1, seed=1, softmax=False, image=64)
+    p = g.to_program()
+    p.lower(fuse=0)
+    v = graphs.make_input(g, 1)
+    for _ in range(PASSES):
+        (want_model,) = p.run(binding, v)
+    L, d = rt.lib(), rt.dims
+    x, w = rand(1, 1, 64, 16, 16), rand(2, 64, 64, 1, 1, scale=0.2)
+    t, tw = rt.DeviceBuffer.from_numpy(x), rt.DeviceBuffer.from_numpy(w)
+    want = x
+    for i in range(4):
+        for _ in range(2):
+            L.DNNConvFunc(None, t.ptr, d(x.shape), tw.ptr, d(w.shape), None, 0, 0, 1, d((0, 0)), d((1, 1)), t.ptr)
+            want = ref.conv2d(want, w)
+        (y,) = p.run(binding, v)
+        assert np.array_equal(y, want_model)
+        assert max_rel_err(t.to_numpy(x.shape), want) <= 5e-2, i
+        want = t.to_numpy(x.shape)
     assert rt.last_error() == 0
