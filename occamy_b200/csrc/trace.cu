@@ -430,6 +430,8 @@ void trace_begin() {
   ts.prefix = nullptr;
   ts.prefix_len = 0;
   ts.elided = 0;
+  ts.last_pool_base = ts.pool_base;   // a pool set up before cudnnCreate; otherwise none yet
+  ts.last_pool_bytes = ts.pool_bytes;
   ts.cands.clear();
   for (size_t i = 0; i < ts.programs.size(); ++i) ts.cands.push_back((int)i);
 }
