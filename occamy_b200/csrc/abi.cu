@@ -143,7 +143,7 @@ void *packed_weights(const float *w, int layout, size_t packed_bytes, int K, int
   if (layout == PACK_KRSC) launch_pack_krsc_bf16(w, (bf16 *)dst, K, C, R, S, Cp, f16, r.stream);
   else if (layout == PACK_DW) launch_pack_dw_f32(w, (float *)dst, C, R, S, r.stream);
   else if (layout == PACK_RAW)
-    OCC_CUDA(cudaMemcpyAsync(dst, w, packed_bytes, cudaMemcpyDeviceToDevice, r.stream));
+    enqueue_copy(dst, w, packed_bytes, r.stream);
   else if (layout == PACK_STEM) launch_pack_stem_bf16(w, (bf16 *)dst, C, R, S, Cp, Sp * Cp, r.stream);
   else if (layout == PACK_BIAS3) launch_pack_bias3(w, (bf16 *)dst, K, f16, r.stream);
   else if (layout == PACK_IR_HALF) launch_pack_ir_half(w, dst, K, R * S, r.stream);
@@ -505,7 +505,7 @@ const bf16 *launch_job(ConvJob &job, bool apart = false) {
       if (!ranges_overlap(olo, ohi + obytes, job.dep_lo[k], job.dep_hi[k])) continue;
       const size_t bytes = job.dep_hi[k] - job.dep_lo[k];
       void *tmp = scratch_get(k ? 7 : 4, bytes);
-      OCC_CUDA(cudaMemcpyAsync(tmp, (const void *)job.dep_lo[k], bytes, cudaMemcpyDeviceToDevice, r.stream));
+      enqueue_copy(tmp, (const void *)job.dep_lo[k], bytes, r.stream);
       if (k) job.a.bias = (const float *)tmp;
       else job.a.x = (const bf16 *)tmp;
       count(CNT_LAUNCHES);
@@ -1715,7 +1715,7 @@ static float *copy_common(int sym, float *x, int64_t *dimIn, int64_t rank, float
     return y;
   }
   ensure_f32(x);
-  OCC_CUDA(cudaMemcpyAsync(y, x, (size_t)n * 4, cudaMemcpyDeviceToDevice, r.stream));
+  enqueue_copy(y, x, (size_t)n * 4, r.stream);
   mark_f32(y);
   return y;
 }

@@ -11,6 +11,8 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "kernels.h"
+
 namespace occ {
 
 constexpr int TC_THREADS = 320;      // pixel-N kernel: 1 producer warp + 1 MMA warp + 8 epilogue warps
@@ -1253,7 +1255,8 @@ inline void tc_launch_pdl(Kernel kernel, int grid, int threads, size_t smem, cud
     attr[1].val.clusterDim.z = 1;
     cfg.numAttrs = 2;
   }
-  cudaLaunchKernelEx(&cfg, kernel, p);
+  void *args[] = {const_cast<void *>(static_cast<const void *>(&p))};
+  enqueue_kernel((const void *)kernel, cfg, args);
 }
 
 // A function attribute (the dynamic shared memory limit) belongs to the current device.  Each

@@ -4,6 +4,8 @@
 #include <cstring>
 #include <map>
 
+#include "kernels.h"
+
 namespace occ {
 
 #ifdef OCCAMY_TUNING
@@ -161,39 +163,156 @@ bool same_registry(const std::vector<SavedRec> &a, uintptr_t base, size_t bytes)
   return it == recs.end() || it->first >= base + bytes;
 }
 
-// ---- capture --------------------------------------------------------------------
+// ---- recording ------------------------------------------------------------------
+// The graph is put together node by node from the runtime's own launches.  (A stream capture would do it too, but
+// while a stream of a device captures, any thread's wait for the device fails and makes the capture invalid.)
+struct Work {   // one node, enough to enqueue it by itself
+  cudaGraphNode_t node;
+  void *dst;             // copies and zero fills; null: a kernel
+  const void *src;       // null: a zero fill
+  size_t bytes;
+};
+struct Recording {
+  cudaGraph_t graph = nullptr;
+  std::vector<Work> work;
+};
+Recording *recording = nullptr;
+
+bool record_begin() {
+  std::unique_ptr<Recording> rec(new Recording);
+  if (cudaGraphCreate(&rec->graph, 0) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  recording = rec.release();
+  return true;
+}
+
+// Appends `w`, whose node has no dependencies yet, behind the last one.
+bool record_append(const Work &w, bool chained) {
+  cudaError_t e = cudaSuccess;
+  if (!recording->work.empty()) {
+    const Work &last = recording->work.back();
+    cudaGraphEdgeData edge = {};
+    if (chained && !last.dst) {   // may start while the kernel before it is still running
+      edge.from_port = cudaGraphKernelNodePortProgrammatic;
+      edge.type = cudaGraphDependencyTypeProgrammatic;
+    }
+    e = cudaGraphAddDependencies_v2(recording->graph, &last.node, &w.node, &edge, 1);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    cudaGraphDestroyNode(w.node);
+    return false;
+  }
+  recording->work.push_back(w);
+  return true;
+}
+
+bool record_kernel(const void *kernel, const cudaLaunchConfig_t &cfg, void **args) {
+  cudaKernelNodeParams p = {};
+  p.func = const_cast<void *>(kernel);
+  p.gridDim = cfg.gridDim;
+  p.blockDim = cfg.blockDim;
+  p.sharedMemBytes = (unsigned)cfg.dynamicSmemBytes;
+  p.kernelParams = args;
+  Work w = {};
+  bool chained = false;
+  cudaError_t e = cudaGraphAddKernelNode(&w.node, recording->graph, nullptr, 0, &p);
+  for (unsigned i = 0; i < cfg.numAttrs && e == cudaSuccess; ++i) {
+    if (cfg.attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization) chained = true;
+    else e = cudaGraphKernelNodeSetAttribute(w.node, cfg.attrs[i].id, &cfg.attrs[i].val);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return record_append(w, chained);
+}
+
+bool record_copy(void *dst, const void *src, size_t bytes) {
+  Work w = {};
+  w.dst = dst;
+  w.src = src;
+  w.bytes = bytes;
+  cudaError_t e;
+  if (src) {
+    e = cudaGraphAddMemcpyNode1D(&w.node, recording->graph, nullptr, 0, dst, src, bytes, cudaMemcpyDeviceToDevice);
+  } else {
+    cudaMemsetParams m = {};
+    m.dst = dst;
+    m.elementSize = 1;
+    m.width = bytes;
+    m.height = 1;
+    e = cudaGraphAddMemsetNode(&w.node, recording->graph, nullptr, 0, &m);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return record_append(w, false);
+}
+
+// Enqueues the recorded work piece by piece.
+void run_recorded(const Recording &rec) {
+  const cudaStream_t s = rt().stream;
+  for (const Work &w : rec.work) {
+    if (w.dst && w.src) {
+      OCC_CUDA(cudaMemcpyAsync(w.dst, w.src, w.bytes, cudaMemcpyDeviceToDevice, s));
+    } else if (w.dst) {
+      OCC_CUDA(cudaMemsetAsync(w.dst, 0, w.bytes, s));
+    } else {
+      cudaKernelNodeParams p = {};
+      cudaLaunchAttribute cluster = {};
+      cluster.id = cudaLaunchAttributeClusterDimension;
+      OCC_CUDA(cudaGraphKernelNodeGetParams(w.node, &p));
+      OCC_CUDA(cudaGraphKernelNodeGetAttribute(w.node, cluster.id, &cluster.val));
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = p.gridDim;
+      cfg.blockDim = p.blockDim;
+      cfg.dynamicSmemBytes = p.sharedMemBytes;
+      cfg.stream = s;
+      cfg.attrs = &cluster;
+      cfg.numAttrs = cluster.val.clusterDim.x > 1 ? 1 : 0;
+      OCC_CUDA(cudaLaunchKernelExC(&cfg, p.func, p.kernelParams));
+    }
+  }
+}
+
+// Ends the recording.  The executable graph, or null when it is empty; false when there is none for another reason.
+// With `enqueue` what was recorded is enqueued, either way.
+bool record_end(cudaGraphExec_t *exec, bool enqueue) {
+  std::unique_ptr<Recording> rec(recording);
+  recording = nullptr;
+  *exec = nullptr;
+  bool ok = true;
+  if (!rec->work.empty()) {
+    ok = cudaGraphInstantiate(exec, rec->graph, 0) == cudaSuccess &&
+         (!enqueue || cudaGraphLaunch(*exec, rt().stream) == cudaSuccess);
+    if (!ok) {
+      cudaGetLastError();
+      if (*exec) cudaGraphExecDestroy(*exec);
+      *exec = nullptr;
+      if (enqueue) run_recorded(*rec);
+    }
+  }
+  cudaGraphDestroy(rec->graph);
+  return ok;
+}
+
 bool begin_segment() {
   Runtime &r = rt();
   memcpy(gr.base_counters, r.counters, sizeof(gr.base_counters));
   gr.base_copies = r.main_copies;
   gr.base_chains = trace_fused_chains();
-  // relaxed: other threads and libraries of the process go on allocating meanwhile
-  const cudaError_t e = cudaStreamBeginCapture(r.stream, cudaStreamCaptureModeRelaxed);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
+  if (!record_begin()) return false;
   gr.state = CAPTURING;
   return true;
 }
 
-// Ends the capture and launches what it holds.  The executable graph, or null when it is empty.
 bool end_segment(cudaGraphExec_t *exec) {
-  Runtime &r = rt();
-  *exec = nullptr;
   gr.state = PLAIN;
-  cudaGraph_t g = nullptr;
-  cudaError_t e = cudaStreamEndCapture(r.stream, &g);
-  size_t nodes = 0;
-  if (e == cudaSuccess && g) e = cudaGraphGetNodes(g, nullptr, &nodes);
-  if (e == cudaSuccess && nodes) e = cudaGraphInstantiate(exec, g, 0);
-  if (e == cudaSuccess && *exec) e = cudaGraphLaunch(*exec, r.stream);
-  if (g) cudaGraphDestroy(g);
-  if (e != cudaSuccess) {
-    set_error((int)e, "capture of a recorded inference");
-    return false;
-  }
-  return true;
+  return record_end(exec, true);
 }
 
 void add_variant(GraphPlan &plan, std::unique_ptr<Variant> v) {
@@ -515,20 +634,15 @@ void build_pieces(TraceProgram &p, const Variant &v) {
   for (int k = 0; k < MAX_PIECES && ok; at += images[k++]) {
     Cut piece = c;
     piece.out = 0;
-    ok = cut_up(p, images[k], piece) && cudaStreamSynchronize(r.stream) == cudaSuccess &&
-         cudaStreamBeginCapture(r.stream, cudaStreamCaptureModeRelaxed) == cudaSuccess;
+    ok = cut_up(p, images[k], piece) && record_begin();
     if (!ok) break;
     fresh();
     memcpy(gr.base_counters, r.counters, sizeof(gr.base_counters));
     const int64_t copies0 = r.main_copies, chains0 = trace_fused_chains();
     make_piece(p, piece, at, images[k], hosts);
     if (k + 1 == MAX_PIECES)
-      OCC_CUDA(cudaMemcpyAsync((void *)(c.out - p.pool_base + v.pool_base), (void *)(mine + p.pool_bytes),
-                               (size_t)c.out_bytes, cudaMemcpyDeviceToDevice, r.stream));
-    cudaGraph_t g = nullptr;
-    ok = cudaStreamEndCapture(r.stream, &g) == cudaSuccess && g &&
-         cudaGraphInstantiate(&s.pieces[k], g, 0) == cudaSuccess;
-    if (g) cudaGraphDestroy(g);
+      enqueue_copy((void *)(c.out - p.pool_base + v.pool_base), (void *)(mine + p.pool_bytes), (size_t)c.out_bytes, r.stream);
+    ok = record_end(&s.pieces[k], false) && s.pieces[k];
     for (int i = 0; i < 8; ++i) s.counters[i] += r.counters[i] - gr.base_counters[i];
     s.copies += r.main_copies - copies0;
     s.chains += trace_fused_chains() - chains0;
@@ -636,6 +750,30 @@ void start_window() {
 }
 
 }  // namespace
+
+void enqueue_kernel(const void *kernel, const cudaLaunchConfig_t &cfg, void **args) {
+  if (recording && cfg.stream == rt().stream) {
+    if (record_kernel(kernel, cfg, args)) return;
+    graph_stop_capture();
+  }
+  cudaLaunchKernelExC(&cfg, kernel, args);
+}
+
+void enqueue_copy(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+  if (recording && s == rt().stream) {
+    if (record_copy(dst, src, bytes)) return;
+    graph_stop_capture();
+  }
+  OCC_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, s));
+}
+
+void enqueue_zero(void *dst, size_t bytes, cudaStream_t s) {
+  if (recording && s == rt().stream) {
+    if (record_copy(dst, nullptr, bytes)) return;
+    graph_stop_capture();
+  }
+  OCC_CUDA(cudaMemsetAsync(dst, 0, bytes, s));
+}
 
 GraphPlan::~GraphPlan() {
   for (auto &v : variants)

@@ -716,8 +716,8 @@ __global__ void pack_bias3_kernel(const float *__restrict__ b, uint16_t *__restr
   }
 }
 void launch_pack_bias3(const float *b, bf16 *out, int E, bool f16, cudaStream_t s) {
-  if (f16) pack_bias3_kernel<true><<<(E + 127) / 128, 128, 0, s>>>(b, (uint16_t *)out, E);
-  else pack_bias3_kernel<false><<<(E + 127) / 128, 128, 0, s>>>(b, (uint16_t *)out, E);
+  if (f16) launch_apart(pack_bias3_kernel<true>, (E + 127) / 128, 128, s, b, (uint16_t *)out, E);
+  else launch_apart(pack_bias3_kernel<false>, (E + 127) / 128, 128, s, b, (uint16_t *)out, E);
   count(CNT_LAUNCHES);
 }
 
@@ -729,7 +729,7 @@ __global__ void pack_ir_half_kernel(const float *__restrict__ w, uint16_t *__res
   out[i] = (uint16_t)(ir_cvt<true>(w[e * T + t], 0.0f) & 0xffffu);
 }
 void launch_pack_ir_half(const float *w, void *out, int E, int T, cudaStream_t s) {
-  pack_ir_half_kernel<<<(T * E + 255) / 256, 256, 0, s>>>(w, (uint16_t *)out, E, T);
+  launch_apart(pack_ir_half_kernel, (T * E + 255) / 256, 256, s, w, (uint16_t *)out, E, T);
   count(CNT_LAUNCHES);
 }
 

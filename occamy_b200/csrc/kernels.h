@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <tuple>
 
 namespace occ {
 
@@ -19,8 +20,14 @@ __device__ __forceinline__ void chain_begin() {
   chain_next();
   chain_wait();
 }
-template <typename... P, typename... A>
-inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+// What an inference enqueues goes through these: while its calls are being recorded as a graph, work for the
+// launch stream becomes nodes of that graph (graph_replay.cu).
+void enqueue_kernel(const void *kernel, const cudaLaunchConfig_t &cfg, void **args);
+void enqueue_copy(void *dst, const void *src, size_t bytes, cudaStream_t s);   // device to device
+void enqueue_zero(void *dst, size_t bytes, cudaStream_t s);
+
+template <bool CHAINED, typename... P, typename... A>
+inline void launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -30,8 +37,23 @@ inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t s
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  cfg.numAttrs = CHAINED ? 1 : 0;
+  std::tuple<P...> values{static_cast<P>(args)...};
+  std::apply(
+      [&](auto &...v) {
+        void *ptrs[] = {const_cast<void *>(static_cast<const void *>(&v))...};
+        enqueue_kernel((const void *)kernel, cfg, ptrs);
+      },
+      values);
+}
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  launch_kernel<true>(kernel, grid, block, smem, s, args...);
+}
+// A kernel without chain_begin(): packing, once per constant.
+template <typename... P, typename... A>
+inline void launch_apart(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args) {
+  launch_kernel<false>(kernel, grid, block, 0, s, args...);
 }
 
 // Activation codes shared by host and device (cuDNN's numbering, which is what crosses

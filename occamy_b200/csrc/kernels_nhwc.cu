@@ -1155,9 +1155,9 @@ void launch_pack_krsc_bf16(const float *w, bf16 *out, int K, int C, int R, int S
   const int64_t total = (int64_t)K * Cp * R * S;
   if (total == 0) return;
   if (f16)
-    pack_krsc_kernel<true><<<grid_for(total, 256), 256, 0, s>>>(w, (uint16_t *)out, K, C, Cp, R * S, total);
+    launch_apart(pack_krsc_kernel<true>, grid_for(total, 256), 256, s, w, (uint16_t *)out, K, C, Cp, R * S, total);
   else
-    pack_krsc_kernel<false><<<grid_for(total, 256), 256, 0, s>>>(w, (uint16_t *)out, K, C, Cp, R * S, total);
+    launch_apart(pack_krsc_kernel<false>, grid_for(total, 256), 256, s, w, (uint16_t *)out, K, C, Cp, R * S, total);
   count(CNT_LAUNCHES);
 }
 
@@ -1207,7 +1207,7 @@ __global__ void pack_dw_kernel(const float *__restrict__ w, float *__restrict__ 
 void launch_pack_dw_f32(const float *w, float *out, int C, int R, int S, cudaStream_t s) {
   const int64_t total = (int64_t)C * R * S;
   if (total == 0) return;
-  pack_dw_kernel<<<grid_for(total, 256), 256, 0, s>>>(w, out, C, R * S, total);
+  launch_apart(pack_dw_kernel, grid_for(total, 256), 256, s, w, out, C, R * S, total);
   count(CNT_LAUNCHES);
 }
 
@@ -1234,9 +1234,9 @@ void launch_pack_fold_bf16(const float *w, bf16 *out, int K, int C, int R, int S
   const int64_t total = (int64_t)R * K * Sp * Cp;
   if (total == 0) return;
   if (f16)
-    pack_fold_kernel<true><<<grid_for(total, 256), 256, 0, s>>>(w, (uint16_t *)out, K, C, R, S, Sp, Cp, total);
+    launch_apart(pack_fold_kernel<true>, grid_for(total, 256), 256, s, w, (uint16_t *)out, K, C, R, S, Sp, Cp, total);
   else
-    pack_fold_kernel<false><<<grid_for(total, 256), 256, 0, s>>>(w, (uint16_t *)out, K, C, R, S, Sp, Cp, total);
+    launch_apart(pack_fold_kernel<false>, grid_for(total, 256), 256, s, w, (uint16_t *)out, K, C, R, S, Sp, Cp, total);
   count(CNT_LAUNCHES);
 }
 

@@ -284,7 +284,7 @@ __global__ void pack_split3_kernel(const float *__restrict__ w, uint16_t *__rest
 void launch_pack_split3(const float *w, bf16 *out, int K, int C, int R, int S, int Sp, int Cp, cudaStream_t s) {
   const int64_t total = (int64_t)K * R * (Sp ? Sp : S) * Cp;
   if (total == 0) return;
-  pack_split3_kernel<<<grid_for(total, 256), 256, 0, s>>>(w, (uint16_t *)out, K, C, R, S, Sp, Cp, total);
+  launch_apart(pack_split3_kernel, grid_for(total, 256), 256, s, w, (uint16_t *)out, K, C, R, S, Sp, Cp, total);
   count(CNT_LAUNCHES);
 }
 

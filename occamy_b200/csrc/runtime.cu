@@ -213,7 +213,7 @@ void ensure_f32(const void *p) {
   if (rec->fmt == FMT_ELIDED) {
     set_error(990, "read of a tensor that cross-call fusion skipped (set OCCAMY_FUSE_ACROSS_CALLS=0)");
   } else if (rec->fmt == FMT_ZERO) {
-    OCC_CUDA(cudaMemsetAsync((void *)base, 0, rec->bytes, r.stream));
+    enqueue_zero((void *)base, rec->bytes, r.stream);
     r.main_copies++;
   } else if (rec->fmt == FMT_PENDING) {
     graph_stop_capture();
@@ -223,7 +223,7 @@ void ensure_f32(const void *p) {
     count(CNT_H2D_BYTES, (int64_t)rec->host_bytes);
   } else if (rec->dev_src) {
     graph_stop_capture();   // the caller's memory, elsewhere in the next inference
-    OCC_CUDA(cudaMemcpyAsync((void *)base, rec->dev_src, (size_t)(rec->n * rec->c * rec->h * rec->w) * 4, cudaMemcpyDeviceToDevice, r.stream));
+    enqueue_copy((void *)base, rec->dev_src, (size_t)(rec->n * rec->c * rec->h * rec->w) * 4, r.stream);
     r.main_copies++;
     rec->home = rec->dev_src = nullptr;
   } else if (fmt_is_16(rec->fmt)) {
@@ -231,7 +231,7 @@ void ensure_f32(const void *p) {
     if (!tmp) {
       const size_t elems = (size_t)(rec->n * rec->c * rec->h * rec->w);
       void *copy = scratch_get(3, elems * 2);
-      OCC_CUDA(cudaMemcpyAsync(copy, (void *)base, elems * 2, cudaMemcpyDeviceToDevice, r.stream));
+      enqueue_copy(copy, (void *)base, elems * 2, r.stream);
       tmp = copy;
     }
     rec->home = nullptr;

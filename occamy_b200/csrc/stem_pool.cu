@@ -466,7 +466,7 @@ size_t stem_pool_weight_bytes(int R, int Cf) { return (size_t)R * Cf * ST_K * 2;
 void launch_pack_stem_bf16(const float *w, bf16 *out, int C, int R, int S, int Cp, int Cf,
                            cudaStream_t s) {
   const int total = R * Cf * ST_K;
-  pack_stem_kernel<<<(total + 255) / 256, 256, 0, s>>>(w, out, C, R, S, Cp, Cf, total);
+  launch_apart(pack_stem_kernel, (total + 255) / 256, 256, s, w, out, C, R, S, Cp, Cf, total);
   count(CNT_LAUNCHES);
 }
 

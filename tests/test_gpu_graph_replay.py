@@ -1,6 +1,7 @@
 """Recorded inferences that run as CUDA graphs: same bits as call by call, and every way out of one
 (another constant, another continuation, a wait or the end in the middle)."""
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -235,4 +236,24 @@ def test_device_input_in_convolution_form(native_libs, c):
             assert max_rel_err(y, ref.conv2d(x, w, b, (1, 1))) <= 2e-2
         else:
             assert np.array_equal(y, np.maximum(x, 0))
+    assert rt.last_error() == 0
+
+
+def test_wait_for_the_device_while_recording(native_libs):
+    """A wait for the device, of whatever thread, neither fails nor costs a result while a graph is put together."""
+    rt.set_math_mode(rt.MATH_BF16)
+    m = _HandModel(layers=23)
+    (want,) = m.run()
+
+    def wait():
+        t = threading.Thread(target=torch.cuda.synchronize)
+        t.start()
+        t.join()
+        torch.cuda.synchronize()
+    for i in (2, 15, 22):
+        rt.lib().occamy_set_cross_call_fusion(0)   # forgets what was recorded
+        rt.lib().occamy_set_cross_call_fusion(1)
+        for _ in range(PASSES):
+            (y,) = m.run(between=(i, wait))
+            assert np.array_equal(y, want)
     assert rt.last_error() == 0
