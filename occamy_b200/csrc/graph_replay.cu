@@ -33,9 +33,21 @@ struct SavedRec {
 // arrive and 3.1 to compute).
 constexpr int MAX_PIECES = 3;
 
+// An executable graph.  One that goes out of use may still be running: it is destroyed later (empty_trash()).
+struct Exec {
+  cudaGraphExec_t e = nullptr;
+  Exec() {}
+  Exec(Exec &&o) : e(o.e) { o.e = nullptr; }
+  Exec &operator=(Exec &&o) {
+    std::swap(e, o.e);
+    return *this;
+  }
+  ~Exec();
+};
+
 struct Segment {
-  cudaGraphExec_t exec = nullptr;   // null: the calls enqueue nothing
-  cudaGraphExec_t pieces[MAX_PIECES] = {};   // instead of exec, in a window cut up by images
+  Exec exec;                        // null: the calls enqueue nothing
+  Exec pieces[MAX_PIECES];          // instead of exec, in a window cut up by images
   size_t end = 0;                   // one past its last call
   std::vector<SavedRec> after;      // registry records of the pool when it has been enqueued
   int64_t counters[8] = {};         // what its calls count
@@ -66,7 +78,6 @@ struct GraphPlan {
   int failures = 0;
   int piece_failures = 0;
   std::vector<std::unique_ptr<Variant>> variants;
-  ~GraphPlan();
 };
 
 namespace {
@@ -98,6 +109,10 @@ struct Replay {
   size_t piece_bytes = 0;
 };
 Replay &gr = *new Replay;   // never destroyed, like the programs it refers to
+
+Exec::~Exec() {
+  if (e) gr.trash.push_back(e);
+}
 
 bool computes(int sym) { return sym >= S_CONV && sym <= S_RESHAPE; }
 
@@ -342,7 +357,7 @@ void close_segment(GraphPlan &plan) {
   s.copies = r.main_copies - gr.base_copies;
   s.chains = trace_fused_chains() - gr.base_chains;
   save_registry(s.after, trace_pool_base(), trace_pool_bytes());
-  if (!end_segment(&s.exec)) {
+  if (!end_segment(&s.exec.e)) {
     plan.failures = MAX_FAILURES;
     gr.building.reset();
     return;
@@ -642,7 +657,7 @@ void build_pieces(TraceProgram &p, const Variant &v) {
     make_piece(p, piece, at, images[k], hosts);
     if (k + 1 == MAX_PIECES)
       enqueue_copy((void *)(c.out - p.pool_base + v.pool_base), (void *)(mine + p.pool_bytes), (size_t)c.out_bytes, r.stream);
-    ok = record_end(&s.pieces[k], false) && s.pieces[k];
+    ok = record_end(&s.pieces[k].e, false) && s.pieces[k].e;
     for (int i = 0; i < 8; ++i) s.counters[i] += r.counters[i] - gr.base_counters[i];
     s.copies += r.main_copies - copies0;
     s.chains += trace_fused_chains() - chains0;
@@ -653,11 +668,7 @@ void build_pieces(TraceProgram &p, const Variant &v) {
   restore_registry(v.segments.back().after, v.pool_base, trace_pool_bytes());
   memcpy(r.counters, counters, sizeof(counters));
   r.main_copies = copies;
-  if (!ok || epoch != gr.epoch) {
-    for (cudaGraphExec_t e : s.pieces)
-      if (e) gr.trash.push_back(e);
-    return;
-  }
+  if (!ok || epoch != gr.epoch) return;
   // of the pool's tensors the result alone is there afterwards
   for (const SavedRec &o : v.segments.back().after) {
     SavedRec rec = o;
@@ -682,12 +693,12 @@ void launch_segment() {
   if (v.pieces) {
     for (int i = 0; i < MAX_PIECES; ++i) {
       if (i < gr.pieces_coming) OCC_CUDA(cudaStreamWaitEvent(r.stream, gr.piece_here[i], 0));
-      OCC_CUDA(cudaGraphLaunch(s.pieces[i], r.stream));
+      OCC_CUDA(cudaGraphLaunch(s.pieces[i].e, r.stream));
     }
     gr.pieces_coming = 0;
   } else {
     wait_for_upload();
-    if (s.exec) OCC_CUDA(cudaGraphLaunch(s.exec, r.stream));
+    if (s.exec.e) OCC_CUDA(cudaGraphLaunch(s.exec.e, r.stream));
   }
   for (int i = 0; i < 8; ++i) r.counters[i] += s.counters[i];
   r.main_copies += s.copies;
@@ -773,15 +784,6 @@ void enqueue_zero(void *dst, size_t bytes, cudaStream_t s) {
     graph_stop_capture();
   }
   OCC_CUDA(cudaMemsetAsync(dst, 0, bytes, s));
-}
-
-GraphPlan::~GraphPlan() {
-  for (auto &v : variants)
-    for (Segment &s : v->segments) {
-      if (s.exec) gr.trash.push_back(s.exec);
-      for (cudaGraphExec_t e : s.pieces)
-        if (e) gr.trash.push_back(e);
-    }
 }
 
 bool graph_upload_in_pieces(void *dst, const void *src, size_t bytes, cudaStream_t copy_stream) {
@@ -881,11 +883,8 @@ void graph_after_call() {
 static void break_capture() {
   if (gr.state != CAPTURING) return;
   GR_LOG("capture broken off at call %zu\n", trace_index());
-  cudaGraphExec_t e = nullptr;
-  end_segment(&e);
-  if (e) gr.trash.push_back(e);
-  for (Segment &s : gr.building->segments)
-    if (s.exec) gr.trash.push_back(s.exec);
+  Exec launched;
+  end_segment(&launched.e);
   gr.building.reset();
   if (gr.prog && gr.prog->graph) gr.prog->graph->failures++;
 }

@@ -257,3 +257,19 @@ def test_wait_for_the_device_while_recording(native_libs):
             (y,) = m.run(between=(i, wait))
             assert np.array_equal(y, want)
     assert rt.last_error() == 0
+
+
+def test_graphs_out_of_use_are_destroyed(binding):
+    """Weights that change again and again: the graphs that refer to the old ones are given back."""
+    g, p = _model("resnet50", rt.MATH_BF16, 1, batch=1)
+    x = graphs.make_input(g, 1)
+    w = next(a for a in p._keep if a.size > 100000)
+    free = []
+    for i in range(120):
+        w *= 1.0 + 1e-3 * (1 if i % 2 else -1)
+        for _ in range(6):   # one pass notices, the next two are captured (one per pool block)
+            p.run(binding, x)
+        rt.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[39] - free[-1] <= 4 << 20, free[::10]
+    assert rt.last_error() == 0
