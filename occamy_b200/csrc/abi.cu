@@ -680,6 +680,7 @@ void put(Entry &e, std::initializer_list<const void *> ptrs) {
 }
 // appends n values behind the ones already there
 void put(Entry &e, int &at, const int64_t *d, int64_t n) {
+  if (n > 24 - at) e.args.whole = false;
   for (int64_t i = 0; i < n && at < 24; ++i) e.args.v[at++] = d[i];
 }
 void put(Entry &e, int &at, int64_t v) { put(e, at, &v, 1); }

@@ -398,6 +398,7 @@ void look_for_window(const std::vector<Entry> &calls, TraceProgram &p) {
     const Entry &e = calls[i];
     const Entry &rec = p.entries[i];
     if (computes(e.sym)) {
+      if (!e.args.whole) break;   // could not be made again
       if (!in_pool(rec.in[0], p) || !in_pool(rec.in[1], p) || !in_pool(rec.in[2], p) || !in_pool(rec.out, p)) break;
       end = i + 1;
     } else if (!(e.sym == S_MEMOFFSET || (e.sym == S_H2D && !e.uploaded))) {

@@ -43,6 +43,7 @@ struct CallArgs {
   void *p[4] = {nullptr, nullptr, nullptr, nullptr};
   int64_t v[24] = {};
   float f[2] = {0.f, 0.f};
+  bool whole = true;   // all of them (the dimensions of a call may be more than fit)
 };
 
 struct Entry {

@@ -7,9 +7,11 @@ import numpy as np
 import pytest
 import torch
 
+from calls import Inference, rand
 from helpers import max_rel_err, run_graph_oracle
 from occamy_b200 import graphs, replay
 from occamy_b200 import runtime as rt
+from oracle import ref
 
 pytestmark = pytest.mark.gpu
 
@@ -272,4 +274,29 @@ def test_graphs_out_of_use_are_destroyed(binding):
         rt.synchronize()
         free.append(torch.cuda.mem_get_info()[0])
     assert free[39] - free[-1] <= 4 << 20, free[::10]
+    assert rt.last_error() == 0
+
+
+def test_call_with_many_dimensions(native_libs):
+    """A call with more dimensions than a recorded call keeps, in the middle of an inference that is left early."""
+    rt.set_math_mode(rt.MATH_BF16)
+    shape, w, b = (1, 16, 12, 12), rand(1, 16, 16, 3, 3, scale=0.1), rand(2, 16)
+    x = rand(3, *shape)
+
+    def run(early):
+        with Inference() as f:
+            y, want = f.put(x), x
+            pw, pb = f.put(w), f.put(b)
+            for i in range(6):
+                y, _ = f.conv(y, shape, pw, w.shape, pb, (1, 1), act=1)
+                want = ref.conv2d(want, w, b, (1, 1), act=1)
+                if i == 2:
+                    z = f.place(x.nbytes)
+                    f.L.CUDAClipFunc(y, z, rt.dims((1,) * 24 + (16, 144)), 0.0, 1.0, 26)
+                    y, want = z, np.clip(want, 0.0, 1.0)
+                if early and i == 4:
+                    break
+            return max_rel_err(f.get(y, shape), want)
+    for early in [False] * PASSES + [True, False] * 4:
+        assert run(early) <= 2e-2
     assert rt.last_error() == 0
