@@ -900,6 +900,7 @@ void graph_before_upload() { break_capture(); }
 void graph_settle() {
   if (gr.state == REPLAYING) take_back();
   else break_capture();
+  wait_for_upload();   // it is among the calls made so far
 }
 
 void graph_forget_all() {

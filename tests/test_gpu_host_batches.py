@@ -4,8 +4,11 @@ import numpy as np
 import pytest
 import torch
 
+from calls import Inference, rand
+from helpers import max_rel_err
 from occamy_b200 import graphs, replay
 from occamy_b200 import runtime as rt
+from oracle import ref
 
 pytestmark = pytest.mark.gpu
 
@@ -45,4 +48,44 @@ def test_batches(binding, N, size, math, fuse):
         rt.synchronize()
         want = want.cpu().numpy()
         assert np.abs(got - want).max() <= {rt.MATH_FP32: 2e-5, rt.MATH_F16: 1e-3}.get(math, 8e-3) * np.abs(want).max()
+    assert rt.last_error() == 0
+
+
+def small_model(N, K=40):
+    w, b, fc = rand(1, 16, 16, 3, 3, scale=0.1), rand(2, 16), rand(3, K, 16, scale=0.3)
+
+    def run(x, between=None, mid=False):
+        """x -> convolution, ReLU -> mean -> product; `between` the upload and the rest."""
+        with Inference(8 * x.nbytes) as f:
+            p = f.put(x)
+            if between is not None:
+                between()
+            y, o = f.conv(p, x.shape, f.put(w), w.shape, f.put(b), (1, 1), act=1)
+            m = f.place(N * 16 * 4)
+            f.L.DNNReduceFunc(f.h, 4, y, rt.dims(o), m, rt.dims((N, 16, 1, 1)), 5)
+            z, o = f.matmul(m, (N, 16), f.put(fc), fc.shape)
+            return [f.get(z, o)] + ([f.get(m, (N, 16))] if mid else [])
+
+    def want(x):
+        m = ref.conv2d(x, w, b, (1, 1), act=1).mean((2, 3))
+        return [m @ fc.T, m]
+    return run, want
+
+
+def test_wait_behind_the_upload(native_libs):
+    """A wait right behind the upload is one for the upload: the host buffer may be used for something else then."""
+    rt.set_math_mode(rt.MATH_BF16)
+    N = 128
+    run, want = small_model(N)
+    xs = [rand(10 + i, N, 16, 96, 96) for i in range(2)]
+    wants = [want(x)[0] for x in xs]
+    buf = torch.empty(xs[0].shape).pin_memory().numpy()
+
+    def refill():
+        rt.synchronize()
+        buf[-8:] = 0   # what is copied last
+    for i in range(PASSES + 6):
+        buf[...] = xs[i % 2]
+        (got,) = run(buf, refill if i >= PASSES else None)
+        assert max_rel_err(got, wants[i % 2]) <= 2e-2, i
     assert rt.last_error() == 0
