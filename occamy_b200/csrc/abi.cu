@@ -1862,6 +1862,12 @@ void occamy_get_counters(int64_t out[8]) {
   for (int i = 0; i < 8; ++i) out[i] = r.counters[i];
 }
 
+int occamy_get_form_counters(int64_t *out, int n) {
+  constexpr int FORMS = CNT_COUNT - CNT_SPLIT_REDUCTION;
+  for (int i = 0; i < n && i < FORMS; ++i) out[i] = rt().counters[CNT_SPLIT_REDUCTION + i];
+  return FORMS;
+}
+
 int64_t occamy_fused_chains(void) { return trace_fused_chains(); }
 void occamy_clear_weight_cache(void);
 

@@ -1102,6 +1102,9 @@ void launch_tc_conv(const TcConvArgs &a, cudaStream_t s) {
   OCC_CUDA(cudaGetLastError());
   count(CNT_LAUNCHES);
   count(CNT_TC_LAUNCHES);
+  if (pl.sk) count(CNT_SPLIT_REDUCTION);
+  else if (pl.p.halo) count(CNT_COLUMN_STRIPS);
+  if (a.pool2) count(CNT_POOLED);
 }
 
 // Launch without touching the runtime's state or any cache: the plan (tensor maps) is

@@ -50,7 +50,7 @@ struct Segment {
   Exec pieces[MAX_PIECES];          // instead of exec, in a window cut up by images
   size_t end = 0;                   // one past its last call
   std::vector<SavedRec> after;      // registry records of the pool when it has been enqueued
-  int64_t counters[8] = {};         // what its calls count
+  int64_t counters[CNT_COUNT] = {};   // what its calls count
   int64_t copies = 0, chains = 0;
 };
 
@@ -99,7 +99,7 @@ struct Replay {
   std::vector<const void *> hosts;    // sources of this inference's constants, per call of the window
   // capturing
   std::unique_ptr<Variant> building;
-  int64_t base_counters[8] = {};
+  int64_t base_counters[CNT_COUNT] = {};
   int64_t base_copies = 0, base_chains = 0;
   std::vector<cudaGraphExec_t> trash;   // launched once, destroyed when the stream is idle
   // an upload that is being made in pieces, and the event behind each
@@ -192,6 +192,7 @@ struct Recording {
   std::vector<Work> work;
 };
 Recording *recording = nullptr;
+bool spoiled = false;   // a piece's recording met work that has to be done at once, and was dropped
 
 bool record_begin() {
   std::unique_ptr<Recording> rec(new Recording);
@@ -352,7 +353,7 @@ void close_segment(GraphPlan &plan) {
   const bool last = s.end == plan.end;
   if (last) flush_held_back();
   if (gr.state != CAPTURING) return;   // what was held back needed a new buffer: the capture is broken off
-  for (int i = 0; i < 8; ++i) s.counters[i] = r.counters[i] - gr.base_counters[i];
+  for (int i = 0; i < CNT_COUNT; ++i) s.counters[i] = r.counters[i] - gr.base_counters[i];
   s.counters[CNT_H2D_SKIPPED] = s.counters[CNT_POOL_HWM] = 0;   // counted as the calls are checked
   s.copies = r.main_copies - gr.base_copies;
   s.chains = trace_fused_chains() - gr.base_chains;
@@ -626,15 +627,12 @@ void build_pieces(TraceProgram &p, const Variant &v) {
   }
   const uintptr_t mine = (uintptr_t)gr.piece_memory;
   const std::vector<const void *> hosts = gr.hosts;
-  int64_t counters[8];
+  int64_t counters[CNT_COUNT];
   memcpy(counters, r.counters, sizeof(counters));
   const int64_t copies = r.main_copies;
   auto fresh = [&]() { reg_drop_range((void *)mine, gr.piece_bytes); };
   // the batch's own record covers its place, as it will when the window begins
   restore_registry(v.before, v.pool_base, trace_pool_bytes());
-  // once as they are, the largest piece: buffers are allocated, constants packed
-  fresh();
-  make_piece(p, c, c.batch - images[2], images[2], hosts);
   std::unique_ptr<Variant> n(new Variant);
   n->pool_base = v.pool_base;
   n->flags = v.flags;
@@ -650,16 +648,27 @@ void build_pieces(TraceProgram &p, const Variant &v) {
   for (int k = 0; k < MAX_PIECES && ok; at += images[k++]) {
     Cut piece = c;
     piece.out = 0;
-    ok = cut_up(p, images[k], piece) && record_begin();
+    ok = cut_up(p, images[k], piece);
+    int64_t copies0 = 0, chains0 = 0;
+    // A piece may take kernels, and with them packed constants and buffers, that neither the whole batch nor
+    // another piece takes.  Packing and allocating are done, not recorded: they end the recording, what follows
+    // runs as it comes (on the pieces' own memory), and the piece is recorded anew.
+    for (int attempt = 0; ok && !s.pieces[k].e; ++attempt) {
+      ok = attempt < 3 && record_begin();
+      if (!ok) break;
+      fresh();
+      spoiled = false;
+      memcpy(gr.base_counters, r.counters, sizeof(gr.base_counters));
+      copies0 = r.main_copies;
+      chains0 = trace_fused_chains();
+      make_piece(p, piece, at, images[k], hosts);
+      if (spoiled) continue;
+      if (k + 1 == MAX_PIECES)
+        enqueue_copy((void *)(c.out - p.pool_base + v.pool_base), (void *)(mine + p.pool_bytes), (size_t)c.out_bytes, r.stream);
+      ok = !spoiled && record_end(&s.pieces[k].e, false) && s.pieces[k].e;
+    }
     if (!ok) break;
-    fresh();
-    memcpy(gr.base_counters, r.counters, sizeof(gr.base_counters));
-    const int64_t copies0 = r.main_copies, chains0 = trace_fused_chains();
-    make_piece(p, piece, at, images[k], hosts);
-    if (k + 1 == MAX_PIECES)
-      enqueue_copy((void *)(c.out - p.pool_base + v.pool_base), (void *)(mine + p.pool_bytes), (size_t)c.out_bytes, r.stream);
-    ok = record_end(&s.pieces[k].e, false) && s.pieces[k].e;
-    for (int i = 0; i < 8; ++i) s.counters[i] += r.counters[i] - gr.base_counters[i];
+    for (int i = 0; i < CNT_COUNT; ++i) s.counters[i] += r.counters[i] - gr.base_counters[i];
     s.copies += r.main_copies - copies0;
     s.chains += trace_fused_chains() - chains0;
   }
@@ -701,9 +710,10 @@ void launch_segment() {
     wait_for_upload();
     if (s.exec.e) OCC_CUDA(cudaGraphLaunch(s.exec.e, r.stream));
   }
-  for (int i = 0; i < 8; ++i) r.counters[i] += s.counters[i];
+  for (int i = 0; i < CNT_COUNT; ++i) r.counters[i] += s.counters[i];
   r.main_copies += s.copies;
   for (int64_t i = 0; i < s.chains; ++i) trace_count_chain();
+  if (gr.seg == 0) count(v.pieces ? CNT_IN_PIECES : CNT_REPLAYED);
   if (++gr.seg == v.segments.size()) {   // the window is done: later calls run one by one
     restore_registry(s.after, trace_pool_base(), trace_pool_bytes());
     trace_adopt_prefix(gr.prog, gr.prog->graph->end);
@@ -882,6 +892,13 @@ void graph_after_call() {
 }
 
 static void break_capture() {
+  if (recording && gr.state != CAPTURING) {   // of a piece: none of it is wanted
+    cudaGraphDestroy(recording->graph);
+    delete recording;
+    recording = nullptr;
+    spoiled = true;
+    return;
+  }
   if (gr.state != CAPTURING) return;
   GR_LOG("capture broken off at call %zu\n", trace_index());
   Exec launched;

@@ -962,6 +962,7 @@ bool launch_ir(const IrArgs &a, cudaStream_t s) {
   OCC_CUDA(cudaGetLastError());
   count(CNT_LAUNCHES);
   count(CNT_TC_LAUNCHES);
+  count(CNT_INVERTED_RESIDUAL);
   return true;
 }
 

@@ -79,7 +79,15 @@ enum Counter {
   CNT_TC_LAUNCHES = 4,
   CNT_MATERIALIZE = 5,
   CNT_TMAP_ENCODES = 6,
-  CNT_SIMT_LAUNCHES = 7
+  CNT_SIMT_LAUNCHES = 7,
+  // which forms ran (occamy_get_form_counters)
+  CNT_SPLIT_REDUCTION = 8,
+  CNT_INVERTED_RESIDUAL = 9,
+  CNT_COLUMN_STRIPS = 10,
+  CNT_POOLED = 11,
+  CNT_REPLAYED = 12,
+  CNT_IN_PIECES = 13,
+  CNT_COUNT = 14
 };
 
 struct Runtime {
@@ -88,7 +96,7 @@ struct Runtime {
   int num_sms = 148;
   MathMode mode = MATH_BF16;
   int last_error = 0;
-  int64_t counters[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  int64_t counters[CNT_COUNT] = {};
   int64_t main_copies = 0;  // copies / memsets enqueued on the launch stream (not kernels)
   std::map<uintptr_t, TensorRec> recs;  // keyed by device base pointer
   std::unordered_map<WeightKey, PackedWeight, WeightKeyHash> wcache;

@@ -81,6 +81,7 @@ _SIGNATURES = {
     "occamy_stream": (C.c_void_p, []),
     "occamy_selftest_bounded_wait": (None, []),
     "occamy_get_counters": (None, [_i64p]),
+    "occamy_get_form_counters": (C.c_int, [_i64p, C.c_int]),
     "occamy_clear_weight_cache": (None, []),
     "occamy_set_weight_cache": (None, [C.c_int]),
     "occamy_set_fp32_tensor_cores": (None, [C.c_int]),
@@ -152,6 +153,16 @@ def counters() -> dict:
     out = (C.c_int64 * 8)()
     lib().occamy_get_counters(out)
     return dict(zip(COUNTER_NAMES, [int(v) for v in out]))
+
+
+FORM_NAMES = ("split_reduction", "inverted_residual", "column_strips", "pooled", "replayed", "in_pieces")
+
+
+def form_counters() -> dict:
+    """Which forms the work took since load (see the header)."""
+    out = (C.c_int64 * len(FORM_NAMES))()
+    lib().occamy_get_form_counters(out, len(FORM_NAMES))
+    return dict(zip(FORM_NAMES, [int(v) for v in out]))
 
 
 class DeviceBuffer:

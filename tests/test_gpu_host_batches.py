@@ -89,3 +89,27 @@ def test_wait_behind_the_upload(native_libs):
         (got,) = run(buf, refill if i >= PASSES else None)
         assert max_rel_err(got, wants[i % 2]) <= 2e-2, i
     assert rt.last_error() == 0
+
+
+def test_pieces_need_other_kernels(binding):
+    """MobileNetV2 at batch 160: a piece of 40 images takes a block as one kernel that neither the whole batch nor the
+    other pieces do.  Batches of other sizes share the packed weights in between."""
+    rt.set_math_mode(rt.MATH_F16)
+    rt.lib().occamy_clear_weight_cache()
+    g = graphs.mobilenet_v2(batch=160, seed=1, image=224)
+    programs = {}
+    for n in (160, 40, 2):
+        h = graphs.mobilenet_v2(batch=n, seed=1, image=224)
+        assert list(h.consts) == list(g.consts)
+        h.consts = g.consts   # the same host arrays
+        programs[n] = h.to_program()
+        programs[n].lower(fuse=replay.FUSE_REFERENCE)
+    x = torch.from_numpy(rand(1, *g.input_shape)).pin_memory().numpy()
+    first = {n: p.run(binding, x[:n])[0] for n, p in programs.items()}
+    n0 = rt.form_counters()["in_pieces"]
+    for i in range(10):
+        for n in ((160, 2) if i < 6 else (160, 40, 2)):
+            (got,) = programs[n].run(binding, x[:n])
+            assert max_rel_err(got, first[n]) <= 5e-2, (i, n)
+    assert rt.form_counters()["in_pieces"] > n0
+    assert rt.last_error() == 0
