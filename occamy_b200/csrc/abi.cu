@@ -258,6 +258,9 @@ void stem_geometry(const ConvGeom &g, int &Cp, int &Sp, int &Wp) {
   Wp = (Wp + 7) / 8 * 8;
 }
 
+// TcConvArgs::form_n of a convolution on n images, a product of n rows.
+int form_n(int64_t n) { return form_images(n) == n ? 0 : (int)form_images(n); }
+
 // A dense convolution of the 16-bit path as the kernels are told of it, but for where its operands are;
 // false when they do not take it.  Cp, Sp, Wp: how the input is stored (stem_geometry(), when it is folded).
 bool dense_args(const ConvGeom &g, TcConvArgs &a, int &Cp, int &Sp, int &Wp) {
@@ -265,6 +268,7 @@ bool dense_args(const ConvGeom &g, TcConvArgs &a, int &Cp, int &Sp, int &Wp) {
   if (g.groups != 1 || g.K % 8 != 0) return false;
   if (g.act != ACT_IDENTITY && g.act != ACT_RELU && g.act != ACT_CLIP) return false;
   a.N = g.N; a.K = g.K; a.P = g.P; a.Q = g.Q;
+  a.form_n = form_n(g.N);
   a.act = g.act; a.lo = g.lo; a.hi = g.hi;
   a.f16 = mode_f16() ? 1 : 0;
   Sp = Cp = Wp = 0;
@@ -374,7 +378,7 @@ bool parts_shape_ok(const ConvGeom &g) {
   // Tiny problems stay on the CUDA-core kernel: the passes around this one cost more than it saves.
   return fp32_on_tensor_cores() && g.groups == 1 && g.R * g.S <= 64 && g.stride_h <= 2 && g.stride_w <= 2 &&
          (g.act == ACT_IDENTITY || g.act == ACT_RELU || g.act == ACT_CLIP) &&
-         (double)g.N * g.P * g.Q * g.K * g.C * g.R * g.S >= 1e6;
+         (double)form_images(g.N) * g.P * g.Q * g.K * g.C * g.R * g.S >= 1e6;
 }
 
 bool prepare_parts(const float *x, const float *w, const float *bias, const ConvGeom &g, ConvJob &job) {
@@ -383,6 +387,7 @@ bool prepare_parts(const float *x, const float *w, const float *bias, const Conv
   TcConvArgs &a = job.a;
   memset(&a, 0, sizeof(a));
   a.N = g.N; a.H = g.H; a.K = g.K; a.P = g.P; a.Q = g.Q; a.R = g.R;
+  a.form_n = form_n(g.N);
   a.pad_h = g.pad_h; a.stride_h = g.stride_h;
   a.act = g.act; a.lo = g.lo; a.hi = g.hi;
   a.split = 1;
@@ -567,9 +572,10 @@ bool launch_block(ConvJob &a, ConvJob &b, ConvJob &c) {
   ir.residual = c.a.residual;
   ir.N = g.N; ir.H = a.g.H; ir.W = a.g.W; ir.C = a.g.C; ir.E = a.g.K; ir.K = g.K; ir.P = g.P; ir.Q = g.Q;
   ir.stride = b.g.stride_h;
+  ir.form_n = (int)form_images(g.N);
   ir.f16 = mode_f16();
   ir.consts_ready = a.a.consts_ready && b.a.consts_ready && c.a.consts_ready;
-  if (!ir_supported(ir.N, ir.C, ir.E, ir.K, ir.H, ir.W, ir.P, ir.Q, ir.stride, ir.f16)) return false;
+  if (!ir_supported(ir.form_n, ir.C, ir.E, ir.K, ir.H, ir.W, ir.P, ir.Q, ir.stride, ir.f16)) return false;
   // the output must not land on anything the block reads: tiles read beyond their own pixels
   const uintptr_t olo = (uintptr_t)c.out;
   const size_t obytes = (size_t)g.N * g.K * g.P * g.Q * 2;
@@ -1595,7 +1601,7 @@ float *CUBLASMatmul2dFunc(int64_t /*rank*/, float *A, int64_t dimA[2], float *B,
   const bool out_zero = is_zero(out);
   const bool parts = r.mode == MATH_FP32;
   e.fusable = !transA && transB && alpha == 1.0f && (beta == 0.0f || out_zero) && M > 0 &&
-              (parts ? fp32_on_tensor_cores() && (double)M * N * K >= 1e6 : K % 16 == 0);
+              (parts ? fp32_on_tensor_cores() && (double)form_images(M) * N * K >= 1e6 : K % 16 == 0);
   const Role role = step(e, false);
   if (role == R_SKIP) return out;
   if (r.log) fprintf(stderr, "[occamy] matmul2d M%d N%d K%d tA%d tB%d\n", M, N, K, (int)transA, (int)transB);
@@ -1607,6 +1613,7 @@ float *CUBLASMatmul2dFunc(int64_t /*rank*/, float *A, int64_t dimA[2], float *B,
     a.split = parts ? 1 : 0;
     a.N = 1; a.H = 1; a.W = M; a.Cf = Kp; a.K = N; a.P = 1; a.Q = M; a.R = 1; a.S = 1;
     a.stride_h = a.stride_w = 1;
+    a.form_n = form_n(M);
     a.act = ACT_IDENTITY;
     a.f16 = mode_f16() ? 1 : 0;
     int c = K;   // channels of A where it is an image that a Flatten passed on

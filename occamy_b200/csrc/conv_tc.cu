@@ -575,16 +575,20 @@ static int sk_pick_issuers(const TcConvArgs &a, int bn, int share) {
 // six k-steps of one part product each on the persistent kernel, with results in fp32 between the layers.
 // The fixed part was 0.8 us longer before the epilogue's code was fetched ahead of time, the exchange
 // 0.7 us longer with a cluster barrier behind plain remote stores.
-static SkChoice sk_choose(const TcConvArgs &a, long sp_tiles, int rows, int ksteps, int bk, int a_bytes, int nsm) {
+// `form`: the tile width and number of CTAs are given.
+static SkChoice sk_choose(const TcConvArgs &a, long sp_tiles, int rows, int ksteps, int bk, int a_bytes, int nsm,
+                          const SkChoice *form) {
   SkChoice best{0, 1, 0, -1.0};
   for (int bn = 128; bn >= 32; bn /= 2) {
     if (bn > 32 && bn / 2 >= a.K) continue;   // half as wide would do
+    if (form && bn != form->bn) continue;
 #ifdef OCCAMY_TUNING
     if (const char *f = getenv("OCCAMY_SK_BN")) if (atoi(f) != bn) continue;
 #endif
     const long tiles = sp_tiles * ((a.K + bn - 1) / bn);
     const int stage_bytes = sk_parts(a.split != 0) * (a_bytes + bn * bk * 2);
     for (int s = 1; s <= (a.w_step ? 1 : SK_MAX_SPLITS) && s <= ksteps; ++s) {
+      if (form && s != form->splits) continue;
       // (clusters of more than two leave some SMs of every GPC without a partner)
       long most = s <= 2 ? nsm : nsm - nsm / 9;
 #ifdef OCCAMY_TUNING
@@ -643,7 +647,8 @@ static void pool_box(int Q, int P, int N, int *tw, int *th, int *tn) {
     }
 }
 
-static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, double rival, Plan *pl) {
+static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, double rival, const SkChoice *form,
+                    Plan *pl) {
 #ifdef OCCAMY_TUNING
   const char *force = getenv("OCCAMY_SK");
   if (force && !strcmp(force, "0")) return false;
@@ -667,12 +672,12 @@ static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, d
   p.cblocks = (a.Cf + bk - 1) / bk;
   p.ksteps = a.R * a.S * p.cblocks;
   p.a_bytes = ((p.rows + 7) / 8 * 8 * bk * 2 + 1023) / 1024 * 1024;
-  const SkChoice c = sk_choose(a, sp_tiles, p.rows, p.ksteps, bk, p.a_bytes, nsm);
+  const SkChoice c = sk_choose(a, sp_tiles, p.rows, p.ksteps, bk, p.a_bytes, nsm, form);
   if (c.cost < 0) return false;
 #ifdef OCCAMY_TUNING
   if (!(force && !strcmp(force, "2")))
 #endif
-  if (rival >= 0 && c.cost >= rival) return false;
+  if (!form && rival >= 0 && c.cost >= rival) return false;
   const int bn = c.bn;
   p.stages = c.stages;
   p.splits = c.splits;
@@ -735,8 +740,22 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   Plan pl;
   memset(&pl, 0, sizeof(pl));
   TcParams &p = pl.p;
+  // A piece of a batch: the split-reduction kernel, with the same shares, where the whole batch takes it.  (The
+  // persistent kernels sum up in one order, whatever their tiles.)
+  const bool piece = a.form_n != 0;
+  SkChoice whole{0, 1, 0, -1.0};
+  if (piece) {
+    TcConvArgs w = a;
+    w.form_n = 0;
+    if (a.N > 1) w.N = a.form_n;
+    else w.W = w.Q = a.form_n;   // a plain product's rows (no piece is one image)
+    const Plan of = build_plan(w, err_word, num_sms, false, allow_halo);
+    if (!of.ok) return pl;
+    if (of.sk) whole = SkChoice{of.bn, of.s.splits, 0, 0.0};
+  }
+  const SkChoice *form = whole.bn ? &whole : nullptr;
   if (a.split) {
-    sk_plan(a, err_word, num_sms > 0 ? num_sms : 148, counted, -1.0, &pl);
+    sk_plan(a, err_word, num_sms > 0 ? num_sms : 148, counted, -1.0, form, &pl);
     return pl;
   }
   const int bk = pick_bk(a.Cf);
@@ -860,7 +879,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
     const double waves = (double)((p.total_tiles + per_wave - 1) / per_wave);
     const int ks = p.cblocks * a.R * a.S;
     const double tile_us = halo ? 0.9 : pn ? 0.49 * ks : (bn == 256 ? 0.1 : 0.0) + 0.27 * ks * (bk == 64 ? 1.0 : 0.75);
-    if (!a.pool2 && sk_plan(a, err_word, nsm, counted, 3.1 + waves * tile_us, &pl)) return pl;
+    if (!a.pool2 && (!piece || form) && sk_plan(a, err_word, nsm, counted, 3.1 + waves * tile_us, form, &pl)) return pl;
     if (a.pool2 && !halo && !pair) return pl;   // (not ok: tc_conv_takes_pool() said so)
   }
   const uint32_t boxA[4] = {(uint32_t)bk, (uint32_t)p.tw, (uint32_t)p.th, (uint32_t)p.tn};

@@ -460,7 +460,6 @@ int piece_images(int64_t n, int64_t *images) {
 
 struct Cut {
   std::vector<Entry> calls;    // of the whole inference, those of the window for one piece
-  std::vector<uint8_t> roles;
   uintptr_t x = 0, out = 0;
   int64_t x_bytes = 0, out_bytes = 0, batch = 0;
   size_t x_until = 0, out_from = 0;   // calls between which these addresses mean the input and the result
@@ -569,12 +568,14 @@ bool cut_up(const TraceProgram &p, int64_t images, Cut &c) {
       if (sym != S_MATMUL && sym != S_SOFTMAX && !(sym == S_TENSOR_OP && c.calls[i].kind == CK_ROW_BIAS)) return false;
       break;
     }
-  trace_roles(c.calls, c.roles);
   return true;
 }
 
 // Makes the window's calls for one piece: images [at, at + images) of the batch.
 void make_piece(const TraceProgram &p, const Cut &c, int64_t at, int64_t images, const std::vector<const void *> &hosts) {
+  Runtime &r = rt();
+  r.piece_images = images;
+  r.batch_images = c.batch;
   const uintptr_t real = trace_pool_base(), mine = (uintptr_t)gr.piece_memory;
   const uintptr_t x = c.x - p.pool_base + real + (uintptr_t)(c.x_bytes / c.batch * at);
   const uintptr_t out = mine + p.pool_bytes + (uintptr_t)(c.out_bytes / c.batch * at);
@@ -584,7 +585,7 @@ void make_piece(const TraceProgram &p, const Cut &c, int64_t at, int64_t images,
       reg_new((void *)out, (size_t)(c.out_bytes / c.batch * images), FMT_ZERO);
       continue;
     }
-    trace_force(c.roles[i]);
+    trace_force(p.roles[i]);
     run_again(c.calls[i],
               [&](void *q) -> void * {
                 const uintptr_t a = (uintptr_t)q;
@@ -598,6 +599,7 @@ void make_piece(const TraceProgram &p, const Cut &c, int64_t at, int64_t images,
   trace_force_end();
   flush_held_back();
   gr.again = false;
+  r.piece_images = r.batch_images = 0;
 }
 
 // An inference has just run its window as the graphs of `v`: make the variant that is cut up by images.

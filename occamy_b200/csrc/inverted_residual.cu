@@ -851,7 +851,7 @@ IrPlan ir_build(const IrArgs &a) {
   Runtime &r = rt();
   IrPlan pl;
   memset(&pl, 0, sizeof(pl));
-  pl.c = ir_choose(a.N, a.C, a.E, a.K, a.P, a.Q, a.stride, a.f16 != 0, r.num_sms);
+  pl.c = ir_choose(a.form_n, a.C, a.E, a.K, a.P, a.Q, a.stride, a.f16 != 0, r.num_sms);
   if (pl.c.us < 0) return pl;
   const IrChoice &c = pl.c;
   IrParams &p = pl.p;

@@ -171,6 +171,7 @@ struct TcConvArgs {
   // Filter (and bias) were resident on the device before this call was made, i.e. no work
   // enqueued earlier in the stream produces them.
   int consts_ready;
+  int form_n;            // images (a product: rows) whose form is taken, see form_images(); 0: its own
   int pool2;             // y is the 2x2 / stride 2 max pool of the result (tc_conv_takes_pool())
 };
 // ---- few-channel convolution fused with the 3x3 / stride 2 / pad 1 max pool after it -----
@@ -203,6 +204,7 @@ struct IrArgs {
   const bf16 *residual;         // like y, or null
   bf16 *y;                      // [N][P][Q][K]
   int N, H, W, C, E, K, P, Q, stride;
+  int form_n;                   // images whose form is taken (form_images())
   float floor[3], lo[3], hi[3]; // activation behind each stage: ReLU's 0 (else -inf), a clip's bounds (else NaN)
   int f16, consts_ready;
 };

@@ -957,7 +957,7 @@ bool depthwise_sums_in_half(const ConvGeom &g) {
   return g.R == 3 && g.S == 3 && g.stride_h == g.stride_w && (g.stride_h == 1 || g.stride_h == 2) &&
          (g.act == ACT_IDENTITY || g.act == ACT_RELU || g.act == ACT_CLIP) && (lo == 0.0f || lo == -INFINITY) &&
          (hi == INFINITY || host_elem_value(host_elem_bits(hi, true), true) == hi) && g.pad_w >= 0 && g.pad_w <= 1 &&
-         (int64_t)g.N * g.P * g.Q * (g.C / 8) * 16 < (int64_t)1 << 31;
+         form_images(g.N) * g.P * g.Q * (g.C / 8) * 16 < (int64_t)1 << 31;
 }
 
 void launch_depthwise_bf16(const bf16 *x, const float *w_rsc, const float *bias, bf16 *y,

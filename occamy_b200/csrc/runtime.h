@@ -119,6 +119,8 @@ struct Runtime {
     size_t bytes;
   };
   std::vector<Home> homes;
+  // while a piece of a batch is computed by itself (graph_replay.cu): its images and those of the batch
+  int64_t piece_images = 0, batch_images = 0;
   // optional CUDA-event pair around every tensor-core launch (occamy_profile_begin/end)
   bool profiling = false;
   int prof_count = 0;
@@ -129,6 +131,13 @@ struct Runtime {
 bool fp32_on_tensor_cores();
 
 Runtime &rt();  // lazily initialised on the current device
+
+// Images that decide in which order a result is summed up: a piece of a batch is computed in the forms (kernel, shares
+// of a reduction) that the whole batch takes, so that an image has the same bits either way.
+inline int64_t form_images(int64_t n) {
+  const Runtime &r = rt();
+  return r.piece_images && n == r.piece_images ? r.batch_images : n;
+}
 
 void set_error(int code, const char *where);
 #define OCC_CUDA(call)                                        \

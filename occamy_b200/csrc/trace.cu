@@ -366,10 +366,6 @@ void te_dims(Entry &e, const int64_t *d, int n) {
   for (int i = 0; i < n; ++i) mix(e.sig, (uint64_t)d[i]);
 }
 
-void trace_roles(const std::vector<Entry> &calls, std::vector<uint8_t> &roles) {
-  std::vector<int> reader;
-  analyse(calls, roles, reader);
-}
 void trace_force(uint8_t role) { g_ts.forced = role; }
 void trace_force_end() { g_ts.forced = -1; }
 

@@ -122,13 +122,12 @@ const std::vector<Entry> &trace_entries();
 void trace_adopt_prefix(TraceProgram *p, size_t n);
 // The same, as if they had been made one by one: what follows is recorded and matched anew.
 void trace_rewind(TraceProgram *p, size_t n);
-// The roles `analyse` gives the calls of an inference; and the role of the next call, whatever was recorded
-// (calls made outside an inference's own sequence).
 // (abi.cu) whether the convolution's kernel can take a following CK_POOL_2S2 along; whether it reads its input
 // as a 16-bit tensor
 bool entry_takes_pool(const Entry &e);
 bool entry_reads_16(const Entry &e);
-void trace_roles(const std::vector<Entry> &calls, std::vector<uint8_t> &roles);
+// The role (with its RF_*) of the calls up to trace_force_end(), whatever was recorded: calls made outside an
+// inference's own sequence.
 void trace_force(uint8_t role);
 void trace_force_end();
 uintptr_t trace_pool_base();

@@ -113,3 +113,21 @@ def test_pieces_need_other_kernels(binding):
             assert max_rel_err(got, first[n]) <= 5e-2, (i, n)
     assert rt.form_counters()["in_pieces"] > n0
     assert rt.last_error() == 0
+
+
+@pytest.mark.parametrize("name,math,N,image", [("resnet50", rt.MATH_BF16, 160, 97), ("mobilenet_v2", rt.MATH_F16, 160, 128),
+                                               ("vgg16", rt.MATH_BF16, 136, 112), ("resnet50", rt.MATH_FP32, 128, 112)])
+def test_same_bits_in_pieces(binding, name, math, N, image):
+    """An image's result does not depend on whether its batch was computed in pieces."""
+    rt.set_math_mode(math)
+    g = getattr(graphs, name)(batch=N, seed=1, image=image, **({"softmax": False} if name == "resnet50" else {}))
+    p = g.to_program()
+    p.lower(fuse=replay.FUSE_REFERENCE)
+    x = torch.from_numpy(rand(1, *g.input_shape)).pin_memory().numpy()
+    outs, n0 = [], rt.form_counters()["in_pieces"]
+    while rt.form_counters()["in_pieces"] < n0 + 3:
+        outs.append(p.run(binding, x)[0])
+        assert len(outs) < 24
+    for y in outs[2:]:   # (the first pass runs unfused)
+        assert np.array_equal(y, outs[1])
+    assert rt.last_error() == 0
