@@ -658,6 +658,7 @@ Role step(Entry &e, bool passive) {
   bool deviated = false;
   const Role role = trace_step(e, &deviated);
   if (deviated) {
+    graph_left_recording();
     graph_stop_capture();
     g_pending.out16 = false;   // who reads it is not known any more
     g_pending.out_parts = g_pending.a.split && g_pending.res_set;

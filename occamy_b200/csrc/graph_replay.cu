@@ -60,6 +60,13 @@ struct Constant {
   uint64_t hash;
 };
 
+// What the last graph of a window cut up by images moves: the result to its tensor; and what was there of the
+// batch, which is still needed should the window have to be made call by call after all, out of the way.
+struct ResultCopy {
+  void *tensor = nullptr, *made = nullptr, *aside = nullptr;
+  size_t bytes = 0;
+};
+
 struct Variant {
   uintptr_t pool_base = 0;
   int flags = 0;
@@ -68,6 +75,7 @@ struct Variant {
   std::vector<Constant> constants;
   std::vector<Segment> segments;
   bool pieces = false;            // one segment, cut up by images
+  ResultCopy result;
 };
 
 }  // namespace
@@ -107,6 +115,9 @@ struct Replay {
   cudaEvent_t piece_here[MAX_PIECES] = {};
   void *piece_memory = nullptr;         // where the tensors of a window cut up by images are
   size_t piece_bytes = 0;
+  // this inference ran its window as pieces
+  TraceProgram *in_pieces = nullptr;
+  const Variant *pieces_of = nullptr;
 };
 Replay &gr = *new Replay;   // never destroyed, like the programs it refers to
 
@@ -550,9 +561,11 @@ bool cut_up(const TraceProgram &p, int64_t images, Cut &c) {
     if (second_scaled) e.in_bytes[1] = e.in_bytes[1] / N * images;
     if (e.sym == S_MATMUL && e.in[2]) e.in_bytes[2] = e.out_bytes;
   }
-  // one tensor is read behind the window: rows of fp32
+  // behind the window one tensor is read, rows of fp32, and nothing else happens (graph_left_recording())
   for (size_t i = end; i < c.calls.size(); ++i) {
     const Entry &e = c.calls[i];
+    const bool to_pool = e.out >= p.pool_base && e.out < p.pool_base + p.pool_bytes;
+    if (e.sym != S_D2H && e.sym != S_POOLFREE && !(e.sym == S_D2D && !to_pool)) return false;
     for (int k = 0; k < 3; ++k) {
       if (!e.in[k] || e.in[k] < p.pool_base || e.in[k] >= p.pool_base + p.pool_bytes) continue;
       if ((c.out && e.in[k] != c.out) || !batch.count(e.in[k]) || e.in_bytes[k] != batch[e.in[k]]) return false;
@@ -578,7 +591,7 @@ void make_piece(const TraceProgram &p, const Cut &c, int64_t at, int64_t images,
   r.batch_images = c.batch;
   const uintptr_t real = trace_pool_base(), mine = (uintptr_t)gr.piece_memory;
   const uintptr_t x = c.x - p.pool_base + real + (uintptr_t)(c.x_bytes / c.batch * at);
-  const uintptr_t out = mine + p.pool_bytes + (uintptr_t)(c.out_bytes / c.batch * at);
+  const uintptr_t out = mine + ((p.pool_bytes + 255) & ~(size_t)255) + (uintptr_t)(c.out_bytes / c.batch * at);
   gr.again = true;
   for (size_t i = p.graph->begin; i < p.graph->end; ++i) {
     if (i == c.out_from) {
@@ -616,7 +629,7 @@ void build_pieces(TraceProgram &p, const Variant &v) {
   }
   Runtime &r = rt();
   plan.piece_failures++;   // taken back below
-  const size_t bytes = p.pool_bytes + (size_t)c.out_bytes;
+  const size_t tensors = (p.pool_bytes + 255) & ~(size_t)255, bytes = tensors + 2 * (((size_t)c.out_bytes + 255) & ~(size_t)255);
   if (gr.piece_bytes < bytes) {
     graph_free_memory();
     if (cudaMalloc(&gr.piece_memory, bytes) != cudaSuccess) {
@@ -642,6 +655,11 @@ void build_pieces(TraceProgram &p, const Variant &v) {
   n->constants = v.constants;
   n->pieces = true;
   n->segments.resize(1);
+  const size_t result_room = ((size_t)c.out_bytes + 255) & ~(size_t)255;
+  n->result.tensor = (void *)(c.out - p.pool_base + v.pool_base);
+  n->result.made = (void *)(mine + tensors);
+  n->result.aside = (void *)(mine + tensors + result_room);
+  n->result.bytes = (size_t)c.out_bytes;
   Segment &s = n->segments[0];
   s.end = plan.end;
   bool ok = true;
@@ -665,8 +683,10 @@ void build_pieces(TraceProgram &p, const Variant &v) {
       chains0 = trace_fused_chains();
       make_piece(p, piece, at, images[k], hosts);
       if (spoiled) continue;
-      if (k + 1 == MAX_PIECES)
-        enqueue_copy((void *)(c.out - p.pool_base + v.pool_base), (void *)(mine + p.pool_bytes), (size_t)c.out_bytes, r.stream);
+      if (k + 1 == MAX_PIECES) {
+        enqueue_copy(n->result.aside, n->result.tensor, n->result.bytes, r.stream);
+        enqueue_copy(n->result.tensor, n->result.made, n->result.bytes, r.stream);
+      }
       ok = !spoiled && record_end(&s.pieces[k].e, false) && s.pieces[k].e;
     }
     if (!ok) break;
@@ -722,7 +742,12 @@ void launch_segment() {
     v.used = ++gr.tick;
     gr.state = PLAIN;
     gr.left.clear();
-    if (!v.pieces) build_pieces(*gr.prog, v);
+    if (v.pieces) {
+      gr.in_pieces = gr.prog;
+      gr.pieces_of = &v;
+    } else {
+      build_pieces(*gr.prog, v);
+    }
   }
 }
 
@@ -830,6 +855,30 @@ bool graph_upload_in_pieces(void *dst, const void *src, size_t bytes, cudaStream
 
 void graph_uncovered() { wait_for_upload(); }
 
+void graph_left_recording() {
+  TraceProgram *p = gr.in_pieces;
+  if (!p || !trace_pool_base()) return;
+  gr.in_pieces = nullptr;
+  const Variant &v = *gr.pieces_of;
+  const uintptr_t base = trace_pool_base();
+  const std::vector<const void *> hosts = gr.hosts;
+  enqueue_copy(v.result.tensor, v.result.aside, v.result.bytes, rt().stream);
+  restore_registry(v.before, base, trace_pool_bytes());
+  gr.again = true;
+  for (size_t i = p->graph->begin; i < p->graph->end; ++i) {
+    trace_force(p->roles[i]);
+    run_again(p->entries[i],
+              [&](void *q) {
+                const uintptr_t a = (uintptr_t)q;
+                return (void *)(a >= p->pool_base && a < p->pool_base + p->pool_bytes ? a - p->pool_base + base : a);
+              },
+              hosts[i - p->graph->begin]);
+  }
+  trace_force_end();
+  flush_held_back();
+  gr.again = false;
+}
+
 void graph_free_memory() {
   if (!gr.piece_memory) return;
   graph_forget_all();
@@ -933,7 +982,7 @@ void graph_inference_begin() {
   wait_for_upload();
   empty_trash(gr.trash.size() > 64);
   gr.state = IDLE;
-  gr.prog = nullptr;
+  gr.prog = gr.in_pieces = nullptr;
   gr.disturbed = false;
   gr.epoch_at_begin = gr.epoch;
 }
@@ -947,6 +996,7 @@ void graph_inference_end() {
   if (trace_active() && p && trace_has_own_entries() && p->sigs.size() == trace_index() &&
       gr.epoch == gr.epoch_at_begin && !gr.disturbed)
     look_for_window(trace_entries(), *p);
+  gr.in_pieces = nullptr;
   gr.state = PLAIN;
 }
 

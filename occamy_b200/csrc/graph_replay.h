@@ -39,6 +39,9 @@ bool graph_upload_in_pieces(void *dst, const void *src, size_t bytes, cudaStream
 void graph_forget_all();
 // A call is about to be carried out that no graph covers.
 void graph_uncovered();
+// This call is not the recorded one, and may read any tensor: a window computed in pieces, which left nothing but its
+// result, is made call by call.
+void graph_left_recording();
 // Frees what windows cut up by images work in.
 void graph_free_memory();
 // cudnnCreate / cudnnDestroy.

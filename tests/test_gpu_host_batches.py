@@ -131,3 +131,20 @@ def test_same_bits_in_pieces(binding, name, math, N, image):
     for y in outs[2:]:   # (the first pass runs unfused)
         assert np.array_equal(y, outs[1])
     assert rt.last_error() == 0
+
+
+def test_other_tensors_behind_pieces(native_libs):
+    """A program that goes on like the recorded one until its result has been read, and then reads another tensor."""
+    rt.set_math_mode(rt.MATH_BF16)
+    N = 128
+    run, want = small_model(N)
+    x = torch.from_numpy(rand(10, N, 16, 96, 96)).pin_memory().numpy()
+    logits, means = want(x)
+    n0 = rt.form_counters()["in_pieces"]
+    for i, mid in enumerate([False] * (PASSES + 2) + [True, False, True, False, False]):
+        got = run(x, mid=mid)
+        assert max_rel_err(got[0], logits) <= 2e-2, i
+        if mid:
+            assert max_rel_err(got[1], means) <= 2e-2, i
+            assert i > PASSES + 2 or rt.form_counters()["in_pieces"] > n0 + 1
+    assert rt.last_error() == 0
