@@ -474,7 +474,47 @@ struct Cut {
   uintptr_t x = 0, out = 0;
   int64_t x_bytes = 0, out_bytes = 0, batch = 0;
   size_t x_until = 0, out_from = 0;   // calls between which these addresses mean the input and the result
+  std::vector<size_t> offset;         // of the tensor that a call of the window hands out, in the pieces' memory
+  size_t bytes = 0;                   // what these tensors need
 };
+
+// Whether the tensor handed out by call `i` is a constant: the first call that writes it is an upload.
+bool is_constant(const std::vector<Entry> &calls, size_t i, size_t end) {
+  const uintptr_t a = calls[i].out;
+  for (size_t j = i + 1; j < end; ++j) {
+    if (calls[j].sym == S_H2D && calls[j].out == a) return true;
+    if (calls[j].out == a) return false;
+  }
+  return false;
+}
+
+// Places for the window's tensors, as large as a piece needs them: first fit, a tensor's place is free again when the
+// pool hands out what it had there.
+void lay_out(const TraceProgram &p, Cut &c) {
+  struct Live {
+    uintptr_t pool;
+    int64_t pool_bytes;
+    size_t at, bytes;
+  };
+  std::vector<Live> live;   // by place
+  c.offset.assign(p.graph->end - p.graph->begin, 0);
+  c.bytes = 0;
+  for (size_t i = p.graph->begin; i < p.graph->end; ++i) {
+    const Entry &e = p.entries[i];
+    if (e.sym != S_MEMOFFSET) continue;
+    for (size_t k = 0; k < live.size();)
+      if (live[k].pool < e.out + (uintptr_t)e.out_bytes && e.out < live[k].pool + (uintptr_t)live[k].pool_bytes)
+        live.erase(live.begin() + k);
+      else ++k;
+    if (i == c.out_from) continue;
+    const size_t bytes = ((size_t)c.calls[i].out_bytes + 255) & ~(size_t)255;
+    size_t at = 0, k = 0;
+    for (; k < live.size() && live[k].at < at + bytes; ++k) at = live[k].at + live[k].bytes;
+    live.insert(live.begin() + k, Live{e.out, e.out_bytes, at, bytes});
+    c.offset[i - p.graph->begin] = at;
+    if (c.bytes < at + bytes) c.bytes = at + bytes;
+  }
+}
 
 // The call that uploads the batch: the one right before the window.
 bool find_input(const TraceProgram &p, Cut &c) {
@@ -515,6 +555,10 @@ bool cut_up(const TraceProgram &p, int64_t images, Cut &c) {
       handed_out[e.out] = i;
       if (i >= begin && c.x_until == end && !batch.count(c.x)) c.x_until = i;
       if (i < begin && e.out == c.x) batch[c.x] = c.x_bytes;
+      if (i >= begin && !is_constant(p.entries, i, end)) {
+        e.out_bytes = ((e.out_bytes * images + N - 1) / N + 31) / 32 * 32;
+        v[0] = e.out_bytes;
+      }
       continue;
     }
     if (e.sym == S_H2D) {
@@ -531,6 +575,7 @@ bool cut_up(const TraceProgram &p, int64_t images, Cut &c) {
       return true;
     };
     if (!batch.count(e.in[0])) return false;
+    if (!handed_out.count(e.out) || handed_out[e.out] < begin) return false;   // (the batch stays as it is)
     bool ok = true, second_scaled = false;
     switch (e.sym) {
       case S_CONV:
@@ -590,14 +635,16 @@ void make_piece(const TraceProgram &p, const Cut &c, int64_t at, int64_t images,
   r.piece_images = images;
   r.batch_images = c.batch;
   const uintptr_t real = trace_pool_base(), mine = (uintptr_t)gr.piece_memory;
+  std::map<uintptr_t, uintptr_t> where;   // of the window's tensors, by their addresses in the pool
   const uintptr_t x = c.x - p.pool_base + real + (uintptr_t)(c.x_bytes / c.batch * at);
-  const uintptr_t out = mine + ((p.pool_bytes + 255) & ~(size_t)255) + (uintptr_t)(c.out_bytes / c.batch * at);
+  const uintptr_t out = mine + c.bytes + (uintptr_t)(c.out_bytes / c.batch * at);
   gr.again = true;
   for (size_t i = p.graph->begin; i < p.graph->end; ++i) {
     if (i == c.out_from) {
       reg_new((void *)out, (size_t)(c.out_bytes / c.batch * images), FMT_ZERO);
       continue;
     }
+    if (c.calls[i].sym == S_MEMOFFSET) where[c.calls[i].out] = mine + c.offset[i - p.graph->begin];
     trace_force(p.roles[i]);
     run_again(c.calls[i],
               [&](void *q) -> void * {
@@ -605,7 +652,7 @@ void make_piece(const TraceProgram &p, const Cut &c, int64_t at, int64_t images,
                 if (a < p.pool_base || a >= p.pool_base + p.pool_bytes) return q;
                 if (a == c.x && i < c.x_until) return (void *)x;
                 if (a == c.out && i > c.out_from) return (void *)out;
-                return (void *)(a - p.pool_base + mine);
+                return (void *)where[a];
               },
               hosts[i - p.graph->begin]);
   }
@@ -629,7 +676,8 @@ void build_pieces(TraceProgram &p, const Variant &v) {
   }
   Runtime &r = rt();
   plan.piece_failures++;   // taken back below
-  const size_t tensors = (p.pool_bytes + 255) & ~(size_t)255, bytes = tensors + 2 * (((size_t)c.out_bytes + 255) & ~(size_t)255);
+  lay_out(p, c);   // for the largest piece; the result of all of them behind it
+  const size_t result_room = ((size_t)c.out_bytes + 255) & ~(size_t)255, bytes = c.bytes + 2 * result_room;
   if (gr.piece_bytes < bytes) {
     graph_free_memory();
     if (cudaMalloc(&gr.piece_memory, bytes) != cudaSuccess) {
@@ -655,10 +703,9 @@ void build_pieces(TraceProgram &p, const Variant &v) {
   n->constants = v.constants;
   n->pieces = true;
   n->segments.resize(1);
-  const size_t result_room = ((size_t)c.out_bytes + 255) & ~(size_t)255;
   n->result.tensor = (void *)(c.out - p.pool_base + v.pool_base);
-  n->result.made = (void *)(mine + tensors);
-  n->result.aside = (void *)(mine + tensors + result_room);
+  n->result.made = (void *)(mine + c.bytes);
+  n->result.aside = (void *)(mine + c.bytes + result_room);
   n->result.bytes = (size_t)c.out_bytes;
   Segment &s = n->segments[0];
   s.end = plan.end;
