@@ -104,6 +104,7 @@ void *packed_weights(const float *w, int layout, size_t packed_bytes, int K, int
     auto it = r.wcache.find(key);
     if (it != r.wcache.end() && it->second.hash == rec->host_hash && it->second.bytes == packed_bytes) {
       g_pack_was_resident = true;
+      r.resident[key.src] = std::make_pair(key.bytes, it->second.hash);   // (another constant may have been there since)
       return it->second.dev;
     }
   }

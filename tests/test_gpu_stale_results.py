@@ -152,3 +152,23 @@ def test_tensor_outside_the_pool_in_a_buffer_of_the_runtime(binding):
         assert max_rel_err(t.to_numpy(x.shape), want) <= 5e-2, i
         want = t.to_numpy(x.shape)
     assert rt.last_error() == 0
+
+
+def test_constants_at_one_address(native_libs):
+    """A constant whose address was another one's for a while is found again: no upload in every inference."""
+    rt.set_math_mode(rt.MATH_BF16)
+    buf = rand(1, 64, 16, 3, 3, scale=0.1)
+    x = rand(2, 1, 16, 12, 12)
+
+    def run(k):
+        w = buf[:k]   # the same address, another size
+        with Inference() as f:
+            n0 = rt.counters()["h2d_bytes"]
+            y, o = f.conv(f.put(x), x.shape, f.put(w), w.shape, pads=(1, 1))
+            got = f.get(y, o)
+        assert max_rel_err(got, ref.conv2d(x, w, None, (1, 1))) <= 2e-2
+        return rt.counters()["h2d_bytes"] - n0
+    for k in [16] * 3 + [64] * 3 + [16]:
+        run(k)
+    assert [run(16) for _ in range(3)] == [x.nbytes] * 3
+    assert rt.last_error() == 0
