@@ -130,7 +130,7 @@ void *packed_weights(const float *w, int layout, size_t packed_bytes, int K, int
       OCC_CUDA(cudaFree(pw.dev));
       pw.dev = nullptr;
     }
-    if (!pw.dev) OCC_CUDA(cudaMalloc(&pw.dev, packed_bytes));
+    if (!pw.dev) OCC_CUDA(device_malloc(&pw.dev, packed_bytes));
     pw.bytes = packed_bytes;
     pw.hash = rec->host_hash;
     pw.layout = layout;
@@ -905,7 +905,7 @@ extern "C" {
 // ---------------------------------------------------------------- memory pool
 cudaError_t wrapDNNMalloc(void **devPtr, size_t size) {
   rt();
-  cudaError_t err = cudaMalloc(devPtr, size ? size : 1);
+  cudaError_t err = device_malloc(devPtr, size ? size : 1);
   if (err != cudaSuccess) die("Malloc", err, size);
   CallScope scope;
   Entry e = trace_entry(S_MALLOC);
@@ -941,9 +941,8 @@ cudaError_t wrapDNNMemPoolInit(void **devPtr, size_t size) {
       } else {
         ++i;
       }
-    cudaError_t err = cudaMalloc(devPtr, size ? size : 1);
+    cudaError_t err = device_malloc(devPtr, size ? size : 1);
     if (err != cudaSuccess && !g_pool_cache.empty()) {   // no room for a second block
-      cudaGetLastError();
       *devPtr = g_pool_cache[0].base;
       ready = g_pool_cache[0].done;
       g_pool_cache.erase(g_pool_cache.begin());
@@ -1931,16 +1930,7 @@ void occamy_clear_weight_cache(void) {
   r.wcache.clear();
   r.resident.clear();
   graph_free_memory();
-  for (size_t i = 0; i < r.homes.size();) {   // buffers no tensor is in
-    bool used = false;
-    for (const auto &kv : r.recs) used = used || kv.second.home == r.homes[i].ptr;
-    if (used) {
-      ++i;
-      continue;
-    }
-    cudaFree(r.homes[i].ptr);
-    r.homes.erase(r.homes.begin() + i);
-  }
+  free_idle_homes();
 }
 
 }  // extern "C"

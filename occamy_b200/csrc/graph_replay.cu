@@ -115,6 +115,7 @@ struct Replay {
   cudaEvent_t piece_here[MAX_PIECES] = {};
   void *piece_memory = nullptr;         // where the tensors of a window cut up by images are
   size_t piece_bytes = 0;
+  bool making_pieces = false;           // build_pieces() is using it
   // this inference ran its window as pieces
   TraceProgram *in_pieces = nullptr;
   const Variant *pieces_of = nullptr;
@@ -688,6 +689,7 @@ void build_pieces(TraceProgram &p, const Variant &v) {
     }
     gr.piece_bytes = bytes;
   }
+  gr.making_pieces = true;
   const uintptr_t mine = (uintptr_t)gr.piece_memory;
   const std::vector<const void *> hosts = gr.hosts;
   int64_t counters[CNT_COUNT];
@@ -741,6 +743,7 @@ void build_pieces(TraceProgram &p, const Variant &v) {
     s.copies += r.main_copies - copies0;
     s.chains += trace_fused_chains() - chains0;
   }
+  gr.making_pieces = false;
   s.counters[CNT_H2D_SKIPPED] = s.counters[CNT_POOL_HWM] = 0;
   cudaGetLastError();
   reg_drop_range((void *)mine, gr.piece_bytes);
@@ -927,7 +930,7 @@ void graph_left_recording() {
 }
 
 void graph_free_memory() {
-  if (!gr.piece_memory) return;
+  if (!gr.piece_memory || gr.making_pieces) return;
   graph_forget_all();
   OCC_CUDA(cudaStreamSynchronize(rt().stream));
   OCC_CUDA(cudaFree(gr.piece_memory));

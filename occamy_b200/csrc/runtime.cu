@@ -124,18 +124,45 @@ const __nv_bfloat16 *act16_ptr(const void *p) {
   return (const __nv_bfloat16 *)(rec && rec->home ? rec->home : p);
 }
 
+static bool home_in_use(const void *h) {
+  Runtime &r = rt();
+  if (r.home_held && r.home_held(h)) return true;
+  for (const auto &kv : r.recs)
+    if (kv.second.home == h) return true;
+  return false;
+}
+
+void free_idle_homes() {
+  Runtime &r = rt();
+  graph_forget_all();
+  OCC_CUDA(cudaStreamSynchronize(r.stream));
+  for (size_t i = 0; i < r.homes.size();) {
+    if (home_in_use(r.homes[i].ptr)) {
+      ++i;
+      continue;
+    }
+    OCC_CUDA(cudaFree(r.homes[i].ptr));
+    r.homes.erase(r.homes.begin() + i);
+  }
+}
+
+cudaError_t device_malloc(void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  graph_free_memory();
+  free_idle_homes();
+  e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
 void *home_acquire(size_t bytes) {
   Runtime &r = rt();
   constexpr size_t MOST = 6;
-  auto in_use = [&](const void *h) {
-    if (r.home_held && r.home_held(h)) return true;
-    for (const auto &kv : r.recs)
-      if (kv.second.home == h) return true;
-    return false;
-  };
   Runtime::Home *fit = nullptr, *spare = nullptr;
   for (Runtime::Home &h : r.homes) {
-    if (in_use(h.ptr)) continue;
+    if (home_in_use(h.ptr)) continue;
     spare = &h;
     if (h.bytes >= bytes && (!fit || h.bytes < fit->bytes)) fit = &h;
   }
@@ -149,7 +176,7 @@ void *home_acquire(size_t bytes) {
   }
   void *p = nullptr;
   const size_t want = (bytes + 0xFFFFF) & ~(size_t)0xFFFFF;
-  OCC_CUDA(cudaMalloc(&p, want));
+  OCC_CUDA(device_malloc(&p, want));
   if (p) r.homes.push_back(Runtime::Home{p, want});
   return p;
 }
@@ -266,7 +293,7 @@ void *scratch_get(int slot, size_t bytes) {
   size_t want = bytes + bytes / 8;
   want = (want + 0xFFFFF) & ~(size_t)0xFFFFF;
   void *p = nullptr;
-  OCC_CUDA(cudaMalloc(&p, want));
+  OCC_CUDA(device_malloc(&p, want));
   r.scratch[slot] = p;
   r.scratch_bytes[slot] = p ? want : 0;
   return p;

@@ -174,13 +174,18 @@ void mark_parts(void *p, int64_t n, int64_t c, int64_t h, int64_t w, const void 
 // The bytes of a tensor that is_act16() or is_parts().
 const __nv_bfloat16 *act16_ptr(const void *p);
 // A buffer for a 16-bit tensor that cannot be written at its own address; in use as long as a tensor
-// record (or a kernel that is held back, see home_held) refers to it.  A handful are kept.
+// record (or a kernel that is held back, see home_held) refers to it.  Up to six are kept for the next tensors, more
+// while more are in use at a time.
 void *home_acquire(size_t bytes);
 // The current mode stores fp16 (else bf16) in its 16-bit tensors.
 bool mode_f16();
 // A tensor that reads as zero and has not been written since it was handed out.
 bool is_zero(const void *p);
 
+// cudaMalloc, with a second attempt when the runtime has memory to give back (buffers no tensor is in, what batches in
+// pieces work in).
+cudaError_t device_malloc(void **p, size_t bytes);
+void free_idle_homes();
 void *scratch_get(int slot, size_t bytes);
 // Error word of the allocation-free entry point on the current device (0 when it was never
 // used there); see no_alloc.cu.

@@ -1,5 +1,9 @@
 """Large batches from host memory, which are computed in pieces while they arrive: every pass with another
 batch, and with a constant that changes, against the same model computed from device memory."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -148,3 +152,35 @@ def test_other_tensors_behind_pieces(native_libs):
             assert max_rel_err(got[1], means) <= 2e-2, i
             assert i > PASSES + 2 or rt.form_counters()["in_pieces"] > n0 + 1
     assert rt.last_error() == 0
+
+
+def test_memory_is_given_back(native_libs):
+    """When an allocation fails, what batches in pieces work in makes room for it.  (In a process of its own, which
+    would end at the failure.)"""
+    code = """
+import numpy as np, torch
+import test_gpu_host_batches as t
+from occamy_b200 import graphs, replay, runtime as rt
+rt.set_math_mode(rt.MATH_BF16)
+b = replay.Binding()
+g = t.net(512, 224)
+p = g.to_program()
+p.lower(fuse=1)
+x = torch.from_numpy(t.rand(1, *g.input_shape)).pin_memory().numpy()
+for _ in range(t.PASSES + 3):
+    (want,) = p.run(b, x)
+assert rt.form_counters()["in_pieces"] > 0
+free = torch.cuda.mem_get_info()[0]
+keep = torch.empty(free - (96 << 20), dtype=torch.uint8, device="cuda")
+buf = rt.DeviceBuffer(192 << 20)   # more than is left: the pieces' memory (some 500 MB) has to go
+del keep
+torch.cuda.empty_cache()
+for _ in range(t.PASSES):
+    (got,) = p.run(b, x)
+    assert np.array_equal(got, want)
+assert rt.last_error() == 0
+"""
+    here = os.path.dirname(os.path.abspath(__file__))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([here, os.path.dirname(here)]))
+    r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
