@@ -1051,15 +1051,6 @@ cudaError_t wrapDNNMemcpy(void *dst, const void *src, size_t count_, int kind,
       trace_mark_uploaded();
       pending_guard_range(dst, count_, true);
     }
-    if (kind == 1 && whole && count_ >= (4u << 20)) {
-      if (!g_copy_stream) OCC_CUDA(cudaStreamCreateWithFlags(&g_copy_stream, cudaStreamNonBlocking));
-      if (graph_upload_in_pieces(dst, src, count_, g_copy_stream)) {
-        count(CNT_H2D_BYTES, (int64_t)count_);
-        rec->fmt = FMT_F32;
-        rec->home = rec->dev_src = nullptr;
-        return cudaSuccess;
-      }
-    }
     const bool in_pool = g_cur_pool && (uintptr_t)dst >= (uintptr_t)g_cur_pool &&
                          (uintptr_t)dst + count_ <= (uintptr_t)g_cur_pool + g_cur_pool_bytes;
     if (kind == 1 && whole && in_pool && count_ >= (1u << 20) && pool_cache_blocks() >= 2) {
@@ -1077,6 +1068,12 @@ cudaError_t wrapDNNMemcpy(void *dst, const void *src, size_t count_, int kind,
         OCC_CUDA(cudaEventRecord(before, r.stream));
         OCC_CUDA(cudaStreamWaitEvent(g_copy_stream, before, 0));
         OCC_CUDA(cudaEventDestroy(before));
+      }
+      if (graph_upload_in_pieces(dst, src, count_, g_copy_stream)) {
+        count(CNT_H2D_BYTES, (int64_t)count_);
+        rec->fmt = FMT_F32;
+        rec->home = rec->dev_src = nullptr;
+        return cudaSuccess;
       }
       err = cudaMemcpyAsync(dst, src, count_, cudaMemcpyHostToDevice, g_copy_stream);
       cudaEvent_t ev;

@@ -887,11 +887,8 @@ bool graph_upload_in_pieces(void *dst, const void *src, size_t bytes, cudaStream
   if (!there || !find_input(*p, c) || (size_t)c.x_bytes != bytes || c.x - p->pool_base + base != (uintptr_t)dst ||
       !piece_images(c.batch, images))
     return false;
-  // behind what is enqueued already: it may still read or write the memory
   for (cudaEvent_t &e : gr.piece_here)
     if (!e) OCC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  OCC_CUDA(cudaEventRecord(gr.piece_here[0], rt().stream));
-  OCC_CUDA(cudaStreamWaitEvent(copy_stream, gr.piece_here[0], 0));
   size_t at = 0;
   for (int k = 0; k < MAX_PIECES; ++k) {
     const size_t n = bytes / (size_t)c.batch * (size_t)images[k];

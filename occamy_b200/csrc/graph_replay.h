@@ -31,9 +31,10 @@ void graph_settle();
 void graph_stop_capture();
 // The same for an upload, which the trace notes as well: a window does not reach across it.
 void graph_before_upload();
-// An upload of `bytes` to `dst`, recorded just now, is about to start.  When the inference's window exists
-// cut up by images, the upload is made in as many pieces on `copy_stream`, and true is returned: the window
-// takes the pieces as they arrive, and any other call waits for the last.
+// An upload of `bytes` to `dst`, recorded just now, is about to start; `copy_stream` waits for what may still use that
+// memory.  When the inference's window exists cut up by images, the upload is made in as many pieces on
+// `copy_stream`, and true is returned: the window takes the pieces as they arrive, and any other call waits for the
+// last.
 bool graph_upload_in_pieces(void *dst, const void *src, size_t bytes, cudaStream_t copy_stream);
 // Device memory that graphs may refer to is about to be freed or its contents replaced.
 void graph_forget_all();
