@@ -14,8 +14,7 @@
 //     list, coalescing free, pool size = high-water mark
 //     (Transform/DNN/mallocPoolOpt.hpp:21-140, mallocPoolOpt.cpp:41-76)
 // and then replays the resulting straight-line program against any shared library that
-// exports the runtime ABI (DNNToLLVM/DNNAPISpecs.inc), as main_graph would (the stream for its copies
-// is made once per binding, not once per inference).
+// exports the runtime ABI (DNNToLLVM/DNNAPISpecs.inc), exactly as main_graph would.
 #include <dlfcn.h>
 
 #include <chrono>
@@ -24,8 +23,6 @@
 #include <cstdlib>
 #include <algorithm>
 #include <cstring>
-#include <map>
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -39,6 +36,7 @@ struct Api {
   int (*cudnnCreate)(Handle *) = nullptr;
   int (*cudnnDestroy)(Handle) = nullptr;
   int (*cudaStreamCreate)(Stream *) = nullptr;
+  int (*cudaStreamDestroy)(Stream) = nullptr;
   int (*cudaDeviceSynchronize)() = nullptr;
   int (*wrapDNNMalloc)(void **, size_t) = nullptr;
   int (*wrapDNNMemPoolInit)(void **, size_t) = nullptr;
@@ -64,25 +62,7 @@ struct Api {
   float *(*CUDAClipFunc)(float *, float *, int64_t *, float, float, int64_t) = nullptr;
   float *(*CUDAFlattenFunc)(float *, int64_t *, float *, int64_t *, int32_t, int64_t) = nullptr;
   int (*occamy_synchronize)() = nullptr;  // optional
-  int (*cudaGetDevice)(int *) = nullptr;  // optional
-  // The stream handed to the copies, one per device and kept with the binding: creating and
-  // destroying one around every inference took 109 us, twice the GPU time of a small program.
-  std::mutex stream_lock;
-  std::map<int, Stream> streams;
   std::string error;
-
-  Stream stream() {
-    int dev = 0;
-    if (cudaGetDevice) cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> hold(stream_lock);
-    auto it = streams.find(dev);
-    if (it == streams.end()) {
-      Stream s = nullptr;
-      cudaStreamCreate(&s);
-      it = streams.emplace(dev, s).first;
-    }
-    return it->second;
-  }
 };
 
 template <typename F>
@@ -762,6 +742,7 @@ void *occ_bind(const char *so_path, char *err, int err_cap) {
   if (!ok) api->error = std::string("dlopen failed: ") + dlerror();
   ok = ok && bind(*api, api->cudnnCreate, "cudnnCreate") && bind(*api, api->cudnnDestroy, "cudnnDestroy") &&
        bind(*api, api->cudaStreamCreate, "cudaStreamCreate") &&
+       bind(*api, api->cudaStreamDestroy, "cudaStreamDestroy") &&
        bind(*api, api->cudaDeviceSynchronize, "cudaDeviceSynchronize") &&
        bind(*api, api->wrapDNNMalloc, "wrapDNNMalloc") &&
        bind(*api, api->wrapDNNMemPoolInit, "wrapDNNMemPoolInit") &&
@@ -776,10 +757,7 @@ void *occ_bind(const char *so_path, char *err, int err_cap) {
        bind(*api, api->CUBLASMatmul2dFunc, "CUBLASMatmul2dFunc") &&
        bind(*api, api->CUDASoftmaxFunc, "CUDASoftmaxFunc") && bind(*api, api->CUDAClipFunc, "CUDAClipFunc") &&
        bind(*api, api->CUDAFlattenFunc, "CUDAFlattenFunc");
-  if (ok) {
-    bind(*api, api->occamy_synchronize, "occamy_synchronize", false);
-    bind(*api, api->cudaGetDevice, "cudaGetDevice", false);
-  }
+  if (ok) bind(*api, api->occamy_synchronize, "occamy_synchronize", false);
   if (!ok) {
     if (err && err_cap > 0) snprintf(err, err_cap, "%s", api->error.c_str());
     delete api;
@@ -800,8 +778,9 @@ int occ_run(void *h, void *api_h, const float *input, int input_kind, float **ou
   Program &p = *static_cast<Program *>(h);
   Api &api = *static_cast<Api *>(api_h);
   Handle handle = nullptr;
+  Stream stream = nullptr;
   api.cudnnCreate(&handle);
-  const Stream stream = api.stream();
+  api.cudaStreamCreate(&stream);
   void *pool = nullptr;
   if (p.pool) api.wrapDNNMemPoolInit(&pool, (size_t)p.pool_bytes);
   for (Instr &in : p.prog) {
@@ -880,6 +859,7 @@ int occ_run(void *h, void *api_h, const float *input, int input_kind, float **ou
   }
   if (p.pool) api.wrapDNNDealloc(pool);
   else api.cudaDeviceSynchronize();
+  api.cudaStreamDestroy(stream);
   api.cudnnDestroy(handle);
   return 0;
 }
