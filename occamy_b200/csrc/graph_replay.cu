@@ -460,10 +460,16 @@ void wait_for_upload() {
 
 // ---- windows cut up by images -------------------------------------------------------
 // Images of each piece: the first is what is waited for, so it is the smallest (256 images: 64, 96, 96
-// took 4.5 ms where three of 85 took 4.7).  None for batches below 128, whose pieces lose more in
-// efficiency than the upload takes.
+// took 4.5 ms where three of 85 took 4.7).  None for batches below 128, nor in the fp32 mode, which computes for
+// longer than the upload takes.  Milliseconds per inference from pinned memory to host memory, 224x224, whole batch
+// and pieces:
+//     images               64             96            128            192            256
+//     ResNet-50    1.87 / 2.12    2.50 / 2.53    3.24 / 2.91    4.56 / 3.68    5.96 / 4.49
+//     MobileNetV2  1.38 / 1.30    1.89 / 1.67    2.44 / 2.06                   4.53 / 3.69
+//     VGG-16       2.64 / 2.43                   4.94 / 4.45
+//     fp32 ResNet  5.72 / 6.44                  10.44 / 10.67
 int piece_images(int64_t n, int64_t *images) {
-  if (n < 128) return 0;
+  if (n < 128 || rt().mode == MATH_FP32) return 0;
   images[0] = n / 4 / 8 * 8;
   images[1] = (n - images[0]) / 2 / 8 * 8;
   images[2] = n - images[0] - images[1];
