@@ -21,7 +21,9 @@ def test_conv(binding, N, H, W, shortcut):
     rt.set_math_mode(rt.MATH_BF16)
     p = g.to_program()
     p.lower(fuse=replay.FUSE_REFERENCE)
+    n0 = rt.form_counters()["column_strips"]
     for _ in range(3):
         (got,) = p.run(binding, x)
         assert max_rel_err(got, want) <= 2e-2
+    assert rt.form_counters()["column_strips"] == n0 + 3
     assert rt.last_error() == 0

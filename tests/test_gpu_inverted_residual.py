@@ -47,13 +47,16 @@ def test_block(binding, shape, fuse, mode):
     rt.lib().occamy_set_cross_call_fusion(1)
     p = g.to_program()
     p.lower(fuse=fuse)
-    launches = []
+    launches, forms = [], rt.form_counters()["inverted_residual"]
     for _ in range(4):
         before = rt.counters()["launches"]
         (got,) = p.run(binding, v)
         launches.append(rt.counters()["launches"] - before)
         assert max_rel_err(got, want) <= 2e-2
     assert launches[2] < launches[0]
+    # large batches of small images run faster apart, and so does the last shape where the depthwise sums are fp32
+    apart = shape == SHAPES[7] or (shape == SHAPES[9] and mode == rt.MATH_BF16)
+    assert rt.form_counters()["inverted_residual"] - forms == (0 if apart else 3)
     assert rt.last_error() == 0
 
 
@@ -109,10 +112,12 @@ def test_last_chunk(binding, N, C, H, E, K, act, mode):
     v = graphs.make_input(g, 1)
     bad = np.full_like(v, np.nan)
     (want,) = run_graph_oracle(g, v)
+    forms = rt.form_counters()["inverted_residual"]
     for i in range(6):
         p.run(binding, bad)   # leaves NaN in every shared memory
         (got,) = p.run(binding, v)
         assert max_rel_err(got, want) <= 2e-2, i
+    assert rt.form_counters()["inverted_residual"] >= forms + 10
     assert rt.last_error() == 0
 
 
@@ -134,9 +139,11 @@ def test_overflow_of_the_depthwise_sums(binding, act):
     p = g.to_program()
     p.lower(fuse=replay.FUSE_REFERENCE)
     v = graphs.make_input(g, 1)
+    forms = rt.form_counters()["inverted_residual"]
     for i in range(4):   # the first runs convolution by convolution
         (got,) = p.run(binding, v)
         assert np.isnan(got[:, :, 1:-1]).all(), i
+    assert rt.form_counters()["inverted_residual"] >= forms + 3
     assert rt.last_error() == 0
 
 
@@ -156,7 +163,9 @@ def test_precision_of_the_depthwise_sums(binding, hi, sums_in_half):
     p = g.to_program()
     p.lower(fuse=replay.FUSE_REFERENCE)
     v = graphs.make_input(g, 1)
+    forms = rt.form_counters()["inverted_residual"]
     for i in range(4):
         (got,) = p.run(binding, v)
         assert i == 0 or (got[:, :, 1:-1, 1:-1] == (0.0 if sums_in_half else E / 8)).all(), i
+    assert (rt.form_counters()["inverted_residual"] > forms) == sums_in_half
     assert rt.last_error() == 0

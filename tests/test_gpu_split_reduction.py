@@ -44,9 +44,12 @@ def test_conv_with_residual(binding, shape, mode):
     rt.set_math_mode(mode)
     p = g.to_program()
     p.lower(fuse=replay.FUSE_REFERENCE)
+    n0 = rt.form_counters()["split_reduction"]
     for _ in range(3):
         (got,) = p.run(binding, x)
         assert max_rel_err(got, want) <= TOL[mode]
+    if mode != rt.MATH_FP32 or N * H * W * C * K * R * R >= 1e6 * st * st:   # (smaller ones stay on the CUDA cores)
+        assert rt.form_counters()["split_reduction"] >= n0 + 3
     assert rt.last_error() == 0
 
 
@@ -60,9 +63,12 @@ def test_gemm(binding, M, K, N, mode):
     rt.set_math_mode(mode)
     p = g.to_program()
     p.lower(fuse=replay.FUSE_REFERENCE)
+    n0 = rt.form_counters()["split_reduction"]
     for _ in range(2):
         (got,) = p.run(binding, x)
         assert max_rel_err(got, want) <= TOL[mode]
+    if mode != rt.MATH_FP32 or M * K * N >= 1e6:
+        assert rt.form_counters()["split_reduction"] == n0 + 2
     assert rt.last_error() == 0
 
 
