@@ -12,6 +12,10 @@
 // Per 64-byte line: acc += lo32(w ^ key) * hi32(w ^ key) in every 64-bit lane, plus the neighbouring
 // half's words unmixed, so that no single changed word goes unseen; the key steps from line to line,
 // so that exchanged lines count as a change.
+//
+// Published methods it builds on: the step per line is the long-input accumulation of XXH3 (Y. Collet, xxHash), the
+// final mix is one round of splitmix64's (S. Vigna); the constants are odd 64-bit numbers known from these and from
+// wyhash (W. Yi).  The choice of lines and their completion are this file's.
 #include <cstddef>
 #include <cstdint>
 #include <cstring>
