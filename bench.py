@@ -521,7 +521,8 @@ def main():
                      "frac_of_sustained_peak": achieved / peaks["bf16_tflops_sustained"],
                      "traffic": profiled_traffic(per_rank, args.graph) if world == 1 else None,
                      "traffic_note": "DRAM read+write bytes of the tensor-core launches of one "
-                                     "step (ncu, profiles/tc_conv_traffic_resnet50_b256.txt)",
+                                     "step (ncu, profiles/tc_conv_traffic_resnet50_b256.txt; taken of the "
+                                     "persistent kernels before the column strips)",
                      "kernel": "tc_conv_kernel (+ tc_conv_pn_kernel, stem_pool_kernel)",
                      "launches_per_step": per_step,
                      "kernel_ms_per_step": tc_total_ms,

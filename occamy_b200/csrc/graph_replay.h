@@ -4,9 +4,9 @@
 // signatures, format registry, tensor maps, some sixty launches - took 300 to 400 us of host time,
 // more than the GPU needs for a small batch.  Once an inference has run call by call with nothing
 // left to upload or allocate, its calls from the one after the input's arrival up to the last
-// computing one (the window) are captured while they run; later inferences only check that each call
+// computing one (the window) are recorded as graphs; later inferences only check that each call
 // is the recorded one (signature, and for a constant its host address and fingerprint) and the
-// captured graphs are launched in its place, each as soon as the last of its calls has come by.
+// graphs are launched in its place, each as soon as the last of its calls has come by.
 //
 // A call that differs - another shape, a changed constant, anything outside the window - takes the
 // inference back: the calls that no launched graph covers are made again one by one, then the
@@ -26,8 +26,8 @@ void graph_after_call();
 // Something is about to happen that calls held back must come before (another entry point waits for
 // the stream, reads a result, changes a mode): everything up to here is enqueued.
 void graph_settle();
-// Work that cannot be captured follows (an allocation, a packing, a wait): what has been captured is
-// launched, the rest of the inference is not captured.
+// Work that cannot be recorded follows (an allocation, a packing, a wait): what has been recorded is
+// launched, the rest of the inference is not recorded.
 void graph_stop_capture();
 // The same for an upload, which the trace notes as well: a window does not reach across it.
 void graph_before_upload();
