@@ -97,8 +97,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_conv_pn_kernel(const __grid_
       uint32_t phase = 0;
       const uint32_t tx_bytes = (uint32_t)rows_valid * bk * 2u + w_bytes;
       for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x) {
-        const int kt = tile % p.tiles_k;
-        int sp = tile / p.tiles_k;
+        const int at = p.descending ? p.total_tiles - 1 - tile : tile;
+        const int kt = at % p.tiles_k;
+        int sp = at / p.tiles_k;
         const int q0 = (sp % p.tiles_w) * p.tw;
         sp /= p.tiles_w;
         const int p0 = (sp % p.tiles_h) * p.th;
@@ -189,8 +190,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_conv_pn_kernel(const __grid_
     const bool one_slab = p.K <= 64;
     uint32_t flip = 0;
     for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x) {
-      const int kt = tile % p.tiles_k;
-      int sp = tile / p.tiles_k;
+      const int at = p.descending ? p.total_tiles - 1 - tile : tile;
+      const int kt = at % p.tiles_k;
+      int sp = at / p.tiles_k;
       const int q0 = (sp % p.tiles_w) * p.tw;
       sp /= p.tiles_w;
       const int p0 = (sp % p.tiles_h) * p.th;
@@ -1099,13 +1101,15 @@ void launch_tc_conv(const TcConvArgs &a, cudaStream_t s) {
     if (plans.size() > 4096) plans.clear();
     it = plans.emplace(key, build_plan(a, rt().dev_err, rt().num_sms, true)).first;
   }
-  const Plan &pl = it->second;
+  Plan &pl = it->second;
   if (!pl.ok) {
     set_error(998, "tensor-core conv plan");
     return;
   }
   if (pl.p.total_tiles == 0) return;
   Runtime &r = rt();
+  pl.p.descending = r.descending;
+  r.descending ^= 1;
   int prof_slot = -1;
   if (r.profiling) {
     prof_slot = r.prof_count++;

@@ -71,6 +71,7 @@ struct alignas(64) TcParams {
   int n_mma;             // pixel-N variant: N of the MMA (pixels per tile rounded up to 16)
   int sp_tiles;          // pixel tiles (tiles_w * tiles_h * tiles_n); with TC_MODE_PAIR the tile
                          // index counts PAIRS of them and total_tiles = ceil(sp_tiles / 2) * tiles_k
+  int descending;        // tiles are taken from the last to the first (Runtime::descending)
   int *err;
 };
 
@@ -473,6 +474,7 @@ struct TcTile {
 template <int BN, bool PAIR = false>
 __device__ __forceinline__ TcTile tc_decode(const TcParams &p, int tile, uint32_t rank = 0,
                                             bool *ghost = nullptr) {
+  if (p.descending) tile = p.total_tiles - 1 - tile;
   uint32_t sp = tc_fdiv((uint32_t)tile, p.div_k);
   const uint32_t kt = (uint32_t)tile - sp * (uint32_t)p.tiles_k;
   if constexpr (PAIR) {

@@ -51,6 +51,7 @@ struct StemParams {
   int bands, band_rows, units;
   int cr_bytes;        // bytes of one convolution-row ring slot
   float lo, hi;
+  int descending;      // units are taken from the last to the first (Runtime::descending)
   int *err;
 };
 
@@ -178,6 +179,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stem_pool_kernel(const StemPara
 
   // pooled rows [i0, i1) and convolution rows [h_lo, h_hi] of a unit
   auto unit_rows = [&](int unit, int &n, int &i0, int &i1, int &h_lo, int &h_hi) {
+    if (p.descending) unit = p.units - 1 - unit;
     n = unit / p.bands;
     const int b = unit - n * p.bands;
     i0 = b * p.band_rows;
@@ -484,6 +486,8 @@ bool launch_stem_pool(const StemPoolArgs &a, int *err_word, int num_sms, cudaStr
   p.PP = a.PP; p.QP = a.QP;
   p.lo = a.lo; p.hi = a.hi;
   p.err = err_word;
+  p.descending = rt().descending;
+  rt().descending ^= 1;
   // bands: enough units to balance the SMs, each band re-computes one convolution row
   int bands = 1;
   while ((int64_t)a.N * bands < 6ll * num_sms && a.PP / (bands * 2) >= 4) bands *= 2;
