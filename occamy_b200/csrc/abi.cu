@@ -208,7 +208,8 @@ struct ConvJob {
   int absorbed = 0;           // later calls folded into this one so far
   // device ranges still to be read: [0] input, [1] residual operand, [2] a bias that is read
   // from the caller's tensor (no resident copy exists)
-  uintptr_t dep_lo[3] = {0, 0, 0}, dep_hi[3] = {0, 0, 0};
+  // ([3], [4]: input and bias of a second summand)
+  uintptr_t dep_lo[5] = {}, dep_hi[5] = {};
   // a matrix product: `g` says N x K results (P = Q = 1), `a` how they are computed
   bool product = false;
   bool out16 = false;             // ... whose reader is another product: 16-bit result
@@ -217,6 +218,8 @@ struct ConvJob {
   // one of the convolutions of an inverted residual: its result only goes to the next one / its input
   // only comes from the one before (and is not there yet)
   bool linked = false, joined = false;
+  // held back until a sum takes its result along (RF_SUM) / the other summand, which g_front[0] still is
+  bool summand = false, after_summand = false;
   // (the constants of one once more, packed_for_block(): a first bias, a depthwise filter and bias)
   const void *block_w = nullptr, *block_b = nullptr;
   // folded (few-channel) form: what the fused convolution + pool kernel needs besides `a`
@@ -229,7 +232,7 @@ int g_fronts = 0;
 const ConvJob *g_launching = nullptr;   // job whose output buffer is being looked for
 
 bool job_reads(const ConvJob &j, const void *home) {
-  return j.a.x == home || j.a.residual == home || j.dw_x == home;
+  return j.a.x == home || j.a.x2 == home || j.a.residual == home || j.dw_x == home;
 }
 bool home_held_hook(const void *home) {
   for (int i = 0; i < g_fronts; ++i)
@@ -526,7 +529,8 @@ const bf16 *launch_job(ConvJob &job, bool apart = false) {
   const bool in_place = olo == job.dep_lo[1] && ohi == job.dep_hi[1];
   if (apart || ranges_overlap(olo, ohi, job.dep_lo[0], job.dep_hi[0]) ||
       (ranges_overlap(olo, ohi, job.dep_lo[1], job.dep_hi[1]) && !in_place) ||
-      ranges_overlap(olo, ohi, job.dep_lo[2], job.dep_hi[2])) {
+      ranges_overlap(olo, ohi, job.dep_lo[2], job.dep_hi[2]) || ranges_overlap(olo, ohi, job.dep_lo[3], job.dep_hi[3]) ||
+      ranges_overlap(olo, ohi, job.dep_lo[4], job.dep_hi[4])) {
     g_launching = &job;
     dst = home_acquire(obytes);
     g_launching = nullptr;
@@ -591,6 +595,38 @@ bool launch_block(ConvJob &a, ConvJob &b, ConvJob &c) {
   return true;
 }
 
+// Makes the sum of two held-back convolutions one kernel's: `b` takes `a` along.  False when no kernel does, or one of
+// the operands is not there to stay.
+bool join_summands(const ConvJob &a, ConvJob &b) {
+  auto plain = [](const TcConvArgs &t) {
+    return t.R == 1 && t.S == 1 && t.pad_h == 0 && t.pad_w == 0 && !t.w_step;
+  };
+  auto strided = [](const TcConvArgs &t) { return t.stride_h != 1 || t.stride_w != 1; };
+  // the second summand is a 1x1 convolution, the strided one of two
+  const bool swap = plain(a.a) && (!plain(b.a) || (strided(a.a) && !strided(b.a)));
+  const TcConvArgs &first = swap ? b.a : a.a, &second = swap ? a.a : b.a;
+  if (!plain(second) || (b.a.split && b.g.K % 16)) return false;
+  TcConvArgs c = first;
+  c.x2 = second.x; c.w2 = second.w; c.bias2 = second.bias;
+  c.H2 = second.H; c.W2 = second.W; c.Cf2 = second.Cf;
+  c.stride2_h = second.stride_h; c.stride2_w = second.stride_w;
+  c.consts_ready = a.a.consts_ready && b.a.consts_ready;
+  c.y = b.a.y; c.out_f32 = b.a.out_f32;
+  if (!tc_conv_supported(c)) return false;
+  b.a = c;
+  b.dep_lo[3] = a.dep_lo[0]; b.dep_hi[3] = a.dep_hi[0];
+  b.dep_lo[4] = a.dep_lo[2]; b.dep_hi[4] = a.dep_hi[2];
+  return true;
+}
+
+// The other summand by itself: no kernel takes both.
+void launch_summand() {
+  if (!g_pending.after_summand) return;
+  g_pending.after_summand = false;
+  launch_job(g_front[0]);
+  g_fronts = 0;
+}
+
 // Executes the held-back convolution as far as it has been built up.
 void flush_pending() {
   if (!g_pending.active) return;
@@ -598,6 +634,7 @@ void flush_pending() {
   for (int i = 0; i < g_fronts; ++i)
     if (g_front[i].absorbed) trace_count_chain();
   if (g_pending.absorbed && !g_pending.product) trace_count_chain();   // convolution chains
+  launch_summand();
   if (g_fronts != 2 || !launch_block(g_front[0], g_front[1], g_pending)) {
     const bf16 *x = nullptr;
     auto resolve = [&](ConvJob &job) {
@@ -630,7 +667,7 @@ void pending_guard_range(const void *p, size_t bytes, bool writes) {
   if (writes)
     for (int j = 0; j <= g_fronts; ++j) {
       const ConvJob &job = j < g_fronts ? g_front[j] : g_pending;
-      for (int k = 0; k < 3; ++k)
+      for (int k = 0; k < 5; ++k)
         if (ranges_overlap(lo, hi, job.dep_lo[k], job.dep_hi[k])) {
           if (rt().log) fprintf(stderr, "[occamy] held-back conv runs early: input %d overwritten\n", k);
           flush_pending();
@@ -638,10 +675,12 @@ void pending_guard_range(const void *p, size_t bytes, bool writes) {
         }
     }
   // the tensor it is going to write must also still belong to it
-  const uintptr_t olo = (uintptr_t)g_pending.out;
-  const size_t elem = g_pending.a.split || g_pending.product ? 4 : 2;
-  const uintptr_t ohi = olo + (size_t)g_pending.g.N * g_pending.g.K * g_pending.g.P * g_pending.g.Q * elem;
-  if (ranges_overlap(lo, hi, olo, ohi)) {
+  auto takes_output = [&](const ConvJob &job) {
+    const uintptr_t olo = (uintptr_t)job.out;
+    const size_t elem = job.a.split || job.product ? 4 : 2;
+    return ranges_overlap(lo, hi, olo, olo + (size_t)job.g.N * job.g.K * job.g.P * job.g.Q * elem);
+  };
+  if (takes_output(g_pending) || (g_pending.after_summand && takes_output(g_front[0]))) {
     if (rt().log) fprintf(stderr, "[occamy] held-back conv runs early: output re-handed out\n");
     flush_pending();
   }
@@ -672,7 +711,8 @@ Role step(Entry &e, bool passive) {
     if (trace_has_elided() && rt().log)
       fprintf(stderr, "[occamy] call sequence left the recorded one after tensors were skipped\n");
   }
-  if (!passive && role != R_ABSORB && !((trace_last_flags() & RF_JOIN) && g_pending.active && g_pending.linked)) {
+  if (!passive && role != R_ABSORB && !((trace_last_flags() & RF_JOIN) && g_pending.active && g_pending.linked) &&
+      !((trace_last_flags() & RF_SUM) && g_pending.active && g_pending.summand)) {
     if (g_pending.active && rt().log)
       fprintf(stderr, "[occamy] held-back conv closed by call sym %d (absorbed %d)\n", e.sym,
               g_pending.absorbed);
@@ -803,8 +843,14 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
                g.S <= 16 && g.R <= 11;
   const Role role = step(e, false);
   if (role == R_SKIP) return y;
-  bool join = false;
-  if (g_pending.active) {   // left by step() because this call was recorded as joining it
+  const uint8_t flags = trace_last_flags();
+  bool join = false, sum = false;
+  if (g_pending.active && g_pending.summand) {   // left by step(): this call was recorded as the other summand
+    const ConvGeom &f = g_pending.g;
+    sum = role == R_DEFER && e.fusable && !depthwise && e.parts == (g_pending.a.split != 0) && f.N == g.N && f.K == g.K &&
+          f.P == g.P && f.Q == g.Q && !g_pending.act_set && !g_pending.res_set;
+    if (!sum) flush_pending();
+  } else if (g_pending.active) {   // left by step() because this call was recorded as joining it
     const ConvGeom &f = g_pending.g;
     join = role == R_DEFER && e.fusable && !e.parts && stays_packed(w) && g_fronts < 2 && g_pending.out == x && f.N == g.N && f.K == g.C &&
            f.P == g.H && f.Q == g.W && (depthwise ? g_fronts == 0 : g_fronts == 1 && g.C % 16 == 0);
@@ -820,9 +866,19 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
     fprintf(stderr, "[occamy] conv x[%d,%d,%d,%d] w[%d,%d,%d,%d] g%d s%d p%d act%d role%d\n", g.N,
             g.C, g.H, g.W, g.K, (int)dW[1], g.R, g.S, g.groups, g.stride_h, g.pad_h, act,
             (int)role);
+  // One of two summands, prepared: the second finds the first held back (unless an upload had to run it), the first
+  // may wait for it when its operands stay where they are.
+  auto hold_summand = [&](ConvJob &job, bool in_place) {
+    if (sum && g_pending.active) {
+      g_front[0] = g_pending;
+      g_fronts = 1;
+      job.after_summand = true;
+    } else if (!sum) {
+      job.summand = role == R_DEFER && (flags & RF_SUM) && !depthwise && in_place && stays_packed(w);
+    }
+  };
   if (r.mode != MATH_FP32) {
     ConvJob job;
-    const uint8_t flags = trace_last_flags();
     // (the first of three takes its input as it is)
     job.linked = role == R_DEFER && (flags & RF_LINK) && stays_packed(w) && (join || (!(flags & RF_JOIN) && is_act16(x, g.N, g.C, g.H, g.W)));
     job.joined = join;
@@ -841,6 +897,7 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
     }
     if (ok) {
       job.out = y;
+      hold_summand(job, is_act16(x, g.N, g.C, g.H, g.W) && g.C % 16 == 0);
       if (role == R_DEFER) {   // later calls of the recorded sequence fold into this one
         if (e.poolable && !depthwise && job.a.w_step) {
           // the pool that may join later runs after the filter tensor has been given back
@@ -860,7 +917,8 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
     ConvJob job;
     job.out = y;
     if (prepare_parts(x, w, bias, g, job)) {
-      job.out_parts = (trace_last_flags() & RF_FOR_PARTS) && g.K % 16 == 0;
+      job.out_parts = (flags & RF_FOR_PARTS) && g.K % 16 == 0;
+      hold_summand(job, is_parts(x, g.N, g.C, g.H, g.W));
       if (role == R_DEFER) {
         g_pending = job;
         g_pending.active = true;
@@ -870,6 +928,7 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
       return y;
     }
   }
+  flush_pending();   // (a summand that this convolution does not go with after all)
   ensure_f32(x);
   const float *wd = operand_f32(w, (size_t)numel4(dW) * 4);
   const float *bd = bias ? operand_f32(bias, (size_t)g.K * 4) : nullptr;
@@ -1380,6 +1439,16 @@ float *DNNTensorOpFunc(cudnnContext *, int64_t opMode, float *A, int64_t *dimA, 
     if (g_pending.active && e.kind == CK_SAME_ADD && dims_ok && !g_pending.depthwise && !g_pending.product && !g_pending.res_set &&
         !g_pending.act_set && ((A == g_pending.out) != (B == g_pending.out))) {
       const float *other = A == g_pending.out ? B : A;
+      if (g_pending.after_summand && other == g_front[0].out && join_summands(g_front[0], g_pending)) {
+        if (g_front[0].absorbed) trace_count_chain();
+        g_pending.after_summand = false;
+        g_fronts = 0;
+        g_pending.res_set = true;
+        if (other != out) elide(const_cast<float *>(other));
+        pending_retarget(out);
+        return out;
+      }
+      launch_summand();
       const bool parts = g_pending.a.split && g.K % 16 == 0 && is_parts(other, g.N, g.K, g.P, g.Q);
       if (parts || (!g_pending.a.split && is_act16(other, g.N, g.K, g.P, g.Q))) {
         g_pending.a.residual = act16_ptr(other);

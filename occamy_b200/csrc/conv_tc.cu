@@ -442,6 +442,13 @@ bool tc_conv_supported(const TcConvArgs &a) {
   if (a.y && (uintptr_t)a.y % 16) return false;
   if ((int64_t)a.N * a.P * a.Q >= (1ll << 31)) return false;
   if (a.K > 4096 && !a.split) return false;   // the bias vector has to fit in shared memory
+  if (a.x2) {
+    if (a.residual || a.w_step || a.pool2 || (a.out_f32 && !a.split) || a.R * a.S + 1 > TC_MAX_TAPS) return false;
+    if (a.stride2_h < 1 || a.stride2_w < 1 || a.stride2_h > 2 || a.stride2_w > 2) return false;
+    if ((a.H2 - 1) / a.stride2_h + 1 != a.P || (a.W2 - 1) / a.stride2_w + 1 != a.Q) return false;
+    if (a.split ? a.Cf2 % 16 || (a.Cf > 16) != (a.Cf2 > 16) : pick_bk(a.Cf2) != pick_bk(a.Cf)) return false;
+    if ((uintptr_t)a.x2 % 16 || (uintptr_t)a.w2 % 16) return false;
+  }
   return true;
 }
 
@@ -499,11 +506,22 @@ extern "C" void occamy_tc_timers(long long *out, int clear) {
 }
 #endif
 
+// Channels per k-step of the split-operand form: six tiles per stage, so half as deep (twice as deep is 5 to 9 %
+// slower, one CTA to an SM).
+static int parts_bk(int Cf) { return Cf > 16 ? 32 : 16; }
+// A layer whose pixels are looked at as one row of them, a plain product.
+static bool is_flat(const TcConvArgs &a) {
+  return a.R == 1 && a.S == 1 && a.stride_h == 1 && a.stride_w == 1 && a.pad_h == 0 && a.pad_w == 0 && a.w_step == 0 &&
+         (!a.x2 || (a.stride2_h == 1 && a.stride2_w == 1));
+}
+// Multiply-adds per output value, in the 64-channel k-steps the rules count in.
+static int reduction64(const TcConvArgs &a) { return (a.R * a.S * a.Cf + (a.x2 ? a.Cf2 : 0) + 63) / 64; }
+
 static int floordiv(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
 // Tensor maps of the A operand and the list of filter taps that read through them.
-static bool make_operand_maps(const TcConvArgs &a, bool flat, int Qg, int bk, const uint32_t *boxA,
-                              CUtensorMap *tmA, TcTap *taps, int *num_taps, bool counted) {
+static bool make_main_maps(const TcConvArgs &a, bool flat, int Qg, int bk, const uint32_t *boxA,
+                           CUtensorMap *tmA, TcTap *taps, int *num_taps, int *num_maps, bool counted) {
   const int parts = sk_parts(a.split != 0);   // fp32 operands: three planes, as many maps next to one another
   const int64_t plane = (int64_t)a.N * a.H * (a.row_elems ? a.row_elems : a.W * a.Cf);
   bool ok = true;
@@ -514,6 +532,7 @@ static bool make_operand_maps(const TcConvArgs &a, bool flat, int Qg, int bk, co
     for (int part = 0; part < parts; ++part)
       ok &= make_map(&tmA[part], a.x + part * plane, 4, dims, st, boxA, bk * 2, counted);
     taps[(*num_taps)++] = TcTap{0, 0, 0};
+    *num_maps = parts;
     return ok;
   }
   // one tensor map per (row phase, column phase) of the stride
@@ -542,7 +561,30 @@ static bool make_operand_maps(const TcConvArgs &a, bool flat, int Qg, int bk, co
       }
       taps[(*num_taps)++] = TcTap{map_of[bh][bw] * parts, aw, ah};
     }
+  *num_maps = nmaps * parts;
   return ok;
+}
+// ... and, behind them, those of a second summand, whose tap is the last.
+static bool make_operand_maps(const TcConvArgs &a, bool flat, int Qg, int bk, const uint32_t *boxA,
+                              CUtensorMap *tmA, TcTap *taps, int *num_taps, bool counted) {
+  int num_maps = 0;
+  bool ok = make_main_maps(a, flat, Qg, bk, boxA, tmA, taps, num_taps, &num_maps, counted);
+  if (!a.x2) return ok;
+  TcConvArgs b = a;
+  b.x = a.x2; b.H = a.H2; b.W = a.W2; b.Cf = a.Cf2; b.R = b.S = 1;
+  b.pad_h = b.pad_w = 0; b.stride_h = a.stride2_h; b.stride_w = a.stride2_w;
+  int one = 0, more = 0;
+  ok &= make_main_maps(b, flat, Qg, bk, boxA, tmA + num_maps, taps + *num_taps, &one, &more, counted);
+  taps[*num_taps].map += num_maps;
+  *num_taps += one;
+  return ok;
+}
+// The weights of a second summand.
+static bool make_second_weights(const TcConvArgs &a, int bk, int rows, CUtensorMap *m, bool counted) {
+  const uint64_t dims[3] = {(uint64_t)a.Cf2, (uint64_t)a.K, (uint64_t)sk_parts(a.split != 0)};
+  const uint64_t st[2] = {(uint64_t)a.Cf2 * 2, (uint64_t)a.K * a.Cf2 * 2};
+  const uint32_t box[3] = {(uint32_t)bk, (uint32_t)rows, 1};
+  return make_map(m, a.w2, 3, dims, st, box, bk * 2, counted);
 }
 
 // ---- split-reduction kernel (conv_tc_split.cu) -------------------------------------
@@ -655,10 +697,8 @@ static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, d
   const char *force = getenv("OCCAMY_SK");
   if (force && !strcmp(force, "0")) return false;
 #endif
-  const bool flat = a.R == 1 && a.S == 1 && a.stride_h == 1 && a.stride_w == 1 && a.pad_h == 0 &&
-                    a.pad_w == 0 && a.w_step == 0;
-  // (split operands: six tiles per stage, so half as deep; twice as deep is 5 to 9 % slower, one CTA to an SM)
-  const int bk = a.split ? (a.Cf > 16 ? 32 : 16) : pick_bk(a.Cf);
+  const bool flat = is_flat(a);
+  const int bk = a.split ? parts_bk(a.Cf) : pick_bk(a.Cf);
   int Qg = a.Q, Pg = a.P, Ng = a.N;
   if (flat) {
     Qg = a.N * a.P * a.Q;
@@ -672,7 +712,8 @@ static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, d
   p.rows = p.tw * p.th * p.tn;
   p.bk = bk;
   p.cblocks = (a.Cf + bk - 1) / bk;
-  p.ksteps = a.R * a.S * p.cblocks;
+  p.ksteps1 = a.R * a.S * p.cblocks;
+  p.ksteps = p.ksteps1 + (a.x2 ? (a.Cf2 + bk - 1) / bk : 0);
   p.a_bytes = ((p.rows + 7) / 8 * 8 * bk * 2 + 1023) / 1024 * 1024;
   const SkChoice c = sk_choose(a, sp_tiles, p.rows, p.ksteps, bk, p.a_bytes, nsm, form);
   if (c.cost < 0) return false;
@@ -694,6 +735,7 @@ static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, d
   p.K = a.K;
   p.gq = Qg; p.gp = Pg; p.gn = Ng;
   p.bias = a.bias;
+  p.bias2 = a.x2 ? a.bias2 : nullptr;
   p.residual = a.residual;
   p.y = a.y;
   p.plane = (int64_t)a.N * a.P * a.Q * a.K;
@@ -713,6 +755,10 @@ static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, d
   for (int t = 0; t < num_taps; ++t) {
     if (abs(taps[t].dw) > 127 || abs(taps[t].dh) > 127) return false;
     p.taps[t] = SkTap{(int8_t)taps[t].map, (int8_t)taps[t].dw, (int8_t)taps[t].dh, 0};
+  }
+  if (a.x2) {
+    p.map2 = taps[--num_taps].map;
+    ok &= make_second_weights(a, bk, bn, &p.tmB2, counted);
   }
   const uint64_t dims[3] = {(uint64_t)a.Cf, (uint64_t)a.K, (uint64_t)num_taps * sk_parts(a.split != 0)};
   const uint64_t st[2] = {(uint64_t)a.Cf * 2, (uint64_t)a.K * a.Cf * 2};
@@ -763,8 +809,10 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   const int bk = pick_bk(a.Cf);
   p.bk = bk;
   p.cblocks = (a.Cf + bk - 1) / bk;
+  p.cblocks2 = a.x2 ? (a.Cf2 + bk - 1) / bk : 0;
   p.K = a.K;
   p.bias = a.bias;
+  p.bias2 = a.x2 ? a.bias2 : nullptr;
   p.has_res = a.residual ? 1 : 0;
   p.act = a.act;
   p.floor = a.act == ACT_RELU ? 0.0f : -INFINITY;
@@ -778,8 +826,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   p.timers = tc_timer_words();
 #endif
   p.consts_ready = a.consts_ready;
-  const bool flat = a.R == 1 && a.S == 1 && a.stride_h == 1 && a.stride_w == 1 && a.pad_h == 0 &&
-                    a.pad_w == 0 && a.w_step == 0;
+  const bool flat = is_flat(a);
   // output grid the tiles are cut from
   int Qg = a.Q, Pg = a.P, Ng = a.N;
   if (flat) {
@@ -801,11 +848,11 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   // than the plain one, which hurts the HBM-bound 1x1 layers
   // 3x3 / stride 1 / pad 1 with 64 -> 64 channels: the input block of a tile is loaded once and the taps are
   // windows of it (TC_MODE_HALO)
-  const bool halo = allow_halo && halo_allowed && !a.f16 && !a.out_f32 && a.R == 3 && a.S == 3 &&
+  const bool halo = allow_halo && halo_allowed && !a.f16 && !a.out_f32 && !a.x2 && a.R == 3 && a.S == 3 &&
                     a.stride_h == 1 && a.stride_w == 1 && a.pad_h == 1 && a.pad_w == 1 &&
                     a.Cf == 64 && a.K == 64 && a.w_step == 0 && a.Q == a.W &&
                     a.P == a.H;
-  const bool pn = !halo && pn_allowed && !a.f16 && !a.out_f32 && a.K <= 128 && a.R * a.S > 1 &&
+  const bool pn = !halo && pn_allowed && !a.f16 && !a.out_f32 && !a.x2 && a.K <= 128 && a.R * a.S > 1 &&
                   a.R * a.S * a.Cf >= 9 * 64;
   pl.pn = pn;
   if (halo && a.pool2) {
@@ -847,12 +894,12 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   const int bn = pn ? 128
                     : halo ? 64
                     : pick_bn(a.K, (long)p.tiles_w * p.tiles_h * p.tiles_n,
-                              (a.R * a.S * a.Cf + 63) / 64, nsm);
+                              reduction64(a), nsm);
   pl.bn = bn;
   p.tiles_k = (a.K + bn - 1) / bn;
   p.sp_tiles = p.tiles_w * p.tiles_h * p.tiles_n;
   // CTA pairs (see TC_MODE_PAIR) for the 256-channel tiles of 1x1 layers with a long reduction
-  const int ksteps64p = (a.R * a.S * a.Cf + 63) / 64;
+  const int ksteps64p = reduction64(a);
 #ifdef OCCAMY_TUNING
   static const bool pair_allowed = !(getenv("OCCAMY_TC_PAIR") && !strcmp(getenv("OCCAMY_TC_PAIR"), "0"));
 #else
@@ -879,7 +926,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
     // whose tiles are twice as tall; a whole tile of the halo form takes 0.9 us).
     const int per_wave = pair ? nsm / 2 : nsm;
     const double waves = (double)((p.total_tiles + per_wave - 1) / per_wave);
-    const int ks = p.cblocks * a.R * a.S;
+    const int ks = p.cblocks * a.R * a.S + p.cblocks2;
     const double tile_us = halo ? 0.9 : pn ? 0.49 * ks : (bn == 256 ? 0.1 : 0.0) + 0.27 * ks * (bk == 64 ? 1.0 : 0.75);
     if (!a.pool2 && (!piece || form) && sk_plan(a, err_word, nsm, counted, 3.1 + waves * tile_us, form, &pl)) return pl;
     if (a.pool2 && !halo && !pair) return pl;   // (not ok: tc_conv_takes_pool() said so)
@@ -895,6 +942,9 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   } else {
     ok &= make_operand_maps(a, flat, Qg, bk, boxA, p.tmA, p.taps, &p.num_taps, counted);
   }
+  p.second_tap = a.x2 ? p.num_taps - 1 : -1;
+  p.ksteps = (p.num_taps - (a.x2 ? 1 : 0)) * p.cblocks + p.cblocks2;
+  if (a.x2) ok &= make_second_weights(a, bk, pair ? bn / 2 : bn, &p.tmB2, counted);
   {
     const uint64_t dims[3] = {(uint64_t)a.Cf, (uint64_t)a.K, (uint64_t)(a.R * a.S)};
     const uint64_t st[2] = {(uint64_t)a.Cf * 2, (uint64_t)a.K * a.Cf * 2};
@@ -903,7 +953,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   }
   // For 256-wide tiles with a long reduction, 32-channel slabs free enough shared memory
   // for a fourth ring stage, which those layers need more than a cheap epilogue.
-  const int ksteps64 = (a.R * a.S * a.Cf + 63) / 64;
+  const int ksteps64 = reduction64(a);
   int dc = pn ? 64 : (bn < 64 ? bn : (bn == 256 && bk == 64 && ksteps64 >= 16 ? 32 : 64));
   if (bn == 64 && a.w_step && a.R <= 3 && !pn && !halo && !a.out_f32 && nsm >= 2) dc = 32;   // few-channel stems: two CTAs per SM, below
   if (a.out_f32 && bn >= 64) dc = 64;   // the fp32-output flavour is compiled for 64-channel slabs
@@ -932,13 +982,13 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   // CTAs asking L2 for the same 16 to 32 lines of weights for every tile is what bounded the
   // few-channel layers (1.5x on 32->16 and 16->96 channels at 112x112).  Measured: no gain at
   // 6 to 9 KB of weights, slower at 8 KB (64->64) and 32 KB (64->256 with residual).
-  const int ksteps_tile = p.num_taps * p.cblocks;
+  const int ksteps_tile = p.ksteps;
   const size_t b_tile_bytes = (size_t)(pair ? bn / 2 : bn) * bk * 2;
   // (With two CTAs per SM the single loading thread of a CTA is what the others wait for, and
   // weights of up to 16 KB pay as well: 144->24 at 56x56 has nine k-steps of 1 KB each.)
   const bool duo_wanted = !pn && !halo && !pair && !a.out_f32 && nsm >= 2 &&
                           dc == 32 && bn <= 64;
-  bool bres = !pn && !halo && !pair && p.tiles_k == 1 &&
+  bool bres = !pn && !halo && !pair && !a.x2 && p.tiles_k == 1 &&
               ksteps_tile * b_tile_bytes <= (size_t)(duo_wanted ? 16 : 4) * 1024;
 #ifdef OCCAMY_TUNING
   if (const char *f = getenv("OCCAMY_TC_BRES")) bres = bres && atoi(f) != 0;
@@ -1124,10 +1174,11 @@ void launch_tc_conv(const TcConvArgs &a, cudaStream_t s) {
   if (prof_slot >= 0) OCC_CUDA(cudaEventRecord(r.prof_events[2 * prof_slot + 1], s));
   OCC_CUDA(cudaGetLastError());
   count(CNT_LAUNCHES);
-  count(CNT_TC_LAUNCHES);
+  count(CNT_TC_LAUNCHES, a.x2 ? 2 : 1);
   if (pl.sk) count(CNT_SPLIT_REDUCTION);
   else if (pl.p.halo) count(CNT_COLUMN_STRIPS);
   if (a.pool2) count(CNT_POOLED);
+  if (a.x2) count(CNT_SUMMED);
 }
 
 // Launch without touching the runtime's state or any cache: the plan (tensor maps) is

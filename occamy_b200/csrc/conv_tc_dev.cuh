@@ -21,7 +21,7 @@ constexpr int TC_NSTORE = 2;         // tc_conv_kernel: slab-store threads (slab
 constexpr int TC_EPI_THREADS = 256;
 constexpr int TC_DBUF = 3;           // output slab buffers in shared memory
 constexpr int TC_MAX_TAPS = 64;
-constexpr int TC_MAX_AMAPS = 12;      // A tensor maps: 4 stride phases x 3 operand parts
+constexpr int TC_MAX_AMAPS = 5;       // A tensor maps: 4 stride phases, the second summand's
 constexpr int TC_SMEM_LIMIT = 232448;  // 227 KB
 constexpr size_t TC_SMEM_DUO = 113 * 1024;  // per CTA when two share an SM (1 KB each is reserved)
 
@@ -38,10 +38,14 @@ struct TcTap {
 struct alignas(64) TcParams {
   CUtensorMap tmA[TC_MAX_AMAPS];
   CUtensorMap tmB;
+  CUtensorMap tmB2;                    // weights of the second summand
   CUtensorMap tmD;
   CUtensorMap tmR;
   TcTap taps[TC_MAX_TAPS];
   int num_taps, cblocks, bk, stages;
+  int second_tap, cblocks2;            // tap that is the second summand (TcConvArgs::x2; else -1), its channel blocks
+  int ksteps;                          // of a tile
+  const float *bias2;                  // added to `bias`, or null
   int tiles_w, tiles_h, tiles_n, tiles_k, total_tiles;
   TcFastDiv div_k, div_w, div_h;   // divisions by tiles_k / tiles_w / tiles_h
   int tw, th, tn, K;
@@ -637,7 +641,11 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
   const int rows_valid = p.tw * p.th * p.tn;
-  const int ksteps = p.num_taps * p.cblocks;
+  const int ksteps = p.ksteps;
+  // a tap's channel blocks, weight map and place in it
+  auto blocks_of = [&](int t) { return t == p.second_tap ? p.cblocks2 : p.cblocks; };
+  auto map_b = [&](int t) { return t == p.second_tap ? &p.tmB2 : &p.tmB; };
+  auto tap_b = [&](int t) { return t == p.second_tap ? 0 : t; };
   int err_code = 0;
   // Everything above touched only this CTA's shared memory and TMEM, so it may overlap the
   // previous kernel in the stream.  Resident weights may be fetched early as well: the
@@ -666,8 +674,8 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
       for (int s = 0; s < pre_b; ++s) {
         // a lone loader arms the barrier for both operands here; of two, each arms its own
         mbar_expect_tx(full_bar(s), two_loaders ? b_bytes : (uint32_t)rows_valid * bk * 2u + b_bytes);
-        tma_load_3d(sB + s * b_bytes, &p.tmB, full_bar(s), cb * bk, tl.k0, t);
-        if (++cb == p.cblocks) {
+        tma_load_3d(sB + s * b_bytes, map_b(t), full_bar(s), cb * bk, tl.k0, tap_b(t));
+        if (++cb == blocks_of(t)) {
           cb = 0;
           ++t;
         }
@@ -713,7 +721,9 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
         const TcTile tl = tc_decode<BN, PAIR>(p, tile, rank);
         for (int t = 0; t < p.num_taps && !err_code; ++t) {
           const TcTap tap = p.taps[t];
-          for (int cb = 0; cb < p.cblocks; ++cb) {
+          const int blocks = blocks_of(t), tb = tap_b(t);
+          const CUtensorMap *mb = map_b(t);
+          for (int cb = 0; cb < blocks; ++cb) {
             if (!TCT_WAIT(0, mbar_wait_hot(empty_bar(stage), phase ^ 1u, abort_flag))) {
               err_code = 1;
               break;
@@ -723,8 +733,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
               // for the two of them; each CTA fetches its own pixels and its half of B.
               const uint32_t fb = cluster_map(full_bar(stage), 0);
               if (rank == 0) mbar_expect_tx(full_bar(stage), 2u * tx_bytes);
-              tma_load_3d_pair(sB + stage * b_bytes, &p.tmB, fb, cb * bk,
-                               tl.k0 + (int)rank * BROWS, t);
+              tma_load_3d_pair(sB + stage * b_bytes, mb, fb, cb * bk, tl.k0 + (int)rank * BROWS, tb);
               tma_load_4d_pair(sA + stage * a_bytes, &p.tmA[tap.map], fb, cb * bk, tl.q0 + tap.dw,
                                tl.p0 + tap.dh, tl.n0);
               if (++stage == stages) {
@@ -741,7 +750,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
               mbar_expect_tx(full_bar(stage), tx_bytes);   // the weights are resident
             } else {
               mbar_expect_tx(full_bar(stage), tx_bytes);
-              tma_load_3d(sB + stage * b_bytes, &p.tmB, full_bar(stage), cb * bk, tl.k0, t);
+              tma_load_3d(sB + stage * b_bytes, mb, full_bar(stage), cb * bk, tl.k0, tb);
             }
             tma_load_4d(sA + stage * a_bytes, &p.tmA[tap.map], full_bar(stage), cb * bk,
                         tl.q0 + tap.dw, tl.p0 + tap.dh, tl.n0);
@@ -996,7 +1005,9 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
       for (int tile = tile0; tile < p.total_tiles && !err_code; tile += tstep) {
         const TcTile tl = tc_decode<BN, PAIR>(p, tile, rank);
         for (int t = 0; t < p.num_taps && !err_code; ++t) {
-          for (int cb = 0; cb < p.cblocks; ++cb) {
+          const int blocks = blocks_of(t), tb = tap_b(t);
+          const CUtensorMap *mb = map_b(t);
+          for (int cb = 0; cb < blocks; ++cb) {
             if (pre_b > 0) {
               --pre_b;   // requested before the wait for the previous kernel
             } else {
@@ -1005,7 +1016,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
                 break;
               }
               mbar_expect_tx(full_bar(stage), b_bytes);
-              tma_load_3d(sB + stage * b_bytes, &p.tmB, full_bar(stage), cb * bk, tl.k0, t);
+              tma_load_3d(sB + stage * b_bytes, mb, full_bar(stage), cb * bk, tl.k0, tb);
             }
             if (++stage == stages) {
               stage = 0;
@@ -1042,7 +1053,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
     // The whole bias vector goes to shared memory once: a global load per tile would put
     // the memory latency on every tile's critical path.
     for (int i = et; i < p.bias_floats; i += EPI_THREADS)
-      bias_s[i] = (p.bias && i < p.K) ? p.bias[i] : 0.0f;
+      bias_s[i] = ((p.bias && i < p.K) ? p.bias[i] : 0.0f) + ((p.bias2 && i < p.K) ? p.bias2[i] : 0.0f);
     epi_bar_n<EPI_THREADS>();
     const float act_floor = p.floor, act_lo = p.lo, act_hi = p.hi;
     int acc = 0;

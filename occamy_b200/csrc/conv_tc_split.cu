@@ -252,19 +252,25 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
 
   // (tap, channel block) of a k-step of this CTA
   auto load_b = [&](int i, int s) {
-    const uint32_t t = tc_fdiv((uint32_t)(ks0 + i), p.div_cb);
+    const int k = ks0 + i;
+    const bool second = k >= p.ksteps1;
+    const int t = second ? 0 : (int)tc_fdiv((uint32_t)k, p.div_cb);
+    const CUtensorMap *m = second ? &p.tmB2 : &p.tmB;
+    const int c = (second ? k - p.ksteps1 : k - t * p.cblocks) * bk;
 #pragma unroll
     for (int j = 0; j < PARTS; ++j)
-      tma_load_3d(sB + s * b_bytes + j * b_tile, &p.tmB, full_bar(s), (ks0 + i - (int)t * p.cblocks) * bk, tl.k0,
-                  (int)t * PARTS + j);
+      tma_load_3d(sB + s * b_bytes + j * b_tile, m, full_bar(s), c, tl.k0, t * PARTS + j);
   };
   auto load_a = [&](int i, int s) {
-    const uint32_t t = tc_fdiv((uint32_t)(ks0 + i), p.div_cb);
+    const int k = ks0 + i;
+    const bool second = k >= p.ksteps1;
+    const int t = second ? 0 : (int)tc_fdiv((uint32_t)k, p.div_cb);
     const SkTap tap = p.taps[t];
+    const int map = second ? p.map2 : tap.map, c = (second ? k - p.ksteps1 : k - t * p.cblocks) * bk;
+    const int q = tl.q0 + (second ? 0 : tap.dw), h = tl.p0 + (second ? 0 : tap.dh);
 #pragma unroll
     for (int j = 0; j < PARTS; ++j)
-      tma_load_4d(sA + s * a_bytes + j * a_tile, &p.tmA[tap.map + j], full_bar(s),
-                  (ks0 + i - (int)t * p.cblocks) * bk, tl.q0 + tap.dw, tl.p0 + tap.dh, tl.n0);
+      tma_load_4d(sA + s * a_bytes + j * a_tile, &p.tmA[map + j], full_bar(s), c, q, h, tl.n0);
   };
   // The k-steps of the first ring turn are requested by one lane each: a single thread's chain of
   // index arithmetic, arming arrival and request per k-step is time on the layer's critical path.
@@ -290,7 +296,9 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   }
   if (warp >= 4) {   // (the other four warps issue MMAs)
     const int i = (int)threadIdx.x - 128;
-    if (i < BN) bias_s[i] = (p.bias && tl.k0 + i < p.K) ? p.bias[tl.k0 + i] : 0.0f;
+    if (i < BN)
+      bias_s[i] = ((p.bias && tl.k0 + i < p.K) ? p.bias[tl.k0 + i] : 0.0f) +
+                  ((p.bias2 && tl.k0 + i < p.K) ? p.bias2[tl.k0 + i] : 0.0f);
   }
   if (!F32 && !SPLIT && p.residual) {
     if constexpr (CL) {

@@ -7,16 +7,19 @@ namespace occ {
 constexpr int SK_THREADS = 256;
 constexpr int SK_MAX_SPLITS = 8;       // portable cluster size
 constexpr int SK_MAX_STAGES = 16;
+constexpr int SK_MAX_AMAPS = 15;       // A tensor maps: 4 stride phases and the second summand, 3 operand parts each
 
 struct SkTap {
   int8_t map, dw, dh, pad;
 };
 
 struct alignas(64) SkParams {
-  CUtensorMap tmA[TC_MAX_AMAPS];
+  CUtensorMap tmA[SK_MAX_AMAPS];
   CUtensorMap tmB;
+  CUtensorMap tmB2;                    // weights of the second summand
   SkTap taps[TC_MAX_TAPS];
-  int cblocks, bk, stages, ksteps;     // ksteps = taps * cblocks
+  int cblocks, bk, stages, ksteps;     // ksteps = taps * cblocks, and the second summand's
+  int ksteps1, map2;                   // k-steps before the second summand's (TcConvArgs::x2), its A map
   int issuers;                         // threads that issue MMAs: sk_issuers(), but no more than k-steps
   int splits;                          // CTAs (one cluster) that share a tile's reduction
   TcFastDiv div_k, div_w, div_h, div_cb;
@@ -26,7 +29,7 @@ struct alignas(64) SkParams {
   int rows_owner;                      // rows each CTA of the cluster sums up and stores
   int a_bytes;                         // bytes of an activation tile in a stage (multiple of 1024)
   int K, gq, gp, gn;
-  const float *bias;
+  const float *bias, *bias2;           // bias2 is added to bias (either may be null)
   const void *residual;                // in the form of y, or null
   void *y;                             // 16-bit NHWC output (when out_f32 is null); with split operands
                                        // three planes (hi, mid, lo) of `plane` elements each

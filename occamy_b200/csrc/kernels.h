@@ -173,6 +173,11 @@ struct TcConvArgs {
   int consts_ready;
   int form_n;            // images (a product: rows) whose form is taken, see form_images(); 0: its own
   int pool2;             // y is the 2x2 / stride 2 max pool of the result (tc_conv_takes_pool())
+  // A second summand (else x2 null): a 1x1 convolution without padding of another tensor onto the same
+  // output, y = act(x * w + bias + x2 * w2 + bias2) -- a block's projection shortcut.  No residual then.
+  const bf16 *x2, *w2;
+  const float *bias2;
+  int H2, W2, Cf2, stride2_h, stride2_w;
 };
 // ---- few-channel convolution fused with the 3x3 / stride 2 / pad 1 max pool after it -----
 struct StemPoolArgs {

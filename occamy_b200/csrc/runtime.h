@@ -87,7 +87,8 @@ enum Counter {
   CNT_POOLED = 11,
   CNT_REPLAYED = 12,
   CNT_IN_PIECES = 13,
-  CNT_COUNT = 14
+  CNT_SUMMED = 14,
+  CNT_COUNT = 15
 };
 
 struct Runtime {

@@ -149,7 +149,8 @@ void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles, std::ve
   // of every convolution: the last call folded into it, and the tensor that one writes
   std::vector<size_t> chain_last(rec.size(), 0);
   std::vector<uintptr_t> chain_out(rec.size(), 0);
-  std::vector<bool> chain_res(rec.size(), false);
+  std::vector<bool> chain_res(rec.size(), false), chain_act(rec.size(), false);
+  std::vector<size_t> chain_add(rec.size(), 0);   // the sum with another tensor
   for (size_t i = 0; i < rec.size(); ++i) {
     const Entry &c = rec[i];
     if (c.sym == S_D2D && (reader[i] = only_convs_read(rec, c.out, c.out_bytes, i + 1)) >= 0)
@@ -221,7 +222,7 @@ void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles, std::ve
       // skipping the write of `cur` is allowed only if this call was its sole reader
       if (f.out != cur && !dies_unread(rec, cur, cur_bytes, j + 1)) break;
       if (f.sym == S_TENSOR_OP && f.kind == CK_BIAS_ADD) bias_set = true;
-      else if (f.sym == S_TENSOR_OP) res_set = true;
+      else if (f.sym == S_TENSOR_OP) res_set = true, chain_add[i] = j;
       else act_set = true;
       members.push_back(j);
       cur = f.out;
@@ -247,6 +248,7 @@ void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles, std::ve
     chain_last[i] = members.empty() ? i : members.back();
     chain_out[i] = cur;
     chain_res[i] = res_set;
+    chain_act[i] = act_set;
     if (members.empty()) continue;
     roles[i] |= R_DEFER;
     for (size_t m : members) roles[m] |= R_ABSORB;
@@ -290,6 +292,40 @@ void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles, std::ve
     roles[i] = (uint8_t)(R_DEFER | RF_LINK);
     roles[j] = (uint8_t)(R_DEFER | RF_LINK | RF_JOIN);
     roles[k] = (uint8_t)(R_DEFER | RF_JOIN);
+  }
+  // Sums of two convolutions: the chain in front of one that ends in a sum is the other summand, nobody else
+  // reads it, and nothing but constants arriving lies between the two.
+  auto passive_past = [&](size_t from, size_t to, uintptr_t p, int64_t bytes) {   // [p, p+bytes) stays what it is
+    for (size_t t = from; t < to; ++t) {
+      const Entry &e = rec[t];
+      if (!is_passive(e.sym)) return false;
+      if (e.out && overlaps(e.out, e.out_bytes > 0 ? e.out_bytes : 1, p, bytes)) return false;
+    }
+    return true;
+  };
+  for (size_t i = 1; i < rec.size(); ++i) {
+    if (!chain_res[i]) continue;
+    const Entry &b = rec[i], &add = rec[chain_add[i]];
+    size_t a = i;
+    while (a > 0 && !((rec[a - 1].sym == S_CONV || rec[a - 1].sym == S_CONV_BIAS_ACT) && rec[a - 1].fusable)) --a;
+    if (a-- == 0) continue;
+    const Entry &c = rec[a];
+    const uintptr_t sum = chain_out[a];
+    if (c.depthwise || b.depthwise || c.parts != b.parts || chain_res[a] || chain_act[a] || !same_dims(c, b) ||
+        ((roles[a] | roles[i]) & (RF_LINK | RF_JOIN)) || !sum || (add.in[0] != sum && add.in[1] != sum) ||
+        !passive_past(chain_last[a] + 1, i, sum, c.out_bytes))
+      continue;
+    bool ok = true;
+    for (size_t t = i; t < chain_add[i] && ok; ++t) {   // the second chain up to the sum
+      const Entry &e = rec[t];
+      if (is_passive(e.sym)) ok = passive_past(t, t + 1, sum, c.out_bytes);
+      else if (overlaps(e.out, e.out_bytes, sum, c.out_bytes)) ok = false;
+      for (int k = 0; k < 3; ++k)
+        if (e.in[k] && overlaps(e.in[k], e.in_bytes[k] > 0 ? e.in_bytes[k] : 1, sum, c.out_bytes)) ok = false;
+    }
+    if (!ok || (add.out != sum && !dies_unread(rec, sum, c.out_bytes, chain_add[i] + 1))) continue;
+    roles[a] = (uint8_t)((roles[a] & ~ROLE_BITS) | R_DEFER | RF_SUM);
+    roles[i] |= RF_SUM;
   }
   for (size_t i = 0; i < rec.size(); ++i)   // (after the roles are known)
     if ((rec[i].parts || (roles[i] & ROLE_BITS) == R_ABSORB) &&

@@ -7,6 +7,7 @@
 //     convolution -> [+ bias [1,K,1,1]] -> [+ same-shape tensor] -> [ReLU | Clip]
 //     matrix product -> [+ bias row] -> [ReLU]
 //     1x1 convolution chain -> 3x3 depthwise chain -> 1x1 convolution chain
+//     convolution chain + convolution chain [-> ReLU | Clip]
 // (and, for a few-channel stem convolution, a 3x3 / stride 2 max pool behind it)
 // whose intermediate results nobody else reads before their memory is handed out again,
 // and marks them.  The next time the same call sequence comes by, the convolution of such
@@ -91,6 +92,9 @@ constexpr uint8_t RF_FOR_PARTS = 0x40;
 // an inverted residual, which become one kernel
 constexpr uint8_t RF_LINK = 0x04;
 constexpr uint8_t RF_JOIN = 0x08;
+// on two convolutions whose results are added, one chain behind the other: the first is held back until the sum
+// comes by, which one kernel then computes (a block's last convolution and its projection shortcut)
+constexpr uint8_t RF_SUM = 0x80;
 constexpr uint8_t ROLE_BITS = 0x03;
 struct TraceProgram {
   std::vector<uint64_t> sigs;
