@@ -204,7 +204,7 @@ cudaStream_t occamy_stream(void);
  * [7] fp32 CUDA-core conv/GEMM launches. */
 void occamy_get_counters(int64_t out[8]);
 /* Which forms the work took since load, the first n of: [0] split-reduction launches, [1] inverted
- * residuals as one kernel, [2] 3x3 layers on 64 channels as column strips, [3] convolutions that took a
+ * residuals as one kernel, [2] 3x3 layers as column strips, [3] convolutions that took a
  * 2x2 max pool along, [4] inferences whose recorded part ran as graphs, [5] such that were computed in
  * pieces while their batch arrived, [6] convolutions that took another one's result along as a second
  * summand.  Returns how many there are. */

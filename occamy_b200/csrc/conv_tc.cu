@@ -470,6 +470,7 @@ struct Plan {
   int bn;
   int dc;    // channels per output slab
   bool pn;   // pixel-N variant
+  bool wide; // pixel-N variant on input blocks (conv_tc_wide.cu)
   bool pair; // CTA-pair form: the grid is launched as clusters of two
   bool duo;  // two independent CTAs per SM (one epilogue warp per TMEM quadrant)
   bool sk;   // split-reduction kernel (conv_tc_split.cu): `s` instead of `p`
@@ -513,6 +514,11 @@ static int parts_bk(int Cf) { return Cf > 16 ? 32 : 16; }
 static bool is_flat(const TcConvArgs &a) {
   return a.R == 1 && a.S == 1 && a.stride_h == 1 && a.stride_w == 1 && a.pad_h == 0 && a.pad_w == 0 && a.w_step == 0 &&
          (!a.x2 || (a.stride2_h == 1 && a.stride2_w == 1));
+}
+// 3x3, stride 1, an output as large as the input.
+static bool is_3x3_same(const TcConvArgs &a) {
+  return a.R == 3 && a.S == 3 && a.stride_h == 1 && a.stride_w == 1 && a.pad_h == 1 && a.pad_w == 1 && a.w_step == 0 &&
+         a.Q == a.W && a.P == a.H;
 }
 // Multiply-adds per output value, in the 64-channel k-steps the rules count in.
 static int reduction64(const TcConvArgs &a) { return (a.R * a.S * a.Cf + (a.x2 ? a.Cf2 : 0) + 63) / 64; }
@@ -691,6 +697,42 @@ static void pool_box(int Q, int P, int N, int *tw, int *th, int *tn) {
     }
 }
 
+// A layer of the wide form: strips of columns, whose pixels and the two columns between their rows are the N side (at
+// most 256).  The cheapest cover of the image, by tiles per SM and cycles of a tile (two per column of an MMA and tap,
+// and what a tile costs by itself).  False when none fits shared memory.
+static bool wide_box(const TcConvArgs &a, int nsm, TcParams *p, size_t *smem) {
+  const int even = a.pool2 ? 2 : 1, cblocks = a.Cf / 64;
+  double best = -1.0;
+  for (int n = 1; n <= (a.W + 7) / 8; ++n) {
+    const int tw = ((a.W + n - 1) / n + even - 1) / even * even, wp = tw + 2, c16 = (tw + 15) / 16 * 16;
+    if (c16 > 256 || wp > 256) continue;
+    int most = (256 - c16) / wp + 1;
+    if (most > a.P) most = a.P;
+    most = (most + even - 1) / even * even;
+    for (int th = most; th >= even; th -= even) {
+      if ((th - 1) * wp + c16 > 256) continue;
+      const long rows = (a.P + th - 1) / th;
+      const int x_bytes = ((th + 2) * wp * 128 + 1023) / 1024 * 1024;
+      const int slab = (tw * th * 128 / (even * even) + 1023) / 1024 * 1024;
+      const size_t bytes = tc_wide_smem(x_bytes, (a.K + 63) / 64, slab);
+      if (bytes > (size_t)TC_SMEM_LIMIT) continue;
+      const int n_mma = ((th - 1) * wp + tw + 15) / 16 * 16;
+      const long tiles = rows * ((a.W + tw - 1) / tw) * a.N;
+      const double cost = (double)((tiles + nsm - 1) / nsm) * (9.0 * cblocks * (2.0 * n_mma + 80.0) + 1500.0);
+      if (best >= 0 && cost >= best) continue;
+      best = cost;
+      p->tw = tw; p->th = th; p->tn = 1;
+      p->halo_wp = wp;
+      p->halo_a_bytes = x_bytes;
+      p->wide_slab_bytes = slab;
+      *smem = bytes;
+    }
+  }
+  if (best < 0) return false;
+  p->halo = 1;
+  return true;
+}
+
 static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, double rival, const SkChoice *form,
                     Plan *pl) {
 #ifdef OCCAMY_TUNING
@@ -848,14 +890,20 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   // than the plain one, which hurts the HBM-bound 1x1 layers
   // 3x3 / stride 1 / pad 1 with 64 -> 64 channels: the input block of a tile is loaded once and the taps are
   // windows of it (TC_MODE_HALO)
-  const bool halo = allow_halo && halo_allowed && !a.f16 && !a.out_f32 && !a.x2 && a.R == 3 && a.S == 3 &&
-                    a.stride_h == 1 && a.stride_w == 1 && a.pad_h == 1 && a.pad_w == 1 &&
-                    a.Cf == 64 && a.K == 64 && a.w_step == 0 && a.Q == a.W &&
-                    a.P == a.H;
-  const bool pn = !halo && pn_allowed && !a.f16 && !a.out_f32 && !a.x2 && a.K <= 128 && a.R * a.S > 1 &&
-                  a.R * a.S * a.Cf >= 9 * 64;
+  const bool halo = allow_halo && halo_allowed && !a.f16 && !a.out_f32 && !a.x2 && is_3x3_same(a) && a.Cf == 64 &&
+                    a.K == 64;
+  const int nsm = num_sms > 0 ? num_sms : 148;
+  const bool few = !halo && pn_allowed && !a.f16 && !a.out_f32 && !a.x2 && a.K <= 128 && a.R * a.S > 1 &&
+                   a.R * a.S * a.Cf >= 9 * 64;
+  // Of the layers with few channels, the 3x3 ones of stride 1 go to the wide form (figures there); others, and those
+  // with a shortcut tensor, to the form whose k-steps load their pixels one by one.
+  const bool wide = few && allow_halo && halo_allowed && is_3x3_same(a) && a.Cf % 64 == 0 && !a.residual &&
+                    wide_box(a, nsm, &p, &pl.smem);
+  const bool pn = few && !wide && !a.pool2;
   pl.pn = pn;
-  if (halo && a.pool2) {
+  pl.wide = wide;
+  if (wide) {   // (the box is chosen)
+  } else if (halo && a.pool2) {
     p.tw = 14;   // 16 lanes to an input row
     p.th = 8;
     p.tn = 1;
@@ -886,12 +934,11 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   } else {
     choose_box(Qg, Pg, Ng, pn ? 256 : 128, &p.tw, &p.th, &p.tn);
   }
-  p.n_mma = (p.tw * p.th * p.tn + 15) / 16 * 16;
+  p.n_mma = ((wide ? (p.th - 1) * p.halo_wp + p.tw : p.tw * p.th * p.tn) + 15) / 16 * 16;
   p.tiles_w = (Qg + p.tw - 1) / p.tw;
   p.tiles_h = (Pg + p.th - 1) / p.th;
   p.tiles_n = (Ng + p.tn - 1) / p.tn;
-  const int nsm = num_sms > 0 ? num_sms : 148;
-  const int bn = pn ? 128
+  const int bn = pn || wide ? 128
                     : halo ? 64
                     : pick_bn(a.K, (long)p.tiles_w * p.tiles_h * p.tiles_n,
                               reduction64(a), nsm);
@@ -908,11 +955,11 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   // Measured on ResNet-50 at batch 256: 5-8 % faster on the 1x1 layers with 1024 and 2048
   // input channels, 3-4 % on the 3x3 layers with 256 and 512 channels, 25 % slower on
   // reductions of four steps: taken for reductions of 16 k-steps and more.
-  bool pair = pair_allowed && !pn && !halo && !a.out_f32 && bn == 256 && ksteps64p >= 16 &&
+  bool pair = pair_allowed && !pn && !wide && !halo && !a.out_f32 && bn == 256 && ksteps64p >= 16 &&
               p.sp_tiles >= 2 && nsm >= 2;
 #ifdef OCCAMY_TUNING
   if (getenv("OCCAMY_TC_PAIR") && !strcmp(getenv("OCCAMY_TC_PAIR"), "2"))   // every 256-channel tile
-    pair = !pn && !halo && !a.out_f32 && !a.split && bn == 256 && p.sp_tiles >= 2 && nsm >= 2;
+    pair = !pn && !wide && !halo && !a.out_f32 && !a.split && bn == 256 && p.sp_tiles >= 2 && nsm >= 2;
 #endif
   pl.pair = pair;
   p.total_tiles = (pair ? (p.sp_tiles + 1) / 2 : p.sp_tiles) * p.tiles_k;
@@ -927,13 +974,13 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
     const int per_wave = pair ? nsm / 2 : nsm;
     const double waves = (double)((p.total_tiles + per_wave - 1) / per_wave);
     const int ks = p.cblocks * a.R * a.S + p.cblocks2;
-    const double tile_us = halo ? 0.9 : pn ? 0.49 * ks : (bn == 256 ? 0.1 : 0.0) + 0.27 * ks * (bk == 64 ? 1.0 : 0.75);
+    const double tile_us = halo ? 0.9 : wide ? (0.05 + 0.0011 * p.n_mma) * ks : pn ? 0.49 * ks : (bn == 256 ? 0.1 : 0.0) + 0.27 * ks * (bk == 64 ? 1.0 : 0.75);
     if (!a.pool2 && (!piece || form) && sk_plan(a, err_word, nsm, counted, 3.1 + waves * tile_us, form, &pl)) return pl;
-    if (a.pool2 && !halo && !pair) return pl;   // (not ok: tc_conv_takes_pool() said so)
+    if (a.pool2 && !halo && !wide && !pair) return pl;   // (not ok: tc_conv_takes_pool() said so)
   }
   const uint32_t boxA[4] = {(uint32_t)bk, (uint32_t)p.tw, (uint32_t)p.th, (uint32_t)p.tn};
   bool ok = true;
-  if (halo) {
+  if (halo || wide) {
     const uint64_t dims[4] = {(uint64_t)a.Cf, (uint64_t)a.W, (uint64_t)a.H, (uint64_t)a.N};
     const uint64_t st[3] = {(uint64_t)a.Cf * 2, (uint64_t)a.W * a.Cf * 2, (uint64_t)a.H * a.W * a.Cf * 2};
     const uint32_t box[4] = {64u, (uint32_t)p.halo_wp, (uint32_t)(p.th + 2), 1u};
@@ -954,7 +1001,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   // For 256-wide tiles with a long reduction, 32-channel slabs free enough shared memory
   // for a fourth ring stage, which those layers need more than a cheap epilogue.
   const int ksteps64 = reduction64(a);
-  int dc = pn ? 64 : (bn < 64 ? bn : (bn == 256 && bk == 64 && ksteps64 >= 16 ? 32 : 64));
+  int dc = pn || wide ? 64 : (bn < 64 ? bn : (bn == 256 && bk == 64 && ksteps64 >= 16 ? 32 : 64));
   if (bn == 64 && a.w_step && a.R <= 3 && !pn && !halo && !a.out_f32 && nsm >= 2) dc = 32;   // few-channel stems: two CTAs per SM, below
   if (a.out_f32 && bn >= 64) dc = 64;   // the fp32-output flavour is compiled for 64-channel slabs
 #ifdef OCCAMY_TUNING
@@ -976,6 +1023,11 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
     const uint32_t box[4] = {(uint32_t)dc, (uint32_t)(p.tw / half), (uint32_t)(p.th / half), (uint32_t)p.tn};
     ok &= make_map(&p.tmD, a.y, 4, dims, st, box, dc * 2, counted);
     if (a.residual) ok &= make_map(&p.tmR, a.residual, 4, dims, st, box, dc * 2, counted);
+  }
+  if (wide) {
+    if (!ok) return build_plan(a, err_word, num_sms, counted, false);   // e.g. the block map was refused
+    pl.ok = true;
+    return pl;
   }
   // One channel tile: every tile multiplies by the same weights.  If they are tiny they are
   // fetched once per CTA into an area of their own instead of once per tile into the ring: all
@@ -1084,10 +1136,9 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
 // Whether a 2x2 / stride 2 max pool behind this convolution is better taken along.
 bool tc_conv_takes_pool(TcConvArgs a) {
   if (a.P < 2 || a.Q < 2 || a.split || a.out_f32 || a.residual || a.w_step || a.K % 8 || !tc_conv_supported(a)) return false;
-  const bool halo = !a.f16 && a.R == 3 && a.S == 3 && a.stride_h == 1 && a.stride_w == 1 && a.pad_h == 1 &&
-                    a.pad_w == 1 && a.Cf == 64 && a.K == 64;
+  const bool strips = !a.f16 && is_3x3_same(a) && a.Cf % 64 == 0 && a.K <= 128;
   const bool flat = a.R == 1 && a.S == 1;
-  if (flat || (!halo && (a.K % 256 || a.R * a.S * a.Cf < 16 * 64))) return false;
+  if (flat || (!strips && (a.K % 256 || a.R * a.S * a.Cf < 16 * 64))) return false;
   const Plan alone = build_plan(a, nullptr, rt().num_sms, false);
   if (!alone.ok || alone.sk || !(alone.p.halo || alone.pair)) return false;
   a.pool2 = 1;
@@ -1112,6 +1163,11 @@ static void launch_any(const Plan &pl, int num_sms, cudaStream_t s) {
   }
   if (pl.pn) {
     launch_plan_pn(pl, num_sms, s);
+    return;
+  }
+  if (pl.wide) {
+    tc_launch_wide(pl.p, (pl.mode & TC_MODE_CLAMP) != 0, (pl.mode & TC_MODE_POOL) != 0,
+                   pl.p.total_tiles < num_sms ? pl.p.total_tiles : num_sms, pl.smem, s);
     return;
   }
   int grid = pl.p.total_tiles < num_sms ? pl.p.total_tiles : num_sms;

@@ -23,6 +23,8 @@ constexpr int TC_DBUF = 3;           // output slab buffers in shared memory
 constexpr int TC_MAX_TAPS = 64;
 constexpr int TC_MAX_AMAPS = 5;       // A tensor maps: 4 stride phases, the second summand's
 constexpr int TC_SMEM_LIMIT = 232448;  // 227 KB
+constexpr int WD_THREADS = 384;      // wide form (conv_tc_wide.cu)
+constexpr int WD_MISC_BYTES = 256;
 constexpr size_t TC_SMEM_DUO = 113 * 1024;  // per CTA when two share an SM (1 KB each is reserved)
 
 // Division of a tile index (< 2^31) by a positive constant: q = umulhi(x, mul) >> shift,
@@ -72,7 +74,8 @@ struct alignas(64) TcParams {
 #ifdef OCCAMY_TC_TIMERS
   long long *timers;     // 5 roles x 4 counters, or null
 #endif
-  int n_mma;             // pixel-N variant: N of the MMA (pixels per tile rounded up to 16)
+  int n_mma;             // pixel-N variants: N of the MMA (pixels per tile rounded up to 16)
+  int wide_slab_bytes;   // wide form: 64 channels of a tile's pixels
   int sp_tiles;          // pixel tiles (tiles_w * tiles_h * tiles_n); with TC_MODE_PAIR the tile
                          // index counts PAIRS of them and total_tiles = ceil(sp_tiles / 2) * tiles_k
   int descending;        // tiles are taken from the last to the first (Runtime::descending)
@@ -1245,6 +1248,9 @@ bool tc_launch_128_64(const TcParams &p, int mode, int grid, size_t smem, cudaSt
 bool tc_launch_64_64(const TcParams &p, int mode, int grid, size_t smem, cudaStream_t s);
 bool tc_launch_32_32(const TcParams &p, int mode, int grid, size_t smem, cudaStream_t s);
 bool tc_launch_32_32_duo(const TcParams &p, int mode, int grid, size_t smem, cudaStream_t s);
+// the wide form (conv_tc_wide.cu): weights on the M side, input blocks; its shared memory
+void tc_launch_wide(const TcParams &p, bool clamp, bool pool, int grid, size_t smem, cudaStream_t s);
+size_t tc_wide_smem(int x_bytes, int slabs, int slab_bytes);
 bool tc_launch_64_32_duo(const TcParams &p, int mode, int grid, size_t smem, cudaStream_t s);
 
 // Launch with programmatic stream serialisation (see pdl_wait); `cluster` > 1 launches the
