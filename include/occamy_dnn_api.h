@@ -199,7 +199,7 @@ cudaStream_t occamy_stream(void);
 /* Counters since load: [0] kernel launches, [1] bytes uploaded host->device,
  * [2] bytes of uploads skipped because the packed weight was already resident,
  * [3] pool high-water mark in bytes, [4] tensor-core conv/GEMM launches (one that takes a second
- * convolution along as a summand counts for both),
+ * convolution along counts for both),
  * [5] layout materialisations (NHWC bf16 -> NCHW fp32), [6] tensor-map encodes,
  * [7] fp32 CUDA-core conv/GEMM launches. */
 void occamy_get_counters(int64_t out[8]);
@@ -207,7 +207,7 @@ void occamy_get_counters(int64_t out[8]);
  * residuals as one kernel, [2] 3x3 layers as column strips, [3] convolutions that took a
  * 2x2 max pool along, [4] inferences whose recorded part ran as graphs, [5] such that were computed in
  * pieces while their batch arrived, [6] convolutions that took another one's result along as a second
- * summand.  Returns how many there are. */
+ * summand, [7] pairs of layers as one kernel.  Returns how many there are. */
 int occamy_get_form_counters(int64_t *out, int n);
 /* Per-launch timing of the tensor-core convolution / GEMM kernel: after _begin, every such
  * launch is bracketed by a CUDA-event pair on the launch stream; _end waits for the stream,

@@ -21,7 +21,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 RUNTIME_SRCS = ["runtime.cu", "kernels_f32.cu", "kernels_nhwc.cu", "kernels_parts.cu", "conv_tc.cu", "conv_tc_inst_256_64.cu",
                 "conv_tc_inst_256_32.cu", "conv_tc_inst_128_64.cu", "conv_tc_inst_64_64.cu",
-                "conv_tc_inst_32_32.cu", "conv_tc_split.cu", "conv_tc_wide.cu", "inverted_residual.cu", "stem_pool.cu", "trace.cu", "graph_replay.cu", "abi.cu", "misc_ops.cu", "no_alloc.cu",
+                "conv_tc_inst_32_32.cu", "conv_tc_split.cu", "conv_tc_wide.cu", "conv_pair.cu", "inverted_residual.cu", "stem_pool.cu", "trace.cu", "graph_replay.cu", "abi.cu", "misc_ops.cu", "no_alloc.cu",
                 os.path.join("host", "fingerprint.cpp")]
 REPLAY_SRCS = [os.path.join("host", "replay.cpp")]
 

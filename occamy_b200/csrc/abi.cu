@@ -220,6 +220,8 @@ struct ConvJob {
   bool linked = false, joined = false;
   // held back until a sum takes its result along (RF_SUM) / the other summand, which g_front[0] still is
   bool summand = false, after_summand = false;
+  // its result is read by the convolution behind it (RF_LEAD) / the one in front, g_front[0], writes its input
+  bool leads = false, follows = false;
   // (the constants of one once more, packed_for_block(): a first bias, a depthwise filter and bias)
   const void *block_w = nullptr, *block_b = nullptr;
   // folded (few-channel) form: what the fused convolution + pool kernel needs besides `a`
@@ -232,7 +234,7 @@ int g_fronts = 0;
 const ConvJob *g_launching = nullptr;   // job whose output buffer is being looked for
 
 bool job_reads(const ConvJob &j, const void *home) {
-  return j.a.x == home || j.a.x2 == home || j.a.residual == home || j.dw_x == home;
+  return j.a.x == home || j.a.y == home || j.a.x2 == home || j.a.residual == home || j.dw_x == home;
 }
 bool home_held_hook(const void *home) {
   for (int i = 0; i < g_fronts; ++i)
@@ -627,6 +629,39 @@ void launch_summand() {
   g_fronts = 0;
 }
 
+// A convolution and the one behind it that reads its result as one kernel; false when they have to run one by one.
+bool launch_two(ConvJob &a, ConvJob &b) {
+  a.a.act = a.g.act;
+  b.a.act = b.g.act;
+  if (a.depthwise || b.depthwise || a.product || b.product || !tc_pair_supported(a.a, b.a)) return false;
+  const size_t ybytes = (size_t)a.g.N * a.g.K * a.g.P * a.g.Q * 2, tbytes = (size_t)b.g.N * b.g.K * b.g.P * b.g.Q * 2;
+  // neither result may land on what other tiles have still to read; the shortcut tensor's place, exactly, is
+  // as good as any (each tile reads its part before it stores)
+  auto clash = [&](const void *p, size_t bytes, const ConvJob &j, bool in_place_ok) {
+    const uintptr_t lo = (uintptr_t)p, hi = lo + bytes;
+    for (int k = 0; k < 5; ++k)
+      if (ranges_overlap(lo, hi, j.dep_lo[k], j.dep_hi[k]) &&
+          !(in_place_ok && k == 1 && lo == j.dep_lo[k] && hi == j.dep_hi[k]))
+        return true;
+    return false;
+  };
+  void *y = a.out, *t = b.out;
+  if (clash(y, ybytes, a, true) || clash(y, ybytes, b, false)) y = home_acquire(ybytes);
+  if (!y) return false;
+  a.a.y = (bf16 *)y;
+  const uintptr_t ylo = (uintptr_t)y;
+  if (clash(t, tbytes, a, false) || clash(t, tbytes, b, false) ||
+      ranges_overlap((uintptr_t)t, (uintptr_t)t + tbytes, ylo, ylo + ybytes))
+    t = home_acquire(tbytes);
+  if (!t) return false;
+  b.a.y = (bf16 *)t;
+  b.a.x = nullptr;
+  if (!launch_tc_pair(a.a, b.a, rt().stream)) return false;
+  mark_act16(a.out, a.g.N, a.g.K, a.g.P, a.g.Q, y == a.out ? nullptr : y);
+  mark_act16(b.out, b.g.N, b.g.K, b.g.P, b.g.Q, t == b.out ? nullptr : t);
+  return true;
+}
+
 // Executes the held-back convolution as far as it has been built up.
 void flush_pending() {
   if (!g_pending.active) return;
@@ -635,6 +670,21 @@ void flush_pending() {
     if (g_front[i].absorbed) trace_count_chain();
   if (g_pending.absorbed && !g_pending.product) trace_count_chain();   // convolution chains
   launch_summand();
+  if (g_pending.follows) {
+    g_pending.follows = false;
+    ConvJob &lead = g_front[0];
+    if (!launch_two(lead, g_pending)) {
+      launch_job(lead);
+      g_pending.a.x = act16_ptr(lead.out);
+      if ((const void *)g_pending.a.x == lead.out) {
+        g_pending.dep_lo[0] = (uintptr_t)lead.out;
+        g_pending.dep_hi[0] = (uintptr_t)lead.out + (size_t)lead.g.N * lead.g.K * lead.g.P * lead.g.Q * 2;
+      }
+      launch_job(g_pending);
+    }
+    g_fronts = 0;
+    return;
+  }
   if (g_fronts != 2 || !launch_block(g_front[0], g_front[1], g_pending)) {
     const bf16 *x = nullptr;
     auto resolve = [&](ConvJob &job) {
@@ -680,7 +730,7 @@ void pending_guard_range(const void *p, size_t bytes, bool writes) {
     const size_t elem = job.a.split || job.product ? 4 : 2;
     return ranges_overlap(lo, hi, olo, olo + (size_t)job.g.N * job.g.K * job.g.P * job.g.Q * elem);
   };
-  if (takes_output(g_pending) || (g_pending.after_summand && takes_output(g_front[0]))) {
+  if (takes_output(g_pending) || ((g_pending.after_summand || g_pending.follows) && takes_output(g_front[0]))) {
     if (rt().log) fprintf(stderr, "[occamy] held-back conv runs early: output re-handed out\n");
     flush_pending();
   }
@@ -712,7 +762,8 @@ Role step(Entry &e, bool passive) {
       fprintf(stderr, "[occamy] call sequence left the recorded one after tensors were skipped\n");
   }
   if (!passive && role != R_ABSORB && !((trace_last_flags() & RF_JOIN) && g_pending.active && g_pending.linked) &&
-      !((trace_last_flags() & RF_SUM) && g_pending.active && g_pending.summand)) {
+      !((trace_last_flags() & RF_SUM) && g_pending.active && g_pending.summand) &&
+      !((trace_last_flags() & RF_FOLLOW) && g_pending.active && g_pending.leads)) {
     if (g_pending.active && rt().log)
       fprintf(stderr, "[occamy] held-back conv closed by call sym %d (absorbed %d)\n", e.sym,
               g_pending.absorbed);
@@ -843,9 +894,14 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
                g.S <= 16 && g.R <= 11;
   const Role role = step(e, false);
   if (role == R_SKIP) return y;
-  const uint8_t flags = trace_last_flags();
-  bool join = false, sum = false;
-  if (g_pending.active && g_pending.summand) {   // left by step(): this call was recorded as the other summand
+  const uint16_t flags = trace_last_flags();
+  bool join = false, sum = false, follow = false;
+  if (g_pending.active && g_pending.leads) {   // left by step(): this call was recorded as reading its result
+    const ConvGeom &f = g_pending.g;
+    follow = role == R_DEFER && e.fusable && !e.parts && !depthwise && stays_packed(w) && !g_fronts && g_pending.out == x &&
+             f.N == g.N && f.K == g.C && f.P == g.H && f.Q == g.W && g.C % 16 == 0;
+    if (!follow) flush_pending();
+  } else if (g_pending.active && g_pending.summand) {   // left by step(): this call was recorded as the other summand
     const ConvGeom &f = g_pending.g;
     sum = role == R_DEFER && e.fusable && !depthwise && e.parts == (g_pending.a.split != 0) && f.N == g.N && f.K == g.K &&
           f.P == g.P && f.Q == g.Q && !g_pending.act_set && !g_pending.res_set;
@@ -881,10 +937,20 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
     ConvJob job;
     // (the first of three takes its input as it is)
     job.linked = role == R_DEFER && (flags & RF_LINK) && stays_packed(w) && (join || (!(flags & RF_JOIN) && is_act16(x, g.N, g.C, g.H, g.W)));
-    job.joined = join;
+    job.joined = join || follow;
+    job.leads = role == R_DEFER && (flags & RF_LEAD) && !depthwise && stays_packed(w);
     bool ok = depthwise ? prepare_depthwise(x, w, bias, g, job)
                         : (g.groups == 1 && prepare_dense(x, w, bias, g, job));
-    if (join && ok && g_pending.active) {
+    if (follow && ok && g_pending.active) {
+      g_front[0] = g_pending;
+      g_fronts = 1;
+      job.joined = false;
+      job.follows = true;
+    } else if (follow) {   // (an upload had to run it, or this one is not taken)
+      flush_pending();
+      job = ConvJob();
+      ok = prepare_dense(x, w, bias, g, job);
+    } else if (join && ok && g_pending.active) {
       // nothing else reads what the one in front would have written
       g_front[g_fronts++] = g_pending;
       elide(g_pending.out);
@@ -1313,7 +1379,7 @@ float *DNNActiveFunc(cudnnContext *, float *x, int64_t dimX[4], int32_t mode, fl
       pending_retarget(y);
       g_pending.g.act = ACT_RELU;
       g_pending.act_set = true;
-      if (!g_pending.linked) flush_pending();   // an activation closes the chain
+      if (!g_pending.linked && !g_pending.leads) flush_pending();   // an activation closes the chain
       return y;
     }
     flush_pending();

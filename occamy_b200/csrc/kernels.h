@@ -227,6 +227,9 @@ void launch_selftest_bounded_wait(cudaStream_t s);
 bool tc_conv_supported(const TcConvArgs &a);
 bool tc_conv_takes_pool(TcConvArgs a);
 void launch_tc_conv(const TcConvArgs &a, cudaStream_t s);
+// Two layers as one kernel (conv_pair.cu): `b` is a 1x1 convolution of what `a` writes (b.x is not looked at).
+bool tc_pair_supported(const TcConvArgs &a, const TcConvArgs &b);
+bool launch_tc_pair(const TcConvArgs &a, const TcConvArgs &b, cudaStream_t s);
 // Same kernel, no runtime state, no caches, no allocation; false when the plan fails.
 bool launch_tc_conv_stateless(const TcConvArgs &a, int *err_word, int num_sms, cudaStream_t s);
 

@@ -88,7 +88,8 @@ enum Counter {
   CNT_REPLAYED = 12,
   CNT_IN_PIECES = 13,
   CNT_SUMMED = 14,
-  CNT_COUNT = 15
+  CNT_PAIRS = 15,
+  CNT_COUNT = 16
 };
 
 struct Runtime {

@@ -25,7 +25,7 @@ struct TraceState {
   size_t pool_bytes = 0;
   uintptr_t last_pool_base = 0;   // the pool of this inference, also after it was given back
   size_t last_pool_bytes = 0;
-  uint8_t last_flags = 0;
+  uint16_t last_flags = 0;
   int forced = -1;               // role of the next call, see trace_force()
   int elided = 0;
   int64_t fused_chains = 0;
@@ -118,7 +118,7 @@ int only_convs_read(const std::vector<Entry> &rec, uintptr_t p, int64_t bytes, s
 // True when everything that reads [p, p+bytes) from entry `from` on, until the range is handed out again
 // or freed, takes fp32 values in three planes: dense convolutions of fp32 mode, sums folded into one,
 // pools and means.
-bool only_parts_read(const std::vector<Entry> &rec, const std::vector<uint8_t> &roles, uintptr_t p, int64_t bytes,
+bool only_parts_read(const std::vector<Entry> &rec, const std::vector<uint16_t> &roles, uintptr_t p, int64_t bytes,
                      size_t from) {
   bool any = false;
   for (size_t t = from; t < rec.size(); ++t) {
@@ -143,7 +143,7 @@ bool only_parts_read(const std::vector<Entry> &rec, const std::vector<uint8_t> &
 
 // Marks the chains of a finished inference: R_DEFER on the convolution, R_ABSORB on the
 // calls folded into it.
-void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles, std::vector<int> &reader) {
+void analyse(const std::vector<Entry> &rec, std::vector<uint16_t> &roles, std::vector<int> &reader) {
   roles.assign(rec.size(), R_EAGER);
   reader.assign(rec.size(), -1);
   // of every convolution: the last call folded into it, and the tensor that one writes
@@ -289,9 +289,9 @@ void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles, std::ve
     if (!ir_supported((int)v[0], (int)v[1], (int)v[4], (int)rec[k].args.v[4], (int)v[2], (int)v[3],
                       (int)rec[k].dims[2], (int)rec[k].dims[3], (int)w[10], mode_f16()))
       continue;
-    roles[i] = (uint8_t)(R_DEFER | RF_LINK);
-    roles[j] = (uint8_t)(R_DEFER | RF_LINK | RF_JOIN);
-    roles[k] = (uint8_t)(R_DEFER | RF_JOIN);
+    roles[i] = (uint16_t)(R_DEFER | RF_LINK);
+    roles[j] = (uint16_t)(R_DEFER | RF_LINK | RF_JOIN);
+    roles[k] = (uint16_t)(R_DEFER | RF_JOIN);
   }
   // Sums of two convolutions: the chain in front of one that ends in a sum is the other summand, nobody else
   // reads it, and nothing but constants arriving lies between the two.
@@ -324,8 +324,23 @@ void analyse(const std::vector<Entry> &rec, std::vector<uint8_t> &roles, std::ve
         if (e.in[k] && overlaps(e.in[k], e.in_bytes[k] > 0 ? e.in_bytes[k] : 1, sum, c.out_bytes)) ok = false;
     }
     if (!ok || (add.out != sum && !dies_unread(rec, sum, c.out_bytes, chain_add[i] + 1))) continue;
-    roles[a] = (uint8_t)((roles[a] & ~ROLE_BITS) | R_DEFER | RF_SUM);
+    roles[a] = (uint16_t)((roles[a] & ~ROLE_BITS) | R_DEFER | RF_SUM);
     roles[i] |= RF_SUM;
+  }
+  // A block's last convolution and the next block's first.
+  for (size_t i = 0; i < rec.size(); ++i) {
+    const Entry &c = rec[i];
+    if (!chain_res[i] || !chain_act[i] || c.depthwise || c.parts || (roles[i] & (RF_LINK | RF_JOIN)) || c.dims[1] % 128)
+      continue;
+    size_t j = chain_last[i] + 1;
+    while (j < rec.size() && is_passive(rec[j].sym)) ++j;
+    if (j == rec.size() || (rec[j].sym != S_CONV && rec[j].sym != S_CONV_BIAS_ACT)) continue;
+    const Entry &f = rec[j];
+    if (!f.fusable || f.parts || !one_by_one(f) || f.in[0] != chain_out[i] || f.in_bytes[0] != c.out_bytes || chain_res[j] ||
+        !chain_act[j] || (roles[j] & (RF_LINK | RF_JOIN | RF_SUM)) || !passive_past(chain_last[i] + 1, j, chain_out[i], c.out_bytes))
+      continue;
+    roles[i] |= RF_LEAD;
+    roles[j] = (uint16_t)((roles[j] & ~ROLE_BITS) | R_DEFER | RF_FOLLOW);
   }
   for (size_t i = 0; i < rec.size(); ++i)   // (after the roles are known)
     if ((rec[i].parts || (roles[i] & ROLE_BITS) == R_ABSORB) &&
@@ -402,7 +417,7 @@ void te_dims(Entry &e, const int64_t *d, int n) {
   for (int i = 0; i < n; ++i) mix(e.sig, (uint64_t)d[i]);
 }
 
-void trace_force(uint8_t role) { g_ts.forced = role; }
+void trace_force(uint16_t role) { g_ts.forced = role; }
 void trace_force_end() { g_ts.forced = -1; }
 
 Role trace_step(Entry &e, bool *deviated) {
@@ -410,7 +425,7 @@ Role trace_step(Entry &e, bool *deviated) {
   TraceState &ts = g_ts;
   ts.last_flags = 0;
   if (ts.forced >= 0) {
-    ts.last_flags = (uint8_t)(ts.forced & ~ROLE_BITS);
+    ts.last_flags = (uint16_t)(ts.forced & ~ROLE_BITS);
     return (Role)(ts.forced & ROLE_BITS);
   }
   if (!trace_enabled() || !ts.in_inference) return R_EAGER;
@@ -433,9 +448,9 @@ Role trace_step(Entry &e, bool *deviated) {
     if (keep) {
       // recorded programs that share this prefix must agree on the call's role (two models
       // with the same first layers may continue differently); otherwise it runs as it stands
-      const uint8_t r = ts.programs[ts.cands[0]].roles[index];
+      const uint16_t r = ts.programs[ts.cands[0]].roles[index];
       role = (Role)(r & ROLE_BITS);
-      ts.last_flags = r & (uint8_t)~ROLE_BITS;
+      ts.last_flags = r & (uint16_t)~ROLE_BITS;
       for (size_t k = 1; k < keep; ++k)
         if (ts.programs[ts.cands[k]].roles[index] != r ||
             ((r & RF_FOR_CONV) && ts.programs[ts.cands[k]].sigs[ts.programs[ts.cands[k]].reader[index]] !=
@@ -495,7 +510,7 @@ void trace_end() {
 }
 
 // ---- prefixes made in one go (graph_replay.cu) ------------------------------------
-uint8_t trace_last_flags() { return g_ts.last_flags; }
+uint16_t trace_last_flags() { return g_ts.last_flags; }
 const Entry *trace_last_reader() {
   TraceProgram *p = g_ts.cands.empty() ? nullptr : &g_ts.programs[g_ts.cands[0]];
   const size_t n = trace_index();

@@ -8,6 +8,7 @@
 //     matrix product -> [+ bias row] -> [ReLU]
 //     1x1 convolution chain -> 3x3 depthwise chain -> 1x1 convolution chain
 //     convolution chain + convolution chain [-> ReLU | Clip]
+//     convolution chain with a sum and ReLU -> 1x1 convolution chain with ReLU, both of whose results are kept
 // (and, for a few-channel stem convolution, a 3x3 / stride 2 max pool behind it)
 // whose intermediate results nobody else reads before their memory is handed out again,
 // and marks them.  The next time the same call sequence comes by, the convolution of such
@@ -81,24 +82,28 @@ void te_ptr_or_elsewhere(Entry &e, const void *p);
 struct GraphPlan;
 // flag beside a call's role: whatever reads its result is a matrix product (possibly behind a Flatten),
 // so the result may be kept in the 16-bit form that product takes
-constexpr uint8_t RF_FOR_MATMUL = 0x10;
+constexpr uint16_t RF_FOR_MATMUL = 0x10;
 // on a device-to-device copy: what reads the tensor are convolutions on the 16-bit path, so the copy may
 // bring it in in their form (TraceProgram::reader names the first of them)
-constexpr uint8_t RF_FOR_CONV = 0x20;
+constexpr uint16_t RF_FOR_CONV = 0x20;
 // on a convolution in fp32 mode or a call folded into one: all that reads the result takes it in three
 // planes of parts (FMT_PARTS)
-constexpr uint8_t RF_FOR_PARTS = 0x40;
+constexpr uint16_t RF_FOR_PARTS = 0x40;
 // on convolutions that run together with the next one (RF_LINK) or the one before (RF_JOIN): the three of
 // an inverted residual, which become one kernel
-constexpr uint8_t RF_LINK = 0x04;
-constexpr uint8_t RF_JOIN = 0x08;
+constexpr uint16_t RF_LINK = 0x04;
+constexpr uint16_t RF_JOIN = 0x08;
 // on two convolutions whose results are added, one chain behind the other: the first is held back until the sum
 // comes by, which one kernel then computes (a block's last convolution and its projection shortcut)
-constexpr uint8_t RF_SUM = 0x80;
-constexpr uint8_t ROLE_BITS = 0x03;
+constexpr uint16_t RF_SUM = 0x80;
+// on a convolution whose chain ends in a sum and ReLU, and on the 1x1 convolution right behind it that reads the
+// result: one kernel may write both (launch_tc_pair())
+constexpr uint16_t RF_LEAD = 0x100;
+constexpr uint16_t RF_FOLLOW = 0x200;
+constexpr uint16_t ROLE_BITS = 0x03;
 struct TraceProgram {
   std::vector<uint64_t> sigs;
-  std::vector<uint8_t> roles;   // Role | RF_*
+  std::vector<uint16_t> roles;   // Role | RF_*
   std::vector<int> reader;      // RF_FOR_CONV: call that reads the result first
   std::vector<Entry> entries;
   uintptr_t pool_base = 0;     // pool the entries' pointers refer to
@@ -111,7 +116,7 @@ struct TraceProgram {
 // program although earlier calls did.
 Role trace_step(Entry &e, bool *deviated);
 
-uint8_t trace_last_flags();         // RF_* of the call trace_step() was last given
+uint16_t trace_last_flags();        // RF_* of the call trace_step() was last given
 const Entry *trace_last_reader();   // the recorded call that first reads its result (RF_FOR_CONV)
 void trace_begin();                 // cudnnCreate
 void trace_end();                   // cudnnDestroy: analyse and store if the sequence is new
@@ -132,7 +137,7 @@ bool entry_takes_pool(const Entry &e);
 bool entry_reads_16(const Entry &e);
 // The role (with its RF_*) of the calls up to trace_force_end(), whatever was recorded: calls made outside an
 // inference's own sequence.
-void trace_force(uint8_t role);
+void trace_force(uint16_t role);
 void trace_force_end();
 uintptr_t trace_pool_base();
 size_t trace_pool_bytes();

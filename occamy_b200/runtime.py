@@ -155,7 +155,8 @@ def counters() -> dict:
     return dict(zip(COUNTER_NAMES, [int(v) for v in out]))
 
 
-FORM_NAMES = ("split_reduction", "inverted_residual", "column_strips", "pooled", "replayed", "in_pieces", "summed")
+FORM_NAMES = ("split_reduction", "inverted_residual", "column_strips", "pooled", "replayed", "in_pieces", "summed",
+              "pairs")
 
 
 def form_counters() -> dict:
