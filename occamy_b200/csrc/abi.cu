@@ -1603,6 +1603,7 @@ static float *pool_common(int sym, float *x, int64_t *dI, float *y, int64_t *dO,
       sa.lo = j.a.act == ACT_RELU ? 0.0f : (j.a.act == ACT_CLIP ? j.a.lo : -INFINITY);
       sa.hi = j.a.act == ACT_CLIP ? j.a.hi : INFINITY;
       sa.w = j.w_stem;
+      sa.w_fold = j.a.w;
       if (stem_pool_supported(sa)) {
         if (launch_stem_pool(sa, r.dev_err, r.num_sms, r.stream)) {
           j.active = false;

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
   volatile uint32_t *tmem_holder = reinterpret_cast<volatile uint32_t *>(tail);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tail + 8);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     tma_prefetch_map(&p.tmA[0]);
     tma_prefetch_map(&p.tmB1[0]);
@@ -137,20 +137,20 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
 
   if (warp == 0) {
     // ------------------------------------------------------------ x
-    if (lane == 0) {
+    {
       int s = 0;
       uint32_t phase = 0;
       const uint32_t bytes = (uint32_t)p.rows * 128u;
       for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x) {
         const TcTile tl = pixels(tile);
         for (int k = 0; k < k1; ++k) {
-          if (!mbar_wait_hot(a_empty(s), phase ^ 1u, abort_flag)) {
+          if (!mbar_wait_warp(a_empty(s), phase ^ 1u, abort_flag)) {
             err_code = 1;
             break;
           }
           const bool second = k >= p.blocks1;
-          mbar_expect_tx(a_full(s), bytes);
-          tma_load_4d(sA + s * PR_BLOCK, &p.tmA[second], a_full(s), (second ? k - p.blocks1 : k) * 64, tl.q0, tl.p0, tl.n0);
+          expect_tx_warp(a_full(s), bytes);
+          load_4d_warp(sA + s * PR_BLOCK, &p.tmA[second], a_full(s), (second ? k - p.blocks1 : k) * 64, tl.q0, tl.p0, tl.n0);
           if (++s == nA) {
             s = 0;
             phase ^= 1u;
@@ -160,19 +160,19 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
     }
   } else if (warp == 10) {
     // ------------------------------------------------------------ weights of product 1
-    if (lane == 0) {
+    {
       int s = 0;
       uint32_t phase = 0;
       for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x)
         for (int c = 0; c < chunks && !err_code; ++c)
           for (int k = 0; k < k1; ++k) {
-            if (!mbar_wait_hot(w_empty(s), phase ^ 1u, abort_flag)) {
+            if (!mbar_wait_warp(w_empty(s), phase ^ 1u, abort_flag)) {
               err_code = 1;
               break;
             }
             const bool second = k >= p.blocks1;
-            mbar_expect_tx(w_full(s), PR_BLOCK);
-            tma_load_3d(sW + s * PR_BLOCK, &p.tmB1[second], w_full(s), (second ? k - p.blocks1 : k) * 64, c * 128, 0);
+            expect_tx_warp(w_full(s), PR_BLOCK);
+            load_3d_warp(sW + s * PR_BLOCK, &p.tmB1[second], w_full(s), (second ? k - p.blocks1 : k) * 64, c * 128, 0);
             if (++s == nW) {
               s = 0;
               phase ^= 1u;
@@ -181,17 +181,17 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
     }
   } else if (warp == 15) {
     // ------------------------------------------------------------ weights of product 2
-    if (lane == 0) {
+    {
       int s = 0;
       uint32_t phase = 0;
       for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x)
         for (int c = 0; c < p.K1; c += 64) {
-          if (!mbar_wait_hot(v_empty(s), phase ^ 1u, abort_flag)) {
+          if (!mbar_wait_warp(v_empty(s), phase ^ 1u, abort_flag)) {
             err_code = 1;
             break;
           }
-          mbar_expect_tx(v_full(s), (uint32_t)p.K2 * 128u);
-          tma_load_3d(sV + s * PR_BLOCK, &p.tmB2, v_full(s), c, 0, 0);
+          expect_tx_warp(v_full(s), (uint32_t)p.K2 * 128u);
+          load_3d_warp(sV + s * PR_BLOCK, &p.tmB2, v_full(s), c, 0, 0);
           if (++s == nV) {
             s = 0;
             phase ^= 1u;
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ product 1
-    if (lane == 0) {
+    {
       const uint32_t idesc = FORMAT | ((uint32_t)(128 >> 3) << 17);
       const uint64_t d0 = make_smem_desc(sA, 64);
       const uint32_t hi = (uint32_t)(d0 >> 32), a_lo0 = (uint32_t)d0, w_lo0 = (uint32_t)make_smem_desc(sW, 64);
@@ -210,15 +210,15 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
       for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x) {
         a_base = a_next;
         for (int c = 0; c < chunks && !err_code; ++c) {
-          if (!mbar_wait_hot(d1_empty(d1), d1_phase ^ 1u, abort_flag)) {
+          if (!mbar_wait_warp(d1_empty(d1), d1_phase ^ 1u, abort_flag)) {
             err_code = 2;
             break;
           }
           int as = a_base;
 #pragma unroll 1
           for (int k = 0; k < k1; ++k) {
-            if ((c == 0 && !mbar_wait_hot(a_full(as), a_phase, abort_flag)) ||
-                !mbar_wait_hot(w_full(ws), w_phase, abort_flag)) {
+            if ((c == 0 && !mbar_wait_warp(a_full(as), a_phase, abort_flag)) ||
+                !mbar_wait_warp(w_full(ws), w_phase, abort_flag)) {
               err_code = 3;
               break;
             }
@@ -226,9 +226,9 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
             const uint32_t a_lo = a_lo0 + (uint32_t)as * STEP, b_lo = w_lo0 + (uint32_t)ws * STEP;
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-              mma_lohi(tmem + (uint32_t)(d1 * 128), a_lo + 2u * kk, hi, b_lo + 2u * kk, hi, idesc, kk ? 1u : (uint32_t)(k != 0));
-            tc_commit(w_empty(ws));
-            if (c == chunks - 1) tc_commit(a_empty(as));
+              mma_warp(tmem + (uint32_t)(d1 * 128), a_lo + 2u * kk, hi, b_lo + 2u * kk, hi, idesc, kk ? 1u : (uint32_t)(k != 0));
+            commit_warp(w_empty(ws));
+            if (c == chunks - 1) commit_warp(a_empty(as));
             if (++ws == nW) {
               ws = 0;
               w_phase ^= 1u;
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
           }
           if (err_code) break;
           a_next = as;
-          tc_commit(d1_full(d1));
+          commit_warp(d1_full(d1));
           d1 ^= 1;
           if (d1 == 0) d1_phase ^= 1u;
         }
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
     }
   } else if (warp == 14) {
     // ------------------------------------------------------------ product 2
-    if (lane == 0) {
+    {
       const uint32_t idesc = FORMAT | ((uint32_t)(p.K2 >> 3) << 17);
       const uint64_t d0 = make_smem_desc(sS, 64);
       const uint32_t hi = (uint32_t)(d0 >> 32), s_lo0 = (uint32_t)d0, v_lo0 = (uint32_t)make_smem_desc(sV, 64);
@@ -256,14 +256,14 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
       int vs = 0, ss = 0;
       uint32_t v_phase = 0, s_phase = 0, d2_phase = 0;
       for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x) {
-        if (!mbar_wait_hot(d2_empty, d2_phase ^ 1u, abort_flag)) {
+        if (!mbar_wait_warp(d2_empty, d2_phase ^ 1u, abort_flag)) {
           err_code = 2;
           break;
         }
         d2_phase ^= 1u;
 #pragma unroll 1
         for (int c = 0; c < p.K1; c += 64) {
-          if (!mbar_wait_hot(v_full(vs), v_phase, abort_flag) || !mbar_wait_hot(s_full(ss), s_phase, abort_flag)) {
+          if (!mbar_wait_warp(v_full(vs), v_phase, abort_flag) || !mbar_wait_warp(s_full(ss), s_phase, abort_flag)) {
             err_code = 3;
             break;
           }
@@ -271,9 +271,9 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
           const uint32_t a_lo = s_lo0 + (uint32_t)ss * STEP, b_lo = v_lo0 + (uint32_t)vs * STEP;
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            mma_lohi(tmem2, a_lo + 2u * kk, hi, b_lo + 2u * kk, hi, idesc, kk ? 1u : (uint32_t)(c != 0));
-          tc_commit(v_empty(vs));
-          tc_commit(s_read(ss));
+            mma_warp(tmem2, a_lo + 2u * kk, hi, b_lo + 2u * kk, hi, idesc, kk ? 1u : (uint32_t)(c != 0));
+          commit_warp(v_empty(vs));
+          commit_warp(s_read(ss));
           if (++vs == nV) {
             vs = 0;
             v_phase ^= 1u;
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
             s_phase ^= 1u;
           }
         }
-        if (!err_code) tc_commit(d2_full);
+        if (!err_code) commit_warp(d2_full);
       }
     }
   } else if (warp == 11 || warp == 12) {

@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_conv_pn_kernel(const __grid_
   volatile uint32_t *tmem_holder = reinterpret_cast<volatile uint32_t *>(bars + 2 * stages + 5);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 2 * stages + 6);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
       mbar_init(full_bar(s), 1);
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_conv_pn_kernel(const __grid_
   int err_code = 0;
 
   if (warp == 0) {
-    if (lane == 0) {
+    {
       int stage = 0;
       uint32_t phase = 0;
       const uint32_t tx_bytes = (uint32_t)rows_valid * bk * 2u + w_bytes;
@@ -109,14 +109,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_conv_pn_kernel(const __grid_
         for (int t = 0; t < p.num_taps && !err_code; ++t) {
           const TcTap tap = p.taps[t];
           for (int cb = 0; cb < p.cblocks; ++cb) {
-            if (!mbar_wait_hot(empty_bar(stage), phase ^ 1u, abort_flag)) {
+            if (!mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag)) {
               err_code = 1;
               break;
             }
-            mbar_expect_tx(full_bar(stage), tx_bytes);
-            tma_load_4d(sX + stage * x_bytes, &p.tmA[tap.map], full_bar(stage), cb * bk,
+            expect_tx_warp(full_bar(stage), tx_bytes);
+            load_4d_warp(sX + stage * x_bytes, &p.tmA[tap.map], full_bar(stage), cb * bk,
                         q0 + tap.dw, p0 + tap.dh, n0);
-            tma_load_3d(sW + stage * w_bytes, &p.tmB, full_bar(stage), cb * bk, k0, t);
+            load_3d_warp(sW + stage * w_bytes, &p.tmB, full_bar(stage), cb * bk, k0, t);
             if (++stage == stages) {
               stage = 0;
               phase ^= 1u;
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_conv_pn_kernel(const __grid_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
                              ((uint32_t)(p.n_mma >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
       int stage = 0, acc = 0;
@@ -142,23 +142,23 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_conv_pn_kernel(const __grid_
         constexpr int NK = decltype(nk_c)::value;
         uint32_t w_lo = w_lo0, x_lo = x_lo0;
         for (int tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
-          if (!mbar_wait_hot(tempty_bar(acc), acc_phase ^ 1u, abort_flag)) {
+          if (!mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag)) {
             err_code = 2;
             return;
           }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + (uint32_t)(acc * 256);
           for (int ks = 0; ks < ksteps; ++ks) {
-            if (!mbar_wait_hot(full_bar(stage), phase, abort_flag)) {
+            if (!mbar_wait_warp(full_bar(stage), phase, abort_flag)) {
               err_code = 3;
               return;
             }
             tc_fence_after();
 #pragma unroll
             for (int kk = 0; kk < NK; ++kk)
-              mma_lohi(d_tmem, w_lo + 2u * kk, w_hi, x_lo + 2u * kk, x_hi, idesc,
+              mma_warp(d_tmem, w_lo + 2u * kk, w_hi, x_lo + 2u * kk, x_hi, idesc,
                        kk ? 1u : (uint32_t)(ks != 0));
-            tc_commit(empty_bar(stage));
+            commit_warp(empty_bar(stage));
             w_lo += w_step;
             x_lo += x_step;
             if (++stage == stages) {
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_conv_pn_kernel(const __grid_
               x_lo = x_lo0;
             }
           }
-          tc_commit(tfull_bar(acc));
+          commit_warp(tfull_bar(acc));
           acc ^= 1;
           if (acc == 0) acc_phase ^= 1u;
         }

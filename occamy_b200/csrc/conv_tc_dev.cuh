@@ -216,6 +216,23 @@ __device__ __forceinline__ bool mbar_wait_hot(uint32_t a, uint32_t parity,
   }
   return true;
 }
+// The same wait for a whole warp, whose lanes go on together or give up together.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t a, uint32_t parity, volatile int *abort_flag) {
+  if (__all_sync(0xffffffffu, mbar_try(a, parity))) return true;
+  const long long t0 = clock64();
+  int it = 0;
+  while (!__all_sync(0xffffffffu, mbar_try(a, parity))) {
+    if ((++it & 15) == 0) {
+      const bool late = clock64() - t0 > 4000000000LL;
+      if (__any_sync(0xffffffffu, *abort_flag != 0 || late)) {
+        if (late) *abort_flag = 1;
+        return false;
+      }
+    }
+  }
+  return true;
+}
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *m, uint32_t bar,
                                             int c0, int c1, int c2, int c3) {
   asm volatile(
@@ -239,24 +256,8 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap *m, uint32_t src,
       "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
-// ---- CTA-pair forms (TC_MODE_PAIR).  `bar` is a shared::cluster address, normally of a
+// ---- CTA-pair forms (TC_MODE_PAIR; loads and MMAs further down).  `bar` is a shared::cluster address, normally of a
 // barrier in the pair's first CTA; the data always lands in the issuing CTA's own memory.
-__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap *m, uint32_t bar,
-                                                 int c0, int c1, int c2, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(dst),
-      "l"(m), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap *m, uint32_t bar,
-                                                 int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
-      "l"(m), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -275,26 +276,6 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n"
                "barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Completion of the pair's MMAs so far, signalled on the barrier at this offset in both CTAs.
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 "
-      "[%0], %1;" ::"r"(bar),
-      "h"((uint16_t)3)
-      : "memory");
-}
-__device__ __forceinline__ void mma_lohi_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi,
-                                              uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
-                                              uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\n.reg .b64 da, db;\n"
-      "setp.ne.b32 p, %6, 0;\n"
-      "mov.b64 da, {%1, %2};\n"
-      "mov.b64 db, {%3, %4};\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n}" ::"r"(d_tmem),
-      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_map(const CUtensorMap *m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
@@ -391,6 +372,93 @@ __device__ __forceinline__ void mma_lohi(uint32_t d_tmem, uint32_t a_lo, uint32_
       "mov.b64 db, {%3, %4};\n"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}" ::"r"(d_tmem),
       "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// ---- the same by one lane of a warp that executes them as a whole.
+// These instructions take their operands from uniform registers.  In code that one lane runs by itself the operands are
+// that lane's, and every instruction waits for a handful of moves: an MMA was issued every 100 cycles or so, although the
+// tensor core takes a small one in 48.  Warps that load or issue MMAs therefore run their role as a whole, on values that
+// are the same in all lanes, and elect a lane for the instruction alone.  By launch (256 images, ncu): 3x3 64 -> 64 at
+// 56x56 66 -> 60 us, 128 -> 128 at 28x28 51 -> 46.5, 512 -> 128 there 46 -> 43.  ResNet-50 with 8 images 328 -> 303 us,
+// 32 554 -> 520, 61 at 201x201 804 -> 770, 16 in fp32 1438 -> 1308; MobileNetV2 with 128 860 -> 805; VGG-16 with 64
+// 1888 -> 1823, 5 290 -> 277.
+__device__ __forceinline__ void mma_warp(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                         uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p, q;\n.reg .b64 da, db;\n"
+      "elect.sync _|q, 0xffffffff;\n"
+      "setp.ne.b32 p, %6, 0;\n"
+      "mov.b64 da, {%1, %2};\n"
+      "mov.b64 db, {%3, %4};\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}" ::"r"(d_tmem),
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void mma_pair_warp(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
+                                              uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p, q;\n.reg .b64 da, db;\n"
+      "elect.sync _|q, 0xffffffff;\n"
+      "setp.ne.b32 p, %6, 0;\n"
+      "mov.b64 da, {%1, %2};\n"
+      "mov.b64 db, {%3, %4};\n"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n}" ::"r"(d_tmem),
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void expect_tx_warp(uint32_t a, uint32_t bytes) {
+  asm volatile(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}" ::"r"(a),
+      "r"(bytes)
+      : "memory");
+}
+__device__ __forceinline__ void load_4d_warp(uint32_t dst, const CUtensorMap *m, uint32_t bar, int c0, int c1, int c2,
+                                             int c3) {
+  asm volatile(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5, %6}], [%2];\n}" ::"r"(dst),
+      "l"(m), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
+__device__ __forceinline__ void load_3d_warp(uint32_t dst, const CUtensorMap *m, uint32_t bar, int c0, int c1, int c2) {
+  asm volatile(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5}], [%2];\n}" ::"r"(dst),
+      "l"(m), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+__device__ __forceinline__ void load_4d_pair_warp(uint32_t dst, const CUtensorMap *m, uint32_t bar, int c0, int c1,
+                                                  int c2, int c3) {
+  asm volatile(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5, %6}], [%2];\n}" ::"r"(dst),
+      "l"(m), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
+__device__ __forceinline__ void load_3d_pair_warp(uint32_t dst, const CUtensorMap *m, uint32_t bar, int c0, int c1,
+                                                  int c2) {
+  asm volatile(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5}], [%2];\n}" ::"r"(dst),
+      "l"(m), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+__device__ __forceinline__ void commit_warp(uint32_t bar) {
+  asm volatile(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void commit_pair_warp(uint32_t bar) {
+  asm volatile(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}" ::"r"(bar),
+      "h"((uint16_t)3)
       : "memory");
 }
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t *r) {
@@ -594,7 +662,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
       reinterpret_cast<volatile uint32_t *>(bars + 2 * stages + 5 + 2 * dbuf);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 2 * stages + 6 + 2 * dbuf);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u;     // 0: the CTA that issues the MMAs
   const int tile0 = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
   const int tstep = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
@@ -656,18 +724,18 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
   int pre_b = 0;   // leading k-steps of the first tile whose weight tile is already on its way
   // resident form: the weight tiles of every k-step, once, announced on the "weights landed" barrier
   auto load_resident_b = [&]() {
-    mbar_expect_tx(wfull_bar, (uint32_t)ksteps * b_bytes);
+    expect_tx_warp(wfull_bar, (uint32_t)ksteps * b_bytes);
     int i = 0;
     for (int t = 0; t < p.num_taps; ++t)
       for (int cb = 0; cb < p.cblocks; ++cb, ++i)
-        tma_load_3d(sB + i * b_bytes, &p.tmB, wfull_bar, cb * bk, 0, t);
+        load_3d_warp(sB + i * b_bytes, &p.tmB, wfull_bar, cb * bk, 0, t);
   };
-  if (!PAIR && warp == (two_loaders ? WLOAD_WARP : 0) && lane == 0 && p.consts_ready &&
+  if (!PAIR && warp == (two_loaders ? WLOAD_WARP : 0) && p.consts_ready &&
       (int)blockIdx.x < p.total_tiles) {
     if constexpr (HALO) {
-      mbar_expect_tx(wfull_bar, (uint32_t)p.num_taps * b_bytes);
+      expect_tx_warp(wfull_bar, (uint32_t)p.num_taps * b_bytes);
       for (int t = 0; t < p.num_taps; ++t)
-        tma_load_3d(sB + t * b_bytes, &p.tmB, wfull_bar, 0, 0, t);
+        load_3d_warp(sB + t * b_bytes, &p.tmB, wfull_bar, 0, 0, t);
     } else if (bres) {
       load_resident_b();
     } else {
@@ -676,8 +744,8 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
       int t = 0, cb = 0;
       for (int s = 0; s < pre_b; ++s) {
         // a lone loader arms the barrier for both operands here; of two, each arms its own
-        mbar_expect_tx(full_bar(s), two_loaders ? b_bytes : (uint32_t)rows_valid * bk * 2u + b_bytes);
-        tma_load_3d(sB + s * b_bytes, map_b(t), full_bar(s), cb * bk, tl.k0, tap_b(t));
+        expect_tx_warp(full_bar(s), two_loaders ? b_bytes : (uint32_t)rows_valid * bk * 2u + b_bytes);
+        load_3d_warp(sB + s * b_bytes, map_b(t), full_bar(s), cb * bk, tl.k0, tap_b(t));
         if (++cb == blocks_of(t)) {
           cb = 0;
           ++t;
@@ -690,27 +758,27 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    {
       int stage = 0;
       uint32_t phase = 0;
       if constexpr (HALO) {
         // weights of all taps once (unless they were requested early), then one input block
         // per tile
         if (!p.consts_ready) {
-          mbar_expect_tx(wfull_bar, (uint32_t)p.num_taps * b_bytes);
+          expect_tx_warp(wfull_bar, (uint32_t)p.num_taps * b_bytes);
           for (int t = 0; t < p.num_taps; ++t)
-            tma_load_3d(sB + t * b_bytes, &p.tmB, wfull_bar, 0, 0, t);
+            load_3d_warp(sB + t * b_bytes, &p.tmB, wfull_bar, 0, 0, t);
         }
         const uint32_t blk_bytes = (uint32_t)((p.th + 2) * p.halo_wp) * 128u;
         for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x) {
           const TcTile tl = tc_decode<BN>(p, tile);
-          if (!mbar_wait_hot(empty_bar(stage), phase ^ 1u, abort_flag)) {
+          if (!mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag)) {
             err_code = 1;
             break;
           }
-          mbar_expect_tx(full_bar(stage), blk_bytes);
+          expect_tx_warp(full_bar(stage), blk_bytes);
           // column q0 - 1 and row p0 - 1 onwards; what lies outside the image arrives as zeros
-          tma_load_4d(sA + stage * a_bytes, &p.tmA[0], full_bar(stage), 0, tl.q0 - 1, tl.p0 - 1, tl.n0);
+          load_4d_warp(sA + stage * a_bytes, &p.tmA[0], full_bar(stage), 0, tl.q0 - 1, tl.p0 - 1, tl.n0);
           if (++stage == stages) {
             stage = 0;
             phase ^= 1u;
@@ -727,7 +795,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
           const int blocks = blocks_of(t), tb = tap_b(t);
           const CUtensorMap *mb = map_b(t);
           for (int cb = 0; cb < blocks; ++cb) {
-            if (!TCT_WAIT(0, mbar_wait_hot(empty_bar(stage), phase ^ 1u, abort_flag))) {
+            if (!TCT_WAIT(0, mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag))) {
               err_code = 1;
               break;
             }
@@ -735,9 +803,9 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
               // Both CTAs' bytes are counted on the first CTA's barrier, which that CTA arms
               // for the two of them; each CTA fetches its own pixels and its half of B.
               const uint32_t fb = cluster_map(full_bar(stage), 0);
-              if (rank == 0) mbar_expect_tx(full_bar(stage), 2u * tx_bytes);
-              tma_load_3d_pair(sB + stage * b_bytes, mb, fb, cb * bk, tl.k0 + (int)rank * BROWS, tb);
-              tma_load_4d_pair(sA + stage * a_bytes, &p.tmA[tap.map], fb, cb * bk, tl.q0 + tap.dw,
+              if (rank == 0) expect_tx_warp(full_bar(stage), 2u * tx_bytes);
+              load_3d_pair_warp(sB + stage * b_bytes, mb, fb, cb * bk, tl.k0 + (int)rank * BROWS, tb);
+              load_4d_pair_warp(sA + stage * a_bytes, &p.tmA[tap.map], fb, cb * bk, tl.q0 + tap.dw,
                                tl.p0 + tap.dh, tl.n0);
               if (++stage == stages) {
                 stage = 0;
@@ -746,16 +814,16 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
               continue;
             }
             if (two_loaders) {
-              mbar_expect_tx(full_bar(stage), tx_bytes - b_bytes);   // the weight loader arms its own
+              expect_tx_warp(full_bar(stage), tx_bytes - b_bytes);   // the weight loader arms its own
             } else if (pre_b > 0) {
               --pre_b;   // this stage's barrier is armed and its weight tile on its way
             } else if (bres) {
-              mbar_expect_tx(full_bar(stage), tx_bytes);   // the weights are resident
+              expect_tx_warp(full_bar(stage), tx_bytes);   // the weights are resident
             } else {
-              mbar_expect_tx(full_bar(stage), tx_bytes);
-              tma_load_3d(sB + stage * b_bytes, mb, full_bar(stage), cb * bk, tl.k0, tb);
+              expect_tx_warp(full_bar(stage), tx_bytes);
+              load_3d_warp(sB + stage * b_bytes, mb, full_bar(stage), cb * bk, tl.k0, tb);
             }
-            tma_load_4d(sA + stage * a_bytes, &p.tmA[tap.map], full_bar(stage), cb * bk,
+            load_4d_warp(sA + stage * a_bytes, &p.tmA[tap.map], full_bar(stage), cb * bk,
                         tl.q0 + tap.dw, tl.p0 + tap.dh, tl.n0);
             if (++stage == stages) {
               stage = 0;
@@ -769,7 +837,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
     }
   } else if (warp == 1 || (HALO && warp == STORE_WARP + TC_NSTORE)) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       if constexpr (HALO) {
@@ -782,7 +850,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
         const uint32_t b_lo0 = (uint32_t)make_smem_desc(sB, 64);
         const uint32_t stage_desc = a_bytes >> 4, tap_desc = b_bytes >> 4;
         const uint32_t wp8 = (uint32_t)p.halo_wp * 8u;   // one block row in descriptor units
-        if (!mbar_wait_hot(wfull_bar, 0, abort_flag)) err_code = 3;
+        if (!mbar_wait_warp(wfull_bar, 0, abort_flag)) err_code = 3;
         // Two issuing threads take alternate tiles (and with them alternate accumulators):
         // 36 MMAs of 48 cycles per tile are more than one thread issues in that time.
         const int me = warp == 1 ? 0 : 1;
@@ -797,11 +865,11 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
           const int my_acc = it & 1;
           const uint32_t my_acc_phase = (uint32_t)(it >> 1) & 1u;
           if ((it & 1) != me) continue;
-          if (!mbar_wait_hot(tempty_bar(my_acc), my_acc_phase ^ 1u, abort_flag)) {
+          if (!mbar_wait_warp(tempty_bar(my_acc), my_acc_phase ^ 1u, abort_flag)) {
             err_code = 2;
             break;
           }
-          if (!mbar_wait_hot(full_bar(my_stage), my_phase, abort_flag)) {
+          if (!mbar_wait_warp(full_bar(my_stage), my_phase, abort_flag)) {
             err_code = 3;
             break;
           }
@@ -814,14 +882,14 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
             const uint32_t bt = b_lo0 + (uint32_t)t * tap_desc;
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-              mma_lohi(d_tmem, at + 2 * kk, a_hi, bt + 2 * kk, b_hi, IDESC, (t | kk) ? 1u : 0u);
+              mma_warp(d_tmem, at + 2 * kk, a_hi, bt + 2 * kk, b_hi, IDESC, (t | kk) ? 1u : 0u);
           }
-          tc_commit(empty_bar(my_stage));
-          tc_commit(tfull_bar(my_acc));
+          commit_warp(empty_bar(my_stage));
+          commit_warp(tfull_bar(my_acc));
         }
       } else {
       TCT_DECL
-      if (bres && !mbar_wait_hot(wfull_bar, 0, abort_flag)) err_code = 3;
+      if (bres && !mbar_wait_warp(wfull_bar, 0, abort_flag)) err_code = 3;
       {
         // This thread's instruction stream is the kernel's critical path on the tensor-bound
         // layers: the tensor pipe takes MMAs in order and holds very few that have not started,
@@ -838,14 +906,14 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
           constexpr int NK = decltype(nk_c)::value;   // MMAs per k-step: bk / 16
           uint32_t a_lo = a_lo0, b_lo = b_lo0;
           for (int tile = tile0; tile < p.total_tiles; tile += tstep) {
-            if (!TCT_WAIT(0, mbar_wait_hot(tempty_bar(acc), acc_phase ^ 1u, abort_flag))) {
+            if (!TCT_WAIT(0, mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag))) {
               err_code = 2;
               return;
             }
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
             for (int ks = 0; ks < ksteps; ++ks) {
-              if (!TCT_WAIT(1, mbar_wait_hot(full_bar(stage), phase, abort_flag))) {
+              if (!TCT_WAIT(1, mbar_wait_warp(full_bar(stage), phase, abort_flag))) {
                 err_code = 3;
                 return;
               }
@@ -855,12 +923,12 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
                 for (int kk = 0; kk < NK; ++kk) {
                   const uint32_t accumulate = kk ? 1u : (uint32_t)(ks != 0);
                   if constexpr (PAIR)   // the same offsets in the other CTA hold its pixels and B half
-                    mma_lohi_pair(d_tmem, a_lo + 2u * kk, a_hi, bl + 2u * kk, b_hi, IDESC, accumulate);
+                    mma_pair_warp(d_tmem, a_lo + 2u * kk, a_hi, bl + 2u * kk, b_hi, IDESC, accumulate);
                   else
-                    mma_lohi(d_tmem, a_lo + 2u * kk, a_hi, bl + 2u * kk, b_hi, IDESC, accumulate);
+                    mma_warp(d_tmem, a_lo + 2u * kk, a_hi, bl + 2u * kk, b_hi, IDESC, accumulate);
                 }
-              if constexpr (PAIR) tc_commit_pair(empty_bar(stage));   // frees the stage in both CTAs
-              else tc_commit(empty_bar(stage));
+              if constexpr (PAIR) commit_pair_warp(empty_bar(stage));   // frees the stage in both CTAs
+              else commit_warp(empty_bar(stage));
               a_lo += a_step;
               b_lo += b_step;
               if (++stage == stages) {
@@ -870,8 +938,8 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
                 b_lo = b_lo0;
               }
             }
-            if constexpr (PAIR) tc_commit_pair(tfull_bar(acc));
-            else tc_commit(tfull_bar(acc));
+            if constexpr (PAIR) commit_pair_warp(tfull_bar(acc));
+            else commit_warp(tfull_bar(acc));
             acc ^= 1;
             if (acc == 0) acc_phase ^= 1u;
           }
@@ -1002,7 +1070,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
     }
   } else if (SPLIT_LOAD && warp == WLOAD_WARP) {
     // ------------------------------------------------------------ weight loader (see two_loaders)
-    if (lane == 0 && two_loaders) {
+    if (two_loaders) {
       int stage = 0;
       uint32_t phase = 0;
       for (int tile = tile0; tile < p.total_tiles && !err_code; tile += tstep) {
@@ -1014,12 +1082,12 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
             if (pre_b > 0) {
               --pre_b;   // requested before the wait for the previous kernel
             } else {
-              if (!mbar_wait_hot(empty_bar(stage), phase ^ 1u, abort_flag)) {
+              if (!mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag)) {
                 err_code = 1;
                 break;
               }
-              mbar_expect_tx(full_bar(stage), b_bytes);
-              tma_load_3d(sB + stage * b_bytes, mb, full_bar(stage), cb * bk, tl.k0, tb);
+              expect_tx_warp(full_bar(stage), b_bytes);
+              load_3d_warp(sB + stage * b_bytes, mb, full_bar(stage), cb * bk, tl.k0, tb);
             }
             if (++stage == stages) {
               stage = 0;

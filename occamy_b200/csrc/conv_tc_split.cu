@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   // which accumulators hold anything, one word per issuer
   volatile int *used = reinterpret_cast<volatile int *>(bars + 2 * stages + 4);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   // Fewer accumulators when there are fewer k-steps: CTAs of the next layer that share this SM need
   // TMEM columns as well.  A power of two.
   const int ni = p.issuers;
@@ -251,17 +251,20 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   const int ahead = min(stages, mine);        // k-steps that need no stage to become free
 
   // (tap, channel block) of a k-step of this CTA
-  auto load_b = [&](int i, int s) {
+  // (as a warp, or by one of its lanes)
+  auto load_b = [&](int i, int s, auto as_warp) {
     const int k = ks0 + i;
     const bool second = k >= p.ksteps1;
     const int t = second ? 0 : (int)tc_fdiv((uint32_t)k, p.div_cb);
     const CUtensorMap *m = second ? &p.tmB2 : &p.tmB;
     const int c = (second ? k - p.ksteps1 : k - t * p.cblocks) * bk;
 #pragma unroll
-    for (int j = 0; j < PARTS; ++j)
-      tma_load_3d(sB + s * b_bytes + j * b_tile, m, full_bar(s), c, tl.k0, t * PARTS + j);
+    for (int j = 0; j < PARTS; ++j) {
+      if constexpr (decltype(as_warp)::value) load_3d_warp(sB + s * b_bytes + j * b_tile, m, full_bar(s), c, tl.k0, t * PARTS + j);
+      else tma_load_3d(sB + s * b_bytes + j * b_tile, m, full_bar(s), c, tl.k0, t * PARTS + j);
+    }
   };
-  auto load_a = [&](int i, int s) {
+  auto load_a = [&](int i, int s, auto as_warp) {
     const int k = ks0 + i;
     const bool second = k >= p.ksteps1;
     const int t = second ? 0 : (int)tc_fdiv((uint32_t)k, p.div_cb);
@@ -269,15 +272,17 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
     const int map = second ? p.map2 : tap.map, c = (second ? k - p.ksteps1 : k - t * p.cblocks) * bk;
     const int q = tl.q0 + (second ? 0 : tap.dw), h = tl.p0 + (second ? 0 : tap.dh);
 #pragma unroll
-    for (int j = 0; j < PARTS; ++j)
-      tma_load_4d(sA + s * a_bytes + j * a_tile, &p.tmA[map + j], full_bar(s), c, q, h, tl.n0);
+    for (int j = 0; j < PARTS; ++j) {
+      if constexpr (decltype(as_warp)::value) load_4d_warp(sA + s * a_bytes + j * a_tile, &p.tmA[map + j], full_bar(s), c, q, h, tl.n0);
+      else tma_load_4d(sA + s * a_bytes + j * a_tile, &p.tmA[map + j], full_bar(s), c, q, h, tl.n0);
+    }
   };
   // The k-steps of the first ring turn are requested by one lane each: a single thread's chain of
   // index arithmetic, arming arrival and request per k-step is time on the layer's critical path.
   const int first = warp >= 4 ? warp - 4 + 4 * lane : SK_MAX_STAGES;
   if (first < ahead && p.consts_ready) {
     mbar_expect_tx(full_bar(first), tx_bytes);
-    load_b(first, first);
+    load_b(first, first, std::false_type{});
   }
   pdl_launch_dependents();
   pdl_wait();   // from here on memory that other kernels write is read and written
@@ -291,8 +296,8 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
 
   if (first < ahead) {
     if (!p.consts_ready) mbar_expect_tx(full_bar(first), tx_bytes);
-    load_a(first, first);
-    if (!p.consts_ready) load_b(first, first);
+    load_a(first, first, std::false_type{});
+    if (!p.consts_ready) load_b(first, first, std::false_type{});
   }
   if (warp >= 4) {   // (the other four warps issue MMAs)
     const int i = (int)threadIdx.x - 128;
@@ -354,25 +359,25 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
     const bool real = pass != 0;
     int used_all[NI];
     if (real) {
-    if (warp >= 4 && warp < 4 + ni && lane == 0) {
+    if (warp >= 4 && warp < 4 + ni) {
       // later turns (stages is a multiple of ni then): k-step i goes to stage i % stages, loader i % ni
       int s = warp - 4;
       uint32_t phase = 0;
       for (int i = stages + s; i < mine; i += ni) {
-        if (!mbar_wait_hot(empty_bar(s), phase, abort_flag)) {
+        if (!mbar_wait_warp(empty_bar(s), phase, abort_flag)) {
           err_code = 1;
           break;
         }
-        mbar_expect_tx(full_bar(s), tx_bytes);
-        load_b(i, s);
-        load_a(i, s);
+        expect_tx_warp(full_bar(s), tx_bytes);
+        load_b(i, s, std::true_type{});
+        load_a(i, s, std::true_type{});
         s += ni;
         if (s >= stages) {
           s -= stages;
           phase ^= 1u;
         }
       }
-    } else if (warp < ni && lane == 0) {
+    } else if (warp < ni) {
       const uint64_t a0 = make_smem_desc(sA, bk), b0 = make_smem_desc(sB, bk);
       const uint32_t a_hi = (uint32_t)(a0 >> 32), b_hi = (uint32_t)(b0 >> 32);
       const uint32_t a_step = a_bytes >> 4, b_step = b_bytes >> 4;
@@ -385,7 +390,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
         for (int i = warp; i < mine; i += ni) {
           const uint32_t a_lo = (uint32_t)a0 + (uint32_t)s * a_step, b_lo = (uint32_t)b0 + (uint32_t)s * b_step;
           const uint32_t more = seen;
-          if (!mbar_wait_hot(full_bar(s), phase, abort_flag)) {
+          if (!mbar_wait_warp(full_bar(s), phase, abort_flag)) {
             err_code = 3;
             return;
           }
@@ -395,7 +400,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
           auto products = [&](int pa, int pb, int d, uint32_t n, bool opens) {
 #pragma unroll
             for (int kk = 0; kk < NK; ++kk)
-              mma_lohi(d0 + (uint32_t)(d * BN), a_lo + (uint32_t)pa * (a_tile >> 4) + 2u * kk, a_hi,
+              mma_warp(d0 + (uint32_t)(d * BN), a_lo + (uint32_t)pa * (a_tile >> 4) + 2u * kk, a_hi,
                        b_lo + (uint32_t)pb * (b_tile >> 4) + 2u * kk, b_hi, IDESC0 | (n << NSHIFT),
                        opens && kk == 0 ? more : 1u);
           };
@@ -413,14 +418,14 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
             products(2, 0, 2, BN, false);
           }
           seen = 1u;
-          if (i + stages < mine) tc_commit(empty_bar(s));   // nobody waits for the last ones
+          if (i + stages < mine) commit_warp(empty_bar(s));   // nobody waits for the last ones
           s += ni;
           if (s >= stages) {   // (a ring as long as the share is never reused)
             s -= stages;
             phase ^= 1u;
           }
         }
-        tc_commit(done_bar);
+        commit_warp(done_bar);
       };
       if (bk == 64) run(std::integral_constant<int, 4>{});
       else if (bk == 32) run(std::integral_constant<int, 2>{});

@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(WD_THREADS, 1) tc_conv_wide_kernel(const __gri
   volatile uint32_t *tmem_holder = reinterpret_cast<volatile uint32_t *>(misc);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(misc + 8);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     tma_prefetch_map(&p.tmA[0]);
     tma_prefetch_map(&p.tmB);
@@ -105,20 +105,20 @@ __global__ void __launch_bounds__(WD_THREADS, 1) tc_conv_wide_kernel(const __gri
 
   if (warp == 0) {
     // ------------------------------------------------------------ input blocks
-    if (lane == 0) {
+    {
       const uint32_t bytes = (uint32_t)((p.th + 2) * p.halo_wp) * 128u;
       int s = 0;
       uint32_t phase = 0;
       for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x) {
         const TcTile tl = tc_decode<128>(p, tile);
         for (int cb = 0; cb < p.cblocks; ++cb) {
-          if (!mbar_wait_hot(x_empty(s), phase ^ 1u, abort_flag)) {
+          if (!mbar_wait_warp(x_empty(s), phase ^ 1u, abort_flag)) {
             err_code = 1;
             break;
           }
-          mbar_expect_tx(x_full(s), bytes);
+          expect_tx_warp(x_full(s), bytes);
           // what lies outside the image arrives as zeros: the padding
-          tma_load_4d(sX + s * x_bytes, &p.tmA[0], x_full(s), cb * 64, tl.q0 - 1, tl.p0 - 1, tl.n0);
+          load_4d_warp(sX + s * x_bytes, &p.tmA[0], x_full(s), cb * 64, tl.q0 - 1, tl.p0 - 1, tl.n0);
           if (++s == WD_X) {
             s = 0;
             phase ^= 1u;
@@ -128,18 +128,18 @@ __global__ void __launch_bounds__(WD_THREADS, 1) tc_conv_wide_kernel(const __gri
     }
   } else if (warp == 10) {
     // ------------------------------------------------------------ weights
-    if (lane == 0) {
+    {
       int s = 0;
       uint32_t phase = 0;
       for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x)
         for (int cb = 0; cb < p.cblocks && !err_code; ++cb)
           for (int t = 0; t < 9; ++t) {
-            if (!mbar_wait_hot(w_empty(s), phase ^ 1u, abort_flag)) {
+            if (!mbar_wait_warp(w_empty(s), phase ^ 1u, abort_flag)) {
               err_code = 1;
               break;
             }
-            mbar_expect_tx(w_full(s / 3), WD_W_BYTES);
-            tma_load_3d(sW + s * WD_W_BYTES, &p.tmB, w_full(s / 3), cb * 64, 0, t);
+            expect_tx_warp(w_full(s / 3), WD_W_BYTES);
+            load_3d_warp(sW + s * WD_W_BYTES, &p.tmB, w_full(s / 3), cb * 64, 0, t);
             if (++s == WD_TAPS) {
               s = 0;
               phase ^= 1u;
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(WD_THREADS, 1) tc_conv_wide_kernel(const __gri
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.n_mma >> 3) << 17) |
                              ((uint32_t)(128 >> 4) << 24);
       const uint64_t w0 = make_smem_desc(sW, 64), x0 = make_smem_desc(sX, 64);
@@ -157,20 +157,20 @@ __global__ void __launch_bounds__(WD_THREADS, 1) tc_conv_wide_kernel(const __gri
       int xs = 0, acc = 0, g = 0;
       uint32_t x_phase = 0, acc_phase = 0, w_phase = 0;
       for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x) {
-        if (!mbar_wait_hot(t_empty(acc), acc_phase ^ 1u, abort_flag)) {
+        if (!mbar_wait_warp(t_empty(acc), acc_phase ^ 1u, abort_flag)) {
           err_code = 2;
           break;
         }
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * 256);
         for (int cb = 0; cb < p.cblocks && !err_code; ++cb) {
-          if (!mbar_wait_hot(x_full(xs), x_phase, abort_flag)) {
+          if (!mbar_wait_warp(x_full(xs), x_phase, abort_flag)) {
             err_code = 3;
             break;
           }
           uint32_t x_lo = x_lo0 + (uint32_t)xs * (x_bytes >> 4);
 #pragma unroll 1
           for (int r = 0; r < 3; ++r) {
-            if (!mbar_wait_hot(w_full(g), w_phase, abort_flag)) {
+            if (!mbar_wait_warp(w_full(g), w_phase, abort_flag)) {
               err_code = 4;
               break;
             }
@@ -181,21 +181,21 @@ __global__ void __launch_bounds__(WD_THREADS, 1) tc_conv_wide_kernel(const __gri
             for (int c = 0; c < 3; ++c) {
 #pragma unroll
               for (int kk = 0; kk < 4; ++kk)
-                mma_lohi(d_tmem, w_lo + (uint32_t)c * (WD_W_BYTES >> 4) + 2u * kk, hi, x_lo + 8u * c + 2u * kk, hi, idesc,
+                mma_warp(d_tmem, w_lo + (uint32_t)c * (WD_W_BYTES >> 4) + 2u * kk, hi, x_lo + 8u * c + 2u * kk, hi, idesc,
                          (c | kk) ? 1u : more);
-              tc_commit(w_empty(g * 3 + c));
+              commit_warp(w_empty(g * 3 + c));
             }
             x_lo += wp8;
             g ^= 1;
             if (g == 0) w_phase ^= 1u;
           }
-          tc_commit(x_empty(xs));
+          commit_warp(x_empty(xs));
           if (++xs == WD_X) {
             xs = 0;
             x_phase ^= 1u;
           }
         }
-        tc_commit(t_full(acc));
+        commit_warp(t_full(acc));
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
       }

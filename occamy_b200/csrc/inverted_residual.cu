@@ -30,7 +30,7 @@
 namespace occ {
 
 constexpr int IR_WORKERS = 256;         // drain, depthwise, finish
-constexpr int IR_THREADS = IR_WORKERS + 32;   // and a warp (one lane) that loads and issues MMAs
+constexpr int IR_THREADS = IR_WORKERS + 32;   // and a warp that loads and issues MMAs
 constexpr int IR_MAX_E = 1024;
 constexpr int IR_MAX_SPLITS = 8;
 constexpr int IR_MAX_BLOCKS = 4;       // 128-pixel blocks of a tile's input
@@ -77,10 +77,12 @@ __device__ __forceinline__ void ir_sts128(uint32_t addr, const uint32_t *r) {
 __device__ __forceinline__ void ir_sts64(uint32_t addr, uint32_t a, uint32_t b) {
   asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
 }
-__device__ __forceinline__ void ir_bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
+__device__ __forceinline__ void ir_bulk_load_warp(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+  asm volatile(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n}" ::"r"(dst),
+      "l"(src), "r"(bytes), "r"(bar)
+      : "memory");
 }
 __device__ __forceinline__ uint2 ir_lds64(uint32_t addr) {
   uint2 v;
@@ -200,7 +202,7 @@ __global__ void __launch_bounds__(IR_THREADS, 2) ir_kernel(const __grid_constant
   const uint32_t sWD = bar0 + 96;                       // two stages
   float *b3_s = reinterpret_cast<float *>(misc + 96 + 2 * WD_STAGE);   // Kp floats
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int quad = warp & 3, part = warp >> 2;
   const int rank = CL ? (int)cluster_ctarank() : 0;
   const int total_tiles = p.tiles, first_tile = (int)blockIdx.x / splits;
@@ -256,32 +258,32 @@ __global__ void __launch_bounds__(IR_THREADS, 2) ir_kernel(const __grid_constant
   const int chunks_all = mine * ((total_tiles - first_tile + step_tiles - 1) / step_tiles);
   auto chunk_e0 = [&](int c) { return (rank + c * splits) * EC; };
 
-  if (threadIdx.x == IR_WORKERS) {
+  if (warp == IR_WORKERS / 32) {
     // Loads and products, in a warp of their own: done by one of the workers they kept all of them waiting
     // at the next barrier for a third of a chunk's time.
     auto load_w1 = [&](int g, int c) {
       const uint32_t st = (uint32_t)(g & 1), bar = w1_bar + 8u * st, dst = sW1 + st * w1_stage;
-      mbar_expect_tx(bar, w1_bytes);
+      expect_tx_warp(bar, w1_bytes);
       for (int k = 0; k < p.kcs; ++k)
-        tma_load_3d(dst + (uint32_t)k * w1_tile, &p.tmW1, bar, k * p.bk, chunk_e0(c), 0);
-      tma_load_3d(dst + (uint32_t)p.kcs * w1_tile, &p.tmB1, bar, 0, chunk_e0(c), 0);
+        load_3d_warp(dst + (uint32_t)k * w1_tile, &p.tmW1, bar, k * p.bk, chunk_e0(c), 0);
+      load_3d_warp(dst + (uint32_t)p.kcs * w1_tile, &p.tmB1, bar, 0, chunk_e0(c), 0);
     };
     auto load_w2 = [&](int g, int c) {
       const uint32_t st = (uint32_t)(g & 1), bar = w2_bar + 8u * st;
       const int e0 = chunk_e0(c), n = min(EC, p.E - e0) * (F16 ? 2 : 4);
       const int rows = p.b2 ? 10 : 9;
-      mbar_expect_tx(bar, w2_bytes + (uint32_t)(rows * n));
-      tma_load_3d(sW2 + st * w2_stage, &p.tmW2, bar, e0, 0, 0);
+      expect_tx_warp(bar, w2_bytes + (uint32_t)(rows * n));
+      load_3d_warp(sW2 + st * w2_stage, &p.tmW2, bar, e0, 0, 0);
       for (int t = 0; t < rows; ++t)
-        ir_bulk_load(sWD + st * WD_STAGE + (uint32_t)t * WD_ROW,
+        ir_bulk_load_warp(sWD + st * WD_STAGE + (uint32_t)t * WD_ROW,
                      reinterpret_cast<const uint8_t *>(t < 9 ? p.w2 : p.b2) + ((int64_t)(t % 9) * p.E + e0) * (F16 ? 2 : 4),
                      (uint32_t)n, bar);
     };
     auto load_x = [&](int t) {
       const Tile o = tile_of(t);
-      mbar_expect_tx(x_bar, (uint32_t)(p.kcs * pin * p.bk) * 2u);
+      expect_tx_warp(x_bar, (uint32_t)(p.kcs * pin * p.bk) * 2u);
       for (int k = 0; k < p.kcs; ++k)
-        tma_load_4d(sX + (uint32_t)k * p.x_bytes, &p.tmX, x_bar, k * p.bk, o.q0 * ST - 1, o.p0 * ST - 1, o.n);
+        load_4d_warp(sX + (uint32_t)k * p.x_bytes, &p.tmX, x_bar, k * p.bk, o.q0 * ST - 1, o.p0 * ST - 1, o.n);
     };
     auto gemm1 = [&](int g) {
       const uint32_t w = sW1 + (uint32_t)(g & 1) * w1_stage;
@@ -294,24 +296,24 @@ __global__ void __launch_bounds__(IR_THREADS, 2) ir_kernel(const __grid_constant
       for (int b = 0; b < blocks; ++b) {
         const uint32_t d = d1 + (uint32_t)(b * EC);
         // the bias: a column of ones per part of it, zero for pixels outside the image
-        mma_lohi(d, (uint32_t)a1 + (uint32_t)b * ((128u * ONE_ROW) >> 4), (uint32_t)(a1 >> 32), (uint32_t)b1,
+        mma_warp(d, (uint32_t)a1 + (uint32_t)b * ((128u * ONE_ROW) >> 4), (uint32_t)(a1 >> 32), (uint32_t)b1,
                  (uint32_t)(b1 >> 32), IDESC0 | ((uint32_t)(EC >> 3) << 17), 0u);
 #pragma unroll 1
         for (int k = 0; k < p.kcs; ++k)
 #pragma unroll 4
           for (int kk = 0; kk < kks; ++kk)
-            mma_lohi(d, (uint32_t)a0 + (uint32_t)k * x_step + (uint32_t)b * a_block + 2u * kk, a_hi,
+            mma_warp(d, (uint32_t)a0 + (uint32_t)k * x_step + (uint32_t)b * a_block + 2u * kk, a_hi,
                      (uint32_t)b0 + (uint32_t)k * w_step + 2u * kk, b_hi, IDESC0 | ((uint32_t)(EC >> 3) << 17), 1u);
       }
-      tc_commit(g1_bar);
+      commit_warp(g1_bar);
     };
     auto gemm2 = [&](int g, int c) {
       const uint64_t a0 = make_smem_desc(sDW, EC), b0 = make_smem_desc(sW2 + (uint32_t)(g & 1) * w2_stage, EC);
 #pragma unroll
       for (int kk = 0; kk < EC / 16; ++kk)
-        mma_lohi(d2, (uint32_t)a0 + 2u * kk, (uint32_t)(a0 >> 32), (uint32_t)b0 + 2u * kk, (uint32_t)(b0 >> 32),
+        mma_warp(d2, (uint32_t)a0 + 2u * kk, (uint32_t)(a0 >> 32), (uint32_t)b0 + 2u * kk, (uint32_t)(b0 >> 32),
                  IDESC0 | ((uint32_t)(p.Kp >> 3) << 17), (c | kk) ? 1u : 0u);
-      tc_commit(g2_bar);
+      commit_warp(g2_bar);
     };
     auto first_filters = [&]() {
       load_w1(0, 0);
@@ -328,26 +330,26 @@ __global__ void __launch_bounds__(IR_THREADS, 2) ir_kernel(const __grid_constant
       const int before = c == 0 ? mine - 1 : c - 1, after = c + 1 == mine ? 0 : c + 1;
       if (g < chunks_all) {
         // the last chunk has been drained, this tile's ones are there
-        if (!mbar_wait(drained_bar, g & 1, abort_flag)) err_code = 1;
+        if (!mbar_wait_warp(drained_bar, g & 1, abort_flag)) err_code = 1;
         if (err_code) break;
         tc_fence_after();
         if (c == 0) load_x(t);
         if (g + 1 < chunks_all) load_w1(g + 1, after);
-        if (!mbar_wait(w1_bar + 8u * (g & 1), (g >> 1) & 1, abort_flag)) err_code = 2;
-        if (c == 0 && !mbar_wait(x_bar, xs & 1, abort_flag)) err_code = 3;
+        if (!mbar_wait_warp(w1_bar + 8u * (g & 1), (g >> 1) & 1, abort_flag)) err_code = 2;
+        if (c == 0 && !mbar_wait_warp(x_bar, xs & 1, abort_flag)) err_code = 3;
         if (err_code) break;
         tc_fence_after();
         gemm1(g);
         if (g >= 2) {   // these filters replace those of chunk g - 2
-          if (!mbar_wait(g2_bar, g & 1, abort_flag)) err_code = 4;
+          if (!mbar_wait_warp(g2_bar, g & 1, abort_flag)) err_code = 4;
           if (err_code) break;
           load_w2(g, c);
         }
       }
       if (g >= 1) {
         const int h = g - 1;
-        if (!mbar_wait(dwdone_bar, h & 1, abort_flag)) err_code = 5;
-        if (!mbar_wait(w2_bar + 8u * (h & 1), (h >> 1) & 1, abort_flag)) err_code = 6;
+        if (!mbar_wait_warp(dwdone_bar, h & 1, abort_flag)) err_code = 5;
+        if (!mbar_wait_warp(w2_bar + 8u * (h & 1), (h >> 1) & 1, abort_flag)) err_code = 6;
         if (err_code) break;
         tc_fence_after();
         gemm2(h, before);

@@ -183,6 +183,7 @@ struct TcConvArgs {
 struct StemPoolArgs {
   const bf16 *x;      // padded channels-last rows [N][H][row_bytes / 2] (launch_pad_input_bf16)
   const bf16 *w;      // launch_pack_stem_bf16 layout
+  const bf16 *w_fold; // launch_pack_fold_bf16 layout, or null
   const float *bias;  // [K] or null
   bf16 *y;            // pooled output, NHWC bf16 [N][PP][QP][K]
   int N, H, row_bytes, w_step_bytes;
