@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
     }
   } else if (warp == 11 || warp == 12) {
     // ------------------------------------------------------------ slabs of y
-    if (lane == 0) {
+    {
       const int me = warp - 11, per_tile = 2 * chunks;
       // hand-outs: slab number `r` of this CTA is slab r_sl of tile r_tile, in buffer r_buf
       int r_tile = blockIdx.x, r_sl = me, r_buf = me;
@@ -296,10 +296,10 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
         if (r_tile >= p.total_tiles) return;
         if constexpr (RES) {
           const TcTile tl = pixels(r_tile);
-          mbar_expect_tx(s_ready(r_buf), (uint32_t)p.rows * 128u);
-          tma_load_4d(sS + r_buf * PR_BLOCK, &p.tmR, s_ready(r_buf), r_sl * 64, tl.q0, tl.p0, tl.n0);
+          expect_tx_warp(s_ready(r_buf), (uint32_t)p.rows * 128u);
+          load_4d_warp(sS + r_buf * PR_BLOCK, &p.tmR, s_ready(r_buf), r_sl * 64, tl.q0, tl.p0, tl.n0);
         } else {
-          mbar_arrive(s_ready(r_buf));
+          arrive_warp(s_ready(r_buf));
         }
         r_buf += 2;
         if (r_buf >= nS) r_buf -= nS;
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
       // the slab stored before the newest is free when product 2 has been made with it
       auto give_back = [&]() {
         if (last < 0) return true;
-        if (!mbar_wait(s_read(last), last_phase, abort_flag)) {
+        if (!mbar_wait_warp(s_read(last), last_phase, abort_flag)) {
           err_code = 6;
           return false;
         }
@@ -325,11 +325,11 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
       for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x) {
         const TcTile tl = pixels(tile);
         for (int sl = me; sl < per_tile; sl += 2) {
-          if (!mbar_wait(s_full(buf), phase, abort_flag)) {
+          if (!mbar_wait_warp(s_full(buf), phase, abort_flag)) {
             err_code = 6;
             break;
           }
-          tma_store_4d(&p.tmY, sS + buf * PR_BLOCK, sl * 64, tl.q0, tl.p0, tl.n0);
+          store_4d_warp(&p.tmY, sS + buf * PR_BLOCK, sl * 64, tl.q0, tl.p0, tl.n0);
           tma_store_commit();
           tma_store_wait_read<1>();
           if (!give_back()) break;
@@ -346,20 +346,20 @@ __global__ void __launch_bounds__(PR_THREADS, 1) tc_pair_kernel(const __grid_con
     }
   } else if (warp == 13) {
     // ------------------------------------------------------------ slabs of t
-    if (lane == 0) {
+    {
       int b = 0;
       uint32_t phase = 0;
       for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x) {
         const TcTile tl = pixels(tile);
         for (int c = 0; c < p.K2; c += 32) {
-          if (!mbar_wait(t_full(b), phase, abort_flag)) {
+          if (!mbar_wait_warp(t_full(b), phase, abort_flag)) {
             err_code = 8;
             break;
           }
-          tma_store_4d(&p.tmT, sT + b * PR_T, c, tl.q0, tl.p0, tl.n0);
+          store_4d_warp(&p.tmT, sT + b * PR_T, c, tl.q0, tl.p0, tl.n0);
           tma_store_commit();
           tma_store_wait_read<0>();
-          mbar_arrive(t_empty(b));
+          arrive_warp(t_empty(b));
           b ^= 1;
           if (b == 0) phase ^= 1u;
         }

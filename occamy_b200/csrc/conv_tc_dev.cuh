@@ -448,6 +448,20 @@ __device__ __forceinline__ void load_3d_pair_warp(uint32_t dst, const CUtensorMa
       "l"(m), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
+__device__ __forceinline__ void arrive_warp(uint32_t a) {
+  asm volatile(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q mbarrier.arrive.shared::cta.b64 _, [%0];\n}" ::"r"(a)
+      : "memory");
+}
+// (a store's group belongs to the elected lane; the others commit and wait for empty ones)
+__device__ __forceinline__ void store_4d_warp(const CUtensorMap *m, uint32_t src, int c0, int c1, int c2, int c3) {
+  asm volatile(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];\n}" ::"l"(m),
+      "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
 __device__ __forceinline__ void commit_warp(uint32_t bar) {
   asm volatile(
       "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
@@ -962,7 +976,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
     // because a single thread's issue rate (TMA store + residual load + bookkeeping per slab)
     // limits the layers whose tiles are short.
     if constexpr (!F32) {
-      if (lane == 0) {
+      {
         const uint32_t me = (uint32_t)(warp - STORE_WARP);
         auto nslab_of = [&](const TcTile &t) { return min(NSLAB, (p.K - t.k0 + DC - 1) / DC); };
         // cursor over the slabs this thread makes ready: (tile, slab) of slab number r_next
@@ -1000,18 +1014,18 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
           if (uniform) {
             if (left == 0) return;
             --left;
-            mbar_arrive(rfull_bar(rb));
+            arrive_warp(rfull_bar(rb));
             rb += TC_NSTORE;
             if (rb >= (uint32_t)dbuf) rb -= (uint32_t)dbuf;
             return;
           }
           if (r_tile >= p.total_tiles) return;
           if constexpr (RES) {
-            mbar_expect_tx(rfull_bar(rb), (uint32_t)rows_valid * DC * 2u);
-            tma_load_4d(sD + rb * SLAB_BYTES, &p.tmR, rfull_bar(rb), rt_.k0 + r_sl * DC, rt_.q0,
+            expect_tx_warp(rfull_bar(rb), (uint32_t)rows_valid * DC * 2u);
+            load_4d_warp(sD + rb * SLAB_BYTES, &p.tmR, rfull_bar(rb), rt_.k0 + r_sl * DC, rt_.q0,
                         rt_.p0, rt_.n0);
           } else {
-            mbar_arrive(rfull_bar(rb));
+            arrive_warp(rfull_bar(rb));
           }
           r_next += TC_NSTORE;
           rb += TC_NSTORE;
@@ -1029,12 +1043,12 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
           const int nslab = nslab_of(tl);
           for (int sl = 0; sl < nslab; ++sl, ++d) {
             if (d % TC_NSTORE != me) continue;
-            if (!TCT_WAIT(0, mbar_wait(dfull_bar(b), ph, abort_flag))) {
+            if (!TCT_WAIT(0, mbar_wait_warp(dfull_bar(b), ph, abort_flag))) {
               err_code = 6;
               break;
             }
             if (!ghost)   // the duplicate tile of an odd last pair is computed, not stored
-              tma_store_4d(&p.tmD, sD + b * SLAB_BYTES, tl.k0 + sl * DC, POOL ? tl.q0 >> 1 : tl.q0,
+              store_4d_warp(&p.tmD, sD + b * SLAB_BYTES, tl.k0 + sl * DC, POOL ? tl.q0 >> 1 : tl.q0,
                            POOL ? tl.p0 >> 1 : tl.p0, tl.n0);
             tma_store_commit();
             // Up to store_pend of my earlier stores may still be reading their buffers; the

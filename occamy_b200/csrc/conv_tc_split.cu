@@ -251,20 +251,17 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   const int ahead = min(stages, mine);        // k-steps that need no stage to become free
 
   // (tap, channel block) of a k-step of this CTA
-  // (as a warp, or by one of its lanes)
-  auto load_b = [&](int i, int s, auto as_warp) {
+  auto load_b = [&](int i, int s) {
     const int k = ks0 + i;
     const bool second = k >= p.ksteps1;
     const int t = second ? 0 : (int)tc_fdiv((uint32_t)k, p.div_cb);
     const CUtensorMap *m = second ? &p.tmB2 : &p.tmB;
     const int c = (second ? k - p.ksteps1 : k - t * p.cblocks) * bk;
 #pragma unroll
-    for (int j = 0; j < PARTS; ++j) {
-      if constexpr (decltype(as_warp)::value) load_3d_warp(sB + s * b_bytes + j * b_tile, m, full_bar(s), c, tl.k0, t * PARTS + j);
-      else tma_load_3d(sB + s * b_bytes + j * b_tile, m, full_bar(s), c, tl.k0, t * PARTS + j);
-    }
+    for (int j = 0; j < PARTS; ++j)
+      load_3d_warp(sB + s * b_bytes + j * b_tile, m, full_bar(s), c, tl.k0, t * PARTS + j);
   };
-  auto load_a = [&](int i, int s, auto as_warp) {
+  auto load_a = [&](int i, int s) {
     const int k = ks0 + i;
     const bool second = k >= p.ksteps1;
     const int t = second ? 0 : (int)tc_fdiv((uint32_t)k, p.div_cb);
@@ -272,18 +269,16 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
     const int map = second ? p.map2 : tap.map, c = (second ? k - p.ksteps1 : k - t * p.cblocks) * bk;
     const int q = tl.q0 + (second ? 0 : tap.dw), h = tl.p0 + (second ? 0 : tap.dh);
 #pragma unroll
-    for (int j = 0; j < PARTS; ++j) {
-      if constexpr (decltype(as_warp)::value) load_4d_warp(sA + s * a_bytes + j * a_tile, &p.tmA[map + j], full_bar(s), c, q, h, tl.n0);
-      else tma_load_4d(sA + s * a_bytes + j * a_tile, &p.tmA[map + j], full_bar(s), c, q, h, tl.n0);
-    }
+    for (int j = 0; j < PARTS; ++j)
+      load_4d_warp(sA + s * a_bytes + j * a_tile, &p.tmA[map + j], full_bar(s), c, q, h, tl.n0);
   };
-  // The k-steps of the first ring turn are requested by one lane each: a single thread's chain of
-  // index arithmetic, arming arrival and request per k-step is time on the layer's critical path.
-  const int first = warp >= 4 ? warp - 4 + 4 * lane : SK_MAX_STAGES;
-  if (first < ahead && p.consts_ready) {
-    mbar_expect_tx(full_bar(first), tx_bytes);
-    load_b(first, first, std::false_type{});
-  }
+  // The k-steps of the first ring turn are requested by four warps in turn.
+  const int first = warp >= 4 ? warp - 4 : SK_MAX_STAGES;
+  if (p.consts_ready)
+    for (int i = first; i < ahead; i += 4) {
+      expect_tx_warp(full_bar(i), tx_bytes);
+      load_b(i, i);
+    }
   pdl_launch_dependents();
   pdl_wait();   // from here on memory that other kernels write is read and written
 
@@ -294,10 +289,10 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   const int items = nrows * G8;
   const int quad = warp & 3, part = warp >> 2, row = quad * 32 + lane;
 
-  if (first < ahead) {
-    if (!p.consts_ready) mbar_expect_tx(full_bar(first), tx_bytes);
-    load_a(first, first, std::false_type{});
-    if (!p.consts_ready) load_b(first, first, std::false_type{});
+  for (int i = first; i < ahead; i += 4) {
+    if (!p.consts_ready) expect_tx_warp(full_bar(i), tx_bytes);
+    load_a(i, i);
+    if (!p.consts_ready) load_b(i, i);
   }
   if (warp >= 4) {   // (the other four warps issue MMAs)
     const int i = (int)threadIdx.x - 128;
@@ -369,8 +364,8 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
           break;
         }
         expect_tx_warp(full_bar(s), tx_bytes);
-        load_b(i, s, std::true_type{});
-        load_a(i, s, std::true_type{});
+        load_b(i, s);
+        load_a(i, s);
         s += ni;
         if (s >= stages) {
           s -= stages;
