@@ -5,20 +5,24 @@
 // Input: the padded channels-last image rows the folded convolution uses,
 // x[n][h][wp][Cp] bf16 with 16 bytes per output-column step, so the A vector of output
 // column q (Cf = Sp*Cp values starting at pixel q*stride) is a window at byte 16*q of the
-// row and neighbouring windows overlap.  A row is copied to shared memory ONCE (bulk copy)
-// and the tensor core reads the overlapping windows in place: the operand descriptor is the
-// un-swizzled K-major form with 16 bytes from one 8-element K chunk to the next and 128
-// bytes from one group of 8 rows to the next, which is exactly "row m starts at byte 16*m".
-// One MMA row block is one convolution output row (Q <= 128 columns).
+// row and neighbouring windows overlap.  One MMA row block is one convolution output row
+// (Q <= 128 columns).
+//   TILED  TMA writes a row's windows out side by side (a tensor map whose pixel stride is shorter than its innermost
+//          extent), rows of 32, 64 or 128 bytes in the swizzle of that width.  Four times the bytes in shared memory.
+//   else   a row is copied once and the tensor core reads the overlapping windows in place: the operand descriptor is
+//          the un-swizzled K-major form with 16 bytes from one 8-element K chunk to the next and 128 bytes from one
+//          group of 8 rows to the next, "row m starts at byte 16*m".
+// 256 images of 224x224: 139 us tiled, 155 in place; the first where its shared memory suffices.
 //
 // One persistent CTA per SM works through units of (image, band of pooled rows):
-//   warp 0      producer (one lane): bulk-copies the weights once, then input rows into a ring
-//   2 warps     MMA issuers (one lane each, alternate convolution rows): per row R taps x
+//   warp 0      producer: the weights once, then input rows into a ring
+//   2 warps     MMA issuers (alternate convolution rows): per row R taps x
 //               Cf/16 tcgen05.mma (128 x 64 x 16) into one of four TMEM accumulators;
 //               release input rows
-//   8 warps     epilogue: accumulator -> + bias -> clamp -> bf16 -> convolution-row ring in
-//               shared memory (swizzled so that a warp's 128-byte rows spread over banks)
-//   8 warps     pool: max over the 3x3 windows of three ring rows -> global memory
+//   16 warps    epilogue: accumulator -> + bias -> clamp -> bf16, the largest of a window's three
+//               rows in registers (a thread owns 16 channels of one column) -> a buffer in shared
+//               memory (swizzled so that a warp's 128-byte rows spread over banks)
+//   4 warps     pool: the largest of three columns -> global memory
 // Every wait is bounded; a wait that runs out records a code and the kernel drains.
 #include "conv_tc_dev.cuh"
 #include "kernels.h"
@@ -28,38 +32,42 @@ namespace occ {
 
 namespace {
 
-constexpr int ST_EPI_WARPS = 8;    // two per TMEM lane quadrant, 32 channels each
-constexpr int ST_POOL_WARPS = 8;
-constexpr int ST_ISSUER_B = 2 + ST_EPI_WARPS + ST_POOL_WARPS;   // warp of the second MMA issuer
-constexpr int ST_THREADS = 32 * (ST_ISSUER_B + 1);
-constexpr int ST_NIN = 8;     // input ring slots (a slot holds stride_h rows)
-constexpr int ST_NCR = 6;     // convolution-row ring slots
+constexpr int ST_EPI_WARPS = 16;   // four per TMEM lane quadrant, 16 channels each
+constexpr int ST_POOL_WARPS = 4;
+constexpr int ST_ISSUERS = 2;
+// warps: producer, the first issuer, epilogue, pool, the other issuers
+constexpr int ST_ISSUER_B = 2 + ST_EPI_WARPS + ST_POOL_WARPS;
+constexpr int ST_THREADS = 32 * (ST_ISSUER_B + ST_ISSUERS - 1);
+constexpr int ST_MAX_CHUNKS = 8;   // of the input ring (StemParams::ring)
+constexpr int ST_NMR = 3;     // buffers of a pooled row before its columns are taken together
 constexpr int ST_NACC = 4;    // TMEM accumulators (64 columns each)
 constexpr int ST_K = 64;      // output channels
 
-struct StemParams {
+struct alignas(64) StemParams {
+  CUtensorMap tmX, tmW;   // TILED
   const bf16 *x;       // [N][H][row_bytes / 2]
   const bf16 *w;       // packed [R][Cf / 8][64][8]
   const float *bias;   // [64] or null
   bf16 *y;             // [N][PP][QP][64]
   int N, H, row_bytes;
-  int row_slot, slot_bytes;   // bytes reserved per input row / per group of stride_h rows
+  int in_row, slot_bytes;     // an input row in shared memory, a group of stride_h of them
+  int bk;                     // TILED: channels of a window there (16, 32 or 64)
+  int ring, chunk;            // groups the input ring holds, and how many of them one copy brings (powers of two)
   int G;                      // groups one convolution row reads
   int P, Q;            // convolution output
   int R, Cf, pad_h, stride_h;
   int PP, QP;          // pooled output
   int bands, band_rows, units;
-  int cr_bytes;        // bytes of one convolution-row ring slot
+  int mr_bytes;        // bytes of such a buffer
   float lo, hi;
   int descending;      // units are taken from the last to the first (Runtime::descending)
   int *err;
 };
 
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes,
-                                         uint32_t bar) {
+__device__ __forceinline__ void bulk_g2s_warp(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-          "r"(dst),
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n}" ::"r"(dst),
       "l"(src), "r"(bytes), "r"(bar)
       : "memory");
 }
@@ -77,9 +85,10 @@ __device__ __forceinline__ void mma_lohi_if(uint32_t valid, uint32_t d_tmem, uin
                                             uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
                                             uint32_t accumulate) {
   asm volatile(
-      "{\n.reg .pred p, q;\n.reg .b64 da, db;\n"
+      "{\n.reg .pred p, q, e;\n.reg .b64 da, db;\n"
       "setp.ne.b32 p, %6, 0;\n"
-      "setp.ne.b32 q, %7, 0;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "setp.ne.and.b32 q, %7, 0, e;\n"
       "mov.b64 da, {%1, %2};\n"
       "mov.b64 db, {%3, %4};\n"
       "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}" ::"r"(d_tmem),
@@ -92,13 +101,13 @@ __device__ __forceinline__ void mma_lohi_if(uint32_t valid, uint32_t d_tmem, uin
 // s0 + r / SH.
 template <int R, int KK, int SH>
 __device__ __forceinline__ void issue_row(uint32_t d_tmem, int r_lo, int r_hi, uint32_t s0,
-                                          uint32_t a_lo0, uint32_t a_hi, uint32_t slot_desc,
+                                          uint32_t ring, uint32_t a_lo0, uint32_t a_hi, uint32_t slot_desc,
                                           uint32_t row_desc, uint32_t b_lo0, uint32_t b_hi,
                                           uint32_t tap_desc, uint32_t kstep_desc, uint32_t idesc) {
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const uint32_t valid = (r >= r_lo && r <= r_hi) ? 1u : 0u;
-    const uint32_t s = (s0 + (uint32_t)(r / SH)) % ST_NIN;
+    const uint32_t s = (s0 + (uint32_t)(r / SH)) & (ring - 1u);
     const uint32_t a_lo = a_lo0 + s * slot_desc + (uint32_t)(r % SH) * row_desc;
     const uint32_t b_lo = b_lo0 + (uint32_t)r * tap_desc;
 #pragma unroll
@@ -108,58 +117,72 @@ __device__ __forceinline__ void issue_row(uint32_t d_tmem, int r_lo, int r_hi, u
   }
 }
 
-// byte offset of 16-byte chunk `c` (0..7) of pixel `px` in a convolution-row ring slot
-__device__ __forceinline__ uint32_t cr_off(int px, int c) {
+// ... of a row whose taps all lie inside the image.
+template <int R, int KK, int SH>
+__device__ __forceinline__ void issue_whole_row(uint32_t d_tmem, uint32_t s0, uint32_t ring, uint32_t a_lo0, uint32_t a_hi,
+                                                uint32_t slot_desc, uint32_t row_desc, uint32_t b_lo0, uint32_t b_hi,
+                                                uint32_t tap_desc, uint32_t kstep_desc, uint32_t idesc) {
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const uint32_t s = (s0 + (uint32_t)(r / SH)) & (ring - 1u);
+    const uint32_t a_lo = a_lo0 + s * slot_desc + (uint32_t)(r % SH) * row_desc, b_lo = b_lo0 + (uint32_t)r * tap_desc;
+#pragma unroll
+    for (int kk = 0; kk < KK; ++kk)
+      mma_warp(d_tmem, a_lo + 2 * kk, a_hi, b_lo + kk * kstep_desc, b_hi, idesc, (r | kk) ? 1u : 0u);
+  }
+}
+
+// byte offset of 16-byte chunk `c` (0..7) of pixel `px` in such a buffer
+__device__ __forceinline__ uint32_t mr_off(int px, int c) {
   return (uint32_t)(px * 128 + ((c ^ (px & 7)) << 4));
 }
 
-__global__ void __launch_bounds__(ST_THREADS, 1) stem_pool_kernel(const StemParams p) {
+template <bool TILED>
+__global__ void __launch_bounds__(ST_THREADS, 1) stem_pool_kernel(const __grid_constant__ StemParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t *base_ptr = smem_raw + (base - smem_u32(smem_raw));
-  const uint32_t w_bytes = (uint32_t)p.R * p.Cf * ST_K * 2;
+  const uint32_t w_tap = (uint32_t)(TILED ? p.bk : p.Cf) * ST_K * 2, w_bytes = (uint32_t)p.R * w_tap;
   const uint32_t sW = base;
   const uint32_t sIn = sW + ((w_bytes + 1023u) & ~1023u);
-  const uint32_t sCr = sIn + ST_NIN * p.slot_bytes;
-  const uint32_t sMisc = sCr + ST_NCR * p.cr_bytes;
+  // (the MMA rows beyond Q reach into what lies behind a row, 16 * 128 + 2 * Cf bytes at most: read, and left out)
+  const uint32_t sMr = sIn + ((p.ring * p.slot_bytes + 1023u) & ~1023u);
+  const uint32_t sMisc = sMr + ST_NMR * p.mr_bytes;
   uint8_t *misc_ptr = base_ptr + (sMisc - base);
   float *bias_s = reinterpret_cast<float *>(misc_ptr);                 // 64 floats
   uint64_t *bars = reinterpret_cast<uint64_t *>(misc_ptr + 256);
   const uint32_t bar0 = sMisc + 256;
   const uint32_t w_full = bar0;
   auto in_full = [&](int s) { return bar0 + 8u * (1 + s); };
-  auto in_empty = [&](int s) { return bar0 + 8u * (1 + ST_NIN + s); };
-  auto tfull = [&](int s) { return bar0 + 8u * (1 + 2 * ST_NIN + s); };
-  auto tempty = [&](int s) { return bar0 + 8u * (1 + 2 * ST_NIN + ST_NACC + s); };
-  auto cr_full = [&](int s) { return bar0 + 8u * (1 + 2 * ST_NIN + 2 * ST_NACC + s); };
-  auto cr_empty = [&](int s) { return bar0 + 8u * (1 + 2 * ST_NIN + 2 * ST_NACC + ST_NCR + s); };
-  constexpr int NBARS = 1 + 2 * ST_NIN + 2 * ST_NACC + 2 * ST_NCR;
+  auto in_empty = [&](int s) { return bar0 + 8u * (1 + ST_MAX_CHUNKS + s); };
+  auto tfull = [&](int s) { return bar0 + 8u * (1 + 2 * ST_MAX_CHUNKS + s); };
+  auto tempty = [&](int s) { return bar0 + 8u * (1 + 2 * ST_MAX_CHUNKS + ST_NACC + s); };
+  auto mr_full = [&](int s) { return bar0 + 8u * (1 + 2 * ST_MAX_CHUNKS + 2 * ST_NACC + s); };
+  auto mr_empty = [&](int s) { return bar0 + 8u * (1 + 2 * ST_MAX_CHUNKS + 2 * ST_NACC + ST_NMR + s); };
+  constexpr int NBARS = 1 + 2 * ST_MAX_CHUNKS + 2 * ST_NACC + 2 * ST_NMR;
   volatile uint32_t *tmem_holder = reinterpret_cast<volatile uint32_t *>(bars + NBARS);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + NBARS + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   constexpr uint32_t TMEM_COLS = ST_NACC * ST_K;
 
   if (threadIdx.x == 0) {
     mbar_init(w_full, 1);
-    for (int s = 0; s < ST_NIN; ++s) {
+    for (int s = 0; s < p.ring / p.chunk; ++s) {
       mbar_init(in_full(s), 1);
-      mbar_init(in_empty(s), 2);   // both MMA issuers hand a group back
+      mbar_init(in_empty(s), ST_ISSUERS);   // every MMA issuer hands a group back
     }
     for (int s = 0; s < ST_NACC; ++s) {
       mbar_init(tfull(s), 1);
       mbar_init(tempty(s), ST_EPI_WARPS);
     }
-    for (int s = 0; s < ST_NCR; ++s) {
-      mbar_init(cr_full(s), ST_EPI_WARPS);
-      mbar_init(cr_empty(s), ST_POOL_WARPS);
+    for (int s = 0; s < ST_NMR; ++s) {
+      mbar_init(mr_full(s), ST_EPI_WARPS);
+      mbar_init(mr_empty(s), ST_POOL_WARPS);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  // the tail of every input slot (past the row) is read by the MMA rows beyond Q: keep it finite
-  for (uint32_t i = threadIdx.x * 16u; i < (uint32_t)ST_NIN * p.slot_bytes; i += ST_THREADS * 16u)
-    *reinterpret_cast<uint4 *>(base_ptr + (sIn - base) + i) = make_uint4(0, 0, 0, 0);
   if (threadIdx.x < ST_K) bias_s[threadIdx.x] = p.bias ? p.bias[threadIdx.x] : 0.0f;
   fence_async_smem();
   if (warp == 2) {
@@ -188,233 +211,276 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stem_pool_kernel(const StemPara
     h_hi = min(2 * (i1 - 1) + 1, p.P - 1);
   };
 
+  const uint32_t chunks = (uint32_t)(p.ring / p.chunk);
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    // Input rows travel in groups of stride_h rows, one ring slot and one barrier per
-    // group: group g holds rows g*stride_h - pad_h ... + stride_h - 1, convolution row h
-    // reads groups h ... h + G - 1 and is the last reader of group h.
-    if (lane == 0) {
-      mbar_expect_tx(w_full, w_bytes);
-      bulk_g2s(sW, p.w, w_bytes, w_full);
-      uint32_t gq = 0;   // groups loaded so far
+    // Group g of a unit is rows (h_lo + g) * stride_h - pad_h ... + stride_h - 1; convolution row k of the unit reads
+    // groups k ... k + G - 1 and is the last reader of group k.  `chunk` groups lie next to one another in memory
+    // and come in one copy.
+    {
+      expect_tx_warp(w_full, w_bytes);
+      if constexpr (TILED) {
+        for (int r = 0; r < p.R; ++r) load_3d_warp(sW + r * w_tap, &p.tmW, w_full, 0, 0, r);
+      } else {
+        bulk_g2s_warp(sW, p.w, w_bytes, w_full);
+      }
+      uint32_t q = 0;   // chunks loaded so far
       for (int unit = blockIdx.x; unit < p.units && !err_code; unit += gridDim.x) {
         int n, i0, i1, h_lo, h_hi;
         unit_rows(unit, n, i0, i1, h_lo, h_hi);
-        const uint8_t *img = reinterpret_cast<const uint8_t *>(p.x) +
-                             (size_t)n * p.H * p.row_bytes;
-        for (int g = h_lo; g <= h_hi + p.G - 1; ++g, ++gq) {
-          const uint32_t s = gq % ST_NIN, ph = (gq / ST_NIN) & 1u;
-          if (!mbar_wait_sleepy(in_empty(s), ph ^ 1u, abort_flag)) {
+        const uint8_t *img = reinterpret_cast<const uint8_t *>(p.x) + (size_t)n * p.H * p.row_bytes;
+        const int groups = h_hi - h_lo + p.G;
+        for (int g = 0; g < groups; g += p.chunk, ++q) {
+          const uint32_t s = q % chunks, ph = (q / chunks) & 1u;
+          if (!mbar_wait_warp(in_empty(s), ph ^ 1u, abort_flag)) {
             err_code = 1;
             break;
           }
-          const int j0 = g * p.stride_h - p.pad_h;
-          int valid = 0;
-          for (int k = 0; k < p.stride_h; ++k) valid += (j0 + k >= 0 && j0 + k < p.H);
-          mbar_expect_tx(in_full(s), (uint32_t)(valid * p.row_bytes));   // 0 bytes: a plain arrival
-          for (int k = 0; k < p.stride_h; ++k)
-            if (j0 + k >= 0 && j0 + k < p.H)
-              bulk_g2s(sIn + s * p.slot_bytes + k * p.row_slot, img + (size_t)(j0 + k) * p.row_bytes,
-                       (uint32_t)p.row_bytes, in_full(s));
+          const int j0 = (h_lo + g) * p.stride_h - p.pad_h;
+          if constexpr (TILED) {   // (rows outside the image arrive as zeros)
+            expect_tx_warp(in_full(s), (uint32_t)(p.chunk * p.slot_bytes));
+            load_4d_warp(sIn + s * p.chunk * p.slot_bytes, &p.tmX, in_full(s), 0, 0, j0, n);
+            continue;
+          }
+          const int lo = max(j0, 0), hi = min(j0 + min(p.chunk, groups - g) * p.stride_h, p.H);
+          const uint32_t bytes = hi > lo ? (uint32_t)((hi - lo) * p.row_bytes) : 0u;
+          expect_tx_warp(in_full(s), bytes);   // 0 bytes: a plain arrival
+          if (bytes)
+            bulk_g2s_warp(sIn + s * p.chunk * p.slot_bytes + (lo - j0) * p.row_bytes, img + (size_t)lo * p.row_bytes, bytes,
+                     in_full(s));
         }
       }
     }
-  } else if (warp == 1 || warp == ST_ISSUER_B) {
+  } else if (warp == 1 || warp >= ST_ISSUER_B) {
     // ------------------------------------------------------------ MMA issuers
     // Two threads (in two warps) take alternate convolution rows: the MMAs are short (64
     // columns) and one thread cannot issue them as fast as the tensor core retires them.
     // Both read every input group, so a group goes back to the producer when both have
     // committed it (each does so once it will not read the group again).
-    if (lane == 0) {
-      const int me = warp == 1 ? 0 : 1;
+    {
+      const int me = warp == 1 ? 0 : warp - ST_ISSUER_B + 1;
       constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) |
                                  ((uint32_t)(ST_K >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-      if (!mbar_wait_hot(w_full, 0, abort_flag)) err_code = 2;
-      uint32_t gbase = 0;   // ring index of the unit's first group
+      if (!mbar_wait_warp(w_full, 0, abort_flag)) err_code = 2;
+      uint32_t gbase = 0;   // ring index of the unit's first group (whole chunks)
       uint32_t cbase = 0;   // convolution rows before this unit
-      const int kk_n = p.Cf / 16;
-      const uint64_t adesc0 = desc_plain(sIn, 16, 128);
-      const uint64_t bdesc0 = desc_plain(sW, ST_K * 16, 128);
+      const int kk_n = (TILED ? p.bk : p.Cf) / 16;
+      const uint64_t adesc0 = TILED ? make_smem_desc(sIn, p.bk) : desc_plain(sIn, 16, 128);
+      const uint64_t bdesc0 = TILED ? make_smem_desc(sW, p.bk) : desc_plain(sW, ST_K * 16, 128);
       const uint32_t a_lo0 = (uint32_t)adesc0, a_hi = (uint32_t)(adesc0 >> 32);
       const uint32_t b_lo0 = (uint32_t)bdesc0, b_hi = (uint32_t)(bdesc0 >> 32);
       const uint32_t slot_desc = (uint32_t)p.slot_bytes >> 4;        // descriptor steps
-      const uint32_t row_desc = (uint32_t)p.row_slot >> 4;
-      const uint32_t tap_desc = ((uint32_t)p.Cf * ST_K * 2) >> 4;
-      const uint32_t kstep_desc = (2 * ST_K * 16) >> 4;
+      const uint32_t row_desc = (uint32_t)p.in_row >> 4, ring = (uint32_t)p.ring;
+      const uint32_t tap_desc = w_tap >> 4;
+      const uint32_t kstep_desc = TILED ? 2u : (2 * ST_K * 16) >> 4;
       for (int unit = blockIdx.x; unit < p.units && !err_code; unit += gridDim.x) {
         int n, i0, i1, h_lo, h_hi;
         unit_rows(unit, n, i0, i1, h_lo, h_hi);
         const int rows = h_hi - h_lo + 1;
-        const int groups = rows + p.G - 1;        // groups the producer loads for this unit
+        const int groups = (rows + p.G - 1 + p.chunk - 1) / p.chunk * p.chunk;   // of the chunks loaded for this unit
         int waited = 0, released = 0;             // groups (unit-relative) waited for / committed
+        auto arrived = [&](int upto) {
+          for (; waited < upto; waited += p.chunk) {
+            const uint32_t q = (gbase + (uint32_t)waited) / (uint32_t)p.chunk;
+            if (!mbar_wait_warp(in_full(q % chunks), (q / chunks) & 1u, abort_flag)) {
+              err_code = 4;
+              return false;
+            }
+          }
+          return true;
+        };
+        // chunks whose groups are all below `upto` are of no more use to me (none is handed back before it has come, or this thread
+        // could be a turn of the ring ahead of the others)
+        auto release = [&](int upto) {
+          for (; released + p.chunk <= upto; released += p.chunk) {
+            if (!arrived(released + 1)) return;
+            commit_warp(in_empty((gbase + (uint32_t)released) / (uint32_t)p.chunk % chunks));
+          }
+        };
         // rows of the unit whose running number (over all units) has my parity
-        for (int k = (int)((cbase + (uint32_t)me) & 1u); k < rows && !err_code; k += 2) {
+        for (int k = (int)(((uint32_t)me + ST_ISSUERS - cbase % ST_ISSUERS) % ST_ISSUERS); k < rows && !err_code; k += ST_ISSUERS) {
           const uint32_t c = cbase + (uint32_t)k;
           const uint32_t a = c % ST_NACC, aph = (c / ST_NACC) & 1u;
-          if (!mbar_wait_hot(tempty(a), aph ^ 1u, abort_flag)) {
+          if (!mbar_wait_warp(tempty(a), aph ^ 1u, abort_flag)) {
             err_code = 3;
             break;
           }
-          for (; waited < k + p.G; ++waited) {     // row k reads groups k ... k + G - 1
-            const uint32_t gq = gbase + (uint32_t)waited;
-            if (!mbar_wait_hot(in_full(gq % ST_NIN), (gq / ST_NIN) & 1u, abort_flag)) err_code = 4;
-          }
-          if (err_code) break;
+          if (!arrived(k + p.G)) break;            // row k reads groups k ... k + G - 1
           tc_fence_after();
           // taps whose input row lies inside the image (a row of padding contributes nothing)
           const int h = h_lo + k;
           const int jb = h * p.stride_h - p.pad_h;
           const int r_lo = max(0, -jb), r_hi = min(p.R - 1, p.H - 1 - jb);
           const uint32_t d_tmem = tmem_base + a * ST_K;
-          const uint32_t s0 = (gbase + (uint32_t)k) % ST_NIN;
+          const uint32_t s0 = (gbase + (uint32_t)k) & (ring - 1u);
           // The issue code is straight-line: every taken branch costs the issuing thread more
           // than an MMA.
-          if (p.R == 7 && kk_n == 2 && p.stride_h == 2) {
-            issue_row<7, 2, 2>(d_tmem, r_lo, r_hi, s0, a_lo0, a_hi, slot_desc, row_desc, b_lo0, b_hi,
+          if (p.R == 7 && kk_n == 2 && p.stride_h == 2 && r_lo == 0 && r_hi == 6) {
+            issue_whole_row<7, 2, 2>(d_tmem, s0, ring, a_lo0, a_hi, slot_desc, row_desc, b_lo0, b_hi, tap_desc, kstep_desc,
+                                     IDESC);
+          } else if (p.R == 7 && kk_n == 2 && p.stride_h == 2) {
+            issue_row<7, 2, 2>(d_tmem, r_lo, r_hi, s0, ring, a_lo0, a_hi, slot_desc, row_desc, b_lo0, b_hi,
                                tap_desc, kstep_desc, IDESC);
           } else {
             uint32_t accumulate = 0;
             for (int r = r_lo; r <= r_hi; ++r) {
-              const uint32_t s = (s0 + (uint32_t)(r / p.stride_h)) % ST_NIN;
+              const uint32_t s = (s0 + (uint32_t)(r / p.stride_h)) & (ring - 1u);
               const uint32_t a_lo = a_lo0 + s * slot_desc + (uint32_t)(r % p.stride_h) * row_desc;
               const uint32_t b_lo = b_lo0 + (uint32_t)r * tap_desc;
               // 16 K values further on: 32 bytes along the row for A, two K chunks for B
               for (int kk = 0; kk < kk_n; ++kk) {
-                mma_lohi(d_tmem, a_lo + 2 * kk, a_hi, b_lo + kk * kstep_desc, b_hi, IDESC, accumulate);
+                mma_warp(d_tmem, a_lo + 2 * kk, a_hi, b_lo + kk * kstep_desc, b_hi, IDESC, accumulate);
                 accumulate = 1;
               }
             }
           }
-          tc_commit(tfull(a));
-          // my next row is k + 2: groups below it are of no more use to me
-          for (; released < k + 2 && released < groups; ++released)
-            tc_commit(in_empty((gbase + (uint32_t)released) % ST_NIN));
+          commit_warp(tfull(a));
+          release(min(k + ST_ISSUERS, groups));   // (my next row)
         }
         // whatever of the unit I have not committed yet (also when none of its rows was mine)
-        for (; released < groups; ++released)
-          tc_commit(in_empty((gbase + (uint32_t)released) % ST_NIN));
+        if (!err_code) release(groups);
         gbase += (uint32_t)groups;
         cbase += (uint32_t)rows;
       }
     }
   } else if (warp < 2 + ST_EPI_WARPS) {
     // ------------------------------------------------------------ epilogue
+    // The accumulator of the next row is requested before this one's is worked on.  What bounds the kernel: a row's 14
+    // MMAs (680 cycles of the tensor core, 48 each whatever N up to 64), and the chain from a row's last product to its
+    // accumulator being free again, which sixteen warps shorten: 256 images at 224x224, 167 us with eight warps here, eight
+    // for 3x3 windows of a ring of rows, and issuers and loader that were single lanes; eight and four 160; sixteen and
+    // four 137 to 139; three issuers 148, one 184.
     const int quad = warp & 3;               // TMEM lane quadrant this warp may read
-    const int half = (warp - 2) >> 2;        // channels [32 * half, 32 * half + 32)
+    const int part = (warp - 2) >> 2;        // channels [16 * part, 16 * part + 16)
     const int px = quad * 32 + lane;         // convolution output column
     const float lo = p.lo, hi = p.hi;
     const bool relu_only = lo == 0.0f && hi == INFINITY;
-    uint32_t off[4];                         // this thread's four 16-byte pieces of a ring row
+    uint32_t off[2];                         // this thread's two 16-byte pieces of a buffer
 #pragma unroll
-    for (int k = 0; k < 4; ++k) off[k] = cr_off(px, half * 4 + k);
-    uint32_t c = 0;
-    for (int unit = blockIdx.x; unit < p.units && !err_code; unit += gridDim.x) {
-      int n, i0, i1, h_lo, h_hi;
-      unit_rows(unit, n, i0, i1, h_lo, h_hi);
-      for (int h = h_lo; h <= h_hi; ++h, ++c) {
-        const uint32_t a = c % ST_NACC, aph = (c / ST_NACC) & 1u;
-        const uint32_t cs = c % ST_NCR, cph = (c / ST_NCR) & 1u;
-        if (!mbar_wait_sleepy(tfull(a), aph, abort_flag)) {
-          err_code = 5;
-          break;
+    for (int k = 0; k < 2; ++k) off[k] = mr_off(px, part * 2 + k);
+    const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + part * 16;
+    uint32_t c = 0, pooled = 0;              // rows and pooled rows so far
+    int unit = blockIdx.x, n, i0, i1, h_lo = 0, h_hi = 0, h = 0;
+    uint32_t m[8], prev[8];                 // largest so far of the window's rows; its last row, the next one's first
+    auto request = [&](uint32_t *r) -> bool {   // the accumulator of row `c`
+      if (!mbar_wait_hot(tfull(c % ST_NACC), (c / ST_NACC) & 1u, abort_flag)) {
+        err_code = 5;
+        return false;
+      }
+      tc_fence_after();
+      tc_ld16(t_row + (c % ST_NACC) * ST_K, r);
+      return true;
+    };
+    // one row, whose accumulator arrives in `r`; false when it was the last
+    auto row = [&](uint32_t *r, uint32_t *next) -> bool {
+      const int this_h = h, this_lo = h_lo;
+      tc_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tempty(c % ST_NACC));
+      ++c;
+      if (++h > h_hi) {
+        unit += gridDim.x;
+        if (unit < p.units) {
+          unit_rows(unit, n, i0, i1, h_lo, h_hi);
+          h = h_lo;
         }
-        tc_fence_after();
-        uint32_t r[32];
-        tc_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + a * ST_K + half * 32, r);
-        tc_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(tempty(a));
-        uint32_t pk[16];
-        const float4 *b4 = reinterpret_cast<const float4 *>(bias_s + half * 32);
+      }
+      const bool more = unit < p.units;
+      if (more && !request(next)) return false;
+      uint32_t pk[8];
+      const float4 *b4 = reinterpret_cast<const float4 *>(bias_s + part * 16);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float4 b = b4[j];
+        const uint64_t v0 =
+            f2_add(f2_pack(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1])), f2_pack(b.x, b.y));
+        const uint64_t v1 =
+            f2_add(f2_pack(__uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3])), f2_pack(b.z, b.w));
+        if (relu_only) {
+          pk[2 * j] = f2_to_bf16x2_relu(v0);
+          pk[2 * j + 1] = f2_to_bf16x2_relu(v1);
+        } else {
+          float x0, x1, x2, x3;
+          f2_unpack(v0, x0, x1);
+          f2_unpack(v1, x2, x3);
+          pk[2 * j] = f2_to_bf16x2(f2_pack(tc_clip(x0, lo, hi), tc_clip(x1, lo, hi)));
+          pk[2 * j + 1] = f2_to_bf16x2(f2_pack(tc_clip(x2, lo, hi), tc_clip(x3, lo, hi)));
+        }
+      }
+      // Pooled row i takes rows 2i - 1 ... 2i + 1, those of them that exist.
+      if (this_h & 1) {
+        if (this_h == this_lo) {   // the unit's first row belongs to the window above as well
+#pragma unroll
+          for (int j = 0; j < 8; ++j) prev[j] = pk[j];
+          return more;
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const float4 b = b4[j];
-          const uint64_t v0 = f2_add(f2_pack(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1])),
-                                     f2_pack(b.x, b.y));
-          const uint64_t v1 =
-              f2_add(f2_pack(__uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3])),
-                     f2_pack(b.z, b.w));
-          if (relu_only) {
-            pk[2 * j] = f2_to_bf16x2_relu(v0);
-            pk[2 * j + 1] = f2_to_bf16x2_relu(v1);
-          } else {
-            float x0, x1, x2, x3;
-            f2_unpack(v0, x0, x1);
-            f2_unpack(v1, x2, x3);
-            pk[2 * j] = f2_to_bf16x2(f2_pack(tc_clip(x0, lo, hi), tc_clip(x1, lo, hi)));
-            pk[2 * j + 1] = f2_to_bf16x2(f2_pack(tc_clip(x2, lo, hi), tc_clip(x3, lo, hi)));
-          }
+          m[j] = tc_max2<false>(m[j], pk[j]);
+          prev[j] = pk[j];
         }
-        if (!mbar_wait_sleepy(cr_empty(cs), cph ^ 1u, abort_flag)) {
-          err_code = 6;
-          break;
-        }
-        if (px < p.Q) {
-          uint8_t *row = base_ptr + (sCr - base) + cs * p.cr_bytes;
+      } else {
+        const bool first = this_h == 0;
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            *reinterpret_cast<uint4 *>(row + off[k]) =
-                make_uint4(pk[4 * k], pk[4 * k + 1], pk[4 * k + 2], pk[4 * k + 3]);
+        for (int j = 0; j < 8; ++j) m[j] = first ? pk[j] : tc_max2<false>(prev[j], pk[j]);
+        if (this_h != p.P - 1) return more;
+      }
+      const uint32_t buf = pooled % ST_NMR, buf_phase = (pooled / ST_NMR) & 1u;
+      uint8_t *mr = base_ptr + (sMr - base) + buf * p.mr_bytes;
+      ++pooled;
+      if (!mbar_wait_hot(mr_empty(buf), buf_phase ^ 1u, abort_flag)) {
+        err_code = 6;
+        return false;
+      }
+      if (px < p.Q) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+          *reinterpret_cast<uint4 *>(mr + off[k]) = make_uint4(m[4 * k], m[4 * k + 1], m[4 * k + 2], m[4 * k + 3]);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(mr_full(buf));
+      return more;
+    };
+    if (unit < p.units) {
+      unit_rows(unit, n, i0, i1, h_lo, h_hi);
+      h = h_lo;
+      uint32_t ra[16], rb[16];
+      if (request(ra)) {
+#pragma unroll 1
+        while (row(ra, rb) && row(rb, ra)) {
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(cr_full(cs));
       }
     }
-  } else if (warp < ST_ISSUER_B) {
+  } else {
     // ------------------------------------------------------------ pool
     const int pt = threadIdx.x - 32 * (2 + ST_EPI_WARPS);
-    constexpr int PT = 32 * ST_POOL_WARPS;
-    uint32_t cbase = 0;                    // ring index of the unit's first convolution row
-    const int items = p.QP * 8;            // (pooled column, 16-byte channel chunk)
+    const int items = p.QP * 8;              // (pooled column, 16-byte channel chunk)
+    uint32_t pooled = 0;
     for (int unit = blockIdx.x; unit < p.units && !err_code; unit += gridDim.x) {
       int n, i0, i1, h_lo, h_hi;
       unit_rows(unit, n, i0, i1, h_lo, h_hi);
-      int rel = h_lo;   // next convolution row to hand back to the epilogue
-      for (int i = i0; i < i1 && !err_code; ++i) {
-        // Window rows / columns outside the image are replaced by the nearest inside one:
-        // a duplicate does not change a maximum, and the code stays free of branches.
-        const uint8_t *rows[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const int hh = min(max(2 * i - 1 + k, 0), p.P - 1);
-          const uint32_t cc = cbase + (uint32_t)(hh - h_lo);
-          if (!mbar_wait_sleepy(cr_full(cc % ST_NCR), (cc / ST_NCR) & 1u, abort_flag)) err_code = 7;
-          rows[k] = base_ptr + (sCr - base) + (cc % ST_NCR) * p.cr_bytes;
+      for (int i = i0; i < i1; ++i, ++pooled) {
+        const uint32_t buf = pooled % ST_NMR;
+        if (!mbar_wait_sleepy(mr_full(buf), (pooled / ST_NMR) & 1u, abort_flag)) {
+          err_code = 7;
+          break;
         }
-        if (err_code) break;
+        const uint8_t *mr = base_ptr + (sMr - base) + buf * p.mr_bytes;
         bf16 *yrow = p.y + ((size_t)n * p.PP + i) * p.QP * ST_K;
-        for (int it = pt; it < items; it += PT) {
+        for (int it = pt; it < items; it += 32 * ST_POOL_WARPS) {
           const int jq = it >> 3, ch = it & 7;
-          uint32_t o3[3];
-#pragma unroll
-          for (int k = 0; k < 3; ++k) o3[k] = cr_off(min(max(2 * jq - 1 + k, 0), p.Q - 1), ch);
-          uint4 v[9];
-#pragma unroll
-          for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int k = 0; k < 3; ++k) v[a * 3 + k] = *reinterpret_cast<const uint4 *>(rows[a] + o3[k]);
-          uint4 o;
-          uint32_t *ow = reinterpret_cast<uint32_t *>(&o);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            __nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162 *>(
-                reinterpret_cast<const uint32_t *>(&v[0]) + e);
-#pragma unroll
-            for (int t = 1; t < 9; ++t)
-              m = __hmax2_nan(m, *reinterpret_cast<const __nv_bfloat162 *>(
-                                     reinterpret_cast<const uint32_t *>(&v[t]) + e));
-            ow[e] = *reinterpret_cast<uint32_t *>(&m);
-          }
-          *reinterpret_cast<uint4 *>(yrow + (size_t)jq * ST_K + ch * 8) = o;
+          // (a column outside the image is replaced by the nearest inside it: a duplicate changes no maximum)
+          const uint4 a = *reinterpret_cast<const uint4 *>(mr + mr_off(max(2 * jq - 1, 0), ch));
+          const uint4 b = *reinterpret_cast<const uint4 *>(mr + mr_off(2 * jq, ch));
+          const uint4 d = *reinterpret_cast<const uint4 *>(mr + mr_off(min(2 * jq + 1, p.Q - 1), ch));
+          *reinterpret_cast<uint4 *>(yrow + (size_t)jq * ST_K + ch * 8) =
+              make_uint4(tc_max2<false>(tc_max2<false>(a.x, b.x), d.x), tc_max2<false>(tc_max2<false>(a.y, b.y), d.y),
+                         tc_max2<false>(tc_max2<false>(a.z, b.z), d.z), tc_max2<false>(tc_max2<false>(a.w, b.w), d.w));
         }
-        // convolution rows the next pooled row does not read go back to the epilogue
-        const int keep = i + 1 == i1 ? h_hi + 1 : 2 * (i + 1) - 1;
         __syncwarp();
-        for (; rel < keep && rel <= h_hi; ++rel)
-          if (lane == 0) mbar_arrive(cr_empty((cbase + (uint32_t)(rel - h_lo)) % ST_NCR));
+        if (lane == 0) mbar_arrive(mr_empty(buf));
       }
-      cbase += (uint32_t)(h_hi - h_lo + 1);
     }
   }
 
@@ -455,7 +521,7 @@ bool stem_pool_supported(const StemPoolArgs &a) {
   if (a.K != ST_K || a.Cf % 16 || a.Cf > 64 || a.R < 1 || a.R > 11) return false;
   if (a.w_step_bytes != 16 || a.row_bytes % 16 || a.row_bytes > 8192) return false;
   if (a.Q < 1 || a.Q > 128 || a.P < 1 || a.stride_h < 1 || a.stride_h > 4) return false;
-  if ((a.R - 1) / a.stride_h + 1 > ST_NIN - 2) return false;   // groups a row holds at once
+  if ((a.R - 1) / a.stride_h + 1 > 6) return false;   // groups a row holds at once
   if (a.PP != (a.P + 2 - 3) / 2 + 1 || a.QP != (a.Q + 2 - 3) / 2 + 1) return false;
   if ((uintptr_t)a.x % 16 || (uintptr_t)a.w % 16 || (uintptr_t)a.y % 16) return false;
   // the last window the tensor core reads for a real column must lie inside the row
@@ -478,9 +544,6 @@ bool launch_stem_pool(const StemPoolArgs &a, int *err_word, int num_sms, cudaStr
   memset(&p, 0, sizeof(p));
   p.x = a.x; p.w = a.w; p.bias = a.bias; p.y = a.y;
   p.N = a.N; p.H = a.H; p.row_bytes = a.row_bytes;
-  const int reach = 16 * 127 + a.Cf * 2;   // last byte + 1 the 128 MMA rows touch
-  p.row_slot = ((a.row_bytes > reach ? a.row_bytes : reach) + 127) / 128 * 128;
-  p.slot_bytes = p.row_slot * a.stride_h;
   p.G = (a.R - 1) / a.stride_h + 1;
   p.P = a.P; p.Q = a.Q; p.R = a.R; p.Cf = a.Cf; p.pad_h = a.pad_h; p.stride_h = a.stride_h;
   p.PP = a.PP; p.QP = a.QP;
@@ -495,15 +558,38 @@ bool launch_stem_pool(const StemPoolArgs &a, int *err_word, int num_sms, cudaStr
   p.band_rows = (a.PP + bands - 1) / bands;
   p.bands = (a.PP + p.band_rows - 1) / p.band_rows;
   p.units = a.N * p.bands;
-  p.cr_bytes = (a.Q * 128 + 1023) / 1024 * 1024;
-  const size_t w_bytes = (stem_pool_weight_bytes(a.R, a.Cf) + 1023) / 1024 * 1024;
-  const size_t smem = 1024 + w_bytes + (size_t)ST_NIN * p.slot_bytes + (size_t)ST_NCR * p.cr_bytes +
-                      256 + 8 * 64;
-  if (smem > (size_t)TC_SMEM_LIMIT || p.units == 0) return false;
+  p.mr_bytes = (a.Q * 128 + 1023) / 1024 * 1024;
+  // Shared memory: as many groups of input rows as fit, sixteen or eight.
+  size_t smem = 0;
+  auto fits = [&](bool tiled, int ring, int chunk) {
+    p.ring = ring;
+    p.chunk = chunk;
+    p.bk = a.Cf <= 16 ? 16 : a.Cf <= 32 ? 32 : 64;
+    p.in_row = tiled ? (a.Q + 7) / 8 * 8 * p.bk * 2 : a.row_bytes;
+    p.slot_bytes = p.in_row * a.stride_h;
+    const size_t w = ((size_t)a.R * (tiled ? p.bk : a.Cf) * ST_K * 2 + 1023) / 1024 * 1024;
+    smem = 1024 + w + ((size_t)ring * p.slot_bytes + 1023) / 1024 * 1024 + (size_t)ST_NMR * p.mr_bytes + 256 + 8 * 64;
+    return smem <= (size_t)TC_SMEM_LIMIT;
+  };
+  const bool tiled = a.w_fold && (fits(true, 16, 4) || fits(true, 8, 2));
+  if (!tiled && !fits(false, 16, 4) && !fits(false, 8, 1)) return false;
+  if (p.units == 0) return false;
+  if (tiled) {
+    const uint64_t dims[4] = {(uint64_t)a.Cf, (uint64_t)a.Q, (uint64_t)a.H, (uint64_t)a.N};
+    const uint64_t st[3] = {16, (uint64_t)a.row_bytes, (uint64_t)a.H * a.row_bytes};
+    const uint32_t box[4] = {(uint32_t)p.bk, (uint32_t)(a.Q + 7) / 8 * 8, (uint32_t)(a.stride_h * p.chunk), 1};
+    const uint64_t wdims[3] = {(uint64_t)a.Cf, ST_K, (uint64_t)a.R};
+    const uint64_t wst[2] = {(uint64_t)a.Cf * 2, (uint64_t)a.Cf * 2 * ST_K};
+    const uint32_t wbox[3] = {(uint32_t)p.bk, ST_K, 1};
+    if (!make_map(&p.tmX, a.x, 4, dims, st, box, p.bk * 2, true) || !make_map(&p.tmW, a.w_fold, 3, wdims, wst, wbox, p.bk * 2, true))
+      return false;
+  }
+  auto kernel = tiled ? stem_pool_kernel<true> : stem_pool_kernel<false>;
   static unsigned char attr_done[TC_MAX_DEVICES] = {};
-  if (tc_first_use_on_device(attr_done))
-    cudaFuncSetAttribute(stem_pool_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         TC_SMEM_LIMIT);
+  if (tc_first_use_on_device(attr_done)) {
+    cudaFuncSetAttribute(stem_pool_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_LIMIT);
+    cudaFuncSetAttribute(stem_pool_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_LIMIT);
+  }
   const int grid = p.units < num_sms ? p.units : num_sms;
   Runtime &r = rt();
   int prof_slot = -1;
@@ -517,7 +603,7 @@ bool launch_stem_pool(const StemPoolArgs &a, int *err_word, int num_sms, cudaStr
     OCC_CUDA(cudaEventRecord(r.prof_events[2 * prof_slot], s));
   }
   // at least half of the shared memory, so that one CTA (one TMEM allocation) runs per SM
-  tc_launch_pdl(stem_pool_kernel, grid, ST_THREADS, smem < 120 * 1024 ? 120 * 1024 : smem, s, p);
+  tc_launch_pdl(kernel, grid, ST_THREADS, smem < 120 * 1024 ? 120 * 1024 : smem, s, p);
   if (prof_slot >= 0) OCC_CUDA(cudaEventRecord(r.prof_events[2 * prof_slot + 1], s));
   count(CNT_LAUNCHES);
   count(CNT_TC_LAUNCHES);
