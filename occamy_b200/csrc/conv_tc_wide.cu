@@ -202,25 +202,26 @@ __global__ void __launch_bounds__(WD_THREADS, 1) tc_conv_wide_kernel(const __gri
     }
   } else if (warp == 11) {
     // ------------------------------------------------------------ slab store
-    {
+    // (as a whole warp, polling, it takes issue slots from the epilogue: 64 -> 128 at 112x112 103 us this way, 122 that way)
+    if (lane == 0) {
       uint32_t phase = 0;
       for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x, phase ^= 1u) {
         const TcTile tl = tc_decode<128>(p, tile);
         for (int sl = 0; sl < nslab; ++sl) {
-          if (!mbar_wait_warp(d_full(sl), phase, abort_flag)) {
+          if (!mbar_wait(d_full(sl), phase, abort_flag)) {
             err_code = 6;
             break;
           }
-          store_4d_warp(&p.tmD, sD + sl * slab_bytes, sl * 64, POOL ? tl.q0 >> 1 : tl.q0, POOL ? tl.p0 >> 1 : tl.p0, tl.n0);
+          tma_store_4d(&p.tmD, sD + sl * slab_bytes, sl * 64, POOL ? tl.q0 >> 1 : tl.q0, POOL ? tl.p0 >> 1 : tl.p0, tl.n0);
           tma_store_commit();
         }
         if (err_code) break;
         if (nslab == 2) {
           tma_store_wait_read<1>();
-          arrive_warp(d_empty(0));
+          mbar_arrive(d_empty(0));
         }
         tma_store_wait_read<0>();
-        arrive_warp(d_empty(nslab - 1));
+        mbar_arrive(d_empty(nslab - 1));
       }
       tma_store_wait_read<0>();
     }

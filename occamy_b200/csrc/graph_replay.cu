@@ -31,7 +31,7 @@ struct SavedRec {
 // graph, on tensors in memory of the runtime's.  What it is for is a batch that comes from the host: the
 // pieces are computed while the later ones are still on their way (batch 256 of a ResNet-50 takes 2.9 ms to
 // arrive and 3.1 to compute).
-constexpr int MAX_PIECES = 3;
+constexpr int MAX_PIECES = 4;
 
 // An executable graph.  One that goes out of use may still be running: it is destroyed later (empty_trash()).
 struct Exec {
@@ -470,10 +470,13 @@ void wait_for_upload() {
 //     fp32 ResNet  5.72 / 6.44                  10.44 / 10.67
 int piece_images(int64_t n, int64_t *images) {
   if (n < 128 || rt().mode == MATH_FP32) return 0;
-  images[0] = n / 4 / 8 * 8;
-  images[1] = (n - images[0]) / 2 / 8 * 8;
-  images[2] = n - images[0] - images[1];
-  return MAX_PIECES;
+  const int pieces = n < 192 ? 3 : 4;
+  images[0] = n / (pieces == 3 ? 8 : 16) * (pieces == 3 ? 2 : 3) / 8 * 8;
+  int64_t left = n - images[0];
+  if (pieces == 4) left -= images[1] = n / 4 / 8 * 8;
+  images[pieces - 2] = left / 2 / 8 * 8;
+  images[pieces - 1] = left - images[pieces - 2];   // (none is larger)
+  return pieces;
 }
 
 struct Cut {
@@ -677,7 +680,8 @@ void build_pieces(TraceProgram &p, const Variant &v) {
   if (plan.piece_failures >= MAX_FAILURES) return;
   for (const auto &o : plan.variants)
     if (o->pieces && o->pool_base == v.pool_base && o->flags == v.flags && o->epoch == gr.epoch) return;
-  if (!find_input(p, c) || c.x_bytes < (16 << 20) || !piece_images(c.batch, images) || !cut_up(p, images[2], c)) {
+  const int pieces = find_input(p, c) && c.x_bytes >= (16 << 20) ? piece_images(c.batch, images) : 0;
+  if (!pieces || !cut_up(p, images[pieces - 1], c)) {
     plan.piece_failures = MAX_FAILURES;
     return;
   }
@@ -720,7 +724,7 @@ void build_pieces(TraceProgram &p, const Variant &v) {
   bool ok = true;
   const uint64_t epoch = gr.epoch;
   int64_t at = 0;
-  for (int k = 0; k < MAX_PIECES && ok; at += images[k++]) {
+  for (int k = 0; k < pieces && ok; at += images[k++]) {
     Cut piece = c;
     piece.out = 0;
     ok = cut_up(p, images[k], piece);
@@ -738,7 +742,7 @@ void build_pieces(TraceProgram &p, const Variant &v) {
       chains0 = trace_fused_chains();
       make_piece(p, piece, at, images[k], hosts);
       if (spoiled) continue;
-      if (k + 1 == MAX_PIECES) {
+      if (k + 1 == pieces) {
         enqueue_copy(n->result.aside, n->result.tensor, n->result.bytes, r.stream);
         enqueue_copy(n->result.tensor, n->result.made, n->result.bytes, r.stream);
       }
@@ -779,7 +783,7 @@ void launch_segment() {
   const Segment &s = v.segments[gr.seg];
   gr.left.resize(1);   // the others may differ from here on
   if (v.pieces) {
-    for (int i = 0; i < MAX_PIECES; ++i) {
+    for (int i = 0; i < MAX_PIECES && s.pieces[i].e; ++i) {
       if (i < gr.pieces_coming) OCC_CUDA(cudaStreamWaitEvent(r.stream, gr.piece_here[i], 0));
       OCC_CUDA(cudaGraphLaunch(s.pieces[i].e, r.stream));
     }
@@ -890,19 +894,19 @@ bool graph_upload_in_pieces(void *dst, const void *src, size_t bytes, cudaStream
     there = there || (v->pieces && v->pool_base == base && v->flags == mode_flags() && v->epoch == gr.epoch);
   Cut c;
   int64_t images[MAX_PIECES];
-  if (!there || !find_input(*p, c) || (size_t)c.x_bytes != bytes || c.x - p->pool_base + base != (uintptr_t)dst ||
-      !piece_images(c.batch, images))
-    return false;
+  if (!there || !find_input(*p, c) || (size_t)c.x_bytes != bytes || c.x - p->pool_base + base != (uintptr_t)dst) return false;
+  const int pieces = piece_images(c.batch, images);
+  if (!pieces) return false;
   for (cudaEvent_t &e : gr.piece_here)
     if (!e) OCC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   size_t at = 0;
-  for (int k = 0; k < MAX_PIECES; ++k) {
+  for (int k = 0; k < pieces; ++k) {
     const size_t n = bytes / (size_t)c.batch * (size_t)images[k];
     OCC_CUDA(cudaMemcpyAsync((char *)dst + at, (const char *)src + at, n, cudaMemcpyHostToDevice, copy_stream));
     OCC_CUDA(cudaEventRecord(gr.piece_here[k], copy_stream));
     at += n;
   }
-  gr.pieces_coming = MAX_PIECES;
+  gr.pieces_coming = pieces;
   return true;
 }
 
