@@ -903,7 +903,14 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   const bool pn = few && !wide && !a.pool2;
   pl.pn = pn;
   pl.wide = wide;
+  // Few-channel stems with up to three filter rows whose kernel runs twice on an SM (below) read their windows in place
+  // (TC_MODE_ROWS); every row of the output has a filter row inside the image.
+  bool rows = allow_halo && a.w_step == 8 && a.S == 1 && a.R <= 3 && a.pad_h < a.R && a.Cf <= 32 && a.K <= 64 && !a.out_f32 && !a.residual &&
+              !a.pool2 && !pn && num_sms >= 2;
   if (wide) {   // (the box is chosen)
+  } else if (rows) {
+    p.tw = (Qg + (Qg + 127) / 128 - 1) / ((Qg + 127) / 128);
+    p.th = p.tn = 1;
   } else if (halo && a.pool2) {
     p.tw = 14;   // 16 lanes to an input row
     p.th = 8;
@@ -939,7 +946,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   p.tiles_w = (Qg + p.tw - 1) / p.tw;
   p.tiles_h = (Pg + p.th - 1) / p.th;
   p.tiles_n = (Ng + p.tn - 1) / p.tn;
-  const int bn = pn || wide ? 128
+  const int bn = rows ? (a.K <= 32 ? 32 : 64) : pn || wide ? 128
                     : halo ? 64
                     : pick_bn(a.K, (long)p.tiles_w * p.tiles_h * p.tiles_n,
                               reduction64(a), nsm);
@@ -1049,7 +1056,17 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
 #endif
   p.b_resident = bres ? 1 : 0;
   // shared memory: ring + output slabs + bias + barriers + alignment
-  const size_t stage_bytes = pn     ? (size_t)(128 + 256) * bk * 2
+  if (rows) {
+    p.rows_x = (const uint8_t *)a.x;
+    p.row_bytes = a.row_elems * 2;
+    p.window = a.Cf * 2;
+    p.row_slot = (16 * 127 + p.window + 127) / 128 * 128;
+    p.halo_a_bytes = (a.R * p.row_slot + 1023) / 1024 * 1024;
+    p.in_h = a.H; p.stride_h = a.stride_h; p.pad_h = a.pad_h;
+    pl.mode |= TC_MODE_ROWS;
+  }
+  const size_t stage_bytes = rows   ? (size_t)p.halo_a_bytes
+                             : pn   ? (size_t)(128 + 256) * bk * 2
                              : halo ? (size_t)p.halo_a_bytes
                                     : 128 * bk * 2 + (bres ? 0 : b_tile_bytes);
   p.bias_floats = (a.K + bn - 1) / bn * bn;
@@ -1130,7 +1147,8 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
             a.K, a.Cf, a.R * a.S, Qg, Pg, Ng, p.tw, p.th, p.tn, bn, dc, (int)pn, bk, stages, dbuf, pend, (int)duo,
             p.total_tiles, pl.smem);
 #endif
-  if (halo && !ok) return build_plan(a, err_word, num_sms, counted, false);   // e.g. the block map was refused
+  if (rows && !(duo && bres)) ok = false;
+  if ((halo || rows) && !ok) return build_plan(a, err_word, num_sms, counted, false);   // e.g. the block map was refused
   pl.ok = ok;
   return pl;
 }

@@ -70,6 +70,9 @@ struct alignas(64) TcParams {
   int bias_floats;       // K rounded up to whole channel tiles: bias entries kept in shared memory
   int dbuf;              // output slab buffers in shared memory (an even number, 4..12)
   int store_pend;        // stores a store thread may leave in flight behind its newest (0..3)
+  // TC_MODE_ROWS: the padded input rows, their length, their place in a stage, bytes of a window; the filter's geometry
+  const uint8_t *rows_x;
+  int row_bytes, row_slot, window, in_h, stride_h, pad_h;
   int b_resident;        // one channel tile: the weight tiles of all k-steps are fetched once per CTA
 #ifdef OCCAMY_TC_TIMERS
   long long *timers;     // 5 roles x 4 counters, or null
@@ -132,6 +135,13 @@ constexpr int TC_MODE_PAIR = 32;
 // 16-bit results meet by shuffles and a quarter of the slab is stored.  (A pass of its own over the
 // 224x224 layer of a VGG-16 took 85 us at batch 64, and its input 60 to write.)
 constexpr int TC_MODE_POOL = 64;
+// Few input channels, the folded form with 16 bytes from one column to the next: a tile is (a part of) one output row,
+// its input rows are copied as they lie, once, and the tensor core reads the overlapping windows in place (un-swizzled,
+// "row m starts at byte 16 * m").  Through tensor maps whose windows overlap TMA takes 3.3 cycles for each of the 128
+// windows of a tap, twice what it takes for rows that do not, and that was these layers' time: 3 -> 64 at 224x224, 64
+// images, 144 -> 84 us (63 of HBM time); 3 -> 32 with stride 2 there, 128 images, 47 -> 31 (24).  VGG-16 with 64 images
+// 1821 -> 1762 us, 5 278 -> 272; MobileNetV2 with 128 799 -> 773.
+constexpr int TC_MODE_ROWS = 128;
 
 // ------------------------------------------------------------------ PTX wrappers
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -448,6 +458,13 @@ __device__ __forceinline__ void load_3d_pair_warp(uint32_t dst, const CUtensorMa
       "l"(m), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
+__device__ __forceinline__ void bulk_load_warp(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+  asm volatile(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n}" ::"r"(dst),
+      "l"(src), "r"(bytes), "r"(bar)
+      : "memory");
+}
 __device__ __forceinline__ void arrive_warp(uint32_t a) {
   asm volatile(
       "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
@@ -530,6 +547,13 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, int bk) {
   const uint64_t layout = bk == 64 ? 2ull : (bk == 32 ? 4ull : 6ull);
   return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(sbo >> 4) << 32) |
          (1ull << 46) | (layout << 61);
+}
+
+// Un-swizzled K-major operand: `lbo` bytes between 8-element K chunks, `sbo` bytes between
+// groups of 8 rows.
+__device__ __forceinline__ uint64_t desc_plain(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) |
+         ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
 }
 
 // The fused activations (identity, ReLU, clipped ReLU) are all a clamp to [lo, hi]; keeping
@@ -618,6 +642,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
   constexpr bool F16 = (MODE & TC_MODE_F16) != 0;
   constexpr bool PAIR = (MODE & TC_MODE_PAIR) != 0;
   constexpr bool POOL = (MODE & TC_MODE_POOL) != 0;
+  constexpr bool ROWS = (MODE & TC_MODE_ROWS) != 0;
   static_assert(!POOL || (!(MODE & (TC_MODE_RES | TC_MODE_F32)) && (HALO || PAIR)), "pooled forms");
   static_assert(!(PAIR && (HALO || F32)), "the CTA-pair form exists for the plain epilogues only");
   constexpr int EPI_THREADS = 128 * EW;
@@ -644,7 +669,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
   uint8_t *base_ptr = smem_raw;
   const int bk = p.bk, stages = p.stages, dbuf = p.dbuf;
   // halo form: the ring carries input blocks only, the weights of all taps sit behind it
-  const uint32_t a_bytes = HALO ? (uint32_t)p.halo_a_bytes : 128u * bk * 2u;
+  const uint32_t a_bytes = HALO || ROWS ? (uint32_t)p.halo_a_bytes : 128u * bk * 2u;
   const uint32_t b_bytes = (uint32_t)BROWS * bk * 2u;
   const uint32_t sA = base;
   const uint32_t sB = sA + stages * a_bytes;
@@ -683,7 +708,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
 
   if (threadIdx.x == 0) {
     // descriptor fetches are off the critical path of the first loads / stores
-    tma_prefetch_map(&p.tmA[0]);
+    if (!ROWS) tma_prefetch_map(&p.tmA[0]);
     tma_prefetch_map(&p.tmB);
     if (!F32) tma_prefetch_map(&p.tmD);
     for (int s = 0; s < stages; ++s) {
@@ -798,6 +823,28 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
             phase ^= 1u;
           }
         }
+      } else if constexpr (ROWS) {
+        if (!p.consts_ready) load_resident_b();
+        TCT_DECL
+        for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x) {
+          const TcTile tl = tc_decode<BN>(p, tile);
+          const uint32_t bytes = 16u * (uint32_t)(min(p.tw, p.gq - tl.q0) - 1) + (uint32_t)p.window;
+          const int j0 = tl.p0 * p.stride_h - p.pad_h;
+          const int r0 = max(0, -j0), r1 = min(p.num_taps, p.in_h - j0);   // (rows outside the image: no products)
+          if (!TCT_WAIT(0, mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag))) {
+            err_code = 1;
+            break;
+          }
+          expect_tx_warp(full_bar(stage), (uint32_t)(r1 - r0) * bytes);
+          const uint8_t *src = p.rows_x + ((size_t)tl.n0 * p.in_h + j0) * p.row_bytes + 16 * tl.q0;
+          for (int r = r0; r < r1; ++r)
+            bulk_load_warp(sA + stage * a_bytes + r * p.row_slot, src + (int64_t)r * p.row_bytes, bytes, full_bar(stage));
+          if (++stage == stages) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+        TCT_FLUSH(0)
       } else {
       const uint32_t tx_bytes = (uint32_t)rows_valid * bk * 2u + (bres ? 0u : b_bytes);
       if (bres && !p.consts_ready) load_resident_b();
@@ -901,6 +948,43 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
           commit_warp(empty_bar(my_stage));
           commit_warp(tfull_bar(my_acc));
         }
+      } else if constexpr (ROWS) {
+        TCT_DECL
+        if (!mbar_wait_warp(wfull_bar, 0, abort_flag)) err_code = 3;
+        const uint64_t a0 = desc_plain(sA, 16, 128), b0 = make_smem_desc(sB, bk);
+        const uint32_t a_hi = (uint32_t)(a0 >> 32), b_hi = (uint32_t)(b0 >> 32);
+        const uint32_t row_desc = (uint32_t)p.row_slot >> 4, b_step = b_bytes >> 4;
+        for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x) {
+          const TcTile tl = tc_decode<BN>(p, tile);
+          const int j0 = tl.p0 * p.stride_h - p.pad_h;
+          const int r0 = max(0, -j0), r1 = min(p.num_taps, p.in_h - j0);
+          if (!TCT_WAIT(0, mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag))) {
+            err_code = 2;
+            break;
+          }
+          if (!TCT_WAIT(1, mbar_wait_warp(full_bar(stage), phase, abort_flag))) {
+            err_code = 3;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
+          const uint32_t a_lo = (uint32_t)a0 + (uint32_t)stage * (a_bytes >> 4);
+#pragma unroll 1
+          for (int r = r0; r < r1; ++r) {
+            const uint32_t ar = a_lo + (uint32_t)r * row_desc, br = (uint32_t)b0 + (uint32_t)r * b_step;
+            mma_warp(d_tmem, ar, a_hi, br, b_hi, IDESC, r > r0 ? 1u : 0u);
+            if (bk == 32) mma_warp(d_tmem, ar + 2u, a_hi, br + 2u, b_hi, IDESC, 1u);
+          }
+          commit_warp(empty_bar(stage));
+          commit_warp(tfull_bar(acc));
+          if (++stage == stages) {
+            stage = 0;
+            phase ^= 1u;
+          }
+          acc ^= 1;
+          if (acc == 0) acc_phase ^= 1u;
+        }
+        TCT_FLUSH(1)
       } else {
       TCT_DECL
       if (bres && !mbar_wait_warp(wfull_bar, 0, abort_flag)) err_code = 3;
@@ -1401,7 +1485,7 @@ inline void tc_launch_one(const TcParams &p, int grid, size_t smem, cudaStream_t
 // 256 threads, two of which fit an SM.
 template <int BN, int DC>
 inline bool tc_launch_mode_duo(const TcParams &p, int mode, int grid, size_t smem, cudaStream_t s) {
-  constexpr int H = TC_MODE_F16, R = TC_MODE_RES, C = TC_MODE_CLAMP;
+  constexpr int H = TC_MODE_F16, R = TC_MODE_RES, C = TC_MODE_CLAMP, W = TC_MODE_ROWS;
   switch (mode) {
     case 0: tc_launch_one<BN, DC, 0, 1>(p, grid, smem, s); return true;
     case R: tc_launch_one<BN, DC, R, 1>(p, grid, smem, s); return true;
@@ -1411,6 +1495,10 @@ inline bool tc_launch_mode_duo(const TcParams &p, int mode, int grid, size_t sme
     case H | R: tc_launch_one<BN, DC, H | R, 1>(p, grid, smem, s); return true;
     case H | C: tc_launch_one<BN, DC, H | C, 1>(p, grid, smem, s); return true;
     case H | R | C: tc_launch_one<BN, DC, H | R | C, 1>(p, grid, smem, s); return true;
+    case W: tc_launch_one<BN, DC, W, 1>(p, grid, smem, s); return true;
+    case W | C: tc_launch_one<BN, DC, W | C, 1>(p, grid, smem, s); return true;
+    case W | H: tc_launch_one<BN, DC, W | H, 1>(p, grid, smem, s); return true;
+    case W | H | C: tc_launch_one<BN, DC, W | H | C, 1>(p, grid, smem, s); return true;
     default: return false;
   }
 }

@@ -77,13 +77,6 @@ __device__ __forceinline__ void ir_sts128(uint32_t addr, const uint32_t *r) {
 __device__ __forceinline__ void ir_sts64(uint32_t addr, uint32_t a, uint32_t b) {
   asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
 }
-__device__ __forceinline__ void ir_bulk_load_warp(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-  asm volatile(
-      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
-      "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n}" ::"r"(dst),
-      "l"(src), "r"(bytes), "r"(bar)
-      : "memory");
-}
 __device__ __forceinline__ uint2 ir_lds64(uint32_t addr) {
   uint2 v;
   asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
@@ -275,7 +268,7 @@ __global__ void __launch_bounds__(IR_THREADS, 2) ir_kernel(const __grid_constant
       expect_tx_warp(bar, w2_bytes + (uint32_t)(rows * n));
       load_3d_warp(sW2 + st * w2_stage, &p.tmW2, bar, e0, 0, 0);
       for (int t = 0; t < rows; ++t)
-        ir_bulk_load_warp(sWD + st * WD_STAGE + (uint32_t)t * WD_ROW,
+        bulk_load_warp(sWD + st * WD_STAGE + (uint32_t)t * WD_ROW,
                      reinterpret_cast<const uint8_t *>(t < 9 ? p.w2 : p.b2) + ((int64_t)(t % 9) * p.E + e0) * (F16 ? 2 : 4),
                      (uint32_t)n, bar);
     };

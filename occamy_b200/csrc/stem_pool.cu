@@ -64,22 +64,7 @@ struct alignas(64) StemParams {
   int *err;
 };
 
-__device__ __forceinline__ void bulk_g2s_warp(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-  asm volatile(
-      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
-      "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n}" ::"r"(dst),
-      "l"(src), "r"(bytes), "r"(bar)
-      : "memory");
-}
-
-// Un-swizzled K-major operand: `lbo` bytes between 8-element K chunks, `sbo` bytes between
-// groups of 8 rows.
-__device__ __forceinline__ uint64_t desc_plain(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) |
-         ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
-}
-
-// The same, issued only when `valid` is non-zero (a predicated instruction, not a branch:
+// An MMA that is issued only when `valid` is non-zero (a predicated instruction, not a branch:
 // a taken branch costs the single issuing thread more than the MMA it would skip).
 __device__ __forceinline__ void mma_lohi_if(uint32_t valid, uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi,
                                             uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
@@ -222,7 +207,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stem_pool_kernel(const __grid_c
       if constexpr (TILED) {
         for (int r = 0; r < p.R; ++r) load_3d_warp(sW + r * w_tap, &p.tmW, w_full, 0, 0, r);
       } else {
-        bulk_g2s_warp(sW, p.w, w_bytes, w_full);
+        bulk_load_warp(sW, p.w, w_bytes, w_full);
       }
       uint32_t q = 0;   // chunks loaded so far
       for (int unit = blockIdx.x; unit < p.units && !err_code; unit += gridDim.x) {
@@ -246,7 +231,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stem_pool_kernel(const __grid_c
           const uint32_t bytes = hi > lo ? (uint32_t)((hi - lo) * p.row_bytes) : 0u;
           expect_tx_warp(in_full(s), bytes);   // 0 bytes: a plain arrival
           if (bytes)
-            bulk_g2s_warp(sIn + s * p.chunk * p.slot_bytes + (lo - j0) * p.row_bytes, img + (size_t)lo * p.row_bytes, bytes,
+            bulk_load_warp(sIn + s * p.chunk * p.slot_bytes + (lo - j0) * p.row_bytes, img + (size_t)lo * p.row_bytes, bytes,
                      in_full(s));
         }
       }
