@@ -607,13 +607,13 @@ bool join_summands(const ConvJob &a, ConvJob &b) {
   // the second summand is a 1x1 convolution, the strided one of two
   const bool swap = plain(a.a) && (!plain(b.a) || (strided(a.a) && !strided(b.a)));
   const TcConvArgs &first = swap ? b.a : a.a, &second = swap ? a.a : b.a;
-  if (!plain(second) || (b.a.split && b.g.K % 16)) return false;
+  if (!plain(second)) return false;
   TcConvArgs c = first;
   c.x2 = second.x; c.w2 = second.w; c.bias2 = second.bias;
   c.H2 = second.H; c.W2 = second.W; c.Cf2 = second.Cf;
   c.stride2_h = second.stride_h; c.stride2_w = second.stride_w;
   c.consts_ready = a.a.consts_ready && b.a.consts_ready;
-  c.y = b.a.y; c.out_f32 = b.a.out_f32;
+  c.y = b.a.y;
   if (!tc_conv_supported(c)) return false;
   b.a = c;
   b.dep_lo[3] = a.dep_lo[0]; b.dep_hi[3] = a.dep_hi[0];
@@ -903,7 +903,7 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
     if (!follow) flush_pending();
   } else if (g_pending.active && g_pending.summand) {   // left by step(): this call was recorded as the other summand
     const ConvGeom &f = g_pending.g;
-    sum = role == R_DEFER && e.fusable && !depthwise && e.parts == (g_pending.a.split != 0) && f.N == g.N && f.K == g.K &&
+    sum = role == R_DEFER && e.fusable && !depthwise && !e.parts && f.N == g.N && f.K == g.K &&
           f.P == g.P && f.Q == g.Q && !g_pending.act_set && !g_pending.res_set;
     if (!sum) flush_pending();
   } else if (g_pending.active) {   // left by step() because this call was recorded as joining it
@@ -984,7 +984,6 @@ float *conv_common(int sym, float *x, const int64_t *dX, float *w, const int64_t
     job.out = y;
     if (prepare_parts(x, w, bias, g, job)) {
       job.out_parts = (flags & RF_FOR_PARTS) && g.K % 16 == 0;
-      hold_summand(job, is_parts(x, g.N, g.C, g.H, g.W));
       if (role == R_DEFER) {
         g_pending = job;
         g_pending.active = true;

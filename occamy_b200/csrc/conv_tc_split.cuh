@@ -7,7 +7,7 @@ namespace occ {
 constexpr int SK_THREADS = 256;
 constexpr int SK_MAX_SPLITS = 8;       // portable cluster size
 constexpr int SK_MAX_STAGES = 16;
-constexpr int SK_MAX_AMAPS = 15;       // A tensor maps: 4 stride phases and the second summand, 3 operand parts each
+constexpr int SK_MAX_AMAPS = 12;       // A tensor maps: 4 stride phases of 3 operand parts, or of one and the second summand's
 
 struct SkTap {
   int8_t map, dw, dh, pad;

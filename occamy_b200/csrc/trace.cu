@@ -311,7 +311,7 @@ void analyse(const std::vector<Entry> &rec, std::vector<uint16_t> &roles, std::v
     if (a-- == 0) continue;
     const Entry &c = rec[a];
     const uintptr_t sum = chain_out[a];
-    if (c.depthwise || b.depthwise || c.parts != b.parts || chain_res[a] || chain_act[a] || !same_dims(c, b) ||
+    if (c.depthwise || b.depthwise || c.parts || b.parts || chain_res[a] || chain_act[a] || !same_dims(c, b) ||
         ((roles[a] | roles[i]) & (RF_LINK | RF_JOIN)) || !sum || (add.in[0] != sum && add.in[1] != sum) ||
         !passive_past(chain_last[a] + 1, i, sum, c.out_bytes))
       continue;

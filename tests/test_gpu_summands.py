@@ -1,6 +1,5 @@
 """Sums of two convolutions in one kernel (a block's last convolution and its projection shortcut): odd sizes, strides on
-either side, 3x3 against 1x1, channel counts with remainders, in the three modes, against the CPU oracle; and sums that
-are not taken."""
+either side, 3x3 against 1x1, channel counts with remainders, against the CPU oracle; and sums that are not taken."""
 import numpy as np
 import pytest
 
@@ -51,7 +50,7 @@ def _run(binding, g, mode, fuse, taken):
     assert rt.last_error() == 0
 
 
-@pytest.mark.parametrize("mode", [rt.MATH_BF16, rt.MATH_F16, rt.MATH_FP32])
+@pytest.mark.parametrize("mode", [rt.MATH_BF16, rt.MATH_F16])
 @pytest.mark.parametrize("fuse", [replay.FUSE_REFERENCE, replay.FUSE_NONE])
 @pytest.mark.parametrize("N,C,H,W,M,K,R,s_main,s_short", [
     (2, 64, 56, 56, 64, 256, 1, 1, 1),      # one row of pixels for both
@@ -64,19 +63,16 @@ def _run(binding, g, mode, fuse, taken):
     (5, 128, 17, 19, 64, 72, 3, 2, 2),      # both strided, channel tile with a remainder
 ])
 def test_summands(binding, N, C, H, W, M, K, R, s_main, s_short, fuse, mode):
-    if mode == rt.MATH_FP32:
-        if N > 40:
-            pytest.skip("the fp32 oracle of this size takes minutes")
-        N += 1   # (calls recorded in one mode are not looked at anew in another)
-    _run(binding, _block(N, C, H, W, M, K, R, s_main, s_short), mode, fuse, mode != rt.MATH_FP32 or K % 16 == 0)
+    _run(binding, _block(N, C, H, W, M, K, R, s_main, s_short), mode, fuse, True)
 
 
-@pytest.mark.parametrize("mode", [rt.MATH_BF16, rt.MATH_FP32])
+@pytest.mark.parametrize("mode", [rt.MATH_BF16, rt.MATH_FP32])   # (fp32: apart, for the longer sum would cost digits)
 @pytest.mark.parametrize("N,kw,taken", [(4, dict(shortcut_first=True), True), (6, dict(act=False), True),
                                         (8, dict(relu_before=True), False), (10, dict(twice=True), False)])
 def test_summand_forms(binding, N, kw, taken, mode):
     # (batches of their own: what a recorded sequence skips stays skipped for another one that begins like it)
-    _run(binding, _block(N + (mode == rt.MATH_FP32), 64, 21, 23, 64, 128, 1, 1, 1, **kw), mode, replay.FUSE_REFERENCE, taken)
+    _run(binding, _block(N + (mode == rt.MATH_FP32), 64, 21, 23, 64, 128, 1, 1, 1, **kw), mode, replay.FUSE_REFERENCE,
+         taken and mode != rt.MATH_FP32)
 
 
 def test_summands_of_unlike_steps_run_apart(binding):
