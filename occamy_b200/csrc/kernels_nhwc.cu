@@ -423,11 +423,22 @@ __global__ void __launch_bounds__(8 * GAP_ROWS) gap_bf16_kernel(const bf16x8 *__
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (c8 < C8) {
     const bf16x8 *xp = x + n * HW * C8 + c8;
-    for (int p = prow; p < HW; p += GAP_ROWS) {
-      float f[8];
-      unpack8<F16>(xp[(int64_t)p * C8], f);
+    // Four pixels are requested at a time: one by one, a thread waited for each (2048 channels at 7x7, 256 images, 20.3 ->
+    // 12.3 us, 8 of HBM time; 1280, 128 images, 10.8 -> 6.3).
+    constexpr int AHEAD = 4;
+    for (int p = prow; p < HW; p += AHEAD * GAP_ROWS) {
+      bf16x8 v[AHEAD];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) acc[k] += f[k];
+      for (int u = 0; u < AHEAD; ++u)
+        if (p + u * GAP_ROWS < HW) v[u] = xp[(int64_t)(p + u * GAP_ROWS) * C8];
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u) {
+        if (p + u * GAP_ROWS >= HW) break;
+        float f[8];
+        unpack8<F16>(v[u], f);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[k] += f[k];
+      }
     }
   }
 #pragma unroll
