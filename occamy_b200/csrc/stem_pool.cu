@@ -327,6 +327,11 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stem_pool_kernel(const __grid_c
         gbase += (uint32_t)groups;
         cbase += (uint32_t)rows;
       }
+      // The last commits are waited for, so that none arrives when this CTA has gone.
+      if (!err_code && gbase) {
+        const uint32_t q = gbase / (uint32_t)p.chunk - 1;
+        if (!mbar_wait_warp(in_empty(q % chunks), (q / chunks) & 1u, abort_flag)) err_code = 8;
+      }
     }
   } else if (warp < 2 + ST_EPI_WARPS) {
     // ------------------------------------------------------------ epilogue
