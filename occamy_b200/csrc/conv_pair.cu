@@ -17,14 +17,15 @@
 //   epilogue 2  behind the next tile's first chunk, so that nobody waits for the last products
 // The tensor core works on one chunk's product 1 and another one's product 2 while the epilogue works on a third.
 //
-//   warp 0      x (one lane)
-//   warps 1, 14 MMA issuers (one lane each) of product 1 and product 2: an issuer's polls of barriers, some 200 cycles
+//   (all but the epilogue: whole warps that elect a lane for each instruction)
+//   warp 0      x
+//   warps 1, 14 MMA issuers of product 1 and product 2: an issuer's polls of barriers, some 200 cycles
 //               each, are its time, and the two products share none
 //   warps 2-9   epilogue, two per TMEM lane quadrant
-//   warps 10, 15 weights of product 1 and product 2 (one lane each), a ring of tiles each
-//   warps 11-12 slabs of y (one lane each, alternate slabs): handed out empty or with the shortcut's values, stored;
+//   warps 10, 15 weights of product 1 and product 2, a ring of tiles each
+//   warps 11-12 slabs of y (alternate slabs): handed out empty or with the shortcut's values, stored;
 //               a slab is free again when the store has read it and product 2 is done
-//   warp 13     slabs of t (one lane)
+//   warp 13     slabs of t
 // Every wait is bounded; one that runs out records a code and the kernel drains.
 #include "conv_pair.h"
 

@@ -617,13 +617,14 @@ __device__ __forceinline__ TcTile tc_decode(const TcParams &p, int tile, uint32_
 //        instruction-cache misses stall all of them
 //
 // One persistent CTA per SM:
-//   warp 0            TMA producer (one lane): fills a ring of {A, B} stages
-//   warp 1            MMA issuer (one lane): tcgen05.mma 128 x BN x 16, fp32 accumulators in
+//   (producer, issuer and store warps run as a whole and elect a lane for each instruction)
+//   warp 0            TMA producer: fills a ring of {A, B} stages
+//   warp 1            MMA issuer: tcgen05.mma 128 x BN x 16, fp32 accumulators in
 //                     TMEM, two accumulator buffers
 //   warps 2..2+4*EW   epilogue: tcgen05.ld the finished accumulator, add bias / residual,
 //                     activation, convert to bf16, write 128-pixel slabs of DC channels into
 //                     swizzled shared memory
-//   TC_NSTORE warps   slab store (one lane each): hand slab buffers to the epilogue (empty,
+//   TC_NSTORE warps   slab store: hand slab buffers to the epilogue (empty,
 //                     or pre-loaded with the residual slab) and TMA-store written slabs
 //   last warp         second MMA issuer of the halo form (idle otherwise)
 // Every wait on an mbarrier is bounded; when a bound is hit the kernel records a code in the
@@ -1053,11 +1054,11 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
     }
   } else if (warp >= STORE_WARP && warp < STORE_WARP + TC_NSTORE) {
     // ------------------------------------------------------------ slab store
-    // TC_NSTORE threads (one per warp) own the output slab buffers, slab d belonging to
-    // thread d % TC_NSTORE: the owner hands the buffer to the epilogue warps ("ready": free,
+    // TC_NSTORE warps own the output slab buffers, slab d belonging to
+    // warp d % TC_NSTORE: the owner hands the buffer to the epilogue warps ("ready": free,
     // or holding the residual slab the epilogue adds in place) and sends the written slab to
-    // global memory.  The epilogue warps never wait for one another.  More than one thread,
-    // because a single thread's issue rate (TMA store + residual load + bookkeeping per slab)
+    // global memory.  The epilogue warps never wait for one another.  More than one warp,
+    // because a single one's issue rate (TMA store + residual load + bookkeeping per slab)
     // limits the layers whose tiles are short.
     if constexpr (!F32) {
       {

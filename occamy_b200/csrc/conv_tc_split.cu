@@ -15,8 +15,8 @@
 //     TMA store the tile's end took 0.5 to 0.9 us longer: 256->64 at 56x56, batch 1, 3.3 -> 4.2 us.)
 // Measured times are at the dispatch rule (conv_tc.cu, sk_choose).
 //
-// Up to four warps issue the MMAs (one lane each, k-steps in turn, an accumulator of their own each)
-// and as many load (one lane each, k-steps in turn), then all eight warps drain the accumulators (two
+// Up to four warps issue the MMAs (whole warps, k-steps in turn, an accumulator of their own each)
+// and as many load (k-steps in turn), then all eight warps drain the accumulators (two
 // per TMEM lane quadrant, half of the columns each).  Several threads per role, because one thread's
 // round of barrier poll, issue and commit takes 450 to 600 cycles whatever it moves, and the four MMAs
 // of a k-step 200 to 260.  A ring that is reused has a multiple of that many stages: a stage then always

@@ -8,17 +8,17 @@
 // plus one on either side, 64 channels) comes in once and the nine taps are windows of it, shifted by whole pixels: a
 // swizzled operand may start at any multiple of 128 bytes.  The N index runs through the block's rows, so two of its
 // columns are junk (an eighth of 14-column strips), which the epilogue leaves out.
-// Before (tc_conv_pn_kernel, pool by itself) and now: 128 -> 128 at 28x28, 256 images, 59.6 -> 51.0 us, 32 images
-// 17.7 -> 13.3; 64 -> 128 at 112x112, 64 images, 159 -> 108; 128 -> 128 there with its pool 193 + 36 -> 160.  The last is
-// 1480 TFLOP/s of MMAs made, 0.9 of the burst rate, an eighth of them on junk columns.
+// Before (tc_conv_pn_kernel, pool by itself) and now: 128 -> 128 at 28x28, 256 images, 59.6 -> 46.0 us, 32 images
+// 17.7 -> 13.3; 64 -> 128 at 112x112, 64 images, 159 -> 102; 128 -> 128 there with its pool 193 + 36 -> 151.  The last is
+// 1570 TFLOP/s of MMAs made, 0.95 of the burst rate, an eighth of them on junk columns.
 //
 // One persistent CTA per SM, roles by warp:
-//   warp 0      input blocks (one lane), two buffers of 64 channels each
-//   warp 1      MMA issuer (one lane): three taps, 12 MMAs, per barrier -- a poll and what goes with it cost the issuing
-//               thread as much as two MMAs; two accumulators of up to 256 pixels
+//   (warps 0, 1 and 10: whole warps that elect a lane for each instruction)
+//   warp 0      input blocks, two buffers of 64 channels each
+//   warp 1      MMA issuer: three taps, 12 MMAs, per barrier -- a poll and what goes with it cost as much as two MMAs; two accumulators of up to 256 pixels
 //   warps 2-9   epilogue: a thread owns a channel; bias and clamp, 16-bit values into the staged slabs (64 channels of
 //               all the tile's pixels), two bytes at a time, the 32 lanes of a warp next to one another
-//   warp 10     weights (one lane): six tiles of one tap and 64 channels, handed back one by one
+//   warp 10     weights: six tiles of one tap and 64 channels, handed back one by one
 //   warp 11     slab store (one lane)
 // POOL: a 2x2 / stride 2 max pool behind the layer.  A thread has all the pixels of its channel.
 // Every wait is bounded; one that runs out records a code and the kernel drains.
