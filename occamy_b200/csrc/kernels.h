@@ -194,6 +194,14 @@ struct StemPoolArgs {
   float lo, hi;       // clamp applied before the pool
 };
 bool stem_pool_supported(const StemPoolArgs &a);
+// Its shared memory, in bytes behind the first multiple of 1024; false when there is not enough.
+struct StemPoolLayout {
+  int tiled, ring, chunk, bk;        // StemParams
+  int in_at;                         // where the ring of input rows begins, behind the weights
+  int in_row, slot_bytes, mr_bytes;  // an input row, a group of them, a row of column maxima
+  int smem;                          // of the launch, with 1024 for the alignment
+};
+bool stem_pool_layout(int R, int Cf, int stride_h, int Q, int row_bytes, bool may_tile, StemPoolLayout *l);
 size_t stem_pool_weight_bytes(int R, int Cf);
 // fp32 KCRS (C <= Cp) -> the weight layout of the fused kernel
 void launch_pack_stem_bf16(const float *w, bf16 *out, int C, int R, int S, int Cp, int Cf,

@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stem_pool_kernel(const __grid_c
   const uint32_t w_tap = (uint32_t)(TILED ? p.bk : p.Cf) * ST_K * 2, w_bytes = (uint32_t)p.R * w_tap;
   const uint32_t sW = base;
   const uint32_t sIn = sW + ((w_bytes + 1023u) & ~1023u);
-  // (the MMA rows beyond Q reach into what lies behind a row, 16 * 128 + 2 * Cf bytes at most: read, and left out)
+  // (the MMA rows beyond Q reach into what lies behind a row: read, and left out; stem_pool_layout() has room for it)
   const uint32_t sMr = sIn + ((p.ring * p.slot_bytes + 1023u) & ~1023u);
   const uint32_t sMisc = sMr + ST_NMR * p.mr_bytes;
   uint8_t *misc_ptr = base_ptr + (sMisc - base);
@@ -528,6 +528,29 @@ void launch_pack_stem_bf16(const float *w, bf16 *out, int C, int R, int S, int C
   count(CNT_LAUNCHES);
 }
 
+// As many groups of input rows as fit, sixteen or eight; tiled where that suffices.
+bool stem_pool_layout(int R, int Cf, int stride_h, int Q, int row_bytes, bool may_tile, StemPoolLayout *l) {
+  auto fits = [&](bool tiled, int ring, int chunk) {
+    l->tiled = tiled;
+    l->ring = ring;
+    l->chunk = chunk;
+    l->bk = Cf <= 16 ? 16 : Cf <= 32 ? 32 : 64;
+    l->in_row = tiled ? (Q + 7) / 8 * 8 * l->bk * 2 : row_bytes;
+    l->slot_bytes = l->in_row * stride_h;
+    l->mr_bytes = (Q * 128 + 1023) / 1024 * 1024;
+    l->in_at = (R * (tiled ? l->bk : Cf) * ST_K * 2 + 1023) / 1024 * 1024;
+    const int ring_bytes = ring * l->slot_bytes;
+    const int used = l->in_at + (ring_bytes + 1023) / 1024 * 1024 + ST_NMR * l->mr_bytes + 256 + 8 * 64;
+    // An MMA reads 128 windows from the start of a row, of the ring's last one too, however few the row has.
+    const int reach = l->in_at + ring_bytes - l->in_row + (tiled ? 128 * l->bk * 2 : 127 * 16 + Cf * 2);
+    l->smem = 1024 + (used > reach ? used : reach);   // (the first 1024 to align the rest)
+    // at least half of the shared memory, so that one CTA (one TMEM allocation) runs per SM
+    if (l->smem < 120 * 1024) l->smem = 120 * 1024;
+    return l->smem <= TC_SMEM_LIMIT;
+  };
+  return (may_tile && (fits(true, 16, 4) || fits(true, 8, 2))) || fits(false, 16, 4) || fits(false, 8, 1);
+}
+
 bool launch_stem_pool(const StemPoolArgs &a, int *err_word, int num_sms, cudaStream_t s) {
   if (!stem_pool_supported(a)) return false;
   StemParams p;
@@ -548,21 +571,11 @@ bool launch_stem_pool(const StemPoolArgs &a, int *err_word, int num_sms, cudaStr
   p.band_rows = (a.PP + bands - 1) / bands;
   p.bands = (a.PP + p.band_rows - 1) / p.band_rows;
   p.units = a.N * p.bands;
-  p.mr_bytes = (a.Q * 128 + 1023) / 1024 * 1024;
-  // Shared memory: as many groups of input rows as fit, sixteen or eight.
-  size_t smem = 0;
-  auto fits = [&](bool tiled, int ring, int chunk) {
-    p.ring = ring;
-    p.chunk = chunk;
-    p.bk = a.Cf <= 16 ? 16 : a.Cf <= 32 ? 32 : 64;
-    p.in_row = tiled ? (a.Q + 7) / 8 * 8 * p.bk * 2 : a.row_bytes;
-    p.slot_bytes = p.in_row * a.stride_h;
-    const size_t w = ((size_t)a.R * (tiled ? p.bk : a.Cf) * ST_K * 2 + 1023) / 1024 * 1024;
-    smem = 1024 + w + ((size_t)ring * p.slot_bytes + 1023) / 1024 * 1024 + (size_t)ST_NMR * p.mr_bytes + 256 + 8 * 64;
-    return smem <= (size_t)TC_SMEM_LIMIT;
-  };
-  const bool tiled = a.w_fold && (fits(true, 16, 4) || fits(true, 8, 2));
-  if (!tiled && !fits(false, 16, 4) && !fits(false, 8, 1)) return false;
+  StemPoolLayout l;
+  if (!stem_pool_layout(a.R, a.Cf, a.stride_h, a.Q, a.row_bytes, a.w_fold != nullptr, &l)) return false;
+  const bool tiled = l.tiled != 0;
+  p.ring = l.ring; p.chunk = l.chunk; p.bk = l.bk;
+  p.in_row = l.in_row; p.slot_bytes = l.slot_bytes; p.mr_bytes = l.mr_bytes;
   if (p.units == 0) return false;
   if (tiled) {
     const uint64_t dims[4] = {(uint64_t)a.Cf, (uint64_t)a.Q, (uint64_t)a.H, (uint64_t)a.N};
@@ -592,8 +605,7 @@ bool launch_stem_pool(const StemPoolArgs &a, int *err_word, int num_sms, cudaStr
     }
     OCC_CUDA(cudaEventRecord(r.prof_events[2 * prof_slot], s));
   }
-  // at least half of the shared memory, so that one CTA (one TMEM allocation) runs per SM
-  tc_launch_pdl(kernel, grid, ST_THREADS, smem < 120 * 1024 ? 120 * 1024 : smem, s, p);
+  tc_launch_pdl(kernel, grid, ST_THREADS, (size_t)l.smem, s, p);
   if (prof_slot >= 0) OCC_CUDA(cudaEventRecord(r.prof_events[2 * prof_slot + 1], s));
   count(CNT_LAUNCHES);
   count(CNT_TC_LAUNCHES);
