@@ -1988,6 +1988,7 @@ int occamy_synchronize(void) {
 cudaStream_t occamy_stream(void) {
   rt();
   graph_settle();   // the caller may order work of its own behind the calls made so far
+  flush_pending();
   settle_sources();
   return rt().stream;
 }
