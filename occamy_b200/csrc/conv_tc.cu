@@ -1364,10 +1364,7 @@ bool launch_tc_pair(const TcConvArgs &a, const TcConvArgs &b, cudaStream_t s) {
     it->second.ok = pair_plan(a, b, it->second.p, &it->second.smem);
   }
   PairPlan &pl = it->second;
-  if (!pl.ok) {
-    set_error(998, "two-layer plan");
-    return false;
-  }
+  if (!pl.ok) return false;   // (they run one by one)
   Runtime &r = rt();
   pl.p.descending = r.descending;
   r.descending ^= 1;
