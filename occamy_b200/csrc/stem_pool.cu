@@ -562,8 +562,6 @@ bool launch_stem_pool(const StemPoolArgs &a, int *err_word, int num_sms, cudaStr
   p.PP = a.PP; p.QP = a.QP;
   p.lo = a.lo; p.hi = a.hi;
   p.err = err_word;
-  p.descending = rt().descending;
-  rt().descending ^= 1;
   // bands: enough units to balance the SMs, each band re-computes one convolution row
   int bands = 1;
   while ((int64_t)a.N * bands < 6ll * num_sms && a.PP / (bands * 2) >= 4) bands *= 2;
@@ -595,6 +593,8 @@ bool launch_stem_pool(const StemPoolArgs &a, int *err_word, int num_sms, cudaStr
   }
   const int grid = p.units < num_sms ? p.units : num_sms;
   Runtime &r = rt();
+  p.descending = r.descending;
+  r.descending ^= 1;
   int prof_slot = -1;
   if (r.profiling) {   // timed like the other tensor-core launches
     prof_slot = r.prof_count++;
