@@ -24,6 +24,8 @@
 //               memory (swizzled so that a warp's 128-byte rows spread over banks)
 //   4 warps     pool: the largest of three columns -> global memory
 // Every wait is bounded; a wait that runs out records a code and the kernel drains.
+#include <map>
+
 #include "conv_tc_dev.cuh"
 #include "kernels.h"
 #include "runtime.h"
@@ -551,10 +553,21 @@ bool stem_pool_layout(int R, int Cf, int stride_h, int Q, int row_bytes, bool ma
   return (may_tile && (fits(true, 16, 4) || fits(true, 8, 2))) || fits(false, 16, 4) || fits(false, 8, 1);
 }
 
-bool launch_stem_pool(const StemPoolArgs &a, int *err_word, int num_sms, cudaStream_t s) {
-  if (!stem_pool_supported(a)) return false;
+namespace {
+
+struct StemPlan {
   StemParams p;
-  memset(&p, 0, sizeof(p));
+  StemPoolLayout l;
+  int grid;
+  bool ok;
+};
+
+StemPlan stem_plan(const StemPoolArgs &a, int *err_word, int num_sms) {
+  StemPlan pl;
+  memset(&pl, 0, sizeof(pl));
+  StemParams &p = pl.p;
+  StemPoolLayout &l = pl.l;
+  if (!stem_pool_supported(a)) return pl;
   p.x = a.x; p.w = a.w; p.bias = a.bias; p.y = a.y;
   p.N = a.N; p.H = a.H; p.row_bytes = a.row_bytes;
   p.G = (a.R - 1) / a.stride_h + 1;
@@ -569,13 +582,10 @@ bool launch_stem_pool(const StemPoolArgs &a, int *err_word, int num_sms, cudaStr
   p.band_rows = (a.PP + bands - 1) / bands;
   p.bands = (a.PP + p.band_rows - 1) / p.band_rows;
   p.units = a.N * p.bands;
-  StemPoolLayout l;
-  if (!stem_pool_layout(a.R, a.Cf, a.stride_h, a.Q, a.row_bytes, a.w_fold != nullptr, &l)) return false;
-  const bool tiled = l.tiled != 0;
+  if (p.units == 0 || !stem_pool_layout(a.R, a.Cf, a.stride_h, a.Q, a.row_bytes, a.w_fold != nullptr, &l)) return pl;
   p.ring = l.ring; p.chunk = l.chunk; p.bk = l.bk;
   p.in_row = l.in_row; p.slot_bytes = l.slot_bytes; p.mr_bytes = l.mr_bytes;
-  if (p.units == 0) return false;
-  if (tiled) {
+  if (l.tiled) {
     const uint64_t dims[4] = {(uint64_t)a.Cf, (uint64_t)a.Q, (uint64_t)a.H, (uint64_t)a.N};
     const uint64_t st[3] = {16, (uint64_t)a.row_bytes, (uint64_t)a.H * a.row_bytes};
     const uint32_t box[4] = {(uint32_t)p.bk, (uint32_t)(a.Q + 7) / 8 * 8, (uint32_t)(a.stride_h * p.chunk), 1};
@@ -583,17 +593,38 @@ bool launch_stem_pool(const StemPoolArgs &a, int *err_word, int num_sms, cudaStr
     const uint64_t wst[2] = {(uint64_t)a.Cf * 2, (uint64_t)a.Cf * 2 * ST_K};
     const uint32_t wbox[3] = {(uint32_t)p.bk, ST_K, 1};
     if (!make_map(&p.tmX, a.x, 4, dims, st, box, p.bk * 2, true) || !make_map(&p.tmW, a.w_fold, 3, wdims, wst, wbox, p.bk * 2, true))
-      return false;
+      return pl;
   }
-  auto kernel = tiled ? stem_pool_kernel<true> : stem_pool_kernel<false>;
+  pl.grid = p.units < num_sms ? p.units : num_sms;
+  pl.ok = true;
+  return pl;
+}
+
+}  // namespace
+
+bool launch_stem_pool(const StemPoolArgs &a, int *err_word, int num_sms, cudaStream_t s) {
+  struct Key {
+    unsigned char b[sizeof(StemPoolArgs)];
+    bool operator<(const Key &o) const { return memcmp(b, o.b, sizeof(b)) < 0; }
+  };
+  static std::map<Key, StemPlan> plans;   // (two tensor maps take longer to encode than the launch)
+  Key key;
+  memcpy(key.b, &a, sizeof(key.b));
+  auto it = plans.find(key);
+  if (it == plans.end()) {
+    if (plans.size() > 256) plans.clear();
+    it = plans.emplace(key, stem_plan(a, err_word, num_sms)).first;
+  }
+  StemPlan &pl = it->second;
+  if (!pl.ok) return false;
+  auto kernel = pl.l.tiled ? stem_pool_kernel<true> : stem_pool_kernel<false>;
   static unsigned char attr_done[TC_MAX_DEVICES] = {};
   if (tc_first_use_on_device(attr_done)) {
     cudaFuncSetAttribute(stem_pool_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_LIMIT);
     cudaFuncSetAttribute(stem_pool_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_LIMIT);
   }
-  const int grid = p.units < num_sms ? p.units : num_sms;
   Runtime &r = rt();
-  p.descending = r.descending;
+  pl.p.descending = r.descending;
   r.descending ^= 1;
   int prof_slot = -1;
   if (r.profiling) {   // timed like the other tensor-core launches
@@ -605,7 +636,7 @@ bool launch_stem_pool(const StemPoolArgs &a, int *err_word, int num_sms, cudaStr
     }
     OCC_CUDA(cudaEventRecord(r.prof_events[2 * prof_slot], s));
   }
-  tc_launch_pdl(kernel, grid, ST_THREADS, (size_t)l.smem, s, p);
+  tc_launch_pdl(kernel, pl.grid, ST_THREADS, (size_t)pl.l.smem, s, pl.p);
   if (prof_slot >= 0) OCC_CUDA(cudaEventRecord(r.prof_events[2 * prof_slot + 1], s));
   count(CNT_LAUNCHES);
   count(CNT_TC_LAUNCHES);

@@ -63,3 +63,22 @@ def test_wide_stem_with_max_pool(binding, N, H, W, R, S, pad, form, act):
             assert max_rel_err(y, want) <= 2e-2
     assert np.array_equal(got, apart)       # rounded the same way, and the largest of the same values
     assert rt.last_error() == 0
+
+
+def test_a_launch_that_was_made_before_encodes_nothing(binding):
+    """Call by call (while launches are timed nothing is replayed), the tensor maps of a stem are those of the call before."""
+    rt.set_math_mode(rt.MATH_BF16)
+    g = graphs.Graph((2, 3, 60, 66), seed=5)
+    y = g.relu(g.conv(0, *g.he_conv(64, 3, 7, 7), pads=(3, 3), strides=(2, 2)))
+    g.mark_output(g.maxpool(y, (3, 3), (1, 1), (2, 2)))
+    x = graphs.make_input(g, 1)
+    p = g.to_program()
+    p.lower(fuse=replay.FUSE_REFERENCE)
+    rt.lib().occamy_profile_begin()
+    encodes = []
+    for _ in range(8):   # (two pool blocks in turn)
+        p.run(binding, x)
+        encodes.append(rt.counters()["tmap_encodes"])
+    ms = (C.c_float * 64)()
+    assert rt.lib().occamy_profile_end(ms, 64) >= 8
+    assert encodes[4] == encodes[7], encodes
