@@ -514,6 +514,7 @@ bool stem_pool_supported(const StemPoolArgs &a) {
   if (a.w_step_bytes != 16 || a.row_bytes % 16 || a.row_bytes > 8192) return false;
   if (a.Q < 1 || a.Q > 128 || a.P < 1 || a.stride_h < 1 || a.stride_h > 4) return false;
   if ((a.R - 1) / a.stride_h + 1 > 6) return false;   // groups a row holds at once
+  if (a.pad_h >= a.R) return false;   // every row of the output has a filter row inside the image
   if (a.PP != (a.P + 2 - 3) / 2 + 1 || a.QP != (a.Q + 2 - 3) / 2 + 1) return false;
   if ((uintptr_t)a.x % 16 || (uintptr_t)a.w % 16 || (uintptr_t)a.y % 16) return false;
   // the last window the tensor core reads for a real column must lie inside the row

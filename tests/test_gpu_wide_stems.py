@@ -82,3 +82,20 @@ def test_a_launch_that_was_made_before_encodes_nothing(binding):
     ms = (C.c_float * 64)()
     assert rt.lib().occamy_profile_end(ms, 64) >= 8
     assert encodes[4] == encodes[7], encodes
+
+
+@pytest.mark.parametrize("R,pad", [(3, 3), (3, 5), (5, 5), (5, 4)])
+def test_rows_of_padding_alone(binding, R, pad):
+    """Padding as high as the filter: the first and last rows of the output are the bias."""
+    rt.set_math_mode(rt.MATH_BF16)
+    g = graphs.Graph((3, 3, 21, 26), seed=R + pad)
+    y = g.relu(g.conv(0, *g.he_conv(64, 3, R, R), pads=(pad, pad), strides=(2, 2)))
+    g.mark_output(g.maxpool(y, (3, 3), (1, 1), (2, 2)))
+    x = graphs.make_input(g, 1)
+    (want,) = run_graph_oracle(g, x)
+    p = g.to_program()
+    p.lower(fuse=replay.FUSE_REFERENCE)
+    for _ in range(4):
+        (got,) = p.run(binding, x)
+        assert max_rel_err(got, want) <= 2e-2
+    assert rt.last_error() == 0
