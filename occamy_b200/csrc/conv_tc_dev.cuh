@@ -17,7 +17,7 @@ namespace occ {
 
 constexpr int TC_THREADS = 320;      // pixel-N kernel: 1 producer warp + 1 MMA warp + 8 epilogue warps
 constexpr int TC_EW = 2;             // tc_conv_kernel: epilogue warps per TMEM lane quadrant
-constexpr int TC_NSTORE = 2;         // tc_conv_kernel: slab-store threads (slab buffers: a multiple)
+constexpr int TC_NSTORE = 2;         // tc_conv_kernel: slab-store warps (slab buffers: a multiple)
 constexpr int TC_EPI_THREADS = 256;
 constexpr int TC_DBUF = 3;           // output slab buffers in shared memory
 constexpr int TC_MAX_TAPS = 64;
@@ -69,7 +69,7 @@ struct alignas(64) TcParams {
   int halo_a_bytes;      //   bytes of one staged block, a multiple of 1024
   int bias_floats;       // K rounded up to whole channel tiles: bias entries kept in shared memory
   int dbuf;              // output slab buffers in shared memory (an even number, 4..12)
-  int store_pend;        // stores a store thread may leave in flight behind its newest (0..3)
+  int store_pend;        // stores a store warp may leave in flight behind its newest (0..3)
   // TC_MODE_ROWS: the padded input rows, their length, their place in a stage, bytes of a window; the filter's geometry
   const uint8_t *rows_x;
   int row_bytes, row_slot, window, in_h, stride_h, pad_h;
@@ -251,14 +251,6 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *m, 
       "l"(m), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *m, uint32_t bar,
-                                            int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
-      "l"(m), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap *m, uint32_t src, int c0, int c1,
                                              int c2, int c3) {
   asm volatile(
@@ -367,24 +359,7 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   bar)
-               : "memory");
-}
-// One MMA; the descriptors arrive as 32-bit halves (address field in the low word).
-__device__ __forceinline__ void mma_lohi(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
-                                         uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\n.reg .b64 da, db;\n"
-      "setp.ne.b32 p, %6, 0;\n"
-      "mov.b64 da, {%1, %2};\n"
-      "mov.b64 db, {%3, %4};\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}" ::"r"(d_tmem),
-      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// ---- the same by one lane of a warp that executes them as a whole.
+// ---- loads, MMAs, commits and arrivals by one lane of a warp that executes them as a whole.
 // These instructions take their operands from uniform registers.  In code that one lane runs by itself the operands are
 // that lane's, and every instruction waits for a handful of moves: an MMA was issued every 100 cycles or so, although the
 // tensor core takes a small one in 48.  Warps that load or issue MMAs therefore run their role as a whole, on values that
@@ -392,6 +367,7 @@ __device__ __forceinline__ void mma_lohi(uint32_t d_tmem, uint32_t a_lo, uint32_
 // 56x56 66 -> 60 us, 128 -> 128 at 28x28 51 -> 46.5, 512 -> 128 there 46 -> 43.  ResNet-50 with 8 images 328 -> 303 us,
 // 32 554 -> 520, 61 at 201x201 804 -> 770, 16 in fp32 1438 -> 1308; MobileNetV2 with 128 860 -> 805; VGG-16 with 64
 // 1888 -> 1823, 5 290 -> 277.
+// (The descriptors of an MMA arrive as 32-bit halves, the address field in the low word.)
 __device__ __forceinline__ void mma_warp(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
                                          uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -713,7 +689,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
     tma_prefetch_map(&p.tmB);
     if (!F32) tma_prefetch_map(&p.tmD);
     for (int s = 0; s < stages; ++s) {
-      mbar_init(full_bar(s), two_loaders ? 2 : 1);   // one arming arrival per loading thread
+      mbar_init(full_bar(s), two_loaders ? 2 : 1);   // one arming arrival per loading warp
       mbar_init(empty_bar(s), 1);
     }
     for (int s = 0; s < 2; ++s) {
@@ -905,7 +881,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
       if constexpr (HALO) {
         // 3x3 taps as shifted windows of the staged block: (dh * wp + dw) pixels of 128 bytes
         // further on.  Straight-line issue code: the MMAs are short when BN is small, and a
-        // taken branch costs the issuing thread more than one of them.
+        // taken branch costs the issuing warp more than one of them.
         const uint64_t d0 = make_smem_desc(sA, 64);
         const uint32_t a_hi = (uint32_t)(d0 >> 32), b_hi = a_hi;
         const uint32_t a_lo0 = (uint32_t)d0;
@@ -913,8 +889,8 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
         const uint32_t stage_desc = a_bytes >> 4, tap_desc = b_bytes >> 4;
         const uint32_t wp8 = (uint32_t)p.halo_wp * 8u;   // one block row in descriptor units
         if (!mbar_wait_warp(wfull_bar, 0, abort_flag)) err_code = 3;
-        // Two issuing threads take alternate tiles (and with them alternate accumulators):
-        // 36 MMAs of 48 cycles per tile are more than one thread issues in that time.
+        // Two issuing warps take alternate tiles (and with them alternate accumulators):
+        // 36 MMAs of 48 cycles per tile are more than one issues in that time.
         const int me = warp == 1 ? 0 : 1;
         int it = 0;   // tiles of this CTA so far
         for (int tile = blockIdx.x; tile < p.total_tiles && !err_code; tile += gridDim.x, ++it) {
@@ -1345,7 +1321,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), EW == 1 ? 2 : 1)
             if (keep)
               *reinterpret_cast<uint4 *>(dptr + soff[c4]) =
                   make_uint4(pk[c4 * 4], pk[c4 * 4 + 1], pk[c4 * 4 + 2], pk[c4 * 4 + 3]);
-          // this warp's part of the slab is written: tell the store thread
+          // this warp's part of the slab is written: tell the store warp
           fence_async_smem();
           __syncwarp();
           if (lane == 0) mbar_arrive(dfull_bar(buf));

@@ -17,10 +17,10 @@
 //
 // Up to four warps issue the MMAs (whole warps, k-steps in turn, an accumulator of their own each)
 // and as many load (k-steps in turn), then all eight warps drain the accumulators (two
-// per TMEM lane quadrant, half of the columns each).  Several threads per role, because one thread's
-// round of barrier poll, issue and commit takes 450 to 600 cycles whatever it moves, and the four MMAs
-// of a k-step 200 to 260.  A ring that is reused has a multiple of that many stages: a stage then always
-// belongs to the same two threads, and no barrier can be two phases behind the one that waits on it.
+// per TMEM lane quadrant, half of the columns each).  Several warps per role, because a
+// round of barrier poll, issue and commit takes longer than the four MMAs of a k-step (200 to 260 cycles): a lone
+// thread's took 450 to 600, whatever it moved.  A ring that is reused has a multiple of that many stages: a stage then always
+// belongs to the same two warps, and no barrier can be two phases behind the one that waits on it.
 #include "conv_tc_split.cuh"
 
 #include "kernels.h"

@@ -67,7 +67,7 @@ struct alignas(64) StemParams {
 };
 
 // An MMA that is issued only when `valid` is non-zero (a predicated instruction, not a branch:
-// a taken branch costs the single issuing thread more than the MMA it would skip).
+// a taken branch costs the issuing warp more than the MMA it would skip).
 __device__ __forceinline__ void mma_lohi_if(uint32_t valid, uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi,
                                             uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
                                             uint32_t accumulate) {
@@ -240,8 +240,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stem_pool_kernel(const __grid_c
     }
   } else if (warp == 1 || warp >= ST_ISSUER_B) {
     // ------------------------------------------------------------ MMA issuers
-    // Two threads (in two warps) take alternate convolution rows: the MMAs are short (64
-    // columns) and one thread cannot issue them as fast as the tensor core retires them.
+    // Two warps take alternate convolution rows: the MMAs are short (64
+    // columns) and one cannot issue them as fast as the tensor core retires them.
     // Both read every input group, so a group goes back to the producer when both have
     // committed it (each does so once it will not read the group again).
     {
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stem_pool_kernel(const __grid_c
           const int r_lo = max(0, -jb), r_hi = min(p.R - 1, p.H - 1 - jb);
           const uint32_t d_tmem = tmem_base + a * ST_K;
           const uint32_t s0 = (gbase + (uint32_t)k) & (ring - 1u);
-          // The issue code is straight-line: every taken branch costs the issuing thread more
+          // The issue code is straight-line: every taken branch costs the issuing warp more
           // than an MMA.
           if (p.R == 7 && kk_n == 2 && p.stride_h == 2 && r_lo == 0 && r_hi == 6) {
             issue_whole_row<7, 2, 2>(d_tmem, s0, ring, a_lo0, a_hi, slot_desc, row_desc, b_lo0, b_hi, tap_desc, kstep_desc,
