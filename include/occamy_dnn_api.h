@@ -207,7 +207,8 @@ void occamy_get_counters(int64_t out[8]);
  * residuals as one kernel, [2] 3x3 layers as column strips, [3] convolutions that took a
  * 2x2 max pool along, [4] inferences whose recorded part ran as graphs, [5] such that were computed in
  * pieces while their batch arrived, [6] convolutions that took another one's result along as a second
- * summand, [7] pairs of layers as one kernel.  Returns how many there are. */
+ * summand, [7] pairs of layers as one kernel, [8] few-channel convolutions that read whole input rows.  Returns how
+ * many there are. */
 int occamy_get_form_counters(int64_t *out, int n);
 /* Per-launch timing of the tensor-core convolution / GEMM kernel: after _begin, every such
  * launch is bracketed by a CUDA-event pair on the launch stream; _end waits for the stream,

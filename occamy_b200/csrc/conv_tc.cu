@@ -1262,6 +1262,7 @@ void launch_tc_conv(const TcConvArgs &a, cudaStream_t s) {
   count(CNT_TC_LAUNCHES, a.x2 ? 2 : 1);
   if (pl.sk) count(CNT_SPLIT_REDUCTION);
   else if (pl.p.halo) count(CNT_COLUMN_STRIPS);
+  else if (pl.mode & TC_MODE_ROWS) count(CNT_ROWS);
   if (a.pool2) count(CNT_POOLED);
   if (a.x2) count(CNT_SUMMED);
 }

@@ -89,7 +89,8 @@ enum Counter {
   CNT_IN_PIECES = 13,
   CNT_SUMMED = 14,
   CNT_PAIRS = 15,
-  CNT_COUNT = 16
+  CNT_ROWS = 16,
+  CNT_COUNT = 17
 };
 
 struct Runtime {

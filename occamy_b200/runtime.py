@@ -156,7 +156,7 @@ def counters() -> dict:
 
 
 FORM_NAMES = ("split_reduction", "inverted_residual", "column_strips", "pooled", "replayed", "in_pieces", "summed",
-              "pairs")
+              "pairs", "input_rows")
 
 
 def form_counters() -> dict:
