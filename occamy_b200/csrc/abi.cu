@@ -1327,7 +1327,7 @@ int cudnnCreate(cudnnContext **handle) {
   rt();
   *handle = reinterpret_cast<cudnnContext *>(malloc(16));
   graph_inference_begin();
-  rt().descending = 1;   // (the input passes write from the first image to the last)
+  went_forwards();   // (whatever brought the input in)
   flush_pending();
   trace_begin();
   return *handle ? 0 : 2;

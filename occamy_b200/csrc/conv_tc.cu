@@ -1255,8 +1255,12 @@ void launch_tc_conv(const TcConvArgs &a, cudaStream_t s) {
   }
   if (pl.p.total_tiles == 0) return;
   Runtime &r = rt();
-  pl.p.descending = r.descending;
-  r.descending ^= 1;
+  if (pl.sk) {
+    went_forwards();
+  } else {
+    pl.p.descending = r.descending;
+    r.descending ^= 1;
+  }
   profiled(s, [&] { launch_any(pl, r.num_sms, s); });
   count(CNT_LAUNCHES);
   count(CNT_TC_LAUNCHES, a.x2 ? 2 : 1);

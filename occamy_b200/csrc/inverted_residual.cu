@@ -820,6 +820,7 @@ void ir_launch_one(const IrPlan &pl, cudaStream_t s) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   }
   tc_launch_pdl(kernel, pl.grid, IR_THREADS, pl.c.smem, s, pl.p, pl.p.splits);
+  went_forwards();
 }
 template <int EC, int ST>
 void ir_launch_es(const IrPlan &pl, bool f16, cudaStream_t s) {

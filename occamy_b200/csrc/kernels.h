@@ -26,6 +26,8 @@ void enqueue_kernel(const void *kernel, const cudaLaunchConfig_t &cfg, void **ar
 void enqueue_copy(void *dst, const void *src, size_t bytes, cudaStream_t s);   // device to device
 void enqueue_zero(void *dst, size_t bytes, cudaStream_t s);
 
+void went_forwards();   // the kernel being launched writes from the first image to the last (Runtime::descending)
+
 template <bool CHAINED, typename... P, typename... A>
 inline void launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
@@ -49,6 +51,7 @@ inline void launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t sm
 template <typename... P, typename... A>
 inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
   launch_kernel<true>(kernel, grid, block, smem, s, args...);
+  went_forwards();
 }
 // A kernel without chain_begin(): packing, once per constant.
 template <typename... P, typename... A>

@@ -274,6 +274,8 @@ void ensure_f32(const void *p) {
   rec->fmt = FMT_F32;
 }
 
+void went_forwards() { rt().descending = 1; }
+
 void settle_sources() {
   std::vector<uintptr_t> all;
   for (const auto &kv : rt().recs)

@@ -112,8 +112,9 @@ struct Runtime {
   void *host_stage = nullptr;   // pinned, STAGE_BYTES: small results on their way to pageable memory
   bool log = false;
   bool cache_weights = true;
-  // The next tensor-core kernel takes its tiles from the last to the first, in turn with the one before it: what that
-  // one wrote last is still in L2 (126 MB, of tensors of 100 to 400 MB).  ResNet-50 at 256 images 3287 -> 3221 us, 61
+  // The next tensor-core kernel takes its tiles from the last to the first: the one before it took them from the first
+  // to the last, and what it wrote last is still in L2 (126 MB, of tensors of 100 to 400 MB).  Kernels that know one
+  // order only (went_forwards()) leave it set; the others take turns.  ResNet-50 at 256 images 3287 -> 3221 us, 61
   // at 201x201 938 -> 931, host batches 4531 -> 4493, VGG-16 at 64 1999 -> 1988; small batches the same.
   int descending = 0;
   // called before the runtime itself writes into a caller-owned range (lazy zero fill,
