@@ -29,8 +29,8 @@ struct SavedRec {
 
 // A window cut up by images: its calls are made for a piece of the batch after the other, each piece as one
 // graph, on tensors in memory of the runtime's.  What it is for is a batch that comes from the host: the
-// pieces are computed while the later ones are still on their way (batch 256 of a ResNet-50 takes 2.9 ms to
-// arrive and 3.1 to compute).
+// pieces are computed while the later ones are still on their way (batch 256 of a ResNet-50 takes 2.8 ms to
+// arrive and 2.6 to compute).
 constexpr int MAX_PIECES = 4;
 
 // An executable graph.  One that goes out of use may still be running: it is destroyed later (empty_trash()).
@@ -459,23 +459,28 @@ void wait_for_upload() {
 }
 
 // ---- windows cut up by images -------------------------------------------------------
-// Images of each piece: the first is what is waited for, so it is the smallest (256 images: 64, 96, 96
-// took 4.5 ms where three of 85 took 4.7).  None for batches below 128, nor in the fp32 mode, which computes for
-// longer than the upload takes.  Milliseconds per inference from pinned memory to host memory, 224x224, whole batch
-// and pieces:
-//     images               64             96            128            192            256
-//     ResNet-50    1.87 / 2.12    2.50 / 2.53    3.24 / 2.91    4.56 / 3.68    5.96 / 4.49
-//     MobileNetV2  1.38 / 1.30    1.89 / 1.67    2.44 / 2.06                   4.53 / 3.69
-//     VGG-16       2.64 / 2.43                   4.94 / 4.45
-//     fp32 ResNet  5.72 / 6.44                  10.44 / 10.67
+// Images of each piece.  The first has to arrive before anything is computed and the last is computed when nothing
+// arrives any more; the others cost a start of fifty kernels each.  None is larger than the last (lay_out() makes room for
+// that one).  None for batches below 128, nor in the fp32 mode, which computes for longer than the upload takes.
+// Milliseconds per inference from pinned memory to host memory, 224x224: whole batch, 1/4 + 3/8 + 3/8, and 3/16 + 1/4 +
+// 9/32 + 9/32.
+//     images               128                  160                  192                  224                  256
+//     ResNet-50    2.89 / 2.36 / 2.47   3.47 / 2.73 / 2.77   4.10 / 3.12 / 3.14   4.78 / 3.55 / 3.51   5.32 / 3.98 / 3.81
+//     MobileNetV2  2.32 / 1.99 / 1.96                        3.36 / 2.77 / 2.76                        4.36 / 3.63 / 3.49
+//     VGG-16       4.34 / 3.69 / 3.67
+// (Below 128, and in the fp32 mode, with the kernels of an earlier build: ResNet-50 with 64 images 1.87 whole and 2.12 in
+// pieces, 96 2.50 and 2.53; MobileNetV2 1.38 / 1.30 and 1.89 / 1.67; VGG-16 with 64 2.64 / 2.43; fp32 5.72 / 6.44, 128
+// 10.44 / 10.67.)
+// The first inference on newly pinned memory takes 1.2 ms longer with 256 images, whole or in pieces: its upload does (a
+// copy by itself 4.7 ms there and 3.6 from then on).
 int piece_images(int64_t n, int64_t *images) {
   if (n < 128 || rt().mode == MATH_FP32) return 0;
-  const int pieces = n < 192 ? 3 : 4;
+  const int pieces = n < 208 ? 3 : 4;
   images[0] = n / (pieces == 3 ? 8 : 16) * (pieces == 3 ? 2 : 3) / 8 * 8;
   int64_t left = n - images[0];
   if (pieces == 4) left -= images[1] = n / 4 / 8 * 8;
   images[pieces - 2] = left / 2 / 8 * 8;
-  images[pieces - 1] = left - images[pieces - 2];   // (none is larger)
+  images[pieces - 1] = left - images[pieces - 2];
   return pieces;
 }
 

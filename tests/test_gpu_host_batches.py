@@ -120,7 +120,10 @@ def test_pieces_need_other_kernels(binding):
 
 
 @pytest.mark.parametrize("name,math,N,image", [("resnet50", rt.MATH_BF16, 160, 97), ("mobilenet_v2", rt.MATH_F16, 160, 128),
-                                               ("vgg16", rt.MATH_BF16, 136, 112)])
+                                               ("vgg16", rt.MATH_BF16, 136, 112),
+                                               # four pieces
+                                               ("resnet50", rt.MATH_BF16, 208, 97), ("resnet50", rt.MATH_BF16, 253, 129),
+                                               ("mobilenet_v2", rt.MATH_F16, 235, 112), ("vgg16", rt.MATH_BF16, 209, 97)])
 def test_same_bits_in_pieces(binding, name, math, N, image):
     """An image's result does not depend on whether its batch was computed in pieces."""
     rt.set_math_mode(math)
