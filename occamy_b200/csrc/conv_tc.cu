@@ -702,7 +702,8 @@ static void pool_box(int Q, int P, int N, int *tw, int *th, int *tn) {
 
 // A layer of the wide form: strips of columns, whose pixels and the two columns between their rows are the N side (at
 // most 256).  The cheapest cover of the image, by tiles per SM and cycles of a tile (two per column of an MMA and tap,
-// and what a tile costs by itself).  False when none fits shared memory.
+// and what a tile costs by itself).  False when none fits shared memory,
+// which does not depend on how many images there are: the form sums up in an order of its own.
 static bool wide_box(const TcConvArgs &a, int nsm, TcParams *p, size_t *smem) {
   const int even = a.pool2 ? 2 : 1, cblocks = a.Cf / 64;
   double best = -1.0;
@@ -833,8 +834,10 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   Plan pl;
   memset(&pl, 0, sizeof(pl));
   TcParams &p = pl.p;
-  // A piece of a batch: the split-reduction kernel, with the same shares, where the whole batch takes it.  (The
-  // persistent kernels sum up in one order, whatever their tiles.)
+  // A piece of a batch: the split-reduction kernel, with the same shares, where the whole batch takes it.  (Each of the
+  // persistent kernels sums up in one order, whatever its tiles: filter taps outside and channels inside, the wide form the
+  // other way round.  So that an image has the same bits in a piece, which of them a layer takes must not depend on the
+  // number of images; `wide` below does not: wide_box() finds a box or none by the image and the channels.)
   const bool piece = a.form_n != 0;
   SkChoice whole{0, 1, 0, -1.0};
   if (piece) {

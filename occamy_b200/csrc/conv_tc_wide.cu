@@ -9,8 +9,8 @@
 // swizzled operand may start at any multiple of 128 bytes.  The N index runs through the block's rows, so two of its
 // columns are junk (an eighth of 14-column strips), which the epilogue leaves out.
 // Before (tc_conv_pn_kernel, pool by itself) and now: 128 -> 128 at 28x28, 256 images, 59.6 -> 46.0 us, 32 images
-// 17.7 -> 13.3; 64 -> 128 at 112x112, 64 images, 159 -> 102; 128 -> 128 there with its pool 193 + 36 -> 151.  The last is
-// 1570 TFLOP/s of MMAs made, 0.95 of the burst rate, an eighth of them on junk columns.
+// 17.7 -> 13.3; 64 -> 128 at 112x112, 64 images, 159 -> 103; 128 -> 128 there with its pool 193 + 36 -> 152.  The last is
+// 1560 TFLOP/s of the layer's own operations, 0.94 of the burst rate; what the junk columns take comes on top.
 //
 // One persistent CTA per SM, roles by warp:
 //   (warps 0, 1 and 10: whole warps that elect a lane for each instruction)

@@ -933,12 +933,15 @@ bool ir_supported(int N, int C, int E, int K, int H, int W, int P, int Q, int st
   const IrChoice c = ir_choose(N, C, E, K, P, Q, stride, f16, rt().num_sms);
   // Worth it where the separate kernels (3.3 us each, 4.6 TB/s of their tensors) take longer.  MobileNetV2's
   // blocks, fp16: at batch 1 all of them (10.5 -> 5.5 us each), at batch 128 those at 112x112 and 56x56 (197 ->
-  // 117, 150 -> 121, 125 -> 61 us) and some later ones; not those at 28x28 (37 -> 45 us).
-  // The last factor is for the model's error: a block is fused where the gain is plain.  The model's kernel loaded and
-  // issued by one lane; as a whole warp it takes 0.77 to 0.95 of the time, where no cluster shares the chunks: fused and
+  // 117, 150 -> 121, 125 -> 61 us) and some later ones.
+  // The last factor is for the model's error: a block is fused where the gain is plain.  The model was fitted to a kernel
+  // that loaded and issued by one lane, and has not been since; as a whole warp it takes 0.77 to 0.95 of the time, where no
+  // cluster shares the chunks: fused and
   // apart now 112 and 118 us (24 -> 144 -> 24 at 56x56, batch 128; 61 and 70 at 64), 37 and 46 (32 -> 192 -> 32 at 28x28),
   // 24 and 29 (96 -> 576 -> 160, stride 2), 24 and 31 (96 -> 576 -> 96 at 14x14, batch 64), 47 and 47 (there at 128, 1.18
-  // by the model).  In clusters 35 against 25 (96 -> 576 -> 160 at 64, 1.06 by the model).
+  // by the model).  In clusters 35 against 25 (96 -> 576 -> 160 at 64, 1.06 by the model).  With fp32 sums in the depthwise
+  // stage it is slower again, and the lower factor stays: MobileNetV2 in bf16 with factors of 0.9, 1.0, 1.1 and 1.2 takes
+  // 203, 203, 203 and 203 us (4 images), 314, 314, 315, 315 (16), 574, 577, 590, 604 (64), 966, 964, 956, 976 (128).
   double bytes = 2.0 * N * ((double)H * W * (C + 2.0 * E) + (double)P * Q * (2.0 * E + K + (C == K ? K : 0)));
   if (C % 16) bytes += 5.0 * N * H * W * (C + 16);   // the separate kernels' input is padded in a pass of its own
   const double margin = f16 && c.splits == 1 ? 1.1 : 0.9;
