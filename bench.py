@@ -521,9 +521,9 @@ def main():
                      "frac_of_sustained_peak": achieved / peaks["bf16_tflops_sustained"],
                      "traffic": profiled_traffic(per_rank, args.graph) if world == 1 else None,
                      "traffic_note": "DRAM read+write bytes of the tensor-core launches of one "
-                                     "step (ncu, profiles/tc_conv_traffic_resnet50_b256.txt; taken of the "
-                                     "persistent kernels before the column strips)",
-                     "kernel": "tc_conv_kernel (+ tc_conv_pn_kernel, stem_pool_kernel)",
+                                     "step (ncu, profiles/tc_conv_traffic_resnet50_b256.txt)",
+                     "kernel": "tc_conv_kernel (+ tc_pair_kernel, tc_conv_wide_kernel, "
+                               "tc_split_kernel, stem_pool_kernel)",
                      "launches_per_step": per_step,
                      "kernel_ms_per_step": tc_total_ms,
                      "peak_source": peaks["source"] + " (burst cuBLAS bf16: launches are timed "
