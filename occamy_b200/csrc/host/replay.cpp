@@ -289,7 +289,8 @@ struct Lowering {
           const bool has_bias = nd.in[2] >= 0;
           if (fuse && has_bias && nd.groups == 1) {
             act_mode = 5;
-            if (users[nd.out].size() == 1) {
+            const bool kept = std::find(p.outputs.begin(), p.outputs.end(), nd.out) != p.outputs.end();
+            if (users[nd.out].size() == 1 && !kept) {   // (the model's caller is a consumer, too)
               Node &u = p.nodes[users[nd.out][0]];
               if (u.kind == N_RELU) { act_mode = 1; act_node = users[nd.out][0]; }
               else if (fuse == 2 && u.kind == N_CLIP && u.lo == 0.f && u.hi == 6.f) {

@@ -162,3 +162,21 @@ def test_offline_plan_is_valid_and_not_larger(name, batch, native_libs):
             if a1 <= b2 and a2 <= b1:          # live together
                 assert e1 <= o2 or e2 <= o1, (spans[i], spans[j])
         assert spans[i][1] <= p2.pool_bytes
+
+
+@pytest.mark.parametrize("fuse", [replay.FUSE_REFERENCE, replay.FUSE_WITH_CLIP])
+@pytest.mark.parametrize("kept", [False, True])
+def test_a_result_of_the_model_is_not_fused_away(native_libs, fuse, kept):
+    """A convolution whose own result is an output of the model keeps it: the activation behind it is a call of its own."""
+    g = graphs.Graph((1, 16, 8, 8), seed=0)
+    a = g.conv(0, *g.he_conv(16, 16, 1, 1))
+    b = g.conv(g.relu(a), *g.he_conv(16, 16, 1, 1))
+    g.mark_output(g.clip(b, 0.0, 6.0))
+    for v in (a, b) if kept else ():
+        g.mark_output(v)
+    p = g.to_program()
+    p.lower(fuse=fuse)
+    c = p.instr_counts()
+    assert c["conv_bias_act"] == 2 and c["d2h_output"] == (3 if kept else 1)
+    assert c["active"] == (1 if kept else 0)
+    assert c["clip"] == (0 if fuse == replay.FUSE_WITH_CLIP and not kept else 1)
