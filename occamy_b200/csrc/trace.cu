@@ -339,6 +339,11 @@ void analyse(const std::vector<Entry> &rec, std::vector<uint16_t> &roles, std::v
     if (!f.fusable || f.parts || !one_by_one(f) || f.in[0] != chain_out[i] || f.in_bytes[0] != c.out_bytes || chain_res[j] ||
         !chain_act[j] || (roles[j] & (RF_LINK | RF_JOIN | RF_SUM)) || !passive_past(chain_last[i] + 1, j, chain_out[i], c.out_bytes))
       continue;
+    // The first result is written when both chains are complete: its place must not be handed out again before that.
+    bool stays = true;
+    for (size_t t = j; t <= chain_last[j] && stays; ++t)
+      stays = !is_passive(rec[t].sym) || passive_past(t, t + 1, chain_out[i], c.out_bytes);
+    if (!stays) continue;
     roles[i] |= RF_LEAD;
     roles[j] = (uint16_t)((roles[j] & ~ROLE_BITS) | R_DEFER | RF_FOLLOW);
   }

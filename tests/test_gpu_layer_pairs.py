@@ -56,3 +56,37 @@ def test_pairs(binding, N, C, H, W, M, K1, K2, stride, kw, taken, fuse, mode):
         assert max_rel_err(y, want) <= 2e-2
     assert np.array_equal(got[2], got[3])
     assert rt.last_error() == 0
+
+
+@pytest.mark.parametrize("mode", [rt.MATH_BF16, rt.MATH_F16])
+@pytest.mark.parametrize("act", ["relu", "clip"])
+@pytest.mark.parametrize("N,C,H,W,M,K1,K2", [(3, 64, 19, 23, 64, 128, 64), (61, 64, 26, 25, 64, 256, 64), (9, 32, 25, 28, 128, 256, 256)])
+def test_first_result_that_is_read_once(binding, N, C, H, W, M, K1, K2, act, mode):
+    """Nobody but the second layer reads the first one's result, whose memory is handed out again while that layer's bias and
+    activation, calls of their own, are still to come: they are part of it all the same, with the bits of the fused call."""
+    g = graphs.Graph((N, C, H, W), seed=N + K1)
+    x = g.relu(g.conv(0, *g.he_conv(C, C, 1, 1)))
+    t = g.relu(g.conv(x, *g.he_conv(M, C, 3, 3), pads=(1, 1)))
+    y = g.relu(g.add(g.conv(t, *g.he_conv(K1, M, 1, 1)), g.conv(x, *g.he_conv(K1, C, 1, 1))))
+    r = g.conv(y, *g.he_conv(K2, K1, 1, 1))
+    r = g.relu(r) if act == "relu" else g.clip(r, 0.0, 6.0)
+    for _ in range(2):
+        r = g.relu(g.conv(r, *g.he_conv(K2, K2, 3, 3), pads=(1, 1)))
+    g.mark_output(r)
+    x = graphs.make_input(g, 3)
+    (want,) = run_graph_oracle(g, x)
+    rt.set_math_mode(mode)
+    got, launches = [], []
+    for fuse in (replay.FUSE_WITH_CLIP, replay.FUSE_NONE):
+        p = g.to_program()
+        p.lower(fuse=fuse)
+        for _ in range(4):
+            n0 = rt.counters()["launches"]
+            y = p.run(binding, x)[0]
+            n = rt.counters()["launches"] - n0
+        got.append(y)
+        launches.append(n)
+        assert max_rel_err(y, want) <= 2e-2
+    assert np.array_equal(got[0], got[1])
+    assert launches[1] <= launches[0] + 1   # (one more where the pair is one kernel in the first)
+    assert rt.last_error() == 0
