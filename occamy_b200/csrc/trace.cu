@@ -452,12 +452,15 @@ Role trace_step(Entry &e, bool *deviated) {
     ts.cands.resize(keep);
     if (keep) {
       // recorded programs that share this prefix must agree on the call's role (two models
-      // with the same first layers may continue differently); otherwise it runs as it stands
-      const uint16_t r = ts.programs[ts.cands[0]].roles[index];
+      // with the same first layers may continue differently); otherwise it runs as it stands.  What
+      // it does together with the convolution behind or before it is left out if they disagree on that alone.
+      uint16_t r = ts.programs[ts.cands[0]].roles[index];
+      for (size_t k = 1; k < keep; ++k)
+        r &= ~((r ^ ts.programs[ts.cands[k]].roles[index]) & RF_TOGETHER);
       role = (Role)(r & ROLE_BITS);
       ts.last_flags = r & (uint16_t)~ROLE_BITS;
       for (size_t k = 1; k < keep; ++k)
-        if (ts.programs[ts.cands[k]].roles[index] != r ||
+        if (((ts.programs[ts.cands[k]].roles[index] ^ r) & ~RF_TOGETHER) ||
             ((r & RF_FOR_CONV) && ts.programs[ts.cands[k]].sigs[ts.programs[ts.cands[k]].reader[index]] !=
                                       ts.programs[ts.cands[0]].sigs[ts.programs[ts.cands[0]].reader[index]])) {
           role = R_EAGER;

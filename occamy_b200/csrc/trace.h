@@ -100,6 +100,7 @@ constexpr uint16_t RF_SUM = 0x80;
 // result: one kernel may write both (launch_tc_pair())
 constexpr uint16_t RF_LEAD = 0x100;
 constexpr uint16_t RF_FOLLOW = 0x200;
+constexpr uint16_t RF_TOGETHER = RF_SUM | RF_LEAD | RF_FOLLOW;   // each may be left out
 constexpr uint16_t ROLE_BITS = 0x03;
 struct TraceProgram {
   std::vector<uint64_t> sigs;

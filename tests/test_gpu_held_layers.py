@@ -131,3 +131,25 @@ def test_sequences_that_part_while_layers_are_held(native_libs, way, front):
                 continue
             assert err <= 2e-2, (i, name)
         assert rt.last_error() == 0, i   # ... and the sequence that reads it is recorded anew
+
+
+@pytest.mark.parametrize("way", ["another layer behind", "end read", "summand read"])
+def test_programs_that_part_share_what_they_agree_on(native_libs, way):
+    """Two recorded programs with the same first layers: a chain that both have is one kernel in both, whatever one of them
+    would have done with it together with the next convolution."""
+    rt.set_math_mode(rt.MATH_BF16)
+    block = _Block(20 + WAYS.index(way), 1)
+
+    def steady(w, passes):
+        for _ in range(passes):
+            n0 = rt.counters()["launches"]
+            errs = block.run(w)
+            n = rt.counters()["launches"] - n0
+        assert max(errs.values()) <= 2e-2 and rt.last_error() == 0
+        return n
+
+    alone = steady(way, 5)   # (recorded first: nothing that it reads has been skipped)
+    steady("", 2)
+    # both summands as one kernel, if one of the programs reads one of them: not in the other either
+    assert steady(way, 3) <= alone
+    assert steady("", 3) <= alone + 1
