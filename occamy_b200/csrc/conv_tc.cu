@@ -701,12 +701,17 @@ static void pool_box(int Q, int P, int N, int *tw, int *th, int *tn) {
 }
 
 // A layer of the wide form: strips of columns, whose pixels and the two columns between their rows are the N side (at
-// most 256).  The cheapest cover of the image, by tiles per SM and cycles of a tile (two per column of an MMA and tap,
-// and what a tile costs by itself).  False when none fits shared memory,
+// most 256).  The cheapest cover of the image, by tiles per SM and cycles of a tile (two per column of an MMA and tap, the
+// tap's weights, and what a tile costs by itself).  False when none fits shared memory,
 // which does not depend on how many images there are: the form sums up in an order of its own.
-static bool wide_box(const TcConvArgs &a, int nsm, TcParams *p, size_t *smem) {
+struct WideBox {
+  int tw, th, wp, x_bytes, slab;
+  size_t smem;
+  double cycles;   // of an SM
+};
+static bool wide_box(const TcConvArgs &a, int nsm, WideBox *box) {
   const int even = a.pool2 ? 2 : 1, cblocks = a.Cf / 64;
-  double best = -1.0;
+  box->cycles = -1.0;
   for (int n = 1; n <= (a.W + 7) / 8; ++n) {
     const int tw = ((a.W + n - 1) / n + even - 1) / even * even, wp = tw + 2, c16 = (tw + 15) / 16 * 16;
     if (c16 > 256 || wp > 256) continue;
@@ -722,19 +727,24 @@ static bool wide_box(const TcConvArgs &a, int nsm, TcParams *p, size_t *smem) {
       if (bytes > (size_t)TC_SMEM_LIMIT) continue;
       const int n_mma = ((th - 1) * wp + tw + 15) / 16 * 16;
       const long tiles = rows * ((a.W + tw - 1) / tw) * a.N;
-      const double cost = (double)((tiles + nsm - 1) / nsm) * (9.0 * cblocks * (2.0 * n_mma + 80.0) + 1500.0);
-      if (best >= 0 && cost >= best) continue;
-      best = cost;
-      p->tw = tw; p->th = th; p->tn = 1;
-      p->halo_wp = wp;
-      p->halo_a_bytes = x_bytes;
-      p->wide_slab_bytes = slab;
-      *smem = bytes;
+      const double cycles = (double)((tiles + nsm - 1) / nsm) * (9.0 * cblocks * (2.0 * n_mma + 140.0) + 1500.0);
+      if (box->cycles >= 0 && cycles >= box->cycles) continue;
+      *box = WideBox{tw, th, wp, x_bytes, slab, bytes, cycles};
     }
   }
-  if (best < 0) return false;
-  p->halo = 1;
-  return true;
+  return box->cycles >= 0;
+}
+
+// Whether the pixel-N form that loads its pixels anew takes such a layer in less: its tiles hold 256 pixels of several
+// images, where images are small and the wide form's tile is a part of one.  Of the whole batch, a.form_n: a piece takes
+// the form the batch takes.  Fitted to 276 layers, 64 and 128 onto 64, 96 and 128 channels at 4x4 to 112x112 (what is
+// taken is 1 % slower on average than the faster one; the factor is for the model's error): 128 -> 128 with 300 000 pixels at 4x4 76 us in that form and
+// 334 in the wide one, 7x7 76 and 134, 8x8 78 and 113, 10x10 76 and 84, 12x12 78 and 76, 14x14 76 and 72, 28x28 78 and 68.
+static bool pixel_n_is_faster(const TcConvArgs &a, int nsm, double wide_cycles) {
+  int tw, th, tn;
+  choose_box(a.Q, a.P, a.N, 256, &tw, &th, &tn);
+  const long tiles = (long)((a.Q + tw - 1) / tw) * ((a.P + th - 1) / th) * ((a.N + tn - 1) / tn);
+  return 1.15 * (double)((tiles + nsm - 1) / nsm) * (9.0 * (a.Cf / 64) * 600.0 + 8000.0) <= wide_cycles;
 }
 
 static bool sk_plan(const TcConvArgs &a, int *err_word, int nsm, bool counted, double rival, const SkChoice *form,
@@ -836,10 +846,11 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   TcParams &p = pl.p;
   // A piece of a batch: the split-reduction kernel, with the same shares, where the whole batch takes it.  (Each of the
   // persistent kernels sums up in one order, whatever its tiles: filter taps outside and channels inside, the wide form the
-  // other way round.  So that an image has the same bits in a piece, which of them a layer takes must not depend on the
-  // number of images; `wide` below does not: wide_box() finds a box or none by the image and the channels.)
+  // other way round.  So that an image has the same bits in a piece, a piece takes the
+  // one that the whole batch does.)
   const bool piece = a.form_n != 0;
   SkChoice whole{0, 1, 0, -1.0};
+  bool whole_wide = false;
   if (piece) {
     TcConvArgs w = a;
     w.form_n = 0;
@@ -848,6 +859,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
     const Plan of = build_plan(w, err_word, num_sms, false, allow_halo);
     if (!of.ok) return pl;
     if (of.sk) whole = SkChoice{of.bn, of.s.splits, 0, 0.0};
+    whole_wide = of.wide;
   }
   const SkChoice *form = whole.bn ? &whole : nullptr;
   if (a.split) {
@@ -901,10 +913,19 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   const int nsm = num_sms > 0 ? num_sms : 148;
   const bool few = !halo && pn_allowed && !a.f16 && !a.out_f32 && !a.x2 && a.K <= 128 && a.R * a.S > 1 &&
                    a.R * a.S * a.Cf >= 9 * 64;
-  // Of the layers with few channels, the 3x3 ones of stride 1 go to the wide form (figures there); others, and those
-  // with a shortcut tensor, to the form whose k-steps load their pixels one by one.
+  // Of the layers with few channels, the 3x3 ones of stride 1 go to the wide form (figures there) unless images are small;
+  // others, and those with a shortcut tensor, to the form whose k-steps load their pixels one by one.
+  WideBox box;
   const bool wide = few && allow_halo && halo_allowed && is_3x3_same(a) && a.Cf % 64 == 0 && !a.residual &&
-                    wide_box(a, nsm, &p, &pl.smem);
+                    wide_box(a, nsm, &box) && (piece ? whole_wide : a.pool2 || !pixel_n_is_faster(a, nsm, box.cycles));
+  if (wide) {
+    p.tw = box.tw; p.th = box.th; p.tn = 1;
+    p.halo = 1;
+    p.halo_wp = box.wp;
+    p.halo_a_bytes = box.x_bytes;
+    p.wide_slab_bytes = box.slab;
+    pl.smem = box.smem;
+  }
   const bool pn = few && !wide && !a.pool2;
   pl.pn = pn;
   pl.wide = wide;
@@ -988,8 +1009,10 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
     const int per_wave = pair ? nsm / 2 : nsm;
     const double waves = (double)((p.total_tiles + per_wave - 1) / per_wave);
     const int ks = p.cblocks * a.R * a.S + p.cblocks2;
-    const double tile_us = halo ? 0.9 : wide ? (0.05 + 0.0011 * p.n_mma) * ks : pn ? 0.49 * ks : (bn == 256 ? 0.1 : 0.0) + 0.27 * ks * (bk == 64 ? 1.0 : 0.75);
-    if (!a.pool2 && (!piece || form) && sk_plan(a, err_word, nsm, counted, 3.1 + waves * tile_us, form, &pl)) return pl;
+    const double tile_us = halo ? 0.9 : pn ? 0.49 * ks : (bn == 256 ? 0.1 : 0.0) + 0.27 * ks * (bk == 64 ? 1.0 : 0.75);
+    if (!a.pool2 && (!piece || form) &&
+        sk_plan(a, err_word, nsm, counted, 3.1 + (wide ? box.cycles / 1900.0 : waves * tile_us), form, &pl))
+      return pl;
     if (a.pool2 && !halo && !wide && !pair) return pl;   // (not ok: tc_conv_takes_pool() said so)
   }
   const uint32_t boxA[4] = {(uint32_t)bk, (uint32_t)p.tw, (uint32_t)p.th, (uint32_t)p.tn};

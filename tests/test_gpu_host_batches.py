@@ -140,6 +140,29 @@ def test_same_bits_in_pieces(binding, name, math, N, image):
     assert rt.last_error() == 0
 
 
+def test_pieces_take_the_forms_of_the_batch(binding):
+    """Layers on 8x8 images, for which 450 of them share tiles and a piece's 80 to 150 by themselves would not: the two forms
+    sum up in orders of their own, and an image has the same bits all the same."""
+    rt.set_math_mode(rt.MATH_BF16)
+    g = graphs.Graph((450, 3, 64, 64), seed=1)
+    v = g.maxpool(g.relu(g.conv(0, *g.he_conv(64, 3, 7, 7), pads=(3, 3), strides=(2, 2))), (3, 3), (1, 1), (2, 2))
+    v = g.relu(g.conv(v, *g.he_conv(128, 64, 1, 1), strides=(2, 2)))
+    for _ in range(3):
+        v = g.relu(g.conv(v, *g.he_conv(128, 128, 3, 3), pads=(1, 1)))
+    g.mark_output(g.linear(g.flatten(g.gap(v)), 128, 40))
+    p = g.to_program()
+    p.lower(fuse=replay.FUSE_REFERENCE)
+    x = torch.from_numpy(rand(1, *g.input_shape)).pin_memory().numpy()
+    outs, n0 = [], rt.form_counters()
+    for _ in range(12):
+        outs.append(p.run(binding, x)[0])
+    n1 = rt.form_counters()
+    assert n1["in_pieces"] > n0["in_pieces"] and n1["column_strips"] == n0["column_strips"]
+    for y in outs[2:]:
+        assert np.array_equal(y, outs[1])
+    assert rt.last_error() == 0
+
+
 def test_other_tensors_behind_pieces(native_libs):
     """A program that goes on like the recorded one until its result has been read, and then reads another tensor."""
     rt.set_math_mode(rt.MATH_BF16)

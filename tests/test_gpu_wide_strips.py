@@ -51,3 +51,22 @@ def test_wide(binding, N, C, H, W, K, act, pool):
         assert max_rel_err(y, want) <= 2.0 ** -8 * 1.02   # (and what sums in another order differ by)
         assert np.array_equal(y, got[2])
     assert rt.last_error() == 0
+
+
+@pytest.mark.parametrize("N,C,H,W,K", [(600, 128, 7, 6, 128), (700, 64, 4, 4, 128), (900, 192, 9, 8, 72), (2000, 128, 8, 8, 64)])
+def test_small_images_share_tiles(binding, N, C, H, W, K):
+    """Images much smaller than a tile go to the form whose tiles hold several."""
+    g = graphs.Graph((N, C, H, W), seed=N + C + H)
+    w, b = g.he_conv(K, C, 3, 3)
+    g.mark_output(g.relu(g.conv(0, _bf16(w), b, pads=(1, 1))))
+    x = _bf16(graphs.make_input(g, 1))
+    (want,) = run_graph_oracle(g, x)
+    rt.set_math_mode(rt.MATH_BF16)
+    p = g.to_program()
+    p.lower(fuse=replay.FUSE_REFERENCE)
+    before = rt.form_counters()["column_strips"]
+    got = [p.run(binding, x)[0] for _ in range(3)]
+    assert rt.form_counters()["column_strips"] == before
+    for y in got:
+        assert max_rel_err(y, want) <= 2.0 ** -8 * 1.02
+    assert rt.last_error() == 0
