@@ -42,10 +42,11 @@ def _run(binding, N, C, H, W, K, R, pad, stride, act, mode):
     (8, 3, 224, 224, 64, 3, 1, 1, "relu"),
     (20, 3, 97, 131, 64, 3, 1, 1, "relu"),     # two tiles to a row, neither whole
     (9, 3, 60, 300, 40, 3, 1, 1, "clip"),      # three; channels with a remainder
-    (30, 3, 160, 97, 32, 3, 1, 2, "clip"),
+    (30, 3, 160, 112, 32, 3, 1, 2, "clip"),    # the shortest rows that are read this way
+    (30, 3, 91, 56, 32, 3, 1, 1, "clip"),
     (12, 4, 222, 171, 24, 3, 1, 2, None),
     (7, 1, 150, 129, 64, 3, 2, 1, "relu"),     # a row of padding beyond the filter's reach into the image
-    (40, 2, 120, 64, 16, 2, 0, 1, "relu"),
+    (40, 2, 120, 69, 16, 2, 0, 1, "relu"),
     (24, 3, 128, 128, 64, 1, 0, 1, "relu"),
 ])
 def test_rows(binding, N, C, H, W, K, R, pad, stride, act, mode):
@@ -57,6 +58,9 @@ def test_rows(binding, N, C, H, W, K, R, pad, stride, act, mode):
     (8, 3, 120, 130, 72, 3, 1, 1),     # ... channels of the result
     (8, 9, 120, 130, 64, 3, 1, 1),     # ... of the input
     (8, 3, 120, 130, 64, 3, 3, 1),     # padding as high as the filter
+    (30, 3, 160, 97, 32, 3, 1, 2),     # short rows
+    (40, 2, 120, 64, 16, 2, 0, 1),
+    (24, 3, 97, 79, 64, 1, 0, 1),
 ])
 def test_other_stems_read_windows(binding, N, C, H, W, K, R, pad, stride):
     assert _run(binding, N, C, H, W, K, R, pad, stride, "relu", rt.MATH_BF16) == 0
