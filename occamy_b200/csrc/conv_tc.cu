@@ -846,8 +846,7 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   TcParams &p = pl.p;
   // A piece of a batch: the split-reduction kernel, with the same shares, where the whole batch takes it.  (Each of the
   // persistent kernels sums up in one order, whatever its tiles: filter taps outside and channels inside, the wide form the
-  // other way round.  So that an image has the same bits in a piece, a piece takes the
-  // one that the whole batch does.)
+  // other way round.  So that an image has the same bits in a piece, a piece takes the one that the whole batch does.)
   const bool piece = a.form_n != 0;
   SkChoice whole{0, 1, 0, -1.0};
   bool whole_wide = false;
@@ -931,13 +930,13 @@ static Plan build_plan(const TcConvArgs &a, int *err_word, int num_sms, bool cou
   pl.wide = wide;
   // Few-channel stems with up to three filter rows whose kernel runs twice on an SM (below) read their windows in place
   // (TC_MODE_ROWS); every row of the output has a filter row inside the image.  A tile is one row, or a part of one, and
-  // takes some 800 cycles however short it is; through the maps it takes 128 windows of several rows, and as long for each
+  // takes 0.4 to 1 us however short it is (one of an SM's two); through the maps it is 128 windows of several rows, for each
   // row of the filter.  3 -> 64 3x3 with 2.4 million outputs, this way and the other, by the columns of a tile: 24 86 and 34
   // us, 40 44 and 34, 48 39 and 33, 56 34 and 34, 72 29 and 35, 128 22 and 36; two filter rows (3 -> 48) 57 31 and 27, 65 27
   // and 27, 81 24 and 26; one (3 -> 16) 64 18 and 16, 80 16 and 16, 112 14 and 16.
   const int row_cols = (Qg + (Qg + 127) / 128 - 1) / ((Qg + 127) / 128);
-  bool rows = row_cols >= 92 - 12 * a.R && allow_halo && a.w_step == 8 && a.S == 1 && a.R <= 3 && a.pad_h < a.R && a.Cf <= 32 && a.K <= 64 && !a.out_f32 && !a.residual &&
-              !a.pool2 && !pn && num_sms >= 2;
+  bool rows = allow_halo && a.w_step == 8 && a.S == 1 && a.R <= 3 && row_cols >= 92 - 12 * a.R && a.pad_h < a.R &&
+              a.Cf <= 32 && a.K <= 64 && !a.out_f32 && !a.residual && !a.pool2 && !pn && num_sms >= 2;
   if (wide) {   // (the box is chosen)
   } else if (rows) {
     p.tw = row_cols;
